@@ -6,6 +6,7 @@
     run(state)       one pass through the public entry points
     work(c)          bytes and operations the pass cannot do without
     tolerance(c)     how far two correct implementations may differ
+    exact(c, s)      what run returns for these inputs, in 64 bits, where it is a computed number
 
 Kinds of work (the key "kind"):
   attend     one layer's share of a decode step: KVCompCache.attend over a compressed cache plus its recent window
@@ -307,3 +308,45 @@ def tolerance(case):
     if case["kind"] in ("prefill", "readback") or (case["kind"] == "generate" and case["api"] == "update"):
         return "exact"
     return {"rel": 1e-3, "max": 1e-2}
+
+
+# ---- the same in 64 bits -------------------------------------------------------------------------------
+def _dequantised(c, x, is_k, shared):
+    """x [T,B,H,D] as the compressed cache holds it, in 64 bits: round(x / step) * step, the quotient in 16 bits,
+    step = rel * range in 16 bits.  shared: a unit spans the sequences."""
+    rel, mode = (c["krel"], c["kmode"]) if is_k else (c["vrel"], c["vmode"])
+    T, B, H, _ = x.shape
+    n = c["block"] if mode in ("BlockQuant", "ChannelQuant") else 1
+    u = x.view(T // n, n, B, H, D)
+    dims = {"BlockQuant": (1, 3, 4), "ChannelQuant": (1,), "TokenQuant": (3, 4), "VectorQuant": (4,)}[mode]
+    dims += (2,) if shared else ()
+    step = ((u.amax(dims, keepdim=True) - u.amin(dims, keepdim=True)).float() * torch.tensor(rel, dtype=torch.float32)).half()
+    return ((u / step).round().double() * step.double()).view(T, B, H, D)
+
+
+def exact(case, seed):
+    c = case
+    if c["kind"] not in ("attend", "matvec", "operators"):       # bytes and 16-bit rows, exact as they are
+        return None
+    B, H, G, T = c["B"], c["Hkv"], c["G"], c["T"]
+    k, v, q = _kv(c, T, seed)
+    if c["kind"] == "attend":
+        over = T + c["block"] - T % c["block"] - c["recent"]      # whole blocks beyond the recent window are compressed
+        n = min(max(0, over) // c["block"] * c["block"], T) // c["block"] * c["block"]
+        out = torch.empty(B, H * G, 1, D, dtype=torch.float64, device="cuda")
+        for b in range(B):
+            kb, vb = (torch.cat([_dequantised(c, x[:n, b:b + 1], is_k, False), x[n:, b:b + 1].double()])[:, 0].transpose(0, 1)
+                      for x, is_k in ((k, True), (v, False)))      # [H, T, D]
+            s = torch.matmul(q[b].double().view(H, G, D), kb.transpose(1, 2)) / math.sqrt(D)
+            out[b] = torch.matmul(torch.softmax(s, dim=-1), vb).view(H * G, 1, D)
+        return out
+    p = torch.softmax(2.5 * torch.randn(B, H, T, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed)), dim=-1).half()
+    scores = torch.empty(B, H, T, dtype=torch.float64, device="cuda")
+    parts = torch.empty(T // 128, B, H, D, dtype=torch.float64, device="cuda")
+    for t in range(0, T, 128):                                    # 128 is a whole number of units of either tensor
+        kt, vt = _dequantised(c, k[t:t + 128], True, True), _dequantised(c, v[t:t + 128], False, True)
+        scores[:, :, t:t + 128] = torch.einsum("tbhd,bhd->bht", kt, q.double())
+        parts[t // 128] = torch.einsum("tbhd,bht->bhd", vt, p[:, :, t:t + 128].double())
+    if c["kind"] == "matvec":
+        return scores, parts.sum(dim=0, keepdim=True)
+    return [None] * 8 + [scores, parts]
