@@ -120,19 +120,46 @@ __device__ short heap_pop(Heap &hp, long long *f_out) {
     return top_id;
 }
 
+// The heap is a serial chain by contract (its layout decides ties), everything around it is spread over the CTA:
+// with one thread walking the trees and symbols too, a book of 20 to 30 symbols took 76 us; now 19 to 26 us, of which
+// the heap takes most.
+constexpr int BOOK_THREADS = 1024;
+
 struct BookSmem {
     long long hf[512];
     short hid[512];
-    short left[512], right[512];
+    short parent[512];           // of a leaf (its symbol) or an inner node of the Huffman tree: node << 1 | bit
+    uint8_t listed[256];         // the symbols that have a code, ascending
+    uint32_t aligned[256];       // per listed symbol: its code, first bit on top
+    short first_new[256], node0[256];   // per listed symbol: the shortest prefix no earlier symbol has, and its node
+    uint32_t warp_sum[BOOK_THREADS / 32];
+    int total;
     uint32_t enc_code[256], enc_len[256];
     uint32_t tree[512];          // wide tree: lo16 = child0 (or LEAF), hi16 = child1 (or symbol)
     long long count[256];        // the histogram, fetched by all threads at once
     int n_nodes, n_symbols, min_sym, max_sym, max_len, flags;
 };
 
+// Exclusive prefix sum of x over the CTA's first 256 threads (the others pass 0); *total receives the sum.
+// All threads call; contains barriers.
+__device__ uint32_t book_scan(BookSmem &s, uint32_t x, int tid, uint32_t *total) {
+    const int lane = tid & 31, warp = tid >> 5;
+    uint32_t y = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t z = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += z; }
+    __syncthreads();
+    if (lane == 31) s.warp_sum[warp] = y;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) { const uint32_t t = s.warp_sum[w]; if (w < warp) before += t; all += t; }
+    *total = all;
+    return before + y - x;
+}
+
 // insert every code into the decode trees in ascending symbol order
 // (build_decode_code_book, src/huffman.cpp:229-252); run by one thread
-__device__ void build_trees(BookSmem &s) {      // s.tree was cleared to {NONE, NONE} by the whole CTA
+__device__ void build_trees_serial(BookSmem &s) {      // s.tree was cleared to {NONE, NONE} by the whole CTA
     int n = 2;
     for (int sym = 0; sym < 256; sym++) {
         int len = (int)s.enc_len[sym];
@@ -158,6 +185,54 @@ __device__ void build_trees(BookSmem &s) {      // s.tree was cleared to {NONE, 
     s.n_nodes = n;
 }
 
+// The same tree, a thread per symbol.  The symbols inserted before symbol i share at most a prefix of m bits with it, so
+// its insertion appends the nodes of its prefixes of m + 1 .. length bits, in this order (the one-bit prefixes are
+// nodes 0 and 1); a prefix sum over the symbols gives their numbers, and the node of the m-bit prefix is one of the
+// first symbol that has this prefix.  Codes beyond 32 bits and trees that do not fit take the serial form.
+// All threads call; s.enc_code / enc_len / tree / flags / max_len are set.
+__device__ void build_trees(BookSmem &s, int tid) {
+    const uint32_t has = tid < 256 && s.enc_len[tid & 255] ? 1u : 0u;
+    uint32_t n, total;
+    const uint32_t slot = book_scan(s, has, tid, &n);
+    if (has) {
+        s.listed[slot] = (uint8_t)tid;
+        s.aligned[slot] = s.enc_len[tid] <= 32 ? s.enc_code[tid] << (32 - s.enc_len[tid]) : 0u;
+    }
+    __syncthreads();
+    const bool mine = tid < (int)n;
+    const uint32_t sym = mine ? s.listed[tid] : 0u, a = mine ? s.aligned[tid] : 0u;
+    const int len = mine ? (int)s.enc_len[sym] : 0;
+    int m = 1, owner = -1;                              // at least the one-bit prefix is there
+    if (mine && len <= 32) {
+        for (int j = 0; j < tid; j++) {
+            const int c = __clz((int)(a ^ s.aligned[j]));
+            if (c > m) { m = c; owner = j; }            // the first one that shares m bits owns the prefix
+        }
+        m = min(m, len);
+    }
+    const int fresh = mine ? len - m : 0;
+    const uint32_t base = 2u + book_scan(s, (uint32_t)fresh, tid, &total);
+    if (s.max_len > 32 || total + 2u > 512u) {
+        if (tid == 0) build_trees_serial(s);
+        __syncthreads();
+        return;
+    }
+    if (mine) { s.first_new[tid] = (short)(m + 1); s.node0[tid] = (short)base; }
+    __syncthreads();
+    if (mine) {
+        unsigned short *half = reinterpret_cast<unsigned short *>(s.tree);         // child 0 below child 1
+        int at = owner < 0 ? (int)(a >> 31) : s.node0[owner] + (m - s.first_new[owner]);
+        for (int k = m; k < len; k++) {
+            const int next = (int)base + (k - m);
+            half[2 * at + ((a >> (31 - k)) & 1u)] = (unsigned short)next;
+            at = next;
+        }
+        s.tree[at] = KVC_TREE_LEAF | (sym << 16);
+    }
+    if (tid == 0) s.n_nodes = (int)total + 2;
+    __syncthreads();
+}
+
 // Decode table entry for a KVC_LUT_BITS-bit window w (first stream bit = MSB), 32 bits:
 //   byte 0      how far the decoder state advances: (symbols << 6) | bits consumed   (0 = escape)
 //   bytes 1..3  up to three complete symbols found in the window, unused bytes 0
@@ -166,16 +241,17 @@ __device__ void build_trees(BookSmem &s) {      // s.tree was cleared to {NONE, 
 // byte 0 is 0 and the upper bytes hold the wide-tree node the window's bits lead to; the slow path
 // continues from there one bit at a time.
 __device__ uint32_t lut_entry(const uint32_t *tree, uint32_t w) {
-    uint32_t syms = 0, nsym = 0, used = 0;
+    uint32_t syms = 0, nsym = 0, used = 0, node = 0;
     int idx = -1, pos = 0;
     while (pos < KVC_LUT_BITS) {
         int bit = (w >> (KVC_LUT_BITS - 1 - pos)) & 1;
-        uint32_t ch = idx == -1 ? (uint32_t)bit : ((tree[idx] >> (16 * bit)) & 0xffffu);
+        uint32_t ch = idx == -1 ? (uint32_t)bit : ((node >> (16 * bit)) & 0xffffu);
         pos++;
         if (ch == KVC_TREE_NONE || ch >= 512) { idx = -2; break; }     // no such code
         idx = (int)ch;
-        if ((tree[idx] & 0xffffu) == KVC_TREE_LEAF) {
-            syms |= (tree[idx] >> 16) << (8 * nsym);
+        node = tree[idx];
+        if ((node & 0xffffu) == KVC_TREE_LEAF) {
+            syms |= (node >> 16) << (8 * nsym);
             nsym++; used = pos; idx = -1;
             if (nsym == 3) break;
         }
@@ -220,70 +296,63 @@ __device__ void write_book(const BookSmem &s, uint8_t *book, int tid, int nthr) 
     }
 }
 
-__global__ void __launch_bounds__(256) build_codebook_kernel(const unsigned long long *__restrict__ hist,
-                                                             uint8_t *__restrict__ book) {
+__global__ void __launch_bounds__(BOOK_THREADS) build_codebook_kernel(const unsigned long long *__restrict__ hist,
+                                                                      uint8_t *__restrict__ book) {
     __shared__ BookSmem s;
     const int tid = threadIdx.x;
-    s.enc_code[tid] = 0; s.enc_len[tid] = 0;
-    s.count[tid] = (long long)hist[tid];                    // one coalesced load instead of 256 dependent ones
-    s.tree[tid] = s.tree[tid + 256] = KVC_TREE_NONE | (KVC_TREE_NONE << 16);
+    const long long count = tid < 256 ? (long long)hist[tid] : 0;
+    if (tid < 256) { s.enc_code[tid] = 0; s.enc_len[tid] = 0; }
+    if (tid < 512) s.tree[tid] = KVC_TREE_NONE | (KVC_TREE_NONE << 16);
+    if (tid == 0) { s.flags = 0; s.max_len = 0; }
+    uint32_t nsym;
+    const uint32_t slot = book_scan(s, count > 0 ? 1u : 0u, tid, &nsym);
+    if (count > 0) { s.listed[slot] = (uint8_t)tid; s.count[slot] = count; }
     __syncthreads();
     if (tid == 0) {
-        Heap hp; hp.w = reinterpret_cast<unsigned long long *>(s.hf); hp.n = 0;
-        int nsym = 0, mn = 256, mx = -1;
-        s.flags = 0;
-        for (int i = 0; i < 256; i++) {
-            long long c = s.count[i];
-            if (c > 0) { heap_push(hp, c, (short)i); nsym++; if (i < mn) mn = i; mx = i; }
-        }
-        s.n_symbols = nsym; s.min_sym = nsym ? mn : 0; s.max_sym = nsym ? mx : 0; s.max_len = 0;
+        s.n_symbols = (int)nsym; s.min_sym = nsym ? s.listed[0] : 0; s.max_sym = nsym ? s.listed[nsym - 1] : 0;
         if (nsym == 0) s.flags |= KVC_FLAG_NO_SYMBOLS;
-        else if (nsym == 1) {          // utils/huffman.py:42-44: the lone symbol gets '0'
-            const int lone = (int)(hp.w[0] & 0x3ff);
-            s.enc_code[lone] = 0; s.enc_len[lone] = 1; s.max_len = 1;
-        } else {
-            short next = 256;
-            while (hp.n > 1) {
-                long long fa, fb;
-                short a = heap_pop(hp, &fa);
-                short b = heap_pop(hp, &fb);
-                s.left[next] = a; s.right[next] = b;
-                heap_push(hp, fa + fb, next);
-                next++;
-            }
-            // iterative walk; the heap arrays are free now and serve as the stack
-            short *st_node = s.hid; long long *st_code = s.hf;     // code | (len << 40)
-            int sp = 1;
-            st_node[0] = (short)(hp.w[0] & 0x3ff); st_code[0] = 0;
-            while (sp) {
-                sp--;
-                short nd = st_node[sp];
-                unsigned long long cl = (unsigned long long)st_code[sp];
-                unsigned long long code = cl & 0xffffffffffull, len = cl >> 40;
-                if (nd < 256) {
-                    if (len > 32) s.flags |= KVC_FLAG_CODE_TOO_LONG;
-                    s.enc_code[nd] = (uint32_t)code; s.enc_len[nd] = (uint32_t)len;
-                    if ((int)len > s.max_len) s.max_len = (int)len;
-                } else {
-                    st_node[sp] = s.right[nd]; st_code[sp] = (long long)((((code << 1) | 1) & 0xffffffffffull) | ((len + 1) << 40)); sp++;
-                    st_node[sp] = s.left[nd];  st_code[sp] = (long long)(((code << 1) & 0xffffffffffull) | ((len + 1) << 40)); sp++;
-                }
-            }
+        Heap hp; hp.w = reinterpret_cast<unsigned long long *>(s.hf); hp.n = 0;
+        for (uint32_t i = 0; i < nsym; i++) heap_push(hp, s.count[i], (short)s.listed[i]);
+        short next = 256;
+        while (hp.n > 1) {
+            long long fa, fb;
+            short a = heap_pop(hp, &fa);
+            short b = heap_pop(hp, &fb);
+            s.parent[a] = (short)(next << 1); s.parent[b] = (short)(next << 1 | 1);
+            heap_push(hp, fa + fb, next);
+            next++;
         }
-        build_trees(s);
+        s.total = next - 1;                                 // the root
     }
     __syncthreads();
-    write_book(s, book, tid, 256);
+    if (count > 0) {                                        // a symbol's code, from its leaf up: last bit first
+        uint32_t code = 0;
+        int len = 0;
+        if (nsym == 1) len = 1;                             // utils/huffman.py:42-44: the lone symbol gets '0'
+        else for (int nd = tid; nd != s.total; len++) {
+            const int up = s.parent[nd];
+            if (len < 32) code |= (uint32_t)(up & 1) << len;
+            nd = up >> 1;
+        }
+        s.enc_code[tid] = code; s.enc_len[tid] = (uint32_t)len;
+        atomicMax(&s.max_len, len);
+        if (len > 32) atomicOr(&s.flags, KVC_FLAG_CODE_TOO_LONG);
+    }
+    __syncthreads();
+    build_trees(s, tid);
+    write_book(s, book, tid, BOOK_THREADS);
 }
 
 // A reference-format decode tensor (3-byte nodes; child bytes read as unsigned, 0xff = unset)
 // -> the same book.  Codes are recovered by walking the tree from both root children.
-__global__ void __launch_bounds__(256) book_from_tree_kernel(const uint8_t *__restrict__ rt, int n_nodes,
-                                                             uint8_t *__restrict__ book) {
+__global__ void __launch_bounds__(BOOK_THREADS) book_from_tree_kernel(const uint8_t *__restrict__ tree, int n_nodes,
+                                                                      uint8_t *__restrict__ book) {
     __shared__ BookSmem s;
+    __shared__ uint8_t rt[3 * 256];                         // child bytes reach no further node
     const int tid = threadIdx.x;
-    s.enc_code[tid] = 0; s.enc_len[tid] = 0;
-    s.tree[tid] = s.tree[tid + 256] = KVC_TREE_NONE | (KVC_TREE_NONE << 16);
+    if (tid < 256) { s.enc_code[tid] = 0; s.enc_len[tid] = 0; }
+    if (tid < 512) s.tree[tid] = KVC_TREE_NONE | (KVC_TREE_NONE << 16);
+    if (tid < 3 * min(n_nodes, 256)) rt[tid] = tree[tid];
     __syncthreads();
     if (tid == 0) {
         s.flags = 0; s.max_len = 0;
@@ -312,10 +381,10 @@ __global__ void __launch_bounds__(256) book_from_tree_kernel(const uint8_t *__re
         }
         s.n_symbols = nsym; s.min_sym = nsym ? mn : 0; s.max_sym = nsym ? mx : 0;
         if (nsym == 0) s.flags |= KVC_FLAG_NO_SYMBOLS;
-        build_trees(s);
     }
     __syncthreads();
-    write_book(s, book, tid, 256);
+    build_trees(s, tid);
+    write_book(s, book, tid, BOOK_THREADS);
 }
 
 }  // namespace
@@ -335,7 +404,7 @@ extern "C" int kvc_histogram(const uint8_t *codes, int64_t n, unsigned long long
 extern "C" int kvc_build_codebook(const unsigned long long *hist, void *book, kvc_stream_t stream) {
     KVC_REQUIRE(hist && book, "kvc_build_codebook: null pointer");
     KVC_REQUIRE((reinterpret_cast<uintptr_t>(book) & 15) == 0, "kvc_build_codebook: book must be 16-byte aligned");
-    build_codebook_kernel<<<1, 256, 0, kvc_cu(stream)>>>(hist, reinterpret_cast<uint8_t *>(book));
+    build_codebook_kernel<<<1, BOOK_THREADS, 0, kvc_cu(stream)>>>(hist, reinterpret_cast<uint8_t *>(book));
     KVC_LAUNCH_OK();
     return KVC_OK;
 }
@@ -345,7 +414,7 @@ extern "C" int kvc_book_from_tree(const uint8_t *ref_tree, int64_t tree_bytes, v
     KVC_REQUIRE(tree_bytes % 3 == 0 && tree_bytes >= 6, "kvc_book_from_tree: a decode tensor holds 3-byte nodes, at least two");
     KVC_REQUIRE(tree_bytes / 3 <= 255, "kvc_book_from_tree: %lld nodes; 8-bit child indices address at most 255", (long long)(tree_bytes / 3));
     KVC_REQUIRE((reinterpret_cast<uintptr_t>(book) & 15) == 0, "kvc_book_from_tree: book must be 16-byte aligned");
-    book_from_tree_kernel<<<1, 256, 0, kvc_cu(stream)>>>(ref_tree, (int)(tree_bytes / 3), reinterpret_cast<uint8_t *>(book));
+    book_from_tree_kernel<<<1, BOOK_THREADS, 0, kvc_cu(stream)>>>(ref_tree, (int)(tree_bytes / 3), reinterpret_cast<uint8_t *>(book));
     KVC_LAUNCH_OK();
     return KVC_OK;
 }
