@@ -77,17 +77,26 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     return v;
 }
 
-// ---- grouped queries (G >= 2): decode first, multiply afterwards -----------------------------------
-// With several query heads per KV head the weight records of a position grow to 16 or 32 bytes, and
-// 32 lanes at 32 different positions fetch 0.5-1 KB per lookup: the kernel becomes bound by shared-memory
-// wavefronts.  So a thread first decodes its vector into a private row of bytes in shared memory and
-// then walks the row four positions at a time; now all lanes of a warp are at the same position, the
-// weight words are one broadcast read, and they need no overlapping window: a word holds the hi (or lo)
-// bytes of 4 consecutive positions.  The integer sums are the same as in the one-pass form.
-constexpr int ROW_STRIDE = 140;           // bytes of a thread's row: 128 symbols + up to 8 of overrun, + 1 word; 35 words spread the banks
-static_assert(ROW_STRIDE >= 128 + KVC_DECODE_OVERRUN_PAIR + 3, "rows too short for paired lookups");
+// ---- grouped queries (the attention kernel, G >= 2): decode first, multiply on the tensor cores -------
+// With several query heads per KV head the weight records of a position grow to 16 bytes and more, and 32
+// lanes at 32 different positions fetch 0.5 KB and more per lookup: the kernel becomes bound by shared-memory
+// wavefronts.  So a thread first decodes its vector into a private row of bytes in shared memory; then the
+// 32 rows of a warp are a 32 x 128 matrix of unsigned bytes, the weights of up to 8 heads a 128 x 8 matrix of
+// hi bytes and one of lo bytes, and m16n8k32 integer instructions multiply them.  The integer sums are the
+// same as in the one-pass form.  What bounds it: two CTAs of eight warps fit an SM (tables, slots, rows), 0.55
+// instructions issue per cycle and scheduler, half of the shared-memory pipe's wavefronts are used.  Against byte
+// stores and four dp4a pairs per word (one layer, rel 0.05 / 0.1): 16 sequences x 32768 tokens, 8 x 4 heads, 981 -> 836 us,
+// 1777 -> 1000 shared-memory wavefronts per warp and tile; 3 x 2881 tokens, 4 x 6 heads, 46 -> 31 us.
+// Rows of 36 words: 128 symbols, the overrun of paired lookups, and a 16-byte alignment at which the fragment
+// loads (16 bytes of row 4r+i by lane 4r+q) touch every bank once per quarter warp.
+constexpr int ROW_WORDS = 36;
+static_assert(ROW_WORDS * 4 >= 128 + KVC_DECODE_OVERRUN_PAIR + 3, "rows too short for paired lookups");
 constexpr int WROW = 136;                 // weight words per vector of the one-pass form: 128 positions + zeroed overrun
-template <int G, bool ROWS> struct VecWords { static constexpr int value = ROWS ? 32 * 2 * G : 2 * WROW * G; };   // weight words of one vector
+// weight words of one vector: rows form [hi | lo][G][32 groups of 4 positions], one-pass form w_hi / w_lo
+template <int G, bool ROWS> struct VecWords { static constexpr int value = ROWS ? 2 * G * 32 : 2 * WROW * G; };
+// word of head g and position group w in the rows form: 16-byte chunks swizzled by the head, so that neither the
+// fragment loads (two heads x four chunks per quarter warp) nor the V phase's stores meet in a bank more than twice
+__device__ __forceinline__ uint32_t w_rows(uint32_t g, uint32_t w) { return g * 32u + (w ^ ((((g & 1u) << 2) | (g >> 1)) << 2)); }
 
 // {hi word, lo word} of 4 consecutive positions (byte i = position i)
 __device__ __forceinline__ uint2 pack4_dense(int q0, int q1, int q2, int q3) {
@@ -97,40 +106,46 @@ __device__ __forceinline__ uint2 pack4_dense(int q0, int q1, int q2, int q3) {
     return r;
 }
 
-// decode the thread's vector into `row` (its own 33 words), then dot it with the weight words at w:
-// [32 groups of 4 positions][hi | lo][G]
+// c += A (16 x 32 unsigned bytes) * B (32 x 8 signed / unsigned bytes)
+__device__ __forceinline__ void mma_us(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_uu(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// decode the thread's vector into its row (shared address, 16-byte aligned)
+__device__ __forceinline__ bool decode_row(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, uint32_t tree_s, bool esc, uint32_t row_s) {
+    KvcRowWriter put;
+    return esc ? kvc_decode_vector<true, 0>(slot_s, byte_pos, lut_s, tree_s, row_s, put)
+               : kvc_decode_vector<false, 0, decltype(put), true>(slot_s, byte_pos, lut_s, tree_s, row_s, put);
+}
+
+// The products of a warp's 32 rows (first one at shared address rows_s) with the weight words at shared address
+// w_s.  d[i][j]: row 4 * (lane >> 2) + i, head (2 * (lane & 3) + j) % G (fewer than 8 heads: the columns repeat).
+// Which row is which row of a fragment and which word is which k index are free as long as A and B agree: a lane
+// then reads 16 consecutive bytes of four neighbouring rows and ends up with four neighbouring rows' sums.
 template <int G>
-__device__ __forceinline__ bool decode_rows(const uint8_t *slot, uint32_t byte_pos, const KvcBookSmem &book, bool esc,
-                                            uint32_t *row, const uint32_t *w, int (&hi)[G], int (&lo)[G]) {
-    static_assert(G == 2 || G == 4, "two or four query heads");
-    const uint32_t slot_s = kvc_smem_addr(slot), lut_s = kvc_smem_addr(book.lut), tree_s = kvc_smem_addr(book.tree);
-    const uint32_t row_s0 = kvc_smem_addr(row);
-    // three byte stores per lookup at the position the decoder hands out (its counter starts at the
-    // row's address); bytes past the lookup's symbols are rewritten by the next lookup, bytes past
-    // position 127 (two lookups per round: up to 8 of them) land in the row's last three words
-    auto put = [&](uint32_t e, uint32_t a) {
-        asm volatile("st.shared.u8 [%0], %1;\n\tst.shared.u8 [%0+1], %2;\n\tst.shared.u8 [%0+2], %3;"
-                     :: "r"(a), "r"(e >> 8), "r"(e >> 16), "r"(e >> 24) : "memory");
-    };
-    const bool ok = esc ? kvc_decode_vector<true, 0>(slot_s, byte_pos, lut_s, tree_s, row_s0, put)
-                        : kvc_decode_vector<false, 0, decltype(put), true>(slot_s, byte_pos, lut_s, tree_s, row_s0, put);
-    const uint32_t row_s = kvc_smem_addr(row), w_s = kvc_smem_addr(w);
-#pragma unroll 8
-    for (int wg = 0; wg < 32; wg++) {
-        const uint32_t x = kvc_lds32(row_s + wg * 4);
-        if (G == 4) {
-            const uint4 a = lds128(w_s + wg * 32), b = lds128(w_s + wg * 32 + 16);
-            hi[0] = kvc_dp4a_us(x, a.x, hi[0]); lo[0] = kvc_dp4a_uu(x, b.x, lo[0]);
-            hi[1 % G] = kvc_dp4a_us(x, a.y, hi[1 % G]); lo[1 % G] = kvc_dp4a_uu(x, b.y, lo[1 % G]);
-            hi[2 % G] = kvc_dp4a_us(x, a.z, hi[2 % G]); lo[2 % G] = kvc_dp4a_uu(x, b.z, lo[2 % G]);
-            hi[3 % G] = kvc_dp4a_us(x, a.w, hi[3 % G]); lo[3 % G] = kvc_dp4a_uu(x, b.w, lo[3 % G]);
-        } else {
-            const uint4 a = lds128(w_s + wg * 16);
-            hi[0] = kvc_dp4a_us(x, a.x, hi[0]); lo[0] = kvc_dp4a_uu(x, a.z, lo[0]);
-            hi[1 % G] = kvc_dp4a_us(x, a.y, hi[1 % G]); lo[1 % G] = kvc_dp4a_uu(x, a.w, lo[1 % G]);
-        }
+__device__ __forceinline__ void rows_dot(uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][2]) {
+    const uint32_t r = lane >> 2, q = lane & 3, g = r % G;
+    int h0[4] = {0, 0, 0, 0}, h1[4] = {0, 0, 0, 0}, l0[4] = {0, 0, 0, 0}, l1[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (uint32_t p = 0; p < 2; p++) {
+        const uint32_t aw = rows_s + (4 * r * ROW_WORDS + 16 * p + 4 * q) * 4, bw = w_s + w_rows(g, 16 * p + 4 * q) * 4;
+        const uint4 a0 = lds128(aw), a1 = lds128(aw + ROW_WORDS * 4), a2 = lds128(aw + ROW_WORDS * 8), a3 = lds128(aw + ROW_WORDS * 12);
+        const uint4 bh = lds128(bw), bl = lds128(bw + G * 32 * 4);
+        mma_us(h0, a0.x, a1.x, a0.y, a1.y, bh.x, bh.y); mma_us(h1, a2.x, a3.x, a2.y, a3.y, bh.x, bh.y);
+        mma_uu(l0, a0.x, a1.x, a0.y, a1.y, bl.x, bl.y); mma_uu(l1, a2.x, a3.x, a2.y, a3.y, bl.x, bl.y);
+        mma_us(h0, a0.z, a1.z, a0.w, a1.w, bh.z, bh.w); mma_us(h1, a2.z, a3.z, a2.w, a3.w, bh.z, bh.w);
+        mma_uu(l0, a0.z, a1.z, a0.w, a1.w, bl.z, bl.w); mma_uu(l1, a2.z, a3.z, a2.w, a3.w, bl.z, bl.w);
     }
-    return ok;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {                              // |256 hi + lo| <= 128 * 255 * 32767 < 2^31
+        d[0][j] = 256 * h0[j] + l0[j]; d[1][j] = 256 * h0[2 + j] + l0[2 + j];
+        d[2][j] = 256 * h1[j] + l1[j]; d[3][j] = 256 * h1[2 + j] + l1[2 + j];
+    }
 }
 
 // Where the hi / lo weight word of position c and head g sits in a vector's 2 * WROW * G words.  One or
@@ -145,7 +160,7 @@ template <int G, bool ESC>
 __device__ __forceinline__ bool decode_dot_impl(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, uint32_t tree_s,
                                                 uint32_t w_s, int (&hi)[G], int (&lo)[G]) {
     constexpr int SHIFT = G == 1 ? 3 : 4;                      // log2 of the record's bytes
-    auto emit = [&](uint32_t syms, uint32_t a) {
+    auto emit = [&](uint32_t syms, uint32_t a, uint32_t, uint32_t) {
         if (G == 4) {
             const uint4 x = lds128(a), y = lds128(a + WROW * 16);
             hi[0] = kvc_dp4a_us(syms, x.x, hi[0]); lo[0] = kvc_dp4a_uu(syms, y.x, lo[0]);
@@ -267,8 +282,7 @@ __device__ __forceinline__ void k_units_load(KUnit &u, const kvc_qmeta_dev &m, l
     }
 }
 
-// ROWS: the layout of decode_rows (grouped queries in the attention kernel) instead of w_hi / w_lo
-template <int G, bool ROWS = false>
+template <int G>
 __device__ __forceinline__ void k_weights_build(uint32_t *w, float *step, float *zp, const float *qf, const KUnit &u,
                                                 bool channel_units, int min_bytes, long long tok0, long long T, int tid) {
     const int lane = tid & 31, wp = tid >> 5, sub = wp & 3;
@@ -293,23 +307,48 @@ __device__ __forceinline__ void k_weights_build(uint32_t *w, float *step, float 
         int q4[7];
 #pragma unroll
         for (int i = 0; i < 4; i++) q4[i] = __float2int_rn(wv[i] * inv);
-        uint32_t *row = w + (size_t)sub * VecWords<G, ROWS>::value;
-        if (ROWS) {                                             // the lane's 4 positions are one group: [group][hi | lo][g]
-            const uint2 r = pack4_dense(q4[0], q4[1], q4[2], q4[3]);
-            row[(lane * 2 + 0) * G + g] = r.x; row[(lane * 2 + 1) * G + g] = r.y;
-        } else {
+        uint32_t *row = w + (size_t)sub * VecWords<G, false>::value;
 #pragma unroll
-            for (int i = 0; i < 3; i++) {                       // the next lane's first three values
-                int nv = __shfl_down_sync(0xffffffffu, q4[i], 1);
-                q4[4 + i] = lane == 31 ? 0 : nv;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {                       // layout: w_hi / w_lo
-                const uint2 r = pack4(q4[i], q4[i + 1], q4[i + 2], q4[i + 3]);
-                row[w_hi<G>(lane * 4 + i, g)] = r.x; row[w_lo<G>(lane * 4 + i, g)] = r.y;
-            }
-            if (lane < WROW - 128) { row[w_hi<G>(128 + lane, g)] = 0u; row[w_lo<G>(128 + lane, g)] = 0u; }
+        for (int i = 0; i < 3; i++) {                           // the next lane's first three values
+            int nv = __shfl_down_sync(0xffffffffu, q4[i], 1);
+            q4[4 + i] = lane == 31 ? 0 : nv;
         }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {                           // layout: w_hi / w_lo
+            const uint2 r = pack4(q4[i], q4[i + 1], q4[i + 2], q4[i + 3]);
+            row[w_hi<G>(lane * 4 + i, g)] = r.x; row[w_lo<G>(lane * 4 + i, g)] = r.y;
+        }
+        if (lane < WROW - 128) { row[w_hi<G>(128 + lane, g)] = 0u; row[w_lo<G>(128 + lane, g)] = 0u; }
+        if (lane == 0) { step[sub * G + g] = st; zp[sub * G + g] = z; }
+    }
+}
+
+// The same in the rows form: qh holds the query heads' fp16 bits [G][128]; lane = 4 consecutive channels = one word.
+template <int G>
+__device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *zp, const uint16_t *qh, float scaling,
+                                               const KUnit &u, bool channel_units, int min_bytes, bool live, int tid) {
+    const int lane = tid & 31, wp = tid >> 5, sub = wp & 3;
+    float sc[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) sc[i] = kvc_scale_value(ku_scale(u, i));
+#pragma unroll
+    for (int gi = 0; gi < G / 2; gi++) {
+        const int g = (wp >> 2) * (G / 2) + gi;
+        const uint2 qb = *reinterpret_cast<const uint2 *>(qh + g * 128 + lane * 4);
+        const uint32_t q2[2] = {live ? qb.x : 0u, live ? qb.y : 0u};
+        float wv[4], z = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float q = kvc_scale_value((unsigned short)(q2[i >> 1] >> (16 * (i & 1)))) * scaling;
+            wv[i] = q * sc[i];
+            z = fmaf((float)ku_min(u, i, min_bytes) * sc[i], q, z);
+        }
+        const float mx = kvc_warp_max(fmaxf(fmaxf(fabsf(wv[0]), fabsf(wv[1])), fmaxf(fabsf(wv[2]), fabsf(wv[3]))));
+        z = channel_units ? kvc_warp_sum(z) : 0.f;
+        const float st = fix_step(mx), inv = st > 0.f ? 1.0f / st : 0.f;
+        const uint2 r = pack4_dense(__float2int_rn(wv[0] * inv), __float2int_rn(wv[1] * inv), __float2int_rn(wv[2] * inv), __float2int_rn(wv[3] * inv));
+        uint32_t *vec = w + sub * VecWords<G, true>::value;
+        vec[w_rows(g, lane)] = r.x; vec[G * 32 + w_rows(g, lane)] = r.y;
         if (lane == 0) { step[sub * G + g] = st; zp[sub * G + g] = z; }
     }
 }
@@ -370,37 +409,15 @@ __device__ __forceinline__ void k_finish(float (&s)[G], const int (&hi)[G], cons
 // ---- V weights --------------------------------------------------------------------------------------
 // Called by all 256 threads (thread = token of the tile, grp = its 128-token group, tl = its index in
 // the group) with wv[g] = p[g] * scale of the token.  Builds records ps[grp][tl][hi|lo][g], step[grp][g].
-// `red` is scratch for 8*G floats, `q16` for 2*G*(128+4) int16 (unused with ROWS).  Contains three block
-// barriers (two with ROWS).
-template <int G, bool ROWS = false>
+// `red` is scratch for 8*G floats, `q16` for 2*G*(128+4) int16.  Contains three block barriers.
+template <int G>
 __device__ __forceinline__ void v_weights(uint32_t *ps, float *vstep, float *red, int16_t *q16, const float (&wv)[G],
                                           int tid) {
     const int lane = tid & 31, warp = tid >> 5, grp = tid >> 7, tl = tid & 127;
 #pragma unroll
     for (int g = 0; g < G; g++) { float mx = kvc_warp_max(fabsf(wv[g])); if (lane == 0) red[warp * G + g] = mx; }
-    if (!ROWS && tl < 4) for (int g = 0; g < G; g++) q16[(grp * G + g) * 132 + 128 + tl] = 0;
+    if (tl < 4) for (int g = 0; g < G; g++) q16[(grp * G + g) * 132 + 128 + tl] = 0;
     __syncthreads();
-    if (ROWS) {
-        // four consecutive tokens make one weight word per head: their 16-bit values reach the first of
-        // the four lanes by shuffles, no scratch and no barrier in between
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            const float mx = fmaxf(fmaxf(red[(grp * 4 + 0) * G + g], red[(grp * 4 + 1) * G + g]),
-                                   fmaxf(red[(grp * 4 + 2) * G + g], red[(grp * 4 + 3) * G + g]));
-            const float st = fix_step(mx);
-            const int q0 = fix_quant(wv[g], st);
-            const int q1 = __shfl_down_sync(0xffffffffu, q0, 1), q2 = __shfl_down_sync(0xffffffffu, q0, 2),
-                      q3 = __shfl_down_sync(0xffffffffu, q0, 3);
-            if (tl == 0) vstep[grp * G + g] = st;
-            if ((tl & 3) == 0) {                               // [group of 4 tokens][hi | lo][g]
-                uint32_t *row = ps + (size_t)grp * VecWords<G, ROWS>::value;
-                const uint2 r = pack4_dense(q0, q1, q2, q3);
-                row[((tl >> 2) * 2 + 0) * G + g] = r.x; row[((tl >> 2) * 2 + 1) * G + g] = r.y;
-            }
-        }
-        __syncthreads();
-        return;
-    }
 #pragma unroll
     for (int g = 0; g < G; g++) {
         const float mx = fmaxf(fmaxf(red[(grp * 4 + 0) * G + g], red[(grp * 4 + 1) * G + g]),
@@ -413,7 +430,7 @@ __device__ __forceinline__ void v_weights(uint32_t *ps, float *vstep, float *red
 #pragma unroll
     for (int g = 0; g < G; g++) {
         const int16_t *qq = q16 + (grp * G + g) * 132 + tl;
-        uint32_t *row = ps + (size_t)grp * VecWords<G, ROWS>::value;    // layout: w_hi / w_lo
+        uint32_t *row = ps + (size_t)grp * VecWords<G, false>::value;    // layout: w_hi / w_lo
         const uint2 r = pack4(qq[0], qq[1], qq[2], qq[3]);
         row[w_hi<G>(tl, g)] = r.x; row[w_lo<G>(tl, g)] = r.y;
         if (tl < WROW - 128) { row[w_hi<G>(128 + tl, g)] = 0u; row[w_lo<G>(128 + tl, g)] = 0u; }
@@ -542,13 +559,14 @@ __global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T
 template <int G>
 struct alignas(32) AttnSmem {                     // followed in shared memory by 4 K slots, 4 V slots (sized at launch),
     KvcBookSmem bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
-    alignas(32) uint32_t w[4 * VecWords<G, (G >= 2)>::value];     // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum
-    alignas(32) uint32_t ps[2 * VecWords<G, (G >= 2)>::value];    // V weight words
+    // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum, in the rows form by the V weight words
+    alignas(32) uint32_t w[4 * VecWords<G, (G >= 2)>::value];
+    alignas(32) uint32_t ps[G >= 2 ? 8 : 2 * VecWords<G, false>::value];    // V weight words (one-pass form)
+    alignas(16) float red[4][8 * G];  // per-warp max, sum, zpv and weight-max partials
+    alignas(16) float q[G >= 2 ? G * 64 : 128];   // the query: scaled values, in the rows form fp16 bits [G][128]
     float kstep[4 * G], zp[4 * G];
-    float vstep[2 * G];
-    float qf[G * 128];
+    float vstep[2];
     float qsum[G];
-    float red[4][8 * G];              // per-warp max, sum, zpv and weight-max partials
     uint64_t bar[2];                  // K and V staging barriers
     uint32_t leadK[4], leadV[4];
     uint32_t nbK[4], nbV[4];          // byte counts of the staged blocks
@@ -560,6 +578,7 @@ struct alignas(32) AttnSmem {                     // followed in shared memory b
 struct AttnParams {
     CacheDev k, v;
     long long T, B, Hkv, Hq, g0, Tr;
+    int nh;                       // query heads of this launch (per KV head, from g0): 1 .. G
     const __half *q, *ktail, *vtail;
     __half *out;
     float scaling;
@@ -579,14 +598,18 @@ struct AttnParams {
 
 // BULK: stage with bulk asynchronous copies (one tile phase ahead) instead of plain loads.
 template <int G, bool BULK>
-__global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnParams p) {
+__global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnSmem<G> &sm = *reinterpret_cast<AttnSmem<G> *>(smem_raw);
     uint8_t *const slotsK = smem_raw + sizeof(AttnSmem<G>), *const slotsV = slotsK + 4 * p.slotK_bytes;
     constexpr bool ROWS = G >= 2;                          // grouped queries: decode into rows, multiply afterwards
-    uint32_t *const myrow = reinterpret_cast<uint32_t *>(slotsV + 4 * p.slotV_bytes + SLOT_PAD) + threadIdx.x * (ROW_STRIDE / 4);
+    // rows form: the rows lie behind the slots and are their padding too
+    const uint32_t rows_s = kvc_smem_addr(slotsV + 4 * p.slotV_bytes), warp_rows_s = rows_s + (threadIdx.x & ~31u) * (ROW_WORDS * 4);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
     const int grp = tid >> 7, ch = tid & 127;
+    // rows form: the lane's two heads and its four neighbouring rows (tokens in the K phase, channels in the V phase)
+    const int h2 = (2 * (lane & 3)) % G, r4 = lane & ~3;
+    const bool own = 2 * (lane & 3) < G;                   // with fewer than 8 heads the other lanes hold copies
     // Launched with programmatic stream serialisation.  This kernel's own set-up -- the books' tables, the first
     // blocks, the first tile's metadata: cache data that no kernel of a decode step writes -- runs before
     // griddepcontrol.wait, i.e. possibly while the kernel ahead of it in the stream (the merge of the layer
@@ -683,14 +706,17 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
         for (int i = 0; i < QN; i++) {
             const int idx = tid + i * NTHR;
             qn[i] = 0;
-            if (idx < G * 128) qn[i] = reinterpret_cast<const unsigned short *>(p.q)[(row0 + (idx >> 7)) * 128 + (idx & 127)];
+            if (idx < (ROWS ? p.nh * 128 : 128)) qn[i] = reinterpret_cast<const unsigned short *>(p.q)[(row0 + (idx >> 7)) * 128 + (idx & 127)];
         }
     };
     auto q_store = [&]() {
 #pragma unroll
         for (int i = 0; i < QN; i++) {
             const int idx = tid + i * NTHR;
-            if (idx < G * 128) sm.qf[idx] = kvc_scale_value(qn[i]) * p.scaling;
+            if (idx < G * 128) {
+                if (ROWS) reinterpret_cast<unsigned short *>(sm.q)[idx] = qn[i];
+                else sm.q[idx] = kvc_scale_value(qn[i]) * p.scaling;
+            }
         }
     };
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -703,11 +729,26 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
     if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
     q_store();                                             // fetched during the previous item's last tile
     __syncthreads();
-    q_sums<G>(sm.qf, sm.qsum, tid);
-    __syncthreads();                                       // books, q and (unbuffered) slots are in place
-    float m_run[G], l_run[G], acc[G];
+    if constexpr (ROWS) {                                  // sum of each query head's 128 (scaled) values
+        const unsigned short *qh = reinterpret_cast<const unsigned short *>(sm.q);
+        if (warp < G) {
+            float a = 0.f;
 #pragma unroll
-    for (int g = 0; g < G; g++) { m_run[g] = -CUDART_INF_F; l_run[g] = 0.f; acc[g] = 0.f; }
+            for (int k = 0; k < 4; k++) a += kvc_scale_value(qh[warp * 128 + k * 32 + lane]) * p.scaling;
+            a = kvc_warp_sum(a);
+            if (lane == 0) sm.qsum[warp] = a;
+        }
+    } else q_sums<1>(sm.q, sm.qsum, tid);
+    __syncthreads();                                       // books, q and (unbuffered) slots are in place
+    // running maximum, sum and output: of the one head and the thread's channel, or of the lane's two heads and four channels
+    constexpr int NH = ROWS ? 2 : 1, NC = ROWS ? 4 : 1;
+    float m_run[NH], l_run[NH], acc[NC][NH];
+#pragma unroll
+    for (int j = 0; j < NH; j++) {
+        m_run[j] = -CUDART_INF_F; l_run[j] = 0.f;
+#pragma unroll
+        for (int i = 0; i < NC; i++) acc[i][j] = 0.f;
+    }
 
     for (int tile = it.t_lo; tile < it.t_hi; tile++) {
         const long long tok0 = (long long)tile * 256, t = tok0 + tid;
@@ -725,7 +766,8 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
             if (actK) { uint32_t ld, nb; bool ok = stage(p.k, blkK, slotsK + sub * p.slotK_bytes, &ld, &nb, v); if (v == 0) { sm.leadK[sub] = ld; sm.nbK[sub] = nb; sm.okK[sub] = ok; } }
             if (actV) { uint32_t ld, nb; bool ok = stage(p.v, blkV, slotsV + sub * p.slotV_bytes, &ld, &nb, v); if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; } }
         }
-        k_weights_build<G, ROWS>(sm.w, sm.kstep, sm.zp, sm.qf, cur.ku, km.sc != 0, km.min_bytes, tok0, T, tid);
+        if constexpr (ROWS) k_weights_rows<G>(sm.w, sm.kstep, sm.zp, reinterpret_cast<const uint16_t *>(sm.q), p.scaling, cur.ku, km.sc != 0, km.min_bytes, tok0 + (warp & 3) * 64 < T, tid);
+        else k_weights_build<1>(sm.w, sm.kstep, sm.zp, sm.q, cur.ku, km.sc != 0, km.min_bytes, tok0, T, tid);
         // A wait that runs out: the thread does not decode.  The warp that issues the copies looks at its own
         // verdict: a barrier whose phase it did not see complete is never armed again (a second arrival on an
         // open phase is an error), and the CTA is marked; it takes no further item, and what it had in flight
@@ -737,26 +779,61 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
         }
         __syncthreads();
         // ---- K: scores of this tile's tokens
-        float s[G];
-        if (actK) {
-            int hi[G], lo[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
+        float s[NC][NH];
+        if (actK) {                                        // the same for a whole warp
             bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
-            if (ok) {
-                if constexpr (ROWS) ok = decode_rows<G>(slotsK + sub * p.slotK_bytes, sm.leadK[sub] + (cur.startK >> 3), sm.bookK, escK, myrow, sm.w + sub * VecWords<G, true>::value, hi, lo);
-                else ok = decode_dot<G>(slotsK + sub * p.slotK_bytes, sm.leadK[sub] + (cur.startK >> 3), sm.bookK, escK, sm.w + sub * VecWords<G, false>::value, hi, lo);
+            const uint32_t posK = sm.leadK[sub] + (cur.startK >> 3);
+            if constexpr (ROWS) {
+                if (ok) ok = decode_row(kvc_smem_addr(slotsK + sub * p.slotK_bytes), posK, kvc_smem_addr(sm.bookK.lut), kvc_smem_addr(sm.bookK.tree), escK, rows_s + tid * (ROW_WORDS * 4));
+                __syncwarp();
+                int d[4][2];
+                rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + sub * VecWords<G, true>::value), lane, d);
+                const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the thread's own token
+                const float2 st = *reinterpret_cast<const float2 *>(&sm.kstep[sub * G + h2]), z = *reinterpret_cast<const float2 *>(&sm.zp[sub * G + h2]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    s[i][0] = st.x * (float)d[i][0]; s[i][NH - 1] = st.y * (float)d[i][1];
+                    if (km.sc != 0) { s[i][0] += z.x; s[i][NH - 1] += z.y; }
+                    else {
+                        const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
+                        const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
+                        s[i][0] = sc * fmaf(mi, sm.qsum[h2], s[i][0]); s[i][NH - 1] = sc * fmaf(mi, sm.qsum[h2 + NH - 1], s[i][NH - 1]);
+                    }
+                }
+            } else {
+                int hi[1] = {0}, lo[1] = {0};
+                if (ok) ok = decode_dot<1>(slotsK + sub * p.slotK_bytes, posK, sm.bookK, escK, sm.w + sub * VecWords<1, false>::value, hi, lo);
+                k_finish<1>(s[0], hi, lo, sm.kstep + sub, sm.zp + sub, sm.qsum, km.sc != 0, kvc_scale_value(cur.ksc), (float)cur.kmi);
             }
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
-            k_finish<G>(s, hi, lo, sm.kstep + sub * G, sm.zp + sub * G, sm.qsum, km.sc != 0, kvc_scale_value(cur.ksc), (float)cur.kmi);
         } else {
 #pragma unroll
-            for (int g = 0; g < G; g++) s[g] = -CUDART_INF_F;
+            for (int i = 0; i < NC; i++)
+#pragma unroll
+                for (int j = 0; j < NH; j++) s[i][j] = -CUDART_INF_F;
         }
         // ---- online softmax over the tile
+        // over a warp's tokens: in the rows form the lane's four, then the eight lanes with the same heads
+        auto warp_max = [&](float x) { if constexpr (ROWS) { x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4)); x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8)); return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16)); } else return kvc_warp_max(x); };
+        auto warp_sum = [&](float x) { if constexpr (ROWS) { x += __shfl_xor_sync(0xffffffffu, x, 4); x += __shfl_xor_sync(0xffffffffu, x, 8); return x + __shfl_xor_sync(0xffffffffu, x, 16); } else return kvc_warp_sum(x); };
+        auto red_put = [&](int k, const float (&x)[NH]) {      // the warp's value of each head
+            if constexpr (ROWS) { if (lane < G / 2) *reinterpret_cast<float2 *>(&sm.red[k][warp * G + h2]) = make_float2(x[0], x[NH - 1]); }
+            else if (lane == 0) sm.red[k][warp] = x[0];
+        };
+        auto red_get = [&](int k, int w8, float (&x)[NH]) {
+            if constexpr (ROWS) { const float2 v2 = *reinterpret_cast<const float2 *>(&sm.red[k][w8 * G + h2]); x[0] = v2.x; x[NH - 1] = v2.y; }
+            else x[0] = sm.red[k][w8];
+        };
+        float t1[NH], t2[NH];
 #pragma unroll
-        for (int g = 0; g < G; g++) { float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
-        __syncthreads();                                   // also: every thread is done with the K slots
+        for (int j = 0; j < NH; j++) {
+            t1[j] = s[0][j];
+#pragma unroll
+            for (int i = 1; i < NC; i++) t1[j] = fmaxf(t1[j], s[i][j]);
+            t1[j] = warp_max(t1[j]);
+        }
+        red_put(0, t1);
+        __syncthreads();                                   // also: every thread is done with the K slots and weights
         // the next tile's per-thread metadata is asked for now and first touched when that tile begins: it is in
         // flight during the V phase only, and the K decode above ran without its registers
         load_meta(n_on, n_col, n_tile, nxt);
@@ -765,54 +842,115 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
                 stage_bulk(p.k, validK(n_on, n_tile, lane & 3), blkK_of(n_col, n_tile, lane & 3), slotsK + (lane & 3) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0);
             else if (lane == 0) sm.dead = 1;
         }
-        float alpha[G], wv[G];
+        float alpha[NH], vst[NH];
+        red_get(0, 0, t1);
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            float mt = sm.red[0][g];
+        for (int w8 = 1; w8 < 8; w8++) {
+            red_get(0, w8, t2);
 #pragma unroll
-            for (int w8 = 1; w8 < 8; w8++) mt = fmaxf(mt, sm.red[0][w8 * G + g]);
-            const float m_new = fmaxf(m_run[g], mt);
-            alpha[g] = __expf(m_run[g] - m_new);           // exp(-inf) = 0 on the first tile
-            const float pr = actK ? __expf(s[g] - m_new) : 0.f;
-            m_run[g] = m_new;
-            wv[g] = pr * kvc_scale_value(cur.vsc);
-            const float ssum = kvc_warp_sum(pr), zsum = kvc_warp_sum(wv[g] * (float)cur.vmi);
-            if (lane == 0) { sm.red[1][warp * G + g] = ssum; sm.red[2][warp * G + g] = zsum; }
+            for (int j = 0; j < NH; j++) t1[j] = fmaxf(t1[j], t2[j]);
         }
-        // (the K weights are spent: their memory is the scratch of the V weights' 16-bit values)
-        v_weights<G, ROWS>(sm.ps, sm.vstep, sm.red[3], reinterpret_cast<int16_t *>(sm.w), wv, tid);      // three barriers inside
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            float lt = 0.f;
-#pragma unroll
-            for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + g];
-            l_run[g] = l_run[g] * alpha[g] + lt;
+        for (int j = 0; j < NH; j++) {
+            const float m_new = fmaxf(m_run[j], t1[j]);
+            alpha[j] = __expf(m_run[j] - m_new);           // exp(-inf) = 0 on the first tile
+            m_run[j] = m_new;
         }
+        if constexpr (ROWS) {
+            float wv[4][2], ssum[2] = {0.f, 0.f}, zsum[2] = {0.f, 0.f}, wmax[2] = {0.f, 0.f};
+            const uint32_t unit = (uint32_t)cur.vsc | ((uint32_t)cur.vmi << 16);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
+                const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const float pr = actK ? __expf(s[i][j] - m_run[j]) : 0.f;
+                    wv[i][j] = pr * sc;
+                    ssum[j] += pr; zsum[j] = fmaf(wv[i][j], mi, zsum[j]); wmax[j] = fmaxf(wmax[j], fabsf(wv[i][j]));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) { ssum[j] = warp_sum(ssum[j]); zsum[j] = warp_sum(zsum[j]); wmax[j] = warp_max(wmax[j]); }
+            red_put(1, ssum); red_put(2, zsum); red_put(3, wmax);
+            __syncthreads();
+            // the V weights' words: the lane's four tokens are one word of each of its heads
+            red_get(3, grp * 4, t1);
+#pragma unroll
+            for (int w4 = 1; w4 < 4; w4++) {
+                red_get(3, grp * 4 + w4, t2);
+                t1[0] = fmaxf(t1[0], t2[0]); t1[1] = fmaxf(t1[1], t2[1]);
+            }
+            uint32_t *vec = sm.w + grp * VecWords<G, true>::value;         // the K weights are spent
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                vst[j] = fix_step(t1[j]);
+                const float inv = vst[j] > 0.f ? 1.0f / vst[j] : 0.f;
+                const uint2 w2 = pack4_dense(__float2int_rn(wv[0][j] * inv), __float2int_rn(wv[1][j] * inv), __float2int_rn(wv[2][j] * inv), __float2int_rn(wv[3][j] * inv));
+                const uint32_t at = w_rows(h2 + j, (warp & 3) * 8 + (lane >> 2));
+                if (own) { vec[at] = w2.x; vec[G * 32 + at] = w2.y; }
+            }
+            __syncthreads();
+        } else {
+            float wv[1];
+            const float pr = actK ? __expf(s[0][0] - m_run[0]) : 0.f;
+            wv[0] = pr * kvc_scale_value(cur.vsc);
+            const float ssum = kvc_warp_sum(pr), zsum = kvc_warp_sum(wv[0] * (float)cur.vmi);
+            if (lane == 0) { sm.red[1][warp] = ssum; sm.red[2][warp] = zsum; }
+            // (the K weights are spent: their memory is the scratch of the V weights' 16-bit values)
+            v_weights<1>(sm.ps, sm.vstep, sm.red[3], reinterpret_cast<int16_t *>(sm.w), wv, tid);      // three barriers inside
+        }
+        red_get(1, 0, t1);
+#pragma unroll
+        for (int w8 = 1; w8 < 8; w8++) {
+            red_get(1, w8, t2);
+#pragma unroll
+            for (int j = 0; j < NH; j++) t1[j] += t2[j];
+        }
+#pragma unroll
+        for (int j = 0; j < NH; j++) l_run[j] = l_run[j] * alpha[j] + t1[j];
         const bool v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
         if (BULK && v_landed) par ^= 2u;
         if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
-        // ---- V: accumulate this tile's contribution for the thread's (group, channel)
-        float dv[G];
+        // ---- V: accumulate this tile's contribution for the thread's (group, channels)
+        float dv[NC][NH];
 #pragma unroll
-        for (int g = 0; g < G; g++) dv[g] = 0.f;
-        if (actV) {
-            int hi[G], lo[G];
+        for (int i = 0; i < NC; i++)
 #pragma unroll
-            for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
+            for (int j = 0; j < NH; j++) dv[i][j] = 0.f;
+        if (actV) {                                        // the same for a whole warp
             bool ok = v_landed && sm.okV[sub] && (uint32_t)(cur.startV >> 3) < sm.nbV[sub];
-            if (ok) {
-                if constexpr (ROWS) ok = decode_rows<G>(slotsV + sub * p.slotV_bytes, sm.leadV[sub] + (cur.startV >> 3), sm.bookV, escV, myrow, sm.ps + grp * VecWords<G, true>::value, hi, lo);
-                else ok = decode_dot<G>(slotsV + sub * p.slotV_bytes, sm.leadV[sub] + (cur.startV >> 3), sm.bookV, escV, sm.ps + grp * VecWords<G, false>::value, hi, lo);
+            const uint32_t posV = sm.leadV[sub] + (cur.startV >> 3);
+            float z[NH];
+            auto zero_points = [&]() {                     // of the group's four warps
+#pragma unroll
+                for (int w4 = 0; w4 < 4; w4++) {
+                    float x[NH];
+                    red_get(2, grp * 4 + w4, x);
+#pragma unroll
+                    for (int j = 0; j < NH; j++) z[j] = w4 ? z[j] + x[j] : x[j];
+                }
+            };
+            if constexpr (ROWS) {
+                if (ok) ok = decode_row(kvc_smem_addr(slotsV + sub * p.slotV_bytes), posV, kvc_smem_addr(sm.bookV.lut), kvc_smem_addr(sm.bookV.tree), escV, rows_s + tid * (ROW_WORDS * 4));
+                __syncwarp();
+                int d[4][2];
+                rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + grp * VecWords<G, true>::value), lane, d);
+                zero_points();
+#pragma unroll
+                for (int i = 0; i < 4; i++) { dv[i][0] = fmaf(vst[0], (float)d[i][0], z[0]); dv[i][NH - 1] = fmaf(vst[NH - 1], (float)d[i][1], z[NH - 1]); }
+            } else {
+                int hi[1] = {0}, lo[1] = {0};
+                if (ok) ok = decode_dot<1>(slotsV + sub * p.slotV_bytes, posV, sm.bookV, escV, sm.ps + grp * VecWords<1, false>::value, hi, lo);
+                zero_points();
+                dv[0][0] = fix_value(sm.vstep[grp], hi[0], lo[0]) + z[0];
             }
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                dv[g] = fix_value(sm.vstep[grp * G + g], hi[g], lo[g]) +
-                        sm.red[2][(grp * 4 + 0) * G + g] + sm.red[2][(grp * 4 + 1) * G + g] +
-                        sm.red[2][(grp * 4 + 2) * G + g] + sm.red[2][(grp * 4 + 3) * G + g];
         }
 #pragma unroll
-        for (int g = 0; g < G; g++) acc[g] = fmaf(acc[g], alpha[g], dv[g]);
+        for (int i = 0; i < NC; i++)
+#pragma unroll
+            for (int j = 0; j < NH; j++) acc[i][j] = fmaf(acc[i][j], alpha[j], dv[i][j]);
         __syncthreads();                                   // every thread is done with the V slots, weights and sums
         if (BULK && warp == 0) {                           // next tile's V blocks land during its K phase
             if (__all_sync(0xffffffffu, v_landed))
@@ -835,6 +973,7 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
             for (int g = 0; g < G; g++) s[g] = act ? 0.f : -CUDART_INF_F;
             if (act) {
                 const __half *kr = p.ktail + ((r * B + b) * Hkv + h) * 128;
+#pragma unroll 1
                 for (int c8 = 0; c8 < 16; c8++) {
                     uint4 kv = *reinterpret_cast<const uint4 *>(kr + c8 * 8);
                     const __half *kh = reinterpret_cast<const __half *>(&kv);
@@ -842,47 +981,59 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
                     for (int k = 0; k < 8; k++) {
                         const float kf = __half2float(kh[k]);
 #pragma unroll
-                        for (int g = 0; g < G; g++) s[g] = fmaf(kf, sm.qf[g * 128 + c8 * 8 + k], s[g]);
+                        for (int g = 0; g < G; g++) {
+                            const int at = g * 128 + c8 * 8 + k;
+                            const float qv = ROWS ? kvc_scale_value(reinterpret_cast<const unsigned short *>(sm.q)[at]) * p.scaling : sm.q[at];
+                            s[g] = fmaf(kf, qv, s[g]);
+                        }
                     }
                 }
             }
 #pragma unroll
-            for (int g = 0; g < G; g++) { float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
+            for (int g = 0; g < G; g++) { const float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
             __syncthreads();
-            float alpha[G];
+            float alpha[NH], dv[NC][NH];
 #pragma unroll
-            for (int g = 0; g < G; g++) {
+            for (int j = 0; j < NH; j++) {
+                const int g = ROWS ? h2 + j : 0;
                 float mt = sm.red[0][g];
 #pragma unroll
                 for (int w8 = 1; w8 < 8; w8++) mt = fmaxf(mt, sm.red[0][w8 * G + g]);
-                const float m_new = fmaxf(m_run[g], mt);
-                alpha[g] = __expf(m_run[g] - m_new);
-                const float pr = act ? __expf(s[g] - m_new) : 0.f;
-                m_run[g] = m_new;
+                const float m_new = fmaxf(m_run[j], mt);
+                alpha[j] = __expf(m_run[j] - m_new);
+                m_run[j] = m_new;
+                if (ROWS && tid < 4) sm.red[3][g] = m_new;
+#pragma unroll
+                for (int i = 0; i < NC; i++) dv[i][j] = 0.f;
+            }
+            if (ROWS) __syncthreads();
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const float pr = act ? __expf(s[g] - (ROWS ? sm.red[3][g] : m_run[0])) : 0.f;
                 pt[tid * G + g] = pr;
                 const float ssum = kvc_warp_sum(pr);
                 if (lane == 0) sm.red[1][warp * G + g] = ssum;
             }
             __syncthreads();
-            float dv[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                float lt = 0.f;
-#pragma unroll
-                for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + g];
-                l_run[g] = l_run[g] * alpha[g] + lt;
-                dv[g] = 0.f;
-            }
-            // thread (grp, ch) sums rows r0 + 128*grp .. +127 of its channel
+            // the thread's channel, or the lane's four, over rows r0 + 128*grp .. +127
             for (int i = 0; i < 128; i++) {
                 const long long rr = r0 + grp * 128 + i;
                 if (rr >= p.Tr) break;
-                const float vf = __half2float(p.vtail[((rr * B + b) * Hkv + h) * 128 + ch]);
+                const __half *vr = p.vtail + ((rr * B + b) * Hkv + h) * 128 + (ROWS ? (warp & 3) * 32 + r4 : ch);
 #pragma unroll
-                for (int g = 0; g < G; g++) dv[g] = fmaf(pt[(grp * 128 + i) * G + g], vf, dv[g]);
+                for (int c = 0; c < NC; c++)
+#pragma unroll
+                    for (int j = 0; j < NH; j++) dv[c][j] = fmaf(pt[(grp * 128 + i) * G + (ROWS ? h2 + j : 0)], __half2float(vr[c]), dv[c][j]);
             }
 #pragma unroll
-            for (int g = 0; g < G; g++) acc[g] = fmaf(acc[g], alpha[g], dv[g]);
+            for (int j = 0; j < NH; j++) {
+                float lt = 0.f;
+#pragma unroll
+                for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + (ROWS ? h2 + j : 0)];
+                l_run[j] = l_run[j] * alpha[j] + lt;
+#pragma unroll
+                for (int c = 0; c < NC; c++) acc[c][j] = fmaf(acc[c][j], alpha[j], dv[c][j]);
+            }
         }
     }
     if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without tiles fetched nothing yet
@@ -890,23 +1041,38 @@ __global__ void __launch_bounds__(NTHR, G == 4 ? 2 : 3) attn_decode_kernel(AttnP
     if (!p.partial) {
         // ---- the item is the whole column: combine the CTA's two token groups and write the output
         __syncthreads();
-        float *sumbuf = reinterpret_cast<float *>(sm.w);       // [2][128][G]
+        float *sumbuf = reinterpret_cast<float *>(sm.w);       // [128][G]
+        const int c0 = ROWS ? (warp & 3) * 32 + r4 : ch;       // the first of the thread's channels
+        if (grp == 1 && (own || !ROWS)) {
 #pragma unroll
-        for (int g = 0; g < G; g++) sumbuf[(grp * 128 + ch) * G + g] = acc[g];
-        __syncthreads();
-        if (tid < 128) {
+            for (int i = 0; i < NC; i++)
 #pragma unroll
-            for (int g = 0; g < G; g++)
-                p.out[(head0 + g) * 128 + tid] = __float2half_rn((sumbuf[tid * G + g] + sumbuf[(128 + tid) * G + g]) / l_run[g]);
+                for (int j = 0; j < NH; j++) sumbuf[(c0 + i) * G + (ROWS ? h2 + j : 0)] = acc[i][j];
         }
-    } else {
+        __syncthreads();
+        if (grp == 0 && (own || !ROWS)) {
+#pragma unroll
+            for (int j = 0; j < NH; j++) {
+                const int g = ROWS ? h2 + j : 0;
+                if (g >= p.nh) continue;
+#pragma unroll
+                for (int i = 0; i < NC; i++)
+                    p.out[(head0 + g) * 128 + c0 + i] = __float2half_rn((acc[i][j] + sumbuf[(c0 + i) * G + g]) / l_run[j]);
+            }
+        }
+    } else if constexpr (ROWS) {
         // ---- a partial result {m, l, -, -, acc of group 0 [128], acc of group 1 [128]}; a second kernel merges
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            float *dst = p.ws_part + ((head0 + g) * p.splits + it.part) * ATTN_PART_FLOATS;
-            dst[4 + tid] = acc[g];                             // tid = grp * 128 + ch
-            if (tid == 0) { dst[0] = m_run[g]; dst[1] = l_run[g]; }
+        for (int j = 0; j < 2; j++) {
+            if (!own || h2 + j >= p.nh) continue;
+            float *dst = p.ws_part + ((head0 + h2 + j) * p.splits + it.part) * ATTN_PART_FLOATS;
+            *reinterpret_cast<float4 *>(dst + 4 + grp * 128 + (warp & 3) * 32 + r4) = make_float4(acc[0][j], acc[1 % NC][j], acc[2 % NC][j], acc[3 % NC][j]);
+            if (warp == 0 && lane < 4) { dst[0] = m_run[j]; dst[1] = l_run[j]; }
         }
+    } else {
+        float *dst = p.ws_part + (head0 * p.splits + it.part) * ATTN_PART_FLOATS;
+        dst[4 + tid] = acc[0][0];                              // tid = grp * 128 + ch
+        if (tid == 0) { dst[0] = m_run[0]; dst[1] = l_run[0]; }
     }
     if (draw && tid == 0) sm.next_j = drawn;
     __syncthreads();                                       // the sums are read before the next column's weights overwrite them
@@ -1133,7 +1299,7 @@ int check_cache(const kvc_cache *c, const char *who, bool is_k) {
     return KVC_OK;
 }
 
-// the G query heads of a KV head are processed in chunks of 4, 2 or 1
+// the query heads of a KV head are processed in chunks of 4, 2 or 1 by the two unfused kernels
 int next_chunk(long long remaining) { return remaining >= 4 ? 4 : (remaining >= 2 ? 2 : 1); }
 
 }  // namespace
@@ -1194,6 +1360,8 @@ extern "C" int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hk
 static int g_wait_limit = 0, g_starve = 0;
 extern "C" void kvc_attn_debug(int wait_limit, int starve) { g_wait_limit = wait_limit; g_starve = starve; }
 
+// shared memory of an SM (each resident CTA takes 1 KB more than it asks for)
+constexpr size_t SM_SHARED_BYTES = 228 * 1024;
 // CTAs per SM the attention kernel is launched with at most (its launch bounds ask for this many)
 constexpr int ATTN_CTAS_PER_SM = 3;
 // items a resident CTA should get on average: enough that the draws even out the CTAs' speeds and the
@@ -1303,16 +1471,21 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.slotK_bytes = ((p.k.max_block + 15u + 15u) & ~15u) + 16u;
     p.slotV_bytes = ((p.v.max_block + 15u + 15u) & ~15u) + 16u;
     const size_t slot_total = 4 * (size_t)(p.slotK_bytes + p.slotV_bytes) + SLOT_PAD;
+    auto rows_smem = [&](size_t fixed) { return fixed + 4 * (size_t)(p.slotK_bytes + p.slotV_bytes) + NTHR * ROW_WORDS * 4; };
     // bulk copies widen every block to 16-byte boundaries: both streams must start on one
     const bool bulk = T > 0 && (reinterpret_cast<uintptr_t>(k->encoded) & 15) == 0 && (reinterpret_cast<uintptr_t>(v->encoded) & 15) == 0;
     const int sms = kvc_sm_count();
     const long long Gt = Hq / Hkv;
     for (long long g0 = 0; g0 < Gt && !(T == 0 && tail_in_merge);) {       // nothing compressed: the merge kernel alone
-        const int G = next_chunk(Gt - g0);
-        p.g0 = g0;
+        // Heads per launch: every launch decodes the whole cache, so up to 8 go together where two such CTAs fit an SM;
+        // with one CTA an SM idles at every barrier, and then up to 4 go together.  The launches get equal shares.
+        const long long most = 2 * (rows_smem(sizeof(AttnSmem<8>)) + 1024) <= SM_SHARED_BYTES ? 8 : 4;
+        const long long launches = (Gt - g0 + most - 1) / most;
+        const int nh = (int)((Gt - g0 + launches - 1) / launches), G = nh > 4 ? 8 : (nh > 2 ? 4 : nh);
+        p.g0 = g0; p.nh = nh;
 #define KVC_AT(GG, BB)                                                                                          \
     {                                                                                                           \
-        const size_t smem = slot_total + sizeof(AttnSmem<GG>) + ((GG) >= 2 ? NTHR * ROW_STRIDE : 0);               \
+        const size_t smem = (GG) >= 2 ? rows_smem(sizeof(AttnSmem<GG>)) : slot_total + sizeof(AttnSmem<GG>);     \
         if (int rc = set_smem(attn_decode_kernel<GG, BB>, smem)) return rc;                                     \
         int occ = 0;                                                                                            \
         KVC_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, attn_decode_kernel<GG, BB>, NTHR, smem)); \
@@ -1321,10 +1494,10 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         if (ctas > p.work) ctas = p.work;                                                                       \
         if (int rc = launch_overlapped(attn_decode_kernel<GG, BB>, dim3((unsigned)ctas), dim3(NTHR), smem, kvc_cu(stream), p)) return rc; \
     }
-        if (bulk) { if (G == 4) KVC_AT(4, true) else if (G == 2) KVC_AT(2, true) else KVC_AT(1, true) }
-        else { if (G == 4) KVC_AT(4, false) else if (G == 2) KVC_AT(2, false) else KVC_AT(1, false) }
+        if (bulk) { if (G == 8) KVC_AT(8, true) else if (G == 4) KVC_AT(4, true) else if (G == 2) KVC_AT(2, true) else KVC_AT(1, true) }
+        else { if (G == 8) KVC_AT(8, false) else if (G == 4) KVC_AT(4, false) else if (G == 2) KVC_AT(2, false) else KVC_AT(1, false) }
 #undef KVC_AT
-        g0 += G;
+        g0 += nh;
     }
     if (p.partial || tail_in_merge) {
         TailArgs ta = {};

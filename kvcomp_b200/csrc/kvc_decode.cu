@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) decode_kernel(
             unsigned long long buf = 0;
             uint32_t fill = 0;                               // bytes held in buf, < 4 between lookups
             uint32_t *wrow = reinterpret_cast<uint32_t *>(trow);
-            auto put = [&](uint32_t e, uint32_t) {
+            auto put = [&](uint32_t e, uint32_t, uint32_t, uint32_t) {
                 buf |= (unsigned long long)(e >> 8) << (fill * 8);
                 fill += (e >> 6) & 3u;
                 if (fill >= 4u) { *wrow++ = (uint32_t)buf; buf >>= 32; fill -= 4u; }

@@ -114,10 +114,11 @@ __device__ __forceinline__ bool kvc_book_needs_escape(const void *book) {
 // where the vector starts in it; lut_s / tree_s: shared-space addresses of the book's tables.
 // The decoder state is (position << 6) | bit offset into the (hi, lo) register pair, so applying a
 // table entry is one add of its low byte.
-// emit(e, a): `e` holds up to three symbols in bytes 1..3 for positions c..c+2 of the vector (unused
+// emit(e, a, s0, s1): `e` holds up to three symbols in bytes 1..3 for positions c..c+2 of the vector (unused
 // bytes are 0; byte 0 is the table entry's advance byte: its bits 6-7 count the symbols); a = (base + c) << SHIFT:
 // the position counter starts at `base`, so a consumer that keeps one record of 2^SHIFT bytes per
-// position at shared address A passes base = A >> SHIFT and gets the record's address with no add.
+// position at shared address A passes base = A >> SHIFT and gets the record's address with no add;
+// s0, s1: the state before and after the lookup (position from bit 6 up), for consumers that track word borders.
 // The end of the vector is tested once per KVC_DECODE_UNROLL lookups, so emit may be handed symbols for
 // positions up to 127 + KVC_DECODE_OVERRUN; the consumer keeps room for them (zero weights, padding).
 // ESC = false is for books whose longest code fits the table window: no escape test in the loop;
@@ -144,13 +145,15 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
         do {
             const uint32_t w0 = __funnelshift_l(lo, hi, state);
             const uint32_t e0 = kvc_lds32(lut_s + ((w0 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-            emit(e0, (state >> (6 - SHIFT)) & AMASK);
-            state = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);
+            const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);
+            emit(e0, (state >> (6 - SHIFT)) & AMASK, state, s1);
+            state = s1;
             const bool up = (state & 32u) != 0;
             const uint32_t w1 = __funnelshift_l(up ? nx : lo, up ? lo : hi, state);
             const uint32_t e1 = kvc_lds32(lut_s + ((w1 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-            emit(e1, (state >> (6 - SHIFT)) & AMASK);
-            state = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)state);
+            const uint32_t s2 = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)state);
+            emit(e1, (state >> (6 - SHIFT)) & AMASK, state, s2);
+            state = s2;
             if (state & 32u) { hi = lo; lo = nx; nx = kvc_bswap(kvc_lds32(ptr)); ptr += 4; state -= 32u; }
         } while (state < end);
         return true;
@@ -164,8 +167,9 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
         const uint32_t win = __funnelshift_l(lo, hi, state);          // the shift uses the low 5 bits
         const uint32_t e = kvc_lds32(lut_s + ((win >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
         if (!ESC || (e & 0xffu) != 0) {
-            emit(e, (state >> (6 - SHIFT)) & AMASK);
-            state = (uint32_t)kvc_dp4a_uu(e, 1u, (int)state);         // state += byte 0 of e, off the integer ALU pipe
+            const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e, 1u, (int)state);   // state + byte 0 of e, off the integer ALU pipe
+            emit(e, (state >> (6 - SHIFT)) & AMASK, state, s1);
+            state = s1;
         } else {                                                      // code longer than the window
             uint32_t node = e >> 8, sym = 0;
             bool found = false;
@@ -181,7 +185,7 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
                 node = (nd >> (16 * bit)) & 0xffffu;
             }
             ok = ok && found;
-            emit((sym << 8) | (1u << 6), a);                          // advance byte: one symbol
+            emit((sym << 8) | (1u << 6), a, state, state + (1u << 6));   // advance byte: one symbol
             state += 1u << 6;
         }
         if (state & 32u) { hi = lo; lo = kvc_bswap(nxt); nxt = kvc_lds32(ptr); ptr += 4; state -= 32u; }
@@ -189,3 +193,19 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
     } while (state < end);
     return ok;
 }
+
+// A consumer for kvc_decode_vector (SHIFT = 0, base = the shared address of the thread's row): the symbols collect in a
+// word that is stored when its last byte is known.  One predicated store per word; three byte stores per lookup cost as
+// many instructions and, with 32 lanes at 32 places of their rows, three times the bank conflicts.  (The two shifts
+// as one wide multiplication: 2.5 % slower in the attention kernel.)  Symbols past position 127 reach at most KVC_DECODE_OVERRUN_PAIR bytes beyond the row's 128.
+struct KvcRowWriter {
+    uint32_t cur = 0;
+    __device__ __forceinline__ void operator()(uint32_t e, uint32_t a, uint32_t s0, uint32_t s1) {
+        const uint32_t syms = e >> 8, sh = a << 3;             // the funnel shifts take the low five bits of the amount
+        const uint32_t w = cur | __funnelshift_l(0u, syms, sh), over = __funnelshift_l(syms, 0u, sh);
+        const uint32_t left = (s0 ^ s1) & (4u << 6);           // not 0: the position left its word
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.u32 [%1], %2;\n\t}"
+                     :: "r"(left), "r"(a & ~3u), "r"(w) : "memory");
+        cur = left ? over : w;
+    }
+};

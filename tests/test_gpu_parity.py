@@ -547,6 +547,26 @@ def test_attn_decode_llama7b_shape_small(ops):
     assert_attn_close(out, O)
 
 
+@pytest.mark.parametrize("G", [2, 3, 5, 6, 7, 8, 9, 16])
+@pytest.mark.parametrize("kmode,krel,T,Tr,tight", [(orc.MODE_CHANNEL, 0.05, 640, 0, True),     # half a tile at the end
+                                                   (orc.MODE_TOKEN, 0.05, 384, 131, True),    # one K unit per token, a tail of two passes
+                                                   (orc.MODE_BLOCK, 0.02, 256, 300, False)])  # slots for the largest block: four heads per launch at most
+def test_attn_decode_query_heads_per_kv_head(ops, G, kmode, krel, T, Tr, tight):
+    """Grouped queries go up to eight heads per launch through the tensor cores, padded to 2, 4 or 8 columns:
+    every number of heads, with the merge kernel and with the column's output and tail written directly."""
+    B, Hkv = 2, 2
+    k, v, q = synth(T + Tr, B, Hkv, seed=60 + G, Hq=Hkv * G)
+    rk, rv, kc, vc = _caches(ops, k[:T], v[:T], kmode, orc.MODE_TOKEN, krel, 0.1, 64, False, torch.int16, tight)
+    scaling = 1.0 / math.sqrt(128)
+    kt, vt = (dev(k[T:]), dev(v[T:])) if Tr else (None, None)
+    O = orc.attention(*_oracle_q(rk, T, B, Hkv, kmode, 64, False), *_oracle_q(rv, T, B, Hkv, orc.MODE_TOKEN, 128, False),
+                      q, scaling, k[T:] if Tr else None, v[T:] if Tr else None)
+    for kw in (dict(splits=0), dict(splits=1, workspace=False)):
+        out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, kt, vt, **kw)
+        assert ops.read_status(st) == 0
+        assert_attn_close(out, O, str(kw))
+
+
 def _skewed_cache(ops, rng, is_k, T, B, H):
     """Codes drawn from a very skewed alphabet (a code longer than the 12-bit decode window exists), with
     made-up units: K per 64-token block and sequence, V per token and sequence."""
