@@ -215,6 +215,11 @@ int kvc_decode(const uint8_t *encoded, int64_t encoded_bytes, const void *block_
 int kvc_decode_bounded(const uint8_t *encoded, int64_t encoded_bytes, const void *block_info,
                        const uint16_t *thread_info, const void *book, int64_t T, int64_t cols, int is_k,
                        uint32_t max_block_bytes, uint8_t *codes, int32_t *status, kvc_stream_t stream);
+/* kvc_decode_bounded and kvc_dequant in one launch: the stream of T tokens -> fp16 values [T,B,H,128], the same bits
+ * as the two calls give; the codes never reach memory.  Units that depend on the channel (K only) are contiguous
+ * over the channels and cover whole blocks of 64 tokens.  out: device, 16-byte aligned. */
+int kvc_decode_values(const kvc_cache *c, int64_t T, int64_t B, int64_t H, int is_k, void *out, int32_t *status,
+                      kvc_stream_t stream);
 
 /* k_decode_and_mat_vec_mul_cuda_export (kernels.cu:1093-1136): raw scores
  * S[b,hq,t] = sum_c x^K[t,b,hkv,c] * q[b,hq,c], fp32 accumulation.  q: device fp16

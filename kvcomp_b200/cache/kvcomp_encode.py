@@ -431,23 +431,39 @@ class KVCompCtx:
             out = self._pending if out is None else torch.cat([out, self._pending], dim=0)
         return out.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim), start.elapsed_time(stop)
 
-    def get_only_compressed(self):
-        """Dequantised compressed part [T, B, H, D] and the time of decode + dequantisation in ms."""
-        codes, t = self.get_decode_quant_ints()
+    def _values(self, rows):
+        """An fp16 tensor of `rows` tokens whose first compressed_ctx_len are the dequantised values, decoded and
+        dequantised by one kernel (plain codes that wait for their Huffman block: dequantised behind them), and its
+        time in ms."""
+        self._require()
+        n, shape = self.encoded_ctx_len, (self.batch_size, self.head_num, self.head_dim)
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
-        x = ops.dequant(codes.view(self.compressed_ctx_len, self.batch_size, self.head_num, self.head_dim),
-                        self._mi.used(), self._sc.used(), self.spec)
+        x = torch.empty((rows,) + shape, dtype=torch.float16, device=self.device)
+        st = ops.decode_values(self.cache(), n, *shape[:2], self.is_k, x[:n]) if n else None
+        if self._pending is not None:
+            first = n // self.spec.tok_div * self.spec.sj                    # unit of the first waiting token
+            ops.dequant(self._pending, self._mi.used()[first:], self._sc.used()[first:], self.spec, out=x[n:self.compressed_ctx_len])
         stop.record()
         stop.synchronize()
-        return x, t + start.elapsed_time(stop)
+        if st is not None:
+            ops.read_status(st, what="entropy_decode")
+        return x, start.elapsed_time(stop)
+
+    def get_only_compressed(self):
+        """Dequantised compressed part [T, B, H, D] and the time of decode + dequantisation in ms."""
+        return self._values(self.compressed_ctx_len)
 
     def get(self):
         """Whole cache [ctx_len, B, H, D]: dequantised compressed part followed by the recent window."""
         if self.compressed_ctx_len == 0:
             return self.buffer, 0.0
-        x, t = self.get_only_compressed()
-        return (torch.cat([x, self.buffer], dim=0) if self.buffer is not None and self.buffer.shape[0] else x), t
+        recent = self.buffer
+        live = 0 if recent is None else recent.shape[0]
+        x, t = self._values(self.compressed_ctx_len + live)
+        if live:
+            x[self.compressed_ctx_len:] = recent
+        return x, t
 
     def cache(self):
         """The kvc_cache argument of the fused kernels over the encoded_ctx_len tokens of the stream (valid

@@ -345,6 +345,19 @@ def decode(encoded, block_info, thread_info, book, T, B, H, is_k, out=None, stat
     return out, status
 
 
+def decode_values(cache, T, B, H, is_k, out, status=None):
+    """Huffman-decode a cache's stream of T tokens and dequantise it in the same launch: out fp16 [T,B,H,128], the bits
+    of dequant(decode(...)).  Returns the status word."""
+    _cuda(out, torch.float16, "out")
+    if tuple(out.shape) != (T, B, H, 128):
+        raise KvcError("out must be [T,B,H,128] = %s, got %s" % ((T, B, H, 128), tuple(out.shape)))
+    status = new_status(out.device) if status is None else status
+    with _on(out.device):
+        _lib.check(_lib.load().kvc_decode_values(C.byref(cache), T, B, H, int(is_k), _p(out), _p(status), _stream()),
+                   "kvc_decode_values")
+    return status
+
+
 def make_cache(encoded, block_info, thread_info, book, min_int, scale, spec, encoded_bytes=None, max_block_bytes=0):
     """The kvc_cache argument of the fused kernels.  The tensors must stay alive during the call."""
     n = encoded.numel() if encoded_bytes is None else int(encoded_bytes)

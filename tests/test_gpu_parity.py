@@ -354,6 +354,25 @@ def test_encode_random_shapes_books_and_alignments(ops):
         assert ops.read_status(st) == 0 and np.array_equal(out.cpu().numpy(), codes), case
 
 
+@pytest.mark.parametrize("is_k,mode,block,shared,min_dtype", [
+    (True, orc.MODE_CHANNEL, 64, False, torch.int16), (True, orc.MODE_CHANNEL, 128, True, torch.int8),
+    (True, orc.MODE_BLOCK, 64, False, torch.int8), (True, orc.MODE_TOKEN, 64, True, torch.int16), (True, orc.MODE_VECTOR, 64, False, torch.int16),
+    (False, orc.MODE_TOKEN, 128, False, torch.int16), (False, orc.MODE_VECTOR, 128, False, torch.int8), (False, orc.MODE_BLOCK, 64, True, torch.int16)])
+@pytest.mark.parametrize("T,B,H", [(128, 1, 1), (384, 3, 5)])
+def test_decode_values_equals_decode_then_dequant(ops, is_k, mode, block, shared, min_dtype, T, B, H):
+    """One launch from the stream to fp16 values, bit for bit what decode and dequant give: every unit layout a
+    cache can have, one block and odd numbers of columns."""
+    k, v, _ = synth(T, B, H, seed=5)
+    r = _pipeline(ops, k if is_k else v, is_k, mode, block, 0.05, shared, min_dtype)
+    codes, st = ops.decode(r["enc"][:r["n"]], r["bi"], r["ti"], r["book"], T, B, H, is_k)
+    assert ops.read_status(st) == 0
+    want = ops.dequant(codes, r["mi"], r["sc"], r["spec"])
+    out = torch.full((T, B, H, 128), 7.0, dtype=torch.float16, device="cuda")
+    cache = ops.make_cache(r["enc"], r["bi"], r["ti"], r["book"], r["mi"], r["sc"], r["spec"], r["n"], r["maxb"])
+    assert ops.read_status(ops.decode_values(cache, T, B, H, is_k, out)) == 0
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
 def test_book_from_reference_decode_tensor(ops):
     k, _, _ = synth(128, 1, 2, seed=4)
     r = _pipeline(ops, k, True, 0, 64, 0.05, True)
