@@ -101,12 +101,15 @@ class KVCompCache(_BASE):
         if k_rows is not False:
             kc.store(k_rows if k_rows is not None else key_states.permute(2, 0, 1, 3).contiguous().half())
         t = value_states.shape[2]
-        place = None
+        place, rows = None, None
         if value_states.is_cuda and value_states.dtype == torch.float16 and value_states.is_contiguous() and value_states.shape[3] % 16 == 0:
             place = vc.recent_place(t, value_states.device)
-        if place is not None:                                   # the transposition writes straight into the window
-            ops.rope_store(value_states, None, None, out=place)
+            if place is not None or value_states.data_ptr() % 16 == 0:
+                rows = ops.rope_store(value_states, None, None, out=place)   # the transposition alone
+        if place is not None:                                   # it wrote straight into the window
             vc.recent_commit(t)
+        elif rows is not None:
+            vc.store(rows)
         else:
             vc.store(value_states.permute(2, 0, 1, 3).contiguous().half())
 

@@ -75,6 +75,29 @@ __device__ __forceinline__ unsigned short kvc_load_scale_bits(const kvc_qmeta_de
 }
 __device__ __forceinline__ float kvc_scale_value(unsigned short bits) { return __half2float(__ushort_as_half(bits)); }
 
+// fp16((code + min_int) * scale) of two codes, each of its steps rounded to fp16: the byte becomes
+// a float as the low bits of 2^23, and the sum with min_int - 2^23 is exact.
+__device__ __forceinline__ uint32_t kvc_dequant2(uint32_t w, uint32_t sel0, uint32_t sel1, float mi0, float mi1, __half2 sc) {
+    const float a = __uint_as_float(__byte_perm(w, 0x4b000000u, sel0)) + mi0, b = __uint_as_float(__byte_perm(w, 0x4b000000u, sel1)) + mi1;
+    const __half2 r = __hmul2(__floats2half2_rn(a, b), sc);
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+// eight codes of two words; per pair of codes the scales, per code min_int - 2^23
+__device__ __forceinline__ uint4 kvc_dequant8(uint32_t x, uint32_t y, const float (&mi)[8], const __half2 (&sc)[4]) {
+    return make_uint4(kvc_dequant2(x, 0x7440, 0x7441, mi[0], mi[1], sc[0]), kvc_dequant2(x, 0x7442, 0x7443, mi[2], mi[3], sc[1]),
+                      kvc_dequant2(y, 0x7440, 0x7441, mi[4], mi[5], sc[2]), kvc_dequant2(y, 0x7442, 0x7443, mi[6], mi[7], sc[3]));
+}
+__device__ __forceinline__ uint4 kvc_dequant8(uint32_t x, uint32_t y, float mi, __half2 sc) {
+    return make_uint4(kvc_dequant2(x, 0x7440, 0x7441, mi, mi, sc), kvc_dequant2(x, 0x7442, 0x7443, mi, mi, sc),
+                      kvc_dequant2(y, 0x7440, 0x7441, mi, mi, sc), kvc_dequant2(y, 0x7442, 0x7443, mi, mi, sc));
+}
+// unit parameters that all channels of a (token, sequence, head) row share
+__device__ __forceinline__ void kvc_row_unit(const kvc_qmeta_dev &m, long long t, long long b, long long h, float &mi, __half2 &sc) {
+    const long long u = kvc_tok_unit(t, m.tok_div) * m.sj + b * m.sb + h * m.sh;
+    mi = (float)kvc_load_min(m, u) - 8388608.0f;
+    sc = __half2half2(m.scale[u]);
+}
+
 __device__ __forceinline__ uint32_t kvc_bswap(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
 // 4x4 byte transpose: in a, b, c, d = rows; out a = {a0,b0,c0,d0}, b = {a1,b1,c1,d1}, ...

@@ -16,29 +16,6 @@ struct DecodeSmem {                         // followed by 4 staging slots (size
 };
 constexpr int TILE_BYTES = 64 * TILE_STRIDE; // a tile; the tiles are also the padding a corrupt stream's overrun reads land in
 
-// fp16((code + min_int) * scale) of two codes, each of its steps rounded to fp16 as dequant_kernel does: the byte becomes
-// a float as the low bits of 2^23, and the sum with min_int - 2^23 is exact.
-__device__ __forceinline__ uint32_t dequant2(uint32_t w, uint32_t sel0, uint32_t sel1, float mi0, float mi1, __half2 sc) {
-    const float a = __uint_as_float(__byte_perm(w, 0x4b000000u, sel0)) + mi0, b = __uint_as_float(__byte_perm(w, 0x4b000000u, sel1)) + mi1;
-    const __half2 r = __hmul2(__floats2half2_rn(a, b), sc);
-    return *reinterpret_cast<const uint32_t *>(&r);
-}
-// eight codes of two words; per pair of codes the scales, per code min_int - 2^23
-__device__ __forceinline__ uint4 dequant8(uint32_t x, uint32_t y, const float (&mi)[8], const __half2 (&sc)[4]) {
-    return make_uint4(dequant2(x, 0x7440, 0x7441, mi[0], mi[1], sc[0]), dequant2(x, 0x7442, 0x7443, mi[2], mi[3], sc[1]),
-                      dequant2(y, 0x7440, 0x7441, mi[4], mi[5], sc[2]), dequant2(y, 0x7442, 0x7443, mi[6], mi[7], sc[3]));
-}
-__device__ __forceinline__ uint4 dequant8(uint32_t x, uint32_t y, float mi, __half2 sc) {
-    return make_uint4(dequant2(x, 0x7440, 0x7441, mi, mi, sc), dequant2(x, 0x7442, 0x7443, mi, mi, sc),
-                      dequant2(y, 0x7440, 0x7441, mi, mi, sc), dequant2(y, 0x7442, 0x7443, mi, mi, sc));
-}
-// unit parameters that all channels of a (token, sequence, head) row share
-__device__ __forceinline__ void row_unit(const kvc_qmeta_dev &m, long long t, long long b, long long h, float &mi, __half2 &sc) {
-    const long long u = kvc_tok_unit(t, m.tok_div) * m.sj + b * m.sb + h * m.sh;
-    mi = (float)kvc_load_min(m, u) - 8388608.0f;
-    sc = __half2half2(m.scale[u]);
-}
-
 // VALUES: fp16 values [T, cols, 128] instead of the codes.  The units either do not depend on the channel (m.sc == 0), or
 // (K) lie side by side over the channels and cover whole blocks of 64 tokens.
 template <bool VALUES>
@@ -98,13 +75,13 @@ __global__ void __launch_bounds__(256) decode_kernel(
                     for (int k = 0; k < 4; k++) sc[k] = __halves2half2(m.scale[u + 2 * k], m.scale[u + 2 * k + 1]);
 #pragma unroll 4
                     for (int r = v >> 4; r < 64; r += 4)
-                        *reinterpret_cast<uint4 *>(dst + r * row) = dequant8(t4[r * (TILE_STRIDE / 4)], t4[r * (TILE_STRIDE / 4) + 1], mi, sc);
+                        *reinterpret_cast<uint4 *>(dst + r * row) = kvc_dequant8(t4[r * (TILE_STRIDE / 4)], t4[r * (TILE_STRIDE / 4) + 1], mi, sc);
                 } else {
 #pragma unroll 4
                     for (int r = v >> 4; r < 64; r += 4) {
                         float mi; __half2 sc;
-                        row_unit(m, j * 64 + r, b, h, mi, sc);
-                        *reinterpret_cast<uint4 *>(dst + r * row) = dequant8(t4[r * (TILE_STRIDE / 4)], t4[r * (TILE_STRIDE / 4) + 1], mi, sc);
+                        kvc_row_unit(m, j * 64 + r, b, h, mi, sc);
+                        *reinterpret_cast<uint4 *>(dst + r * row) = kvc_dequant8(t4[r * (TILE_STRIDE / 4)], t4[r * (TILE_STRIDE / 4) + 1], mi, sc);
                     }
                 }
             } else if (VALUES) {                             // 32 groups of 4 tokens x 8 chunks of 8 channels
@@ -121,8 +98,8 @@ __global__ void __launch_bounds__(256) decode_kernel(
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         float mi; __half2 sc;
-                        row_unit(m, g * 128 + tg * 4 + k, b, h, mi, sc);
-                        *reinterpret_cast<uint4 *>(dst + (tg * 4 + k) * row + c8 * 8) = dequant8(x[k], x[4 + k], mi, sc);
+                        kvc_row_unit(m, g * 128 + tg * 4 + k, b, h, mi, sc);
+                        *reinterpret_cast<uint4 *>(dst + (tg * 4 + k) * row + c8 * 8) = kvc_dequant8(x[k], x[4 + k], mi, sc);
                     }
                 }
             } else if (is_k) {

@@ -422,26 +422,72 @@ __global__ void __launch_bounds__(256) quant_block_apply_kernel(
 }
 
 // ---- dequantise: fp16((code + min_int) * scale), models/cache/kvcomp_encode.py:146 -------------
+// Bound by memory (1 byte in, 2 out).  A thread takes four groups of 8 channels, all their loads in flight together;
+// wide_units: units side by side over the channels, 8 of them fetched with one load per array.  With one group per
+// thread, 64-bit divisions and a load per unit: 67 M values 95 us (units per channel) and 85 us (per token); now 70 and 38 us.
+constexpr int DEQ_GROUPS = 4;
 __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t *__restrict__ codes, kvc_qmeta_dev m,
-                                                      long long rows, long long B, long long H, int D,
+                                                      long long rows, uint32_t B, uint32_t H, uint32_t D, int wide_units,
                                                       __half *__restrict__ out) {
-    // one thread = 8 consecutive channels of one (t, b, h) row
-    const long long per_row = D / 8;
-    long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (i >= rows * per_row) return;
-    const long long row = i / per_row; const int c0 = (int)(i % per_row) * 8;
-    const long long h = row % H, b = (row / H) % B, t = row / (H * B);
-    const long long ub = kvc_tok_unit(t, m.tok_div) * m.sj + b * m.sb + h * m.sh;
-    uint2 cv = *reinterpret_cast<const uint2 *>(codes + row * D + c0);
-    const uint8_t *cb = reinterpret_cast<const uint8_t *>(&cv);
-    uint4 o; __half *oh = reinterpret_cast<__half *>(&o);
+    const uint32_t per_row = D / 8;
+    const long long n = rows * per_row, i0 = (long long)blockIdx.x * (256 * DEQ_GROUPS) + threadIdx.x;
+    uint2 cv[DEQ_GROUPS];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        long long u = ub + (long long)(c0 + k) * m.sc;
-        float s = __half2float(__float2half_rn((float)((int)cb[k] + kvc_load_min(m, u))));
-        oh[k] = __float2half_rn(__fmul_rn(s, __half2float(m.scale[u])));
+    for (int g = 0; g < DEQ_GROUPS; g++) {
+        const long long i = i0 + g * 256;
+        if (i < n) cv[g] = *reinterpret_cast<const uint2 *>(codes + i * 8);
     }
-    *reinterpret_cast<uint4 *>(out + row * D + c0) = o;
+#pragma unroll
+    for (int g = 0; g < DEQ_GROUPS; g++) {
+        const long long i = i0 + g * 256;
+        if (i >= n) return;
+        uint32_t c0, h, b;
+        long long t;
+        if (n < (1ll << 32)) {                               // the same for the whole grid
+            uint32_t r = (uint32_t)i / per_row;
+            c0 = ((uint32_t)i - r * per_row) * 8;
+            h = r % H; r /= H; b = r % B; t = r / B;
+        } else {
+            long long r = i / per_row;
+            c0 = (uint32_t)(i - r * per_row) * 8;
+            h = (uint32_t)(r % H); r /= H; b = (uint32_t)(r % B); t = r / B;
+        }
+        uint4 o;
+        if (m.sc == 0) {
+            float mi; __half2 sc;
+            kvc_row_unit(m, t, b, h, mi, sc);
+            o = kvc_dequant8(cv[g].x, cv[g].y, mi, sc);
+        } else {
+            const long long u = kvc_tok_unit(t, m.tok_div) * m.sj + b * m.sb + h * m.sh + (long long)c0 * m.sc;
+            float mi[8];
+            __half2 sc[4];
+            if (wide_units) {
+                const uint4 sv = *reinterpret_cast<const uint4 *>(m.scale + u);
+                const __half2 *s2 = reinterpret_cast<const __half2 *>(&sv);
+#pragma unroll
+                for (int k = 0; k < 4; k++) sc[k] = s2[k];
+                if (m.min_bytes == 1) {
+                    const uint2 mv = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(m.min_int) + u);
+                    const int8_t *mb = reinterpret_cast<const int8_t *>(&mv);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) mi[k] = (float)mb[k] - 8388608.0f;
+                } else {
+                    const uint4 mv = *reinterpret_cast<const uint4 *>(reinterpret_cast<const int16_t *>(m.min_int) + u);
+                    const int16_t *mh = reinterpret_cast<const int16_t *>(&mv);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) mi[k] = (float)mh[k] - 8388608.0f;
+                }
+            } else {
+                __half s1[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) { mi[k] = (float)kvc_load_min(m, u + k * m.sc) - 8388608.0f; s1[k] = m.scale[u + k * m.sc]; }
+#pragma unroll
+                for (int k = 0; k < 4; k++) sc[k] = __halves2half2(s1[2 * k], s1[2 * k + 1]);
+            }
+            o = kvc_dequant8(cv[g].x, cv[g].y, mi, sc);
+        }
+        *reinterpret_cast<uint4 *>(out + i * 8) = o;
+    }
 }
 
 // ---- dense q.k over uncompressed K (kernels.cu:1192-1219), fp32 accumulation --------------------
@@ -572,8 +618,11 @@ extern "C" int kvc_dequant(const uint8_t *codes, const kvc_qmeta *q, int64_t T, 
     KVC_REQUIRE(q->min_bytes == 1 || q->min_bytes == 2, "kvc_dequant: min_bytes must be 1 or 2");
     long long rows = T * B * H, n = rows * (D / 8);
     if (n == 0) return KVC_OK;
-    dequant_kernel<<<(unsigned)((n + 255) / 256), 256, 0, kvc_cu(stream)>>>(codes, kvc_to_dev(*q), rows, B, H, (int)D,
-                                                                            reinterpret_cast<__half *>(out));
+    const kvc_qmeta_dev m = kvc_to_dev(*q);
+    const int wide_units = m.sc == 1 && m.sj % 8 == 0 && m.sb % 8 == 0 && m.sh % 8 == 0 &&
+                           (reinterpret_cast<uintptr_t>(m.scale) & 15) == 0 && (reinterpret_cast<uintptr_t>(m.min_int) & (8 * m.min_bytes - 1)) == 0;
+    dequant_kernel<<<(unsigned)((n + 256 * DEQ_GROUPS - 1) / (256 * DEQ_GROUPS)), 256, 0, kvc_cu(stream)>>>(
+        codes, m, rows, (uint32_t)B, (uint32_t)H, (uint32_t)D, wide_units, reinterpret_cast<__half *>(out));
     KVC_LAUNCH_OK();
     return KVC_OK;
 }
@@ -587,6 +636,22 @@ extern "C" int kvc_k_matvec(const void *k, const void *q, void *out, int64_t ctx
         reinterpret_cast<const __half *>(k), reinterpret_cast<const __half *>(q), reinterpret_cast<__half *>(out), rows, H);
     KVC_LAUNCH_OK();
     return KVC_OK;
+}
+
+// eight channels of the lower half (xa) and their partners of the upper half (xb), rotated with torch's roundings
+__device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const uint4 &ca, const uint4 &cb, const uint4 &sa, const uint4 &sb,
+                                      uint4 &oa, uint4 &ob) {
+    const __half *x1 = reinterpret_cast<const __half *>(&xa), *x2 = reinterpret_cast<const __half *>(&xb);
+    const __half *c1 = reinterpret_cast<const __half *>(&ca), *c2 = reinterpret_cast<const __half *>(&cb);
+    const __half *s1 = reinterpret_cast<const __half *>(&sa), *s2 = reinterpret_cast<const __half *>(&sb);
+    __half *o1 = reinterpret_cast<__half *>(&oa), *o2 = reinterpret_cast<__half *>(&ob);
+    auto mul = [](__half a, __half b2) { return __half2float(__float2half_rn(__fmul_rn(__half2float(a), __half2float(b2)))); };
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        // rotate_half: the lower half meets -x2, the upper half x1
+        o1[k] = __float2half_rn(__fadd_rn(mul(x1[k], c1[k]), mul(__hneg(x2[k]), s1[k])));
+        o2[k] = __float2half_rn(__fadd_rn(mul(x2[k], c2[k]), mul(x1[k], s2[k])));
+    }
 }
 
 // ---- rotary embedding of new keys on their way into the cache -------------------------------------
@@ -618,20 +683,44 @@ __global__ void __launch_bounds__(256) rope_store_kernel(const __half *__restric
     const __half *cr = cs + b * cs_bstride + tok * D, *sr = sn + b * cs_bstride + tok * D;
     const uint4 ca = *reinterpret_cast<const uint4 *>(cr + c0), cb = *reinterpret_cast<const uint4 *>(cr + c0 + half);
     const uint4 sa = *reinterpret_cast<const uint4 *>(sr + c0), sb = *reinterpret_cast<const uint4 *>(sr + c0 + half);
-    const __half *x1 = reinterpret_cast<const __half *>(&xa), *x2 = reinterpret_cast<const __half *>(&xb);
-    const __half *c1 = reinterpret_cast<const __half *>(&ca), *c2 = reinterpret_cast<const __half *>(&cb);
-    const __half *s1 = reinterpret_cast<const __half *>(&sa), *s2 = reinterpret_cast<const __half *>(&sb);
     uint4 oa, ob;
-    __half *o1 = reinterpret_cast<__half *>(&oa), *o2 = reinterpret_cast<__half *>(&ob);
-    auto mul = [](__half a, __half b2) { return __half2float(__float2half_rn(__fmul_rn(__half2float(a), __half2float(b2)))); };
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        // rotate_half: the lower half meets -x2, the upper half x1
-        o1[k] = __float2half_rn(__fadd_rn(mul(x1[k], c1[k]), mul(__hneg(x2[k]), s1[k])));
-        o2[k] = __float2half_rn(__fadd_rn(mul(x2[k], c2[k]), mul(x1[k], s2[k])));
-    }
+    rope8(xa, xb, ca, cb, sa, sb, oa, ob);
     *reinterpret_cast<uint4 *>(orow + c0) = oa;
     *reinterpret_cast<uint4 *>(orow + c0 + half) = ob;
+}
+
+// The same for a prompt (head_dim 128): a CTA takes 32 tokens of HT neighbouring heads.  rope_store_kernel's order, one row
+// per head of a token, reads 256 bytes of a page at a time and fetches cos and sin for every head: 1 GiB of keys 515 us,
+// and values went through torch's strided copy (1232 us).  Here a warp reads 1 KB runs of each head, writes runs of
+// HT rows, and a thread keeps cos and sin over its heads and HT x 2 loads in flight.
+template <int HT>
+__global__ void __launch_bounds__(256) rope_tile_kernel(const __half *__restrict__ x, const __half *__restrict__ cs,
+                                                        const __half *__restrict__ sn, __half *__restrict__ out,
+                                                        uint32_t B, uint32_t H, long long t, long long cs_bstride) {
+    const uint32_t groups = H / HT, b = blockIdx.x / groups, h0 = (blockIdx.x % groups) * HT;
+    const long long tok = (long long)blockIdx.y * 32 + (threadIdx.x >> 3);
+    const int c0 = (threadIdx.x & 7) * 8;
+    if (tok >= t) return;
+    const __half *xr = x + (((long long)b * H + h0) * t + tok) * 128 + c0;
+    __half *orow = out + ((tok * B + b) * H + h0) * 128 + c0;
+    uint4 xa[HT], xb[HT];
+#pragma unroll
+    for (int k = 0; k < HT; k++) {
+        xa[k] = *reinterpret_cast<const uint4 *>(xr + k * t * 128);
+        xb[k] = *reinterpret_cast<const uint4 *>(xr + k * t * 128 + 64);
+    }
+    if (cs != nullptr) {
+        const __half *cr = cs + b * cs_bstride + tok * 128 + c0, *sr = sn + b * cs_bstride + tok * 128 + c0;
+        const uint4 ca = *reinterpret_cast<const uint4 *>(cr), cb = *reinterpret_cast<const uint4 *>(cr + 64);
+        const uint4 sa = *reinterpret_cast<const uint4 *>(sr), sb = *reinterpret_cast<const uint4 *>(sr + 64);
+#pragma unroll
+        for (int k = 0; k < HT; k++) { uint4 oa, ob; rope8(xa[k], xb[k], ca, cb, sa, sb, oa, ob); xa[k] = oa; xb[k] = ob; }
+    }
+#pragma unroll
+    for (int k = 0; k < HT; k++) {
+        *reinterpret_cast<uint4 *>(orow + k * 128) = xa[k];
+        *reinterpret_cast<uint4 *>(orow + k * 128 + 64) = xb[k];
+    }
 }
 
 extern "C" int kvc_rope_store(const void *x, const void *cos_, const void *sin_, void *out, int64_t B, int64_t H, int64_t t,
@@ -644,6 +733,17 @@ extern "C" int kvc_rope_store(const void *x, const void *cos_, const void *sin_,
     const long long n = t * B * H * (D / 16);
     if (n == 0) return KVC_OK;
     KVC_REQUIRE((n + 255) / 256 < (1ll << 31), "kvc_rope_store: too many elements");
+    // tiles when there are enough of them to fill the device twice over; else a thread per 16 channels of a row
+    const int ht = H % 4 == 0 ? 4 : (H % 2 == 0 ? 2 : 1);
+    const long long col_groups = B * (H / ht), tok_tiles = (t + 31) / 32;
+    if (D == 128 && t >= 32 && col_groups * tok_tiles >= 2ll * kvc_sm_count() && tok_tiles <= 65535 && col_groups < (1ll << 31)) {
+        auto *kernel = ht == 4 ? rope_tile_kernel<4> : (ht == 2 ? rope_tile_kernel<2> : rope_tile_kernel<1>);
+        kernel<<<dim3((unsigned)col_groups, (unsigned)tok_tiles), 256, 0, kvc_cu(stream)>>>(
+            reinterpret_cast<const __half *>(x), reinterpret_cast<const __half *>(cos_), reinterpret_cast<const __half *>(sin_),
+            reinterpret_cast<__half *>(out), (uint32_t)B, (uint32_t)H, t, cos_batch_stride);
+        KVC_LAUNCH_OK();
+        return KVC_OK;
+    }
     rope_store_kernel<<<(unsigned)((n + 255) / 256), 256, 0, kvc_cu(stream)>>>(
         reinterpret_cast<const __half *>(x), reinterpret_cast<const __half *>(cos_), reinterpret_cast<const __half *>(sin_),
         reinterpret_cast<__half *>(out), B, H, t, (int)D, cos_batch_stride, nullptr, nullptr);

@@ -472,6 +472,23 @@ def test_attend_pre_rope_and_plain(cfg):
         assert out.shape == (B, Hq, 1, 128) and (out.float() - ref).abs().max() <= 2e-3 * ref.abs().max()
 
 
+@pytest.mark.parametrize("B,H,t", [(8, 12, 400), (5, 6, 681), (9, 3, 415), (2, 32, 1024)])
+def test_rope_store_of_a_prompt_equals_torch_ops(B, H, t):
+    """Prompts take 32 tokens of 4, 2 or 1 heads per CTA (ragged last tile): the bits of torch's op sequence, and of
+    its transposing copy without a rotation."""
+    import torch
+    from kvcomp_b200 import ops
+    from kvcomp_b200.utils.compute import apply_rotary_pos_emb_single
+    g = torch.Generator(device="cuda").manual_seed(B)
+    x = torch.randn(B, H, t, 128, device="cuda", generator=g).half()
+    ang = 6.0 * torch.rand(B, t, 128, device="cuda", generator=g)
+    cos, sin = ang.cos().half(), ang.sin().half()
+    for c, s in ((cos, sin), (cos[:1].contiguous(), sin[:1].contiguous())):
+        want = apply_rotary_pos_emb_single(x, c, s).permute(2, 0, 1, 3).contiguous()
+        assert torch.equal(ops.rope_store(x, c, s), want)
+    assert torch.equal(ops.rope_store(x, None, None), x.permute(2, 0, 1, 3).contiguous())
+
+
 def test_rope_store_equals_torch_ops():
     """kvc_rope_store against the reference's op sequence (utils/compute.py:25-33) evaluated by torch on
     CUDA fp16 tensors, followed by the transposition to token-major: the same bits, for batch-wide and

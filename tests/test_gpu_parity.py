@@ -373,6 +373,24 @@ def test_decode_values_equals_decode_then_dequant(ops, is_k, mode, block, shared
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
 
 
+@pytest.mark.parametrize("mode,block", [(orc.MODE_CHANNEL, 64), (orc.MODE_TOKEN, 64), (orc.MODE_VECTOR, 64), (orc.MODE_BLOCK, 128)])
+@pytest.mark.parametrize("min_dtype", [torch.int8, torch.int16])
+@pytest.mark.parametrize("offset", [0, 1])                  # 1: unit arrays off the boundaries of the wide loads
+def test_dequant_matches_torch(ops, mode, block, min_dtype, offset):
+    T, B, H = 128, 3, 5
+    spec = ops.qspec(mode, False, B, H, 128, block)
+    n = spec.units(T, B, H, 128)
+    g = torch.Generator().manual_seed(2)
+    codes = torch.randint(0, 256, (T, B, H, 128), generator=g, dtype=torch.uint8).cuda()
+    lim = 128 if min_dtype == torch.int8 else 32768
+    mi = torch.randint(-lim, lim, (n + 1,), generator=g).to(min_dtype).cuda()[offset:offset + n]
+    sc = (2.0 ** (6 * torch.randn(n + 1, generator=g) - 8)).half().cuda()[offset:offset + n]
+    t, b, h, c = torch.meshgrid(*(torch.arange(k, device="cuda") for k in (T, B, H, 128)), indexing="ij")
+    u = t // spec.tok_div * spec.sj + b * spec.sb + h * spec.sh + c * spec.sc
+    want = (codes.float() + mi[u].float()).half() * sc[u]
+    assert torch.equal(ops.dequant(codes, mi, sc, spec), want)
+
+
 def test_book_from_reference_decode_tensor(ops):
     k, _, _ = synth(128, 1, 2, seed=4)
     r = _pipeline(ops, k, True, 0, 64, 0.05, True)
