@@ -28,6 +28,7 @@
 #include <math_constants.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "kvc_decode.cuh"
 
@@ -117,10 +118,11 @@ __device__ __forceinline__ void mma_uu(int (&c)[4], uint32_t a0, uint32_t a1, ui
 }
 
 // decode the thread's vector into its row (shared address, 16-byte aligned)
-__device__ __forceinline__ bool decode_row(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, uint32_t tree_s, bool esc, uint32_t row_s) {
+__device__ __forceinline__ bool decode_row(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, const void *book, bool esc, uint32_t row_s) {
+    const KvcTreeGlobal tree(book);
     KvcRowWriter put;
-    return esc ? kvc_decode_vector<true, 0>(slot_s, byte_pos, lut_s, tree_s, row_s, put)
-               : kvc_decode_vector<false, 0, decltype(put), true>(slot_s, byte_pos, lut_s, tree_s, row_s, put);
+    return esc ? kvc_decode_vector<true, 0, KvcRowWriter, false>(slot_s, byte_pos, lut_s, tree, row_s, put)
+               : kvc_decode_vector<false, 0, KvcRowWriter, true>(slot_s, byte_pos, lut_s, tree, row_s, put);
 }
 
 // The products of a warp's 32 rows (first one at shared address rows_s) with the weight words at shared address
@@ -179,7 +181,7 @@ __device__ __forceinline__ bool decode_dot_impl(uint32_t slot_s, uint32_t byte_p
     };
     // two lookups per round: the weight rows keep WROW - 128 zeroed positions for what is emitted past 127
     static_assert(WROW >= 128 + KVC_DECODE_OVERRUN_PAIR + 1, "weight rows too short for paired lookups");
-    return kvc_decode_vector<ESC, SHIFT, decltype(emit), true>(slot_s, byte_pos, lut_s, tree_s, w_s >> SHIFT, emit);
+    return kvc_decode_vector<ESC, SHIFT, decltype(emit), true>(slot_s, byte_pos, lut_s, KvcTreeShared{tree_s}, w_s >> SHIFT, emit);
 }
 // esc: the book has codes longer than the table window (uniform over the CTA)
 template <int G>
@@ -556,9 +558,10 @@ __global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T
 }
 
 // ---- one-pass decode attention -------------------------------------------------------------------
+struct LutSmem { uint32_t lut[KVC_LUT_SIZE]; };        // rows form: the trees stay in global memory, shared memory decides how many CTAs fit
 template <int G>
 struct alignas(32) AttnSmem {                     // followed in shared memory by 4 K slots, 4 V slots (sized at launch),
-    KvcBookSmem bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
+    typename std::conditional<(G >= 2), LutSmem, KvcBookSmem>::type bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
     // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum, in the rows form by the V weight words
     alignas(32) uint32_t w[4 * VecWords<G, (G >= 2)>::value];
     alignas(32) uint32_t ps[G >= 2 ? 8 : 2 * VecWords<G, false>::value];    // V weight words (one-pass form)
@@ -669,8 +672,8 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
     }
     bool escK = false, escV = false;
     if (p.T > 0) {                                         // (no streams at all while nothing is compressed yet)
-        kvc_load_book(sm.bookK, p.k.book, tid, NTHR);
-        kvc_load_book(sm.bookV, p.v.book, tid, NTHR);
+        if constexpr (ROWS) { kvc_load_lut(sm.bookK.lut, p.k.book, tid, NTHR); kvc_load_lut(sm.bookV.lut, p.v.book, tid, NTHR); }
+        else { kvc_load_book(sm.bookK, p.k.book, tid, NTHR); kvc_load_book(sm.bookV, p.v.book, tid, NTHR); }
         escK = book_has_long_codes(p.k.book); escV = book_has_long_codes(p.v.book);
     }
 
@@ -784,7 +787,7 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
             bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
             const uint32_t posK = sm.leadK[sub] + (cur.startK >> 3);
             if constexpr (ROWS) {
-                if (ok) ok = decode_row(kvc_smem_addr(slotsK + sub * p.slotK_bytes), posK, kvc_smem_addr(sm.bookK.lut), kvc_smem_addr(sm.bookK.tree), escK, rows_s + tid * (ROW_WORDS * 4));
+                if (ok) ok = decode_row(kvc_smem_addr(slotsK + sub * p.slotK_bytes), posK, kvc_smem_addr(sm.bookK.lut), p.k.book, escK, rows_s + tid * (ROW_WORDS * 4));
                 __syncwarp();
                 int d[4][2];
                 rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + sub * VecWords<G, true>::value), lane, d);
@@ -932,7 +935,7 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
                 }
             };
             if constexpr (ROWS) {
-                if (ok) ok = decode_row(kvc_smem_addr(slotsV + sub * p.slotV_bytes), posV, kvc_smem_addr(sm.bookV.lut), kvc_smem_addr(sm.bookV.tree), escV, rows_s + tid * (ROW_WORDS * 4));
+                if (ok) ok = decode_row(kvc_smem_addr(slotsV + sub * p.slotV_bytes), posV, kvc_smem_addr(sm.bookV.lut), p.v.book, escV, rows_s + tid * (ROW_WORDS * 4));
                 __syncwarp();
                 int d[4][2];
                 rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + grp * VecWords<G, true>::value), lane, d);
@@ -1360,8 +1363,6 @@ extern "C" int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hk
 static int g_wait_limit = 0, g_starve = 0;
 extern "C" void kvc_attn_debug(int wait_limit, int starve) { g_wait_limit = wait_limit; g_starve = starve; }
 
-// shared memory of an SM (each resident CTA takes 1 KB more than it asks for)
-constexpr size_t SM_SHARED_BYTES = 228 * 1024;
 // CTAs per SM the attention kernel is launched with at most (its launch bounds ask for this many)
 constexpr int ATTN_CTAS_PER_SM = 3;
 // items a resident CTA should get on average: enough that the draws even out the CTAs' speeds and the
@@ -1477,9 +1478,10 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     const int sms = kvc_sm_count();
     const long long Gt = Hq / Hkv;
     for (long long g0 = 0; g0 < Gt && !(T == 0 && tail_in_merge);) {       // nothing compressed: the merge kernel alone
-        // Heads per launch: every launch decodes the whole cache, so up to 8 go together where two such CTAs fit an SM;
-        // with one CTA an SM idles at every barrier, and then up to 4 go together.  The launches get equal shares.
-        const long long most = 2 * (rows_smem(sizeof(AttnSmem<8>)) + 1024) <= SM_SHARED_BYTES ? 8 : 4;
+        // Heads per launch: every launch decodes the whole cache, so up to 8 go together, in launches of equal shares.
+        // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 461 us in two launches of 4, 244 us in one; where only one
+        // CTA of 8 heads fits an SM, K rel 0.02 and both trees in shared memory: 502 and 399 us; 2 x 5 heads, 0.01: 701 and 442 us.)
+        const long long most = 8;
         const long long launches = (Gt - g0 + most - 1) / most;
         const int nh = (int)((Gt - g0 + launches - 1) / launches), G = nh > 4 ? 8 : (nh > 2 ? 4 : nh);
         p.g0 = g0; p.nh = nh;

@@ -52,9 +52,10 @@ __global__ void __launch_bounds__(256) decode_kernel(
             // (at most KVC_DECODE_OVERRUN_PAIR) stay within the row's padding words
             KvcRowWriter put;
             const uint32_t slot_s = kvc_smem_addr(slots + sub * slot_bytes), lut_s = kvc_smem_addr(sm.book.lut),
-                           tree_s = kvc_smem_addr(sm.book.tree), row_s = kvc_smem_addr(trow);
-            if (ok) ok = esc ? kvc_decode_vector<true, 0>(slot_s, lead + start, lut_s, tree_s, row_s, put)
-                             : kvc_decode_vector<false, 0, decltype(put), true>(slot_s, lead + start, lut_s, tree_s, row_s, put);
+                           row_s = kvc_smem_addr(trow);
+            const KvcTreeShared tree{kvc_smem_addr(sm.book.tree)};
+            if (ok) ok = esc ? kvc_decode_vector<true, 0>(slot_s, lead + start, lut_s, tree, row_s, put)
+                             : kvc_decode_vector<false, 0, decltype(put), true>(slot_s, lead + start, lut_s, tree, row_s, put);
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
         }
         __syncthreads();

@@ -26,6 +26,22 @@ __device__ __forceinline__ void kvc_load_book(KvcBookSmem &b, const void *book, 
     for (int i = tid; i < N16; i += nthr) dst[i] = src[i];
 }
 
+// the wide decode tree, read only for codes longer than the table's window
+struct KvcTreeShared {
+    uint32_t addr;
+    __device__ __forceinline__ uint32_t operator()(uint32_t node) const;
+};
+struct KvcTreeGlobal {                    // for kernels short of shared memory
+    const uint32_t *nodes;
+    __device__ __forceinline__ KvcTreeGlobal(const void *book) : nodes(reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_TREE)) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t node) const { return nodes[node]; }
+};
+// the table alone
+__device__ __forceinline__ void kvc_load_lut(uint32_t *lut, const void *book, int tid, int nthr) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_LUT);
+    for (int i = tid; i < KVC_LUT_SIZE / 4; i += nthr) reinterpret_cast<uint4 *>(lut)[i] = src[i];
+}
+
 // Copy the bytes [off, off+n) of `encoded` into `slot` so that slot and source agree modulo 16:
 // the first stream byte lands at slot[lead], lead = address & 15.  Whole 16-byte chunks inside the
 // buffer move as 128-bit loads; the ragged edges move bytewise, never touching memory outside
@@ -96,6 +112,7 @@ __device__ __forceinline__ uint32_t kvc_lds32(uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
+__device__ __forceinline__ uint32_t KvcTreeShared::operator()(uint32_t node) const { return kvc_lds32(addr + node * 4); }
 __device__ __forceinline__ uint2 kvc_lds64(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
@@ -111,7 +128,7 @@ __device__ __forceinline__ bool kvc_book_needs_escape(const void *book) {
 }
 
 // Decode one vector.  slot_s: shared-space address of the staged block (16-byte aligned); byte_pos:
-// where the vector starts in it; lut_s / tree_s: shared-space addresses of the book's tables.
+// where the vector starts in it; lut_s: shared-space address of the book's table; tree: its tree (KvcTree*).
 // The decoder state is (position << 6) | bit offset into the (hi, lo) register pair, so applying a
 // table entry is one add of its low byte.
 // emit(e, a, s0, s1): `e` holds up to three symbols in bytes 1..3 for positions c..c+2 of the vector (unused
@@ -126,8 +143,8 @@ __device__ __forceinline__ bool kvc_book_needs_escape(const void *book) {
 // Every round advances by at least one symbol, so the loop ends after at most 128 rounds; a corrupt
 // stream can read at most a few hundred bytes past its vector, for which the kernels keep padding
 // behind the last slot.  Returns false when the bits do not form valid codes.
-template <bool ESC, int SHIFT, class Emit, bool PAIR = false>
-__device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, uint32_t tree_s,
+template <bool ESC, int SHIFT, class Emit, bool PAIR = false, class Tree = KvcTreeShared>
+__device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, Tree tree,
                                                   uint32_t base, Emit emit) {
     static_assert(SHIFT >= 0 && SHIFT <= 6, "record size");
     constexpr uint32_t AMASK = 0xffffffffu << SHIFT;       // drops the bit-offset bits left below the position
@@ -178,7 +195,7 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
             for (int guard = 0; guard < 40; guard++) {
                 if (state & 32u) { hi = lo; lo = kvc_bswap(nxt); nxt = kvc_lds32(ptr); ptr += 4; state -= 32u; }
                 if (node >= 512u) break;
-                const uint32_t nd = kvc_lds32(tree_s + node * 4);
+                const uint32_t nd = tree(node);
                 if ((nd & 0xffffu) == KVC_TREE_LEAF) { sym = nd >> 16; found = true; break; }
                 const uint32_t bit = __funnelshift_l(lo, hi, state) >> 31;
                 state += 1u;

@@ -587,7 +587,7 @@ def test_attn_decode_llama7b_shape_small(ops):
 @pytest.mark.parametrize("G", [2, 3, 5, 6, 7, 8, 9, 16])
 @pytest.mark.parametrize("kmode,krel,T,Tr,tight", [(orc.MODE_CHANNEL, 0.05, 640, 0, True),     # half a tile at the end
                                                    (orc.MODE_TOKEN, 0.05, 384, 131, True),    # one K unit per token, a tail of two passes
-                                                   (orc.MODE_BLOCK, 0.02, 256, 300, False)])  # slots for the largest block: four heads per launch at most
+                                                   (orc.MODE_BLOCK, 0.02, 256, 300, False)])  # slots for the largest block: one CTA per SM
 def test_attn_decode_query_heads_per_kv_head(ops, G, kmode, krel, T, Tr, tight):
     """Grouped queries go up to eight heads per launch through the tensor cores, padded to 2, 4 or 8 columns:
     every number of heads, with the merge kernel and with the column's output and tail written directly."""
