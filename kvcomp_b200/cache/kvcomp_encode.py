@@ -169,7 +169,7 @@ class KVCompCtx:
         self._ti = _Arena(torch.int16)
         self._mi = _Arena(self.min_dtype)
         self._sc = _Arena(torch.float16)
-        self._hist = None
+        self._cache_arg = self._cache_q = None   # cache()'s argument structure, refilled at every call
 
     # ---- views with the reference's attribute names --------------------------------------------
     @property
@@ -251,14 +251,15 @@ class KVCompCtx:
             self.device = cache.device
         assert self.device == cache.device, "device mismatch"
 
-    def _quantize(self, x, hist):
+    def _quantize(self, x, report):
         T = x.shape[0]
         n = self.spec.units(T, self.batch_size, self.head_num, self.head_dim)
         mi = self._mi.reserve(n, self.device)
         sc = self._sc.reserve(n, self.device)
-        codes, _, _, _, st = ops.quantize(x, _MODE[self.quant_mode], self.block_size, self.quant_scale_rel,
-                                          self.batch_shared, min_dtype=self.min_dtype, hist=hist, min_int=mi, scale=sc)
-        return codes, n, st
+        codes, _, _, _, _ = ops.quantize(x, _MODE[self.quant_mode], self.block_size, self.quant_scale_rel,
+                                         self.batch_shared, min_dtype=self.min_dtype, hist=report.hist, min_int=mi,
+                                         scale=sc, status=report.quant_status)
+        return codes, n
 
     def store(self, cache):
         """Append tokens [t, B, H, D]; whole blocks beyond the recent window are quantised and encoded.
@@ -281,13 +282,20 @@ class KVCompCtx:
         else:
             x, rest = torch.cat([self._recent.view(), cache[:n - live]], dim=0), cache[n - live:]
         T = x.shape[0]
-        hist = None
+        # quantise, book and encode are launched one behind the other; one copy brings back what all of them report
+        # (a wait and a copy for each of them: a 333-token prompt 637 us, now 466)
+        report = ops.Report(self.device, with_hist=self.book is None)
+        codes, n_units = self._quantize(x, report)
         if self.book is None:
-            hist = torch.zeros(256, dtype=torch.int64, device=self.device)
-        codes, n_units, st_q = self._quantize(x, hist)
-        if self.book is None:
-            self.book = ops.build_codebook(hist)
-        flags = ops.read_status(st_q, what="quantize")
+            self.book = ops.build_codebook(report.hist)
+        pend = codes if self._pending is None else torch.cat([self._pending, codes], dim=0)
+        n_enc = pend.shape[0] // self.enc_block * self.enc_block
+        part = pend[:n_enc].contiguous() if n_enc else None
+        stream_room, cap = self._encode_room(part) if n_enc else (0, 0)
+        if n_enc:
+            self._encode_launch(part, stream_room, report)
+        words = report.read()                                 # synchronises, as the reference does
+        flags = ops.check_flags(words[2], what="quantize")
         if flags & ops._lib.FLAG_MIN_OVERFLOW:
             # int8 is the reference's CUDA path, which wraps silently (kvcomp_encode.py:97); its model path
             # keeps min_ints in floating point (utils/compute.py:89).  Wrapped values dequantise wrongly.
@@ -321,11 +329,8 @@ class KVCompCtx:
         self._mi.n += n_units
         self._sc.n += n_units
         self.compressed_ctx_len += T
-        pend = codes if self._pending is None else torch.cat([self._pending, codes], dim=0)
-        n_enc = pend.shape[0] // self.enc_block * self.enc_block
         if n_enc:
-            part = pend[:n_enc].contiguous()
-            if not self._encode(part):
+            if not self._encode_finish(part, stream_room, cap, words):
                 # A symbol the frozen book has no code for.  The reference drops such symbols silently
                 # (kernels.cu:197-205: a table entry of length 0 adds no bits), which corrupts the stream.
                 # Here the book is rebuilt over everything stored so far plus every reachable code, and the
@@ -335,37 +340,46 @@ class KVCompCtx:
         self._pending = pend[n_enc:].contiguous() if pend.shape[0] > n_enc else None
         return codes.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim)
 
-    def _encode(self, codes):
-        """Append the stream of `codes` [T, B, H, D] to the arenas.  False if the book lacks a symbol."""
-        T = codes.shape[0]
-        cols = self.batch_size * self.head_num
-        bsz, tsz, _, cap = ops.buffer_sizes(T, cols * self.head_dim, self.is_k)
-        bi = self._bi.reserve(bsz, self.device)
-        ti = self._ti.reserve(tsz // 2, self.device)
+    def _encode_room(self, codes):
+        """Bytes to reserve for the stream of `codes` [T, B, H, D]: (a first guess, the most it can take)."""
         # The reference reserves one byte per symbol (numel) for every store (kernels.cu:903); the stream
         # needs a fraction of that, so room is reserved from the density seen so far (8 bits per symbol at
         # first) with a quarter on top, and the store is repeated with the full reserve in the rare case
         # that the encoder reports the room as exceeded.
-        seen = self.encoded_ctx_len * cols * self.head_dim
-        est = cap if seen == 0 else min(cap, int(1.25 * self._enc.n / seen * codes.numel()) + 4096)
-        for room in (est, cap):
-            enc = self._enc.reserve(room, self.device)
-            total = torch.tensor([0, self.max_block_bytes], dtype=torch.int64, device=self.device)
-            total, st_e = ops.encode(codes, self.is_k, self.book.encode_table(), bi, ti, enc,
-                                     base_offset=self._enc.n, total=total)
-            n_bytes, max_block = (int(v) for v in total.tolist())      # synchronises, as the reference does
-            flags = ops.read_status(st_e, raise_on_fatal=False)
-            if not (flags & ops._lib.FLAG_STREAM_FULL) or room == cap:
-                break
+        cap = ops.buffer_sizes(codes.shape[0], self.batch_size * self.head_num * self.head_dim, self.is_k)[3]
+        seen = self.encoded_ctx_len * self.batch_size * self.head_num * self.head_dim
+        return (cap if seen == 0 else min(cap, int(1.25 * self._enc.n / seen * codes.numel()) + 4096)), cap
+
+    def _encode_launch(self, codes, room, report):
+        """Encode `codes` into the arenas behind what they hold; nothing counts before _encode_finish."""
+        bsz, tsz, _, _ = ops.buffer_sizes(codes.shape[0], self.batch_size * self.head_num * self.head_dim, self.is_k)
+        ops.encode(codes, self.is_k, self.book.encode_table(), self._bi.reserve(bsz, self.device),
+                   self._ti.reserve(tsz // 2, self.device), self._enc.reserve(room, self.device),
+                   base_offset=self._enc.n, total=report.total, status=report.enc_status)
+
+    def _encode_finish(self, codes, room, cap, words):
+        """The launched stream joins the arenas.  False if the book lacks a symbol."""
+        if words[3] & ops._lib.FLAG_STREAM_FULL and room != cap:
             self.stream_retries = getattr(self, "stream_retries", 0) + 1
-        if flags & ops._lib.FLAG_SYMBOL_MISSING:
+            report = ops.Report(self.device)
+            self._encode_launch(codes, cap, report)
+            words = report.read()
+        if words[3] & ops._lib.FLAG_SYMBOL_MISSING:
             return False
-        ops.read_status(st_e, what="entropy_encode")
-        self._enc.n += n_bytes
+        ops.check_flags(words[3], what="entropy_encode")
+        bsz, tsz, _, _ = ops.buffer_sizes(codes.shape[0], self.batch_size * self.head_num * self.head_dim, self.is_k)
+        self._enc.n += words[0]
         self._bi.n += bsz
         self._ti.n += tsz // 2
-        self.max_block_bytes = max_block
+        self.max_block_bytes = max(self.max_block_bytes, words[1])
         return True
+
+    def _encode(self, codes):
+        """Append the stream of `codes` [T, B, H, D] to the arenas.  False if the book lacks a symbol."""
+        room, cap = self._encode_room(codes)
+        report = ops.Report(self.device)
+        self._encode_launch(codes, room, report)
+        return self._encode_finish(codes, room, cap, report.read())
 
     def _rebook(self, new_codes):
         old = None
@@ -445,9 +459,9 @@ class KVCompCtx:
             first = n // self.spec.tok_div * self.spec.sj                    # unit of the first waiting token
             ops.dequant(self._pending, self._mi.used()[first:], self._sc.used()[first:], self.spec, out=x[n:self.compressed_ctx_len])
         stop.record()
-        stop.synchronize()
         if st is not None:
-            ops.read_status(st, what="entropy_decode")
+            ops.read_status(st, what="entropy_decode")         # waits for the stream: one wait for both
+        stop.synchronize()
         return x, start.elapsed_time(stop)
 
     def get_only_compressed(self):
@@ -469,8 +483,17 @@ class KVCompCtx:
         """The kvc_cache argument of the fused kernels over the encoded_ctx_len tokens of the stream (valid
         until the next store)."""
         assert self.encoded_ctx_len > 0 and self.book is not None, "nothing has been encoded yet"
-        return ops.make_cache(self._enc.buf, self._bi.buf, self._ti.buf, self.book, self._mi.buf, self._sc.buf,
-                              self.spec, self._enc.n, self.max_block_bytes)
+        c = self._cache_arg
+        if c is None:
+            c = self._cache_arg = ops.make_cache(self._enc.buf, self._bi.buf, self._ti.buf, self.book, self._mi.buf,
+                                                 self._sc.buf, self.spec, self._enc.n, self.max_block_bytes)
+            self._cache_q = c.q
+            return c
+        # the same structure, every field that a store can change filled in again (cheaper than a new one)
+        c.encoded, c.encoded_bytes, c.max_block_bytes = self._enc.buf.data_ptr(), self._enc.n, self.max_block_bytes
+        c.block_info, c.thread_info, c.book = self._bi.buf.data_ptr(), self._ti.buf.data_ptr(), self.book.blob.data_ptr()
+        self._cache_q.min_int, self._cache_q.scale = self._mi.buf.data_ptr(), self._sc.buf.data_ptr()
+        return c
 
     def mat_vec_mul(self, B):
         """K: scores [batch, heads, ctx] = q . K^T; V: [1, batch, heads, 128] = P . V over the compressed
@@ -495,8 +518,8 @@ class KVCompCtx:
             part, st = ops.fused_pv(self.cache(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
             C = part.float().sum(dim=0, keepdim=True).half()
         stop.record()
-        stop.synchronize()
         ops.read_status(st, what="mat_vec_mul")
+        stop.synchronize()
         return C, start.elapsed_time(stop)
 
     def save(self, path):

@@ -1274,14 +1274,6 @@ int launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
     return KVC_OK;
 }
 
-template <class K>
-int set_smem(K kernel, size_t bytes) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e != cudaSuccess) { kvc_set_error("cudaFuncSetAttribute(%zu bytes) failed: %s", bytes, cudaGetErrorString(e)); return KVC_ERR_CUDA; }
-    return KVC_OK;
-}
-
 int check_cache(const kvc_cache *c, const char *who, bool is_k) {
     KVC_REQUIRE(c && c->encoded && c->block_info && c->thread_info && c->book && c->q.min_int && c->q.scale,
                 "%s: null pointer in the %s cache", who, is_k ? "K" : "V");
@@ -1321,7 +1313,9 @@ extern "C" int kvc_fused_qk(const kvc_cache *k, int64_t T, int64_t B, int64_t Hk
         const int G = next_chunk(Gt - g0);
 #define KVC_QK(GG)                                                                                              \
     {                                                                                                           \
-        if (int rc = set_smem(fused_qk_kernel<GG>, sizeof(QkSmem<GG>))) return rc;                              \
+        static kvc_launch_slot slot;                                                                            \
+        int occ = 0;                                                                                            \
+        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(fused_qk_kernel<GG>), NTHR, sizeof(QkSmem<GG>), &occ)) return rc; \
         fused_qk_kernel<GG><<<grid, NTHR, sizeof(QkSmem<GG>), kvc_cu(stream)>>>(                                \
             kc, T, B, Hkv, Hq, g0, reinterpret_cast<const __half *>(q), out, out_f32, status);                  \
     }
@@ -1347,7 +1341,9 @@ extern "C" int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hk
         const int G = next_chunk(Gt - g0);
 #define KVC_PV(GG)                                                                                              \
     {                                                                                                           \
-        if (int rc = set_smem(fused_pv_kernel<GG>, sizeof(PvSmem<GG>))) return rc;                              \
+        static kvc_launch_slot slot;                                                                            \
+        int occ = 0;                                                                                            \
+        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(fused_pv_kernel<GG>), NTHR, sizeof(PvSmem<GG>), &occ)) return rc; \
         fused_pv_kernel<GG><<<grid, NTHR, sizeof(PvSmem<GG>), kvc_cu(stream)>>>(                                \
             vc, T, B, Hkv, Hq, g0, reinterpret_cast<const __half *>(P), reinterpret_cast<__half *>(out), status); \
     }
@@ -1488,9 +1484,9 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
 #define KVC_AT(GG, BB)                                                                                          \
     {                                                                                                           \
         const size_t smem = (GG) >= 2 ? rows_smem(sizeof(AttnSmem<GG>)) : slot_total + sizeof(AttnSmem<GG>);     \
-        if (int rc = set_smem(attn_decode_kernel<GG, BB>, smem)) return rc;                                     \
+        static kvc_launch_slot slot;                                                                            \
         int occ = 0;                                                                                            \
-        KVC_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, attn_decode_kernel<GG, BB>, NTHR, smem)); \
+        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(attn_decode_kernel<GG, BB>), NTHR, smem, &occ)) return rc; \
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);             \
         long long ctas = (long long)sms * (occ < ATTN_CTAS_PER_SM ? occ : ATTN_CTAS_PER_SM);                    \
         if (ctas > p.work) ctas = p.work;                                                                       \
@@ -1525,16 +1521,15 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
 static __device__ __align__(256) unsigned char g_attn_scratch[KVC_STATIC_SCRATCH_BYTES];
 
 namespace {
-constexpr int MAX_DEVICES = 64;
 std::mutex g_scratch_mutex;
-void *g_scratch_ptr[MAX_DEVICES] = {};
+void *g_scratch_ptr[KVC_MAX_DEVICES] = {};
 
 // The array's name is only a host-side handle in host code; the device address has to be asked for,
 // once per device, with that device current.
 int static_scratch(void **ptr) {
     int dev = -1;
     KVC_CUDA_OK(cudaGetDevice(&dev));
-    KVC_REQUIRE(dev >= 0 && dev < MAX_DEVICES, "kvc_attn_decode_static: device %d out of range", dev);
+    KVC_REQUIRE(dev >= 0 && dev < KVC_MAX_DEVICES, "kvc_attn_decode_static: device %d out of range", dev);
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     if (!g_scratch_ptr[dev]) {
         void *p = nullptr;

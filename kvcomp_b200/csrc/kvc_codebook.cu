@@ -9,6 +9,8 @@
 // than the left one, drop the former last element there and sift it up.
 #include <stdarg.h>
 
+#include <mutex>
+
 #include "kvc_common.cuh"
 
 static thread_local char g_err[512] = "";
@@ -24,10 +26,36 @@ extern "C" const char *kvc_last_error(void) { return g_err; }
 extern "C" int kvc_version(void) { return KVC_VERSION; }
 
 int kvc_sm_count() {
+    static std::atomic<int> known[KVC_MAX_DEVICES];
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    const bool keep = dev >= 0 && dev < KVC_MAX_DEVICES;
+    if (keep && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    if (keep) known[dev].store(n, std::memory_order_relaxed);
     return n;
+}
+
+int kvc_prepare(kvc_launch_slot &slot, const void *kernel, int threads, size_t smem, int *occ) {
+    static std::mutex mutex;
+    int dev = 0;
+    KVC_CUDA_OK(cudaGetDevice(&dev));
+    const bool keep = dev >= 0 && dev < KVC_MAX_DEVICES && smem < (1u << 20);
+    if (keep) {
+        const unsigned long long v = slot.known[dev].load(std::memory_order_acquire);
+        if ((v & 0xff) != 0 && ((v >> 8) & 0xfffff) == smem) { *occ = (int)(v & 0xff); return KVC_OK; }
+    }
+    std::lock_guard<std::mutex> lock(mutex);              // the limit never shrinks under another thread's launch
+    const size_t limit = keep ? (size_t)(slot.known[dev].load(std::memory_order_relaxed) >> 28) : 0;
+    if (smem > limit || limit == 0) {
+        KVC_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KVC_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    }
+    KVC_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kernel, threads, smem));
+    if (keep && *occ > 0 && *occ < 256)
+        slot.known[dev].store((unsigned long long)(smem > limit ? smem : limit) << 28 | (unsigned long long)smem << 8 | (unsigned)*occ,
+                              std::memory_order_release);
+    return KVC_OK;
 }
 
 extern "C" int kvc_buffer_sizes(int64_t tokens, int64_t hidden, int is_k, int64_t out[4]) {

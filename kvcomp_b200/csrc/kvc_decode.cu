@@ -162,10 +162,9 @@ static int decode_launch(const char *who, const uint8_t *encoded, int64_t encode
     const uint32_t slot_bytes = ((max_block + 15u + 15u) & ~15u) + 16u;
     const size_t smem = sizeof(DecodeSmem) + 4 * (size_t)slot_bytes + 4 * (size_t)TILE_BYTES;
     auto *kernel = values ? decode_kernel<true> : decode_kernel<false>;
-    KVC_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    KVC_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    static kvc_launch_slot slots[2];
     int occ = 0;
-    KVC_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 256, smem));
+    if (int rc = kvc_prepare(slots[values ? 1 : 0], reinterpret_cast<const void *>(kernel), 256, smem, &occ)) return rc;
     KVC_REQUIRE(occ >= 1, "%s: %zu bytes of shared memory do not fit an SM", who, smem);
     long long groups = (nblk + 3) / 4, cap = (long long)kvc_sm_count() * occ;
     unsigned grid = (unsigned)(groups < cap ? groups : cap);

@@ -37,13 +37,15 @@ def _five_d(t, name):
     return t
 
 
-def _timed(fn):
+def _timed(fn, status=None, what=None):
     """Run fn() between two CUDA events on the current stream; returns elapsed ms (the reference
-    returns cudaEventElapsedTime, kernels.cu:1026-1048)."""
+    returns cudaEventElapsedTime, kernels.cu:1026-1048).  status: fn's status word, read (and checked) with the same wait."""
     start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     start.record()
     fn()
     stop.record()
+    if status is not None:
+        ops.read_status(status, what=what)
     stop.synchronize()
     return start.elapsed_time(stop)
 
@@ -86,10 +88,11 @@ def _encode(is_k, input, encode_code_book, block_infos, thread_infos, idx_offset
     cols = input.shape[2] * input.shape[3]
     bsz, tsz, _, _ = ops.buffer_sizes(tokens, cols * 128, is_k)
     codes = input.contiguous().view(tokens, input.shape[2], input.shape[3], 128)
-    total, status = ops.encode(codes, is_k, encode_code_book, block_infos, thread_infos, encoded_data,
-                               base_offset=int(base_global_offset))
-    n = int(total[0].item())                       # synchronises, like the reference's cudaDeviceSynchronize
-    ops.read_status(status, what="entropy_encode")
+    report = ops.Report(codes.device)
+    ops.encode(codes, is_k, encode_code_book, block_infos, thread_infos, encoded_data,
+               base_offset=int(base_global_offset), total=report.total, status=report.enc_status)
+    n, _, _, flags = report.read()                 # synchronises, like the reference's cudaDeviceSynchronize
+    ops.check_flags(flags, what="entropy_encode")
     if idx_offset is not None and idx_offset.numel() >= 8:     # the reference's cursor: {blocks, bytes}
         idx_offset.view(torch.int32)[:2] = torch.tensor([bsz // 8, n], dtype=torch.int32, device=idx_offset.device)
     return encoded_data[:n], block_infos.view(torch.uint8)[:bsz], thread_infos.view(torch.uint8)[:tsz]
@@ -116,8 +119,7 @@ def _decode(is_k, in_tensor, block_infos, thread_infos, decode_code_book, out, h
     status = ops.new_status(out.device)
     codes = out.view(tokens, out.shape[2], out.shape[3], out.shape[4])
     ms = _timed(lambda: ops.decode(in_tensor, block_infos, thread_infos, book, tokens, out.shape[2], out.shape[3],
-                                   is_k, out=codes, status=status))
-    ops.read_status(status, what="entropy_decode")
+                                   is_k, out=codes, status=status), status, "entropy_decode")
     return ms
 
 
@@ -156,8 +158,7 @@ def k_decode_and_mat_vec_mul_cuda_export(decode_code_book, block_infos, thread_i
     spec = _ref_spec(True, mi.numel(), ctx, batch, head_num)
     cache = ops.make_cache(encoded_data, block_infos, thread_infos, book, mi, sc, spec)
     status = ops.new_status(C.device)
-    ms = _timed(lambda: ops.fused_qk(cache, ctx, batch, head_num, B, out=C, status=status))
-    ops.read_status(status, what="k_decode_and_mat_vec_mul")
+    ms = _timed(lambda: ops.fused_qk(cache, ctx, batch, head_num, B, out=C, status=status), status, "k_decode_and_mat_vec_mul")
     return ms
 
 
@@ -175,8 +176,7 @@ def v_decode_and_mat_vec_mul_cuda_export(decode_code_book, block_infos, thread_i
     spec = _ref_spec(False, mi.numel(), ctx, batch, head_num)
     cache = ops.make_cache(encoded_data, block_infos, thread_infos, book, mi, sc, spec)
     status = ops.new_status(C.device)
-    ms = _timed(lambda: ops.fused_pv(cache, ctx, batch, head_num, B, out=C, status=status))
-    ops.read_status(status, what="v_decode_and_mat_vec_mul")
+    ms = _timed(lambda: ops.fused_pv(cache, ctx, batch, head_num, B, out=C, status=status), status, "v_decode_and_mat_vec_mul")
     return ms
 
 

@@ -25,8 +25,8 @@ _get_device = getattr(torch._C, "_cuda_getDevice", None)
 
 def _stream():
     if _raw_stream is not None and _get_device is not None:
-        return C.c_void_p(_raw_stream(_get_device()))
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_get_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 class _on:
@@ -59,7 +59,7 @@ def _cuda(t, dtype, name):
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)
+    return t.data_ptr() if t is not None else None      # a plain number converts faster than a c_void_p object
 
 
 def new_status(device):
@@ -69,10 +69,31 @@ def new_status(device):
 
 def read_status(status, raise_on_fatal=True, what="kvcomp_b200"):
     """Synchronising read of a status word."""
-    v = int(status.item())
+    return check_flags(int(status.item()), raise_on_fatal, what)
+
+
+def check_flags(v, raise_on_fatal=True, what="kvcomp_b200"):
+    """The flags of a status word that is on the host already."""
     if raise_on_fatal and (v & _lib.FATAL_FLAGS):
         raise KvcError("%s: device reported %s" % (what, "|".join(_lib.flag_names(v))))
     return v
+
+
+class Report:
+    """What a store's kernels report -- the encoder's byte count and largest block, the quantiser's and the encoder's
+    status words -- in one zeroed int64[4] (and the histogram behind it), so that one copy brings all of it to the host."""
+    __slots__ = ("words", "hist", "total", "quant_status", "enc_status")
+
+    def __init__(self, device, with_hist=False):
+        buf = torch.zeros(260 if with_hist else 4, dtype=torch.int64, device=device)
+        self.words, self.hist = (buf[:4], buf[4:]) if with_hist else (buf, None)
+        self.total = buf[:2]
+        half = buf[2:4].view(torch.int32)
+        self.quant_status, self.enc_status = half[0:1], half[2:3]
+
+    def read(self):
+        """(bytes, largest block, quantiser flags, encoder flags); synchronises."""
+        return self.words.tolist()
 
 
 @dataclass
