@@ -5,7 +5,8 @@
 // v_huffman_decode_and_mat_vec_mul (kernels.cu:778-861); attention semantics of
 // eager_attention_forward (models/llama.py:211-234).
 //
-// Work layout (all three kernels): CTA = 256 threads working on 256 tokens of one (b, kv head).
+// Work layout (grouped queries in the attention kernel: see attn_rows_kernel): CTA = 256 threads working on 256 tokens
+// of one (b, kv head).
 //   K phase: thread = token; its vector holds the token's 128 channel codes.
 //            score = sum_c code_c * w[c] + zp, with w[c] = q[c]*scale[c] staged per 64-token block
 //            (dequantisation folded into the weights, the min_int term summed once per block).
@@ -84,17 +85,16 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 // wavefronts.  So a thread first decodes its vector into a private row of bytes in shared memory; then the
 // 32 rows of a warp are a 32 x 128 matrix of unsigned bytes, the weights of up to 8 heads a 128 x 8 matrix of
 // hi bytes and one of lo bytes, and m16n8k32 integer instructions multiply them.  The integer sums are the
-// same as in the one-pass form.  What bounds it: two CTAs of eight warps fit an SM (tables, slots, rows), 0.55
-// instructions issue per cycle and scheduler, half of the shared-memory pipe's wavefronts are used.  Against byte
-// stores and four dp4a pairs per word (one layer, rel 0.05 / 0.1): 16 sequences x 32768 tokens, 8 x 4 heads, 981 -> 836 us,
-// 1777 -> 1000 shared-memory wavefronts per warp and tile; 3 x 2881 tokens, 4 x 6 heads, 46 -> 31 us.
+// same as in the one-pass form.  What bounds it is the issue rate: the chains of dependent lookups leave slots empty, and
+// shared memory (tables, slots, rows) limits an SM to 16 or 20 warps.  Against byte stores and four dp4a pairs per word:
+// 1777 -> 1000 shared-memory wavefronts per warp and 256 tokens.  One layer of 16 sequences x 32768 tokens, 8 x 4 heads,
+// rel 0.05 / 0.1: 981 us -> 822 us with the rows in two CTAs of 256 threads -> 735 us with attn_rows_kernel's workers.
 // Rows of 36 words: 128 symbols, the overrun of paired lookups, and a 16-byte alignment at which the fragment
 // loads (16 bytes of row 4r+i by lane 4r+q) touch every bank once per quarter warp.
 constexpr int ROW_WORDS = 36;
 static_assert(ROW_WORDS * 4 >= 128 + KVC_DECODE_OVERRUN_PAIR + 3, "rows too short for paired lookups");
 constexpr int WROW = 136;                 // weight words per vector of the one-pass form: 128 positions + zeroed overrun
-// weight words of one vector: rows form [hi | lo][G][32 groups of 4 positions], one-pass form w_hi / w_lo
-template <int G, bool ROWS> struct VecWords { static constexpr int value = ROWS ? 2 * G * 32 : 2 * WROW * G; };
+__host__ __device__ constexpr int VEC_ROWS_WORDS(int G) { return 2 * G * 32; }     // weight words of one vector: [hi | lo][G][32 groups of 4 positions]
 // word of head g and position group w in the rows form: 16-byte chunks swizzled by the head, so that neither the
 // fragment loads (two heads x four chunks per quarter warp) nor the V phase's stores meet in a bank more than twice
 __device__ __forceinline__ uint32_t w_rows(uint32_t g, uint32_t w) { return g * 32u + (w ^ ((((g & 1u) << 2) | (g >> 1)) << 2)); }
@@ -309,7 +309,7 @@ __device__ __forceinline__ void k_weights_build(uint32_t *w, float *step, float 
         int q4[7];
 #pragma unroll
         for (int i = 0; i < 4; i++) q4[i] = __float2int_rn(wv[i] * inv);
-        uint32_t *row = w + (size_t)sub * VecWords<G, false>::value;
+        uint32_t *row = w + (size_t)sub * 2 * WROW * G;
 #pragma unroll
         for (int i = 0; i < 3; i++) {                           // the next lane's first three values
             int nv = __shfl_down_sync(0xffffffffu, q4[i], 1);
@@ -325,19 +325,19 @@ __device__ __forceinline__ void k_weights_build(uint32_t *w, float *step, float 
     }
 }
 
-// The same in the rows form: qh holds the query heads' fp16 bits [G][128]; lane = 4 consecutive channels = one word.
+// The same in the rows form, for block `sub` and the heads part * G/2 .. + G/2 - 1: qh holds the query heads' fp16 bits
+// [G][128]; lane = 4 consecutive channels = one word.
 template <int G>
 __device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *zp, const uint16_t *qh, float scaling,
-                                               const KUnit &u, bool channel_units, int min_bytes, bool live, int tid) {
-    const int lane = tid & 31, wp = tid >> 5, sub = wp & 3;
+                                               const KUnit &u, bool channel_units, int min_bytes, int sub, int part, int lane) {
     float sc[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) sc[i] = kvc_scale_value(ku_scale(u, i));
 #pragma unroll
     for (int gi = 0; gi < G / 2; gi++) {
-        const int g = (wp >> 2) * (G / 2) + gi;
+        const int g = part * (G / 2) + gi;
         const uint2 qb = *reinterpret_cast<const uint2 *>(qh + g * 128 + lane * 4);
-        const uint32_t q2[2] = {live ? qb.x : 0u, live ? qb.y : 0u};
+        const uint32_t q2[2] = {qb.x, qb.y};
         float wv[4], z = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -349,7 +349,7 @@ __device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *
         z = channel_units ? kvc_warp_sum(z) : 0.f;
         const float st = fix_step(mx), inv = st > 0.f ? 1.0f / st : 0.f;
         const uint2 r = pack4_dense(__float2int_rn(wv[0] * inv), __float2int_rn(wv[1] * inv), __float2int_rn(wv[2] * inv), __float2int_rn(wv[3] * inv));
-        uint32_t *vec = w + sub * VecWords<G, true>::value;
+        uint32_t *vec = w + sub * VEC_ROWS_WORDS(G);
         vec[w_rows(g, lane)] = r.x; vec[G * 32 + w_rows(g, lane)] = r.y;
         if (lane == 0) { step[sub * G + g] = st; zp[sub * G + g] = z; }
     }
@@ -432,7 +432,7 @@ __device__ __forceinline__ void v_weights(uint32_t *ps, float *vstep, float *red
 #pragma unroll
     for (int g = 0; g < G; g++) {
         const int16_t *qq = q16 + (grp * G + g) * 132 + tl;
-        uint32_t *row = ps + (size_t)grp * VecWords<G, false>::value;    // layout: w_hi / w_lo
+        uint32_t *row = ps + (size_t)grp * 2 * WROW * G;    // layout: w_hi / w_lo
         const uint2 r = pack4(qq[0], qq[1], qq[2], qq[3]);
         row[w_hi<G>(tl, g)] = r.x; row[w_lo<G>(tl, g)] = r.y;
         if (tl < WROW - 128) { row[w_hi<G>(128 + tl, g)] = 0u; row[w_lo<G>(128 + tl, g)] = 0u; }
@@ -558,18 +558,16 @@ __global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T
 }
 
 // ---- one-pass decode attention -------------------------------------------------------------------
-struct LutSmem { uint32_t lut[KVC_LUT_SIZE]; };        // rows form: the trees stay in global memory, shared memory decides how many CTAs fit
 template <int G>
 struct alignas(32) AttnSmem {                     // followed in shared memory by 4 K slots, 4 V slots (sized at launch),
-    typename std::conditional<(G >= 2), LutSmem, KvcBookSmem>::type bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
-    // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum, in the rows form by the V weight words
-    alignas(32) uint32_t w[4 * VecWords<G, (G >= 2)>::value];
-    alignas(32) uint32_t ps[G >= 2 ? 8 : 2 * VecWords<G, false>::value];    // V weight words (one-pass form)
-    alignas(16) float red[4][8 * G];  // per-warp max, sum, zpv and weight-max partials
-    alignas(16) float q[G >= 2 ? G * 64 : 128];   // the query: scaled values, in the rows form fp16 bits [G][128]
+    KvcBookSmem bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
+    alignas(32) uint32_t w[4 * 2 * WROW * G];     // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum
+    alignas(32) uint32_t ps[2 * 2 * WROW * G];    // V weight words
     float kstep[4 * G], zp[4 * G];
-    float vstep[2];
+    float vstep[2 * G];
+    float qf[G * 128];
     float qsum[G];
+    float red[4][8 * G];              // per-warp max, sum, zpv and weight-max partials
     uint64_t bar[2];                  // K and V staging barriers
     uint32_t leadK[4], leadV[4];
     uint32_t nbK[4], nbV[4];          // byte counts of the staged blocks
@@ -599,20 +597,14 @@ struct AttnParams {
     int starve;                   // tests of the bounded waits only: announce bytes that are never copied
 };
 
-// BULK: stage with bulk asynchronous copies (one tile phase ahead) instead of plain loads.
+// One query head per KV head (G = 1).  BULK: stage with bulk asynchronous copies (one tile phase ahead) instead of plain loads.
 template <int G, bool BULK>
-__global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnParams p) {
+__global__ void __launch_bounds__(NTHR, 3) attn_decode_kernel(AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnSmem<G> &sm = *reinterpret_cast<AttnSmem<G> *>(smem_raw);
     uint8_t *const slotsK = smem_raw + sizeof(AttnSmem<G>), *const slotsV = slotsK + 4 * p.slotK_bytes;
-    constexpr bool ROWS = G >= 2;                          // grouped queries: decode into rows, multiply afterwards
-    // rows form: the rows lie behind the slots and are their padding too
-    const uint32_t rows_s = kvc_smem_addr(slotsV + 4 * p.slotV_bytes), warp_rows_s = rows_s + (threadIdx.x & ~31u) * (ROW_WORDS * 4);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
     const int grp = tid >> 7, ch = tid & 127;
-    // rows form: the lane's two heads and its four neighbouring rows (tokens in the K phase, channels in the V phase)
-    const int h2 = (2 * (lane & 3)) % G, r4 = lane & ~3;
-    const bool own = 2 * (lane & 3) < G;                   // with fewer than 8 heads the other lanes hold copies
     // Launched with programmatic stream serialisation.  This kernel's own set-up -- the books' tables, the first
     // blocks, the first tile's metadata: cache data that no kernel of a decode step writes -- runs before
     // griddepcontrol.wait, i.e. possibly while the kernel ahead of it in the stream (the merge of the layer
@@ -672,8 +664,8 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
     }
     bool escK = false, escV = false;
     if (p.T > 0) {                                         // (no streams at all while nothing is compressed yet)
-        if constexpr (ROWS) { kvc_load_lut(sm.bookK.lut, p.k.book, tid, NTHR); kvc_load_lut(sm.bookV.lut, p.v.book, tid, NTHR); }
-        else { kvc_load_book(sm.bookK, p.k.book, tid, NTHR); kvc_load_book(sm.bookV, p.v.book, tid, NTHR); }
+        kvc_load_book(sm.bookK, p.k.book, tid, NTHR);
+        kvc_load_book(sm.bookV, p.v.book, tid, NTHR);
         escK = book_has_long_codes(p.k.book); escV = book_has_long_codes(p.v.book);
     }
 
@@ -709,17 +701,14 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
         for (int i = 0; i < QN; i++) {
             const int idx = tid + i * NTHR;
             qn[i] = 0;
-            if (idx < (ROWS ? p.nh * 128 : 128)) qn[i] = reinterpret_cast<const unsigned short *>(p.q)[(row0 + (idx >> 7)) * 128 + (idx & 127)];
+            if (idx < G * 128) qn[i] = reinterpret_cast<const unsigned short *>(p.q)[(row0 + (idx >> 7)) * 128 + (idx & 127)];
         }
     };
     auto q_store = [&]() {
 #pragma unroll
         for (int i = 0; i < QN; i++) {
             const int idx = tid + i * NTHR;
-            if (idx < G * 128) {
-                if (ROWS) reinterpret_cast<unsigned short *>(sm.q)[idx] = qn[i];
-                else sm.q[idx] = kvc_scale_value(qn[i]) * p.scaling;
-            }
+            if (idx < G * 128) sm.qf[idx] = kvc_scale_value(qn[i]) * p.scaling;
         }
     };
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -732,26 +721,11 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
     if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
     q_store();                                             // fetched during the previous item's last tile
     __syncthreads();
-    if constexpr (ROWS) {                                  // sum of each query head's 128 (scaled) values
-        const unsigned short *qh = reinterpret_cast<const unsigned short *>(sm.q);
-        if (warp < G) {
-            float a = 0.f;
-#pragma unroll
-            for (int k = 0; k < 4; k++) a += kvc_scale_value(qh[warp * 128 + k * 32 + lane]) * p.scaling;
-            a = kvc_warp_sum(a);
-            if (lane == 0) sm.qsum[warp] = a;
-        }
-    } else q_sums<1>(sm.q, sm.qsum, tid);
+    q_sums<G>(sm.qf, sm.qsum, tid);
     __syncthreads();                                       // books, q and (unbuffered) slots are in place
-    // running maximum, sum and output: of the one head and the thread's channel, or of the lane's two heads and four channels
-    constexpr int NH = ROWS ? 2 : 1, NC = ROWS ? 4 : 1;
-    float m_run[NH], l_run[NH], acc[NC][NH];
+    float m_run[G], l_run[G], acc[G];
 #pragma unroll
-    for (int j = 0; j < NH; j++) {
-        m_run[j] = -CUDART_INF_F; l_run[j] = 0.f;
-#pragma unroll
-        for (int i = 0; i < NC; i++) acc[i][j] = 0.f;
-    }
+    for (int g = 0; g < G; g++) { m_run[g] = -CUDART_INF_F; l_run[g] = 0.f; acc[g] = 0.f; }
 
     for (int tile = it.t_lo; tile < it.t_hi; tile++) {
         const long long tok0 = (long long)tile * 256, t = tok0 + tid;
@@ -769,8 +743,7 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
             if (actK) { uint32_t ld, nb; bool ok = stage(p.k, blkK, slotsK + sub * p.slotK_bytes, &ld, &nb, v); if (v == 0) { sm.leadK[sub] = ld; sm.nbK[sub] = nb; sm.okK[sub] = ok; } }
             if (actV) { uint32_t ld, nb; bool ok = stage(p.v, blkV, slotsV + sub * p.slotV_bytes, &ld, &nb, v); if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; } }
         }
-        if constexpr (ROWS) k_weights_rows<G>(sm.w, sm.kstep, sm.zp, reinterpret_cast<const uint16_t *>(sm.q), p.scaling, cur.ku, km.sc != 0, km.min_bytes, tok0 + (warp & 3) * 64 < T, tid);
-        else k_weights_build<1>(sm.w, sm.kstep, sm.zp, sm.q, cur.ku, km.sc != 0, km.min_bytes, tok0, T, tid);
+        k_weights_build<G>(sm.w, sm.kstep, sm.zp, sm.qf, cur.ku, km.sc != 0, km.min_bytes, tok0, T, tid);
         // A wait that runs out: the thread does not decode.  The warp that issues the copies looks at its own
         // verdict: a barrier whose phase it did not see complete is never armed again (a second arrival on an
         // open phase is an error), and the CTA is marked; it takes no further item, and what it had in flight
@@ -782,61 +755,25 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
         }
         __syncthreads();
         // ---- K: scores of this tile's tokens
-        float s[NC][NH];
-        if (actK) {                                        // the same for a whole warp
-            bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
-            const uint32_t posK = sm.leadK[sub] + (cur.startK >> 3);
-            if constexpr (ROWS) {
-                if (ok) ok = decode_row(kvc_smem_addr(slotsK + sub * p.slotK_bytes), posK, kvc_smem_addr(sm.bookK.lut), p.k.book, escK, rows_s + tid * (ROW_WORDS * 4));
-                __syncwarp();
-                int d[4][2];
-                rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + sub * VecWords<G, true>::value), lane, d);
-                const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the thread's own token
-                const float2 st = *reinterpret_cast<const float2 *>(&sm.kstep[sub * G + h2]), z = *reinterpret_cast<const float2 *>(&sm.zp[sub * G + h2]);
+        float s[G];
+        if (actK) {
+            int hi[G], lo[G];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    s[i][0] = st.x * (float)d[i][0]; s[i][NH - 1] = st.y * (float)d[i][1];
-                    if (km.sc != 0) { s[i][0] += z.x; s[i][NH - 1] += z.y; }
-                    else {
-                        const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
-                        const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
-                        s[i][0] = sc * fmaf(mi, sm.qsum[h2], s[i][0]); s[i][NH - 1] = sc * fmaf(mi, sm.qsum[h2 + NH - 1], s[i][NH - 1]);
-                    }
-                }
-            } else {
-                int hi[1] = {0}, lo[1] = {0};
-                if (ok) ok = decode_dot<1>(slotsK + sub * p.slotK_bytes, posK, sm.bookK, escK, sm.w + sub * VecWords<1, false>::value, hi, lo);
-                k_finish<1>(s[0], hi, lo, sm.kstep + sub, sm.zp + sub, sm.qsum, km.sc != 0, kvc_scale_value(cur.ksc), (float)cur.kmi);
+            for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
+            bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
+            if (ok) {
+                ok = decode_dot<G>(slotsK + sub * p.slotK_bytes, sm.leadK[sub] + (cur.startK >> 3), sm.bookK, escK, sm.w + sub * 2 * WROW * G, hi, lo);
             }
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+            k_finish<G>(s, hi, lo, sm.kstep + sub * G, sm.zp + sub * G, sm.qsum, km.sc != 0, kvc_scale_value(cur.ksc), (float)cur.kmi);
         } else {
 #pragma unroll
-            for (int i = 0; i < NC; i++)
-#pragma unroll
-                for (int j = 0; j < NH; j++) s[i][j] = -CUDART_INF_F;
+            for (int g = 0; g < G; g++) s[g] = -CUDART_INF_F;
         }
         // ---- online softmax over the tile
-        // over a warp's tokens: in the rows form the lane's four, then the eight lanes with the same heads
-        auto warp_max = [&](float x) { if constexpr (ROWS) { x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4)); x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8)); return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16)); } else return kvc_warp_max(x); };
-        auto warp_sum = [&](float x) { if constexpr (ROWS) { x += __shfl_xor_sync(0xffffffffu, x, 4); x += __shfl_xor_sync(0xffffffffu, x, 8); return x + __shfl_xor_sync(0xffffffffu, x, 16); } else return kvc_warp_sum(x); };
-        auto red_put = [&](int k, const float (&x)[NH]) {      // the warp's value of each head
-            if constexpr (ROWS) { if (lane < G / 2) *reinterpret_cast<float2 *>(&sm.red[k][warp * G + h2]) = make_float2(x[0], x[NH - 1]); }
-            else if (lane == 0) sm.red[k][warp] = x[0];
-        };
-        auto red_get = [&](int k, int w8, float (&x)[NH]) {
-            if constexpr (ROWS) { const float2 v2 = *reinterpret_cast<const float2 *>(&sm.red[k][w8 * G + h2]); x[0] = v2.x; x[NH - 1] = v2.y; }
-            else x[0] = sm.red[k][w8];
-        };
-        float t1[NH], t2[NH];
 #pragma unroll
-        for (int j = 0; j < NH; j++) {
-            t1[j] = s[0][j];
-#pragma unroll
-            for (int i = 1; i < NC; i++) t1[j] = fmaxf(t1[j], s[i][j]);
-            t1[j] = warp_max(t1[j]);
-        }
-        red_put(0, t1);
-        __syncthreads();                                   // also: every thread is done with the K slots and weights
+        for (int g = 0; g < G; g++) { float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
+        __syncthreads();                                   // also: every thread is done with the K slots
         // the next tile's per-thread metadata is asked for now and first touched when that tile begins: it is in
         // flight during the V phase only, and the K decode above ran without its registers
         load_meta(n_on, n_col, n_tile, nxt);
@@ -845,115 +782,53 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
                 stage_bulk(p.k, validK(n_on, n_tile, lane & 3), blkK_of(n_col, n_tile, lane & 3), slotsK + (lane & 3) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0);
             else if (lane == 0) sm.dead = 1;
         }
-        float alpha[NH], vst[NH];
-        red_get(0, 0, t1);
+        float alpha[G], wv[G];
 #pragma unroll
-        for (int w8 = 1; w8 < 8; w8++) {
-            red_get(0, w8, t2);
+        for (int g = 0; g < G; g++) {
+            float mt = sm.red[0][g];
 #pragma unroll
-            for (int j = 0; j < NH; j++) t1[j] = fmaxf(t1[j], t2[j]);
+            for (int w8 = 1; w8 < 8; w8++) mt = fmaxf(mt, sm.red[0][w8 * G + g]);
+            const float m_new = fmaxf(m_run[g], mt);
+            alpha[g] = __expf(m_run[g] - m_new);           // exp(-inf) = 0 on the first tile
+            const float pr = actK ? __expf(s[g] - m_new) : 0.f;
+            m_run[g] = m_new;
+            wv[g] = pr * kvc_scale_value(cur.vsc);
+            const float ssum = kvc_warp_sum(pr), zsum = kvc_warp_sum(wv[g] * (float)cur.vmi);
+            if (lane == 0) { sm.red[1][warp * G + g] = ssum; sm.red[2][warp * G + g] = zsum; }
         }
+        // (the K weights are spent: their memory is the scratch of the V weights' 16-bit values)
+        v_weights<G>(sm.ps, sm.vstep, sm.red[3], reinterpret_cast<int16_t *>(sm.w), wv, tid);      // three barriers inside
 #pragma unroll
-        for (int j = 0; j < NH; j++) {
-            const float m_new = fmaxf(m_run[j], t1[j]);
-            alpha[j] = __expf(m_run[j] - m_new);           // exp(-inf) = 0 on the first tile
-            m_run[j] = m_new;
+        for (int g = 0; g < G; g++) {
+            float lt = 0.f;
+#pragma unroll
+            for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + g];
+            l_run[g] = l_run[g] * alpha[g] + lt;
         }
-        if constexpr (ROWS) {
-            float wv[4][2], ssum[2] = {0.f, 0.f}, zsum[2] = {0.f, 0.f}, wmax[2] = {0.f, 0.f};
-            const uint32_t unit = (uint32_t)cur.vsc | ((uint32_t)cur.vmi << 16);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
-                const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const float pr = actK ? __expf(s[i][j] - m_run[j]) : 0.f;
-                    wv[i][j] = pr * sc;
-                    ssum[j] += pr; zsum[j] = fmaf(wv[i][j], mi, zsum[j]); wmax[j] = fmaxf(wmax[j], fabsf(wv[i][j]));
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 2; j++) { ssum[j] = warp_sum(ssum[j]); zsum[j] = warp_sum(zsum[j]); wmax[j] = warp_max(wmax[j]); }
-            red_put(1, ssum); red_put(2, zsum); red_put(3, wmax);
-            __syncthreads();
-            // the V weights' words: the lane's four tokens are one word of each of its heads
-            red_get(3, grp * 4, t1);
-#pragma unroll
-            for (int w4 = 1; w4 < 4; w4++) {
-                red_get(3, grp * 4 + w4, t2);
-                t1[0] = fmaxf(t1[0], t2[0]); t1[1] = fmaxf(t1[1], t2[1]);
-            }
-            uint32_t *vec = sm.w + grp * VecWords<G, true>::value;         // the K weights are spent
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                vst[j] = fix_step(t1[j]);
-                const float inv = vst[j] > 0.f ? 1.0f / vst[j] : 0.f;
-                const uint2 w2 = pack4_dense(__float2int_rn(wv[0][j] * inv), __float2int_rn(wv[1][j] * inv), __float2int_rn(wv[2][j] * inv), __float2int_rn(wv[3][j] * inv));
-                const uint32_t at = w_rows(h2 + j, (warp & 3) * 8 + (lane >> 2));
-                if (own) { vec[at] = w2.x; vec[G * 32 + at] = w2.y; }
-            }
-            __syncthreads();
-        } else {
-            float wv[1];
-            const float pr = actK ? __expf(s[0][0] - m_run[0]) : 0.f;
-            wv[0] = pr * kvc_scale_value(cur.vsc);
-            const float ssum = kvc_warp_sum(pr), zsum = kvc_warp_sum(wv[0] * (float)cur.vmi);
-            if (lane == 0) { sm.red[1][warp] = ssum; sm.red[2][warp] = zsum; }
-            // (the K weights are spent: their memory is the scratch of the V weights' 16-bit values)
-            v_weights<1>(sm.ps, sm.vstep, sm.red[3], reinterpret_cast<int16_t *>(sm.w), wv, tid);      // three barriers inside
-        }
-        red_get(1, 0, t1);
-#pragma unroll
-        for (int w8 = 1; w8 < 8; w8++) {
-            red_get(1, w8, t2);
-#pragma unroll
-            for (int j = 0; j < NH; j++) t1[j] += t2[j];
-        }
-#pragma unroll
-        for (int j = 0; j < NH; j++) l_run[j] = l_run[j] * alpha[j] + t1[j];
         const bool v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
         if (BULK && v_landed) par ^= 2u;
         if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
-        // ---- V: accumulate this tile's contribution for the thread's (group, channels)
-        float dv[NC][NH];
+        // ---- V: accumulate this tile's contribution for the thread's (group, channel)
+        float dv[G];
 #pragma unroll
-        for (int i = 0; i < NC; i++)
+        for (int g = 0; g < G; g++) dv[g] = 0.f;
+        if (actV) {
+            int hi[G], lo[G];
 #pragma unroll
-            for (int j = 0; j < NH; j++) dv[i][j] = 0.f;
-        if (actV) {                                        // the same for a whole warp
+            for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
             bool ok = v_landed && sm.okV[sub] && (uint32_t)(cur.startV >> 3) < sm.nbV[sub];
-            const uint32_t posV = sm.leadV[sub] + (cur.startV >> 3);
-            float z[NH];
-            auto zero_points = [&]() {                     // of the group's four warps
-#pragma unroll
-                for (int w4 = 0; w4 < 4; w4++) {
-                    float x[NH];
-                    red_get(2, grp * 4 + w4, x);
-#pragma unroll
-                    for (int j = 0; j < NH; j++) z[j] = w4 ? z[j] + x[j] : x[j];
-                }
-            };
-            if constexpr (ROWS) {
-                if (ok) ok = decode_row(kvc_smem_addr(slotsV + sub * p.slotV_bytes), posV, kvc_smem_addr(sm.bookV.lut), p.v.book, escV, rows_s + tid * (ROW_WORDS * 4));
-                __syncwarp();
-                int d[4][2];
-                rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + grp * VecWords<G, true>::value), lane, d);
-                zero_points();
-#pragma unroll
-                for (int i = 0; i < 4; i++) { dv[i][0] = fmaf(vst[0], (float)d[i][0], z[0]); dv[i][NH - 1] = fmaf(vst[NH - 1], (float)d[i][1], z[NH - 1]); }
-            } else {
-                int hi[1] = {0}, lo[1] = {0};
-                if (ok) ok = decode_dot<1>(slotsV + sub * p.slotV_bytes, posV, sm.bookV, escV, sm.ps + grp * VecWords<1, false>::value, hi, lo);
-                zero_points();
-                dv[0][0] = fix_value(sm.vstep[grp], hi[0], lo[0]) + z[0];
+            if (ok) {
+                ok = decode_dot<G>(slotsV + sub * p.slotV_bytes, sm.leadV[sub] + (cur.startV >> 3), sm.bookV, escV, sm.ps + grp * 2 * WROW * G, hi, lo);
             }
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+#pragma unroll
+            for (int g = 0; g < G; g++)
+                dv[g] = fix_value(sm.vstep[grp * G + g], hi[g], lo[g]) +
+                        sm.red[2][(grp * 4 + 0) * G + g] + sm.red[2][(grp * 4 + 1) * G + g] +
+                        sm.red[2][(grp * 4 + 2) * G + g] + sm.red[2][(grp * 4 + 3) * G + g];
         }
 #pragma unroll
-        for (int i = 0; i < NC; i++)
-#pragma unroll
-            for (int j = 0; j < NH; j++) acc[i][j] = fmaf(acc[i][j], alpha[j], dv[i][j]);
+        for (int g = 0; g < G; g++) acc[g] = fmaf(acc[g], alpha[g], dv[g]);
         __syncthreads();                                   // every thread is done with the V slots, weights and sums
         if (BULK && warp == 0) {                           // next tile's V blocks land during its K phase
             if (__all_sync(0xffffffffu, v_landed))
@@ -976,7 +851,6 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
             for (int g = 0; g < G; g++) s[g] = act ? 0.f : -CUDART_INF_F;
             if (act) {
                 const __half *kr = p.ktail + ((r * B + b) * Hkv + h) * 128;
-#pragma unroll 1
                 for (int c8 = 0; c8 < 16; c8++) {
                     uint4 kv = *reinterpret_cast<const uint4 *>(kr + c8 * 8);
                     const __half *kh = reinterpret_cast<const __half *>(&kv);
@@ -984,59 +858,47 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
                     for (int k = 0; k < 8; k++) {
                         const float kf = __half2float(kh[k]);
 #pragma unroll
-                        for (int g = 0; g < G; g++) {
-                            const int at = g * 128 + c8 * 8 + k;
-                            const float qv = ROWS ? kvc_scale_value(reinterpret_cast<const unsigned short *>(sm.q)[at]) * p.scaling : sm.q[at];
-                            s[g] = fmaf(kf, qv, s[g]);
-                        }
+                        for (int g = 0; g < G; g++) s[g] = fmaf(kf, sm.qf[g * 128 + c8 * 8 + k], s[g]);
                     }
                 }
             }
 #pragma unroll
-            for (int g = 0; g < G; g++) { const float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
+            for (int g = 0; g < G; g++) { float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
             __syncthreads();
-            float alpha[NH], dv[NC][NH];
+            float alpha[G];
 #pragma unroll
-            for (int j = 0; j < NH; j++) {
-                const int g = ROWS ? h2 + j : 0;
+            for (int g = 0; g < G; g++) {
                 float mt = sm.red[0][g];
 #pragma unroll
                 for (int w8 = 1; w8 < 8; w8++) mt = fmaxf(mt, sm.red[0][w8 * G + g]);
-                const float m_new = fmaxf(m_run[j], mt);
-                alpha[j] = __expf(m_run[j] - m_new);
-                m_run[j] = m_new;
-                if (ROWS && tid < 4) sm.red[3][g] = m_new;
-#pragma unroll
-                for (int i = 0; i < NC; i++) dv[i][j] = 0.f;
-            }
-            if (ROWS) __syncthreads();
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                const float pr = act ? __expf(s[g] - (ROWS ? sm.red[3][g] : m_run[0])) : 0.f;
+                const float m_new = fmaxf(m_run[g], mt);
+                alpha[g] = __expf(m_run[g] - m_new);
+                const float pr = act ? __expf(s[g] - m_new) : 0.f;
+                m_run[g] = m_new;
                 pt[tid * G + g] = pr;
                 const float ssum = kvc_warp_sum(pr);
                 if (lane == 0) sm.red[1][warp * G + g] = ssum;
             }
             __syncthreads();
-            // the thread's channel, or the lane's four, over rows r0 + 128*grp .. +127
+            float dv[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                float lt = 0.f;
+#pragma unroll
+                for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + g];
+                l_run[g] = l_run[g] * alpha[g] + lt;
+                dv[g] = 0.f;
+            }
+            // thread (grp, ch) sums rows r0 + 128*grp .. +127 of its channel
             for (int i = 0; i < 128; i++) {
                 const long long rr = r0 + grp * 128 + i;
                 if (rr >= p.Tr) break;
-                const __half *vr = p.vtail + ((rr * B + b) * Hkv + h) * 128 + (ROWS ? (warp & 3) * 32 + r4 : ch);
+                const float vf = __half2float(p.vtail[((rr * B + b) * Hkv + h) * 128 + ch]);
 #pragma unroll
-                for (int c = 0; c < NC; c++)
-#pragma unroll
-                    for (int j = 0; j < NH; j++) dv[c][j] = fmaf(pt[(grp * 128 + i) * G + (ROWS ? h2 + j : 0)], __half2float(vr[c]), dv[c][j]);
+                for (int g = 0; g < G; g++) dv[g] = fmaf(pt[(grp * 128 + i) * G + g], vf, dv[g]);
             }
 #pragma unroll
-            for (int j = 0; j < NH; j++) {
-                float lt = 0.f;
-#pragma unroll
-                for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + (ROWS ? h2 + j : 0)];
-                l_run[j] = l_run[j] * alpha[j] + lt;
-#pragma unroll
-                for (int c = 0; c < NC; c++) acc[c][j] = fmaf(acc[c][j], alpha[j], dv[c][j]);
-            }
+            for (int g = 0; g < G; g++) acc[g] = fmaf(acc[g], alpha[g], dv[g]);
         }
     }
     if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without tiles fetched nothing yet
@@ -1044,38 +906,23 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
     if (!p.partial) {
         // ---- the item is the whole column: combine the CTA's two token groups and write the output
         __syncthreads();
-        float *sumbuf = reinterpret_cast<float *>(sm.w);       // [128][G]
-        const int c0 = ROWS ? (warp & 3) * 32 + r4 : ch;       // the first of the thread's channels
-        if (grp == 1 && (own || !ROWS)) {
+        float *sumbuf = reinterpret_cast<float *>(sm.w);       // [2][128][G]
 #pragma unroll
-            for (int i = 0; i < NC; i++)
-#pragma unroll
-                for (int j = 0; j < NH; j++) sumbuf[(c0 + i) * G + (ROWS ? h2 + j : 0)] = acc[i][j];
-        }
+        for (int g = 0; g < G; g++) sumbuf[(grp * 128 + ch) * G + g] = acc[g];
         __syncthreads();
-        if (grp == 0 && (own || !ROWS)) {
+        if (tid < 128) {
 #pragma unroll
-            for (int j = 0; j < NH; j++) {
-                const int g = ROWS ? h2 + j : 0;
-                if (g >= p.nh) continue;
-#pragma unroll
-                for (int i = 0; i < NC; i++)
-                    p.out[(head0 + g) * 128 + c0 + i] = __float2half_rn((acc[i][j] + sumbuf[(c0 + i) * G + g]) / l_run[j]);
-            }
-        }
-    } else if constexpr (ROWS) {
-        // ---- a partial result {m, l, -, -, acc of group 0 [128], acc of group 1 [128]}; a second kernel merges
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            if (!own || h2 + j >= p.nh) continue;
-            float *dst = p.ws_part + ((head0 + h2 + j) * p.splits + it.part) * ATTN_PART_FLOATS;
-            *reinterpret_cast<float4 *>(dst + 4 + grp * 128 + (warp & 3) * 32 + r4) = make_float4(acc[0][j], acc[1 % NC][j], acc[2 % NC][j], acc[3 % NC][j]);
-            if (warp == 0 && lane < 4) { dst[0] = m_run[j]; dst[1] = l_run[j]; }
+            for (int g = 0; g < G; g++)
+                p.out[(head0 + g) * 128 + tid] = __float2half_rn((sumbuf[tid * G + g] + sumbuf[(128 + tid) * G + g]) / l_run[g]);
         }
     } else {
-        float *dst = p.ws_part + (head0 * p.splits + it.part) * ATTN_PART_FLOATS;
-        dst[4 + tid] = acc[0][0];                              // tid = grp * 128 + ch
-        if (tid == 0) { dst[0] = m_run[0]; dst[1] = l_run[0]; }
+        // ---- a partial result {m, l, -, -, acc of group 0 [128], acc of group 1 [128]}; a second kernel merges
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            float *dst = p.ws_part + ((head0 + g) * p.splits + it.part) * ATTN_PART_FLOATS;
+            dst[4 + tid] = acc[g];                             // tid = grp * 128 + ch
+            if (tid == 0) { dst[0] = m_run[g]; dst[1] = l_run[g]; }
+        }
     }
     if (draw && tid == 0) sm.next_j = drawn;
     __syncthreads();                                       // the sums are read before the next column's weights overwrite them
@@ -1093,6 +940,376 @@ __global__ void __launch_bounds__(NTHR, G >= 2 ? 2 : 3) attn_decode_kernel(AttnP
     if (draw && tid == 0) {               // the last CTA to finish leaves the scheduling counters zeroed for the next launch
         __threadfence();
         if (atomicAdd(&p.sched[1], 1) == (int)gridDim.x - 1) { p.sched[0] = 0; p.sched[1] = 0; __threadfence(); }
+    }
+}
+
+// ---- grouped queries: the same attention with workers of 128 threads --------------------------------
+// A CTA is one resident per SM, with one copy of the two decode tables and up to five (eight heads: four) workers.
+// A worker is four warps with slots, rows, weights and barriers of its own; it draws items like a CTA of the one-head
+// kernel and walks them in steps of 128 tokens (two K blocks, the two V blocks of a column).  The tables take 32 KB
+// and a worker 35 to 45 KB: two CTAs of 256 threads with a copy each held four workers' worth of warps, and all eight
+// warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads; 448 and 404 us at
+// 32 x 16384 tokens, 4 x 2 heads).
+constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]; two of them take the room of one of the one-head kernel
+static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "the workspace is sized in the one-head kernel's partial results");
+template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : 5; }
+
+template <int G>
+struct alignas(32) RowsWorker {
+    uint32_t w[2 * VEC_ROWS_WORDS(G)];       // K weight words of the step's two blocks; then V weight words; scratch of the tail
+    float red[4][4 * G];                     // per-warp max, sum, zero-point and weight-max partials
+    unsigned short q[G * 128];               // the query, fp16 bits
+    float kstep[2 * G], zp[2 * G], qsum[G];
+    uint64_t bar[2];                         // K and V staging barriers
+    uint32_t leadK[4], leadV[4], nbK[4], nbV[4];   // of the two staged blocks (stage_bulk writes four entries)
+    int okK[4], okV[4];
+    int next_j, dead;
+};
+struct alignas(32) RowsTables { uint32_t lutK[KVC_LUT_SIZE], lutV[KVC_LUT_SIZE]; };   // the trees, for codes beyond the window, stay in global memory
+
+// shared memory of a CTA: tables, workers, slots (two of K and two of V each), rows; a corrupt stream's overrun ends in the rows
+template <int G> size_t rows_smem(const AttnParams &p, int workers) {
+    return sizeof(RowsTables) + workers * (sizeof(RowsWorker<G>) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes) + 128 * ROW_WORDS * 4);
+}
+
+template <int G, bool BULK>
+__global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(AttnParams p) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    RowsTables &tab = *reinterpret_cast<RowsTables *>(smem_raw);
+    const int workers = blockDim.x >> 7, wk = threadIdx.x >> 7;
+    const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
+    uint8_t *const wbase = smem_raw + sizeof(RowsTables), *const sbase = wbase + workers * sizeof(RowsWorker<G>);
+    RowsWorker<G> &sm = reinterpret_cast<RowsWorker<G> *>(wbase)[wk];
+    uint8_t *const slotsK = sbase + wk * 2 * (p.slotK_bytes + p.slotV_bytes), *const slotsV = slotsK + 2 * p.slotK_bytes;
+    const uint32_t rows_s = kvc_smem_addr(sbase + workers * 2 * (p.slotK_bytes + p.slotV_bytes)) + wk * (128 * ROW_WORDS * 4);
+    const uint32_t warp_rows_s = rows_s + warp * (32 * ROW_WORDS * 4), row_s = rows_s + tid * (ROW_WORDS * 4);
+    // the lane's two heads and its four neighbouring rows (tokens in the K phase, channels in the V phase)
+    const int h2 = (2 * (lane & 3)) % G, r4 = lane & ~3;
+    const bool own = 2 * (lane & 3) < G;                   // with fewer than 8 heads the other lanes hold copies
+    auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
+    // launched with programmatic stream serialisation, as the one-head kernel: set-up before griddepcontrol.wait reads
+    // cache data only
+    const int B = (int)p.B, Hkv = (int)p.Hkv, Hq = (int)p.Hq;
+    const int cols = B * Hkv, Gt = Hq / Hkv;
+    const kvc_qmeta_dev &km = p.k.q, &vm = p.v.q;
+    int flags = 0;
+
+    struct Item { int col, t_lo, t_hi, part; };            // steps t_lo .. t_hi - 1 of a column; part: the run's index
+    const bool draw = p.sched != nullptr;
+    const int P = (int)gridDim.x * workers, me = (int)blockIdx.x * workers + wk;
+    const int w_hi = draw ? (int)p.work : (int)(p.work * (me + 1) / P);
+    auto item_of = [&](int j, Item &it) -> bool {
+        if (j >= w_hi) return false;
+        const int n_long = cols * p.long_runs;
+        if (j < n_long) {
+            const int r = j % p.long_runs;
+            it.col = j / p.long_runs; it.part = r; it.t_lo = r * p.tiles_per_split; it.t_hi = min(p.n_tiles, it.t_lo + p.tiles_per_split);
+        } else {
+            const int n_short = p.splits - p.long_runs, r = (j - n_long) % n_short;
+            it.col = (j - n_long) / n_short; it.part = p.long_runs + r;
+            it.t_lo = p.long_runs * p.tiles_per_split + r * p.short_tiles; it.t_hi = min(p.n_tiles, it.t_lo + p.short_tiles);
+        }
+        return true;
+    };
+    auto blkK_of = [&](int col, int t, int l) { return ((long long)t * 2 + l) * cols + col; };
+    auto blkV_of = [&](int col, int t, int l) { return (long long)t * (cols * 2) + (long long)col * 2 + l; };
+
+    Item it, nit;
+    int j_n1 = draw ? P + me : (int)(p.work * me / P) + 1;
+    bool have = item_of(draw ? me : j_n1 - 1, it), have_next = have && item_of(j_n1, nit);
+    int drawn = 0;                                         // thread 0: the counter's answer, used an item later
+    const bool any = have && it.t_lo < it.t_hi;
+
+    // the two blocks of a step, by the lanes 0 and 1 of the worker's first warp
+    auto stage_K = [&](bool on, int col, int t) { stage_bulk(p.k, on && lane < 2, blkK_of(col, t, lane & 1), slotsK + (lane & 1) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0); };
+    auto stage_V = [&](bool on, int col, int t) { stage_bulk(p.v, on && lane < 2, blkV_of(col, t, lane & 1), slotsV + (lane & 1) * p.slotV_bytes, sm.leadV, sm.okV, sm.nbV, &sm.bar[1], lane, p.starve != 0); };
+    if (BULK) {
+        if (tid == 0) { kvc_mbar_init(&sm.bar[0], 1); kvc_mbar_init(&sm.bar[1], 1); kvc_mbar_fence_init(); sm.dead = 0; }
+        sync();
+        if (warp == 0 && any) { stage_K(true, it.col, it.t_lo); stage_V(true, it.col, it.t_lo); }
+    }
+    kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
+    kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
+    const bool escK = book_has_long_codes(p.k.book), escV = book_has_long_codes(p.v.book);
+
+    struct StepMeta { unsigned short startK, startV, vsc, ksc; int vmi, kmi; KUnit ku; };   // as loaded: no arithmetic waits on them here
+    auto load_meta = [&](bool on, int col, int step, StepMeta &m) {
+        const long long t = (long long)step * 128 + tid;
+        const int b = col / Hkv, h = col % Hkv;
+        m.startK = m.startV = 0; m.vsc = 0; m.vmi = m.kmi = 0; m.ksc = 0x3c00;
+        m.ku.sc = make_uint2(0x3c003c00u, 0x3c003c00u); m.ku.mi = make_uint2(0u, 0u);          // 1.0, 0
+        if (!on) return;
+        m.startK = vec_start_bits(p.k.thread_info, blkK_of(col, step, sub), v);
+        m.startV = vec_start_bits(p.v.thread_info, blkV_of(col, step, sub), v);
+        const long long u = kvc_tok_unit(t, vm.tok_div) * vm.sj + b * vm.sb + h * vm.sh;
+        m.vsc = kvc_load_scale_bits(vm, u); m.vmi = kvc_load_min(vm, u);
+        if (km.sc == 0) k_token_unit(m.ksc, m.kmi, km, t, b, h);
+        else {                                             // of the block whose weights the warp builds (warp & 1), 4 channels per lane
+            const long long un = kvc_tok_unit((long long)step * 128 + (warp & 1) * 64, km.tok_div) * km.sj + b * km.sb + h * km.sh + lane * 4;
+            m.ku.sc = *reinterpret_cast<const uint2 *>(reinterpret_cast<const unsigned short *>(km.scale) + un);
+            if (km.min_bytes == 1) m.ku.mi.x = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const int8_t *>(km.min_int) + un);
+            else m.ku.mi = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int16_t *>(km.min_int) + un);
+        }
+    };
+    StepMeta cur, nxt;
+    load_meta(any, have ? it.col : 0, have ? it.t_lo : 0, cur);
+    unsigned short qn[G];                                  // the query of an item is fetched while the item before it runs
+    auto q_fetch = [&](int col_) {
+        const long long row0 = (long long)(col_ / Hkv) * Hq + (long long)(col_ % Hkv) * Gt + p.g0;
+#pragma unroll
+        for (int g = 0; g < G; g++) qn[g] = g < p.nh ? reinterpret_cast<const unsigned short *>(p.q)[(row0 + g) * 128 + tid] : (unsigned short)0;
+    };
+    __syncthreads();                                       // the tables are in; from here on the workers go their own ways
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (have) q_fetch(it.col);
+
+    // over a warp's tokens: the lane's four, then the eight lanes with the same heads
+    auto warp_max = [&](float x) { x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4)); x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8)); return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16)); };
+    auto warp_sum = [&](float x) { x += __shfl_xor_sync(0xffffffffu, x, 4); x += __shfl_xor_sync(0xffffffffu, x, 8); return x + __shfl_xor_sync(0xffffffffu, x, 16); };
+    auto red_put = [&](int k, const float (&x)[2]) { if (lane < G / 2) *reinterpret_cast<float2 *>(&sm.red[k][warp * G + h2]) = make_float2(x[0], x[1]); };
+    auto red_get = [&](int k, int w4) { return *reinterpret_cast<const float2 *>(&sm.red[k][w4 * G + h2]); };
+
+    uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
+    while (have) {
+    const int col = it.col, b = col / Hkv, h = col % Hkv;
+    if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
+#pragma unroll
+    for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = qn[g];
+    sync();
+    for (int g = warp; g < G; g += 4) {                    // sum of each query head's 128 (scaled) values
+        float a = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) a += kvc_scale_value(sm.q[g * 128 + k * 32 + lane]) * p.scaling;
+        a = kvc_warp_sum(a);
+        if (lane == 0) sm.qsum[g] = a;
+    }
+    float m_run[2], l_run[2], acc[4][2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        m_run[j] = -CUDART_INF_F; l_run[j] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[i][j] = 0.f;
+    }
+
+    for (int step = it.t_lo; step < it.t_hi; step++) {
+        bool n_on = true; int n_col = col, n_step = step + 1;      // the worker's next step (it may open the next column)
+        if (n_step >= it.t_hi) {
+            n_on = have_next && nit.t_lo < nit.t_hi; n_col = n_on ? nit.col : col; n_step = n_on ? nit.t_lo : 0;
+            if (have_next) q_fetch(nit.col);
+        }
+        if (!BULK) {
+            uint32_t ld, nb;
+            bool ok = stage(p.k, blkK_of(col, step, sub), slotsK + sub * p.slotK_bytes, &ld, &nb, v);
+            if (v == 0) { sm.leadK[sub] = ld; sm.nbK[sub] = nb; sm.okK[sub] = ok; }
+            ok = stage(p.v, blkV_of(col, step, sub), slotsV + sub * p.slotV_bytes, &ld, &nb, v);
+            if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; }
+        }
+        k_weights_rows<G>(sm.w, sm.kstep, sm.zp, sm.q, p.scaling, cur.ku, km.sc != 0, km.min_bytes, warp & 1, warp >> 1, lane);
+        bool k_landed = true;                              // (a wait that runs out: see the one-head kernel)
+        if (BULK) {
+            k_landed = kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit);
+            if (k_landed) par ^= 1u; else flags |= KVC_FLAG_WAIT_TIMEOUT;
+        }
+        sync();
+        // ---- K: scores of this step's tokens
+        float s[4][2];
+        {
+            bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
+            if (ok) ok = decode_row(kvc_smem_addr(slotsK + sub * p.slotK_bytes), sm.leadK[sub] + (cur.startK >> 3), kvc_smem_addr(tab.lutK), p.k.book, escK, row_s);
+            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+            __syncwarp();
+            int d[4][2];
+            rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + sub * VEC_ROWS_WORDS(G)), lane, d);
+            const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the thread's own token
+            const float2 st = *reinterpret_cast<const float2 *>(&sm.kstep[sub * G + h2]), z = *reinterpret_cast<const float2 *>(&sm.zp[sub * G + h2]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                s[i][0] = st.x * (float)d[i][0]; s[i][1] = st.y * (float)d[i][1];
+                if (km.sc != 0) { s[i][0] += z.x; s[i][1] += z.y; }
+                else {
+                    const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
+                    const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
+                    s[i][0] = sc * fmaf(mi, sm.qsum[h2], s[i][0]); s[i][1] = sc * fmaf(mi, sm.qsum[h2 + 1], s[i][1]);
+                }
+            }
+        }
+        // ---- online softmax over the step
+        float t1[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) t1[j] = warp_max(fmaxf(fmaxf(s[0][j], s[1][j]), fmaxf(s[2][j], s[3][j])));
+        red_put(0, t1);
+        sync();                                            // also: every thread is done with the K slots and weights
+        load_meta(n_on, n_col, n_step, nxt);               // in flight during the V phase, first touched in the next step
+        if (BULK && warp == 0) {                           // the next step's K blocks land during the V phase
+            if (__all_sync(0xffffffffu, k_landed)) stage_K(n_on, n_col, n_step);
+            else if (lane == 0) sm.dead = 1;
+        }
+        float alpha[2], vst[2];
+        {
+            const float2 x0 = red_get(0, 0), x1 = red_get(0, 1), x2 = red_get(0, 2), x3 = red_get(0, 3);
+            t1[0] = fmaxf(fmaxf(x0.x, x1.x), fmaxf(x2.x, x3.x)); t1[1] = fmaxf(fmaxf(x0.y, x1.y), fmaxf(x2.y, x3.y));
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float m_new = fmaxf(m_run[j], t1[j]);
+            alpha[j] = __expf(m_run[j] - m_new);           // exp(-inf) = 0 on the first step
+            m_run[j] = m_new;
+        }
+        {
+            float ssum[2] = {0.f, 0.f}, zsum[2] = {0.f, 0.f}, wmax[2] = {0.f, 0.f};
+            const uint32_t unit = (uint32_t)cur.vsc | ((uint32_t)cur.vmi << 16);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
+                const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const float pr = __expf(s[i][j] - m_run[j]);
+                    s[i][j] = pr * sc;                     // from here on the token's V weight
+                    ssum[j] += pr; zsum[j] = fmaf(s[i][j], mi, zsum[j]); wmax[j] = fmaxf(wmax[j], fabsf(s[i][j]));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) { ssum[j] = warp_sum(ssum[j]); zsum[j] = warp_sum(zsum[j]); wmax[j] = warp_max(wmax[j]); }
+            red_put(1, ssum); red_put(2, zsum); red_put(3, wmax);
+        }
+        sync();
+        // the V weights' words: the lane's four tokens are one word of each of its heads (the K weights are spent)
+        {
+            const float2 x0 = red_get(3, 0), x1 = red_get(3, 1), x2 = red_get(3, 2), x3 = red_get(3, 3);
+            t1[0] = fmaxf(fmaxf(x0.x, x1.x), fmaxf(x2.x, x3.x)); t1[1] = fmaxf(fmaxf(x0.y, x1.y), fmaxf(x2.y, x3.y));
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            vst[j] = fix_step(t1[j]);
+            const float inv = vst[j] > 0.f ? 1.0f / vst[j] : 0.f;
+            const uint2 w2 = pack4_dense(__float2int_rn(s[0][j] * inv), __float2int_rn(s[1][j] * inv), __float2int_rn(s[2][j] * inv), __float2int_rn(s[3][j] * inv));
+            const uint32_t at = w_rows(h2 + j, warp * 8 + (lane >> 2));
+            if (own) { sm.w[at] = w2.x; sm.w[G * 32 + at] = w2.y; }
+        }
+        const bool v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
+        if (BULK && v_landed) par ^= 2u;
+        if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        sync();
+        // ---- V: this step's contribution to the lane's four channels
+        {
+            bool ok = v_landed && sm.okV[sub] && (uint32_t)(cur.startV >> 3) < sm.nbV[sub];
+            if (ok) ok = decode_row(kvc_smem_addr(slotsV + sub * p.slotV_bytes), sm.leadV[sub] + (cur.startV >> 3), kvc_smem_addr(tab.lutV), p.v.book, escV, row_s);
+            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+            __syncwarp();
+            int d[4][2];
+            rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w), lane, d);
+            const float2 s0 = red_get(1, 0), s1 = red_get(1, 1), s2 = red_get(1, 2), s3 = red_get(1, 3);
+            l_run[0] = l_run[0] * alpha[0] + ((s0.x + s1.x) + (s2.x + s3.x)); l_run[1] = l_run[1] * alpha[1] + ((s0.y + s1.y) + (s2.y + s3.y));
+            const float2 z0 = red_get(2, 0), z1 = red_get(2, 1), z2 = red_get(2, 2), z3 = red_get(2, 3);
+            const float z[2] = {(z0.x + z1.x) + (z2.x + z3.x), (z0.y + z1.y) + (z2.y + z3.y)};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) acc[i][j] = fmaf(acc[i][j], alpha[j], fmaf(vst[j], (float)d[i][j], z[j]));
+        }
+        sync();                                            // every thread is done with the V slots, weights and sums
+        if (BULK && warp == 0) {                           // the next step's V blocks land during its K phase
+            if (__all_sync(0xffffffffu, v_landed)) stage_V(n_on, n_col, n_step);
+            else if (lane == 0) sm.dead = 1;
+        }
+        cur = nxt;
+    }
+
+    // ---- uncompressed tail, only for callers without a workspace: otherwise the merge kernel adds it
+    if (p.Tr > 0 && !p.partial && it.t_hi == p.n_tiles) {
+        float *pt = reinterpret_cast<float *>(sm.w);       // p[row][g] of 128 rows
+        for (long long r0 = 0; r0 < p.Tr; r0 += 128) {
+            const bool act = r0 + tid < p.Tr;
+            sync();
+            float s[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) s[g] = act ? 0.f : -CUDART_INF_F;
+            if (act) {
+                const __half *kr = p.ktail + (((r0 + tid) * B + b) * Hkv + h) * 128;
+#pragma unroll 1
+                for (int c8 = 0; c8 < 16; c8++) {
+                    uint4 kv = *reinterpret_cast<const uint4 *>(kr + c8 * 8);
+                    const __half *kh = reinterpret_cast<const __half *>(&kv);
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+#pragma unroll
+                        for (int g = 0; g < G; g++) s[g] = fmaf(__half2float(kh[k]), kvc_scale_value(sm.q[g * 128 + c8 * 8 + k]) * p.scaling, s[g]);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < G; g++) { const float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
+            sync();
+            float alpha[2], dv[4][2];
+            {
+                const float2 x0 = red_get(0, 0), x1 = red_get(0, 1), x2 = red_get(0, 2), x3 = red_get(0, 3);
+                const float mt[2] = {fmaxf(fmaxf(x0.x, x1.x), fmaxf(x2.x, x3.x)), fmaxf(fmaxf(x0.y, x1.y), fmaxf(x2.y, x3.y))};
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const float m_new = fmaxf(m_run[j], mt[j]);
+                    alpha[j] = __expf(m_run[j] - m_new);
+                    m_run[j] = m_new;
+                    if (tid < 4) sm.red[3][h2 + j] = m_new;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) dv[i][j] = 0.f;
+                }
+            }
+            sync();
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const float pr = act ? __expf(s[g] - sm.red[3][g]) : 0.f;
+                pt[tid * G + g] = pr;
+                const float ssum = kvc_warp_sum(pr);
+                if (lane == 0) sm.red[1][warp * G + g] = ssum;
+            }
+            sync();
+            const int n_here = (int)min(128ll, p.Tr - r0);
+            for (int i = 0; i < n_here; i++) {             // the lane's four channels over the pass's rows
+                const __half *vr = p.vtail + (((r0 + i) * B + b) * Hkv + h) * 128 + warp * 32 + r4;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) dv[c][j] = fmaf(pt[i * G + h2 + j], __half2float(vr[c]), dv[c][j]);
+            }
+            const float2 s0 = red_get(1, 0), s1 = red_get(1, 1), s2 = red_get(1, 2), s3 = red_get(1, 3);
+            l_run[0] = l_run[0] * alpha[0] + ((s0.x + s1.x) + (s2.x + s3.x)); l_run[1] = l_run[1] * alpha[1] + ((s0.y + s1.y) + (s2.y + s3.y));
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) acc[c][j] = fmaf(acc[c][j], alpha[j], dv[c][j]);
+        }
+    }
+    if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without steps fetched nothing yet
+    const long long head0 = (long long)b * Hq + (long long)h * Gt + p.g0;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (!own || h2 + j >= p.nh) continue;
+        if (!p.partial) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) p.out[(head0 + h2 + j) * 128 + warp * 32 + r4 + i] = __float2half_rn(acc[i][j] / l_run[j]);
+        } else {
+            float *dst = p.ws_part + ((head0 + h2 + j) * p.splits + it.part) * ROWS_PART_FLOATS;     // 8-byte aligned
+            *reinterpret_cast<float2 *>(dst + 2 + warp * 32 + r4) = make_float2(acc[0][j], acc[1][j]);
+            *reinterpret_cast<float2 *>(dst + 4 + warp * 32 + r4) = make_float2(acc[2][j], acc[3][j]);
+            if (warp == 0 && lane < 4) { dst[0] = m_run[j]; dst[1] = l_run[j]; }
+        }
+    }
+    if (draw && tid == 0) sm.next_j = drawn;
+    sync();                                                // the tail's scratch is read before the next column's weights overwrite it
+    if (BULK && sm.dead != 0) break;                       // a staging wait ran out: the status word says so, the item's result is void
+    const int j_n2 = draw ? 2 * P + sm.next_j : j_n1 + 1;
+    it = nit; have = have_next; j_n1 = j_n2;
+    have_next = have && item_of(j_n1, nit);
+    }   // items of the worker
+    if (BULK && any) {                    // the copies issued after the last step are empty, but their phase must end;
+        // after a wait that ran out, these are the phases still open: nothing may be in flight at the return
+        if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        if (!kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+    }
+    if (flags) atomicOr(p.status, flags);
+    if (draw && tid == 0) {               // the last worker to finish leaves the scheduling counters zeroed for the next launch
+        __threadfence();
+        if (atomicAdd(&p.sched[1], 1) == P - 1) { p.sched[0] = 0; p.sched[1] = 0; __threadfence(); }
     }
 }
 
@@ -1127,10 +1344,13 @@ __device__ __forceinline__ unsigned short ld_nc_16_pinned(const void *p) {
 // grid-dependency wait, i.e. while the attention kernel's last CTAs still work: it reads nothing that kernel writes.
 // The loads of the partial results are issued in batches before any is used as well.
 constexpr int MERGE_THREADS = 256;
+// ROWS: the partial results of the grouped kernel
+template <bool ROWS>
 __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *__restrict__ ws_part, __half *__restrict__ out, int splits, TailArgs t) {
     __shared__ float sm_red[8], sm_sum[8], sm_e[128], sm_o[128];
     __shared__ __align__(16) float sm_q[128];
-    const float *src = ws_part + (size_t)blockIdx.x * splits * ATTN_PART_FLOATS;
+    constexpr int PART = ROWS ? ROWS_PART_FLOATS : ATTN_PART_FLOATS;
+    const float *src = ws_part + (size_t)blockIdx.x * splits * PART;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // launched with programmatic stream serialisation: the kernel behind this one in the stream may set up
     // while this one runs (it touches nothing this one writes before its own wait), and this one's CTAs may be
@@ -1210,7 +1430,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float M = -CUDART_INF_F;                              // the maximum over all partial results
-    for (int s2 = tid; s2 < splits; s2 += MERGE_THREADS) M = fmaxf(M, src[(size_t)s2 * ATTN_PART_FLOATS]);
+    for (int s2 = tid; s2 < splits; s2 += MERGE_THREADS) M = fmaxf(M, src[(size_t)s2 * PART]);
     M = kvc_warp_max(M);
     if (lane == 0) sm_red[warp] = M;
     __syncthreads();
@@ -1225,7 +1445,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
         if (tid < 128) {
             float e = 0.f;
             if (tid < ns) {
-                const float *pp = src + (size_t)(s0 + tid) * ATTN_PART_FLOATS;
+                const float *pp = src + (size_t)(s0 + tid) * PART;
                 const float m2 = pp[0];
                 e = m2 == -CUDART_INF_F ? 0.f : __expf(m2 - M);
                 L = fmaf(pp[1], e, L);
@@ -1238,8 +1458,8 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
                 float a[8];
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
-                    const float *pp = src + (size_t)(s0 + min(i0 + k, ns - 1)) * ATTN_PART_FLOATS;
-                    a[k] = pp[4 + c] + pp[4 + 128 + c];
+                    const float *pp = src + (size_t)(s0 + min(i0 + k, ns - 1)) * PART;
+                    a[k] = ROWS ? pp[2 + c] : pp[4 + c] + pp[4 + 128 + c];
                 }
 #pragma unroll
                 for (int k = 0; k < 8; k++) if (i0 + k < ns) O = fmaf(a[k], sm_e[i0 + k], O);
@@ -1361,6 +1581,7 @@ extern "C" void kvc_attn_debug(int wait_limit, int starve) { g_wait_limit = wait
 
 // CTAs per SM the attention kernel is launched with at most (its launch bounds ask for this many)
 constexpr int ATTN_CTAS_PER_SM = 3;
+constexpr size_t MAX_CTA_SHARED = 227 * 1024;
 // items a resident CTA should get on average: enough that the draws even out the CTAs' speeds and the
 // last items end close together, few enough that the per-item work (q, partial results) stays small
 constexpr int ATTN_ITEMS_PER_CTA = 4;
@@ -1370,10 +1591,9 @@ constexpr int ATTN_ITEMS_PER_CTA = 4;
 // short items to finish with.  The short items are handed out last (the item order puts them behind
 // all long ones), so the CTAs of a launch end within one short item of each other.
 struct RunPlan { int tps, long_runs, short_tiles, splits; };
-static RunPlan plan_runs(long long n_tiles, long long cols, int sm_count) {
+static RunPlan plan_runs(long long n_tiles, long long cols, long long P) {      // P: CTAs (grouped queries: workers) at work
     RunPlan r = {1, 1, 1, 1};
     if (n_tiles <= 0 || cols <= 0) { r.tps = 0; r.long_runs = 1; r.short_tiles = 0; return r; }
-    const long long P = (long long)ATTN_CTAS_PER_SM * sm_count;
     long long tps = cols * n_tiles / (P * ATTN_ITEMS_PER_CTA);       // tiles per long item
     if (tps < 1) tps = 1;
     if (tps > n_tiles) tps = n_tiles;
@@ -1395,7 +1615,7 @@ static RunPlan plan_runs(long long n_tiles, long long cols, int sm_count) {
 extern "C" int kvc_attn_splits(int64_t T, int64_t B, int64_t Hkv, int sm_count) {
     if (T <= 0 || B <= 0 || Hkv <= 0) return 1;
     if (sm_count <= 0) sm_count = kvc_sm_count();
-    return plan_runs((T + 255) / 256, B * Hkv, sm_count).splits;
+    return plan_runs((T + 255) / 256, B * Hkv, (long long)ATTN_CTAS_PER_SM * sm_count).splits;
 }
 
 // bytes of the zero-initialised head of a workspace: the two scheduling counters
@@ -1425,8 +1645,9 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     // every column is cut into runs of tiles; each (column, run) is one item of work.  splits > 0: that many
     // equal runs.  Otherwise long runs and, at the end of each column, short ones (plan_runs).
     int tps, long_runs, short_tiles;
+    const int asked = splits;
     if (splits <= 0) {
-        const RunPlan r = plan_runs(n_tiles, cols, kvc_sm_count());
+        const RunPlan r = plan_runs(n_tiles, cols, (long long)ATTN_CTAS_PER_SM * kvc_sm_count());
         tps = r.tps; long_runs = r.long_runs; short_tiles = r.short_tiles; splits = r.splits;
     } else {
         if (splits > n_tiles) splits = (int)(n_tiles > 0 ? n_tiles : 1);
@@ -1468,34 +1689,55 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.slotK_bytes = ((p.k.max_block + 15u + 15u) & ~15u) + 16u;
     p.slotV_bytes = ((p.v.max_block + 15u + 15u) & ~15u) + 16u;
     const size_t slot_total = 4 * (size_t)(p.slotK_bytes + p.slotV_bytes) + SLOT_PAD;
-    auto rows_smem = [&](size_t fixed) { return fixed + 4 * (size_t)(p.slotK_bytes + p.slotV_bytes) + NTHR * ROW_WORDS * 4; };
     // bulk copies widen every block to 16-byte boundaries: both streams must start on one
     const bool bulk = T > 0 && (reinterpret_cast<uintptr_t>(k->encoded) & 15) == 0 && (reinterpret_cast<uintptr_t>(v->encoded) & 15) == 0;
     const int sms = kvc_sm_count();
     const long long Gt = Hq / Hkv;
-    for (long long g0 = 0; g0 < Gt && !(T == 0 && tail_in_merge);) {       // nothing compressed: the merge kernel alone
-        // Heads per launch: every launch decodes the whole cache, so up to 8 go together, in launches of equal shares.
-        // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 461 us in two launches of 4, 244 us in one; where only one
-        // CTA of 8 heads fits an SM, K rel 0.02 and both trees in shared memory: 502 and 399 us; 2 x 5 heads, 0.01: 701 and 442 us.)
-        const long long most = 8;
-        const long long launches = (Gt - g0 + most - 1) / most;
-        const int nh = (int)((Gt - g0 + launches - 1) / launches), G = nh > 4 ? 8 : (nh > 2 ? 4 : nh);
-        p.g0 = g0; p.nh = nh;
-#define KVC_AT(GG, BB)                                                                                          \
+    if (Gt == 1 && T > 0) {
+        const size_t smem = slot_total + sizeof(AttnSmem<1>);
+        p.g0 = 0; p.nh = 1;
+        static kvc_launch_slot slots[2];
+        auto *kernel = bulk ? attn_decode_kernel<1, true> : attn_decode_kernel<1, false>;
+        int occ = 0;
+        if (int rc = kvc_prepare(slots[bulk], reinterpret_cast<const void *>(kernel), NTHR, smem, &occ)) return rc;
+        KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);
+        long long ctas = (long long)sms * (occ < ATTN_CTAS_PER_SM ? occ : ATTN_CTAS_PER_SM);
+        if (ctas > p.work) ctas = p.work;
+        if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(NTHR), smem, kvc_cu(stream), p)) return rc;
+    } else if (T > 0) {
+        // Grouped queries count in steps of 128 tokens.  The workspace, sized for `splits` partial results of the one-head
+        // kernel, holds twice as many of theirs: with more and smaller workers the items are finer where it may be so.
+        p.n_tiles = (int)(T / 128);
+        p.tiles_per_split *= 2; p.short_tiles *= 2;
+        if (asked <= 0 && p.partial && ws_parts) {
+            const RunPlan r = plan_runs(p.n_tiles, cols, (long long)rows_workers<4>() * sms);
+            if (r.splits <= 2 * splits && cols * r.splits < (1ll << 31) - (1ll << 20)) { p.tiles_per_split = r.tps; p.long_runs = r.long_runs; p.short_tiles = r.short_tiles; splits = p.splits = r.splits; }
+        }
+        p.work = cols * splits;
+        for (long long g0 = 0; g0 < Gt; g0 += p.nh) {
+            // Heads per launch: every launch decodes the whole cache, so up to 8 go together, in launches of equal shares.
+            // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 461 us in two launches of 4, 244 us in one.)
+            const long long launches = (Gt - g0 + 7) / 8;
+            p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
+#define KVC_AT(GG)                                                                                              \
     {                                                                                                           \
-        const size_t smem = (GG) >= 2 ? rows_smem(sizeof(AttnSmem<GG>)) : slot_total + sizeof(AttnSmem<GG>);     \
-        static kvc_launch_slot slot;                                                                            \
+        /* as many workers as fit an SM; fewer where the items then spread over more SMs */                     \
+        int workers = rows_workers<GG>();                                                                       \
+        while (workers > 1 && rows_smem<GG>(p, workers) > MAX_CTA_SHARED) workers--;                            \
+        if (p.work < (long long)workers * sms) workers = (int)((p.work + sms - 1) / sms);                       \
+        const size_t smem = rows_smem<GG>(p, workers);                                                          \
+        static kvc_launch_slot slots[2];                                                                        \
+        auto *kernel = bulk ? attn_rows_kernel<GG, true> : attn_rows_kernel<GG, false>;                         \
         int occ = 0;                                                                                            \
-        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(attn_decode_kernel<GG, BB>), NTHR, smem, &occ)) return rc; \
+        if (int rc = kvc_prepare(slots[bulk], reinterpret_cast<const void *>(kernel), 128 * workers, smem, &occ)) return rc; \
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);             \
-        long long ctas = (long long)sms * (occ < ATTN_CTAS_PER_SM ? occ : ATTN_CTAS_PER_SM);                    \
-        if (ctas > p.work) ctas = p.work;                                                                       \
-        if (int rc = launch_overlapped(attn_decode_kernel<GG, BB>, dim3((unsigned)ctas), dim3(NTHR), smem, kvc_cu(stream), p)) return rc; \
+        long long ctas = (p.work + workers - 1) / workers;                                                      \
+        if (ctas > sms) ctas = sms;                                                                             \
+        if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(128 * workers), smem, kvc_cu(stream), p)) return rc; \
     }
-        if (bulk) { if (G == 8) KVC_AT(8, true) else if (G == 4) KVC_AT(4, true) else if (G == 2) KVC_AT(2, true) else KVC_AT(1, true) }
-        else { if (G == 8) KVC_AT(8, false) else if (G == 4) KVC_AT(4, false) else if (G == 2) KVC_AT(2, false) else KVC_AT(1, false) }
+            if (p.nh > 4) KVC_AT(8) else if (p.nh > 2) KVC_AT(4) else KVC_AT(2)
 #undef KVC_AT
-        g0 += nh;
+        }
     }
     if (p.partial || tail_in_merge) {
         TailArgs ta = {};
@@ -1503,7 +1745,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             ta.q = p.q; ta.ktail = p.ktail; ta.vtail = p.vtail; ta.Tr = Tr;
             ta.B = (int)B; ta.Hkv = (int)Hkv; ta.Hq = (int)Hq; ta.scaling = scaling;
         }
-        if (int rc = launch_overlapped(attn_merge_kernel, dim3((unsigned)(B * Hq)), dim3(MERGE_THREADS), 0, kvc_cu(stream),
+        if (int rc = launch_overlapped(Gt > 1 ? attn_merge_kernel<true> : attn_merge_kernel<false>, dim3((unsigned)(B * Hq)), dim3(MERGE_THREADS), 0, kvc_cu(stream),
                                        (const float *)p.ws_part, p.out, T > 0 ? splits : 0, ta)) return rc;
     }
     KVC_LAUNCH_OK();
