@@ -516,7 +516,7 @@ class KVCompCtx:
             assert B.shape[2] == self.compressed_ctx_len, "ctx len mismatch"
             start.record()
             part, st = ops.fused_pv(self.cache(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
-            C = part.float().sum(dim=0, keepdim=True).half()
+            C = part.sum(dim=0, keepdim=True, dtype=torch.float32).half()
         stop.record()
         ops.read_status(st, what="mat_vec_mul")
         stop.synchronize()

@@ -35,7 +35,6 @@
 
 namespace {
 
-constexpr int SLOT_BYTES = 8192 + 32;     // a block is at most 8191 bytes (u16 fields) + alignment lead
 constexpr int SLOT_PAD = 1024;           // readable bytes behind the last staging slot
 constexpr int NTHR = 256;
 constexpr int ATTN_PART_FLOATS = 4 + 256;   // a partial result of the attention kernel: m, l, two unused, acc[2][128]
@@ -49,6 +48,10 @@ struct CacheDev {
     kvc_qmeta_dev q;
     uint32_t max_block;           // upper bound of a block's byte count
 };
+
+// a staging slot holds the largest block plus its alignment lead, widened to 16-byte chunks, plus the decoder's two words
+// of read-ahead
+__host__ __device__ __forceinline__ uint32_t slot_bytes_of(uint32_t max_block) { return ((max_block + 15u + 15u) & ~15u) + 16u; }
 
 CacheDev to_dev(const kvc_cache &c) {
     CacheDev d;
@@ -441,10 +444,13 @@ __device__ __forceinline__ void v_weights(uint32_t *ps, float *vstep, float *red
 }
 
 // ---- fused K: raw scores ------------------------------------------------------------------------
+// Both unfused kernels: the structure, four staging slots sized by the stream's largest block, SLOT_PAD bytes that a
+// corrupt stream's overrun may read.  (Slots for the largest block of the format let three CTAs share an SM; with the
+// stream's own, six do.)
+template <class S> size_t unfused_smem(const CacheDev &c) { return sizeof(S) + 4 * (size_t)slot_bytes_of(c.max_block) + SLOT_PAD; }
 template <int G>
-struct QkSmem {
+struct alignas(32) QkSmem {
     KvcBookSmem book;
-    uint8_t slot[4][SLOT_BYTES];
     alignas(32) uint32_t w[4 * 2 * WROW * G];
     float step[4 * G];
     float zp[4 * G];
@@ -460,6 +466,7 @@ __global__ void __launch_bounds__(NTHR) fused_qk_kernel(CacheDev kc, long long T
                                                         int out_f32, int *__restrict__ status) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     QkSmem<G> &sm = *reinterpret_cast<QkSmem<G> *>(smem_raw);
+    uint8_t *const slot = smem_raw + sizeof(QkSmem<G>) + (threadIdx.x >> 6) * slot_bytes_of(kc.max_block);
     const int tid = threadIdx.x, sub = tid >> 6, v = tid & 63;
     const long long cols = B * Hkv, col = blockIdx.y, b = col / Hkv, h = col % Hkv;
     const long long Gt = Hq / Hkv, hq0 = h * Gt + g0;
@@ -469,7 +476,7 @@ __global__ void __launch_bounds__(NTHR) fused_qk_kernel(CacheDev kc, long long T
     load_q<G>(sm.qf, sm.qsum, q, b, Hq, hq0, 1.0f, tid);
     const long long blk = (tok0 / 64 + sub) * cols + col;
     const bool active = t < T;
-    if (active) { uint32_t ld, nb; bool ok = stage(kc, blk, sm.slot[sub], &ld, &nb, v); if (v == 0) { sm.lead[sub] = ld; sm.nb[sub] = nb; sm.ok[sub] = ok; } }
+    if (active) { uint32_t ld, nb; bool ok = stage(kc, blk, slot, &ld, &nb, v); if (v == 0) { sm.lead[sub] = ld; sm.nb[sub] = nb; sm.ok[sub] = ok; } }
     __syncthreads();
     k_weights<G>(sm.w, sm.step, sm.zp, sm.qf, kc.q, tok0, T, b, h, tid);
     __syncthreads();
@@ -481,7 +488,7 @@ __global__ void __launch_bounds__(NTHR) fused_qk_kernel(CacheDev kc, long long T
     for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
     const uint32_t start = vec_start(kc.thread_info, blk, v);
     bool ok = sm.ok[sub] && start < sm.nb[sub];                // a vector begins inside its block
-    if (ok) ok = decode_dot<G>(sm.slot[sub], sm.lead[sub] + start, sm.book, esc, sm.w + sub * 2 * WROW * G, hi, lo);
+    if (ok) ok = decode_dot<G>(slot, sm.lead[sub] + start, sm.book, esc, sm.w + sub * 2 * WROW * G, hi, lo);
     if (!ok) atomicOr(status, KVC_FLAG_BAD_STREAM);
     float s[G];
     k_finish<G>(s, hi, lo, sm.step + sub * G, sm.zp + sub * G, sm.qsum, kc.q.sc != 0, kvc_scale_value(ksc), (float)kmi);
@@ -495,9 +502,8 @@ __global__ void __launch_bounds__(NTHR) fused_qk_kernel(CacheDev kc, long long T
 
 // ---- fused V: per-group partial outputs ----------------------------------------------------------
 template <int G>
-struct PvSmem {
+struct alignas(32) PvSmem {
     KvcBookSmem book;
-    uint8_t slot[4][SLOT_BYTES];
     alignas(32) uint32_t ps[2 * 2 * WROW * G];
     float vstep[2 * G];
     float zpv[2 * G];
@@ -513,6 +519,7 @@ __global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T
                                                         int *__restrict__ status) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     PvSmem<G> &sm = *reinterpret_cast<PvSmem<G> *>(smem_raw);
+    uint8_t *const slot = smem_raw + sizeof(PvSmem<G>) + (threadIdx.x >> 6) * slot_bytes_of(vc.max_block);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
     const int grp = tid >> 7, ch = tid & 127;
     const long long cols = B * Hkv, col = blockIdx.y, b = col / Hkv, h = col % Hkv;
@@ -524,7 +531,7 @@ __global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T
     const long long gI = tok0 / 128 + grp;
     const long long blk = gI * (cols * 2) + col * 2 + (ch >> 6);
     const bool active = gI * 128 < T;
-    if (active) { uint32_t ld, nb; bool ok = stage(vc, blk, sm.slot[sub], &ld, &nb, v); if (v == 0) { sm.lead[sub] = ld; sm.nb[sub] = nb; sm.ok[sub] = ok; } }
+    if (active) { uint32_t ld, nb; bool ok = stage(vc, blk, slot, &ld, &nb, v); if (v == 0) { sm.lead[sub] = ld; sm.nb[sub] = nb; sm.ok[sub] = ok; } }
     float wv[G];
     {
         float sc = 0.f, mi = 0.f;
@@ -547,7 +554,7 @@ __global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T
     for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
     const uint32_t start = vec_start(vc.thread_info, blk, v);
     bool ok = sm.ok[sub] && start < sm.nb[sub];
-    if (ok) ok = decode_dot<G>(sm.slot[sub], sm.lead[sub] + start, sm.book, esc, sm.ps + grp * 2 * WROW * G, hi, lo);
+    if (ok) ok = decode_dot<G>(slot, sm.lead[sub] + start, sm.book, esc, sm.ps + grp * 2 * WROW * G, hi, lo);
     if (!ok) atomicOr(status, KVC_FLAG_BAD_STREAM);
 #pragma unroll
     for (int g = 0; g < G; g++) {
@@ -1535,8 +1542,9 @@ extern "C" int kvc_fused_qk(const kvc_cache *k, int64_t T, int64_t B, int64_t Hk
     {                                                                                                           \
         static kvc_launch_slot slot;                                                                            \
         int occ = 0;                                                                                            \
-        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(fused_qk_kernel<GG>), NTHR, sizeof(QkSmem<GG>), &occ)) return rc; \
-        fused_qk_kernel<GG><<<grid, NTHR, sizeof(QkSmem<GG>), kvc_cu(stream)>>>(                                \
+        const size_t smem = unfused_smem<QkSmem<GG>>(kc);                                                       \
+        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(fused_qk_kernel<GG>), NTHR, smem, &occ)) return rc; \
+        fused_qk_kernel<GG><<<grid, NTHR, smem, kvc_cu(stream)>>>(                                \
             kc, T, B, Hkv, Hq, g0, reinterpret_cast<const __half *>(q), out, out_f32, status);                  \
     }
         if (G == 4) KVC_QK(4) else if (G == 2) KVC_QK(2) else KVC_QK(1)
@@ -1563,8 +1571,9 @@ extern "C" int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hk
     {                                                                                                           \
         static kvc_launch_slot slot;                                                                            \
         int occ = 0;                                                                                            \
-        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(fused_pv_kernel<GG>), NTHR, sizeof(PvSmem<GG>), &occ)) return rc; \
-        fused_pv_kernel<GG><<<grid, NTHR, sizeof(PvSmem<GG>), kvc_cu(stream)>>>(                                \
+        const size_t smem = unfused_smem<PvSmem<GG>>(vc);                                                       \
+        if (int rc = kvc_prepare(slot, reinterpret_cast<const void *>(fused_pv_kernel<GG>), NTHR, smem, &occ)) return rc; \
+        fused_pv_kernel<GG><<<grid, NTHR, smem, kvc_cu(stream)>>>(                                \
             vc, T, B, Hkv, Hq, g0, reinterpret_cast<const __half *>(P), reinterpret_cast<__half *>(out), status); \
     }
         if (G == 4) KVC_PV(4) else if (G == 2) KVC_PV(2) else KVC_PV(1)
@@ -1684,10 +1693,8 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.status = status;
     p.wait_limit = g_wait_limit > 0 ? g_wait_limit : KVC_WAIT_LIMIT;
     p.starve = g_starve;
-    // a slot holds the largest block plus its alignment lead, widened to 16-byte chunks, plus the
-    // decoder's two words of read-ahead
-    p.slotK_bytes = ((p.k.max_block + 15u + 15u) & ~15u) + 16u;
-    p.slotV_bytes = ((p.v.max_block + 15u + 15u) & ~15u) + 16u;
+    p.slotK_bytes = slot_bytes_of(p.k.max_block);
+    p.slotV_bytes = slot_bytes_of(p.v.max_block);
     const size_t slot_total = 4 * (size_t)(p.slotK_bytes + p.slotV_bytes) + SLOT_PAD;
     // bulk copies widen every block to 16-byte boundaries: both streams must start on one
     const bool bulk = T > 0 && (reinterpret_cast<uintptr_t>(k->encoded) & 15) == 0 && (reinterpret_cast<uintptr_t>(v->encoded) & 15) == 0;
