@@ -95,7 +95,7 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 // Rows of 36 words: 128 symbols, the overrun of paired lookups, and a 16-byte alignment at which the fragment
 // loads (16 bytes of row 4r+i by lane 4r+q) touch every bank once per quarter warp.
 constexpr int ROW_WORDS = 36;
-static_assert(ROW_WORDS * 4 >= 128 + KVC_DECODE_OVERRUN_PAIR + 3, "rows too short for paired lookups");
+static_assert(ROW_WORDS * 4 >= 128 + KVC_DECODE_OVERRUN + 3, "rows too short for paired lookups");
 constexpr int WROW = 136;                 // weight words per vector of the one-pass form: 128 positions + zeroed overrun
 __host__ __device__ constexpr int VEC_ROWS_WORDS(int G) { return 2 * G * 32; }     // weight words of one vector: [hi | lo][G][32 groups of 4 positions]
 // word of head g and position group w in the rows form: 16-byte chunks swizzled by the head, so that neither the
@@ -124,8 +124,8 @@ __device__ __forceinline__ void mma_uu(int (&c)[4], uint32_t a0, uint32_t a1, ui
 __device__ __forceinline__ bool decode_row(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, const void *book, bool esc, uint32_t row_s) {
     const KvcTreeGlobal tree(book);
     KvcRowWriter put;
-    return esc ? kvc_decode_vector<true, 0, KvcRowWriter, false>(slot_s, byte_pos, lut_s, tree, row_s, put)
-               : kvc_decode_vector<false, 0, KvcRowWriter, true>(slot_s, byte_pos, lut_s, tree, row_s, put);
+    return esc ? kvc_decode_vector<true, 0>(slot_s, byte_pos, lut_s, tree, row_s, put)
+               : kvc_decode_vector<false, 0>(slot_s, byte_pos, lut_s, tree, row_s, put);
 }
 
 // The products of a warp's 32 rows (first one at shared address rows_s) with the weight words at shared address
@@ -183,8 +183,8 @@ __device__ __forceinline__ bool decode_dot_impl(uint32_t slot_s, uint32_t byte_p
         }
     };
     // two lookups per round: the weight rows keep WROW - 128 zeroed positions for what is emitted past 127
-    static_assert(WROW >= 128 + KVC_DECODE_OVERRUN_PAIR + 1, "weight rows too short for paired lookups");
-    return kvc_decode_vector<ESC, SHIFT, decltype(emit), true>(slot_s, byte_pos, lut_s, KvcTreeShared{tree_s}, w_s >> SHIFT, emit);
+    static_assert(WROW >= 128 + KVC_DECODE_OVERRUN + 1, "weight rows too short for paired lookups");
+    return kvc_decode_vector<ESC, SHIFT>(slot_s, byte_pos, lut_s, KvcTreeShared{tree_s}, w_s >> SHIFT, emit);
 }
 // esc: the book has codes longer than the table window (uniform over the CTA)
 template <int G>

@@ -9,7 +9,7 @@
 
 namespace {
 
-constexpr int TILE_STRIDE = 140;          // 128 symbols + KVC_DECODE_OVERRUN_PAIR rounded up to words, + 1 word; 35 words keep column reads off one bank
+constexpr int TILE_STRIDE = 140;          // 128 symbols + KVC_DECODE_OVERRUN rounded up to words, + 1 word; 35 words keep column reads off one bank
 
 struct DecodeSmem {                         // followed by 4 staging slots (sized at launch), then the 4 tiles
     KvcBookSmem book;
@@ -49,13 +49,13 @@ __global__ void __launch_bounds__(256) decode_kernel(
             uint8_t *trow = tiles + sub * TILE_BYTES + v * TILE_STRIDE;
             bool ok = start < nbytes;
             // the symbols collect in a word that is stored when its last byte is known; symbols past position 127
-            // (at most KVC_DECODE_OVERRUN_PAIR) stay within the row's padding words
+            // (at most KVC_DECODE_OVERRUN) stay within the row's padding words
             KvcRowWriter put;
             const uint32_t slot_s = kvc_smem_addr(slots + sub * slot_bytes), lut_s = kvc_smem_addr(sm.book.lut),
                            row_s = kvc_smem_addr(trow);
             const KvcTreeShared tree{kvc_smem_addr(sm.book.tree)};
             if (ok) ok = esc ? kvc_decode_vector<true, 0>(slot_s, lead + start, lut_s, tree, row_s, put)
-                             : kvc_decode_vector<false, 0, decltype(put), true>(slot_s, lead + start, lut_s, tree, row_s, put);
+                             : kvc_decode_vector<false, 0>(slot_s, lead + start, lut_s, tree, row_s, put);
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
         }
         __syncthreads();

@@ -10,9 +10,7 @@
 
 #include "kvc_common.cuh"
 
-#define KVC_DECODE_UNROLL 1
-#define KVC_DECODE_OVERRUN (3 * KVC_DECODE_UNROLL)   // positions past 127 a decoder may emit
-#define KVC_DECODE_OVERRUN_PAIR 6                    // ... with two lookups per round (PAIR)
+#define KVC_DECODE_OVERRUN 6              // positions past 127 a decoder may emit (two lookups per round)
 
 struct KvcBookSmem {                      // per-CTA copy of the decode structures of one book
     uint32_t tree[512];
@@ -136,14 +134,13 @@ __device__ __forceinline__ bool kvc_book_needs_escape(const void *book) {
 // the position counter starts at `base`, so a consumer that keeps one record of 2^SHIFT bytes per
 // position at shared address A passes base = A >> SHIFT and gets the record's address with no add;
 // s0, s1: the state before and after the lookup (position from bit 6 up), for consumers that track word borders.
-// The end of the vector is tested once per KVC_DECODE_UNROLL lookups, so emit may be handed symbols for
-// positions up to 127 + KVC_DECODE_OVERRUN; the consumer keeps room for them (zero weights, padding).
-// ESC = false is for books whose longest code fits the table window: no escape test in the loop;
-// PAIR (with ESC = false only) takes two lookups per round.
+// The end of the vector is tested once per two lookups, so emit may be handed symbols for positions up to
+// 127 + KVC_DECODE_OVERRUN; the consumer keeps room for them (zero weights, padding).
+// ESC = false is for books whose longest code fits the table window: no escape test in the loop.
 // Every round advances by at least one symbol, so the loop ends after at most 128 rounds; a corrupt
 // stream can read at most a few hundred bytes past its vector, for which the kernels keep padding
 // behind the last slot.  Returns false when the bits do not form valid codes.
-template <bool ESC, int SHIFT, class Emit, bool PAIR = false, class Tree = KvcTreeShared>
+template <bool ESC, int SHIFT, class Emit, class Tree = KvcTreeShared>
 __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, Tree tree,
                                                   uint32_t base, Emit emit) {
     static_assert(SHIFT >= 0 && SHIFT <= 6, "record size");
@@ -151,18 +148,17 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
     const uint32_t end = (base + KVC_VEC_LEN) << 6;
     uint32_t ptr = slot_s + (byte_pos & ~3u);
     uint32_t state = (base << 6) | ((byte_pos & 3u) << 3);
-    uint32_t hi = kvc_bswap(kvc_lds32(ptr)), lo = kvc_bswap(kvc_lds32(ptr + 4));
-    if (PAIR && !ESC) {
-        // Two lookups per round.  The first leaves the bit offset below 32 + KVC_LUT_BITS, so the second
-        // one's window still lies inside (hi, lo) or (lo, next word) and needs no refill in between:
-        // one refill test and one end test per pair.  The second lookup may run although the first
-        // finished the vector, so up to KVC_DECODE_OVERRUN_PAIR positions past 127 are emitted.
-        uint32_t nx = kvc_bswap(kvc_lds32(ptr + 8));
-        ptr += 12;
+    uint32_t hi = kvc_bswap(kvc_lds32(ptr)), lo = kvc_bswap(kvc_lds32(ptr + 4)), nx = kvc_bswap(kvc_lds32(ptr + 8));
+    ptr += 12;
+    // Two lookups per round.  The first leaves the bit offset below 32 + KVC_LUT_BITS, so the second one's window still
+    // lies inside (hi, lo) or (lo, next word) and needs no refill in between: one refill test and one end test per
+    // pair.  The second lookup may run although the first finished the vector, so up to KVC_DECODE_OVERRUN positions
+    // past 127 are emitted.
+    if (!ESC) {
         do {
             const uint32_t w0 = __funnelshift_l(lo, hi, state);
             const uint32_t e0 = kvc_lds32(lut_s + ((w0 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-            const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);
+            const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);   // state + byte 0 of e0, off the integer ALU pipe
             emit(e0, (state >> (6 - SHIFT)) & AMASK, state, s1);
             state = s1;
             const bool up = (state & 32u) != 0;
@@ -175,38 +171,46 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
         } while (state < end);
         return true;
     }
-    uint32_t nxt = kvc_lds32(ptr + 8);     // one word of read-ahead keeps the refill off the critical path
-    ptr += 12;
+    // The same with a test of each entry; a long code ends its round.  (One lookup per round: one head, rel 0.01 / 0.02,
+    // 8 x 4096 tokens, 309 us against 286.)
     bool ok = true;
-    do {
-#pragma unroll
-      for (int rep = 0; rep < KVC_DECODE_UNROLL; rep++) {             // the end test runs once per UNROLL lookups
-        const uint32_t win = __funnelshift_l(lo, hi, state);          // the shift uses the low 5 bits
-        const uint32_t e = kvc_lds32(lut_s + ((win >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-        if (!ESC || (e & 0xffu) != 0) {
-            const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e, 1u, (int)state);   // state + byte 0 of e, off the integer ALU pipe
-            emit(e, (state >> (6 - SHIFT)) & AMASK, state, s1);
-            state = s1;
-        } else {                                                      // code longer than the window
-            uint32_t node = e >> 8, sym = 0;
-            bool found = false;
-            const uint32_t a = (state >> (6 - SHIFT)) & AMASK;
-            state += KVC_LUT_BITS;
-            for (int guard = 0; guard < 40; guard++) {
-                if (state & 32u) { hi = lo; lo = kvc_bswap(nxt); nxt = kvc_lds32(ptr); ptr += 4; state -= 32u; }
-                if (node >= 512u) break;
-                const uint32_t nd = tree(node);
-                if ((nd & 0xffffu) == KVC_TREE_LEAF) { sym = nd >> 16; found = true; break; }
-                const uint32_t bit = __funnelshift_l(lo, hi, state) >> 31;
-                state += 1u;
-                node = (nd >> (16 * bit)) & 0xffffu;
-            }
-            ok = ok && found;
-            emit((sym << 8) | (1u << 6), a, state, state + (1u << 6));   // advance byte: one symbol
-            state += 1u << 6;
+    auto refill = [&]() { if (state & 32u) { hi = lo; lo = nx; nx = kvc_bswap(kvc_lds32(ptr)); ptr += 4; state -= 32u; } };
+    // a code longer than the window: on from the node the entry names, one bit at a time (the offset is below 32 +
+    // KVC_LUT_BITS here, and below 64 with the window's bits)
+    auto long_code = [&](uint32_t e) {
+        uint32_t node = e >> 8, sym = 0;
+        bool found = false;
+        const uint32_t a = (state >> (6 - SHIFT)) & AMASK;
+        state += KVC_LUT_BITS;
+        for (int guard = 0; guard < 40; guard++) {
+            refill();
+            if (node >= 512u) break;
+            const uint32_t nd = tree(node);
+            if ((nd & 0xffffu) == KVC_TREE_LEAF) { sym = nd >> 16; found = true; break; }
+            const uint32_t bit = __funnelshift_l(lo, hi, state) >> 31;
+            state += 1u;
+            node = (nd >> (16 * bit)) & 0xffffu;
         }
-        if (state & 32u) { hi = lo; lo = kvc_bswap(nxt); nxt = kvc_lds32(ptr); ptr += 4; state -= 32u; }
-      }
+        ok = ok && found;
+        emit((sym << 8) | (1u << 6), a, state, state + (1u << 6));     // advance byte: one symbol
+        state += 1u << 6;
+        refill();
+    };
+    do {
+        const uint32_t w0 = __funnelshift_l(lo, hi, state);
+        const uint32_t e0 = kvc_lds32(lut_s + ((w0 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
+        if ((e0 & 0xffu) == 0) { long_code(e0); continue; }
+        const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);
+        emit(e0, (state >> (6 - SHIFT)) & AMASK, state, s1);
+        state = s1;
+        const bool up = (state & 32u) != 0;
+        const uint32_t w1 = __funnelshift_l(up ? nx : lo, up ? lo : hi, state);
+        const uint32_t e1 = kvc_lds32(lut_s + ((w1 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
+        if ((e1 & 0xffu) == 0) { if (state < end) long_code(e1); continue; }
+        const uint32_t s2 = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)state);
+        emit(e1, (state >> (6 - SHIFT)) & AMASK, state, s2);
+        state = s2;
+        refill();
     } while (state < end);
     return ok;
 }
@@ -214,7 +218,7 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
 // A consumer for kvc_decode_vector (SHIFT = 0, base = the shared address of the thread's row): the symbols collect in a
 // word that is stored when its last byte is known.  One predicated store per word; three byte stores per lookup cost as
 // many instructions and, with 32 lanes at 32 places of their rows, three times the bank conflicts.  (The two shifts
-// as one wide multiplication: 2.5 % slower in the attention kernel.)  Symbols past position 127 reach at most KVC_DECODE_OVERRUN_PAIR bytes beyond the row's 128.
+// as one wide multiplication: 2.5 % slower in the attention kernel.)  Symbols past position 127 reach at most KVC_DECODE_OVERRUN bytes beyond the row's 128.
 struct KvcRowWriter {
     uint32_t cur = 0;
     __device__ __forceinline__ void operator()(uint32_t e, uint32_t a, uint32_t s0, uint32_t s1) {
