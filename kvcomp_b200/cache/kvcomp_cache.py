@@ -180,7 +180,7 @@ class KVCompCache(_BASE):
             self._ws[key] = ops.attn_workspace(B, Hq, parts, q.device)
         if q.device not in self._status:
             self._status[q.device] = ops.new_status(q.device)
-        out, _ = ops.attn_decode(kc.cache() if T else None, vc.cache() if T else None, T, B, kc.head_num, q, scaling,
+        out, _ = ops.attn_decode(kc._argument() if T else None, vc._argument() if T else None, T, B, kc.head_num, q, scaling,
                                  ktail, vtail, splits=0, workspace=self._ws[key], status=self._status[q.device])
         return out.unsqueeze(2) if squeeze else out
 

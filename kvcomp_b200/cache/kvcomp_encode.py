@@ -119,6 +119,14 @@ class _RecentRows:
 
 
 class KVCompCtx:
+    _cache_arg = _cache_q = None             # _argument()'s structure; holds addresses, so no copy or pickle takes it along
+
+    def __getstate__(self):
+        state = self.__dict__.copy()
+        state.pop("_cache_arg", None)
+        state.pop("_cache_q", None)
+        return state
+
     def __init__(self, is_k, batch_size, head_num, head_dim, quant_scale_rel,
                  encode_codebook_path=None, decode_codebook_path=None, batch_shared=None, min_dtype=None,
                  keep_dequantised=False):
@@ -169,7 +177,6 @@ class KVCompCtx:
         self._ti = _Arena(torch.int16)
         self._mi = _Arena(self.min_dtype)
         self._sc = _Arena(torch.float16)
-        self._cache_arg = self._cache_q = None   # cache()'s argument structure, refilled at every call
 
     # ---- views with the reference's attribute names --------------------------------------------
     @property
@@ -454,7 +461,7 @@ class KVCompCtx:
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
         x = torch.empty((rows,) + shape, dtype=torch.float16, device=self.device)
-        st = ops.decode_values(self.cache(), n, *shape[:2], self.is_k, x[:n]) if n else None
+        st = ops.decode_values(self._argument(), n, *shape[:2], self.is_k, x[:n]) if n else None
         if self._pending is not None:
             first = n // self.spec.tok_div * self.spec.sj                    # unit of the first waiting token
             ops.dequant(self._pending, self._mi.used()[first:], self._sc.used()[first:], self.spec, out=x[n:self.compressed_ctx_len])
@@ -481,7 +488,12 @@ class KVCompCtx:
 
     def cache(self):
         """The kvc_cache argument of the fused kernels over the encoded_ctx_len tokens of the stream (valid
-        until the next store)."""
+        until the next store).  A structure of the caller's own."""
+        return ops.copy_cache(self._argument())
+
+    def _argument(self):
+        """The same for a launch made right away: this context's one structure, every field that a store can change
+        filled in again at each call (0.8 us; a new structure 2 us)."""
         assert self.encoded_ctx_len > 0 and self.book is not None, "nothing has been encoded yet"
         c = self._cache_arg
         if c is None:
@@ -489,7 +501,6 @@ class KVCompCtx:
                                                  self._sc.buf, self.spec, self._enc.n, self.max_block_bytes)
             self._cache_q = c.q
             return c
-        # the same structure, every field that a store can change filled in again (cheaper than a new one)
         c.encoded, c.encoded_bytes, c.max_block_bytes = self._enc.buf.data_ptr(), self._enc.n, self.max_block_bytes
         c.block_info, c.thread_info, c.book = self._bi.buf.data_ptr(), self._ti.buf.data_ptr(), self.book.blob.data_ptr()
         self._cache_q.min_int, self._cache_q.scale = self._mi.buf.data_ptr(), self._sc.buf.data_ptr()
@@ -511,11 +522,11 @@ class KVCompCtx:
         if self.is_k:
             assert B.shape[2] == self.head_dim, "head dim mismatch"
             start.record()
-            C, st = ops.fused_qk(self.cache(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
+            C, st = ops.fused_qk(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
         else:
             assert B.shape[2] == self.compressed_ctx_len, "ctx len mismatch"
             start.record()
-            part, st = ops.fused_pv(self.cache(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
+            part, st = ops.fused_pv(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
             C = part.sum(dim=0, keepdim=True, dtype=torch.float32).half()
         stop.record()
         ops.read_status(st, what="mat_vec_mul")

@@ -386,6 +386,11 @@ def make_cache(encoded, block_info, thread_info, book, min_int, scale, spec, enc
                  spec.qmeta(min_int, scale), int(max_block_bytes), 0)
 
 
+def copy_cache(cache):
+    """Another kvc_cache argument with the same contents."""
+    return Cache.from_buffer_copy(cache)
+
+
 def fused_qk(cache, T, B, Hkv, q, out=None, out_dtype=torch.float16, status=None):
     """q fp16 [B,Hq,128] -> raw scores [B,Hq,T]."""
     lib = _lib.load()

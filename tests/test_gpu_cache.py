@@ -582,3 +582,32 @@ def test_rows_behind_the_fused_range_come_from_one_buffer(cfg, is_k, rec):
             if got is not None and keep:
                 assert got.data_ptr() % 16 == 0 and got.is_contiguous()
         assert n > 1200
+
+
+def test_a_copied_cache_goes_its_own_way(cfg):
+    """A prompt's cache deep-copied after it has been used: the copy attends to the same bits, and what either stores
+    afterwards does not reach the other."""
+    import copy
+    from kvcomp_b200.cache.kvcomp_cache import KVCompCache
+    B, H, T, D = 2, 2, 300, 128
+    cfg(kmode="ChannelQuant", vblk=64, krec=64, vrec=64)
+    k, v, q = synth(T + 64, B, H, seed=12, Hq=4)
+    k, v, q = k.permute(1, 2, 0, 3).contiguous().cuda(), v.permute(1, 2, 0, 3).contiguous().cuda(), q.unsqueeze(2).cuda()
+    cos, sin = _rope(T + 64)
+    cos, sin = cos.cuda(), sin.cuda()
+
+    def put(cache, a, b):
+        cache.append(k[:, :, a:b].contiguous(), v[:, :, a:b].contiguous(), 0, {"cos": cos[:, a:b].contiguous(), "sin": sin[:, a:b].contiguous()})
+    one = KVCompCache(B, 4, D, 1)
+    put(one, 0, T)
+    out = one.attend(q, 0)
+    rows = [x.get()[0] for x in (one.k_ctx[0], one.v_ctx[0])]
+    two = copy.deepcopy(one)
+    assert torch.equal(two.attend(q, 0), out)
+    put(two, T, T + 64)                                 # compresses another block of the copy
+    assert two.get_seq_length(0) == T + 64 and one.get_seq_length(0) == T
+    assert torch.equal(one.attend(q, 0), out)
+    assert all(torch.equal(x.get()[0], r) for x, r in zip((one.k_ctx[0], one.v_ctx[0]), rows))
+    put(one, T, T + 64)                                 # the original takes the same tokens: the same cache again
+    assert torch.equal(one.attend(q, 0), two.attend(q, 0))
+    assert all(torch.equal(a.get()[0], b.get()[0]) for a, b in zip((one.k_ctx[0], one.v_ctx[0]), (two.k_ctx[0], two.v_ctx[0])))

@@ -196,3 +196,57 @@ def test_recent_rows_buffer_against_a_list_model():
         moves += before is not None and rr.buf is not None and rr.buf.data_ptr() != before
         check()
     assert nxt > 3000 and moves < 400                 # the buffer is replaced now and then, not at every step
+
+
+def _filled_context():
+    """A KVCompCtx with made-up tables on the CPU, enough for cache() (no kernel runs)."""
+    from kvcomp_b200 import ops
+    from kvcomp_b200.cache.kvcomp_encode import KVCompCtx
+    from kvcomp_b200.utils.config import KVCompCacheConfigStatic
+    KVCompCacheConfigStatic.config = KVCompCacheConfig("", QuantMode.ChannelQuant, QuantMode.TokenQuant, 64, 128, 0, 0, 0.05, 0.1)
+    try:
+        ctx = KVCompCtx(True, 1, 2, 128, 0.05)
+    finally:
+        KVCompCacheConfigStatic.config = None
+    for i, a in enumerate((ctx._enc, ctx._bi, ctx._ti, ctx._mi, ctx._sc)):
+        a.reserve(2048 + 64 * i, "cpu").zero_()
+        a.n = 1024 + i
+    ctx.book = ops.Book(torch.zeros(22080, dtype=torch.uint8))
+    ctx.encoded_ctx_len, ctx.max_block_bytes = 64, 77
+    return ctx
+
+
+def _addresses(c):
+    return c.encoded, c.encoded_bytes, c.block_info, c.thread_info, c.book, c.q.min_int, c.q.scale, c.max_block_bytes
+
+
+def _own_addresses(ctx):
+    return (ctx._enc.buf.data_ptr(), ctx._enc.n, ctx._bi.buf.data_ptr(), ctx._ti.buf.data_ptr(), ctx.book.blob.data_ptr(),
+            ctx._mi.buf.data_ptr(), ctx._sc.buf.data_ptr(), ctx.max_block_bytes)
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "pickle", "copy"])
+def test_a_used_context_can_be_copied(how):
+    """Copying a prompt's cache per request is how a host reuses a prefix: a context whose argument structure has been
+    made can be copied and pickled, and the copy's structure names the copy's own buffers and is not shared."""
+    import copy
+    import pickle
+    ctx = _filled_context()
+    first = ctx.cache()
+    assert _addresses(first) == _own_addresses(ctx)
+    other = {"deepcopy": copy.deepcopy, "copy": copy.copy, "pickle": lambda x: pickle.loads(pickle.dumps(x))}[how](ctx)
+    if how == "copy":                                   # shallow: the same buffers, until one of the two grows its own
+        other._enc = copy.copy(other._enc)
+        other._enc.buf = other._enc.buf.clone()
+    assert _own_addresses(other) != _own_addresses(ctx)
+    assert _addresses(other.cache()) == _own_addresses(other)
+    assert _addresses(first) == _own_addresses(ctx)     # the original's is what it was
+    assert _addresses(ctx.cache()) == _own_addresses(ctx)
+    assert other.quant_mode == ctx.quant_mode and other.encoded_ctx_len == ctx.encoded_ctx_len
+
+
+def test_each_cache_call_returns_a_structure_of_its_own():
+    ctx = _filled_context()
+    a, b = ctx.cache(), ctx.cache()
+    a.max_block_bytes, a.q.tok_div = 0, 999
+    assert (b.max_block_bytes, b.q.tok_div) == (77, 64) and (ctx.cache().max_block_bytes, ctx.cache().q.tok_div) == (77, 64)
