@@ -1348,7 +1348,10 @@ __device__ __forceinline__ unsigned short ld_nc_16_pinned(const void *p) {
 // Inside the attention kernel each column's tail held a 256-thread CTA and its third of an SM for those round
 // trips (a 128-row tail lengthened a 137 us launch by 160 us when its loads depended on one another, by 25 us
 // with deep batches).  Here every head's tail is in flight at once on small CTAs, and it runs before the
-// grid-dependency wait, i.e. while the attention kernel's last CTAs still work: it reads nothing that kernel writes.
+// grid-dependency wait, i.e. while the attention kernel's last CTAs still work: it reads nothing that kernel writes, and
+// that kernel has itself waited for whatever wrote the query and the tail's rows.  With nothing compressed (splits = 0)
+// there is no attention kernel in between: the kernel ahead may be the one that stores the newest rows (it lets its
+// dependents start early), so the wait comes first.
 // The loads of the partial results are issued in batches before any is used as well.
 constexpr int MERGE_THREADS = 256;
 // ROWS: the partial results of the grouped kernel
@@ -1363,6 +1366,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
     // while this one runs (it touches nothing this one writes before its own wait), and this one's CTAs may be
     // resident before the attention kernel has finished; its partial results are complete and visible after the wait
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (splits == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     float m_t = -CUDART_INF_F, l_t = 0.f, o_t = 0.f;      // the tail's running maximum and sum; output of channel tid & 127 over the thread's rows
     if (t.Tr > 0) {
         // q.k: two threads per row, 64 channels each; P.V: thread = (half of the pass's rows, channel)

@@ -721,6 +721,30 @@ def test_attn_decode_tail_only(ops):
     assert_attn_close(out, O)
 
 
+@pytest.mark.parametrize("B,Hkv,Hq,t", [(8, 32, 32, 64), (4, 8, 32, 1), (2, 16, 16, 300)])
+def test_attn_decode_tail_only_right_behind_the_store_of_its_rows(ops, B, Hkv, Hq, t):
+    """The first decode step of a sequence: the kernel that stores the new rows and the one that reads them are queued
+    back to back while the device is busy.  The storing kernel lets its dependents start early, so the reader may not
+    touch the rows before its grid-dependency wait."""
+    k, v, q = synth(t, B, Hkv, seed=54, Hq=Hq)
+    kd, vd, qd = dev(k.transpose(1, 2, 0, 3)), dev(v.transpose(1, 2, 0, 3)), dev(q)
+    cos, sin = torch.ones(1, t, 128, dtype=torch.float16, device="cuda"), torch.zeros(1, t, 128, dtype=torch.float16, device="cuda")
+    ks, vs = (torch.empty(t, B, Hkv, 128, dtype=torch.float16, device="cuda") for _ in range(2))
+    ws, st, out = ops.attn_workspace(B, Hq, 1, "cuda"), ops.new_status("cuda"), torch.empty(B, Hq, 128, dtype=torch.float16, device="cuda")
+    scaling = 1.0 / math.sqrt(128)
+    g = Hq // Hkv
+    S = torch.einsum("bhd,tbhd->bht", qd.double(), dev(k).double().repeat_interleave(g, dim=2)) * scaling
+    O = torch.einsum("bht,tbhd->bhd", torch.softmax(S, -1), dev(v).double().repeat_interleave(g, dim=2)).cpu().numpy()
+    for _ in range(20):
+        ks.fill_(7.0)
+        vs.fill_(-9.0)
+        torch.cuda._sleep(200_000)                       # both launches are queued before the first one begins
+        ops.kv_store(kd, vd, cos, sin, ks, vs)
+        ops.attn_decode(None, None, 0, B, Hkv, qd, scaling, ks, vs, out=out, workspace=ws, status=st)
+        assert_attn_close(out, O)
+    assert ops.read_status(st) == 0
+
+
 def test_attn_decode_many_items(ops):
     """More items than two per resident CTA: the later ones are drawn from the workspace's counter.
     Every way of sharing the work gives the oracle's result, and the counters end at zero."""
