@@ -7,6 +7,7 @@
 // heapq share: push = append + sift up while the parent is strictly larger; pop = walk the
 // hole from the root to a leaf always taking the right child unless it is strictly larger
 // than the left one, drop the former last element there and sift it up.
+#include <cuda.h>
 #include <stdarg.h>
 
 #include <mutex>
@@ -36,25 +37,47 @@ int kvc_sm_count() {
     return n;
 }
 
+// Numbers are given to contexts in the order they are first seen; a context's id is never used again in a process.
+int kvc_context() {
+    typedef CUresult (*get_id_t)(CUcontext, unsigned long long *);
+    static const get_id_t get_id = []() -> get_id_t {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<get_id_t>(f);
+        cudaGetLastError();
+        return nullptr;
+    }();
+    static std::atomic<unsigned long long> seen[KVC_MAX_CONTEXTS];      // id + 1; 0: free
+    unsigned long long id;
+    if (!get_id || get_id(nullptr, &id) != CUDA_SUCCESS) return -1;     // (a thread without a context yet)
+    for (int i = 0; i < KVC_MAX_CONTEXTS; i++) {
+        unsigned long long at = seen[i].load(std::memory_order_relaxed);
+        if (at == 0 && seen[i].compare_exchange_strong(at, id + 1, std::memory_order_relaxed)) return i;
+        if (at == id + 1) return i;
+    }
+    return -1;
+}
+
 int kvc_prepare(kvc_launch_slot &slot, const void *kernel, int threads, size_t smem, int *occ) {
     static std::mutex mutex;
-    int dev = 0;
-    KVC_CUDA_OK(cudaGetDevice(&dev));
-    const bool keep = dev >= 0 && dev < KVC_MAX_DEVICES && smem < (1u << 20);
+    const int ctx = kvc_context();
+    const bool keep = ctx >= 0 && smem < (1u << 20) && threads % 32 == 0;
+    const unsigned long long asked = (unsigned long long)threads / 32 << 48 | (unsigned long long)smem << 8;
+    constexpr unsigned long long ASKED = 0xff0000ull << 32 | 0xfffff00ull;
     if (keep) {
-        const unsigned long long v = slot.known[dev].load(std::memory_order_acquire);
-        if ((v & 0xff) != 0 && ((v >> 8) & 0xfffff) == smem) { *occ = (int)(v & 0xff); return KVC_OK; }
+        const unsigned long long v = slot.known[ctx].load(std::memory_order_acquire);
+        if ((v & 0xff) != 0 && (v & ASKED) == asked) { *occ = (int)(v & 0xff); return KVC_OK; }
     }
     std::lock_guard<std::mutex> lock(mutex);              // the limit never shrinks under another thread's launch
-    const size_t limit = keep ? (size_t)(slot.known[dev].load(std::memory_order_relaxed) >> 28) : 0;
+    const size_t limit = keep ? (size_t)(slot.known[ctx].load(std::memory_order_relaxed) >> 28 & 0xfffff) : 0;
     if (smem > limit || limit == 0) {
         KVC_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         KVC_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     }
     KVC_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kernel, threads, smem));
     if (keep && *occ > 0 && *occ < 256)
-        slot.known[dev].store((unsigned long long)(smem > limit ? smem : limit) << 28 | (unsigned long long)smem << 8 | (unsigned)*occ,
-                              std::memory_order_release);
+        slot.known[ctx].store(asked | (unsigned long long)(smem > limit ? smem : limit) << 28 | (unsigned)*occ, std::memory_order_release);
     return KVC_OK;
 }
 

@@ -42,12 +42,19 @@ static inline cudaStream_t kvc_cu(kvc_stream_t s) { return reinterpret_cast<cuda
 
 int kvc_sm_count();
 
-// What a launch of `kernel` with `smem` dynamic bytes needs to know, asked of the runtime once per kernel, device and
-// size: sets the kernel's shared-memory limit (it only grows) and its carve-out, and returns in *occ how many CTAs of
-// `threads` fit an SM.  Any thread; `slot` is the kernel's own.  (Asked at every launch, a decode step of attention
-// cost 26 us end to end at 1024 tokens, now 22.5.)
 constexpr int KVC_MAX_DEVICES = 64;
-struct kvc_launch_slot { std::atomic<unsigned long long> known[KVC_MAX_DEVICES]; };   // limit << 28 | size last asked for << 8 | its occupancy
+// Number of the calling thread's current context, 0 .. KVC_MAX_CONTEXTS - 1, or -1: nothing is kept for it.  A kernel's
+// attributes and a __device__ array's address belong to a context: a process may have several on a device, and a new one
+// after a reset.
+constexpr int KVC_MAX_CONTEXTS = 64;
+int kvc_context();
+
+// What a launch of `kernel` with `smem` dynamic bytes needs to know: sets the kernel's shared-memory limit (it only grows)
+// and its carve-out, and returns in *occ how many CTAs of `threads` fit an SM.  Any thread; `slot` is the kernel's own and
+// keeps, per context, the limit and the last answer: the runtime is asked again when the size or the number of threads
+// changes (caches whose largest blocks differ, in turn).  Asked at every launch, a decode step of attention cost 26 us end
+// to end at 1024 tokens, now 22.5.
+struct kvc_launch_slot { std::atomic<unsigned long long> known[KVC_MAX_CONTEXTS]; };   // threads / 32 << 48 | limit << 28 | size << 8 | CTAs per SM
 int kvc_prepare(kvc_launch_slot &slot, const void *kernel, int threads, size_t smem, int *occ);
 
 // ---- device helpers ---------------------------------------------------------------
