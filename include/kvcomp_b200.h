@@ -266,12 +266,12 @@ void kvc_attn_debug(int wait_limit, int starve);
 /* No counterpart in the reference.  kvc_attn_decode for callers that cannot allocate device memory
  * (a serving process whose memory pool owns the whole device, a plugin under a fixed memory budget):
  * the split-KV scratch is a fixed array inside the library (kvc_attn_static_capacity() bytes, 4 MiB,
- * held by every GPU that loads the library until the process exits) instead of a caller workspace.
+ * held by every context that loads the library until it ends) instead of a caller workspace.
  * Inputs and outputs are still the caller's.  Nothing is allocated or freed by this call.
  *  - B, Hq and splits whose scratch (kvc_attn_workspace) exceeds the capacity: KVC_ERR_CAPACITY.
- *  - The first call on a device looks the array's device address up (with that device current);
+ *  - The first call in a context looks the array's device address up (with that context current);
  *    make that first call outside any stream capture.
- *  - All calls on a device share the array: the counters are cleared on `stream` at the start of
+ *  - All calls in a context share the array: the counters are cleared on `stream` at the start of
  *    every call, and two calls that overlap on the GPU (different streams) race.  Calls on one
  *    stream are ordered and safe. */
 int64_t kvc_attn_static_capacity(void);

@@ -28,7 +28,6 @@
 // every decode: weight records are stored [position][G].
 #include <math_constants.h>
 
-#include <mutex>
 #include <type_traits>
 
 #include "kvc_decode.cuh"
@@ -1769,27 +1768,21 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
 // runs under a fixed memory budget, or code that runs where an allocation would synchronise the
 // device at the wrong moment.  For them the split-KV scratch of the attention kernel (per-head
 // counters and the per-split partial results) lives in this fixed array instead of a workspace the
-// caller has to provide.  Every GPU that loads the library holds these bytes until the process exits.
+// caller has to provide.  Every context that loads the library holds these bytes until it ends.
 #define KVC_STATIC_SCRATCH_BYTES (4 << 20)
 static __device__ __align__(256) unsigned char g_attn_scratch[KVC_STATIC_SCRATCH_BYTES];
 
 namespace {
-std::mutex g_scratch_mutex;
-void *g_scratch_ptr[KVC_MAX_DEVICES] = {};
+std::atomic<void *> g_scratch_ptr[KVC_MAX_CONTEXTS];
 
-// The array's name is only a host-side handle in host code; the device address has to be asked for,
-// once per device, with that device current.
+// The array's name is only a host-side handle in host code; the device address has to be asked for, once per context,
+// with that context current (each has an array of its own).
 int static_scratch(void **ptr) {
-    int dev = -1;
-    KVC_CUDA_OK(cudaGetDevice(&dev));
-    KVC_REQUIRE(dev >= 0 && dev < KVC_MAX_DEVICES, "kvc_attn_decode_static: device %d out of range", dev);
-    std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (!g_scratch_ptr[dev]) {
-        void *p = nullptr;
-        KVC_CUDA_OK(cudaGetSymbolAddress(&p, g_attn_scratch));
-        g_scratch_ptr[dev] = p;
-    }
-    *ptr = g_scratch_ptr[dev];
+    const int ctx = kvc_context();
+    *ptr = ctx >= 0 ? g_scratch_ptr[ctx].load(std::memory_order_relaxed) : nullptr;
+    if (*ptr) return KVC_OK;
+    KVC_CUDA_OK(cudaGetSymbolAddress(ptr, g_attn_scratch));
+    if (ctx >= 0) g_scratch_ptr[ctx].store(*ptr, std::memory_order_relaxed);
     return KVC_OK;
 }
 }  // namespace

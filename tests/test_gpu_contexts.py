@@ -102,7 +102,7 @@ def _second_context(entry, q):
         q.put(repr(e))
 
 
-@pytest.mark.parametrize("entry", ["decode", "attn"])
+@pytest.mark.parametrize("entry", ["decode", "attn", "static"])
 def test_calls_in_a_second_context_of_the_device(entry):
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
