@@ -240,8 +240,8 @@ int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hkv, int64_t 
  * be NULL).  q: device fp16 [B,Hq,128]; out: device fp16
  * [B,Hq,128].  Scores never leave the SM; no fp16 K/V is written to memory.
  * Work is cut into items, one (sequence, KV head) column x one of `splits` equal runs of
- * 256-token tiles (with several query heads per KV head and splits = 0: runs of its own choice, at most
- * twice as many, in the same workspace); as many CTAs as the device holds at once take items until none is left,
+ * 256-token tiles (with several query heads per KV head and room for partial results: where it pays, runs
+ * of its own choice, at most twice as many, in the same workspace); as many CTAs as the device holds at once take items until none is left,
  * and a second small kernel merges the `splits` partial results of every head and adds the
  * tail's tokens (it does the whole step when T = 0).  splits = 0
  * picks kvc_attn_splits(T, B, Hkv, 0).  workspace: kvc_attn_workspace(B, Hq, splits) bytes

@@ -28,6 +28,7 @@
 // every decode: weight records are stored [position][G].
 #include <math_constants.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "kvc_decode.cuh"
@@ -36,6 +37,7 @@ namespace {
 
 constexpr int SLOT_PAD = 1024;           // readable bytes behind the last staging slot
 constexpr int NTHR = 256;
+constexpr size_t MAX_CTA_SHARED = 227 * 1024;
 constexpr int ATTN_PART_FLOATS = 4 + 256;   // a partial result of the attention kernel: m, l, two unused, acc[2][128]
 
 struct CacheDev {
@@ -598,6 +600,7 @@ struct AttnParams {
     float *ws_part;               // [B*Hq][splits][ATTN_PART_FLOATS]
     int *sched;                   // {items handed out, CTAs finished}, or null: static shares
     int *status;
+    int team;                     // grouped queries without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
     int wait_limit;               // tries of a staging wait before it gives up (KVC_FLAG_WAIT_TIMEOUT)
     int starve;                   // tests of the bounded waits only: announce bytes that are never copied
@@ -978,7 +981,32 @@ template <int G> size_t rows_smem(const AttnParams &p, int workers) {
     return sizeof(RowsTables) + workers * (sizeof(RowsWorker<G>) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes) + 128 * ROW_WORDS * 4);
 }
 
-template <int G, bool BULK>
+template <int G> int rows_fit(const AttnParams &p) {         // workers that an SM holds
+    int workers = rows_workers<G>();
+    while (workers > 1 && rows_smem<G>(p, workers) > MAX_CTA_SHARED) workers--;
+    return workers;
+}
+int rows_fit(const AttnParams &p, int heads) { return heads > 4 ? rows_fit<8>(p) : (heads > 2 ? rows_fit<4>(p) : rows_fit<2>(p)); }
+
+// How many of an SM's workers share a column when every column's output is written directly (no workspace, or a single run
+// without a tail): without company a worker would take all of a column's `units` (steps and passes of the tail) in turn
+// while most of the device is idle.  A unit takes about 6 + a parts of time with `a` workers at work on the SM (2 heads: 9.2 us
+// alone, 14.4 us with five).  2 heads per column, no workspace, a worker per column against teams: 8 columns of 1024 tokens
+// 77.6 and 31.5 us, 64 of 8192 594 and 189 us, 256 of 256 (two teams of two on an SM) 26.1 and 19.6 us.
+int rows_team(long long cols, long long units, int workers, int sms) {
+    if (cols >= (long long)workers * sms) return 0;          // enough columns for all
+    int best = 0;
+    long long least = 0;
+    for (int size = 1; size <= workers && size <= units; size++) {
+        const long long teams = std::min<long long>(workers / size, (cols + sms - 1) / sms);     // of an SM
+        const long long cost = ((cols + teams * sms - 1) / (teams * sms)) * ((units + size - 1) / size) * (6 + teams * size);
+        if (size == 1 || cost < least) { least = cost; best = size > 1 ? size : 0; }
+    }
+    return best;
+}
+
+// TEAM: see rows_team (a kernel of its own: a branch on it costs the other one 0.8 % through registers alone).
+template <int G, bool BULK, bool TEAM>
 __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     RowsTables &tab = *reinterpret_cast<RowsTables *>(smem_raw);
@@ -1001,13 +1029,17 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     int flags = 0;
 
     struct Item { int col, t_lo, t_hi, part; };            // steps t_lo .. t_hi - 1 of a column; part: the run's index
-    const bool draw = p.sched != nullptr;
-    const int P = (int)gridDim.x * workers, me = (int)blockIdx.x * workers + wk;
+    const bool draw = !TEAM && p.sched != nullptr;
+    const int P = (int)gridDim.x * (TEAM ? workers / p.team : workers);
+    const int me = TEAM ? wk / p.team * (int)gridDim.x + (int)blockIdx.x : (int)blockIdx.x * workers + wk;
     const int w_hi = draw ? (int)p.work : (int)(p.work * (me + 1) / P);
     auto item_of = [&](int j, Item &it) -> bool {
         if (j >= w_hi) return false;
         const int n_long = cols * p.long_runs;
-        if (j < n_long) {
+        if constexpr (TEAM) {                              // the worker's share of column j: the same for every column
+            const int tk = wk % p.team;
+            it.col = j; it.part = 0; it.t_lo = (int)((long long)p.n_tiles * tk / p.team); it.t_hi = (int)((long long)p.n_tiles * (tk + 1) / p.team);
+        } else if (j < n_long) {
             const int r = j % p.long_runs;
             it.col = j / p.long_runs; it.part = r; it.t_lo = r * p.tiles_per_split; it.t_hi = min(p.n_tiles, it.t_lo + p.tiles_per_split);
         } else {
@@ -1223,9 +1255,9 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     }
 
     // ---- uncompressed tail, only for callers without a workspace: otherwise the merge kernel adds it
-    if (p.Tr > 0 && !p.partial && it.t_hi == p.n_tiles) {
+    if (p.Tr > 0 && !p.partial && (TEAM || it.t_hi == p.n_tiles)) {
         float *pt = reinterpret_cast<float *>(sm.w);       // p[row][g] of 128 rows
-        for (long long r0 = 0; r0 < p.Tr; r0 += 128) {
+        for (long long r0 = TEAM ? wk % p.team * 128 : 0; r0 < p.Tr; r0 += TEAM ? p.team * 128 : 128) {      // a team's workers take the passes in turn
             const bool act = r0 + tid < p.Tr;
             sync();
             float s[G];
@@ -1287,6 +1319,34 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     }
     if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without steps fetched nothing yet
     const long long head0 = (long long)b * Hq + (long long)h * Gt + p.g0;
+    bool dead;
+    if constexpr (TEAM) {                                  // each worker's share to its own shared memory, then a head per worker
+        const int team = p.team, tm = wk / team, tk = wk % team;      // the worker's team and its place there
+        auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" :: "r"(rows_workers<2>() + 1 + tm), "r"(team * 128) : "memory"); };
+        sync();                                            // (the tail's scratch is read)
+        float *mine = reinterpret_cast<float *>(sm.w);     // acc[G][128]
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            if (!own) continue;
+            *reinterpret_cast<float4 *>(mine + (h2 + j) * 128 + warp * 32 + r4) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+            if (warp == 0 && lane < 4) { sm.red[0][h2 + j] = m_run[j]; sm.red[1][h2 + j] = l_run[j]; }
+        }
+        team_sync();
+        const RowsWorker<G> *mates = &sm - tk;
+        for (int g = tk; g < p.nh; g += team) {
+            float M = -CUDART_INF_F, O = 0.f, L = 0.f;
+            for (int w = 0; w < team; w++) M = fmaxf(M, mates[w].red[0][g]);
+            for (int w = 0; w < team; w++) {
+                const float m = mates[w].red[0][g], e = m == -CUDART_INF_F ? 0.f : __expf(m - M);     // a worker without tokens adds nothing
+                L = fmaf(mates[w].red[1][g], e, L);
+                O = fmaf(reinterpret_cast<const float *>(mates[w].w)[g * 128 + tid], e, O);
+            }
+            p.out[(head0 + g) * 128 + tid] = __float2half_rn(O / L);
+        }
+        dead = false;
+        if (BULK) for (int w = 0; w < team; w++) dead |= mates[w].dead != 0;      // of any: a team stops together
+        team_sync();
+    } else {
 #pragma unroll
     for (int j = 0; j < 2; j++) {
         if (!own || h2 + j >= p.nh) continue;
@@ -1302,7 +1362,9 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     }
     if (draw && tid == 0) sm.next_j = drawn;
     sync();                                                // the tail's scratch is read before the next column's weights overwrite it
-    if (BULK && sm.dead != 0) break;                       // a staging wait ran out: the status word says so, the item's result is void
+    dead = BULK && sm.dead != 0;
+    }
+    if (dead) break;                                       // a staging wait ran out: the status word says so, the item's result is void
     const int j_n2 = draw ? 2 * P + sm.next_j : j_n1 + 1;
     it = nit; have = have_next; j_n1 = j_n2;
     have_next = have && item_of(j_n1, nit);
@@ -1593,7 +1655,6 @@ extern "C" void kvc_attn_debug(int wait_limit, int starve) { g_wait_limit = wait
 
 // CTAs per SM the attention kernel is launched with at most (its launch bounds ask for this many)
 constexpr int ATTN_CTAS_PER_SM = 3;
-constexpr size_t MAX_CTA_SHARED = 227 * 1024;
 // items a resident CTA should get on average: enough that the draws even out the CTAs' speeds and the
 // last items end close together, few enough that the per-item work (q, partial results) stays small
 constexpr int ATTN_ITEMS_PER_CTA = 4;
@@ -1682,6 +1743,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.out = reinterpret_cast<__half *>(out);
     p.scaling = scaling; p.splits = splits; p.tiles_per_split = tps; p.long_runs = long_runs; p.short_tiles = short_tiles;
     p.n_tiles = (int)n_tiles;
+    p.team = 0;
     p.work = cols * splits;
     // with a workspace the CTAs draw their items from its counters (zero before the first launch, left zeroed)
     const bool have_ws = workspace && workspace_bytes >= ATTN_COUNTER_BYTES && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
@@ -1719,9 +1781,21 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         // kernel, holds twice as many of theirs: with more and smaller workers the items are finer where it may be so.
         p.n_tiles = (int)(T / 128);
         p.tiles_per_split *= 2; p.short_tiles *= 2;
-        if (asked <= 0 && p.partial && ws_parts) {
-            const RunPlan r = plan_runs(p.n_tiles, cols, (long long)rows_workers<4>() * sms);
-            if (r.splits <= 2 * splits && cols * r.splits < (1ll << 31) - (1ll << 20)) { p.tiles_per_split = r.tps; p.long_runs = r.long_runs; p.short_tiles = r.short_tiles; splits = p.splits = r.splits; }
+        const int heads = (int)((Gt + (Gt + 7) / 8 - 1) / ((Gt + 7) / 8));                   // of the first launch
+        const long long most = (long long)rows_fit(p, heads) * sms;                         // workers of a full device
+        if (p.partial && ws_parts) {
+            RunPlan r = {0, 0, 0, 0};
+            if (asked <= 0) r = plan_runs(p.n_tiles, cols, most);
+            // The caller's runs in halves where that is fewer steps one after the other: a worker takes a run's steps in turn, each
+            // with half the threads a CTA of the one-head kernel has for its tile.  (32 columns, 2 heads each, 2048 tokens in 4
+            // runs: 46.9 us, in halves 33.7; 64 columns in 8 runs: 36.0, in halves 42.2, as the halves no longer go in one round.)
+            else if ((2 * cols * splits + most - 1) / most < 2 * ((cols * splits + most - 1) / most)) {
+                r.tps = r.short_tiles = tps;
+                r.splits = r.long_runs = (p.n_tiles + tps - 1) / tps;
+            }
+            if (r.splits > 0 && r.splits <= 2 * splits && cols * r.splits < (1ll << 31) - (1ll << 20)) {
+                p.tiles_per_split = r.tps; p.long_runs = r.long_runs; p.short_tiles = r.short_tiles; splits = p.splits = r.splits;
+            }
         }
         p.work = cols * splits;
         for (long long g0 = 0; g0 < Gt; g0 += p.nh) {
@@ -1731,17 +1805,19 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
 #define KVC_AT(GG)                                                                                              \
     {                                                                                                           \
-        /* as many workers as fit an SM; fewer where the items then spread over more SMs */                     \
-        int workers = rows_workers<GG>();                                                                       \
-        while (workers > 1 && rows_smem<GG>(p, workers) > MAX_CTA_SHARED) workers--;                            \
-        if (p.work < (long long)workers * sms) workers = (int)((p.work + sms - 1) / sms);                       \
+        int workers = rows_fit<GG>(p);                                                                          \
+        p.team = p.partial ? 0 : rows_team(cols, p.n_tiles + (Tr + 127) / 128, workers, sms);                   \
+        if (p.team) { const long long n = (cols + sms - 1) / sms; workers = p.team * (int)std::min<long long>(n, workers / p.team); } \
+        /* fewer than fit an SM where the items then spread over more SMs */                                    \
+        else if (p.work < (long long)workers * sms) workers = (int)((p.work + sms - 1) / sms);                  \
         const size_t smem = rows_smem<GG>(p, workers);                                                          \
-        static kvc_launch_slot slots[2];                                                                        \
-        auto *kernel = bulk ? attn_rows_kernel<GG, true> : attn_rows_kernel<GG, false>;                         \
+        static kvc_launch_slot slots[4];                                                                        \
+        auto *kernel = p.team ? (bulk ? attn_rows_kernel<GG, true, true> : attn_rows_kernel<GG, false, true>)   \
+                              : (bulk ? attn_rows_kernel<GG, true, false> : attn_rows_kernel<GG, false, false>); \
         int occ = 0;                                                                                            \
-        if (int rc = kvc_prepare(slots[bulk], reinterpret_cast<const void *>(kernel), 128 * workers, smem, &occ)) return rc; \
+        if (int rc = kvc_prepare(slots[2 * (p.team != 0) + bulk], reinterpret_cast<const void *>(kernel), 128 * workers, smem, &occ)) return rc; \
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);             \
-        long long ctas = (p.work + workers - 1) / workers;                                                      \
+        long long ctas = p.team ? p.work : (p.work + workers - 1) / workers;                                    \
         if (ctas > sms) ctas = sms;                                                                             \
         if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(128 * workers), smem, kvc_cu(stream), p)) return rc; \
     }

@@ -604,6 +604,37 @@ def test_attn_decode_query_heads_per_kv_head(ops, G, kmode, krel, T, Tr, tight):
         assert_attn_close(out, O, str(kw))
 
 
+@pytest.mark.parametrize("B,Hkv,G,T,Tr,splits", [
+    (1, 2, 2, 256, 0, 0),       # two steps: a team of two, each with a step
+    (1, 1, 4, 1152, 0, 1),      # nine steps over five workers
+    (1, 3, 8, 896, 0, 1),       # the eight-column kernel's four workers
+    (2, 2, 9, 640, 70, 1),      # two launches; a tail of one pass
+    (1, 2, 2, 128, 500, 1),     # one step and four passes of the tail: workers without a step
+    (4, 64, 2, 256, 0, 0),      # 256 columns: two teams on an SM, some with two columns
+    (2, 80, 6, 384, 10, 1),     # more columns than SMs, an odd number of steps
+    (1, 2, 4, 1152, 0, 2),      # the caller's two runs in halves: 4 steps' worth of runs, the last one shorter
+    (2, 3, 2, 640, 33, 3),      # three runs over five steps
+    (1, 1, 8, 128, 0, 4),       # more runs than steps
+])
+def test_attn_decode_grouped_queries_on_a_nearly_idle_device(ops, B, Hkv, G, T, Tr, splits):
+    """Few columns: the workers of a CTA share a column when its output is written directly, and the caller's runs are cut in
+    halves when they leave partial results.  The same function of the cache, with and without a workspace."""
+    k, v, q = synth(T + Tr, B, Hkv, seed=70 + G, Hq=Hkv * G)
+    rk, rv, kc, vc = _caches(ops, k[:T], v[:T], orc.MODE_CHANNEL, orc.MODE_TOKEN, 0.05, 0.1, 64, False)
+    scaling = 1.0 / math.sqrt(128)
+    kt, vt = (dev(k[T:]), dev(v[T:])) if Tr else (None, None)
+    O = orc.attention(*_oracle_q(rk, T, B, Hkv, orc.MODE_CHANNEL, 64, False), *_oracle_q(rv, T, B, Hkv, orc.MODE_TOKEN, 128, False),
+                      q, scaling, k[T:] if Tr else None, v[T:] if Tr else None)
+    ws = ops.attn_workspace(B, Hkv * G, max(splits, ops.attn_splits(T, B, Hkv)), "cuda")
+    outs = []
+    for kw in (dict(splits=splits, workspace=ws), dict(splits=1, workspace=False), dict(splits=splits, workspace=ws)):
+        out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, kt, vt, **kw)
+        assert ops.read_status(st) == 0
+        assert_attn_close(out, O, str(kw))
+        outs.append(out)
+    assert torch.equal(outs[0], outs[2]) and int(ws[:256].view(torch.int32).abs().sum()) == 0
+
+
 def _skewed_cache(ops, rng, is_k, T, B, H):
     """Codes drawn from a very skewed alphabet (a code longer than the 12-bit decode window exists), with
     made-up units: K per 64-token block and sequence, V per token and sequence."""
