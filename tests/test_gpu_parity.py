@@ -635,6 +635,20 @@ def test_attn_decode_grouped_queries_on_a_nearly_idle_device(ops, B, Hkv, G, T, 
     assert torch.equal(outs[0], outs[2]) and int(ws[:256].view(torch.int32).abs().sum()) == 0
 
 
+@pytest.mark.parametrize("Hq", [1, 2])
+@pytest.mark.parametrize("parts", [7, 8, 9, 16, 17, 32, 33, 128, 130])
+def test_attn_decode_merges_any_number_of_partial_results(ops, Hq, parts):
+    """The merge kernel takes partial results in batches, by the two halves of its CTA in turn, 128 at a time."""
+    T = parts * 256
+    k, v, q = synth(T, 1, 1, seed=80, Hq=Hq)
+    rk, rv, kc, vc = _caches(ops, k, v, orc.MODE_BLOCK, orc.MODE_TOKEN, 0.05, 0.1, 64, False)
+    scaling = 1.0 / math.sqrt(128)
+    out, st = ops.attn_decode(kc, vc, T, 1, 1, dev(q), scaling, splits=parts)
+    assert ops.read_status(st) == 0
+    assert_attn_close(out, orc.attention(*_oracle_q(rk, T, 1, 1, orc.MODE_BLOCK, 64, False),
+                                         *_oracle_q(rv, T, 1, 1, orc.MODE_TOKEN, 128, False), q, scaling))
+
+
 def _skewed_cache(ops, rng, is_k, T, B, H):
     """Codes drawn from a very skewed alphabet (a code longer than the 12-bit decode window exists), with
     made-up units: K per 64-token block and sequence, V per token and sequence."""
