@@ -119,9 +119,9 @@ class _RecentRows:
 
 
 class KVCompCtx:
-    _cache_arg = _cache_q = None             # _argument()'s structure; holds addresses, so no copy or pickle takes it along
+    _cache_arg = _cache_q = None             # (of a copy)
 
-    def __getstate__(self):
+    def __getstate__(self):                  # the argument structure holds addresses: a copy makes its own
         state = self.__dict__.copy()
         state.pop("_cache_arg", None)
         state.pop("_cache_q", None)
@@ -177,6 +177,7 @@ class KVCompCtx:
         self._ti = _Arena(torch.int16)
         self._mi = _Arena(self.min_dtype)
         self._sc = _Arena(torch.float16)
+        self._cache_arg = self._cache_q = None   # _argument()'s structure
 
     # ---- views with the reference's attribute names --------------------------------------------
     @property
