@@ -422,23 +422,25 @@ __global__ void __launch_bounds__(256) quant_block_apply_kernel(
 }
 
 // ---- dequantise: fp16((code + min_int) * scale), models/cache/kvcomp_encode.py:146 -------------
-// Bound by memory (1 byte in, 2 out).  A thread takes four groups of 8 channels, all their loads in flight together;
-// wide_units: units side by side over the channels, 8 of them fetched with one load per array.  With one group per
-// thread, 64-bit divisions and a load per unit: 67 M values 95 us (units per channel) and 85 us (per token); now 70 and 38 us.
-constexpr int DEQ_GROUPS = 4;
+// Bound by memory (1 byte in, 2 out).  A thread takes GROUPS groups of 8 channels, all their loads in flight together;
+// wide_units: units side by side over the channels, 8 of them fetched with one load per array.  Two groups where the units
+// do not depend on the channel and there are enough of them to fill the device, else one: 64 x 128 values 2.1 us (two
+// groups 2.3, four 2.9), 33.6 M values 24.0 us (20.3, 20.4); per-channel units, more registers each, 2.3 us (2.7, 3.8) and 30.6
+// (33.3, 34.3).  With 64-bit divisions and a load per unit: 2.6 and 42.9, per channel 2.7 and 46.5 us.
+template <int GROUPS>
 __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t *__restrict__ codes, kvc_qmeta_dev m,
                                                       long long rows, uint32_t B, uint32_t H, uint32_t D, int wide_units,
                                                       __half *__restrict__ out) {
     const uint32_t per_row = D / 8;
-    const long long n = rows * per_row, i0 = (long long)blockIdx.x * (256 * DEQ_GROUPS) + threadIdx.x;
-    uint2 cv[DEQ_GROUPS];
+    const long long n = rows * per_row, i0 = (long long)blockIdx.x * (256 * GROUPS) + threadIdx.x;
+    uint2 cv[GROUPS];
 #pragma unroll
-    for (int g = 0; g < DEQ_GROUPS; g++) {
+    for (int g = 0; g < GROUPS; g++) {
         const long long i = i0 + g * 256;
         if (i < n) cv[g] = *reinterpret_cast<const uint2 *>(codes + i * 8);
     }
 #pragma unroll
-    for (int g = 0; g < DEQ_GROUPS; g++) {
+    for (int g = 0; g < GROUPS; g++) {
         const long long i = i0 + g * 256;
         if (i >= n) return;
         uint32_t c0, h, b;
@@ -621,7 +623,8 @@ extern "C" int kvc_dequant(const uint8_t *codes, const kvc_qmeta *q, int64_t T, 
     const kvc_qmeta_dev m = kvc_to_dev(*q);
     const int wide_units = m.sc == 1 && m.sj % 8 == 0 && m.sb % 8 == 0 && m.sh % 8 == 0 &&
                            (reinterpret_cast<uintptr_t>(m.scale) & 15) == 0 && (reinterpret_cast<uintptr_t>(m.min_int) & (8 * m.min_bytes - 1)) == 0;
-    dequant_kernel<<<(unsigned)((n + 256 * DEQ_GROUPS - 1) / (256 * DEQ_GROUPS)), 256, 0, kvc_cu(stream)>>>(
+    const int groups = m.sc == 0 && n > 512ll * kvc_sm_count() ? 2 : 1;
+    (groups == 2 ? dequant_kernel<2> : dequant_kernel<1>)<<<(unsigned)((n + 256 * groups - 1) / (256 * groups)), 256, 0, kvc_cu(stream)>>>(
         codes, m, rows, (uint32_t)B, (uint32_t)H, (uint32_t)D, wide_units, reinterpret_cast<__half *>(out));
     KVC_LAUNCH_OK();
     return KVC_OK;

@@ -376,8 +376,10 @@ def test_decode_values_equals_decode_then_dequant(ops, is_k, mode, block, shared
 @pytest.mark.parametrize("mode,block", [(orc.MODE_CHANNEL, 64), (orc.MODE_TOKEN, 64), (orc.MODE_VECTOR, 64), (orc.MODE_BLOCK, 128)])
 @pytest.mark.parametrize("min_dtype", [torch.int8, torch.int16])
 @pytest.mark.parametrize("offset", [0, 1])                  # 1: unit arrays off the boundaries of the wide loads
-def test_dequant_matches_torch(ops, mode, block, min_dtype, offset):
-    T, B, H = 128, 3, 5
+@pytest.mark.parametrize("T", [128, 384])                   # 384: enough for two groups of channels per thread
+def test_dequant_matches_torch(ops, mode, block, min_dtype, offset, T):
+    B, H = 3, 5
+    T += 1 if mode in (orc.MODE_TOKEN, orc.MODE_VECTOR) else 0      # units of a token: a last CTA that is not full
     spec = ops.qspec(mode, False, B, H, 128, block)
     n = spec.units(T, B, H, 128)
     g = torch.Generator().manual_seed(2)
