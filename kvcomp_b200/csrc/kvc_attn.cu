@@ -515,7 +515,7 @@ struct alignas(32) PvSmem {
 };
 
 template <int G>
-__global__ void __launch_bounds__(NTHR) fused_pv_kernel(CacheDev vc, long long T, long long B, long long Hkv, long long Hq,
+__global__ void __launch_bounds__(NTHR, 6) fused_pv_kernel(CacheDev vc, long long T, long long B, long long Hkv, long long Hq,
                                                         long long g0, const __half *__restrict__ P, __half *__restrict__ out,
                                                         int *__restrict__ status) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
