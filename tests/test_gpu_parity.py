@@ -521,8 +521,8 @@ ATTN_CASES = [  # kmode, vmode, shared, T, B, Hkv, Hq, Tr, splits, min_dtype
     (orc.MODE_BLOCK, orc.MODE_TOKEN, True, 384, 2, 2, 2, 100, 1, torch.int8),
     (orc.MODE_CHANNEL, orc.MODE_TOKEN, False, 896, 1, 2, 12, 300, 2, torch.int16),
     (orc.MODE_CHANNEL, orc.MODE_VECTOR, False, 128, 3, 1, 1, 1, 0, torch.int16),
-    (orc.MODE_CHANNEL, orc.MODE_TOKEN, False, 1152, 3, 5, 15, 0, 0, torch.int16),     # 3 query heads per KV head: chunks of 2 + 1
-    (orc.MODE_BLOCK, orc.MODE_TOKEN, False, 256, 1, 7, 35, 37, 9, torch.int16),       # 5 per KV head (4 + 1), more splits than tiles
+    (orc.MODE_CHANNEL, orc.MODE_TOKEN, False, 1152, 3, 5, 15, 0, 0, torch.int16),     # 3 query heads per KV head: four columns
+    (orc.MODE_BLOCK, orc.MODE_TOKEN, False, 256, 1, 7, 35, 37, 9, torch.int16),       # 5 per KV head: eight columns; more splits than tiles
     (orc.MODE_CHANNEL, orc.MODE_TOKEN, False, 2304, 1, 2, 4, 0, 4, torch.int16),      # 2 per KV head, 9 tiles in 3 runs
     (orc.MODE_CHANNEL, orc.MODE_TOKEN, False, 128, 2, 3, 6, 5, 0, torch.int16),       # half a tile and a tail
 ]
@@ -557,7 +557,7 @@ def test_attn_decode(ops, kmode, vmode, shared, T, B, Hkv, Hq, Tr, splits, min_d
 def test_attn_decode_phi3_settings(ops, B, Hkv, Hq, T, Tr):
     """The Phi-3-medium-shaped configuration's settings: K per channel in 128-token blocks at relative error
     bound 0.02 (about 52 symbols, 5.5 bits each), V per token at 0.15, four query heads per KV head -- and
-    five per KV head, which the kernel handles as chunks of 4 + 1."""
+    five per KV head, which the kernel pads to eight columns."""
     k, v, q = synth(T + Tr, B, Hkv, seed=33, Hq=Hq)
     rk, rv, kc, vc = _caches(ops, k[:T], v[:T], orc.MODE_CHANNEL, orc.MODE_TOKEN, 0.02, 0.15, 128, False)
     assert rk["book"].header()["n_symbols"] >= 45 and rk["book"].header()["escape"] in (0, 1)
@@ -589,10 +589,11 @@ def test_attn_decode_llama7b_shape_small(ops):
 @pytest.mark.parametrize("G", [2, 3, 5, 6, 7, 8, 9, 16])
 @pytest.mark.parametrize("kmode,krel,T,Tr,tight", [(orc.MODE_CHANNEL, 0.05, 640, 0, True),     # half a tile at the end
                                                    (orc.MODE_TOKEN, 0.05, 384, 131, True),    # one K unit per token, a tail of two passes
-                                                   (orc.MODE_BLOCK, 0.02, 256, 300, False)])  # slots for the largest block: one CTA per SM
+                                                   (orc.MODE_BLOCK, 0.02, 256, 300, False)])  # slots for the largest block: fewer workers per SM
 def test_attn_decode_query_heads_per_kv_head(ops, G, kmode, krel, T, Tr, tight):
     """Grouped queries go up to eight heads per launch through the tensor cores, padded to 2, 4 or 8 columns:
-    every number of heads, with the merge kernel and with the column's output and tail written directly."""
+    every number of heads (9 and 16: two launches), with the merge kernel and with the column's output and tail written
+    directly."""
     B, Hkv = 2, 2
     k, v, q = synth(T + Tr, B, Hkv, seed=60 + G, Hq=Hkv * G)
     rk, rv, kc, vc = _caches(ops, k[:T], v[:T], kmode, orc.MODE_TOKEN, krel, 0.1, 64, False, torch.int16, tight)
@@ -677,10 +678,11 @@ def _skewed_cache(ops, rng, is_k, T, B, H):
     return cache, (enc, bi, ti, book, mid, scd), (codes, mi, sc, m), book
 
 
-@pytest.mark.parametrize("G", [1, 2, 4, 3])
+@pytest.mark.parametrize("G", [1, 2, 4, 3, 5, 8, 9])
 def test_attn_decode_books_with_long_codes(ops, G):
     """Books whose header says `escape`: the fused kernels take the decoder that tests every table entry and
-    continues bit by bit from the tree, for one, two and four query heads per KV head (and 3 = 2 + 1)."""
+    continues bit by bit from the tree -- in shared memory with one query head per KV head, in global memory with
+    several, in two, four and eight columns (3, 5: padded; 9: two launches) -- with and without a workspace."""
     rng = np.random.default_rng(5 + G)
     T, B, Hkv = 512, 2, 2
     Hq = Hkv * G
@@ -695,6 +697,9 @@ def test_attn_decode_books_with_long_codes(ops, G):
     assert ops.read_status(st) == 0
     O = orc.attention(*ko, *vo, q, scaling)
     assert_attn_close(out, O)
+    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, splits=1, workspace=False)
+    assert ops.read_status(st) == 0
+    assert_attn_close(out, O)
     # the two-call kernels take the same path
     S, st = ops.fused_qk(kc, T, B, Hkv, dev(q), out_dtype=torch.float32)
     assert ops.read_status(st) == 0
@@ -702,14 +707,20 @@ def test_attn_decode_books_with_long_codes(ops, G):
     assert np.abs(S.cpu().numpy() - So).max() <= 5e-4 * np.abs(So).max()
 
 
-def test_attn_decode_flags_a_vector_that_starts_outside_its_block(ops):
+# query heads per KV head and the way the output is made: each attention kernel (one head; two and eight columns), leaving
+# partial results or writing the output itself (several heads: as teams of workers)
+WAYS = [(G, kw) for G in (1, 2, 8) for kw in (dict(splits=2), dict(splits=1, workspace=False))]
+
+
+@pytest.mark.parametrize("G,kw", WAYS)
+def test_attn_decode_flags_a_vector_that_starts_outside_its_block(ops, G, kw):
     """thread_info is input: an entry that points past its block's bytes (still inside the staging area) must
     be reported, not decoded."""
-    T, B, Hkv, Hq = 512, 1, 2, 2
+    T, B, Hkv, Hq = 512, 1, 2, 2 * G
     k, v, q = synth(T, B, Hkv, seed=51, Hq=Hq)
     rk, rv, kc, vc = _caches(ops, k, v, orc.MODE_CHANNEL, orc.MODE_TOKEN, 0.05, 0.1, 64, False)
     scaling = 1.0 / math.sqrt(128)
-    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling)
+    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **kw)
     assert ops.read_status(st) == 0
     for r, is_k in ((rk, True), (rv, False)):
         ti = r["ti"].clone()
@@ -717,7 +728,7 @@ def test_attn_decode_flags_a_vector_that_starts_outside_its_block(ops):
         # vector 10 of block 3 would start 40 bytes past the largest block
         bad[64 * 3 + 9] = int(np.array([(r["maxb"] + 40) << 3], dtype=np.uint16).view(np.int16)[0])
         r["ti"].copy_(bad)
-        out2, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling)
+        out2, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **kw)
         assert ops.read_status(st, raise_on_fatal=False) & 0x80, "K" if is_k else "V"
         assert torch.isfinite(out2.float()).all()
         if is_k:
@@ -727,30 +738,32 @@ def test_attn_decode_flags_a_vector_that_starts_outside_its_block(ops):
             S, st = ops.fused_pv(vc, T, B, Hkv, P)
         assert ops.read_status(st, raise_on_fatal=False) & 0x80
         r["ti"].copy_(ti)
-    out3, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling)
+    out3, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **kw)
     assert ops.read_status(st) == 0 and torch.equal(out3, out)
 
 
-def test_attn_decode_staging_wait_runs_out_and_returns(ops):
-    """The kernel's waits for its staged blocks are bounded.  With the diagnostic that announces bytes which
+@pytest.mark.parametrize("G,kw", WAYS)
+def test_attn_decode_staging_wait_runs_out_and_returns(ops, G, kw):
+    """The kernels' waits for their staged blocks are bounded.  With the diagnostic that announces bytes which
     are never copied, the first wait runs out after a few tries: the call returns, the status word carries
     KVC_FLAG_WAIT_TIMEOUT, nothing is left in flight, and the next ordinary call is correct."""
-    T, B, Hkv, Hq = 512, 2, 2, 4
+    T, B, Hkv, Hq = 512, 2, 2, 2 * G
     k, v, q = synth(T, B, Hkv, seed=52, Hq=Hq)
     rk, rv, kc, vc = _caches(ops, k, v, orc.MODE_CHANNEL, orc.MODE_TOKEN, 0.05, 0.1, 64, False)
     scaling = 1.0 / math.sqrt(128)
-    want, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, splits=2)
+    want, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **kw)
     assert ops.read_status(st) == 0
     ws = ops.attn_workspace(B, Hq, 2, "cuda")
+    held = dict(workspace=ws, **kw) if "workspace" not in kw else kw
     try:
         ops.attn_debug(wait_limit=8, starve=True)
-        out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, splits=2, workspace=ws)
+        out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **held)
         torch.cuda.synchronize()
         assert ops.read_status(st, raise_on_fatal=False) & 0x400
     finally:
         ops.attn_debug()
     assert int(ws[:256].view(torch.int32).abs().sum()) == 0          # the scheduling counters were left zeroed
-    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, splits=2, workspace=ws)
+    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **held)
     assert ops.read_status(st) == 0 and torch.equal(out, want)
 
 
@@ -812,24 +825,30 @@ def test_attn_decode_many_items(ops):
     assert int(ws[:256].view(torch.int32).abs().sum()) == 0
 
 
-def test_attn_decode_unaligned_stream_and_unknown_bound(ops):
+@pytest.mark.parametrize("G,kw", WAYS)
+def test_attn_decode_unaligned_stream_and_unknown_bound(ops, G, kw):
     """Streams that do not start on a 16-byte boundary take the plain-load staging path; an unknown
-    block bound falls back to the format's maximum.  Same bits either way."""
-    T, B, Hkv, Hq = 512, 2, 2, 4
+    block bound falls back to the format's maximum.  Same bits either way (but for the order of a sum that more
+    workers share)."""
+    T, B, Hkv, Hq = 512, 2, 2, 2 * G
     k, v, q = synth(T, B, Hkv, seed=31, Hq=Hq)
     rk, rv, kc, vc = _caches(ops, k, v, orc.MODE_CHANNEL, orc.MODE_TOKEN, 0.05, 0.1, 64, False)
     scaling = 1.0 / math.sqrt(128)
-    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, splits=2)
+    out, st = ops.attn_decode(kc, vc, T, B, Hkv, dev(q), scaling, **kw)
     assert ops.read_status(st) == 0
     rk0, rv0, kc0, vc0 = _caches(ops, k, v, orc.MODE_CHANNEL, orc.MODE_TOKEN, 0.05, 0.1, 64, False, tight=False)
-    out0, st = ops.attn_decode(kc0, vc0, T, B, Hkv, dev(q), scaling, splits=2)
-    assert ops.read_status(st) == 0 and torch.equal(out, out0)
+    out0, st = ops.attn_decode(kc0, vc0, T, B, Hkv, dev(q), scaling, **kw)
+    assert ops.read_status(st) == 0
+    if G > 1 and kw["splits"] == 1:                      # larger slots, fewer workers: another cut of the column's steps
+        assert_attn_close(out0, out.double().cpu().numpy())
+    else:
+        assert torch.equal(out, out0)
     # shift both streams by 3 bytes
     ek = torch.zeros(rk["n"] + 64, dtype=torch.uint8, device="cuda"); ek[3:3 + rk["n"]] = rk["enc"][:rk["n"]]
     ev = torch.zeros(rv["n"] + 64, dtype=torch.uint8, device="cuda"); ev[3:3 + rv["n"]] = rv["enc"][:rv["n"]]
     kc1 = ops.make_cache(ek[3:], rk["bi"], rk["ti"], rk["book"], rk["mi"], rk["sc"], rk["spec"], rk["n"], rk["maxb"])
     vc1 = ops.make_cache(ev[3:], rv["bi"], rv["ti"], rv["book"], rv["mi"], rv["sc"], rv["spec"], rv["n"], rv["maxb"])
-    out1, st = ops.attn_decode(kc1, vc1, T, B, Hkv, dev(q), scaling, splits=2)
+    out1, st = ops.attn_decode(kc1, vc1, T, B, Hkv, dev(q), scaling, **kw)
     assert ops.read_status(st) == 0 and torch.equal(out, out1)
 
 
