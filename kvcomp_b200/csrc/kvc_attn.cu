@@ -5,8 +5,8 @@
 // v_huffman_decode_and_mat_vec_mul (kernels.cu:778-861); attention semantics of
 // eager_attention_forward (models/llama.py:211-234).
 //
-// Work layout (grouped queries in the attention kernel: see attn_rows_kernel): CTA = 256 threads working on 256 tokens
-// of one (b, kv head).
+// Work layout of the unfused kernels and of the attention kernel with one query head per KV head (with several: see
+// attn_rows_kernel): CTA = 256 threads working on 256 tokens of one (b, kv head).
 //   K phase: thread = token; its vector holds the token's 128 channel codes.
 //            score = sum_c code_c * w[c] + zp, with w[c] = q[c]*scale[c] staged per 64-token block
 //            (dequantisation folded into the weights, the min_int term summed once per block).
@@ -20,12 +20,11 @@
 // each leaves a partial result (max, sum, accumulators) and a second kernel merges them.
 // Both phases are "decode 128 symbols and dot them with a shared 128-vector", so they share one
 // decoder.  The shared vector is held in 16-bit block fixed point (one fp32 step per vector, value
-// = step * (256*hi + lo), hi signed and lo unsigned bytes): every table lookup yields up to four
-// symbols as four bytes, and two dp4a instructions multiply them with the four matching weight
-// bytes -- integer arithmetic, exact, accumulated in int32.  The only rounding is that of the
+// = step * (256*hi + lo), hi signed and lo unsigned bytes): every table lookup yields up to three
+// symbols as bytes, and two dp4a instructions multiply them with the matching weight bytes -- integer arithmetic, exact, accumulated in int32.  The only rounding is that of the
 // weights (2^-16 of the largest weight of the vector); the zero-point terms and everything after
-// the dot product are fp32.  With grouped-query attention the G query heads of a KV head share
-// every decode: weight records are stored [position][G].
+// the dot product are fp32.  With several query heads per KV head they share every decode: in the unfused
+// kernels by weight records [position][G], up to four heads a launch.
 #include <math_constants.h>
 
 #include <algorithm>
@@ -92,7 +91,8 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 // same as in the one-pass form.  What bounds it is the issue rate: the chains of dependent lookups leave slots empty, and
 // shared memory (tables, slots, rows) limits an SM to 16 or 20 warps.  Against byte stores and four dp4a pairs per word:
 // 1777 -> 1000 shared-memory wavefronts per warp and 256 tokens.  One layer of 16 sequences x 32768 tokens, 8 x 4 heads,
-// rel 0.05 / 0.1: 981 us -> 822 us with the rows in two CTAs of 256 threads -> 735 us with attn_rows_kernel's workers.
+// rel 0.05 / 0.1: 981 us -> 822 us with the rows in two CTAs of 256 threads -> 735 us with attn_rows_kernel's workers, 720 with
+// the trees out of shared memory and sums in place of ORs.
 // Rows of 36 words: 128 symbols, the overrun of paired lookups, and a 16-byte alignment at which the fragment
 // loads (16 bytes of row 4r+i by lane 4r+q) touch every bank once per quarter warp.
 constexpr int ROW_WORDS = 36;
@@ -566,16 +566,15 @@ __global__ void __launch_bounds__(NTHR, 6) fused_pv_kernel(CacheDev vc, long lon
 }
 
 // ---- one-pass decode attention -------------------------------------------------------------------
-template <int G>
-struct alignas(32) AttnSmem {                     // followed in shared memory by 4 K slots, 4 V slots (sized at launch),
+struct alignas(32) AttnSmem {                     // of the one-head kernel; followed in shared memory by 4 K slots, 4 V slots (sized at launch),
     KvcBookSmem bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
-    alignas(32) uint32_t w[4 * 2 * WROW * G];     // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum
-    alignas(32) uint32_t ps[2 * 2 * WROW * G];    // V weight words
-    float kstep[4 * G], zp[4 * G];
-    float vstep[2 * G];
-    float qf[G * 128];
-    float qsum[G];
-    float red[4][8 * G];              // per-warp max, sum, zpv and weight-max partials
+    alignas(32) uint32_t w[4 * 2 * WROW];     // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum
+    alignas(32) uint32_t ps[2 * 2 * WROW];    // V weight words
+    float kstep[4], zp[4];
+    float vstep[2];
+    float qf[128];
+    float qsum[1];
+    float red[4][8];                  // per-warp max, sum, zpv and weight-max partials
     uint64_t bar[2];                  // K and V staging barriers
     uint32_t leadK[4], leadV[4];
     uint32_t nbK[4], nbV[4];          // byte counts of the staged blocks
@@ -586,19 +585,20 @@ struct alignas(32) AttnSmem {                     // followed in shared memory b
 
 struct AttnParams {
     CacheDev k, v;
-    long long T, B, Hkv, Hq, g0, Tr;
-    int nh;                       // query heads of this launch (per KV head, from g0): 1 .. G
+    long long T, B, Hkv, Hq, Tr;
+    long long g0;                 // first query head of this launch (of each KV head): 0 in the one-head kernel
+    int nh;                       // and how many, 1 .. G
     const __half *q, *ktail, *vtail;
     __half *out;
     float scaling;
-    int n_tiles;                  // 256-token tiles per column
+    int n_tiles;                  // tiles per column: of 256 tokens, with grouped queries steps of 128
     // every column is cut into `long_runs` runs of `tiles_per_split` tiles followed by `splits - long_runs`
     // runs of `short_tiles` tiles; the items of the long runs of all columns come first, the short ones last
     int splits, tiles_per_split, long_runs, short_tiles;
     long long work;               // columns * splits items
     uint32_t slotK_bytes, slotV_bytes;   // capacity of one staging slot (multiple of 16)
-    float *ws_part;               // [B*Hq][splits][ATTN_PART_FLOATS]
-    int *sched;                   // {items handed out, CTAs finished}, or null: static shares
+    float *ws_part;               // [B*Hq][splits][ATTN_PART_FLOATS], with grouped queries [..][ROWS_PART_FLOATS]
+    int *sched;                   // {items handed out, CTAs (grouped queries: workers) finished}, or null: static shares
     int *status;
     int team;                     // grouped queries without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
@@ -606,12 +606,15 @@ struct AttnParams {
     int starve;                   // tests of the bounded waits only: announce bytes that are never copied
 };
 
-// One query head per KV head (G = 1).  BULK: stage with bulk asynchronous copies (one tile phase ahead) instead of plain loads.
-template <int G, bool BULK>
+// One query head per KV head.  BULK: stage with bulk asynchronous copies (one tile phase ahead) instead of plain loads.
+// (The per-head values are arrays of one: as plain scalars the same kernel gets another register allocation, with 12 bytes of
+// spills: K units per block 2.7 % faster, K at relative bound 0.01 1.2 % slower, 128 columns of 8192 tokens with a tail 1.9 %.)
+template <bool BULK>
 __global__ void __launch_bounds__(NTHR, 3) attn_decode_kernel(AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    AttnSmem<G> &sm = *reinterpret_cast<AttnSmem<G> *>(smem_raw);
-    uint8_t *const slotsK = smem_raw + sizeof(AttnSmem<G>), *const slotsV = slotsK + 4 * p.slotK_bytes;
+    constexpr int G = 1;
+    AttnSmem &sm = *reinterpret_cast<AttnSmem *>(smem_raw);
+    uint8_t *const slotsK = smem_raw + sizeof(AttnSmem), *const slotsV = slotsK + 4 * p.slotK_bytes;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
     const int grp = tid >> 7, ch = tid & 127;
     // Launched with programmatic stream serialisation.  This kernel's own set-up -- the books' tables, the first
@@ -957,8 +960,9 @@ __global__ void __launch_bounds__(NTHR, 3) attn_decode_kernel(AttnParams p) {
 // A worker is four warps with slots, rows, weights and barriers of its own; it draws items like a CTA of the one-head
 // kernel and walks them in steps of 128 tokens (two K blocks, the two V blocks of a column).  The tables take 32 KB
 // and a worker 35 to 45 KB: two CTAs of 256 threads with a copy each held four workers' worth of warps, and all eight
-// warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads; 448 and 404 us at
-// 32 x 16384 tokens, 4 x 2 heads).
+// warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads, now 720; 448 and 404 us at
+// 32 x 16384 tokens, 4 x 2 heads, now 360).  Registers: 96 with two and four columns, where the compiler spills 60 to 70 bytes
+// per thread (five workers leave no more), 128 without spills with eight.
 constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]; two of them take the room of one of the one-head kernel
 static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "the workspace is sized in the one-head kernel's partial results");
 template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : 5; }
@@ -991,7 +995,8 @@ int rows_fit(const AttnParams &p, int heads) { return heads > 4 ? rows_fit<8>(p)
 // How many of an SM's workers share a column when every column's output is written directly (no workspace, or a single run
 // without a tail): without company a worker would take all of a column's `units` (steps and passes of the tail) in turn
 // while most of the device is idle.  A unit takes about 6 + a parts of time with `a` workers at work on the SM (2 heads: 9.2 us
-// alone, 14.4 us with five).  2 heads per column, no workspace, a worker per column against teams: 8 columns of 1024 tokens
+// alone, 14.4 us with five), a team's sums and its next column another 3.5: over 1 to 700 columns of 2 to 19 units the choice is
+// within 1 % of the best size on average, and nowhere behind a worker per column.  2 heads per column, no workspace, a worker per column against teams: 8 columns of 1024 tokens
 // 77.6 and 31.5 us, 64 of 8192 594 and 189 us, 256 of 256 (two teams of two on an SM) 26.1 and 19.6 us.
 int rows_team(long long cols, long long units, int workers, int sms) {
     if (cols >= (long long)workers * sms) return 0;          // enough columns for all
@@ -999,7 +1004,7 @@ int rows_team(long long cols, long long units, int workers, int sms) {
     long long least = 0;
     for (int size = 1; size <= workers && size <= units; size++) {
         const long long teams = std::min<long long>(workers / size, (cols + sms - 1) / sms);     // of an SM
-        const long long cost = ((cols + teams * sms - 1) / (teams * sms)) * ((units + size - 1) / size) * (6 + teams * size);
+        const long long cost = ((cols + teams * sms - 1) / (teams * sms)) * (2 * ((units + size - 1) / size) * (6 + teams * size) + (size > 1 ? 7 : 0));
         if (size == 1 || cost < least) { least = cost; best = size > 1 ? size : 0; }
     }
     return best;
@@ -1770,10 +1775,10 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     const int sms = kvc_sm_count();
     const long long Gt = Hq / Hkv;
     if (Gt == 1 && T > 0) {
-        const size_t smem = slot_total + sizeof(AttnSmem<1>);
+        const size_t smem = slot_total + sizeof(AttnSmem);
         p.g0 = 0; p.nh = 1;
         static kvc_launch_slot slots[2];
-        auto *kernel = bulk ? attn_decode_kernel<1, true> : attn_decode_kernel<1, false>;
+        auto *kernel = bulk ? attn_decode_kernel<true> : attn_decode_kernel<false>;
         int occ = 0;
         if (int rc = kvc_prepare(slots[bulk], reinterpret_cast<const void *>(kernel), NTHR, smem, &occ)) return rc;
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);
@@ -1789,7 +1794,10 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         const long long most = (long long)rows_fit(p, heads) * sms;                         // workers of a full device
         if (p.partial && ws_parts) {
             RunPlan r = {0, 0, 0, 0};
-            if (asked <= 0) r = plan_runs(p.n_tiles, cols, most);
+            // (the plan counts five workers per SM also where the launch has fewer: the items are finer for it.  8 heads, four
+            // workers: 16 x 8 columns of 16384 tokens 412 us, with a plan for four 423; 32 x 2 columns 217 and 224.  Three workers, as the
+            // stream's largest block is unknown: 484 and 490 us, but 16 x 8 columns of 4096 tokens 144 and 137.)
+            if (asked <= 0) r = plan_runs(p.n_tiles, cols, (long long)rows_workers<4>() * sms);
             // The caller's runs in halves where that is fewer steps one after the other: a worker takes a run's steps in turn, each
             // with half the threads a CTA of the one-head kernel has for its tile.  (32 columns, 2 heads each, 2048 tokens in 4
             // runs: 46.9 us, in halves 33.7; 64 columns in 8 runs: 36.0, in halves 42.2, as the halves no longer go in one round.)
@@ -1804,7 +1812,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         p.work = cols * splits;
         for (long long g0 = 0; g0 < Gt; g0 += p.nh) {
             // Heads per launch: every launch decodes the whole cache, so up to 8 go together, in launches of equal shares.
-            // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 461 us in two launches of 4, 244 us in one.)
+            // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 461 us in two launches of 4, 217 us in one.)
             const long long launches = (Gt - g0 + 7) / 8;
             p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
 #define KVC_AT(GG)                                                                                              \
