@@ -471,7 +471,7 @@ def side_workloads(ops, torch, device, seed, names=("c2", "c3"), layers=2):
                      "tokens_per_s_full_model": B / (ms_layer * WORKLOADS[name]["layers"] / 1e3),
                      "algorithmic_bytes_per_layer": alg, "achieved_GBps": alg / ms_layer / 1e6, "frac_of_hbm_peak": alg / ms_layer / 1e6 / peak,
                      "effective_fp16_GBps": 2 * 2 * T * B * Hkv * 128 / ms_layer / 1e6,
-                     "launches_per_layer": sum(1 for _ in _chunks(Hq // Hkv)) + 1,
+                     "launches_per_layer": attn_launches(Hq // Hkv) + 1,
                      "bits_per_symbol": {k: float(np.mean([8.0 * b[3][k]["encoded"] / b[3][k]["symbols"] for b in built])) for k in ("k", "v")}}
         del built, ws, outs
         torch.cuda.empty_cache()
@@ -797,7 +797,7 @@ def main():
     outs = [out_all[i] for i in range(L)]
     gather_buf = torch.empty((world, L, B, Hq, 128), dtype=torch.float16, device=device) if heads_mode else None
     scaling = 1.0 / math.sqrt(128)
-    launches_per_call = sum(1 for _ in _chunks(Hq // Hkv))
+    launches_per_call = attn_launches(Hq // Hkv)
 
     def step():
         for (caches, _, q), out in zip(layers, outs):
@@ -926,11 +926,9 @@ def main():
         dist.destroy_process_group()
 
 
-def _chunks(g):
-    while g > 0:
-        c = 4 if g >= 4 else (2 if g >= 2 else 1)
-        yield c
-        g -= c
+def attn_launches(g):
+    """Launches of the attention kernel for g query heads per KV head (up to 8 share one; the merge kernel comes on top)."""
+    return -(-g // 8)
 
 
 if __name__ == "__main__":

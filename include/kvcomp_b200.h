@@ -241,14 +241,19 @@ int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hkv, int64_t 
  * [B,Hq,128].  Scores never leave the SM; no fp16 K/V is written to memory.
  * Work is cut into items, one (sequence, KV head) column x one of `splits` equal runs of
  * 256-token tiles (with several query heads per KV head and room for partial results: where it pays, runs
- * of its own choice, at most twice as many, in the same workspace); as many CTAs as the device holds at once take items until none is left,
- * and a second small kernel merges the `splits` partial results of every head and adds the
+ * of its own choice, at most twice as many, in the same workspace; without partial results: where it pays, a
+ * column shared by several workers of a CTA); as many CTAs as the device holds at once take items until none
+ * is left, and a second small kernel merges the `splits` partial results of every head and adds the
  * tail's tokens (it does the whole step when T = 0).  splits = 0
  * picks kvc_attn_splits(T, B, Hkv, 0).  workspace: kvc_attn_workspace(B, Hq, splits) bytes
  * of device memory whose first 256 bytes the caller zeroes once before the first use (the
  * kernel leaves them zeroed); NULL is allowed when splits = 1 (a tail then costs more: the
  * first kernel reads it itself, a column's CTA at a time).  Launches that share a
- * workspace must not overlap on the device. */
+ * workspace must not overlap on the device.
+ * The launch uses programmatic stream serialisation: it may read what k and v point to (streams, tables, books,
+ * unit parameters) while the kernel directly ahead of it in the stream ends.  That kernel may write q, the tails and
+ * anything else, but a kernel that writes the caches' memory needs an ordinary kernel, a copy or a host wait behind
+ * it before the launch (kvc_encode's byte count is read back anyway). */
 int64_t kvc_attn_workspace(int64_t B, int64_t Hq, int splits);
 int kvc_attn_splits(int64_t T, int64_t B, int64_t Hkv, int sm_count);
 int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T, int64_t B, int64_t Hkv, int64_t Hq,

@@ -110,8 +110,7 @@ def test_synth_is_seeded_and_shaped():
 def test_bench_accounting_helpers():
     sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     import bench
-    assert list(bench._chunks(1)) == [1] and list(bench._chunks(4)) == [4] and list(bench._chunks(6)) == [4, 2]
-    assert list(bench._chunks(5)) == [4, 1]
+    assert [bench.attn_launches(g) for g in (1, 4, 5, 8, 9, 16, 17)] == [1, 1, 1, 1, 2, 2, 3]
     cfg = bench.WORKLOADS["c1"]
     acct = {"k": dict(encoded=100, block_info=8, thread_info=128, quant_meta=3),
             "v": dict(encoded=50, block_info=8, thread_info=128, quant_meta=3)}
