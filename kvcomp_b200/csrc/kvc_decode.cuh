@@ -17,11 +17,20 @@ struct KvcBookSmem {                      // per-CTA copy of the decode structur
     uint32_t lut[KVC_LUT_SIZE];
 };
 
+// The decode table as the loop below wants it: a book's entries {(symbols << 6) | bits, s0, s1, s2} with 16 - bits in place
+// of the bits (an entry without a complete code: no symbols, still told by bits 6-7).
+__device__ __forceinline__ void kvc_load_lut(uint32_t *lut, const void *book, int tid, int nthr) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_LUT);
+    auto form = [](uint32_t e) { return e + 16u - 2u * (e & 63u); };
+    for (int i = tid; i < KVC_LUT_SIZE / 4; i += nthr) {
+        const uint4 e = src[i];
+        reinterpret_cast<uint4 *>(lut)[i] = make_uint4(form(e.x), form(e.y), form(e.z), form(e.w));
+    }
+}
 __device__ __forceinline__ void kvc_load_book(KvcBookSmem &b, const void *book, int tid, int nthr) {
     const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_TREE);
-    uint4 *dst = reinterpret_cast<uint4 *>(&b);
-    constexpr int N16 = (int)(sizeof(KvcBookSmem) / 16);
-    for (int i = tid; i < N16; i += nthr) dst[i] = src[i];
+    for (int i = tid; i < 512 / 4; i += nthr) reinterpret_cast<uint4 *>(b.tree)[i] = src[i];
+    kvc_load_lut(b.lut, book, tid, nthr);
 }
 
 // the wide decode tree, read only for codes longer than the table's window
@@ -34,11 +43,6 @@ struct KvcTreeGlobal {                    // for kernels short of shared memory
     __device__ __forceinline__ KvcTreeGlobal(const void *book) : nodes(reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_TREE)) {}
     __device__ __forceinline__ uint32_t operator()(uint32_t node) const { return nodes[node]; }
 };
-// the table alone
-__device__ __forceinline__ void kvc_load_lut(uint32_t *lut, const void *book, int tid, int nthr) {
-    const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_LUT);
-    for (int i = tid; i < KVC_LUT_SIZE / 4; i += nthr) reinterpret_cast<uint4 *>(lut)[i] = src[i];
-}
 
 // Copy the bytes [off, off+n) of `encoded` into `slot` so that slot and source agree modulo 16:
 // the first stream byte lands at slot[lead], lead = address & 15.  Whole 16-byte chunks inside the
@@ -125,10 +129,18 @@ __device__ __forceinline__ bool kvc_book_needs_escape(const void *book) {
     return reinterpret_cast<const kvc_book_header *>(book)->escape != 0;    // set for a code beyond the window too
 }
 
-// Decode one vector.  slot_s: shared-space address of the staged block (16-byte aligned); byte_pos:
-// where the vector starts in it; lut_s: shared-space address of the book's table; tree: its tree (KvcTree*).
-// The decoder state is (position << 6) | bit offset into the (hi, lo) register pair, so applying a
-// table entry is one add of its low byte.
+// Decode one vector.  slot_s: shared-space address of the staged block (16-byte aligned; the word before it is readable);
+// byte_pos: where the vector starts in it; lut_s: shared-space address of the book's table (kvc_load_lut's form); tree: its
+// tree (KvcTree*).
+// The stream's next bits lie in the register pair (hi, lo), `off` bits from its top; the decoder state is (position << 6) | f
+// with f = 34 - off, kept in 0..31: `(hi, lo) >> f` then has the next 30 bits below bit 30, the first window's table offset is
+// one shift and one mask away, and the second one's too, as a table entry's low five bits are the shift (16 - bits consumed)
+// that brings the bits behind it to the same place.  Both windows of a round lie in that one word, so nothing is chosen in between
+// and the chain from one lookup to the next is a shift and a mask.  Applying an entry is one add of its low byte; the two
+// 16s of a round are the 32 that a refill (or clearing bit 5) takes off again.
+// (What bounds a decode loop is issue and the shared-memory pipe together with the chain of lookups.  With the second window cut
+// from words chosen by the state, one more shift per window and an end test per round: attention over 16 x 32768 tokens, 8 x 4
+// heads, 724 us, now 652; one head, 8 x 4096 tokens, 142 and 135.)
 // emit(e, a, s0, s1): `e` holds up to three symbols in bytes 1..3 for positions c..c+2 of the vector (unused
 // bytes are 0; byte 0 is the table entry's advance byte: its bits 6-7 count the symbols); a = (base + c) << SHIFT:
 // the position counter starts at `base`, so a consumer that keeps one record of 2^SHIFT bytes per
@@ -145,72 +157,66 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
                                                   uint32_t base, Emit emit) {
     static_assert(SHIFT >= 0 && SHIFT <= 6, "record size");
     constexpr uint32_t AMASK = 0xffffffffu << SHIFT;       // drops the bit-offset bits left below the position
+    constexpr uint32_t WMASK = (KVC_LUT_SIZE - 1) << 2;
     const uint32_t end = (base + KVC_VEC_LEN) << 6;
-    uint32_t ptr = slot_s + (byte_pos & ~3u);
-    uint32_t state = (base << 6) | ((byte_pos & 3u) << 3);
-    uint32_t hi = kvc_bswap(kvc_lds32(ptr)), lo = kvc_bswap(kvc_lds32(ptr + 4)), nx = kvc_bswap(kvc_lds32(ptr + 8));
+    const uint32_t before = slot_s + byte_pos - 1;         // off = 8, 16, 24 or 32: hi is the word that holds this byte
+    uint32_t ptr = before & ~3u;
+    uint32_t state = (base << 6) | (26u - ((before & 3u) << 3));
+    uint32_t hi = kvc_bswap(kvc_lds32(ptr)), lo = kvc_bswap(kvc_lds32(ptr + 4)), nx = kvc_lds32(ptr + 8);
     ptr += 12;
-    // Two lookups per round.  The first leaves the bit offset below 32 + KVC_LUT_BITS, so the second one's window still
-    // lies inside (hi, lo) or (lo, next word) and needs no refill in between: one refill test and one end test per
-    // pair.  The second lookup may run although the first finished the vector, so up to KVC_DECODE_OVERRUN positions
-    // past 127 are emitted.
+    auto refill = [&](uint32_t s) {                        // s: the state after a round, 32 more than the bits say
+        if (!(s & 32u)) { hi = lo; lo = kvc_bswap(nx); nx = kvc_lds32(ptr); ptr += 4; }
+        state = s & ~32u;
+    };
     if (!ESC) {
-        do {
-            const uint32_t w0 = __funnelshift_l(lo, hi, state);
-            const uint32_t e0 = kvc_lds32(lut_s + ((w0 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
+        auto round = [&]() {
+            const uint32_t t = __funnelshift_r(lo, hi, state);
+            const uint32_t e0 = kvc_lds32(lut_s + ((t >> 16) & WMASK));
+            const uint32_t e1 = kvc_lds32(lut_s + (__funnelshift_r(t, 0u, e0) & WMASK));
             const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);   // state + byte 0 of e0, off the integer ALU pipe
             emit(e0, (state >> (6 - SHIFT)) & AMASK, state, s1);
-            state = s1;
-            const bool up = (state & 32u) != 0;
-            const uint32_t w1 = __funnelshift_l(up ? nx : lo, up ? lo : hi, state);
-            const uint32_t e1 = kvc_lds32(lut_s + ((w1 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-            const uint32_t s2 = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)state);
-            emit(e1, (state >> (6 - SHIFT)) & AMASK, state, s2);
-            state = s2;
-            if (state & 32u) { hi = lo; lo = nx; nx = kvc_bswap(kvc_lds32(ptr)); ptr += 4; state -= 32u; }
-        } while (state < end);
+            const uint32_t s2 = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)s1);
+            emit(e1, (s1 >> (6 - SHIFT)) & AMASK, s1, s2);
+            refill(s2);
+        };
+        // A round emits six symbols at most: the first 21 need no test of the end.  (Attention, 16 x 32768 tokens, 8 x 4 heads: every
+        // round tested 670 us, the 21 in threes 656, in sevens 652; one head, 8 x 4096 tokens: 140, 138, 135.)
+#pragma unroll 7
+        for (int i = 0; i < (KVC_VEC_LEN - 1) / 6; i++) round();
+        do round(); while (state < end);
         return true;
     }
     // The same with a test of each entry; a long code ends its round.  (One lookup per round: one head, rel 0.01 / 0.02,
     // 8 x 4096 tokens, 309 us against 286.)
     bool ok = true;
-    auto refill = [&]() { if (state & 32u) { hi = lo; lo = nx; nx = kvc_bswap(kvc_lds32(ptr)); ptr += 4; state -= 32u; } };
-    // a code longer than the window: on from the node the entry names, one bit at a time (the offset is below 32 +
-    // KVC_LUT_BITS here, and below 64 with the window's bits)
+    // a code longer than the window: on from the node the entry names, one bit at a time
     auto long_code = [&](uint32_t e) {
         uint32_t node = e >> 8, sym = 0;
         bool found = false;
-        const uint32_t a = (state >> (6 - SHIFT)) & AMASK;
-        state += KVC_LUT_BITS;
+        refill(state + 32u - KVC_LUT_BITS);
         for (int guard = 0; guard < 40; guard++) {
-            refill();
             if (node >= 512u) break;
             const uint32_t nd = tree(node);
             if ((nd & 0xffffu) == KVC_TREE_LEAF) { sym = nd >> 16; found = true; break; }
-            const uint32_t bit = __funnelshift_l(lo, hi, state) >> 31;
-            state += 1u;
+            const uint32_t bit = (__funnelshift_r(lo, hi, state) >> 29) & 1u;
+            refill(state + 31u);
             node = (nd >> (16 * bit)) & 0xffffu;
         }
         ok = ok && found;
-        emit((sym << 8) | (1u << 6), a, state, state + (1u << 6));     // advance byte: one symbol
+        emit((sym << 8) | (1u << 6), (state >> (6 - SHIFT)) & AMASK, state, state + (1u << 6));     // advance byte: one symbol
         state += 1u << 6;
-        refill();
     };
     do {
-        const uint32_t w0 = __funnelshift_l(lo, hi, state);
-        const uint32_t e0 = kvc_lds32(lut_s + ((w0 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-        if ((e0 & 0xffu) == 0) { long_code(e0); continue; }
+        const uint32_t t = __funnelshift_r(lo, hi, state);
+        const uint32_t e0 = kvc_lds32(lut_s + ((t >> 16) & WMASK));
+        if ((e0 & 0xc0u) == 0) { long_code(e0); continue; }
+        const uint32_t e1 = kvc_lds32(lut_s + (__funnelshift_r(t, 0u, e0) & WMASK));
         const uint32_t s1 = (uint32_t)kvc_dp4a_uu(e0, 1u, (int)state);
         emit(e0, (state >> (6 - SHIFT)) & AMASK, state, s1);
-        state = s1;
-        const bool up = (state & 32u) != 0;
-        const uint32_t w1 = __funnelshift_l(up ? nx : lo, up ? lo : hi, state);
-        const uint32_t e1 = kvc_lds32(lut_s + ((w1 >> (32 - KVC_LUT_BITS - 2)) & ((KVC_LUT_SIZE - 1) << 2)));
-        if ((e1 & 0xffu) == 0) { if (state < end) long_code(e1); continue; }
-        const uint32_t s2 = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)state);
-        emit(e1, (state >> (6 - SHIFT)) & AMASK, state, s2);
-        state = s2;
-        refill();
+        if ((e1 & 0xc0u) == 0) { refill(s1 + 16u); if (state < end) long_code(e1); continue; }
+        const uint32_t s2 = (uint32_t)kvc_dp4a_uu(e1, 1u, (int)s1);
+        emit(e1, (s1 >> (6 - SHIFT)) & AMASK, s1, s2);
+        refill(s2);
     } while (state < end);
     return ok;
 }
