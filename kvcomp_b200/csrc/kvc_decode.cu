@@ -1,67 +1,104 @@
 // Blocked Huffman decoder to uint8 codes (kernels.cu:602-719 restated for sm_100a).
 //
-// CTA = 256 threads = 4 blocks of 64 vectors per round, grid-stride over block groups so that the
-// decode table is brought into shared memory once per CTA.  Thread = one vector; decoded symbols
-// go to a shared-memory tile and leave as coalesced stores (K: rows, V: transposed back), as codes or,
-// for a reader of values, already dequantised: the codes then never reach memory.  Reading back K and V of 8 sequences
-// x 4096 tokens x 32 heads (decode, dequantise): 802 us in two launches per tensor, 361 us in one (the kernels 130 us each).
-// (VALUES: 48 registers, 16 bytes of spills; shared memory -- table, tree, slots, tiles -- lets three CTAs share an SM.)
+// One CTA per SM around one copy of the decode table; its workers are pairs of warps, a pair takes one block of 64 vectors
+// after the other.  Thread = one vector; decoded symbols go to a shared-memory tile and leave as coalesced stores (K: rows,
+// V: transposed back), as codes or, for a reader of values, already dequantised: the codes then never reach memory.  The next
+// block's bytes are brought by a bulk copy while the tile goes out, and only the pair's own 64 threads wait for each other.
+// Reading back K and V of 8 sequences x 4096 tokens x 32 heads: 353 us with CTAs of 256 threads that staged, decoded and wrote
+// four blocks between barriers of their own, three to an SM with a table each; now 309.
 #include "kvc_decode.cuh"
 
 namespace {
 
 constexpr int TILE_STRIDE = 140;          // 128 symbols + KVC_DECODE_OVERRUN rounded up to words, + 1 word; 35 words keep column reads off one bank
-
-struct DecodeSmem {                         // followed by 4 staging slots (sized at launch), then the 4 tiles
-    KvcBookSmem book;
-};
 constexpr int TILE_BYTES = 64 * TILE_STRIDE; // a tile; the tiles are also the padding a corrupt stream's overrun reads land in
+constexpr int MAX_PAIRS = 15;             // named barriers 1 .. 15
+
+struct DecodeSmem {                         // followed by a staging slot per pair (sized at launch), then a tile per pair
+    alignas(16) uint32_t lut[KVC_LUT_SIZE];   // the tree, for codes beyond the window, stays in global memory
+    uint64_t bar[MAX_PAIRS + 1];
+    int dead[MAX_PAIRS + 1];
+};
+static_assert(sizeof(DecodeSmem) % 16 == 0, "slots are 16-byte aligned");
 
 // VALUES: fp16 values [T, cols, 128] instead of the codes.  The units either do not depend on the channel (m.sc == 0), or
-// (K) lie side by side over the channels and cover whole blocks of 64 tokens.
-template <bool VALUES>
-__global__ void __launch_bounds__(256) decode_kernel(
+// (K) lie side by side over the channels and cover whole blocks of 64 tokens.  BULK: the stream starts on 16 bytes.
+template <bool VALUES, bool BULK>
+__global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
     const uint8_t *__restrict__ encoded, long long encoded_bytes, const uint2 *__restrict__ block_info,
     const uint16_t *__restrict__ thread_info, const void *__restrict__ book, long long nblk, long long cols, int is_k,
-    uint32_t max_block, uint32_t slot_bytes, uint8_t *__restrict__ codes, kvc_qmeta_dev m, long long H,
+    uint32_t max_block, uint32_t slot_bytes, int pairs, uint8_t *__restrict__ codes, kvc_qmeta_dev m, long long H,
     __half *__restrict__ values, int *__restrict__ status) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     DecodeSmem &sm = *reinterpret_cast<DecodeSmem *>(smem_raw);
-    uint8_t *const slots = smem_raw + sizeof(DecodeSmem), *const tiles = slots + 4 * slot_bytes;
-    const bool esc = kvc_book_needs_escape(book);           // uniform over the grid
-    const int tid = threadIdx.x, sub = tid >> 6, v = tid & 63;      // sub-block and vector of this thread
-    const long long row = cols * 128;
-    kvc_load_book(sm.book, book, tid, 256);
+    const int pair = threadIdx.x >> 6, v = threadIdx.x & 63;        // v: the thread's vector of the block
+    uint8_t *const slot = smem_raw + sizeof(DecodeSmem) + pair * slot_bytes;
+    uint8_t *const tile = smem_raw + sizeof(DecodeSmem) + pairs * slot_bytes + pair * TILE_BYTES;
+    const long long row = cols * 128, step = (long long)gridDim.x * pairs;
+    const KvcTreeGlobal tree(book);
+    auto sync = [&]() { asm volatile("bar.sync %0, 64;" :: "r"(pair + 1) : "memory"); };    // the pair's threads
     int flags = 0;
-    for (long long grp = blockIdx.x; grp * 4 < nblk; grp += gridDim.x) {
-        const long long blk = grp * 4 + sub;
-        const bool active = blk < nblk;
-        uint32_t lead = 0, nbytes = 0;
-        __syncthreads();                       // previous round's tile and slot are free (and the book is in)
-        if (active) {
-            const uint2 bi = block_info[blk];
-            nbytes = bi.y & 0xffffu;
-            if (nbytes > max_block || (long long)bi.x + nbytes > encoded_bytes) { nbytes = 0; flags |= KVC_FLAG_BAD_STREAM; }
-            lead = kvc_stage_block(slots + sub * slot_bytes, encoded, encoded_bytes, bi.x, nbytes, v, 64);
+    // a block's record, and from it the bytes [lead, lead + nbytes) of the slot (0 bytes: nothing to decode)
+    auto info_of = [&](long long blk) { return blk < nblk ? block_info[blk] : make_uint2(0u, 0u); };
+    auto block_of = [&](uint2 bi, uint32_t &nbytes, uint32_t &lead, const uint8_t *&src) {
+        nbytes = 0; lead = 0; src = encoded;
+        const uint32_t n = bi.y & 0xffffu;
+        if (n > max_block || (long long)bi.x + n > encoded_bytes) { flags |= KVC_FLAG_BAD_STREAM; return; }
+        nbytes = n; src = encoded + bi.x; lead = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
+    };
+    auto start_of = [&](long long blk) { return v && blk < nblk ? (uint32_t)(thread_info[blk * 64 + v - 1] >> 3) : 0u; };
+    // by the pair's first thread: one arrival per phase, even for 0 bytes.  The source widens to 16-byte boundaries (the stream
+    // starts on one, so that these lie inside its memory).
+    auto fetch = [&](const uint8_t *src, uint32_t nbytes, uint32_t lead) {
+        const uint32_t bytes = nbytes ? (lead + nbytes + 15u) & ~15u : 0u;
+        kvc_mbar_expect_tx(&sm.bar[pair], bytes);
+        if (bytes) kvc_bulk_g2s(slot, src - lead, bytes, &sm.bar[pair]);
+    };
+    if (BULK && v == 0 && pair < pairs) { kvc_mbar_init(&sm.bar[pair], 1); kvc_mbar_fence_init(); sm.dead[pair] = 0; }
+    // neighbouring pairs of the grid take neighbouring blocks
+    long long blk = (long long)blockIdx.x * pairs + pair;
+    uint32_t nbytes = 0, lead = 0;
+    const uint8_t *src = encoded;
+    if (pair < pairs) {
+        block_of(info_of(blk), nbytes, lead, src);
+        if (BULK && v == 0) fetch(src, nbytes, lead);
+    }
+    uint32_t start = pair < pairs ? start_of(blk) : 0u;
+    kvc_load_lut(sm.lut, book, threadIdx.x, blockDim.x);
+    const bool esc = kvc_book_needs_escape(book);           // uniform over the grid
+    __syncthreads();                                        // the table and the barriers are in; from here on the pairs go their own ways
+    if (pair >= pairs) return;
+    uint32_t par = 0;
+    for (; blk < nblk; blk += step) {
+        const uint2 next = info_of(blk + step);
+        bool landed = true;
+        if (BULK) {
+            // a wait that runs out: the thread does not decode; a barrier whose phase its issuer did not see complete is
+            // never armed again, and the pair stops
+            landed = kvc_mbar_wait(&sm.bar[pair], par);
+            par ^= 1u;
+            if (!landed) { flags |= KVC_FLAG_WAIT_TIMEOUT; if (v == 0) sm.dead[pair] = 1; }
+        } else {
+            if (nbytes) kvc_stage_block(slot, encoded, encoded_bytes, src - encoded, nbytes, v, 64);
+            sync();
         }
-        __syncthreads();
-        if (active && nbytes) {
-            const uint32_t start = v ? (uint32_t)(thread_info[blk * 64 + v - 1] >> 3) : 0u;
-            uint8_t *trow = tiles + sub * TILE_BYTES + v * TILE_STRIDE;
-            bool ok = start < nbytes;
+        if (nbytes) {
+            bool ok = landed && start < nbytes;
             // the symbols collect in a word that is stored when its last byte is known; symbols past position 127
             // (at most KVC_DECODE_OVERRUN) stay within the row's padding words
             KvcRowWriter put;
-            const uint32_t slot_s = kvc_smem_addr(slots + sub * slot_bytes), lut_s = kvc_smem_addr(sm.book.lut),
-                           row_s = kvc_smem_addr(trow);
-            const KvcTreeShared tree{kvc_smem_addr(sm.book.tree)};
+            const uint32_t slot_s = kvc_smem_addr(slot), lut_s = kvc_smem_addr(sm.lut), row_s = kvc_smem_addr(tile + v * TILE_STRIDE);
             if (ok) ok = esc ? kvc_decode_vector<true, 0>(slot_s, lead + start, lut_s, tree, row_s, put)
                              : kvc_decode_vector<false, 0>(slot_s, lead + start, lut_s, tree, row_s, put);
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
         }
-        __syncthreads();
-        if (active && nbytes) {
-            const uint8_t *tile = tiles + sub * TILE_BYTES;
+        const bool out = nbytes != 0;
+        sync();                                             // the tile is complete, the slot free
+        if (BULK && sm.dead[pair]) break;
+        block_of(next, nbytes, lead, src);
+        if (BULK && v == 0) fetch(src, nbytes, lead);       // lands while the tile goes out
+        start = start_of(blk + step);
+        if (out) {
             if (VALUES && is_k) {                            // thread = 8 channels of every fourth row
                 const long long j = blk / cols, col = blk % cols, b = col / H, h = col % H;
                 const int c8 = v & 15;
@@ -138,7 +175,10 @@ __global__ void __launch_bounds__(256) decode_kernel(
                 }
             }
         }
+        sync();                                             // the tile is free
     }
+    // the last copy asked for is empty; after a wait that ran out, the one still open may be in flight
+    if (BULK && v == 0 && !kvc_mbar_wait(&sm.bar[pair], sm.dead[pair] ? par ^ 1u : par)) flags |= KVC_FLAG_WAIT_TIMEOUT;
     if (flags) atomicOr(status, flags);
 }
 
@@ -161,17 +201,25 @@ static int decode_launch(const char *who, const uint8_t *encoded, int64_t encode
     // a slot holds the largest block plus its alignment lead, in 16-byte chunks, plus the decoder's read-ahead
     const uint32_t max_block = max_block_bytes == 0 || max_block_bytes > 8191u ? 8191u : max_block_bytes;
     const uint32_t slot_bytes = ((max_block + 15u + 15u) & ~15u) + 16u;
-    const size_t smem = sizeof(DecodeSmem) + 4 * (size_t)slot_bytes + 4 * (size_t)TILE_BYTES;
-    auto *kernel = values ? decode_kernel<true> : decode_kernel<false>;
-    static kvc_launch_slot slots[2];
+    // As many pairs as an SM holds; where the blocks then come in a few rounds, the pairs that this many rounds need: each
+    // runs the faster for it.
+    const int sms = kvc_sm_count();
+    int pairs = MAX_PAIRS;
+    while (pairs > 1 && sizeof(DecodeSmem) + pairs * (size_t)(slot_bytes + TILE_BYTES) > 227 * 1024) pairs--;
+    const long long rounds = (nblk + (long long)pairs * sms - 1) / ((long long)pairs * sms);
+    pairs = (int)((nblk + rounds * sms - 1) / (rounds * sms));
+    const size_t smem = sizeof(DecodeSmem) + pairs * (size_t)(slot_bytes + TILE_BYTES);
+    const int threads = 64 * (pairs < 4 ? 4 : pairs);       // (the threads beyond the pairs load the table)
+    const bool bulk = (reinterpret_cast<uintptr_t>(encoded) & 15) == 0;
+    auto *kernel = values ? (bulk ? decode_kernel<true, true> : decode_kernel<true, false>) : (bulk ? decode_kernel<false, true> : decode_kernel<false, false>);
+    static kvc_launch_slot slots[4];
     int occ = 0;
-    if (int rc = kvc_prepare(slots[values ? 1 : 0], reinterpret_cast<const void *>(kernel), 256, smem, &occ)) return rc;
+    if (int rc = kvc_prepare(slots[(values ? 2 : 0) + bulk], reinterpret_cast<const void *>(kernel), threads, smem, &occ)) return rc;
     KVC_REQUIRE(occ >= 1, "%s: %zu bytes of shared memory do not fit an SM", who, smem);
-    long long groups = (nblk + 3) / 4, cap = (long long)kvc_sm_count() * occ;
-    unsigned grid = (unsigned)(groups < cap ? groups : cap);
-    kernel<<<grid, 256, smem, kvc_cu(stream)>>>(
+    const long long ctas = (nblk + pairs - 1) / pairs;
+    kernel<<<(unsigned)(ctas < sms ? ctas : sms), threads, smem, kvc_cu(stream)>>>(
         encoded, encoded_bytes, reinterpret_cast<const uint2 *>(block_info), thread_info, book, nblk, cols, is_k,
-        max_block, slot_bytes, codes, m, H, reinterpret_cast<__half *>(values), status);
+        max_block, slot_bytes, pairs, codes, m, H, reinterpret_cast<__half *>(values), status);
     KVC_LAUNCH_OK();
     return KVC_OK;
 }
