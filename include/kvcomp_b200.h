@@ -159,6 +159,19 @@ int kvc_quantize_ranged(const void *x, int64_t T, int64_t B, int64_t H, int64_t 
  * alone (how new values reach the token-major recent window).  out may be a row range of a larger buffer. */
 int kvc_rope_store(const void *x, const void *cos_, const void *sin_, void *out, int64_t B, int64_t H, int64_t t,
                    int64_t D, int64_t cos_batch_stride, kvc_stream_t stream);
+/* The same for the tokens first .. first + t - 1 of x [B, H, x_tokens, D] and of cos / sin [.., x_tokens, D]
+ * (cos_batch_stride 0 or x_tokens * D): out is [t, B, H, D]. */
+int kvc_rope_store_rows(const void *x, const void *cos_, const void *sin_, void *out, int64_t B, int64_t H, int64_t x_tokens,
+                        int64_t first, int64_t t, int64_t D, int64_t cos_batch_stride, kvc_stream_t stream);
+/* A prompt quantised where its projections left it: the first T tokens of x device fp16 [B, H, x_tokens, 128]
+ * (rotated as kvc_rope_store rotates them when cos / sin are given) -> what kvc_quantize returns for the
+ * rotated, transposed tensor.  For the units that kvc_quantize_heads_fits() answers 1 for; cos / sin only with
+ * units per channel. */
+int kvc_quantize_heads_fits(int mode, int batch_shared, int64_t T, int64_t B, int64_t H, int64_t D, int64_t block);
+int kvc_quantize_heads(const void *x, const void *cos_, const void *sin_, int64_t cos_batch_stride, int64_t B, int64_t H,
+                       int64_t x_tokens, int64_t T, int64_t D, int mode, int batch_shared, int64_t block, float rel,
+                       uint8_t *codes, void *min_int, int min_bytes, void *scale, unsigned long long *hist,
+                       int32_t *status, kvc_stream_t stream);
 /* kvc_rope_store for the new keys (rotated) and for the new values (not rotated) of a decode step in one
  * launch: k, v device fp16 [B, H, t, D] -> kout, vout device fp16 [t, B, H, D]. */
 int kvc_kv_store(const void *k, const void *v, const void *cos_, const void *sin_, void *kout, void *vout,

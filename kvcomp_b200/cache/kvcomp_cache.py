@@ -68,7 +68,7 @@ class KVCompCache(_BASE):
         """Add new tokens (key/value_states: [B, Hkv, t, D]); keys get RoPE here unless pre-RoPE is on."""
         cfg = KVCompCacheConfigStatic.config
         cos, sin = cache_kwargs["cos"], cache_kwargs["sin"]
-        k_rows = None                       # the new keys token-major [t, B, H, D], when one kernel made them so
+        k_stored = False
         if cfg.enable_pre_rope:
             self.coss[layer_idx] = safe_cat(self.coss[layer_idx], cos, dim=1)
             self.sins[layer_idx] = safe_cat(self.sins[layer_idx], sin, dim=1)
@@ -88,9 +88,9 @@ class KVCompCache(_BASE):
             if place is not None:                               # the usual decode step: straight into the recent window
                 ops.rope_store(key_states, cos, sin, out=place)
                 kc0.recent_commit(key_states.shape[2])
-                k_rows = False                                  # stored already
             else:
-                k_rows = ops.rope_store(key_states, cos, sin)  # rotation and transposition in one pass, torch's bits
+                kc0.store_heads(key_states, cos, sin)           # rotated with torch's bits
+            k_stored = True
         else:
             key_states = apply_rotary_pos_emb_single(key_states, cos, sin)
         if not cfg.enable_quant:
@@ -98,18 +98,16 @@ class KVCompCache(_BASE):
             self.v_plain[layer_idx] = safe_cat(self.v_plain[layer_idx], value_states, dim=2)
             return
         kc, vc = self._ctx(layer_idx, key_states.shape[1])
-        if k_rows is not False:
-            kc.store(k_rows if k_rows is not None else key_states.permute(2, 0, 1, 3).contiguous().half())
+        if not k_stored:
+            kc.store(key_states.permute(2, 0, 1, 3).contiguous().half())
         t = value_states.shape[2]
-        place, rows = None, None
-        if value_states.is_cuda and value_states.dtype == torch.float16 and value_states.is_contiguous() and value_states.shape[3] % 16 == 0:
-            place = vc.recent_place(t, value_states.device)
-            if place is not None or value_states.data_ptr() % 16 == 0:
-                rows = ops.rope_store(value_states, None, None, out=place)   # the transposition alone
-        if place is not None:                                   # it wrote straight into the window
+        plain = value_states.is_cuda and value_states.dtype == torch.float16 and value_states.is_contiguous() and value_states.shape[3] % 16 == 0
+        place = vc.recent_place(t, value_states.device) if plain else None
+        if place is not None:                                   # the transposition alone, straight into the window
+            ops.rope_store(value_states, None, None, out=place)
             vc.recent_commit(t)
-        elif rows is not None:
-            vc.store(rows)
+        elif plain and value_states.data_ptr() % 16 == 0:
+            vc.store_heads(value_states)
         else:
             vc.store(value_states.permute(2, 0, 1, 3).contiguous().half())
 

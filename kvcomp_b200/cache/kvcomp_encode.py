@@ -102,6 +102,19 @@ class _RecentRows:
         self.reserve(t, room, rows.shape[1:], rows.dtype, rows.device)[:] = rows
         self.commit(t)
 
+    def restart(self, old, n_kept, n_recent, room, shape, dtype, device):
+        """Start over with the kept rows `old` (or None) followed by places for n_kept more and for n_recent recent
+        rows, which the caller writes: returns the two places."""
+        n_old = 0 if old is None else old.shape[0]
+        n = n_old + n_kept + n_recent
+        if n:
+            buf = torch.empty((n + room,) + tuple(shape), dtype=dtype, device=device)
+            if n_old:
+                buf[:n_old] = old
+            self.buf = buf
+        self.q, self.lo, self.hi = 0, n_old + n_kept, n
+        return (None, None) if not n else (self.buf[n_old:self.lo], self.buf[self.lo:n])
+
     def rebuild(self, kept, recent, room):
         """Start over with the given kept rows and recent rows (either may be None)."""
         parts = [p for p in (kept, recent) if p is not None and p.shape[0]]
@@ -259,26 +272,45 @@ class KVCompCtx:
             self.device = cache.device
         assert self.device == cache.device, "device mismatch"
 
-    def _quantize(self, x, report):
-        T = x.shape[0]
+    def _units(self, T):
+        """Places for the unit parameters of T more tokens: (min_ints, scales, how many)."""
         n = self.spec.units(T, self.batch_size, self.head_num, self.head_dim)
-        mi = self._mi.reserve(n, self.device)
-        sc = self._sc.reserve(n, self.device)
-        codes, _, _, _, _ = ops.quantize(x, _MODE[self.quant_mode], self.block_size, self.quant_scale_rel,
-                                         self.batch_shared, min_dtype=self.min_dtype, hist=report.hist, min_int=mi,
-                                         scale=sc, status=report.quant_status)
-        return codes, n
+        return self._mi.reserve(n, self.device), self._sc.reserve(n, self.device), n
+
+    def _cut(self, live, t):
+        """How many of the first tokens of (recent window + t new tokens) are compressed."""
+        # utils/compute.py:59-72.  With recent_size = 0 and a ragged length the reference's slice clips to the length and
+        # its .view then fails (kvcomp_encode.py:83); here the ragged rest simply stays in the window.
+        return min(cut_len(live + t, self.cut_block, self.recent_size), live + t) // self.cut_block * self.cut_block
+
+    def store_heads(self, x, cos=None, sin=None):
+        """store() of new tokens as a model's projections leave them, [B, H, t, D], rotated with cos / sin where they are
+        given.  A prompt into an empty window is quantised from where it lies."""
+        B, H, t, D = x.shape
+        live, mode = len(self._recent), _MODE[self.quant_mode]
+        n = self._cut(live, t)
+        if live or n == 0 or x.data_ptr() % 16 or not ops.quantize_heads_fits(mode, self.batch_shared, n, B, H, D, self.block_size) \
+                or (cos is not None and mode != ops.MODE_CHANNEL):
+            return self.store(ops.rope_store(x, cos, sin))
+        cos, sin, _ = ops._rotation(x, cos, sin)
+        if cos is not None and (cos.data_ptr() | sin.data_ptr()) % 16:
+            return self.store(ops.rope_store(x, cos, sin))
+        self._check(x.permute(2, 0, 1, 3))
+        self.ctx_len += t
+
+        def quantize(report):
+            mi, sc, units = self._units(n)
+            return ops.quantize_heads(x, n, cos, sin, mode, self.block_size, self.quant_scale_rel, self.batch_shared, mi, sc,
+                                      report.hist, report.quant_status), units
+        return self._compress(quantize, n, 0, t - n, lambda place: ops.rope_store(x, cos, sin, out=place, first=n))
 
     def store(self, cache):
         """Append tokens [t, B, H, D]; whole blocks beyond the recent window are quantised and encoded.
         Returns the uint8 codes of the newly compressed tokens as [n_blocks, block, B, H, D] (or None)."""
         self._check(cache)
         self.ctx_len += cache.shape[0]
-        # utils/compute.py:59-72: the first n tokens of (recent window + new tokens) are compressed.  With
-        # recent_size = 0 and a ragged length the reference's slice clips to the length and its .view then
-        # fails (kvcomp_encode.py:83); here the ragged rest simply stays in the window.
         live, t = len(self._recent), cache.shape[0]
-        n = min(cut_len(live + t, self.cut_block, self.recent_size), live + t) // self.cut_block * self.cut_block
+        n = self._cut(live, t)
         room = self._room()
         if n == 0:
             self._recent.append(cache, room)                  # the usual decode step: the new rows, nothing else moves
@@ -289,11 +321,21 @@ class KVCompCtx:
             x, rest = self._recent.view()[:n].clone(), cache  # the window's front
         else:
             x, rest = torch.cat([self._recent.view(), cache[:n - live]], dim=0), cache[n - live:]
-        T = x.shape[0]
+
+        def quantize(report):
+            mi, sc, units = self._units(n)
+            return ops.quantize(x, _MODE[self.quant_mode], self.block_size, self.quant_scale_rel, self.batch_shared,
+                                min_dtype=self.min_dtype, hist=report.hist, min_int=mi, scale=sc, status=report.quant_status)[0], units
+        return self._compress(quantize, n, live, rest.shape[0], lambda place: place.copy_(rest))
+
+    def _compress(self, quantize, n, live, n_rest, put_rest):
+        """quantize(report) launches the quantiser for the first n tokens of (the `live` rows of the window + new tokens) and
+        returns their codes and how many units they have; put_rest(place) writes the n_rest last of the new tokens as rows."""
+        room, T = self._room(), n
         # quantise, book and encode are launched one behind the other; one copy brings back what all of them report
         # (a wait and a copy for each of them: a 333-token prompt 637 us, now 466)
         report = ops.Report(self.device, with_hist=self.book is None)
-        codes, n_units = self._quantize(x, report)
+        codes, n_units = quantize(report)
         if self.book is None:
             self.book = ops.build_codebook(report.hist)
         pend = codes if self._pending is None else torch.cat([self._pending, codes], dim=0)
@@ -322,18 +364,22 @@ class KVCompCtx:
             else:
                 self._recent.consume(n)
                 self._recent.rows_from_kept(0)
-            if rest.shape[0]:
-                self._recent.append(rest, room)
+            if n_rest:
+                put_rest(self._recent.reserve(n_rest, room, codes.shape[1:], torch.float16, self.device))
+                self._recent.commit(n_rest)
         else:
-            kept = None
+            # the window starts over: the kept rows are dequantised, and the rest written, where they stay
+            k, old = 0, None
             if self.keep_dequantised:
                 k = min(n, max(self.KEEP_ROWS // self.cut_block, 1) * self.cut_block)    # a long prefill keeps its last rows only
                 first = (n - k) // self.spec.tok_div * self.spec.sj                      # unit of the first kept token
-                xh = ops.dequant(codes[n - k:], mi[first:], sc[first:], self.spec)
                 old = self._recent.rows_from_kept(self._recent.kept if k == n else 0)
                 old = None if old is None else old[:self._recent.kept]
-                kept = xh if old is None or not old.shape[0] else torch.cat([old, xh], dim=0)
-            self._recent.rebuild(kept, rest if rest.shape[0] else None, room)
+            kept, recent = self._recent.restart(old, k, n_rest, room, codes.shape[1:], torch.float16, self.device)
+            if k:
+                ops.dequant(codes[n - k:], mi[first:], sc[first:], self.spec, out=kept)
+            if n_rest:
+                put_rest(recent)
         self._mi.n += n_units
         self._sc.n += n_units
         self.compressed_ctx_len += T

@@ -421,6 +421,231 @@ __global__ void __launch_bounds__(256) quant_block_apply_kernel(
     if (ghist) hist_flush(shist, ghist, tid, 256);
 }
 
+// Eight channels of the lower half (xa) and their partners of the upper half (xb), rotated with torch's roundings: t * cos +
+// rotate_half(t) * sin, each op rounded to fp16.  (Torch computes an op in fp32 and rounds: the same fp16 value as one
+// rounding, for a product because it is exact in fp32, for a sum because fp32 has more than twice fp16's digits; the _rn forms
+// are never contracted into a fused multiply-add.  Through fp32 this took three times the instructions.)
+__device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const uint4 &ca, const uint4 &cb, const uint4 &sa, const uint4 &sb,
+                                      uint4 &oa, uint4 &ob) {
+    const __half2 *x1 = reinterpret_cast<const __half2 *>(&xa), *x2 = reinterpret_cast<const __half2 *>(&xb);
+    const __half2 *c1 = reinterpret_cast<const __half2 *>(&ca), *c2 = reinterpret_cast<const __half2 *>(&cb);
+    const __half2 *s1 = reinterpret_cast<const __half2 *>(&sa), *s2 = reinterpret_cast<const __half2 *>(&sb);
+    uint4 a, b;
+    __half2 *o1 = reinterpret_cast<__half2 *>(&a), *o2 = reinterpret_cast<__half2 *>(&b);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        // rotate_half: the lower half meets -x2, the upper half x1
+        o1[k] = __hadd2_rn(__hmul2_rn(x1[k], c1[k]), __hmul2_rn(__hneg2(x2[k]), s1[k]));
+        o2[k] = __hadd2_rn(__hmul2_rn(x2[k], c2[k]), __hmul2_rn(x1[k], s2[k]));
+    }
+    oa = a; ob = b;
+}
+
+// ---- a prompt, quantised where its projections left it --------------------------------------------
+// x [B, H, Tx, 128] (heads first), the first T tokens of it -> codes [T, B, H, 128] (tokens first), keys rotated on the way.
+// Bound by memory: 2 bytes read and 1 written per value, where a rotated and transposed copy of the tensor took 4 more before
+// the quantiser read it (K per channel: twice).
+
+// the packed path of quant_eight with what it needs in registers; param(i): value i's unit, for anything else
+template <class P>
+__device__ __forceinline__ uint2 quant_eight_at(const uint4 &v, const float (&rcp)[8], const __half2 (&mi2)[4], bool small_min, P param,
+                                                int *flags, unsigned int *hist) {
+    const __half2 *h2 = reinterpret_cast<const __half2 *>(&v);
+    const __half2 big = __float2half2_rn(1536.0f), nbig = __float2half2_rn(-1536.0f), k1024 = __float2half2_rn(1024.0f);
+    uint32_t u[4], odd = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 xf = __half22float2(h2[k]);
+        const __half2 qh = __floats2half2_rn(__fmul_rn(xf.x, rcp[2 * k]), __fmul_rn(xf.y, rcp[2 * k + 1]));
+        const __half2 r = __hadd2(__hadd2(qh, big), nbig);
+        const __half2 t = __hadd2(__hsub2(r, mi2[k]), k1024);
+        u[k] = *reinterpret_cast<const uint32_t *>(&t) - 0x64006400u;
+        odd |= u[k];
+    }
+    if (!small_min || (odd & 0xff00ff00u) != 0) {
+        const __half *h = reinterpret_cast<const __half *>(&v);
+#pragma unroll
+        for (int k = 0; k < 4; k++) u[k] = quant_one(h[2 * k], param(2 * k), flags) | (quant_one(h[2 * k + 1], param(2 * k + 1), flags) << 16);
+    }
+    if (hist) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) { atomicAdd(&hist[u[k] & 0xffu], 1u); atomicAdd(&hist[u[k] >> 16], 1u); }
+    }
+    return make_uint2(__byte_perm(u[0], u[1], 0x6420), __byte_perm(u[2], u[3], 0x6420));
+}
+
+// ChannelQuant.  CTA = THREADS / 8 * ROWS tokens (one block) of `heads` heads, one after the other; thread = 8 channels of either
+// half of ROWS rows, whose cos and sin it keeps; the next head's rows are fetched while this one's are at work.
+template <int ROWS, int THREADS, bool ROPE>
+__global__ void __launch_bounds__(THREADS) quant_heads_channel_kernel(
+    const __half *__restrict__ x, const __half *__restrict__ cs, const __half *__restrict__ sn, long long cs_bstride,
+    uint32_t B, uint32_t H, uint32_t heads, long long Tx, float rel, uint8_t *__restrict__ codes, void *__restrict__ min_int,
+    int min_bytes, __half *__restrict__ scale, unsigned long long *__restrict__ ghist, int *__restrict__ status) {
+    constexpr int WARPS = THREADS / 32, RT = THREADS / 8;   // RT: rows side by side
+    __shared__ __align__(16) __half smn[WARPS][128], smx[WARPS][128];
+    __shared__ __align__(16) float psf[128], pmi[128], prcp[128];
+    __shared__ unsigned int shist[WARPS * 256];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cg = tid & 7, r = tid >> 3;
+    const uint32_t groups = (H + heads - 1) / heads, b = blockIdx.x / groups, h0 = (blockIdx.x % groups) * heads, h1 = min(H, h0 + heads);
+    const long long j = blockIdx.y, tok0 = j * (RT * ROWS) + r;
+    if (ghist) hist_clear(shist, tid, THREADS);
+    uint4 ca[ROWS], cb[ROWS], sa[ROWS], sb[ROWS];
+    if (ROPE) {
+#pragma unroll
+        for (int k = 0; k < ROWS; k++) {
+            const __half *c = cs + b * cs_bstride + (tok0 + RT * k) * 128 + cg * 8, *s = sn + b * cs_bstride + (tok0 + RT * k) * 128 + cg * 8;
+            ca[k] = *reinterpret_cast<const uint4 *>(c); cb[k] = *reinterpret_cast<const uint4 *>(c + 64);
+            sa[k] = *reinterpret_cast<const uint4 *>(s); sb[k] = *reinterpret_cast<const uint4 *>(s + 64);
+        }
+    }
+    uint4 na[ROWS], nb[ROWS];
+    auto fetch = [&](uint32_t h) {
+        const __half *xr = x + (((long long)b * H + h) * Tx + tok0) * 128 + cg * 8;
+#pragma unroll
+        for (int k = 0; k < ROWS; k++) { na[k] = *reinterpret_cast<const uint4 *>(xr + k * (RT * 128)); nb[k] = *reinterpret_cast<const uint4 *>(xr + k * (RT * 128) + 64); }
+    };
+    fetch(h0);
+    int flags = 0;
+    for (uint32_t h = h0; h < h1; h++) {
+        uint4 va[ROWS], vb[ROWS];
+#pragma unroll
+        for (int k = 0; k < ROWS; k++) {
+            if (ROPE) rope8(na[k], nb[k], ca[k], cb[k], sa[k], sb[k], va[k], vb[k]);
+            else { va[k] = na[k]; vb[k] = nb[k]; }
+        }
+        if (h + 1 < h1) fetch(h + 1);
+        // extremes of the thread's 16 channels, then of the warp's four row groups: at each step a lane gives half of its
+        // channels away and keeps the other half, so that each ends with four channels' extremes
+        __half2 mn[8], mx[8];                               // 0..3: the lower half's channel pairs, 4..7: the upper half's
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            mn[i] = mx[i] = reinterpret_cast<const __half2 *>(&va[0])[i]; mn[4 + i] = mx[4 + i] = reinterpret_cast<const __half2 *>(&vb[0])[i];
+#pragma unroll
+            for (int k = 1; k < ROWS; k++) {
+                const __half2 p = reinterpret_cast<const __half2 *>(&va[k])[i], q = reinterpret_cast<const __half2 *>(&vb[k])[i];
+                mn[i] = __hmin2(mn[i], p); mx[i] = __hmax2(mx[i], p); mn[4 + i] = __hmin2(mn[4 + i], q); mx[4 + i] = __hmax2(mx[4 + i], q);
+            }
+        }
+        const bool up = (lane & 16) != 0, odd = (lane & 8) != 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const __half2 gn = __shfl_xor_sync(0xffffffffu, up ? mn[i] : mn[4 + i], 16), gx = __shfl_xor_sync(0xffffffffu, up ? mx[i] : mx[4 + i], 16);
+            mn[i] = __hmin2(up ? mn[4 + i] : mn[i], gn); mx[i] = __hmax2(up ? mx[4 + i] : mx[i], gx);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const __half2 gn = __shfl_xor_sync(0xffffffffu, odd ? mn[i] : mn[2 + i], 8), gx = __shfl_xor_sync(0xffffffffu, odd ? mx[i] : mx[2 + i], 8);
+            mn[i] = __hmin2(odd ? mn[2 + i] : mn[i], gn); mx[i] = __hmax2(odd ? mx[2 + i] : mx[i], gx);
+        }
+        const int at = (up ? 64 : 0) + cg * 8 + (odd ? 4 : 0);
+        *reinterpret_cast<__half2 *>(&smn[warp][at]) = mn[0]; *reinterpret_cast<__half2 *>(&smn[warp][at + 2]) = mn[1];
+        *reinterpret_cast<__half2 *>(&smx[warp][at]) = mx[0]; *reinterpret_cast<__half2 *>(&smx[warp][at + 2]) = mx[1];
+        __syncthreads();                                    // (also: the head before is done with its units' parameters)
+        if (tid < 128) {                                    // thread = channel
+            float a = __half2float(smn[0][tid]), z = __half2float(smx[0][tid]);
+#pragma unroll
+            for (int w = 1; w < WARPS; w++) { a = fminf(a, __half2float(smn[w][tid])); z = fmaxf(z, __half2float(smx[w][tid])); }
+            __half sc;
+            const UnitParam q = unit_param(a, z, rel, &sc, &flags);
+            const long long u = ((j * B + b) * H + h) * 128 + tid;
+            scale[u] = sc;
+            store_min(min_int, min_bytes, u, q.mi, &flags);
+            psf[tid] = q.sf; pmi[tid] = q.mi; prcp[tid] = q.rcp;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const int c0 = half * 64 + cg * 8;
+            float rcp[8];
+            __half2 mi2[4];
+            bool small = true;
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4 *>(&rcp[i]) = *reinterpret_cast<const float4 *>(&prcp[c0 + i]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 m = *reinterpret_cast<const float2 *>(&pmi[c0 + 2 * i]);
+                small = small && small_min_int(m.x) && small_min_int(m.y);
+                mi2[i] = __floats2half2_rn(m.x, m.y);
+            }
+            auto param = [&](int i) { UnitParam p; p.sf = psf[c0 + i]; p.mi = pmi[c0 + i]; p.rcp = prcp[c0 + i]; return p; };
+#pragma unroll
+            for (int k = 0; k < ROWS; k++) {
+                const uint2 o = quant_eight_at(half ? vb[k] : va[k], rcp, mi2, small, param, &flags, ghist ? shist + warp * 256 : nullptr);
+                *reinterpret_cast<uint2 *>(codes + (((tok0 + RT * k) * B + b) * H + h) * 128 + c0) = o;
+            }
+        }
+    }
+    if (flags) atomicOr(status, flags);
+    if (ghist) hist_flush(shist, ghist, tid, THREADS);
+}
+
+// TokenQuant (a unit: one token of one sequence, all heads) and VectorQuant (one head of it).  CTA = four tokens of one sequence
+// at a time, all heads in registers (NH x 4 at most); thread = 8 channels of one token in every fourth head.
+template <int NH, bool VECTOR>
+__global__ void __launch_bounds__(256) quant_heads_token_kernel(
+    const __half *__restrict__ x, uint32_t B, uint32_t H, long long Tx, long long T, float rel, uint8_t *__restrict__ codes,
+    void *__restrict__ min_int, int min_bytes, __half *__restrict__ scale, unsigned long long *__restrict__ ghist,
+    int *__restrict__ status) {
+    __shared__ float red[2][4][4];                          // extremes by head group and token
+    __shared__ unsigned int shist[8 * 256];
+    const int tid = threadIdx.x, warp = tid >> 5, c0 = (tid & 15) * 8, tk = (tid >> 4) & 3, hg = tid >> 6;
+    if (ghist) hist_clear(shist, tid, 256);
+    int flags = 0;
+    const long long n4 = (T + 3) / 4, n_groups = n4 * B;
+    for (long long grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
+        const uint32_t b = (uint32_t)(grp / n4);            // neighbouring CTAs: neighbouring tokens of a sequence
+        const long long tok = (grp - b * n4) * 4 + tk;
+        const bool live = tok < T;
+        uint4 v[NH];
+        const __half *xr = x + ((long long)b * H * Tx + tok) * 128 + c0;
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            const uint32_t h = i * 4 + hg;
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (live && h < H) v[i] = *reinterpret_cast<const uint4 *>(xr + h * Tx * 128);
+        }
+        float mn = INFINITY, mx = -INFINITY;
+        UnitParam p = {0.f, 0.f, 0.f};
+        if (!VECTOR) {
+#pragma unroll
+            for (int i = 0; i < NH; i++) if ((uint32_t)(i * 4 + hg) < H) minmax8(v[i], mn, mx);
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) { mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o)); mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); }
+            __syncthreads();                                // the group before is done with its extremes
+            if (c0 == 0) { red[0][hg][tk] = mn; red[1][hg][tk] = mx; }
+            __syncthreads();
+            mn = fminf(fminf(red[0][0][tk], red[0][1][tk]), fminf(red[0][2][tk], red[0][3][tk]));
+            mx = fmaxf(fmaxf(red[1][0][tk], red[1][1][tk]), fmaxf(red[1][2][tk], red[1][3][tk]));
+            if (live) {
+                __half sc;
+                p = unit_param(mn, mx, rel, &sc, &flags);
+                if (c0 == 0 && hg == 0) { scale[tok * B + b] = sc; store_min(min_int, min_bytes, tok * B + b, p.mi, &flags); }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            const uint32_t h = i * 4 + hg;
+            if (VECTOR) {
+                mn = INFINITY; mx = -INFINITY;
+                minmax8(v[i], mn, mx);
+#pragma unroll
+                for (int o = 1; o < 16; o <<= 1) { mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o)); mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); }
+            }
+            if (!live || h >= H) continue;
+            const long long u = (tok * B + b) * H + h;      // also the row of the codes
+            if (VECTOR) {
+                __half sc;
+                p = unit_param(mn, mx, rel, &sc, &flags);
+                if (c0 == 0) { scale[u] = sc; store_min(min_int, min_bytes, u, p.mi, &flags); }
+            }
+            const __half2 mi2 = __float2half2_rn(p.mi);
+            *reinterpret_cast<uint2 *>(codes + u * 128 + c0) = quant_eight<0>(v[i], &p, small_min_int(p.mi), &mi2, &flags, ghist ? shist + warp * 256 : nullptr);
+        }
+    }
+    if (flags) atomicOr(status, flags);
+    if (ghist) hist_flush(shist, ghist, tid, 256);
+}
+
 // ---- dequantise: fp16((code + min_int) * scale), models/cache/kvcomp_encode.py:146 -------------
 // Bound by memory (1 byte in, 2 out).  A thread takes GROUPS groups of 8 channels, all their loads in flight together;
 // wide_units: units side by side over the channels, 8 of them fetched with one load per array.  Two groups where the units
@@ -641,22 +866,6 @@ extern "C" int kvc_k_matvec(const void *k, const void *q, void *out, int64_t ctx
     return KVC_OK;
 }
 
-// eight channels of the lower half (xa) and their partners of the upper half (xb), rotated with torch's roundings
-__device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const uint4 &ca, const uint4 &cb, const uint4 &sa, const uint4 &sb,
-                                      uint4 &oa, uint4 &ob) {
-    const __half *x1 = reinterpret_cast<const __half *>(&xa), *x2 = reinterpret_cast<const __half *>(&xb);
-    const __half *c1 = reinterpret_cast<const __half *>(&ca), *c2 = reinterpret_cast<const __half *>(&cb);
-    const __half *s1 = reinterpret_cast<const __half *>(&sa), *s2 = reinterpret_cast<const __half *>(&sb);
-    __half *o1 = reinterpret_cast<__half *>(&oa), *o2 = reinterpret_cast<__half *>(&ob);
-    auto mul = [](__half a, __half b2) { return __half2float(__float2half_rn(__fmul_rn(__half2float(a), __half2float(b2)))); };
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        // rotate_half: the lower half meets -x2, the upper half x1
-        o1[k] = __float2half_rn(__fadd_rn(mul(x1[k], c1[k]), mul(__hneg(x2[k]), s1[k])));
-        o2[k] = __float2half_rn(__fadd_rn(mul(x2[k], c2[k]), mul(x1[k], s2[k])));
-    }
-}
-
 // ---- rotary embedding of new keys on their way into the cache -------------------------------------
 // models/cache/kvcomp_quant.py:43-48 rotates the new keys (utils/compute.py:25-33: t * cos + rotate_half(t) * sin,
 // every op a rounded fp16 tensor op) before they enter the recent window; the cache keeps tokens token-major.
@@ -664,7 +873,7 @@ __device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const ui
 // blockIdx.y = 1 (kvc_kv_store): the same rows of a second tensor xv -> outv without rotation (the new values)
 __global__ void __launch_bounds__(256) rope_store_kernel(const __half *__restrict__ x, const __half *__restrict__ cs,
                                                          const __half *__restrict__ sn, __half *__restrict__ out,
-                                                         long long B, long long H, long long t, int D, long long cs_bstride,
+                                                         long long B, long long H, long long t, int D, long long cs_bstride, long long x_tokens,
                                                          const __half *__restrict__ xv, __half *__restrict__ outv) {
     // A kernel launched behind this one with programmatic stream serialisation (the fused attention, or its merge kernel
     // while nothing is compressed) may set up while these few rows are written: it touches them only after its own
@@ -676,7 +885,7 @@ __global__ void __launch_bounds__(256) rope_store_kernel(const __half *__restric
     if (i >= t * B * H * per_row) return;
     const int c0 = (int)(i % per_row) * 8, half = D / 2;
     const long long row = i / per_row, h = row % H, b = (row / H) % B, tok = row / (H * B);
-    const __half *xr = x + ((b * H + h) * t + tok) * D;
+    const __half *xr = x + ((b * H + h) * x_tokens + tok) * D;
     __half *orow = out + ((tok * B + b) * H + h) * D;
     const uint4 xa = *reinterpret_cast<const uint4 *>(xr + c0), xb = *reinterpret_cast<const uint4 *>(xr + c0 + half);
     if (cs == nullptr) {                                         // no rotation (values): the transposition alone
@@ -701,18 +910,18 @@ __global__ void __launch_bounds__(256) rope_store_kernel(const __half *__restric
 template <int HT>
 __global__ void __launch_bounds__(256) rope_tile_kernel(const __half *__restrict__ x, const __half *__restrict__ cs,
                                                         const __half *__restrict__ sn, __half *__restrict__ out,
-                                                        uint32_t B, uint32_t H, long long t, long long cs_bstride) {
+                                                        uint32_t B, uint32_t H, long long t, long long cs_bstride, long long x_tokens) {
     const uint32_t groups = H / HT, b = blockIdx.x / groups, h0 = (blockIdx.x % groups) * HT;
     const long long tok = (long long)blockIdx.y * 32 + (threadIdx.x >> 3);
     const int c0 = (threadIdx.x & 7) * 8;
     if (tok >= t) return;
-    const __half *xr = x + (((long long)b * H + h0) * t + tok) * 128 + c0;
+    const __half *xr = x + (((long long)b * H + h0) * x_tokens + tok) * 128 + c0;
     __half *orow = out + ((tok * B + b) * H + h0) * 128 + c0;
     uint4 xa[HT], xb[HT];
 #pragma unroll
     for (int k = 0; k < HT; k++) {
-        xa[k] = *reinterpret_cast<const uint4 *>(xr + k * t * 128);
-        xb[k] = *reinterpret_cast<const uint4 *>(xr + k * t * 128 + 64);
+        xa[k] = *reinterpret_cast<const uint4 *>(xr + k * x_tokens * 128);
+        xb[k] = *reinterpret_cast<const uint4 *>(xr + k * x_tokens * 128 + 64);
     }
     if (cs != nullptr) {
         const __half *cr = cs + b * cs_bstride + tok * 128 + c0, *sr = sn + b * cs_bstride + tok * 128 + c0;
@@ -728,30 +937,86 @@ __global__ void __launch_bounds__(256) rope_tile_kernel(const __half *__restrict
     }
 }
 
-extern "C" int kvc_rope_store(const void *x, const void *cos_, const void *sin_, void *out, int64_t B, int64_t H, int64_t t,
-                              int64_t D, int64_t cos_batch_stride, kvc_stream_t stream) {
+extern "C" int kvc_rope_store_rows(const void *x, const void *cos_, const void *sin_, void *out, int64_t B, int64_t H, int64_t x_tokens,
+                                   int64_t first, int64_t t, int64_t D, int64_t cos_batch_stride, kvc_stream_t stream) {
     KVC_REQUIRE(x && out && ((cos_ == nullptr) == (sin_ == nullptr)), "kvc_rope_store: null pointer");
-    KVC_REQUIRE(B > 0 && H > 0 && t >= 0 && D > 0 && D % 16 == 0, "kvc_rope_store: bad shape");
+    KVC_REQUIRE(B > 0 && H > 0 && t >= 0 && D > 0 && D % 16 == 0 && first >= 0 && first + t <= x_tokens, "kvc_rope_store: bad shape");
     KVC_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_) | reinterpret_cast<uintptr_t>(sin_) |
                   reinterpret_cast<uintptr_t>(out)) & 15) == 0, "kvc_rope_store: pointers must be 16-byte aligned");
-    KVC_REQUIRE(cos_batch_stride == 0 || cos_batch_stride == t * D, "kvc_rope_store: cos/sin must be [B, t, D] or [1, t, D]");
+    KVC_REQUIRE(cos_batch_stride == 0 || cos_batch_stride == x_tokens * D, "kvc_rope_store: cos/sin must be [B, t, D] or [1, t, D]");
     const long long n = t * B * H * (D / 16);
     if (n == 0) return KVC_OK;
     KVC_REQUIRE((n + 255) / 256 < (1ll << 31), "kvc_rope_store: too many elements");
+    const __half *xh = reinterpret_cast<const __half *>(x) + first * D;
+    const __half *ch = cos_ ? reinterpret_cast<const __half *>(cos_) + first * D : nullptr, *sh = sin_ ? reinterpret_cast<const __half *>(sin_) + first * D : nullptr;
+    __half *oh = reinterpret_cast<__half *>(out);
     // tiles when there are enough of them to fill the device twice over; else a thread per 16 channels of a row
     const int ht = H % 4 == 0 ? 4 : (H % 2 == 0 ? 2 : 1);
     const long long col_groups = B * (H / ht), tok_tiles = (t + 31) / 32;
     if (D == 128 && t >= 32 && col_groups * tok_tiles >= 2ll * kvc_sm_count() && tok_tiles <= 65535 && col_groups < (1ll << 31)) {
         auto *kernel = ht == 4 ? rope_tile_kernel<4> : (ht == 2 ? rope_tile_kernel<2> : rope_tile_kernel<1>);
-        kernel<<<dim3((unsigned)col_groups, (unsigned)tok_tiles), 256, 0, kvc_cu(stream)>>>(
-            reinterpret_cast<const __half *>(x), reinterpret_cast<const __half *>(cos_), reinterpret_cast<const __half *>(sin_),
-            reinterpret_cast<__half *>(out), (uint32_t)B, (uint32_t)H, t, cos_batch_stride);
+        kernel<<<dim3((unsigned)col_groups, (unsigned)tok_tiles), 256, 0, kvc_cu(stream)>>>(xh, ch, sh, oh, (uint32_t)B, (uint32_t)H, t, cos_batch_stride, x_tokens);
         KVC_LAUNCH_OK();
         return KVC_OK;
     }
-    rope_store_kernel<<<(unsigned)((n + 255) / 256), 256, 0, kvc_cu(stream)>>>(
-        reinterpret_cast<const __half *>(x), reinterpret_cast<const __half *>(cos_), reinterpret_cast<const __half *>(sin_),
-        reinterpret_cast<__half *>(out), B, H, t, (int)D, cos_batch_stride, nullptr, nullptr);
+    rope_store_kernel<<<(unsigned)((n + 255) / 256), 256, 0, kvc_cu(stream)>>>(xh, ch, sh, oh, B, H, t, (int)D, cos_batch_stride, x_tokens, nullptr, nullptr);
+    KVC_LAUNCH_OK();
+    return KVC_OK;
+}
+
+extern "C" int kvc_rope_store(const void *x, const void *cos_, const void *sin_, void *out, int64_t B, int64_t H, int64_t t,
+                              int64_t D, int64_t cos_batch_stride, kvc_stream_t stream) {
+    return kvc_rope_store_rows(x, cos_, sin_, out, B, H, t, 0, t, D, cos_batch_stride, stream);
+}
+
+// Which prompts kvc_quantize_heads takes: K units per channel in blocks of 64 or 128 tokens; V units per token or vector, up to
+// 64 heads (they are held in registers).  A unit must not span sequences.
+extern "C" int kvc_quantize_heads_fits(int mode, int batch_shared, int64_t T, int64_t B, int64_t H, int64_t D, int64_t block) {
+    if (D != 128 || B <= 0 || H <= 0 || B * H >= (1ll << 31) || T < 0) return 0;
+    if (mode == KVC_MODE_CHANNEL) return (block == 64 || block == 128) && T / block <= 65535;
+    if (mode == KVC_MODE_VECTOR) return H <= 64;
+    return mode == KVC_MODE_TOKEN && H <= 64 && (!batch_shared || B == 1);
+}
+
+extern "C" int kvc_quantize_heads(const void *x, const void *cos_, const void *sin_, int64_t cos_batch_stride, int64_t B, int64_t H,
+                                  int64_t x_tokens, int64_t T, int64_t D, int mode, int batch_shared, int64_t block, float rel,
+                                  uint8_t *codes, void *min_int, int min_bytes, void *scale, unsigned long long *hist,
+                                  int32_t *status, kvc_stream_t stream) {
+    KVC_REQUIRE(x && codes && min_int && scale && status && (cos_ == nullptr) == (sin_ == nullptr), "kvc_quantize_heads: null pointer");
+    KVC_REQUIRE(kvc_quantize_heads_fits(mode, batch_shared, T, B, H, D, block), "kvc_quantize_heads: these units take kvc_quantize");
+    KVC_REQUIRE(T >= 0 && T <= x_tokens, "kvc_quantize_heads: %lld of %lld tokens", (long long)T, (long long)x_tokens);
+    KVC_REQUIRE(min_bytes == 1 || min_bytes == 2, "kvc_quantize_heads: min_bytes must be 1 or 2");
+    KVC_REQUIRE(cos_ == nullptr || mode == KVC_MODE_CHANNEL, "kvc_quantize_heads: only keys are rotated");
+    KVC_REQUIRE(cos_batch_stride == 0 || cos_batch_stride == x_tokens * D, "kvc_quantize_heads: cos/sin must be [B, t, D] or [1, t, D]");
+    KVC_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(cos_) | reinterpret_cast<uintptr_t>(sin_)) & 15) == 0 &&
+                (reinterpret_cast<uintptr_t>(codes) & 7) == 0, "kvc_quantize_heads: x, cos and sin must be 16-byte and codes 8-byte aligned");
+    if (T == 0) return KVC_OK;
+    cudaStream_t s = kvc_cu(stream);
+    const __half *xh = reinterpret_cast<const __half *>(x), *ch = reinterpret_cast<const __half *>(cos_), *sh = reinterpret_cast<const __half *>(sin_);
+    __half *sc = reinterpret_cast<__half *>(scale);
+    const long long sms = kvc_sm_count();
+    if (mode == KVC_MODE_CHANNEL) {
+        KVC_REQUIRE(T % block == 0, "kvc_quantize_heads: T=%lld is not a multiple of block=%lld", (long long)T, (long long)block);
+        // heads per CTA: four share the reading of cos and sin, fewer where the device would not be full twice over
+        long long heads = 4;
+        while (heads > 1 && (T / block) * B * ((H + heads - 1) / heads) < 4 * sms) heads /= 2;
+        // (two rows per thread: with one and twice the threads, 1 GiB of keys in 1.0 ms instead of 0.55)
+        auto *kernel = block == 64 ? (ch ? quant_heads_channel_kernel<2, 256, true> : quant_heads_channel_kernel<2, 256, false>)
+                                   : (ch ? quant_heads_channel_kernel<2, 512, true> : quant_heads_channel_kernel<2, 512, false>);
+        kernel<<<dim3((unsigned)(B * ((H + heads - 1) / heads)), (unsigned)(T / block)), block == 64 ? 256 : 512, 0, s>>>(
+            xh, ch, sh, cos_batch_stride, (uint32_t)B, (uint32_t)H, (uint32_t)heads, x_tokens, rel, codes, min_int, min_bytes, sc, hist, status);
+    } else {
+        const long long groups = (T + 3) / 4 * B;
+        const unsigned grid = (unsigned)std::min<long long>(groups, sms * 8);
+#define KVC_QT(NH_) (mode == KVC_MODE_VECTOR ? quant_heads_token_kernel<NH_, true> : quant_heads_token_kernel<NH_, false>)<<<grid, 256, 0, s>>>( \
+        xh, (uint32_t)B, (uint32_t)H, x_tokens, T, rel, codes, min_int, min_bytes, sc, hist, status)
+        if (H <= 4) KVC_QT(1);
+        else if (H <= 8) KVC_QT(2);
+        else if (H <= 16) KVC_QT(4);
+        else if (H <= 32) KVC_QT(8);
+        else KVC_QT(16);
+#undef KVC_QT
+    }
     KVC_LAUNCH_OK();
     return KVC_OK;
 }
@@ -769,7 +1034,7 @@ extern "C" int kvc_kv_store(const void *k, const void *v, const void *cos_, cons
     KVC_REQUIRE((n + 255) / 256 < (1ll << 31), "kvc_kv_store: too many elements");
     rope_store_kernel<<<dim3((unsigned)((n + 255) / 256), 2), 256, 0, kvc_cu(stream)>>>(
         reinterpret_cast<const __half *>(k), reinterpret_cast<const __half *>(cos_), reinterpret_cast<const __half *>(sin_),
-        reinterpret_cast<__half *>(kout), B, H, t, (int)D, cos_batch_stride,
+        reinterpret_cast<__half *>(kout), B, H, t, (int)D, cos_batch_stride, t,
         reinterpret_cast<const __half *>(v), reinterpret_cast<__half *>(vout));
     KVC_LAUNCH_OK();
     return KVC_OK;

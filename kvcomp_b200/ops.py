@@ -206,25 +206,59 @@ def quantize_ranged(x, mode, block, rel, mn, mx, batch_shared=True, min_dtype=to
     return codes, min_int, scale, spec, status
 
 
-def rope_store(x, cos, sin, out=None):
+def _rotation(x, cos, sin):
+    """cos and sin for x [B, H, t, D], checked, and their stride between sequences (both None: no rotation)."""
+    if cos is None:
+        return None, None, 0
+    B, _, t, D = x.shape
+    cos, sin = _cuda(cos.contiguous(), torch.float16, "cos"), _cuda(sin.contiguous(), torch.float16, "sin")
+    s = cos.shape
+    if s != sin.shape or len(s) != 3 or s[1] != t or s[2] != D or s[0] not in (1, B):
+        raise KvcError("cos / sin must be [B, t, D] or [1, t, D], got %s" % (tuple(s),))
+    return cos, sin, 0 if s[0] == 1 and B > 1 else t * D
+
+
+def rope_store(x, cos, sin, out=None, first=0):
     """New keys x fp16 [B, H, t, D] rotated (t * cos + rotate_half(t) * sin in fp16, as torch evaluates it) and
     laid out token-major: fp16 [t, B, H, D].  cos / sin: fp16 [B, t, D] or [1, t, D]; both None: no rotation,
-    the transposition alone (new values).  out: where the rows go (a row range of the recent window)."""
+    the transposition alone (new values).  out: where the rows go (a row range of the recent window).
+    first: the tokens from this one on, t - first rows."""
     lib = _lib.load()
     _cuda(x, torch.float16, "key_states")
-    B, H, t, D = x.shape
-    stride = 0
-    if cos is not None:
-        cos, sin = _cuda(cos.contiguous(), torch.float16, "cos"), _cuda(sin.contiguous(), torch.float16, "sin")
-        if cos.shape != sin.shape or cos.dim() != 3 or cos.shape[1:] != (t, D) or cos.shape[0] not in (1, B):
-            raise KvcError("cos / sin must be [B, t, D] or [1, t, D], got %s" % (tuple(cos.shape),))
-        stride = 0 if cos.shape[0] == 1 and B > 1 else t * D
+    B, H, x_tokens, D = x.shape
+    cos, sin, stride = _rotation(x, cos, sin)
+    t = x_tokens - first
     out = torch.empty((t, B, H, D), dtype=torch.float16, device=x.device) if out is None else _cuda(out, torch.float16, "out")
     if tuple(out.shape) != (t, B, H, D):
         raise KvcError("out must be [t, B, H, D] = %s, got %s" % ((t, B, H, D), tuple(out.shape)))
     with _on(x.device):
-        _lib.check(lib.kvc_rope_store(_p(x), _p(cos), _p(sin), _p(out), B, H, t, D, stride, _stream()), "kvc_rope_store")
+        _lib.check(lib.kvc_rope_store_rows(_p(x), _p(cos), _p(sin), _p(out), B, H, x_tokens, first, t, D, stride, _stream()), "kvc_rope_store")
     return out
+
+
+def quantize_heads_fits(mode, batch_shared, T, B, H, D, block):
+    """Whether quantize_heads takes T tokens in these units."""
+    return bool(_lib.load().kvc_quantize_heads_fits(mode, int(batch_shared), T, B, H, D, block))
+
+
+def quantize_heads(x, T, cos, sin, mode, block, rel, batch_shared, min_int, scale, hist=None, status=None):
+    """The first T tokens of a prompt x fp16 [B, H, t, 128] as its projections leave it, rotated with cos / sin where
+    they are given: the codes u8 [T, B, H, 128], min_int and scale that quantize gives for rope_store's rows, without
+    the rows."""
+    lib = _lib.load()
+    _cuda(x, torch.float16, "x")
+    B, H, t, D = x.shape
+    cos, sin, stride = _rotation(x, cos, sin)
+    _cuda(min_int, None, "min_int"), _cuda(scale, torch.float16, "scale")
+    codes = torch.empty((T, B, H, D), dtype=torch.uint8, device=x.device)
+    status = new_status(x.device) if status is None else status
+    if hist is not None:
+        _cuda(hist, torch.int64, "hist")
+    with _on(x.device):
+        _lib.check(lib.kvc_quantize_heads(_p(x), _p(cos), _p(sin), stride, B, H, t, T, D, mode, int(batch_shared), block, float(rel),
+                                          _p(codes), _p(min_int), min_int.element_size(), _p(scale), _p(hist), _p(status), _stream()),
+                   "kvc_quantize_heads")
+    return codes
 
 
 def kv_store(k, v, cos, sin, kout, vout):
@@ -234,16 +268,13 @@ def kv_store(k, v, cos, sin, kout, vout):
     _cuda(k, torch.float16, "key_states")
     _cuda(v, torch.float16, "value_states")
     B, H, t, D = k.shape
-    cos, sin = _cuda(cos.contiguous(), torch.float16, "cos"), _cuda(sin.contiguous(), torch.float16, "sin")
-    if cos.shape != sin.shape or cos.dim() != 3 or cos.shape[1:] != (t, D) or cos.shape[0] not in (1, B):
-        raise KvcError("cos / sin must be [B, t, D] or [1, t, D], got %s" % (tuple(cos.shape),))
+    cos, sin, stride = _rotation(k, cos, sin)
     if tuple(v.shape) != (B, H, t, D) or tuple(kout.shape) != (t, B, H, D) or tuple(vout.shape) != (t, B, H, D):
         raise KvcError("kv_store: k, v must be [B, H, t, D] and kout, vout [t, B, H, D]")
     _cuda(kout, torch.float16, "kout")
     _cuda(vout, torch.float16, "vout")
     with _on(k.device):
-        _lib.check(lib.kvc_kv_store(_p(k), _p(v), _p(cos), _p(sin), _p(kout), _p(vout), B, H, t, D,
-                                    0 if cos.shape[0] == 1 and B > 1 else t * D, _stream()), "kvc_kv_store")
+        _lib.check(lib.kvc_kv_store(_p(k), _p(v), _p(cos), _p(sin), _p(kout), _p(vout), B, H, t, D, stride, _stream()), "kvc_kv_store")
 
 
 def dequant(codes, min_int, scale, spec, out=None):

@@ -1,0 +1,58 @@
+"""Prompts quantised where their projections left them (kvc_quantize_heads) against the rotated and transposed rows through
+kvc_quantize, and the decoder's pairs of warps over every split of the blocks: the same bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from kvcomp_b200 import ops as _ops
+    return _ops
+
+
+def _prompt(B, H, t, seed, spread=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = (torch.randn(B, H, t, 128, device="cuda", generator=g) * spread +
+         torch.randn(B, H, 1, 128, device="cuda", generator=g) * 3).half()
+    ang = torch.rand(B, t, 128, device="cuda", generator=g) * 6.28
+    return x, ang.cos().half(), ang.sin().half()
+
+
+@pytest.mark.parametrize("mode,block,B,H,T,more,rope", [
+    ("ChannelQuant", 64, 1, 1, 64, 0, "each"), ("ChannelQuant", 64, 2, 5, 192, 13, "each"), ("ChannelQuant", 64, 3, 8, 1024, 1, "one"),
+    ("ChannelQuant", 128, 2, 3, 256, 77, "one"), ("ChannelQuant", 128, 1, 32, 1280, 0, None), ("ChannelQuant", 64, 16, 8, 640, 5, None),
+    ("TokenQuant", 64, 1, 1, 3, 0, None), ("TokenQuant", 64, 2, 5, 64, 7, None), ("TokenQuant", 64, 2, 8, 129, 0, None),
+    ("TokenQuant", 64, 3, 13, 130, 3, None), ("TokenQuant", 64, 1, 32, 700, 1, None), ("TokenQuant", 64, 2, 40, 66, 0, None),
+    ("TokenQuant", 64, 1, 64, 65, 0, None), ("VectorQuant", 64, 2, 3, 67, 2, None), ("VectorQuant", 64, 1, 33, 64, 0, None),
+])
+def test_prompt_in_place_equals_rows(ops, mode, block, B, H, T, more, rope):
+    m = ops.MODES[mode]
+    assert ops.quantize_heads_fits(m, False, T, B, H, 128, block)
+    for seed, spread, rel in ((1, 1.0, 0.05), (2, 300.0, 0.2), (3, 1e-6, 0.003)):      # the last two leave the packed arithmetic
+        x, cos, sin = _prompt(B, H, T + more, seed, spread)
+        x[0, 0, :T, 5] = 1.5                                                           # a constant channel
+        cos, sin = (None, None) if rope is None else (cos, sin) if rope == "each" else (cos[:1].contiguous(), sin[:1].contiguous())
+        rows = ops.rope_store(x, cos, sin)
+        spec = ops.qspec(m, False, B, H, 128, block)
+        n = spec.units(T, B, H, 128)
+        for dt in (torch.int8, torch.int16):
+            hist, hist2 = (torch.zeros(256, dtype=torch.int64, device="cuda") for _ in range(2))
+            want, mi, sc, _, st = ops.quantize(rows[:T].contiguous(), m, block, rel, False, min_dtype=dt, hist=hist)
+            mi2, sc2, st2 = torch.empty_like(mi), torch.empty_like(sc), ops.new_status(x.device)
+            got = ops.quantize_heads(x, T, cos, sin, m, block, rel, False, mi2, sc2, hist2, st2)
+            assert torch.equal(sc.view(torch.int16), sc2.view(torch.int16)) and torch.equal(mi, mi2) and mi2.numel() == n
+            assert torch.equal(want, got) and torch.equal(hist, hist2)
+            assert int(st.item()) == int(st2.item())
+        if more:
+            assert torch.equal(ops.rope_store(x, cos, sin, first=T), rows[T:])
+
+
+def test_units_that_need_rows_are_refused(ops):
+    fits = ops.quantize_heads_fits
+    assert not fits(ops.MODE_TOKEN, True, 64, 2, 8, 128, 64) and fits(ops.MODE_TOKEN, True, 64, 1, 8, 128, 64)
+    assert not fits(ops.MODE_TOKEN, False, 64, 2, 65, 128, 64) and not fits(ops.MODE_CHANNEL, False, 192, 2, 8, 128, 192)
+    assert not fits(ops.MODE_BLOCK, False, 64, 2, 8, 128, 64) and not fits(ops.MODE_CHANNEL, False, 64, 2, 8, 64, 64)
