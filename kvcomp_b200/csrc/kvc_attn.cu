@@ -5,17 +5,17 @@
 // v_huffman_decode_and_mat_vec_mul (kernels.cu:778-861); attention semantics of
 // eager_attention_forward (models/llama.py:211-234).
 //
-// Work layout of the unfused kernels and of the attention kernel with one query head per KV head (with several: see
-// attn_rows_kernel): CTA = 256 threads working on 256 tokens of one (b, kv head).
+// Work layout of the unfused kernels: CTA = 256 threads working on 256 tokens of one (b, kv head); of the attention kernels: a
+// worker of 128 threads, several to a CTA, walking steps of 128 tokens.
 //   K phase: thread = token; its vector holds the token's 128 channel codes.
 //            score = sum_c code_c * w[c] + zp, with w[c] = q[c]*scale[c] staged per 64-token block
 //            (dequantisation folded into the weights, the min_int term summed once per block).
 //   V phase: thread = (128-token group, channel); its vector holds 128 tokens of that channel.
 //            out[ch] = sum_t code_t * ps[t] + zpv, with ps[t] = p[t]*scale[t] staged per group.
-// The attention kernel is launched with as many CTAs as the device holds at once.  Its work is cut into
-// items (one (b, kv head) column x one run of 256-token tiles); a CTA starts with two items fixed by
-// its index and draws the rest from a counter two items ahead, so that the CTAs an SM's schedulers
-// favour take more of them.  Staging copies, tile metadata and the query vector of the next tile or
+// The attention kernels are launched with as many workers as the device holds at once.  Their work is cut into
+// items (one (b, kv head) column x one run of steps); a worker starts with two items fixed by
+// its index and draws the rest from a counter two items ahead, so that the workers an SM's schedulers
+// favour take more of them.  Staging copies, a step's metadata and the query vector of the next step or
 // item are always fetched while the current one is decoded.  When a column has more than one item,
 // each leaves a partial result (max, sum, accumulators) and a second kernel merges them.
 // Both phases are "decode 128 symbols and dot them with a shared 128-vector", so they share one
@@ -24,7 +24,7 @@
 // symbols as bytes, and two dp4a instructions multiply them with the matching weight bytes -- integer arithmetic, exact, accumulated in int32.  The only rounding is that of the
 // weights (2^-16 of the largest weight of the vector); the zero-point terms and everything after
 // the dot product are fp32.  With several query heads per KV head they share every decode: in the unfused
-// kernels by weight records [position][G], up to four heads a launch.
+// kernels by weight records [position][G], up to four heads a launch, in the attention kernel see attn_rows_kernel.
 #include <math_constants.h>
 
 #include <algorithm>
@@ -37,7 +37,7 @@ namespace {
 constexpr int SLOT_PAD = 1024;           // readable bytes behind the last staging slot
 constexpr int NTHR = 256;
 constexpr size_t MAX_CTA_SHARED = 227 * 1024;
-constexpr int ATTN_PART_FLOATS = 4 + 256;   // a partial result of the attention kernel: m, l, two unused, acc[2][128]
+constexpr int ATTN_PART_FLOATS = 4 + 256;   // workspace per head and run of 256-token tiles: two partial results (ROWS_PART_FLOATS each)
 
 struct CacheDev {
     const uint8_t *encoded;
@@ -162,8 +162,8 @@ template <int G> __device__ __forceinline__ constexpr int w_lo(int c, int g) { r
 
 // decode the thread's vector (staged at shared address slot_s) and dot it with the weight records at
 // shared address w_s (layout: w_hi / w_lo)
-template <int G, bool ESC>
-__device__ __forceinline__ bool decode_dot_impl(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, uint32_t tree_s,
+template <int G, bool ESC, class Tree>
+__device__ __forceinline__ bool decode_dot_impl(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, Tree tree,
                                                 uint32_t w_s, int (&hi)[G], int (&lo)[G]) {
     constexpr int SHIFT = G == 1 ? 3 : 4;                      // log2 of the record's bytes
     auto emit = [&](uint32_t syms, uint32_t a, uint32_t, uint32_t) {
@@ -185,7 +185,7 @@ __device__ __forceinline__ bool decode_dot_impl(uint32_t slot_s, uint32_t byte_p
     };
     // two lookups per round: the weight rows keep WROW - 128 zeroed positions for what is emitted past 127
     static_assert(WROW >= 128 + KVC_DECODE_OVERRUN + 1, "weight rows too short for paired lookups");
-    return kvc_decode_vector<ESC, SHIFT>(slot_s, byte_pos, lut_s, KvcTreeShared{tree_s}, w_s >> SHIFT, emit);
+    return kvc_decode_vector<ESC, SHIFT>(slot_s, byte_pos, lut_s, tree, w_s >> SHIFT, emit);
 }
 // esc: the book has codes longer than the table window (uniform over the CTA)
 template <int G>
@@ -193,8 +193,8 @@ __device__ __forceinline__ bool decode_dot(const uint8_t *slot, uint32_t byte_po
                                            const uint32_t *w, int (&hi)[G], int (&lo)[G]) {
     const uint32_t slot_s = kvc_smem_addr(slot), lut_s = kvc_smem_addr(book.lut), tree_s = kvc_smem_addr(book.tree),
                    w_s = kvc_smem_addr(w);
-    return esc ? decode_dot_impl<G, true>(slot_s, byte_pos, lut_s, tree_s, w_s, hi, lo)
-               : decode_dot_impl<G, false>(slot_s, byte_pos, lut_s, tree_s, w_s, hi, lo);
+    return esc ? decode_dot_impl<G, true>(slot_s, byte_pos, lut_s, KvcTreeShared{tree_s}, w_s, hi, lo)
+               : decode_dot_impl<G, false>(slot_s, byte_pos, lut_s, KvcTreeShared{tree_s}, w_s, hi, lo);
 }
 __device__ __forceinline__ bool book_has_long_codes(const void *book) {
     return kvc_book_needs_escape(book);
@@ -390,17 +390,6 @@ __device__ __forceinline__ void k_token_unit(unsigned short &sc, int &mi, const 
     sc = kvc_load_scale_bits(m, u); mi = kvc_load_min(m, u);
 }
 
-// sum of each query head's 128 (scaled) values: one warp per head; needs a barrier before and after
-template <int G>
-__device__ __forceinline__ void q_sums(const float *qf, float *qsum, int tid) {
-    if (tid < G * 32) {
-        const int g = tid >> 5, lane = tid & 31;
-        float s = qf[g * 128 + lane] + qf[g * 128 + lane + 32] + qf[g * 128 + lane + 64] + qf[g * 128 + lane + 96];
-        s = kvc_warp_sum(s);
-        if (lane == 0) qsum[g] = s;
-    }
-}
-
 // score of the thread's token from its integer dot products
 template <int G>
 __device__ __forceinline__ void k_finish(float (&s)[G], const int (&hi)[G], const int (&lo)[G], const float *step_sub,
@@ -566,406 +555,40 @@ __global__ void __launch_bounds__(NTHR, 6) fused_pv_kernel(CacheDev vc, long lon
 }
 
 // ---- one-pass decode attention -------------------------------------------------------------------
-struct alignas(32) AttnSmem {                     // of the one-head kernel; followed in shared memory by 4 K slots, 4 V slots (sized at launch),
-    KvcBookSmem bookK, bookV;         // SLOT_PAD bytes that a corrupt stream's decoder overrun may read
-    alignas(32) uint32_t w[4 * 2 * WROW];     // K weight words; reused by v_weights (scratch), the tail and the final cross-group sum
-    alignas(32) uint32_t ps[2 * 2 * WROW];    // V weight words
-    float kstep[4], zp[4];
-    float vstep[2];
-    float qf[128];
-    float qsum[1];
-    float red[4][8];                  // per-warp max, sum, zpv and weight-max partials
-    uint64_t bar[2];                  // K and V staging barriers
-    uint32_t leadK[4], leadV[4];
-    uint32_t nbK[4], nbV[4];          // byte counts of the staged blocks
-    int okK[4], okV[4];
-    int next_j;                       // item the CTA drew for after the current one
-    int dead;                         // a staging wait ran out: the CTA takes no further item
-};
-
 struct AttnParams {
     CacheDev k, v;
     long long T, B, Hkv, Hq, Tr;
-    long long g0;                 // first query head of this launch (of each KV head): 0 in the one-head kernel
+    long long g0;                 // first query head of this launch (of each KV head)
     int nh;                       // and how many, 1 .. G
     const __half *q, *ktail, *vtail;
     __half *out;
     float scaling;
-    int n_tiles;                  // tiles per column: of 256 tokens, with grouped queries steps of 128
-    // every column is cut into `long_runs` runs of `tiles_per_split` tiles followed by `splits - long_runs`
-    // runs of `short_tiles` tiles; the items of the long runs of all columns come first, the short ones last
+    int n_tiles;                  // steps of 128 tokens per column
+    // every column is cut into `long_runs` runs of `tiles_per_split` steps followed by `splits - long_runs`
+    // runs of `short_tiles` steps; the items of the long runs of all columns come first, the short ones last
     int splits, tiles_per_split, long_runs, short_tiles;
     long long work;               // columns * splits items
     uint32_t slotK_bytes, slotV_bytes;   // capacity of one staging slot (multiple of 16)
-    float *ws_part;               // [B*Hq][splits][ATTN_PART_FLOATS], with grouped queries [..][ROWS_PART_FLOATS]
-    int *sched;                   // {items handed out, CTAs (grouped queries: workers) finished}, or null: static shares
+    float *ws_part;               // [B*Hq][splits][ROWS_PART_FLOATS]
+    int *sched;                   // {items handed out, workers finished}, or null: static shares
     int *status;
-    int team;                     // grouped queries without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
+    int team;                     // without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
     int wait_limit;               // tries of a staging wait before it gives up (KVC_FLAG_WAIT_TIMEOUT)
     int starve;                   // tests of the bounded waits only: announce bytes that are never copied
 };
 
-// One query head per KV head.  BULK: stage with bulk asynchronous copies (one tile phase ahead) instead of plain loads.
-// (The per-head values are arrays of one: as plain scalars the same kernel gets another register allocation, with 12 bytes of
-// spills: K units per block 2.7 % faster, K at relative bound 0.01 1.2 % slower, 128 columns of 8192 tokens with a tail 1.9 %.)
-template <bool BULK>
-__global__ void __launch_bounds__(NTHR, 3) attn_decode_kernel(AttnParams p) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    constexpr int G = 1;
-    AttnSmem &sm = *reinterpret_cast<AttnSmem *>(smem_raw);
-    uint8_t *const slotsK = smem_raw + sizeof(AttnSmem), *const slotsV = slotsK + 4 * p.slotK_bytes;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
-    const int grp = tid >> 7, ch = tid & 127;
-    // Launched with programmatic stream serialisation.  This kernel's own set-up -- the books' tables, the first
-    // blocks, the first tile's metadata: cache data that no kernel of a decode step writes -- runs before
-    // griddepcontrol.wait, i.e. possibly while the kernel ahead of it in the stream (the merge of the layer
-    // before, which lets its dependents start early) still runs.  What that kernel or the one before it may
-    // write (the query, the scheduling counters, the workspace, the output, the status word) is touched after
-    // the wait.  (Letting this kernel's own dependents start early was measured: their waiting CTAs slow the
-    // launch by a tenth.)
-    // shapes fit 32 bits (the host checks): 64-bit arithmetic only where block ids and addresses are formed
-    const int T = (int)p.T, B = (int)p.B, Hkv = (int)p.Hkv, Hq = (int)p.Hq;
-    const int cols = B * Hkv, Gt = Hq / Hkv;
-    const int n_tiles = p.n_tiles;
-    const kvc_qmeta_dev &km = p.k.q, &vm = p.v.q;
-    int flags = 0;
-
-    // The work is cut into items: a column (one sequence, one KV head) x one of `splits` runs of
-    // `tiles_per_split` tiles; item j = column * splits + run.  Without a scheduling counter CTA i of P
-    // takes the items [work*i/P, work*(i+1)/P).  With one it takes items i and P + i and draws every
-    // further item from the counter, two items ahead of its use so that the answer has an item's time
-    // to arrive: CTAs that run faster (the warp schedulers favour some of an SM's CTAs) take more.
-    struct Item { int col, t_lo, t_hi, part; };            // part: the run's index within its column
-    const bool draw = p.sched != nullptr;
-    const int P = (int)gridDim.x;                           // items are counted in 32 bits (the host checks the range)
-    const int w_hi = draw ? (int)p.work : (int)(p.work * (blockIdx.x + 1) / P);
-    auto item_of = [&](int j, Item &it) -> bool {
-        if (j >= w_hi) return false;
-        const int n_long = (int)cols * p.long_runs;          // items of long runs; the short runs follow: the last
-        if (j < n_long) {                                    // items to be drawn are short, so the CTAs end close together
-            const int r = j % p.long_runs;
-            it.col = j / p.long_runs; it.part = r; it.t_lo = r * p.tiles_per_split; it.t_hi = min(n_tiles, it.t_lo + p.tiles_per_split);
-        } else {
-            const int n_short = p.splits - p.long_runs, r = (j - n_long) % n_short;
-            it.col = (j - n_long) / n_short; it.part = p.long_runs + r;
-            it.t_lo = p.long_runs * p.tiles_per_split + r * p.short_tiles; it.t_hi = min(n_tiles, it.t_lo + p.short_tiles);
-        }
-        return true;
-    };
-
-    // block ids of a tile's four K blocks / four V blocks for lane l < 4 of the issuing warp
-    auto blkK_of = [&](int col, int tile, int l) { return ((long long)tile * 4 + l) * cols + col; };
-    auto blkV_of = [&](int col, int tile, int l) { return ((long long)tile * 2 + (l >> 1)) * (cols * 2) + (long long)col * 2 + (l & 1); };
-    auto validK = [&](bool on, int tile, int l) { return on && (long long)tile * 256 + l * 64 < T; };
-    auto validV = [&](bool on, int tile, int l) { return on && (long long)tile * 256 + (l >> 1) * 128 < T; };
-
-    Item it, nit;
-    int j_it = draw ? (int)blockIdx.x : (int)(p.work * blockIdx.x / P), j_n1 = draw ? P + (int)blockIdx.x : j_it + 1;
-    bool have = item_of(j_it, it), have_next = have && item_of(j_n1, nit);
-    int drawn = 0;                                         // thread 0: the counter's answer, used an item later
-    const bool any_tiles = have && it.t_lo < it.t_hi;      // items are empty only when the cache has no compressed part
-
-    if (BULK) {
-        if (tid == 0) { kvc_mbar_init(&sm.bar[0], 1); kvc_mbar_init(&sm.bar[1], 1); kvc_mbar_fence_init(); sm.dead = 0; }
-        __syncthreads();
-        if (warp == 0 && any_tiles) {
-            stage_bulk(p.k, validK(true, it.t_lo, lane & 3), blkK_of(it.col, it.t_lo, lane & 3), slotsK + (lane & 3) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0);
-            stage_bulk(p.v, validV(true, it.t_lo, lane & 3), blkV_of(it.col, it.t_lo, lane & 3), slotsV + (lane & 3) * p.slotV_bytes, sm.leadV, sm.okV, sm.nbV, &sm.bar[1], lane, p.starve != 0);
-        }
-    }
-    bool escK = false, escV = false;
-    if (p.T > 0) {                                         // (no streams at all while nothing is compressed yet)
-        kvc_load_book(sm.bookK, p.k.book, tid, NTHR);
-        kvc_load_book(sm.bookV, p.v.book, tid, NTHR);
-        escK = book_has_long_codes(p.k.book); escV = book_has_long_codes(p.v.book);
-    }
-
-    // Per-thread metadata of a tile (vector start offsets, the token's V scale / min_int, the K unit
-    // parameters of the warp's block) is fetched one tile ahead, so that no global-memory latency
-    // sits between the phases of a tile.
-    struct TileMeta { unsigned short startK, startV, vsc, ksc; int vmi, kmi; KUnit ku; };   // as loaded: no arithmetic waits on them here
-    auto load_meta = [&](bool on, int col, int tile, TileMeta &tm) {
-        const long long tok0 = (long long)tile * 256, t = tok0 + tid;
-        const long long gI = tok0 / 128 + grp;
-        const int b = col / (int)Hkv, h = col % (int)Hkv;
-        tm.startK = tm.startV = 0; tm.vsc = 0; tm.vmi = tm.kmi = 0; tm.ksc = 0x3c00;
-        if (on) {
-            if (t < T) {
-                tm.startK = vec_start_bits(p.k.thread_info, (tok0 / 64 + sub) * cols + col, v);
-                const long long u = kvc_tok_unit(t, vm.tok_div) * vm.sj + b * vm.sb + h * vm.sh;
-                tm.vsc = kvc_load_scale_bits(vm, u); tm.vmi = kvc_load_min(vm, u);
-                if (km.sc == 0) k_token_unit(tm.ksc, tm.kmi, km, t, b, h);
-            }
-            if (gI * 128 < T) tm.startV = vec_start_bits(p.v.thread_info, gI * (cols * 2) + (long long)col * 2 + (ch >> 6), v);
-        }
-        k_units_load(tm.ku, km, on ? tok0 : T, T, b, h, tid);
-    };
-    TileMeta cur, nxt;
-    load_meta(any_tiles, have ? it.col : 0, have ? it.t_lo : 0, cur);
-
-    // The query values of an item are fetched (as fp16 bits) while the item before it still runs.
-    constexpr int QN = (G * 128 + NTHR - 1) / NTHR;
-    unsigned short qn[QN];
-    auto q_fetch = [&](int col_) {
-        const long long row0 = (long long)(col_ / (int)Hkv) * Hq + (long long)(col_ % (int)Hkv) * Gt + p.g0;
-#pragma unroll
-        for (int i = 0; i < QN; i++) {
-            const int idx = tid + i * NTHR;
-            qn[i] = 0;
-            if (idx < G * 128) qn[i] = reinterpret_cast<const unsigned short *>(p.q)[(row0 + (idx >> 7)) * 128 + (idx & 127)];
-        }
-    };
-    auto q_store = [&]() {
-#pragma unroll
-        for (int i = 0; i < QN; i++) {
-            const int idx = tid + i * NTHR;
-            if (idx < G * 128) sm.qf[idx] = kvc_scale_value(qn[i]) * p.scaling;
-        }
-    };
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (have) q_fetch(it.col);
-
-    uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
-    while (have) {
-    const int col = it.col, b = col / (int)Hkv, h = col % (int)Hkv;
-    const long long hq0 = h * Gt + p.g0;
-    if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
-    q_store();                                             // fetched during the previous item's last tile
-    __syncthreads();
-    q_sums<G>(sm.qf, sm.qsum, tid);
-    __syncthreads();                                       // books, q and (unbuffered) slots are in place
-    float m_run[G], l_run[G], acc[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) { m_run[g] = -CUDART_INF_F; l_run[g] = 0.f; acc[g] = 0.f; }
-
-    for (int tile = it.t_lo; tile < it.t_hi; tile++) {
-        const long long tok0 = (long long)tile * 256, t = tok0 + tid;
-        const long long blkK = (tok0 / 64 + sub) * cols + col;
-        const long long gI = tok0 / 128 + grp;
-        const long long blkV = gI * (cols * 2) + (long long)col * 2 + (ch >> 6);
-        const bool actK = t < T, actV = gI * 128 < T;
-        // the tile after this one in the CTA's sequence (it may open the next column)
-        bool n_on = true; int n_col = col, n_tile = tile + 1;
-        if (n_tile >= it.t_hi) {
-            n_on = have_next && nit.t_lo < nit.t_hi; n_col = n_on ? nit.col : col; n_tile = n_on ? nit.t_lo : 0;
-            if (have_next) q_fetch(nit.col);
-        }
-        if (!BULK) {
-            if (actK) { uint32_t ld, nb; bool ok = stage(p.k, blkK, slotsK + sub * p.slotK_bytes, &ld, &nb, v); if (v == 0) { sm.leadK[sub] = ld; sm.nbK[sub] = nb; sm.okK[sub] = ok; } }
-            if (actV) { uint32_t ld, nb; bool ok = stage(p.v, blkV, slotsV + sub * p.slotV_bytes, &ld, &nb, v); if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; } }
-        }
-        k_weights_build<G>(sm.w, sm.kstep, sm.zp, sm.qf, cur.ku, km.sc != 0, km.min_bytes, tok0, T, tid);
-        // A wait that runs out: the thread does not decode.  The warp that issues the copies looks at its own
-        // verdict: a barrier whose phase it did not see complete is never armed again (a second arrival on an
-        // open phase is an error), and the CTA is marked; it takes no further item, and what it had in flight
-        // is waited for once more, bounded, before it returns.
-        bool k_landed = true;
-        if (BULK) {
-            k_landed = kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit);
-            if (k_landed) par ^= 1u; else flags |= KVC_FLAG_WAIT_TIMEOUT;
-        }
-        __syncthreads();
-        // ---- K: scores of this tile's tokens
-        float s[G];
-        if (actK) {
-            int hi[G], lo[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
-            bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
-            if (ok) {
-                ok = decode_dot<G>(slotsK + sub * p.slotK_bytes, sm.leadK[sub] + (cur.startK >> 3), sm.bookK, escK, sm.w + sub * 2 * WROW * G, hi, lo);
-            }
-            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
-            k_finish<G>(s, hi, lo, sm.kstep + sub * G, sm.zp + sub * G, sm.qsum, km.sc != 0, kvc_scale_value(cur.ksc), (float)cur.kmi);
-        } else {
-#pragma unroll
-            for (int g = 0; g < G; g++) s[g] = -CUDART_INF_F;
-        }
-        // ---- online softmax over the tile
-#pragma unroll
-        for (int g = 0; g < G; g++) { float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
-        __syncthreads();                                   // also: every thread is done with the K slots
-        // the next tile's per-thread metadata is asked for now and first touched when that tile begins: it is in
-        // flight during the V phase only, and the K decode above ran without its registers
-        load_meta(n_on, n_col, n_tile, nxt);
-        if (BULK && warp == 0) {                           // next tile's K blocks land during the V phase
-            if (__all_sync(0xffffffffu, k_landed))
-                stage_bulk(p.k, validK(n_on, n_tile, lane & 3), blkK_of(n_col, n_tile, lane & 3), slotsK + (lane & 3) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0);
-            else if (lane == 0) sm.dead = 1;
-        }
-        float alpha[G], wv[G];
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            float mt = sm.red[0][g];
-#pragma unroll
-            for (int w8 = 1; w8 < 8; w8++) mt = fmaxf(mt, sm.red[0][w8 * G + g]);
-            const float m_new = fmaxf(m_run[g], mt);
-            alpha[g] = __expf(m_run[g] - m_new);           // exp(-inf) = 0 on the first tile
-            const float pr = actK ? __expf(s[g] - m_new) : 0.f;
-            m_run[g] = m_new;
-            wv[g] = pr * kvc_scale_value(cur.vsc);
-            const float ssum = kvc_warp_sum(pr), zsum = kvc_warp_sum(wv[g] * (float)cur.vmi);
-            if (lane == 0) { sm.red[1][warp * G + g] = ssum; sm.red[2][warp * G + g] = zsum; }
-        }
-        // (the K weights are spent: their memory is the scratch of the V weights' 16-bit values)
-        v_weights<G>(sm.ps, sm.vstep, sm.red[3], reinterpret_cast<int16_t *>(sm.w), wv, tid);      // three barriers inside
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            float lt = 0.f;
-#pragma unroll
-            for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + g];
-            l_run[g] = l_run[g] * alpha[g] + lt;
-        }
-        const bool v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
-        if (BULK && v_landed) par ^= 2u;
-        if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
-        // ---- V: accumulate this tile's contribution for the thread's (group, channel)
-        float dv[G];
-#pragma unroll
-        for (int g = 0; g < G; g++) dv[g] = 0.f;
-        if (actV) {
-            int hi[G], lo[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) { hi[g] = 0; lo[g] = 0; }
-            bool ok = v_landed && sm.okV[sub] && (uint32_t)(cur.startV >> 3) < sm.nbV[sub];
-            if (ok) {
-                ok = decode_dot<G>(slotsV + sub * p.slotV_bytes, sm.leadV[sub] + (cur.startV >> 3), sm.bookV, escV, sm.ps + grp * 2 * WROW * G, hi, lo);
-            }
-            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                dv[g] = fix_value(sm.vstep[grp * G + g], hi[g], lo[g]) +
-                        sm.red[2][(grp * 4 + 0) * G + g] + sm.red[2][(grp * 4 + 1) * G + g] +
-                        sm.red[2][(grp * 4 + 2) * G + g] + sm.red[2][(grp * 4 + 3) * G + g];
-        }
-#pragma unroll
-        for (int g = 0; g < G; g++) acc[g] = fmaf(acc[g], alpha[g], dv[g]);
-        __syncthreads();                                   // every thread is done with the V slots, weights and sums
-        if (BULK && warp == 0) {                           // next tile's V blocks land during its K phase
-            if (__all_sync(0xffffffffu, v_landed))
-                stage_bulk(p.v, validV(n_on, n_tile, lane & 3), blkV_of(n_col, n_tile, lane & 3), slotsV + (lane & 3) * p.slotV_bytes, sm.leadV, sm.okV, sm.nbV, &sm.bar[1], lane, p.starve != 0);
-            else if (lane == 0) sm.dead = 1;
-        }
-        cur = nxt;
-    }
-
-    // ---- uncompressed tail (the recent window), handled with the column's last tiles: dense fp16 rows.
-    // Only for callers without a workspace: otherwise the merge kernel adds the tail (see there).
-    if (p.Tr > 0 && !p.partial && it.t_hi == n_tiles) {
-        float *pt = reinterpret_cast<float *>(sm.w);           // p[row][g] for 256 rows
-        for (long long r0 = 0; r0 < p.Tr; r0 += 256) {
-            const long long r = r0 + tid;
-            const bool act = r < p.Tr;
-            __syncthreads();
-            float s[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) s[g] = act ? 0.f : -CUDART_INF_F;
-            if (act) {
-                const __half *kr = p.ktail + ((r * B + b) * Hkv + h) * 128;
-                for (int c8 = 0; c8 < 16; c8++) {
-                    uint4 kv = *reinterpret_cast<const uint4 *>(kr + c8 * 8);
-                    const __half *kh = reinterpret_cast<const __half *>(&kv);
-#pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        const float kf = __half2float(kh[k]);
-#pragma unroll
-                        for (int g = 0; g < G; g++) s[g] = fmaf(kf, sm.qf[g * 128 + c8 * 8 + k], s[g]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < G; g++) { float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
-            __syncthreads();
-            float alpha[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                float mt = sm.red[0][g];
-#pragma unroll
-                for (int w8 = 1; w8 < 8; w8++) mt = fmaxf(mt, sm.red[0][w8 * G + g]);
-                const float m_new = fmaxf(m_run[g], mt);
-                alpha[g] = __expf(m_run[g] - m_new);
-                const float pr = act ? __expf(s[g] - m_new) : 0.f;
-                m_run[g] = m_new;
-                pt[tid * G + g] = pr;
-                const float ssum = kvc_warp_sum(pr);
-                if (lane == 0) sm.red[1][warp * G + g] = ssum;
-            }
-            __syncthreads();
-            float dv[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                float lt = 0.f;
-#pragma unroll
-                for (int w8 = 0; w8 < 8; w8++) lt += sm.red[1][w8 * G + g];
-                l_run[g] = l_run[g] * alpha[g] + lt;
-                dv[g] = 0.f;
-            }
-            // thread (grp, ch) sums rows r0 + 128*grp .. +127 of its channel
-            for (int i = 0; i < 128; i++) {
-                const long long rr = r0 + grp * 128 + i;
-                if (rr >= p.Tr) break;
-                const float vf = __half2float(p.vtail[((rr * B + b) * Hkv + h) * 128 + ch]);
-#pragma unroll
-                for (int g = 0; g < G; g++) dv[g] = fmaf(pt[(grp * 128 + i) * G + g], vf, dv[g]);
-            }
-#pragma unroll
-            for (int g = 0; g < G; g++) acc[g] = fmaf(acc[g], alpha[g], dv[g]);
-        }
-    }
-    if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without tiles fetched nothing yet
-    const long long head0 = b * Hq + hq0;
-    if (!p.partial) {
-        // ---- the item is the whole column: combine the CTA's two token groups and write the output
-        __syncthreads();
-        float *sumbuf = reinterpret_cast<float *>(sm.w);       // [2][128][G]
-#pragma unroll
-        for (int g = 0; g < G; g++) sumbuf[(grp * 128 + ch) * G + g] = acc[g];
-        __syncthreads();
-        if (tid < 128) {
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                p.out[(head0 + g) * 128 + tid] = __float2half_rn((sumbuf[tid * G + g] + sumbuf[(128 + tid) * G + g]) / l_run[g]);
-        }
-    } else {
-        // ---- a partial result {m, l, -, -, acc of group 0 [128], acc of group 1 [128]}; a second kernel merges
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            float *dst = p.ws_part + ((head0 + g) * p.splits + it.part) * ATTN_PART_FLOATS;
-            dst[4 + tid] = acc[g];                             // tid = grp * 128 + ch
-            if (tid == 0) { dst[0] = m_run[g]; dst[1] = l_run[g]; }
-        }
-    }
-    if (draw && tid == 0) sm.next_j = drawn;
-    __syncthreads();                                       // the sums are read before the next column's weights overwrite them
-    if (BULK && sm.dead != 0) break;                       // a staging wait ran out: the status word says so, the item's result is void
-    const int j_n2 = draw ? 2 * P + sm.next_j : j_n1 + 1;
-    it = nit; have = have_next; j_it = j_n1; j_n1 = j_n2;
-    have_next = have && item_of(j_n1, nit);
-    }   // items of the CTA
-    if (BULK && any_tiles) {              // the copies issued after the last tile are empty, but their phase must end;
-        // after a wait that ran out, these are the phases still open: nothing may be in flight at the return
-        if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
-        if (!kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
-    }
-    if (flags) atomicOr(p.status, flags);
-    if (draw && tid == 0) {               // the last CTA to finish leaves the scheduling counters zeroed for the next launch
-        __threadfence();
-        if (atomicAdd(&p.sched[1], 1) == (int)gridDim.x - 1) { p.sched[0] = 0; p.sched[1] = 0; __threadfence(); }
-    }
-}
-
 // ---- grouped queries: the same attention with workers of 128 threads --------------------------------
 // A CTA is one resident per SM, with one copy of the two decode tables and up to five (eight heads: four) workers.
-// A worker is four warps with slots, rows, weights and barriers of its own; it draws items like a CTA of the one-head
-// kernel and walks them in steps of 128 tokens (two K blocks, the two V blocks of a column).  The tables take 32 KB
+// A worker is four warps with slots, rows, weights and barriers of its own; it draws items and walks them in steps of 128
+// tokens (two K blocks, the two V blocks of a column).  The tables take 32 KB
 // and a worker 35 to 45 KB: two CTAs of 256 threads with a copy each held four workers' worth of warps, and all eight
-// warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads, now 720; 448 and 404 us at
-// 32 x 16384 tokens, 4 x 2 heads, now 360).  Registers: 96 with two and four columns, where the compiler spills 60 to 70 bytes
+// warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads, with workers 720; 448 and 404 us at
+// 32 x 16384 tokens, 4 x 2 heads, with workers 360).  Registers: 96 with two and four columns, where the compiler spills 60 to 70 bytes
 // per thread (five workers leave no more), 128 without spills with eight.
-constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]; two of them take the room of one of the one-head kernel
-static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "the workspace is sized in the one-head kernel's partial results");
-template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : 5; }
+constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]
+static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "a workspace for n runs of 256-token tiles holds 2 n partial results");
+template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : (G == 1 ? 7 : 5); }
 
 template <int G>
 struct alignas(32) RowsWorker {
@@ -990,7 +613,8 @@ template <int G> int rows_fit(const AttnParams &p) {         // workers that an 
     while (workers > 1 && rows_smem<G>(p, workers) > MAX_CTA_SHARED) workers--;
     return workers;
 }
-int rows_fit(const AttnParams &p, int heads) { return heads > 4 ? rows_fit<8>(p) : (heads > 2 ? rows_fit<4>(p) : rows_fit<2>(p)); }
+int one_fit(const AttnParams &p);
+int rows_fit(const AttnParams &p, int heads) { return heads == 1 ? one_fit(p) : heads > 4 ? rows_fit<8>(p) : (heads > 2 ? rows_fit<4>(p) : rows_fit<2>(p)); }
 
 // How many of an SM's workers share a column when every column's output is written directly (no workspace, or a single run
 // without a tail): without company a worker would take all of a column's `units` (steps and passes of the tail) in turn
@@ -1026,8 +650,11 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     const int h2 = (2 * (lane & 3)) % G, r4 = lane & ~3;
     const bool own = 2 * (lane & 3) < G;                   // with fewer than 8 heads the other lanes hold copies
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
-    // launched with programmatic stream serialisation, as the one-head kernel: set-up before griddepcontrol.wait reads
-    // cache data only
+    // launched with programmatic stream serialisation: this kernel's own set-up -- the tables, the first blocks, the first step's metadata: cache
+    // data that no kernel of a decode step writes -- runs before griddepcontrol.wait, possibly while the kernel ahead of it in the
+    // stream (the merge of the layer before, which lets its dependents start early) still runs.  What that kernel or the one before it may
+    // write (the query, the scheduling counters, the workspace, the output, the status word) is touched after the wait.  (Letting this
+    // kernel's own dependents start early was measured: their waiting CTAs slow the launch by a tenth.)
     const int B = (int)p.B, Hkv = (int)p.Hkv, Hq = (int)p.Hq;
     const int cols = B * Hkv, Gt = Hq / Hkv;
     const kvc_qmeta_dev &km = p.k.q, &vm = p.v.q;
@@ -1148,7 +775,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; }
         }
         k_weights_rows<G>(sm.w, sm.kstep, sm.zp, sm.q, p.scaling, cur.ku, km.sc != 0, km.min_bytes, warp & 1, warp >> 1, lane);
-        bool k_landed = true;                              // (a wait that runs out: see the one-head kernel)
+        bool k_landed = true;                              // (a wait that runs out: see attn_one_kernel)
         if (BULK) {
             k_landed = kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit);
             if (k_landed) par ^= 1u; else flags |= KVC_FLAG_WAIT_TIMEOUT;
@@ -1386,6 +1013,354 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     }
 }
 
+// ---- one query head per KV head ------------------------------------------------------------------------
+// The same workers with a decoder that multiplies as it goes: each lookup's symbols meet the weight record of its position
+// (decode_dot), so there are no rows, and an SM holds one copy of the tables and up to ONE_WORKERS workers: 28 warps of 72
+// registers where three CTAs of 256 threads with tables of their own, all eight warps at every barrier, were 24.  8 x 32 columns of
+// 4096 tokens, rel 0.05 / 0.1: 135 us, now 128.  (Eight workers of 64 registers, 52 bytes of spills: 145, with runs of other lengths 134.)
+constexpr int ONE_WORKERS = rows_workers<1>();
+
+struct alignas(32) OneWorker {
+    uint32_t w[2 * 2 * WROW];                // K weight records of the step's two blocks; scratch of the tail
+    uint32_t ps_before[8];                   // bytes of the V records' neighbours ahead of the first one
+    uint32_t ps[2 * WROW];                   // V weight records
+    float red[4][4];                         // per-warp max, sum, zero-point and weight-max partials
+    unsigned short q[128];                   // the query, fp16 bits
+    float kstep[2], zp[2], qsum;
+    uint64_t bar[2];                         // K and V staging barriers
+    uint32_t leadK[4], leadV[4], nbK[4], nbV[4];   // of the two staged blocks (stage_bulk writes four entries)
+    int okK[4], okV[4];
+    int next_j, dead;
+};
+// tables, workers, slots (two of K and two of V each), bytes that a corrupt stream's overrun may read
+size_t one_smem(const AttnParams &p, int workers) {
+    return sizeof(RowsTables) + workers * (sizeof(OneWorker) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes)) + SLOT_PAD;
+}
+int one_fit(const AttnParams &p) {
+    int workers = ONE_WORKERS;
+    while (workers > 1 && one_smem(p, workers) > MAX_CTA_SHARED) workers--;
+    return workers;
+}
+
+// K weight records of block `sub`: lane = 4 consecutive channels; qh: the query's fp16 bits
+__device__ __forceinline__ void k_weights_one(uint32_t *w, float *step, float *zp, const uint16_t *qh, float scaling, const KUnit &u,
+                                              bool channel_units, int min_bytes, int sub, int lane) {
+    const uint2 qb = *reinterpret_cast<const uint2 *>(qh + lane * 4);
+    const uint32_t q2[2] = {qb.x, qb.y};
+    float wv[4], z = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float q = kvc_scale_value((unsigned short)(q2[i >> 1] >> (16 * (i & 1)))) * scaling, sc = kvc_scale_value(ku_scale(u, i));
+        wv[i] = q * sc;
+        z = fmaf((float)ku_min(u, i, min_bytes) * sc, q, z);
+    }
+    const float mx = kvc_warp_max(fmaxf(fmaxf(fabsf(wv[0]), fabsf(wv[1])), fmaxf(fabsf(wv[2]), fabsf(wv[3]))));
+    z = channel_units ? kvc_warp_sum(z) : 0.f;
+    const float st = fix_step(mx), inv = st > 0.f ? 1.0f / st : 0.f;
+    int q4[7];
+#pragma unroll
+    for (int i = 0; i < 4; i++) q4[i] = __float2int_rn(wv[i] * inv);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {                               // the next lane's first three values
+        const int nv = __shfl_down_sync(0xffffffffu, q4[i], 1);
+        q4[4 + i] = lane == 31 ? 0 : nv;
+    }
+    uint32_t *row = w + sub * 2 * WROW;
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+        const uint2 a = pack4(q4[i], q4[i + 1], q4[i + 2], 0), b = pack4(q4[i + 1], q4[i + 2], q4[i + 3], 0);
+        *reinterpret_cast<uint4 *>(&row[2 * (lane * 4 + i)]) = make_uint4(a.x, a.y, b.x, b.y);
+    }
+    if (lane < 2 * (WROW - 128)) row[2 * 128 + lane] = 0u;
+    if (lane == 0) { step[sub] = st; zp[sub] = z; }
+}
+
+__device__ __forceinline__ void sts8(uint32_t addr, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" :: "r"(addr), "r"(v) : "memory"); }
+
+template <bool BULK, bool TEAM>
+__global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnParams p) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    RowsTables &tab = *reinterpret_cast<RowsTables *>(smem_raw);
+    const int workers = blockDim.x >> 7, wk = threadIdx.x >> 7;
+    const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
+    uint8_t *const wbase = smem_raw + sizeof(RowsTables), *const sbase = wbase + workers * sizeof(OneWorker);
+    OneWorker &sm = reinterpret_cast<OneWorker *>(wbase)[wk];
+    uint8_t *const slotsK = sbase + wk * 2 * (p.slotK_bytes + p.slotV_bytes), *const slotsV = slotsK + 2 * p.slotK_bytes;
+    auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
+    // launched with programmatic stream serialisation, as the grouped kernel: set-up before griddepcontrol.wait reads cache data only
+    const int B = (int)p.B, Hkv = (int)p.Hkv, cols = B * Hkv;
+    const kvc_qmeta_dev &km = p.k.q, &vm = p.v.q;
+    int flags = 0;
+
+    struct Item { int col, t_lo, t_hi, part; };            // steps t_lo .. t_hi - 1 of a column; part: the run's index
+    const bool draw = !TEAM && p.sched != nullptr;
+    const int P = (int)gridDim.x * (TEAM ? workers / p.team : workers);
+    const int me = TEAM ? wk / p.team * (int)gridDim.x + (int)blockIdx.x : (int)blockIdx.x * workers + wk;
+    const int w_hi = draw ? (int)p.work : (int)(p.work * (me + 1) / P);
+    auto item_of = [&](int j, Item &it) -> bool {
+        if (j >= w_hi) return false;
+        const int n_long = cols * p.long_runs;
+        if constexpr (TEAM) {                              // the worker's share of column j: the same for every column
+            const int tk = wk % p.team;
+            it.col = j; it.part = 0; it.t_lo = (int)((long long)p.n_tiles * tk / p.team); it.t_hi = (int)((long long)p.n_tiles * (tk + 1) / p.team);
+        } else if (j < n_long) {
+            const int r = j % p.long_runs;
+            it.col = j / p.long_runs; it.part = r; it.t_lo = r * p.tiles_per_split; it.t_hi = min(p.n_tiles, it.t_lo + p.tiles_per_split);
+        } else {
+            const int n_short = p.splits - p.long_runs, r = (j - n_long) % n_short;
+            it.col = (j - n_long) / n_short; it.part = p.long_runs + r;
+            it.t_lo = p.long_runs * p.tiles_per_split + r * p.short_tiles; it.t_hi = min(p.n_tiles, it.t_lo + p.short_tiles);
+        }
+        return true;
+    };
+    auto blkK_of = [&](int col, int t, int l) { return ((long long)t * 2 + l) * cols + col; };
+    auto blkV_of = [&](int col, int t, int l) { return (long long)t * (cols * 2) + (long long)col * 2 + l; };
+
+    Item it, nit;
+    int j_n1 = draw ? P + me : (int)(p.work * me / P) + 1;
+    bool have = item_of(draw ? me : j_n1 - 1, it), have_next = have && item_of(j_n1, nit);
+    int drawn = 0;                                         // thread 0: the counter's answer, used an item later
+    const bool any = have && it.t_lo < it.t_hi;
+
+    // the two blocks of a step, by the lanes 0 and 1 of the worker's first warp
+    auto stage_K = [&](bool on, int col, int t) { stage_bulk(p.k, on && lane < 2, blkK_of(col, t, lane & 1), slotsK + (lane & 1) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0); };
+    auto stage_V = [&](bool on, int col, int t) { stage_bulk(p.v, on && lane < 2, blkV_of(col, t, lane & 1), slotsV + (lane & 1) * p.slotV_bytes, sm.leadV, sm.okV, sm.nbV, &sm.bar[1], lane, p.starve != 0); };
+    if (BULK) {
+        if (tid == 0) { kvc_mbar_init(&sm.bar[0], 1); kvc_mbar_init(&sm.bar[1], 1); kvc_mbar_fence_init(); sm.dead = 0; }
+        sync();
+        if (warp == 0 && any) { stage_K(true, it.col, it.t_lo); stage_V(true, it.col, it.t_lo); }
+    }
+    kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
+    kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
+    const bool escK = book_has_long_codes(p.k.book), escV = book_has_long_codes(p.v.book);
+    for (int i = tid; i < 2 * WROW; i += 128) sm.ps[i] = 0u;   // V records: the bytes that no token writes stay zero
+
+    struct StepMeta { unsigned short startK, startV, vsc, ksc; int vmi, kmi; KUnit ku; };   // as loaded: no arithmetic waits on them here
+    auto load_meta = [&](bool on, int col, int step, StepMeta &m) {
+        const long long t = (long long)step * 128 + tid;
+        const int b = col / Hkv, h = col % Hkv;
+        m.startK = m.startV = 0; m.vsc = 0; m.vmi = m.kmi = 0; m.ksc = 0x3c00;
+        m.ku.sc = make_uint2(0x3c003c00u, 0x3c003c00u); m.ku.mi = make_uint2(0u, 0u);          // 1.0, 0
+        if (!on) return;
+        m.startK = vec_start_bits(p.k.thread_info, blkK_of(col, step, sub), v);
+        m.startV = vec_start_bits(p.v.thread_info, blkV_of(col, step, sub), v);
+        const long long u = kvc_tok_unit(t, vm.tok_div) * vm.sj + b * vm.sb + h * vm.sh;
+        m.vsc = kvc_load_scale_bits(vm, u); m.vmi = kvc_load_min(vm, u);
+        if (km.sc == 0) k_token_unit(m.ksc, m.kmi, km, t, b, h);
+        else if (warp < 2) {                               // of the block whose weights the warp builds, 4 channels per lane
+            const long long un = kvc_tok_unit((long long)step * 128 + warp * 64, km.tok_div) * km.sj + b * km.sb + h * km.sh + lane * 4;
+            m.ku.sc = *reinterpret_cast<const uint2 *>(reinterpret_cast<const unsigned short *>(km.scale) + un);
+            if (km.min_bytes == 1) m.ku.mi.x = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const int8_t *>(km.min_int) + un);
+            else m.ku.mi = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int16_t *>(km.min_int) + un);
+        }
+    };
+    StepMeta cur, nxt;
+    load_meta(any, have ? it.col : 0, have ? it.t_lo : 0, cur);
+    unsigned short qn = 0;                                 // the query of an item is fetched while the item before it runs; a column is a head
+    auto q_fetch = [&](int col_) { qn = reinterpret_cast<const unsigned short *>(p.q)[(long long)col_ * 128 + tid]; };
+    __syncthreads();                                       // the tables are in; from here on the workers go their own ways
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (have) q_fetch(it.col);
+
+    uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
+    while (have) {
+    const int col = it.col, b = col / Hkv, h = col % Hkv;
+    if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
+    sm.q[tid] = qn;
+    sync();
+    if (warp == 3) {                                       // sum of the query's 128 (scaled) values (read behind the next barrier)
+        float a = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) a += kvc_scale_value(sm.q[k * 32 + lane]) * p.scaling;
+        a = kvc_warp_sum(a);
+        if (lane == 0) sm.qsum = a;
+    }
+    float m_run = -CUDART_INF_F, l_run = 0.f, acc = 0.f;   // acc: channel tid
+
+    for (int step = it.t_lo; step < it.t_hi; step++) {
+        bool n_on = true; int n_col = col, n_step = step + 1;      // the worker's next step (it may open the next column)
+        if (n_step >= it.t_hi) {
+            n_on = have_next && nit.t_lo < nit.t_hi; n_col = n_on ? nit.col : col; n_step = n_on ? nit.t_lo : 0;
+            if (have_next) q_fetch(nit.col);
+        }
+        if (!BULK) {
+            uint32_t ld, nb;
+            bool ok = stage(p.k, blkK_of(col, step, sub), slotsK + sub * p.slotK_bytes, &ld, &nb, v);
+            if (v == 0) { sm.leadK[sub] = ld; sm.nbK[sub] = nb; sm.okK[sub] = ok; }
+            ok = stage(p.v, blkV_of(col, step, sub), slotsV + sub * p.slotV_bytes, &ld, &nb, v);
+            if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; }
+        }
+        if (warp < 2) k_weights_one(sm.w, sm.kstep, sm.zp, sm.q, p.scaling, cur.ku, km.sc != 0, km.min_bytes, warp, lane);
+        // A wait that runs out: the thread does not decode.  The warp that issues the copies looks at its own verdict: a barrier
+        // whose phase it did not see complete is never armed again (a second arrival on an open phase is an error), and the worker
+        // is marked; it takes no further item, and what it had in flight is waited for once more, bounded, before it returns.
+        bool k_landed = true;
+        if (BULK) {
+            k_landed = kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit);
+            if (k_landed) par ^= 1u; else flags |= KVC_FLAG_WAIT_TIMEOUT;
+        }
+        sync();
+        // ---- K: the score of the thread's token
+        float s;
+        {
+            int hi[1] = {0}, lo[1] = {0};
+            bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
+            if (ok) {
+                const uint32_t slot_s = kvc_smem_addr(slotsK + sub * p.slotK_bytes), at = sm.leadK[sub] + (cur.startK >> 3), w_s = kvc_smem_addr(sm.w + sub * 2 * WROW);
+                ok = escK ? decode_dot_impl<1, true>(slot_s, at, kvc_smem_addr(tab.lutK), KvcTreeGlobal(p.k.book), w_s, hi, lo)
+                          : decode_dot_impl<1, false>(slot_s, at, kvc_smem_addr(tab.lutK), KvcTreeGlobal(p.k.book), w_s, hi, lo);
+            }
+            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+            const float d = fix_value(sm.kstep[sub], hi[0], lo[0]);
+            s = km.sc != 0 ? d + sm.zp[sub] : kvc_scale_value(cur.ksc) * fmaf((float)cur.kmi, sm.qsum, d);
+        }
+        // ---- online softmax over the step
+        {
+            const float mx = kvc_warp_max(s);
+            if (lane == 0) sm.red[0][warp] = mx;
+        }
+        sync();                                            // also: every thread is done with the K slots and weights
+        load_meta(n_on, n_col, n_step, nxt);               // in flight during the V phase, first touched in the next step
+        if (BULK && warp == 0) {                           // the next step's K blocks land during the V phase
+            if (__all_sync(0xffffffffu, k_landed)) stage_K(n_on, n_col, n_step);
+            else if (lane == 0) sm.dead = 1;
+        }
+        float alpha, wv;
+        {
+            const float4 x = *reinterpret_cast<const float4 *>(sm.red[0]);
+            const float m_new = fmaxf(fmaxf(m_run, fmaxf(x.x, x.y)), fmaxf(x.z, x.w));
+            alpha = __expf(m_run - m_new);                 // exp(-inf) = 0 on the first step
+            m_run = m_new;
+            const float pr = __expf(s - m_new);
+            wv = pr * kvc_scale_value(cur.vsc);
+            const float ssum = kvc_warp_sum(pr), zsum = kvc_warp_sum(wv * (float)cur.vmi), wmax = kvc_warp_max(fabsf(wv));
+            if (lane == 0) { sm.red[1][warp] = ssum; sm.red[2][warp] = zsum; sm.red[3][warp] = wmax; }
+        }
+        sync();
+        // The V weights: the token's 16-bit value is a byte of either word of three records -- its own, and those of the two
+        // positions ahead of it (no exchange of values, no barrier for one).
+        float vst;
+        {
+            const float4 x = *reinterpret_cast<const float4 *>(sm.red[3]);
+            vst = fix_step(fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)));
+            const int q16 = __float2int_rn(wv * (vst > 0.f ? 1.0f / vst : 0.f));
+            const uint32_t a = kvc_smem_addr(sm.ps) + tid * 8, qh = (uint32_t)q16 >> 8, ql = (uint32_t)q16;
+            sts8(a + 1, qh); sts8(a + 5, ql); sts8(a - 6, qh); sts8(a - 2, ql); sts8(a - 13, qh); sts8(a - 9, ql);
+        }
+        const bool v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
+        if (BULK && v_landed) par ^= 2u;
+        if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        sync();
+        // ---- V: this step's contribution to the thread's channel
+        {
+            int hi[1] = {0}, lo[1] = {0};
+            bool ok = v_landed && sm.okV[sub] && (uint32_t)(cur.startV >> 3) < sm.nbV[sub];
+            if (ok) {
+                const uint32_t slot_s = kvc_smem_addr(slotsV + sub * p.slotV_bytes), at = sm.leadV[sub] + (cur.startV >> 3), w_s = kvc_smem_addr(sm.ps);
+                ok = escV ? decode_dot_impl<1, true>(slot_s, at, kvc_smem_addr(tab.lutV), KvcTreeGlobal(p.v.book), w_s, hi, lo)
+                          : decode_dot_impl<1, false>(slot_s, at, kvc_smem_addr(tab.lutV), KvcTreeGlobal(p.v.book), w_s, hi, lo);
+            }
+            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+            const float4 x = *reinterpret_cast<const float4 *>(sm.red[1]), z = *reinterpret_cast<const float4 *>(sm.red[2]);
+            l_run = l_run * alpha + ((x.x + x.y) + (x.z + x.w));
+            acc = fmaf(acc, alpha, fix_value(vst, hi[0], lo[0]) + ((z.x + z.y) + (z.z + z.w)));
+        }
+        sync();                                            // every thread is done with the V slots, weights and sums
+        if (BULK && warp == 0) {                           // the next step's V blocks land during its K phase
+            if (__all_sync(0xffffffffu, v_landed)) stage_V(n_on, n_col, n_step);
+            else if (lane == 0) sm.dead = 1;
+        }
+        cur = nxt;
+    }
+
+    // ---- uncompressed tail, only for callers without a workspace: otherwise the merge kernel adds it
+    if (p.Tr > 0 && !p.partial && (TEAM || it.t_hi == p.n_tiles)) {
+        float *pt = reinterpret_cast<float *>(sm.w);       // p of 128 rows
+        for (long long r0 = TEAM ? wk % p.team * 128 : 0; r0 < p.Tr; r0 += TEAM ? p.team * 128 : 128) {      // a team's workers take the passes in turn
+            const bool act = r0 + tid < p.Tr;
+            sync();
+            float s = -CUDART_INF_F;
+            if (act) {
+                s = 0.f;
+                const __half *kr = p.ktail + (((r0 + tid) * B + b) * Hkv + h) * 128;
+#pragma unroll 1
+                for (int c8 = 0; c8 < 16; c8++) {
+                    const uint4 kv = *reinterpret_cast<const uint4 *>(kr + c8 * 8);
+                    const __half *kh = reinterpret_cast<const __half *>(&kv);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) s = fmaf(__half2float(kh[k]), kvc_scale_value(sm.q[c8 * 8 + k]) * p.scaling, s);
+                }
+            }
+            const float mx = kvc_warp_max(s);
+            if (lane == 0) sm.red[0][warp] = mx;
+            sync();
+            const float4 x = *reinterpret_cast<const float4 *>(sm.red[0]);
+            const float m_new = fmaxf(fmaxf(m_run, fmaxf(x.x, x.y)), fmaxf(x.z, x.w)), alpha = __expf(m_run - m_new);
+            m_run = m_new;
+            const float pr = act ? __expf(s - m_new) : 0.f;
+            pt[tid] = pr;
+            const float ssum = kvc_warp_sum(pr);
+            if (lane == 0) sm.red[1][warp] = ssum;
+            sync();
+            const int n_here = (int)min(128ll, p.Tr - r0);
+            float dv = 0.f;
+            for (int i = 0; i < n_here; i++) dv = fmaf(pt[i], __half2float(p.vtail[(((r0 + i) * B + b) * Hkv + h) * 128 + tid]), dv);
+            const float4 y = *reinterpret_cast<const float4 *>(sm.red[1]);
+            l_run = l_run * alpha + ((y.x + y.y) + (y.z + y.w));
+            acc = fmaf(acc, alpha, dv);
+        }
+    }
+    if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without steps fetched nothing yet
+    bool dead;
+    if constexpr (TEAM) {                                  // each worker's share to its own shared memory, then the sum
+        const int team = p.team, tm = wk / team, tk = wk % team;      // the worker's team and its place there
+        auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" :: "r"(ONE_WORKERS + 1 + tm), "r"(team * 128) : "memory"); };
+        sync();                                            // (the tail's scratch is read)
+        reinterpret_cast<float *>(sm.w)[tid] = acc;
+        if (tid == 0) { sm.red[0][0] = m_run; sm.red[0][1] = l_run; }
+        team_sync();
+        const OneWorker *mates = &sm - tk;
+        if (tk == 0) {
+            float M = -CUDART_INF_F, O = 0.f, L = 0.f;
+            for (int w = 0; w < team; w++) M = fmaxf(M, mates[w].red[0][0]);
+            for (int w = 0; w < team; w++) {
+                const float m = mates[w].red[0][0], e = m == -CUDART_INF_F ? 0.f : __expf(m - M);     // a worker without tokens adds nothing
+                L = fmaf(mates[w].red[0][1], e, L);
+                O = fmaf(reinterpret_cast<const float *>(mates[w].w)[tid], e, O);
+            }
+            p.out[(long long)col * 128 + tid] = __float2half_rn(O / L);
+        }
+        dead = false;
+        if (BULK) for (int w = 0; w < team; w++) dead |= mates[w].dead != 0;      // of any: a team stops together
+        team_sync();
+    } else {
+        if (!p.partial) p.out[(long long)col * 128 + tid] = __float2half_rn(acc / l_run);
+        else {
+            float *dst = p.ws_part + ((long long)col * p.splits + it.part) * ROWS_PART_FLOATS;
+            dst[2 + tid] = acc;
+            if (tid == 0) { dst[0] = m_run; dst[1] = l_run; }
+        }
+        if (draw && tid == 0) sm.next_j = drawn;
+        sync();                                            // the tail's scratch is read before the next column's weights overwrite it
+        dead = BULK && sm.dead != 0;
+    }
+    if (dead) break;                                       // a staging wait ran out: the status word says so, the item's result is void
+    const int j_n2 = draw ? 2 * P + sm.next_j : j_n1 + 1;
+    it = nit; have = have_next; j_n1 = j_n2;
+    have_next = have && item_of(j_n1, nit);
+    }   // items of the worker
+    if (BULK && any) {                    // the copies issued after the last step are empty, but their phase must end;
+        // after a wait that ran out, these are the phases still open: nothing may be in flight at the return
+        if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        if (!kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+    }
+    if (flags) atomicOr(p.status, flags);
+    if (draw && tid == 0) {               // the last worker to finish leaves the scheduling counters zeroed for the next launch
+        __threadfence();
+        if (atomicAdd(&p.sched[1], 1) == P - 1) { p.sched[0] = 0; p.sched[1] = 0; __threadfence(); }
+    }
+}
+
 // The uncompressed tail of a cache (the recent window): dense fp16 rows [Tr, B, Hkv, 128] behind the compressed part.
 struct TailArgs {
     const __half *q, *ktail, *vtail;
@@ -1419,15 +1394,12 @@ __device__ __forceinline__ unsigned short ld_nc_16_pinned(const void *p) {
 // there is no attention kernel in between: the kernel ahead may be the one that stores the newest rows (it lets its
 // dependents start early), so the wait comes first.
 // The loads of the partial results are issued in batches of 16 before any is used as well, by both halves of the CTA in turn:
-// grouped queries leave twice as many as the one-head kernel (2 columns of 32768 tokens, 2 heads each, 256 partial results: 32.5 us
-// for the step with batches of 8 by one half, now 24.5; the one-head kernel with 128: 23.1 and 19.7).
+// (2 columns of 32768 tokens, 2 heads each, 256 partial results: 32.5 us for the step with batches of 8 by one half, now 24.5).
 constexpr int MERGE_THREADS = 256;
-// ROWS: the partial results of the grouped kernel
-template <bool ROWS>
 __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *__restrict__ ws_part, __half *__restrict__ out, int splits, TailArgs t) {
     __shared__ float sm_red[8], sm_sum[8], sm_e[128], sm_o[128];
     __shared__ __align__(16) float sm_q[128];
-    constexpr int PART = ROWS ? ROWS_PART_FLOATS : ATTN_PART_FLOATS;
+    constexpr int PART = ROWS_PART_FLOATS;
     const float *src = ws_part + (size_t)blockIdx.x * splits * PART;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // launched with programmatic stream serialisation: the kernel behind this one in the stream may set up
@@ -1533,13 +1505,13 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
         }
         __syncthreads();
         // channel c of BATCH partial results, all loads in flight together, the CTA's two halves in turn
-        constexpr int BATCH = ROWS ? 16 : 8;
+        constexpr int BATCH = 16;
         for (int i0 = (tid >> 7) * BATCH; i0 < ns; i0 += 2 * BATCH) {
             float a[BATCH];
 #pragma unroll
             for (int k = 0; k < BATCH; k++) {
                 const float *pp = src + (size_t)(s0 + min(i0 + k, ns - 1)) * PART;
-                a[k] = ROWS ? pp[2 + c] : pp[4 + c] + pp[4 + 128 + c];
+                a[k] = pp[2 + c];
             }
 #pragma unroll
             for (int k = 0; k < BATCH; k++) if (i0 + k < ns) O = fmaf(a[k], sm_e[i0 + k], O);
@@ -1662,11 +1634,21 @@ extern "C" int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hk
 static int g_wait_limit = 0, g_starve = 0;
 extern "C" void kvc_attn_debug(int wait_limit, int starve) { g_wait_limit = wait_limit; g_starve = starve; }
 
-// CTAs per SM the attention kernel is launched with at most (its launch bounds ask for this many)
+// What a workspace is sized for: runs of 256-token tiles for this many takers per SM (kvc_attn_splits); the kernels' plans may
+// cut twice as many.
 constexpr int ATTN_CTAS_PER_SM = 3;
 // items a resident CTA should get on average: enough that the draws even out the CTAs' speeds and the
 // last items end close together, few enough that the per-item work (q, partial results) stays small
 constexpr int ATTN_ITEMS_PER_CTA = 4;
+
+template <int G, bool BULK, bool TEAM> auto attn_kernel() {
+    if constexpr (G == 1) return attn_one_kernel<BULK, TEAM>;
+    else return attn_rows_kernel<G, BULK, TEAM>;
+}
+template <int G> size_t attn_smem(const AttnParams &p, int workers) {
+    if constexpr (G == 1) return one_smem(p, workers);
+    else return rows_smem<G>(p, workers);
+}
 
 // How the columns are cut when the caller leaves it to the library: long runs of `tps` tiles, and at the
 // end of every column short runs of half that, enough of them that each resident CTA finds about two
@@ -1769,37 +1751,25 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.starve = g_starve;
     p.slotK_bytes = slot_bytes_of(p.k.max_block);
     p.slotV_bytes = slot_bytes_of(p.v.max_block);
-    const size_t slot_total = 4 * (size_t)(p.slotK_bytes + p.slotV_bytes) + SLOT_PAD;
     // bulk copies widen every block to 16-byte boundaries: both streams must start on one
     const bool bulk = T > 0 && (reinterpret_cast<uintptr_t>(k->encoded) & 15) == 0 && (reinterpret_cast<uintptr_t>(v->encoded) & 15) == 0;
     const int sms = kvc_sm_count();
     const long long Gt = Hq / Hkv;
-    if (Gt == 1 && T > 0) {
-        const size_t smem = slot_total + sizeof(AttnSmem);
-        p.g0 = 0; p.nh = 1;
-        static kvc_launch_slot slots[2];
-        auto *kernel = bulk ? attn_decode_kernel<true> : attn_decode_kernel<false>;
-        int occ = 0;
-        if (int rc = kvc_prepare(slots[bulk], reinterpret_cast<const void *>(kernel), NTHR, smem, &occ)) return rc;
-        KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);
-        long long ctas = (long long)sms * (occ < ATTN_CTAS_PER_SM ? occ : ATTN_CTAS_PER_SM);
-        if (ctas > p.work) ctas = p.work;
-        if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(NTHR), smem, kvc_cu(stream), p)) return rc;
-    } else if (T > 0) {
-        // Grouped queries count in steps of 128 tokens.  The workspace, sized for `splits` partial results of the one-head
-        // kernel, holds twice as many of theirs: with more and smaller workers the items are finer where it may be so.
+    if (T > 0) {
+        // The kernels count in steps of 128 tokens.  The workspace, sized for `splits` runs of 256-token tiles, holds twice as many
+        // of their partial results: with many small workers the items are finer where it may be so.
         p.n_tiles = (int)(T / 128);
         p.tiles_per_split *= 2; p.short_tiles *= 2;
         const int heads = (int)((Gt + (Gt + 7) / 8 - 1) / ((Gt + 7) / 8));                   // of the first launch
         const long long most = (long long)rows_fit(p, heads) * sms;                         // workers of a full device
         if (p.partial && ws_parts) {
             RunPlan r = {0, 0, 0, 0};
-            // (the plan counts five workers per SM also where the launch has fewer: the items are finer for it.  8 heads, four
+            // (with grouped queries the plan counts five workers per SM also where the launch has fewer: the items are finer for it.  8 heads, four
             // workers: 16 x 8 columns of 16384 tokens 412 us, with a plan for four 423; 32 x 2 columns 217 and 224.  Three workers, as the
             // stream's largest block is unknown: 484 and 490 us, but 16 x 8 columns of 4096 tokens 144 and 137.)
-            if (asked <= 0) r = plan_runs(p.n_tiles, cols, (long long)rows_workers<4>() * sms);
+            if (asked <= 0) r = plan_runs(p.n_tiles, cols, heads == 1 ? most : (long long)rows_workers<4>() * sms);
             // The caller's runs in halves where that is fewer steps one after the other: a worker takes a run's steps in turn, each
-            // with half the threads a CTA of the one-head kernel has for its tile.  (32 columns, 2 heads each, 2048 tokens in 4
+            // with 128 threads.  (32 columns, 2 heads each, 2048 tokens in 4
             // runs: 46.9 us, in halves 33.7; 64 columns in 8 runs: 36.0, in halves 42.2, as the halves no longer go in one round.)
             else if ((2 * cols * splits + most - 1) / most < 2 * ((cols * splits + most - 1) / most)) {
                 r.tps = r.short_tiles = tps;
@@ -1817,15 +1787,15 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
 #define KVC_AT(GG)                                                                                              \
     {                                                                                                           \
-        int workers = rows_fit<GG>(p);                                                                          \
+        int workers = rows_fit(p, GG);                                                                          \
         p.team = p.partial ? 0 : rows_team(cols, p.n_tiles + (Tr + 127) / 128, workers, sms);                   \
         if (p.team) { const long long n = (cols + sms - 1) / sms; workers = p.team * (int)std::min<long long>(n, workers / p.team); } \
         /* fewer than fit an SM where the items then spread over more SMs */                                    \
         else if (p.work < (long long)workers * sms) workers = (int)((p.work + sms - 1) / sms);                  \
-        const size_t smem = rows_smem<GG>(p, workers);                                                          \
+        const size_t smem = attn_smem<GG>(p, workers);                                                          \
         static kvc_launch_slot slots[4];                                                                        \
-        auto *kernel = p.team ? (bulk ? attn_rows_kernel<GG, true, true> : attn_rows_kernel<GG, false, true>)   \
-                              : (bulk ? attn_rows_kernel<GG, true, false> : attn_rows_kernel<GG, false, false>); \
+        auto *kernel = p.team ? (bulk ? attn_kernel<GG, true, true>() : attn_kernel<GG, false, true>())         \
+                              : (bulk ? attn_kernel<GG, true, false>() : attn_kernel<GG, false, false>());      \
         int occ = 0;                                                                                            \
         if (int rc = kvc_prepare(slots[2 * (p.team != 0) + bulk], reinterpret_cast<const void *>(kernel), 128 * workers, smem, &occ)) return rc; \
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);             \
@@ -1833,7 +1803,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         if (ctas > sms) ctas = sms;                                                                             \
         if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(128 * workers), smem, kvc_cu(stream), p)) return rc; \
     }
-            if (p.nh > 4) KVC_AT(8) else if (p.nh > 2) KVC_AT(4) else KVC_AT(2)
+            if (p.nh > 4) KVC_AT(8) else if (p.nh > 2) KVC_AT(4) else if (p.nh > 1) KVC_AT(2) else KVC_AT(1)
 #undef KVC_AT
         }
     }
@@ -1843,7 +1813,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             ta.q = p.q; ta.ktail = p.ktail; ta.vtail = p.vtail; ta.Tr = Tr;
             ta.B = (int)B; ta.Hkv = (int)Hkv; ta.Hq = (int)Hq; ta.scaling = scaling;
         }
-        if (int rc = launch_overlapped(Gt > 1 ? attn_merge_kernel<true> : attn_merge_kernel<false>, dim3((unsigned)(B * Hq)), dim3(MERGE_THREADS), 0, kvc_cu(stream),
+        if (int rc = launch_overlapped(attn_merge_kernel, dim3((unsigned)(B * Hq)), dim3(MERGE_THREADS), 0, kvc_cu(stream),
                                        (const float *)p.ws_part, p.out, T > 0 ? splits : 0, ta)) return rc;
     }
     KVC_LAUNCH_OK();
