@@ -446,10 +446,39 @@ __device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const ui
 // Bound by memory: 2 bytes read and 1 written per value, where a rotated and transposed copy of the tensor took 4 more before
 // the quantiser read it (K per channel: twice).
 
+// The CTA's histogram: codes below 32 are counted two at a time, pairs[first + 32 * second], others in ones (three instructions
+// per code one by one, a good half of that for a pair; fewer lanes meet on a counter).
+struct PairBins { unsigned int pairs[1024], ones[256]; };
+__device__ __forceinline__ void bins_clear(PairBins &b, int tid, int nthr) {
+    for (int i = tid; i < 1280; i += nthr) b.pairs[i] = 0;              // both arrays
+    __syncthreads();
+}
+__device__ __forceinline__ void bins_add(PairBins &b, const uint32_t (&u)[4]) {     // two codes per word, 16 bits each
+    if (((u[0] | u[1] | u[2] | u[3]) & 0x00e000e0u) == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) atomicAdd(reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(b.pairs) + __dp4a(u[k], 0x00800004u, 0u)), 1u);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) { atomicAdd(&b.ones[u[k] & 0xffu], 1u); atomicAdd(&b.ones[u[k] >> 16], 1u); }
+    }
+}
+__device__ __forceinline__ void bins_flush(const PairBins &b, unsigned long long *gh, int tid) {      // by the first 256 threads
+    __syncthreads();
+    if (tid >= 256) return;
+    unsigned int c = 0;
+    const int s = tid >> 3, part = tid & 7;                 // eight threads fold a symbol's row and column
+#pragma unroll
+    for (int k = 0; k < 4; k++) c += b.pairs[s + 32 * (part * 4 + k)] + b.pairs[32 * s + part * 4 + k];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (part == 0 && c) atomicAdd(&gh[s], (unsigned long long)c);
+    if (b.ones[tid]) atomicAdd(&gh[tid], (unsigned long long)b.ones[tid]);
+}
+
 // the packed path of quant_eight with what it needs in registers; param(i): value i's unit, for anything else
 template <class P>
 __device__ __forceinline__ uint2 quant_eight_at(const uint4 &v, const float (&rcp)[8], const __half2 (&mi2)[4], bool small_min, P param,
-                                                int *flags, unsigned int *hist) {
+                                                int *flags, PairBins *bins) {
     const __half2 *h2 = reinterpret_cast<const __half2 *>(&v);
     const __half2 big = __float2half2_rn(1536.0f), nbig = __float2half2_rn(-1536.0f), k1024 = __float2half2_rn(1024.0f);
     uint32_t u[4], odd = 0;
@@ -467,28 +496,29 @@ __device__ __forceinline__ uint2 quant_eight_at(const uint4 &v, const float (&rc
 #pragma unroll
         for (int k = 0; k < 4; k++) u[k] = quant_one(h[2 * k], param(2 * k), flags) | (quant_one(h[2 * k + 1], param(2 * k + 1), flags) << 16);
     }
-    if (hist) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) { atomicAdd(&hist[u[k] & 0xffu], 1u); atomicAdd(&hist[u[k] >> 16], 1u); }
-    }
+    if (bins) bins_add(*bins, u);
     return make_uint2(__byte_perm(u[0], u[1], 0x6420), __byte_perm(u[2], u[3], 0x6420));
 }
 
 // ChannelQuant.  CTA = THREADS / 8 * ROWS tokens (one block) of `heads` heads, one after the other; thread = 8 channels of either
 // half of ROWS rows, whose cos and sin it keeps; the next head's rows are fetched while this one's are at work.
+// (Issue bounds it, 29 instructions per value, with 128 registers two CTAs per SM: 1 GiB of keys 0.68 ms, values 0.43 ms by
+// quant_heads_token_kernel; copies and the quantisers of rows took 1.17 and 0.79.  80 registers, three CTAs: 5 % slower.)
 template <int ROWS, int THREADS, bool ROPE>
-__global__ void __launch_bounds__(THREADS) quant_heads_channel_kernel(
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_kernel(
     const __half *__restrict__ x, const __half *__restrict__ cs, const __half *__restrict__ sn, long long cs_bstride,
     uint32_t B, uint32_t H, uint32_t heads, long long Tx, float rel, uint8_t *__restrict__ codes, void *__restrict__ min_int,
     int min_bytes, __half *__restrict__ scale, unsigned long long *__restrict__ ghist, int *__restrict__ status) {
     constexpr int WARPS = THREADS / 32, RT = THREADS / 8;   // RT: rows side by side
     __shared__ __align__(16) __half smn[WARPS][128], smx[WARPS][128];
     __shared__ __align__(16) float psf[128], pmi[128], prcp[128];
-    __shared__ unsigned int shist[WARPS * 256];
+    __shared__ __align__(16) __half phm[128];               // min_int of the units of psmall
+    __shared__ unsigned int psmall[4];                      // a bit per channel: small_min_int
+    __shared__ PairBins bins;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cg = tid & 7, r = tid >> 3;
     const uint32_t groups = (H + heads - 1) / heads, b = blockIdx.x / groups, h0 = (blockIdx.x % groups) * heads, h1 = min(H, h0 + heads);
     const long long j = blockIdx.y, tok0 = j * (RT * ROWS) + r;
-    if (ghist) hist_clear(shist, tid, THREADS);
+    if (ghist) bins_clear(bins, tid, THREADS);
     uint4 ca[ROWS], cb[ROWS], sa[ROWS], sb[ROWS];
     if (ROPE) {
 #pragma unroll
@@ -542,15 +572,18 @@ __global__ void __launch_bounds__(THREADS) quant_heads_channel_kernel(
         *reinterpret_cast<__half2 *>(&smx[warp][at]) = mx[0]; *reinterpret_cast<__half2 *>(&smx[warp][at + 2]) = mx[1];
         __syncthreads();                                    // (also: the head before is done with its units' parameters)
         if (tid < 128) {                                    // thread = channel
-            float a = __half2float(smn[0][tid]), z = __half2float(smx[0][tid]);
+            const int at2 = tid & ~1;
+            __half2 a = *reinterpret_cast<const __half2 *>(&smn[0][at2]), z = *reinterpret_cast<const __half2 *>(&smx[0][at2]);
 #pragma unroll
-            for (int w = 1; w < WARPS; w++) { a = fminf(a, __half2float(smn[w][tid])); z = fmaxf(z, __half2float(smx[w][tid])); }
+            for (int w = 1; w < WARPS; w++) { a = __hmin2(a, *reinterpret_cast<const __half2 *>(&smn[w][at2])); z = __hmax2(z, *reinterpret_cast<const __half2 *>(&smx[w][at2])); }
             __half sc;
-            const UnitParam q = unit_param(a, z, rel, &sc, &flags);
+            const UnitParam q = unit_param(tid & 1 ? __high2float(a) : __low2float(a), tid & 1 ? __high2float(z) : __low2float(z), rel, &sc, &flags);
             const long long u = ((j * B + b) * H + h) * 128 + tid;
             scale[u] = sc;
             store_min(min_int, min_bytes, u, q.mi, &flags);
-            psf[tid] = q.sf; pmi[tid] = q.mi; prcp[tid] = q.rcp;
+            psf[tid] = q.sf; pmi[tid] = q.mi; prcp[tid] = q.rcp; phm[tid] = __float2half_rn(q.mi);
+            const unsigned int small = __ballot_sync(0xffffffffu, small_min_int(q.mi));
+            if (lane == 0) psmall[warp] = small;
         }
         __syncthreads();
 #pragma unroll
@@ -558,25 +591,20 @@ __global__ void __launch_bounds__(THREADS) quant_heads_channel_kernel(
             const int c0 = half * 64 + cg * 8;
             float rcp[8];
             __half2 mi2[4];
-            bool small = true;
+            const bool small = (psmall[c0 >> 5] >> (c0 & 31) & 0xffu) == 0xffu;
 #pragma unroll
             for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4 *>(&rcp[i]) = *reinterpret_cast<const float4 *>(&prcp[c0 + i]);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float2 m = *reinterpret_cast<const float2 *>(&pmi[c0 + 2 * i]);
-                small = small && small_min_int(m.x) && small_min_int(m.y);
-                mi2[i] = __floats2half2_rn(m.x, m.y);
-            }
+            *reinterpret_cast<uint4 *>(mi2) = *reinterpret_cast<const uint4 *>(&phm[c0]);
             auto param = [&](int i) { UnitParam p; p.sf = psf[c0 + i]; p.mi = pmi[c0 + i]; p.rcp = prcp[c0 + i]; return p; };
 #pragma unroll
             for (int k = 0; k < ROWS; k++) {
-                const uint2 o = quant_eight_at(half ? vb[k] : va[k], rcp, mi2, small, param, &flags, ghist ? shist + warp * 256 : nullptr);
+                const uint2 o = quant_eight_at(half ? vb[k] : va[k], rcp, mi2, small, param, &flags, ghist ? &bins : nullptr);
                 *reinterpret_cast<uint2 *>(codes + (((tok0 + RT * k) * B + b) * H + h) * 128 + c0) = o;
             }
         }
     }
     if (flags) atomicOr(status, flags);
-    if (ghist) hist_flush(shist, ghist, tid, THREADS);
+    if (ghist) bins_flush(bins, ghist, tid);
 }
 
 // TokenQuant (a unit: one token of one sequence, all heads) and VectorQuant (one head of it).  CTA = four tokens of one sequence
@@ -587,9 +615,9 @@ __global__ void __launch_bounds__(256) quant_heads_token_kernel(
     void *__restrict__ min_int, int min_bytes, __half *__restrict__ scale, unsigned long long *__restrict__ ghist,
     int *__restrict__ status) {
     __shared__ float red[2][4][4];                          // extremes by head group and token
-    __shared__ unsigned int shist[8 * 256];
-    const int tid = threadIdx.x, warp = tid >> 5, c0 = (tid & 15) * 8, tk = (tid >> 4) & 3, hg = tid >> 6;
-    if (ghist) hist_clear(shist, tid, 256);
+    __shared__ PairBins bins;
+    const int tid = threadIdx.x, c0 = (tid & 15) * 8, tk = (tid >> 4) & 3, hg = tid >> 6;
+    if (ghist) bins_clear(bins, tid, 256);
     int flags = 0;
     const long long n4 = (T + 3) / 4, n_groups = n4 * B;
     for (long long grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
@@ -638,12 +666,14 @@ __global__ void __launch_bounds__(256) quant_heads_token_kernel(
                 p = unit_param(mn, mx, rel, &sc, &flags);
                 if (c0 == 0) { scale[u] = sc; store_min(min_int, min_bytes, u, p.mi, &flags); }
             }
-            const __half2 mi2 = __float2half2_rn(p.mi);
-            *reinterpret_cast<uint2 *>(codes + u * 128 + c0) = quant_eight<0>(v[i], &p, small_min_int(p.mi), &mi2, &flags, ghist ? shist + warp * 256 : nullptr);
+            const __half2 m2 = __float2half2_rn(p.mi);
+            const float rcp[8] = {p.rcp, p.rcp, p.rcp, p.rcp, p.rcp, p.rcp, p.rcp, p.rcp};
+            const __half2 mi2[4] = {m2, m2, m2, m2};
+            *reinterpret_cast<uint2 *>(codes + u * 128 + c0) = quant_eight_at(v[i], rcp, mi2, small_min_int(p.mi), [&](int) { return p; }, &flags, ghist ? &bins : nullptr);
         }
     }
     if (flags) atomicOr(status, flags);
-    if (ghist) hist_flush(shist, ghist, tid, 256);
+    if (ghist) bins_flush(bins, ghist, tid);
 }
 
 // ---- dequantise: fp16((code + min_int) * scale), models/cache/kvcomp_encode.py:146 -------------
