@@ -176,6 +176,13 @@ int kvc_quantize_heads(const void *x, const void *cos_, const void *sin_, int64_
  * launch: k, v device fp16 [B, H, t, D] -> kout, vout device fp16 [t, B, H, D]. */
 int kvc_kv_store(const void *k, const void *v, const void *cos_, const void *sin_, void *kout, void *vout,
                  int64_t B, int64_t H, int64_t t, int64_t D, int64_t cos_batch_stride, kvc_stream_t stream);
+/* The same with the arguments in memory (8-byte words, in this order), for a host language that converts arguments one by one. */
+typedef struct {
+    const void *k, *v, *cos_, *sin_;
+    void *kout, *vout;
+    int64_t B, H, t, D, cos_batch_stride;
+} kvc_kv_store_args;
+int kvc_kv_store_packed(const kvc_kv_store_args *args, kvc_stream_t stream);
 
 /* (codes + min_int) * scale -> fp16 (models/cache/kvcomp_encode.py:146). */
 int kvc_dequant(const uint8_t *codes, const kvc_qmeta *q, int64_t T, int64_t B, int64_t H, int64_t D,
@@ -273,6 +280,19 @@ int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T, int64_t B
                     const void *q, float scaling, const void *ktail, const void *vtail, int64_t Tr,
                     void *out, int splits, void *workspace, int64_t workspace_bytes,
                     int32_t *status, kvc_stream_t stream);
+/* The same with the arguments in memory. */
+typedef struct {
+    kvc_cache k, v;               /* not read while T is 0 */
+    int64_t T, B, Hkv, Hq;
+    const void *q, *ktail, *vtail;
+    int64_t Tr;
+    void *out, *workspace;
+    int64_t workspace_bytes;
+    int32_t *status;
+    float scaling;
+    int32_t splits;
+} kvc_attn_args;
+int kvc_attn_decode_packed(const kvc_attn_args *args, kvc_stream_t stream);
 
 /* Diagnostics, no counterpart in the reference (its kernels have no device-side waits).  The attention
  * kernel waits for its staged blocks at most `wait_limit` tries (0 = the default of 2^22); a wait that

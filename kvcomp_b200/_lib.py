@@ -4,6 +4,7 @@ There is no fallback: if the library is missing or a call fails, an exception is
 """
 import ctypes as C
 import os
+import struct
 
 from . import build as _build
 
@@ -42,6 +43,13 @@ class Cache(C.Structure):
                 ("max_block_bytes", C.c_int32), ("reserved", C.c_int32)]
 
 
+# the same layouts for the calls that a decode step makes (kvc_kv_store_packed, kvc_attn_decode_packed): packing all
+# arguments at once costs a fifth of converting them one by one
+CACHE_FIELDS = "7q2i4q2i"
+KV_STORE_ARGS = struct.Struct("<11q")
+ATTN_ARGS = struct.Struct("<" + 2 * CACHE_FIELDS + "12qfi")
+
+
 class KvcError(RuntimeError):
     pass
 
@@ -66,6 +74,7 @@ _SIGNATURES = {
     "kvc_quantize_heads_fits": (_i32, [_i32, _i32, _i64, _i64, _i64, _i64, _i64]),
     "kvc_quantize_heads": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i32, _i32, _i64, _f32, _vp, _vp, _i32, _vp, _vp, _vp, _vp]),
     "kvc_kv_store": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp]),
+    "kvc_kv_store_packed": (_i32, [C.c_char_p, _vp]),
     "kvc_dequant": (_i32, [_vp, C.POINTER(QMeta), _i64, _i64, _i64, _i64, _vp, _vp]),
     "kvc_histogram": (_i32, [_vp, _i64, _vp, _vp]),
     "kvc_build_codebook": (_i32, [_vp, _vp, _vp]),
@@ -82,6 +91,7 @@ _SIGNATURES = {
     "kvc_attn_splits": (_i32, [_i64, _i64, _i64, _i32]),
     "kvc_attn_decode": (_i32, [C.POINTER(Cache), C.POINTER(Cache), _i64, _i64, _i64, _i64, _vp, _f32, _vp, _vp,
                                _i64, _vp, _i32, _vp, _i64, _vp, _vp]),
+    "kvc_attn_decode_packed": (_i32, [C.c_char_p, _vp]),
     "kvc_attn_debug": (None, [_i32, _i32]),
     "kvc_attn_static_capacity": (_i64, []),
     "kvc_attn_decode_static": (_i32, [C.POINTER(Cache), C.POINTER(Cache), _i64, _i64, _i64, _i64, _vp, _f32, _vp, _vp,

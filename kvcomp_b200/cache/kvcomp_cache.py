@@ -78,9 +78,10 @@ class KVCompCache(_BASE):
             t = key_states.shape[2]
             if value_states.is_cuda and value_states.dtype == torch.float16 and value_states.is_contiguous() \
                     and value_states.shape == key_states.shape:
-                kplace, vplace = kc0.recent_place(t, key_states.device), vc0.recent_place(t, key_states.device)
+                device = key_states.device
+                kplace, vplace = kc0.recent_address(t, device), vc0.recent_address(t, device)
                 if kplace is not None and vplace is not None:   # the usual decode step: one launch, straight into both windows
-                    ops.kv_store(key_states, value_states, cos, sin, kplace, vplace)
+                    ops.kv_store_at(key_states, value_states, cos, sin, kplace, vplace)
                     kc0.recent_commit(t)
                     vc0.recent_commit(t)
                     return
@@ -156,9 +157,14 @@ class KVCompCache(_BASE):
         cfg = KVCompCacheConfigStatic.config
         q = query_states
         squeeze = q.dim() == 4
+        if squeeze and q.shape[2] != 1:
+            raise KvcError("attend handles one query token (decode); use update() for prefill")
+        if (squeeze or q.dim() == 3) and cfg.enable_quant and not cfg.enable_pre_rope and q.dtype is torch.float16 and q.is_cuda \
+                and q.is_contiguous() and q.shape[-1] == 128 and self.k_ctx[layer_idx] is not None:
+            out = self._attend_step(q, self.k_ctx[layer_idx], self.v_ctx[layer_idx], scaling)
+            if out is not None:
+                return out
         if squeeze:
-            if q.shape[2] != 1:
-                raise KvcError("attend handles one query token (decode); use update() for prefill")
             q = q[:, :, 0, :]
         q = q.contiguous().half()
         B, Hq, D = q.shape
@@ -172,15 +178,35 @@ class KVCompCache(_BASE):
         T, ktail, vtail = self._tails(kc, vc)
         if T == 0 and ktail is None:
             raise KvcError("empty cache")
-        parts = ops.attn_splits(T, B, kc.head_num)          # partial results per head of the balanced split
-        key = (q.device, B, Hq, parts)
-        if key not in self._ws:
-            self._ws[key] = ops.attn_workspace(B, Hq, parts, q.device)
-        if q.device not in self._status:
-            self._status[q.device] = ops.new_status(q.device)
+        ws, st = self._scratch(q, T, kc.head_num)
         out, _ = ops.attn_decode(kc._argument() if T else None, vc._argument() if T else None, T, B, kc.head_num, q, scaling,
-                                 ktail, vtail, splits=0, workspace=self._ws[key], status=self._status[q.device])
+                                 ktail, vtail, splits=0, workspace=ws, status=st)
         return out.unsqueeze(2) if squeeze else out
+
+    def _scratch(self, q, T, kv_heads):
+        """Workspace and status word of a launch for q [B, Hq, ...] over T tokens of the streams."""
+        B, Hq, device = q.shape[0], q.shape[1], q.device
+        parts = ops.attn_splits(T, B, kv_heads)             # partial results per head of the balanced split
+        ws = self._ws.get((device, B, Hq, parts))
+        if ws is None:
+            ws = self._ws[(device, B, Hq, parts)] = ops.attn_workspace(B, Hq, parts, device)
+        st = self._status.get(device)
+        if st is None:
+            st = self._status[device] = ops.new_status(device)
+        return ws, st
+
+    def _attend_step(self, q, kc, vc, scaling):
+        """attend() for a query that lies ready for the kernel, over tails that are in place; else None.  No tensor is
+        made but the output, and the launch's arguments are packed at once."""
+        T = min(kc.encoded_ctx_len, vc.encoded_ctx_len) // 128 * 128
+        ktail, vtail = kc.tail_at(T), vc.tail_at(T)
+        if ktail is None or vtail is None or (T == 0 and ktail[1] == 0) or (ktail[1] and not vtail[1]):
+            return None
+        ws, st = self._scratch(q, T, kc.head_num)
+        out = torch.empty(q.shape, dtype=torch.float16, device=q.device)
+        ops.attn_decode_at(kc._fields() if T else None, vc._fields() if T else None, T, q.shape[0], kc.head_num, q, out,
+                           1.0 / math.sqrt(q.shape[-1]) if scaling is None else float(scaling), ktail[0], vtail[0], ktail[1], ws, st)
+        return out
 
     def _attend_dense(self, q, layer_idx, scaling):
         """softmax(q K^T * scaling) V over the materialised cache: plain fp16 caches (enable_quant off) and

@@ -259,6 +259,24 @@ class KVCompCtx:
             return None
         return self._recent.reserve(t, self._room(), (self.batch_size, self.head_num, self.head_dim), torch.float16, device)
 
+    def recent_address(self, t, device):
+        """recent_place() as an address."""
+        if self.device is None:
+            self.device = device
+        r = self._recent
+        if self.device != device or self._cut(r.hi - r.lo, t):
+            return None
+        if r.buf is None or r.hi + t > r.buf.shape[0]:
+            r.reserve(t, self._room(), (self.batch_size, self.head_num, self.head_dim), torch.float16, device)
+        return self._row_address(r.hi)
+
+    def _row_address(self, i):
+        """Address of row i of the window's buffer."""
+        b = self._recent.buf
+        if b.dtype is not torch.float16 or not b.is_contiguous() or not b.is_cuda:
+            ops._cuda(b, torch.float16, "buffer")
+        return b.data_ptr() + i * (2 * self.batch_size * self.head_num * self.head_dim)
+
     def recent_commit(self, t):
         self._recent.commit(t)
         self.ctx_len += t
@@ -484,20 +502,16 @@ class KVCompCtx:
     def get_decode_quant_ints(self):
         """Decoded uint8 codes [n_blocks, block, B, H, D] and the kernel time in ms."""
         self._require()
-        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        start.record()
+        call = ops.TimedCall.on(self.device).begin()
         out = None
         if self.encoded_ctx_len:
-            out, st = ops.decode(self._enc.used(), self._bi.used(), self._ti.used(), self.book,
-                                 self.encoded_ctx_len, self.batch_size, self.head_num, self.is_k,
-                                 max_block=self.max_block_bytes)
-        stop.record()
-        stop.synchronize()
-        if out is not None:
-            ops.read_status(st, what="entropy_decode")
+            out, _ = ops.decode(self._enc.used(), self._bi.used(), self._ti.used(), self.book,
+                                self.encoded_ctx_len, self.batch_size, self.head_num, self.is_k,
+                                status=call.status, max_block=self.max_block_bytes)
+        ms = call.end("entropy_decode")
         if self._pending is not None:
             out = self._pending if out is None else torch.cat([out, self._pending], dim=0)
-        return out.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim), start.elapsed_time(stop)
+        return out.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim), ms
 
     def _values(self, rows):
         """An fp16 tensor of `rows` tokens whose first compressed_ctx_len are the dequantised values, decoded and
@@ -505,18 +519,14 @@ class KVCompCtx:
         time in ms."""
         self._require()
         n, shape = self.encoded_ctx_len, (self.batch_size, self.head_num, self.head_dim)
-        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        start.record()
+        call = ops.TimedCall.on(self.device).begin()
         x = torch.empty((rows,) + shape, dtype=torch.float16, device=self.device)
-        st = ops.decode_values(self._argument(), n, *shape[:2], self.is_k, x[:n]) if n else None
+        if n:
+            ops.decode_values(self._argument(), n, *shape[:2], self.is_k, x[:n], status=call.status)
         if self._pending is not None:
             first = n // self.spec.tok_div * self.spec.sj                    # unit of the first waiting token
             ops.dequant(self._pending, self._mi.used()[first:], self._sc.used()[first:], self.spec, out=x[n:self.compressed_ctx_len])
-        stop.record()
-        if st is not None:
-            ops.read_status(st, what="entropy_decode")         # waits for the stream: one wait for both
-        stop.synchronize()
-        return x, start.elapsed_time(stop)
+        return x, call.end("entropy_decode")
 
     def get_only_compressed(self):
         """Dequantised compressed part [T, B, H, D] and the time of decode + dequantisation in ms."""
@@ -553,6 +563,13 @@ class KVCompCtx:
         self._cache_q.min_int, self._cache_q.scale = self._mi.buf.data_ptr(), self._sc.buf.data_ptr()
         return c
 
+    def _fields(self):
+        """cache()'s contents in the order of the structure, for a launch made right away."""
+        assert self.encoded_ctx_len > 0 and self.book is not None, "nothing has been encoded yet"
+        s, e, mi = self.spec, self._enc, self._mi.buf
+        return (e.buf.data_ptr(), e.n, self._bi.buf.data_ptr(), self._ti.buf.data_ptr(), self.book.blob.data_ptr(), mi.data_ptr(),
+                self._sc.buf.data_ptr(), mi.element_size(), s.tok_div, s.sj, s.sb, s.sh, s.sc, self.max_block_bytes, 0)
+
     def mat_vec_mul(self, B):
         """K: scores [batch, heads, ctx] = q . K^T; V: [1, batch, heads, 128] = P . V over the compressed
         tokens (kvcomp_encode.py:209-280).  Returns (tensor, ms)."""
@@ -565,20 +582,17 @@ class KVCompCtx:
         assert B.shape[0] == self.batch_size, "batch size mismatch"
         hq = B.shape[1]
         assert hq % self.head_num == 0, "head num mismatch"
-        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        call = ops.TimedCall.on(self.device)
         if self.is_k:
             assert B.shape[2] == self.head_dim, "head dim mismatch"
-            start.record()
-            C, st = ops.fused_qk(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
+            call.begin()
+            C, _ = ops.fused_qk(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
         else:
             assert B.shape[2] == self.compressed_ctx_len, "ctx len mismatch"
-            start.record()
-            part, st = ops.fused_pv(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B)
+            call.begin()
+            part, _ = ops.fused_pv(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
             C = part.sum(dim=0, keepdim=True, dtype=torch.float32).half()
-        stop.record()
-        ops.read_status(st, what="mat_vec_mul")
-        stop.synchronize()
-        return C, start.elapsed_time(stop)
+        return C, call.end("mat_vec_mul")
 
     def save(self, path):
         """Write this cache to a file (kvcomp_b200.cache.storage describes the format)."""
@@ -614,6 +628,18 @@ class KVCompCtx:
                 return kept if not len(self._recent) else torch.cat([kept, self._recent.view()], dim=0)
             self._recent.rebuild(kept, self._recent.view(), self._room())
         return self._recent.rows_from_kept(need)
+
+    def tail_at(self, T):
+        """tail_from(T) as (address, rows); None when the rows have to be made first."""
+        r = self._recent
+        need = max(0, self.compressed_ctx_len - T)
+        if need > r.lo - r.q:
+            return None
+        r.q = r.lo - need
+        if r.q == r.hi:
+            r.q = r.lo = r.hi = 0
+            return 0, 0
+        return self._row_address(r.q), r.hi - r.q
 
     def trim_dequantised(self, T):
         self._recent.rows_from_kept(min(self._recent.kept, max(0, self.compressed_ctx_len - T)))

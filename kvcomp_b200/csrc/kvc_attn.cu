@@ -26,6 +26,7 @@
 // the dot product are fp32.  With several query heads per KV head they share every decode: in the unfused
 // kernels by weight records [position][G], up to four heads a launch, in the attention kernel see attn_rows_kernel.
 #include <math_constants.h>
+#include <string.h>
 
 #include <algorithm>
 #include <type_traits>
@@ -1818,6 +1819,14 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     }
     KVC_LAUNCH_OK();
     return KVC_OK;
+}
+
+extern "C" int kvc_attn_decode_packed(const kvc_attn_args *args, kvc_stream_t stream) {
+    KVC_REQUIRE(args, "kvc_attn_decode_packed: null pointer");
+    kvc_attn_args a;
+    memcpy(&a, args, sizeof(a));                            // (wherever the caller packed them)
+    return kvc_attn_decode(a.T > 0 ? &a.k : nullptr, a.T > 0 ? &a.v : nullptr, a.T, a.B, a.Hkv, a.Hq, a.q, a.scaling, a.ktail, a.vtail,
+                           a.Tr, a.out, a.splits, a.workspace, a.workspace_bytes, a.status, stream);
 }
 
 // ---- decode attention for callers that cannot allocate device memory ------------------------------

@@ -4,6 +4,8 @@
 // elementwise op widens to fp32, computes, and rounds to nearest-even back to fp16; the
 // Python scalar `rel` stays fp32.  Explicit round-to-nearest intrinsics are used so that no
 // contraction or fast-math rewrite can change a bit.
+#include <string.h>
+
 #include <algorithm>
 
 #include "kvc_common.cuh"
@@ -1068,6 +1070,13 @@ extern "C" int kvc_kv_store(const void *k, const void *v, const void *cos_, cons
         reinterpret_cast<const __half *>(v), reinterpret_cast<__half *>(vout));
     KVC_LAUNCH_OK();
     return KVC_OK;
+}
+
+extern "C" int kvc_kv_store_packed(const kvc_kv_store_args *args, kvc_stream_t stream) {
+    KVC_REQUIRE(args, "kvc_kv_store_packed: null pointer");
+    kvc_kv_store_args a;
+    memcpy(&a, args, sizeof(a));                                // (wherever the caller packed them)
+    return kvc_kv_store(a.k, a.v, a.cos_, a.sin_, a.kout, a.vout, a.B, a.H, a.t, a.D, a.cos_batch_stride, stream);
 }
 
 // ---- the quantiser in two calls: extremes first, codes later --------------------------------------

@@ -37,17 +37,14 @@ def _five_d(t, name):
     return t
 
 
-def _timed(fn, status=None, what=None):
-    """Run fn() between two CUDA events on the current stream; returns elapsed ms (the reference
-    returns cudaEventElapsedTime, kernels.cu:1026-1048).  status: fn's status word, read (and checked) with the same wait."""
-    start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    start.record()
-    fn()
-    stop.record()
-    if status is not None:
-        ops.read_status(status, what=what)
-    stop.synchronize()
-    return start.elapsed_time(stop)
+def _timed(fn, device, what):
+    """Run fn(status word) between two CUDA events on the current stream; returns elapsed ms (the reference
+    returns cudaEventElapsedTime, kernels.cu:1026-1048).  The status is checked with the same wait."""
+    if device.type != "cuda":
+        raise KvcError("%s: the tensors must be CUDA tensors (kvcomp_b200 has no CPU path)" % what)
+    call = ops.TimedCall.on(device).begin()
+    fn(call.status)
+    return call.end(what)
 
 
 def calculate_buffer_size(input, is_k, head_num, head_dim):
@@ -116,11 +113,9 @@ def _decode(is_k, in_tensor, block_infos, thread_infos, decode_code_book, out, h
     _five_d(out, "out")
     tokens = out.shape[0] * out.shape[1]
     book = ops.book_from_tree(decode_code_book)
-    status = ops.new_status(out.device)
     codes = out.view(tokens, out.shape[2], out.shape[3], out.shape[4])
-    ms = _timed(lambda: ops.decode(in_tensor, block_infos, thread_infos, book, tokens, out.shape[2], out.shape[3],
-                                   is_k, out=codes, status=status), status, "entropy_decode")
-    return ms
+    return _timed(lambda status: ops.decode(in_tensor, block_infos, thread_infos, book, tokens, out.shape[2], out.shape[3],
+                                            is_k, out=codes, status=status), out.device, "entropy_decode")
 
 
 def k_entropy_decode_cuda_export(in_tensor, block_infos, thread_infos, decode_code_book, out, head_num, head_dim):
@@ -157,9 +152,7 @@ def k_decode_and_mat_vec_mul_cuda_export(decode_code_book, block_infos, thread_i
     sc = quant_scales.contiguous().view(-1)
     spec = _ref_spec(True, mi.numel(), ctx, batch, head_num)
     cache = ops.make_cache(encoded_data, block_infos, thread_infos, book, mi, sc, spec)
-    status = ops.new_status(C.device)
-    ms = _timed(lambda: ops.fused_qk(cache, ctx, batch, head_num, B, out=C, status=status), status, "k_decode_and_mat_vec_mul")
-    return ms
+    return _timed(lambda status: ops.fused_qk(cache, ctx, batch, head_num, B, out=C, status=status), C.device, "k_decode_and_mat_vec_mul")
 
 
 def v_decode_and_mat_vec_mul_cuda_export(decode_code_book, block_infos, thread_infos, encoded_data, quant_min_ints,
@@ -175,9 +168,7 @@ def v_decode_and_mat_vec_mul_cuda_export(decode_code_book, block_infos, thread_i
     sc = quant_scales.contiguous().view(-1)
     spec = _ref_spec(False, mi.numel(), ctx, batch, head_num)
     cache = ops.make_cache(encoded_data, block_infos, thread_infos, book, mi, sc, spec)
-    status = ops.new_status(C.device)
-    ms = _timed(lambda: ops.fused_pv(cache, ctx, batch, head_num, B, out=C, status=status), status, "v_decode_and_mat_vec_mul")
-    return ms
+    return _timed(lambda status: ops.fused_pv(cache, ctx, batch, head_num, B, out=C, status=status), C.device, "v_decode_and_mat_vec_mul")
 
 
 def k_mat_vec_mul_cuda_export(k, q, out):
@@ -190,4 +181,4 @@ def k_mat_vec_mul_cuda_export(k, q, out):
         raise KvcError("Head num / head dim of A and B must be equal")
     if out.shape[0] != k.shape[0] or out.shape[2] != k.shape[2]:
         raise KvcError("Context length / head num of A and C must be equal")
-    return _timed(lambda: ops.k_matvec(k, q, out))
+    return _timed(lambda status: ops.k_matvec(k, q, out), out.device, "k_mat_vec_mul")

@@ -4,6 +4,7 @@ PyTorch is only the carrier of device memory and streams here; every computation
 libkvcomp_b200.so.  Every function raises when the tensors are not CUDA tensors: there is no CPU path.
 """
 import ctypes as C
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -21,6 +22,7 @@ MODES = {"BlockQuant": MODE_BLOCK, "ChannelQuant": MODE_CHANNEL, "TokenQuant": M
 # some ten microseconds per call, as much as the rest of a call's host work.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _get_device = getattr(torch._C, "_cuda_getDevice", None)
+_current_stream = getattr(torch._C, "_cuda_getCurrentStream", None)
 
 
 def _stream():
@@ -77,6 +79,56 @@ def check_flags(v, raise_on_fatal=True, what="kvcomp_b200"):
     if raise_on_fatal and (v & _lib.FATAL_FLAGS):
         raise KvcError("%s: device reported %s" % (what, "|".join(_lib.flag_names(v))))
     return v
+
+
+class TimedCall:
+    """What a call that returns only after the device has finished, with its time and its status, needs: two events, a status
+    word and its place in pinned memory.  One per thread and device, kept; the status word is zero between calls.
+    (Events, a zeroed word and a pageable read-back made anew cost such a call some 20 us.)"""
+    __slots__ = ("start", "stop", "status", "host", "flags", "raw", "stream")
+    _kept = threading.local()
+
+    def __init__(self, device):
+        self.start, self.stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        self.status = new_status(device)
+        self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        self.flags = self.host.numpy()
+        self.raw = self.stream = None
+        torch.cuda.synchronize(device)                     # zero, whichever stream uses it first
+
+    @staticmethod
+    def on(device):
+        kept = TimedCall._kept.__dict__
+        c = kept.get(device)
+        if c is None:
+            c = kept[device] = TimedCall(device)
+        return c
+
+    def _current(self):
+        """The device's current stream; the object is made anew only when the stream is another one."""
+        if _current_stream is None:
+            return torch.cuda.current_stream(self.status.device)
+        raw = _current_stream(self.status.device.index)
+        if raw != self.raw:
+            self.raw, self.stream = raw, torch.cuda.Stream(stream_id=raw[0], device_index=raw[1], device_type=raw[2])
+        return self.stream
+
+    def begin(self):
+        self.start.record(self._current())
+        return self
+
+    def end(self, what):
+        """Waits; the time since begin() in ms.  Raises on a fatal status."""
+        stream = self._current()
+        self.stop.record(stream)
+        self.host.copy_(self.status, non_blocking=True)
+        stream.synchronize()
+        v = int(self.flags[0])
+        if v:
+            self.status.zero_()
+            stream.synchronize()
+            check_flags(v, what=what)
+        return self.start.elapsed_time(self.stop)
 
 
 class Report:
@@ -275,6 +327,15 @@ def kv_store(k, v, cos, sin, kout, vout):
     _cuda(vout, torch.float16, "vout")
     with _on(k.device):
         _lib.check(lib.kvc_kv_store(_p(k), _p(v), _p(cos), _p(sin), _p(kout), _p(vout), B, H, t, D, stride, _stream()), "kvc_kv_store")
+
+
+def kv_store_at(k, v, cos, sin, kaddr, vaddr):
+    """kv_store of k and v (CUDA fp16 tensors of one shape, contiguous) to addresses with room for their rows."""
+    B, H, t, D = k.shape
+    cos, sin, stride = _rotation(k, cos, sin)
+    args = _lib.KV_STORE_ARGS.pack(k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), kaddr, vaddr, B, H, t, D, stride)
+    with _on(k.device):
+        _lib.check(_lib.load().kvc_kv_store_packed(args, _stream()), "kvc_kv_store")
 
 
 def dequant(codes, min_int, scale, spec, out=None):
@@ -489,6 +550,19 @@ def attn_decode(kcache, vcache, T, B, Hkv, q, scaling, ktail=None, vtail=None, o
                                        _p(workspace if workspace.numel() else None), workspace.numel(),
                                        _p(status), _stream()), "kvc_attn_decode")
     return out, status
+
+
+_NO_CACHE = (0,) * 15
+
+
+def attn_decode_at(kfields, vfields, T, B, Hkv, q, out, scaling, ktail, vtail, Tr, workspace, status):
+    """attn_decode with splits = 0 for a caller that makes the call at every step: q and out CUDA fp16 tensors
+    [B, Hq, 128] (or [B, Hq, 1, 128]), contiguous; the caches as KVCompCtx._fields() (None while T is 0), the tails as
+    addresses."""
+    args = _lib.ATTN_ARGS.pack(*(kfields or _NO_CACHE), *(vfields or _NO_CACHE), T, B, Hkv, q.shape[1], q.data_ptr(), ktail, vtail, Tr,
+                               out.data_ptr(), workspace.data_ptr(), workspace.numel(), status.data_ptr(), scaling, 0)
+    with _on(q.device):
+        _lib.check(_lib.load().kvc_attn_decode_packed(args, _stream()), "kvc_attn_decode")
 
 
 def encode_debug(wait_limit=0, starve=False):
