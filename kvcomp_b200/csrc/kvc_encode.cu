@@ -10,7 +10,7 @@
 //   copy    the image goes out as 128-bit stores, shifted to the destination's alignment on the way
 // Books whose symbols are all below 32 (error bounds of 0.05 and more) keep the code table in registers
 // and look symbols up with warp shuffles.
-#include "kvc_common.cuh"
+#include "kvc_decode.cuh"
 
 namespace {
 
@@ -119,31 +119,31 @@ __device__ __forceinline__ void encode_vector(const uint32_t (&row)[32], const u
 }
 
 // encode_vector<true> for a book whose symbols are all below 32: the table lives in the warp's registers, lane i
-// holding (code << 8) | length of symbol i, and a lookup is a shuffle (one pass of the shared-memory pipe, no
-// bank conflicts) instead of a 64-bit shared load at a data-dependent address.  Every lane of the warp must
+// holding symbol i's code, first bit on top, with its length in the low byte, and a lookup is a shuffle (one pass of the
+// shared-memory pipe, no bank conflicts) instead of a 64-bit shared load at a data-dependent address.  Every lane of the warp must
 // call this, with symbols below 32 only (the shuffle reads lane `symbol mod 32`).
+// `cur` holds the bits of the word at work, `have` how many (only the low five bits count; bit 5 changes when a word is full): a pair
+// of codes is at most 32 bits, so it fills one word at most.
 __device__ __forceinline__ void encode_vector_shfl(const uint32_t (&row)[32], uint32_t entry, uint32_t *out, uint32_t start) {
-    uint32_t wp = start >> 2, have = (start & 3u) * 8;
-    unsigned long long acc = 0;
-    auto flush = [&]() {
-        have -= 32u;
-        atomicOr(&out[wp], (uint32_t)(acc >> have));
-        wp++;
+    uint32_t at = kvc_smem_addr(out) + (start & ~3u), have = (start & 3u) * 8, cur = 0;
+    auto put = [&](uint32_t e0, uint32_t e1) {
+        const uint32_t c = (e0 & 0xffffff00u) + __funnelshift_r(e1 & 0xffffff00u, 0u, e0);
+        cur += __funnelshift_r(c, 0u, have);
+        const uint32_t rest = __funnelshift_r(0u, c, have), next = (uint32_t)kvc_dp4a_uu(e1, 1u, kvc_dp4a_uu(e0, 1u, (int)have));
+        const uint32_t full = (next ^ have) & 32u;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p red.shared.or.b32 [%1], %2;\n\t}" :: "r"(full), "r"(at), "r"(cur) : "memory");
+        at += full >> 3; cur = full ? rest : cur;
+        have = next;
     };
 #pragma unroll
     for (int w = 0; w < 32; w++) {
         const uint32_t x = row[w];
         const uint32_t e0 = __shfl_sync(0xffffffffu, entry, x), e1 = __shfl_sync(0xffffffffu, entry, x >> 8);
         const uint32_t e2 = __shfl_sync(0xffffffffu, entry, x >> 16), e3 = __shfl_sync(0xffffffffu, entry, x >> 24);
-        const uint32_t l1 = e1 & 0xffu, l3 = e3 & 0xffu;
-        const uint32_t la = (e0 & 0xffu) + l1, lb = (e2 & 0xffu) + l3;
-        const uint32_t pa = ((e0 >> 8) << l1) | (e1 >> 8), pb = ((e2 >> 8) << l3) | (e3 >> 8);
-        acc = (acc << la) | pa; have += la;
-        if (have >= 32u) flush();
-        acc = (acc << lb) | pb; have += lb;
-        if (have >= 32u) flush();
+        put(e0, e1);
+        put(e2, e3);
     }
-    if (have) atomicOr(&out[wp], (uint32_t)(acc << (32u - have)));
+    if (have & 31u) asm volatile("red.shared.or.b32 [%0], %1;" :: "r"(at), "r"(cur) : "memory");
 }
 
 // ---- single pass ------------------------------------------------------------------------------
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(ENC_THREADS, 16) encode_onepass_kernel(
     const bool long_codes = (kind & 1) != 0;
     const bool small_book = kind == 0;                      // the table fits a warp's registers
     const long long blk = s_blk;
-    // lane i: symbol i's (code << 8) | length for the encoding, and its length (or the marker) for the sizes
-    const uint32_t my_entry = (tab[lane].x << 8) | tab[lane].y, my_len = lens[lane];
+    // lane i: symbol i's code, first bit on top, and length for the encoding, and its length (or the marker) for the sizes
+    const uint32_t my_entry = small_book && tab[lane].y ? (tab[lane].x << (32 - tab[lane].y)) | tab[lane].y : 0u, my_len = lens[lane];
     stage_tile(tile, codes, blk, cols, is_k, tid);
     __syncthreads();
     int flags = 0;
