@@ -180,7 +180,8 @@ __device__ __forceinline__ bool kvc_decode_vector(uint32_t slot_s, uint32_t byte
             refill(s2);
         };
         // A round emits six symbols at most: the first 21 need no test of the end.  (Attention, 16 x 32768 tokens, 8 x 4 heads: every
-        // round tested 670 us, the 21 in threes 656, in sevens 652; one head, 8 x 4096 tokens: 140, 138, 135.)
+        // round tested 670 us, the 21 in threes 656, in sevens 652, all of them 671; one head, 8 x 4096 tokens,
+        // without the last: 140, 138, 135.)
 #pragma unroll 7
         for (int i = 0; i < (KVC_VEC_LEN - 1) / 6; i++) round();
         do round(); while (state < end);

@@ -1032,7 +1032,8 @@ extern "C" int kvc_quantize_heads(const void *x, const void *cos_, const void *s
         // heads per CTA: four share the reading of cos and sin, fewer where the device would not be full twice over
         long long heads = 4;
         while (heads > 1 && (T / block) * B * ((H + heads - 1) / heads) < 4 * sms) heads /= 2;
-        // (two rows per thread: with one and twice the threads, 1 GiB of keys in 1.0 ms instead of 0.55)
+        // (two rows per thread: with one and twice the threads, a prompt of 32 x 4096 tokens, 1 GiB each of keys and
+        // values, takes 2.94 ms instead of 2.48)
         auto *kernel = block == 64 ? (ch ? quant_heads_channel_kernel<2, 256, true> : quant_heads_channel_kernel<2, 256, false>)
                                    : (ch ? quant_heads_channel_kernel<2, 512, true> : quant_heads_channel_kernel<2, 512, false>);
         kernel<<<dim3((unsigned)(B * ((H + heads - 1) / heads)), (unsigned)(T / block)), block == 64 ? 256 : 512, 0, s>>>(
