@@ -81,6 +81,10 @@ class KVCompCache(_BASE):
                 device = key_states.device
                 kplace, vplace = kc0.recent_address(t, device), vc0.recent_address(t, device)
                 if kplace is not None and vplace is not None:   # the usual decode step: one launch, straight into both windows
+                    if value_states.device != device:
+                        raise KvcError("keys on %s, values on %s" % (device, value_states.device))
+                    kc0.check_new(key_states.shape)
+                    vc0.check_new(key_states.shape)
                     ops.kv_store_at(key_states, value_states, cos, sin, kplace, vplace)
                     kc0.recent_commit(t)
                     vc0.recent_commit(t)

@@ -133,6 +133,7 @@ class _RecentRows:
 
 class KVCompCtx:
     _cache_arg = _cache_q = None             # (of a copy)
+    _given = False                           # a caller has set the window
 
     def __getstate__(self):                  # the argument structure holds addresses: a copy makes its own
         state = self.__dict__.copy()
@@ -200,6 +201,7 @@ class KVCompCtx:
     @buffer.setter
     def buffer(self, rows):
         self._recent.set(rows)
+        self._given = True                                   # the window may have any shape now
 
     @property
     def encoded_data(self):
@@ -260,7 +262,7 @@ class KVCompCtx:
         return self._recent.reserve(t, self._room(), (self.batch_size, self.head_num, self.head_dim), torch.float16, device)
 
     def recent_address(self, t, device):
-        """recent_place() as an address."""
+        """recent_place() as an address, for a caller that has check_new() look at the tokens before it writes them there."""
         if self.device is None:
             self.device = device
         r = self._recent
@@ -276,6 +278,14 @@ class KVCompCtx:
         if b.dtype is not torch.float16 or not b.is_contiguous() or not b.is_cuda:
             ops._cuda(b, torch.float16, "buffer")
         return b.data_ptr() + i * (2 * self.batch_size * self.head_num * self.head_dim)
+
+    def check_new(self, shape):
+        """Raise unless new tokens of this shape [B, H, t, D] are rows of the window: their places are sized by it."""
+        B, H, _, D = shape
+        if B != self.batch_size or H != self.head_num or D != self.head_dim or \
+                (self._given and self._recent.buf.shape[1:] != (B, H, D)):
+            raise KvcError("new tokens %s for a cache of %d sequences, %d heads, dimension %d and a window %s" % (
+                tuple(shape), self.batch_size, self.head_num, self.head_dim, tuple(self._recent.buf.shape)))
 
     def recent_commit(self, t):
         self._recent.commit(t)
