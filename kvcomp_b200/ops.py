@@ -90,8 +90,9 @@ class TimedCall:
 
     def __init__(self, device):
         self.start, self.stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        self.status = new_status(device)
-        self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        with torch.inference_mode(False):                  # normal tensors, whatever mode the thread's first call runs in:
+            self.status = new_status(device)               # they are written again in calls of either mode
+            self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
         self.flags = self.host.numpy()
         self.raw = self.stream = None
         torch.cuda.synchronize(device)                     # zero, whichever stream uses it first
