@@ -512,13 +512,13 @@ class KVCompCtx:
     def get_decode_quant_ints(self):
         """Decoded uint8 codes [n_blocks, block, B, H, D] and the kernel time in ms."""
         self._require()
-        call = ops.TimedCall.on(self.device).begin()
         out = None
-        if self.encoded_ctx_len:
-            out, _ = ops.decode(self._enc.used(), self._bi.used(), self._ti.used(), self.book,
-                                self.encoded_ctx_len, self.batch_size, self.head_num, self.is_k,
-                                status=call.status, max_block=self.max_block_bytes)
-        ms = call.end("entropy_decode")
+        with ops.TimedCall.on(self.device) as call:
+            if self.encoded_ctx_len:
+                out, _ = ops.decode(self._enc.used(), self._bi.used(), self._ti.used(), self.book,
+                                    self.encoded_ctx_len, self.batch_size, self.head_num, self.is_k,
+                                    status=call.status, max_block=self.max_block_bytes)
+            ms = call.end("entropy_decode")
         if self._pending is not None:
             out = self._pending if out is None else torch.cat([out, self._pending], dim=0)
         return out.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim), ms
@@ -529,14 +529,14 @@ class KVCompCtx:
         time in ms."""
         self._require()
         n, shape = self.encoded_ctx_len, (self.batch_size, self.head_num, self.head_dim)
-        call = ops.TimedCall.on(self.device).begin()
-        x = torch.empty((rows,) + shape, dtype=torch.float16, device=self.device)
-        if n:
-            ops.decode_values(self._argument(), n, *shape[:2], self.is_k, x[:n], status=call.status)
-        if self._pending is not None:
-            first = n // self.spec.tok_div * self.spec.sj                    # unit of the first waiting token
-            ops.dequant(self._pending, self._mi.used()[first:], self._sc.used()[first:], self.spec, out=x[n:self.compressed_ctx_len])
-        return x, call.end("entropy_decode")
+        with ops.TimedCall.on(self.device) as call:
+            x = torch.empty((rows,) + shape, dtype=torch.float16, device=self.device)
+            if n:
+                ops.decode_values(self._argument(), n, *shape[:2], self.is_k, x[:n], status=call.status)
+            if self._pending is not None:
+                first = n // self.spec.tok_div * self.spec.sj                # unit of the first waiting token
+                ops.dequant(self._pending, self._mi.used()[first:], self._sc.used()[first:], self.spec, out=x[n:self.compressed_ctx_len])
+            return x, call.end("entropy_decode")
 
     def get_only_compressed(self):
         """Dequantised compressed part [T, B, H, D] and the time of decode + dequantisation in ms."""
@@ -592,17 +592,17 @@ class KVCompCtx:
         assert B.shape[0] == self.batch_size, "batch size mismatch"
         hq = B.shape[1]
         assert hq % self.head_num == 0, "head num mismatch"
-        call = ops.TimedCall.on(self.device)
         if self.is_k:
             assert B.shape[2] == self.head_dim, "head dim mismatch"
-            call.begin()
-            C, _ = ops.fused_qk(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
         else:
             assert B.shape[2] == self.compressed_ctx_len, "ctx len mismatch"
-            call.begin()
-            part, _ = ops.fused_pv(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
-            C = part.sum(dim=0, keepdim=True, dtype=torch.float32).half()
-        return C, call.end("mat_vec_mul")
+        with ops.TimedCall.on(self.device) as call:
+            if self.is_k:
+                C, _ = ops.fused_qk(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
+            else:
+                part, _ = ops.fused_pv(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
+                C = part.sum(dim=0, keepdim=True, dtype=torch.float32).half()
+            return C, call.end("mat_vec_mul")
 
     def save(self, path):
         """Write this cache to a file (kvcomp_b200.cache.storage describes the format)."""

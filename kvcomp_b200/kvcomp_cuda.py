@@ -42,9 +42,9 @@ def _timed(fn, device, what):
     returns cudaEventElapsedTime, kernels.cu:1026-1048).  The status is checked with the same wait."""
     if device.type != "cuda":
         raise KvcError("%s: the tensors must be CUDA tensors (kvcomp_b200 has no CPU path)" % what)
-    call = ops.TimedCall.on(device).begin()
-    fn(call.status)
-    return call.end(what)
+    with ops.TimedCall.on(device) as call:
+        fn(call.status)
+        return call.end(what)
 
 
 def calculate_buffer_size(input, is_k, head_num, head_dim):

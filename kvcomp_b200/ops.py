@@ -84,8 +84,10 @@ def check_flags(v, raise_on_fatal=True, what="kvcomp_b200"):
 class TimedCall:
     """What a call that returns only after the device has finished, with its time and its status, needs: two events, a status
     word and its place in pinned memory.  One per thread and device, kept; the status word is zero between calls.
+    `with TimedCall.on(device) as call:` begins; the launches and end() belong in the block, so that a call which an exception
+    ends is waited for and its flags go with it.
     (Events, a zeroed word and a pageable read-back made anew cost such a call some 20 us.)"""
-    __slots__ = ("start", "stop", "status", "host", "flags", "raw", "stream")
+    __slots__ = ("start", "stop", "status", "host", "flags", "raw", "stream", "open")
     _kept = threading.local()
 
     def __init__(self, device):
@@ -95,6 +97,7 @@ class TimedCall:
             self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
         self.flags = self.host.numpy()
         self.raw = self.stream = None
+        self.open = False                                  # launches may be under way that write the status word
         torch.cuda.synchronize(device)                     # zero, whichever stream uses it first
 
     @staticmethod
@@ -108,27 +111,41 @@ class TimedCall:
     def _current(self):
         """The device's current stream; the object is made anew only when the stream is another one."""
         if _current_stream is None:
-            return torch.cuda.current_stream(self.status.device)
+            self.stream = torch.cuda.current_stream(self.status.device)
+            return self.stream
         raw = _current_stream(self.status.device.index)
         if raw != self.raw:
             self.raw, self.stream = raw, torch.cuda.Stream(stream_id=raw[0], device_index=raw[1], device_type=raw[2])
         return self.stream
 
-    def begin(self):
+    def __enter__(self):
         self.start.record(self._current())
+        self.open = True
         return self
 
+    def __exit__(self, *exc):
+        if self.open:
+            self._clear()
+        return False
+
+    def _clear(self):
+        """Zero the word behind everything the call has launched."""
+        with torch.cuda.stream(self.stream):
+            self.status.zero_()
+        self.stream.synchronize()
+        self.open = False
+
     def end(self, what):
-        """Waits; the time since begin() in ms.  Raises on a fatal status."""
+        """Waits; the time since the call began in ms.  Raises on a fatal status."""
         stream = self._current()
         self.stop.record(stream)
         self.host.copy_(self.status, non_blocking=True)
         stream.synchronize()
         v = int(self.flags[0])
         if v:
-            self.status.zero_()
-            stream.synchronize()
-            check_flags(v, what=what)
+            self._clear()
+        self.open = False
+        check_flags(v, what=what)
         return self.start.elapsed_time(self.stop)
 
 

@@ -62,3 +62,40 @@ def test_inference_mode_and_ordinary_calls_in_one_thread(ops, inference_first):
             with torch.inference_mode(inference):
                 _every_timed_call(ops, c)
     _in_a_new_thread(body)
+
+
+@pytest.mark.parametrize("side_stream", [False, True])
+def test_flags_of_a_call_that_ended_early_are_not_the_next_ones(ops, side_stream):
+    def body():
+        c = _context()
+        for raised in (KeyError, ops.KvcError):                # between the launches and end(); by end() itself
+            with torch.cuda.stream(torch.cuda.Stream() if side_stream else torch.cuda.current_stream()):
+                with pytest.raises(raised):
+                    with ops.TimedCall.on(c.device) as call:
+                        torch.cuda._sleep(100_000_000)         # the call's kernels are still at work when it ends
+                        call.status.fill_(ops._lib.FLAG_BAD_STREAM)
+                        if raised is KeyError:
+                            raise KeyError
+                        call.end("decode")
+            _every_timed_call(ops, c)
+            assert int(ops.TimedCall.on(c.device).status.item()) == 0
+    _in_a_new_thread(body)
+
+
+def test_a_call_that_raises_behind_its_launch(ops, monkeypatch):
+    def body():
+        c, other = _context(), _context(1)
+        bad = c._ti.buf.clone()
+        c._ti.buf.fill_(-1)                                # every vector but a block's first begins outside its block
+        c._pending = torch.zeros(1, 1, 2, 128, dtype=torch.uint8, device="cuda")
+
+        def fail(*a, **kw):
+            raise MemoryError("no room")
+        monkeypatch.setattr(ops, "dequant", fail)
+        with pytest.raises(MemoryError):
+            c.get()
+        monkeypatch.undo()
+        _every_timed_call(ops, other)
+        c._ti.buf, c._pending = bad, None
+        _every_timed_call(ops, c)
+    _in_a_new_thread(body)
