@@ -98,7 +98,7 @@ class TimedCall:
         self.flags = self.host.numpy()
         self.raw = self.stream = None
         self.open = False                                  # launches may be under way that write the status word
-        torch.cuda.synchronize(device)                     # zero, whichever stream uses it first
+        self._current().synchronize()                      # the word is zero, whichever stream uses it first
 
     @staticmethod
     def on(device):

@@ -99,3 +99,18 @@ def test_a_call_that_raises_behind_its_launch(ops, monkeypatch):
         c._ti.buf, c._pending = bad, None
         _every_timed_call(ops, c)
     _in_a_new_thread(body)
+
+
+def test_the_first_call_of_a_thread_waits_for_its_own_stream_only(ops):
+    def body():
+        ops.new_status("cuda:0")                               # memory for both words is at hand
+        torch.empty(1, dtype=torch.int32, pin_memory=True)
+        torch.cuda.synchronize()
+        other, done = torch.cuda.Stream(), torch.cuda.Event()
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(1_000_000_000)                   # half a second
+            done.record()
+        ops.TimedCall.on(torch.device("cuda", 0))
+        assert not done.query()
+        done.synchronize()
+    _in_a_new_thread(body)
