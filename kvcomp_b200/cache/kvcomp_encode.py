@@ -102,18 +102,14 @@ class _RecentRows:
         self.reserve(t, room, rows.shape[1:], rows.dtype, rows.device)[:] = rows
         self.commit(t)
 
-    def restart(self, old, n_kept, n_recent, room, shape, dtype, device):
-        """Start over with the kept rows `old` (or None) followed by places for n_kept more and for n_recent recent
-        rows, which the caller writes: returns the two places."""
-        n_old = 0 if old is None else old.shape[0]
-        n = n_old + n_kept + n_recent
-        if n:
-            buf = torch.empty((n + room,) + tuple(shape), dtype=dtype, device=device)
-            if n_old:
-                buf[:n_old] = old
+    def restart(self, n_old, n_kept, n_recent, buf):
+        """Start over in `buf` with the last n_old kept rows (copied), n_kept more and n_recent recent ones (the caller's,
+        in their places behind them)."""
+        if n_old:
+            buf[:n_old] = self.buf[self.lo - n_old:self.lo]
+        if n_old + n_kept + n_recent:
             self.buf = buf
-        self.q, self.lo, self.hi = 0, n_old + n_kept, n
-        return (None, None) if not n else (self.buf[n_old:self.lo], self.buf[self.lo:n])
+        self.q, self.lo, self.hi = 0, n_old + n_kept, n_old + n_kept + n_recent
 
     def rebuild(self, kept, recent, room):
         """Start over with the given kept rows and recent rows (either may be None)."""
@@ -372,6 +368,17 @@ class KVCompCtx:
         stream_room, cap = self._encode_room(part) if n_enc else (0, 0)
         if n_enc:
             self._encode_launch(part, stream_room, report)
+        # Where the window starts over, the rest of the new tokens is written before the wait: a caller's tensors are then read
+        # when the store returns, whichever stream they belong to.
+        over, k, n_old, buf = live == 0 or n > live, 0, 0, None
+        if over:
+            if self.keep_dequantised:
+                k = min(n, max(self.KEEP_ROWS // self.cut_block, 1) * self.cut_block)    # a long prefill keeps its last rows only
+                n_old = self._recent.kept if k == n else 0
+            if n_old + k + n_rest:
+                buf = torch.empty((n_old + k + n_rest + room,) + tuple(codes.shape[1:]), dtype=torch.float16, device=self.device)
+            if n_rest:
+                put_rest(buf[n_old + k:n_old + k + n_rest])
         words = report.read()                                 # synchronises, as the reference does
         flags = ops.check_flags(words[2], what="quantize")
         if flags & ops._lib.FLAG_MIN_OVERFLOW:
@@ -385,7 +392,7 @@ class KVCompCtx:
         # the fused kernel's range (tail_from); the rest of the new tokens joins the recent rows
         mi = self._mi.buf[self._mi.n:self._mi.n + n_units]
         sc = self._sc.buf[self._sc.n:self._sc.n + n_units]
-        if 0 < live and n <= live:
+        if not over:
             if self.keep_dequantised:
                 ops.dequant(codes, mi, sc, self.spec, out=self._recent.view()[:n])     # in place of the rows themselves
                 self._recent.consume(n)
@@ -396,18 +403,10 @@ class KVCompCtx:
                 put_rest(self._recent.reserve(n_rest, room, codes.shape[1:], torch.float16, self.device))
                 self._recent.commit(n_rest)
         else:
-            # the window starts over: the kept rows are dequantised, and the rest written, where they stay
-            k, old = 0, None
-            if self.keep_dequantised:
-                k = min(n, max(self.KEEP_ROWS // self.cut_block, 1) * self.cut_block)    # a long prefill keeps its last rows only
+            self._recent.restart(n_old, k, n_rest, buf)
+            if k:                                             # dequantised where they stay
                 first = (n - k) // self.spec.tok_div * self.spec.sj                      # unit of the first kept token
-                old = self._recent.rows_from_kept(self._recent.kept if k == n else 0)
-                old = None if old is None else old[:self._recent.kept]
-            kept, recent = self._recent.restart(old, k, n_rest, room, codes.shape[1:], torch.float16, self.device)
-            if k:
-                ops.dequant(codes[n - k:], mi[first:], sc[first:], self.spec, out=kept)
-            if n_rest:
-                put_rest(recent)
+                ops.dequant(codes[n - k:], mi[first:], sc[first:], self.spec, out=buf[n_old:n_old + k])
         self._mi.n += n_units
         self._sc.n += n_units
         self.compressed_ctx_len += T

@@ -56,3 +56,35 @@ def test_units_that_need_rows_are_refused(ops):
     assert not fits(ops.MODE_TOKEN, True, 64, 2, 8, 128, 64) and fits(ops.MODE_TOKEN, True, 64, 1, 8, 128, 64)
     assert not fits(ops.MODE_TOKEN, False, 64, 2, 65, 128, 64) and not fits(ops.MODE_CHANNEL, False, 192, 2, 8, 128, 192)
     assert not fits(ops.MODE_BLOCK, False, 64, 2, 8, 128, 64) and not fits(ops.MODE_CHANNEL, False, 64, 2, 8, 64, 64)
+
+
+@pytest.mark.parametrize("is_k", [True, False])
+@pytest.mark.parametrize("heads_first", [True, False])
+def test_a_prompt_is_read_when_the_store_returns(ops, monkeypatch, is_k, heads_first):
+    from kvcomp_b200.cache.kvcomp_encode import KVCompCtx
+    from kvcomp_b200.utils.compute import QuantMode
+    from kvcomp_b200.utils.config import KVCompCacheConfig, KVCompCacheConfigStatic
+    monkeypatch.setattr(KVCompCacheConfigStatic, "config", KVCompCacheConfig(
+        "synthetic", QuantMode("ChannelQuant"), QuantMode("TokenQuant"), 64, 64, 32, 32, 0.05, 0.1))
+    ctx = KVCompCtx(is_k, 2, 4, 128, 0.1, batch_shared=False, min_dtype=torch.int16, keep_dequantised=True)
+    x, cos, sin = _prompt(2, 4, 300, 1)
+    cos, sin = (cos, sin) if is_k and heads_first else (None, None)
+    rows = ops.rope_store(x, cos, sin)
+    want = rows.clone()
+    dequant = ops.dequant
+
+    def late(*a, **kw):                                        # what the store launches behind its wait comes late
+        torch.cuda._sleep(200_000_000)
+        return dequant(*a, **kw)
+    monkeypatch.setattr(ops, "dequant", late)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        if heads_first:
+            ctx.store_heads(x, cos, sin)
+        else:
+            ctx.store(rows)
+    for t in (x, rows) + ((cos, sin) if cos is not None else ()):
+        t.zero_()                                              # on the tensors' own stream: they are the caller's again
+    torch.cuda.synchronize()
+    live = len(ctx.buffer)
+    assert 32 <= live < 300 and torch.equal(ctx.buffer, want[-live:])
