@@ -575,9 +575,10 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_ke
         __syncthreads();                                    // (also: the head before is done with its units' parameters)
         if (tid < 128) {                                    // thread = channel
             const int at2 = tid & ~1;
-            __half2 a = *reinterpret_cast<const __half2 *>(&smn[0][at2]), z = *reinterpret_cast<const __half2 *>(&smx[0][at2]);
+            // (from the infinities: a channel of nothing but NaN has the extremes +inf and -inf, as in quant_channel_kernel)
+            __half2 a = __float2half2_rn(INFINITY), z = __float2half2_rn(-INFINITY);
 #pragma unroll
-            for (int w = 1; w < WARPS; w++) { a = __hmin2(a, *reinterpret_cast<const __half2 *>(&smn[w][at2])); z = __hmax2(z, *reinterpret_cast<const __half2 *>(&smx[w][at2])); }
+            for (int w = 0; w < WARPS; w++) { a = __hmin2(a, *reinterpret_cast<const __half2 *>(&smn[w][at2])); z = __hmax2(z, *reinterpret_cast<const __half2 *>(&smx[w][at2])); }
             __half sc;
             const UnitParam q = unit_param(tid & 1 ? __high2float(a) : __low2float(a), tid & 1 ? __high2float(z) : __low2float(z), rel, &sc, &flags);
             const long long u = ((j * B + b) * H + h) * 128 + tid;

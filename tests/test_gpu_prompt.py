@@ -51,6 +51,27 @@ def test_prompt_in_place_equals_rows(ops, mode, block, B, H, T, more, rope):
             assert torch.equal(ops.rope_store(x, cos, sin, first=T), rows[T:])
 
 
+@pytest.mark.parametrize("mode,block,rope", [("ChannelQuant", 64, "each"), ("ChannelQuant", 64, None), ("ChannelQuant", 128, None),
+                                             ("TokenQuant", 64, None), ("VectorQuant", 64, None)])
+@pytest.mark.parametrize("special", [float("nan"), float("inf"), float("-inf"), -0.0, 65504.0])
+def test_prompt_of_special_values_equals_rows(ops, mode, block, rope, special):
+    m, (B, H, T) = ops.MODES[mode], (2, 5, 256)
+    for where in ("channel", "token", "head", "half a block", "one"):
+        x, cos, sin = _prompt(B, H, T, 1)
+        at = {"channel": (1, 2, slice(None), 77), "token": (1, slice(None), 130), "head": (0, 4), "one": (0, 1, 3, 100),
+              "half a block": (1, 0, slice(0, block // 2), slice(None))}[where]
+        x[at] = special
+        cos, sin = (None, None) if rope is None else (cos, sin)
+        rows = ops.rope_store(x, cos, sin)
+        hist, hist2 = (torch.zeros(256, dtype=torch.int64, device="cuda") for _ in range(2))
+        want, mi, sc, _, st = ops.quantize(rows, m, block, 0.05, False, min_dtype=torch.int16, hist=hist)
+        mi2, sc2, st2 = torch.empty_like(mi), torch.empty_like(sc), ops.new_status(x.device)
+        got = ops.quantize_heads(x, T, cos, sin, m, block, 0.05, False, mi2, sc2, hist2, st2)
+        assert int(st.item()) == int(st2.item()), where
+        assert torch.equal(sc.view(torch.int16), sc2.view(torch.int16)) and torch.equal(mi, mi2), where
+        assert torch.equal(want, got) and torch.equal(hist, hist2), where
+
+
 def test_units_that_need_rows_are_refused(ops):
     fits = ops.quantize_heads_fits
     assert not fits(ops.MODE_TOKEN, True, 64, 2, 8, 128, 64) and fits(ops.MODE_TOKEN, True, 64, 1, 8, 128, 64)
