@@ -448,20 +448,20 @@ __device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const ui
 // Bound by memory: 2 bytes read and 1 written per value, where a rotated and transposed copy of the tensor took 4 more before
 // the quantiser read it (K per channel: twice).
 
-// The CTA's histogram: codes below 32 are counted two at a time, pairs[first + 32 * second], others in ones (three instructions
-// per code one by one, a good half of that for a pair; fewer lanes meet on a counter).
-struct PairBins { unsigned int pairs[1024], ones[256]; };
+// The CTA's histogram: codes below 32 are counted two at a time, n[first + 32 * second], others one by one behind these 1024
+// counters, n[1024 + code] (three instructions per code one by one, a good half of that for a pair; fewer lanes meet on a counter).
+struct PairBins { unsigned int n[1024 + 256]; };
 __device__ __forceinline__ void bins_clear(PairBins &b, int tid, int nthr) {
-    for (int i = tid; i < 1280; i += nthr) b.pairs[i] = 0;              // both arrays
+    for (int i = tid; i < 1024 + 256; i += nthr) b.n[i] = 0;
     __syncthreads();
 }
 __device__ __forceinline__ void bins_add(PairBins &b, const uint32_t (&u)[4]) {     // two codes per word, 16 bits each
     if (((u[0] | u[1] | u[2] | u[3]) & 0x00e000e0u) == 0) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) atomicAdd(reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(b.pairs) + __dp4a(u[k], 0x00800004u, 0u)), 1u);
+        for (int k = 0; k < 4; k++) atomicAdd(reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(b.n) + __dp4a(u[k], 0x00800004u, 0u)), 1u);
     } else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) { atomicAdd(&b.ones[u[k] & 0xffu], 1u); atomicAdd(&b.ones[u[k] >> 16], 1u); }
+        for (int k = 0; k < 4; k++) { atomicAdd(&b.n[1024 + (u[k] & 0xffu)], 1u); atomicAdd(&b.n[1024 + (u[k] >> 16)], 1u); }
     }
 }
 __device__ __forceinline__ void bins_flush(const PairBins &b, unsigned long long *gh, int tid) {      // by the first 256 threads
@@ -470,11 +470,11 @@ __device__ __forceinline__ void bins_flush(const PairBins &b, unsigned long long
     unsigned int c = 0;
     const int s = tid >> 3, part = tid & 7;                 // eight threads fold a symbol's row and column
 #pragma unroll
-    for (int k = 0; k < 4; k++) c += b.pairs[s + 32 * (part * 4 + k)] + b.pairs[32 * s + part * 4 + k];
+    for (int k = 0; k < 4; k++) c += b.n[s + 32 * (part * 4 + k)] + b.n[32 * s + part * 4 + k];
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if (part == 0 && c) atomicAdd(&gh[s], (unsigned long long)c);
-    if (b.ones[tid]) atomicAdd(&gh[tid], (unsigned long long)b.ones[tid]);
+    if (b.n[1024 + tid]) atomicAdd(&gh[tid], (unsigned long long)b.n[1024 + tid]);
 }
 
 // the packed path of quant_eight with what it needs in registers; param(i): value i's unit, for anything else

@@ -109,3 +109,17 @@ def test_a_prompt_is_read_when_the_store_returns(ops, monkeypatch, is_k, heads_f
     torch.cuda.synchronize()
     live = len(ctx.buffer)
     assert 32 <= live < 300 and torch.equal(ctx.buffer, want[-live:])
+
+
+@pytest.mark.parametrize("mode,block,H", [("ChannelQuant", 64, 3), ("ChannelQuant", 128, 8), ("TokenQuant", 64, 8), ("VectorQuant", 64, 33)])
+@pytest.mark.parametrize("rel", [0.2, 0.033, 0.03, 0.004])      # codes below 32 alone, around it, up to 250
+def test_prompt_counts_start_from_zero(ops, mode, block, H, rel):
+    """Launch behind launch, each over the counters that the one before left in shared memory."""
+    m = ops.MODES[mode]
+    x, _, _ = _prompt(2, H, 512, 7)
+    n = ops.qspec(m, False, 2, H, 128, block).units(512, 2, H, 128)
+    mi, sc = torch.empty(n, dtype=torch.int16, device="cuda"), torch.empty(n, dtype=torch.float16, device="cuda")
+    for _ in range(3):
+        hist = torch.zeros(256, dtype=torch.int64, device="cuda")
+        codes = ops.quantize_heads(x, 512, None, None, m, block, rel, False, mi, sc, hist, ops.new_status(x.device))
+        assert torch.equal(hist, torch.bincount(codes.view(-1), minlength=256))
