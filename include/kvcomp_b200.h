@@ -225,13 +225,13 @@ int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_k,
 void kvc_encode_debug(int wait_limit, int starve);
 
 /* k_/v_entropy_decode_cuda_export (kernels.cu:1013-1087): stream -> u8 codes [T, cols, 128].
- * block_info offsets are relative to `encoded`. */
+ * block_info offsets are relative to `encoded`.  No byte outside encoded .. encoded + encoded_bytes - 1 is read. */
 int kvc_decode(const uint8_t *encoded, int64_t encoded_bytes, const void *block_info,
                const uint16_t *thread_info, const void *book, int64_t T, int64_t cols, int is_k,
                uint8_t *codes, int32_t *status, kvc_stream_t stream);
 /* kvc_decode with the stream's largest block size (kvc_encode's total_bytes[1]; 0 = unknown, the
- * format's 8191): smaller staging slots let more CTAs share an SM.  A block beyond the bound is
- * skipped and flagged KVC_FLAG_BAD_STREAM. */
+ * format's 8191): smaller staging slots let more blocks be at work on an SM.  A block beyond the
+ * bound is skipped and flagged KVC_FLAG_BAD_STREAM. */
 int kvc_decode_bounded(const uint8_t *encoded, int64_t encoded_bytes, const void *block_info,
                        const uint16_t *thread_info, const void *book, int64_t T, int64_t cols, int is_k,
                        uint32_t max_block_bytes, uint8_t *codes, int32_t *status, kvc_stream_t stream);

@@ -40,28 +40,29 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
     int flags = 0;
     // a block's record, and from it the bytes [lead, lead + nbytes) of the slot (0 bytes: nothing to decode)
     auto info_of = [&](long long blk) { return blk < nblk ? block_info[blk] : make_uint2(0u, 0u); };
-    auto block_of = [&](uint2 bi, uint32_t &nbytes, uint32_t &lead, const uint8_t *&src) {
-        nbytes = 0; lead = 0; src = encoded;
+    auto block_of = [&](uint2 bi, uint32_t &off, uint32_t &nbytes, uint32_t &lead) {
+        off = nbytes = lead = 0;
         const uint32_t n = bi.y & 0xffffu;
         if (n > max_block || (long long)bi.x + n > encoded_bytes) { flags |= KVC_FLAG_BAD_STREAM; return; }
-        nbytes = n; src = encoded + bi.x; lead = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
+        off = bi.x; nbytes = n; lead = (uint32_t)(reinterpret_cast<uintptr_t>(encoded + off) & 15);
     };
+    // whether the block's range, widened to 16-byte boundaries as a bulk copy wants it, passes the end of the stream: what lies
+    // behind that is not the caller's to be read.  The pair's threads bring such a block (in the encoder's order the last one).
+    auto beyond = [&](uint32_t off, uint32_t nbytes) { return nbytes && (((long long)off + nbytes + 15) & ~15ll) > encoded_bytes; };
     auto start_of = [&](long long blk) { return v && blk < nblk ? (uint32_t)(thread_info[blk * 64 + v - 1] >> 3) : 0u; };
-    // by the pair's first thread: one arrival per phase, even for 0 bytes.  The source widens to 16-byte boundaries (the stream
-    // starts on one, so that these lie inside its memory).
-    auto fetch = [&](const uint8_t *src, uint32_t nbytes, uint32_t lead) {
-        const uint32_t bytes = nbytes ? (lead + nbytes + 15u) & ~15u : 0u;
+    // by the pair's first thread: one arrival per phase, even for 0 bytes
+    auto fetch = [&](uint32_t off, uint32_t nbytes, uint32_t lead) {
+        const uint32_t bytes = nbytes && !beyond(off, nbytes) ? (lead + nbytes + 15u) & ~15u : 0u;
         kvc_mbar_expect_tx(&sm.bar[pair], bytes);
-        if (bytes) kvc_bulk_g2s(slot, src - lead, bytes, &sm.bar[pair]);
+        if (bytes) kvc_bulk_g2s(slot, encoded + off - lead, bytes, &sm.bar[pair]);
     };
     if (BULK && v == 0 && pair < pairs) { kvc_mbar_init(&sm.bar[pair], 1); kvc_mbar_fence_init(); sm.dead[pair] = 0; }
     // neighbouring pairs of the grid take neighbouring blocks
     long long blk = (long long)blockIdx.x * pairs + pair;
-    uint32_t nbytes = 0, lead = 0;
-    const uint8_t *src = encoded;
+    uint32_t off = 0, nbytes = 0, lead = 0;
     if (pair < pairs) {
-        block_of(info_of(blk), nbytes, lead, src);
-        if (BULK && v == 0) fetch(src, nbytes, lead);
+        block_of(info_of(blk), off, nbytes, lead);
+        if (BULK && v == 0) fetch(off, nbytes, lead);
     }
     uint32_t start = pair < pairs ? start_of(blk) : 0u;
     kvc_load_lut(sm.lut, book, threadIdx.x, blockDim.x);
@@ -78,8 +79,10 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
             landed = kvc_mbar_wait(&sm.bar[pair], par);
             par ^= 1u;
             if (!landed) { flags |= KVC_FLAG_WAIT_TIMEOUT; if (v == 0) sm.dead[pair] = 1; }
-        } else {
-            if (nbytes) kvc_stage_block(slot, encoded, encoded_bytes, src - encoded, nbytes, v, 64);
+        }
+        if (!BULK || beyond(off, nbytes)) {
+            if (nbytes) kvc_stage_block(slot, encoded, encoded_bytes, off, nbytes, v, 64);
+            if (BULK) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // a bulk copy may write there next
             sync();
         }
         if (nbytes) {
@@ -95,8 +98,8 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
         const bool out = nbytes != 0;
         sync();                                             // the tile is complete, the slot free
         if (BULK && sm.dead[pair]) break;
-        block_of(next, nbytes, lead, src);
-        if (BULK && v == 0) fetch(src, nbytes, lead);       // lands while the tile goes out
+        block_of(next, off, nbytes, lead);
+        if (BULK && v == 0) fetch(off, nbytes, lead);       // lands while the tile goes out
         start = start_of(blk + step);
         if (out) {
             if (VALUES && is_k) {                            // thread = 8 channels of every fourth row

@@ -464,7 +464,7 @@ def encode(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset
 
 def decode(encoded, block_info, thread_info, book, T, B, H, is_k, out=None, status=None, max_block=0):
     """Huffman-decode a stream to its uint8 codes [T,B,H,128].  max_block: the stream's largest block in
-    bytes as the encoder reported it (0 = unknown); a known bound lets more CTAs share an SM."""
+    bytes as the encoder reported it (0 = unknown); a known bound lets more blocks be at work on an SM."""
     lib = _lib.load()
     _cuda(encoded, torch.uint8, "encoded")
     dev = encoded.device

@@ -1,5 +1,6 @@
 """The decoder's pairs of warps over every split of the blocks: one block, fewer blocks than SMs, a ragged last round; known
 and unknown largest block; a stream that does not start on 16 bytes."""
+import numpy as np
 import pytest
 import torch
 
@@ -36,3 +37,48 @@ def test_blocks_over_pairs_of_warps(ops, is_k, B, H, T):
             out = torch.empty(T, B, H, 128, dtype=torch.float16, device="cuda")
             st = ops.decode_values(ops.make_cache(enc, bi, ti, book, mi, sc, spec, size, bound), T, B, H, is_k, out)
             assert ops.read_status(st) == 0 and torch.equal(out.view(torch.int16), ops.dequant(codes, mi, sc, spec).view(torch.int16))
+
+
+@pytest.mark.parametrize("is_k", [True, False])
+@pytest.mark.parametrize("B,H,T,leads", [(1, 1, 128, range(16)), (8, 40, 1024, (0, 3, 15))])
+def test_streams_that_end_with_their_memory(ops, is_k, B, H, T, leads):
+    """No byte behind the stream is asked for: the block whose 16-byte chunks pass the end comes by plain loads, be it the
+    last one of the launch or, with blocks in another order, one that the pair goes on from."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, B, H, 128, device="cuda", generator=g).half()
+    hist = torch.zeros(256, dtype=torch.int64, device="cuda")
+    codes, mi, sc, spec, _ = ops.quantize(x, ops.MODE_CHANNEL if is_k else ops.MODE_TOKEN, 64, 0.05, False, min_dtype=torch.int16, hist=hist)
+    book = ops.build_codebook(hist)
+    bsz, tsz, _, n = ops.buffer_sizes(T, B * H * 128, is_k)
+    bi, ti = torch.empty(bsz, dtype=torch.uint8, device="cuda"), torch.empty(tsz, dtype=torch.uint8, device="cuda")
+    enc = torch.empty(n, dtype=torch.uint8, device="cuda")
+    total, st = ops.encode(codes, is_k, book.encode_table(), bi, ti, enc)
+    size, largest = total.tolist()
+    assert ops.read_status(st) == 0
+    values = ops.dequant(codes, mi, sc, spec)
+    rec = bi.cpu().numpy().view(np.uint32).reshape(-1, 2)
+    count = (rec[:, 1] & 0xffff).astype(np.int64)
+    host = enc[:size].cpu().numpy()
+    ends = set()
+    for lead in leads:
+        order = np.random.default_rng(lead).permutation(len(rec)) if lead % 2 else np.arange(len(rec))
+        at = np.empty(len(rec), np.int64)
+        at[order] = lead + np.concatenate(([0], np.cumsum(count[order])[:-1]))
+        stream = np.full(lead + size, 0xff, np.uint8)
+        for i in range(len(rec)):
+            stream[at[i]:at[i] + count[i]] = host[rec[i, 0]:rec[i, 0] + count[i]]
+        moved = rec.copy()
+        moved[:, 0] = at
+        dbi = torch.from_numpy(moved.view(np.uint8).reshape(-1)).cuda()
+        whole = torch.full((lead + size + 64,), 0xff, dtype=torch.uint8, device="cuda")
+        whole[:lead + size] = torch.from_numpy(stream).cuda()
+        cut = whole[:lead + size]
+        assert cut.data_ptr() % 16 == 0
+        ends.add((lead + size) % 16)
+        for bound in (0, largest):
+            back, st = ops.decode(cut, dbi, ti, book, T, B, H, is_k, max_block=bound)
+            assert ops.read_status(st) == 0 and torch.equal(back, codes)
+            out = torch.empty(T, B, H, 128, dtype=torch.float16, device="cuda")
+            st = ops.decode_values(ops.make_cache(cut, dbi, ti, book, mi, sc, spec, lead + size, bound), T, B, H, is_k, out)
+            assert ops.read_status(st) == 0 and torch.equal(out.view(torch.int16), values.view(torch.int16))
+    assert len(ends) == len(leads)
