@@ -241,6 +241,12 @@ int kvc_decode_bounded(const uint8_t *encoded, int64_t encoded_bytes, const void
 int kvc_decode_values(const kvc_cache *c, int64_t T, int64_t B, int64_t H, int is_k, void *out, int32_t *status,
                       kvc_stream_t stream);
 
+/* Diagnostics, no counterpart in the reference.  The decoder waits for a block's bytes at most `wait_limit` tries (0 = the
+ * default of 2^22); a wait that runs out raises KVC_FLAG_WAIT_TIMEOUT, the block is not decoded and its pair of warps takes no
+ * further one.  starve != 0 makes the kernel announce bytes that it never copies, so that a test can see a wait run out with
+ * nothing in flight.  Streams that do not start on 16 bytes are not waited for.  Process-wide, read at every launch. */
+void kvc_decode_debug(int wait_limit, int starve);
+
 /* k_decode_and_mat_vec_mul_cuda_export (kernels.cu:1093-1136): raw scores
  * S[b,hq,t] = sum_c x^K[t,b,hkv,c] * q[b,hq,c], fp32 accumulation.  q: device fp16
  * [B,Hq,128]; out: device [B,Hq,T], fp16 (out_f32 = 0, the reference's C) or fp32. */

@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
     const uint8_t *__restrict__ encoded, long long encoded_bytes, const uint2 *__restrict__ block_info,
     const uint16_t *__restrict__ thread_info, const void *__restrict__ book, long long nblk, long long cols, int is_k,
     uint32_t max_block, uint32_t slot_bytes, int pairs, uint8_t *__restrict__ codes, kvc_qmeta_dev m, long long H,
-    __half *__restrict__ values, int *__restrict__ status) {
+    __half *__restrict__ values, int *__restrict__ status, int wait_limit, int starve) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     DecodeSmem &sm = *reinterpret_cast<DecodeSmem *>(smem_raw);
     const int pair = threadIdx.x >> 6, v = threadIdx.x & 63;        // v: the thread's vector of the block
@@ -50,11 +50,12 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
     // behind that is not the caller's to be read.  The pair's threads bring such a block (in the encoder's order the last one).
     auto beyond = [&](uint32_t off, uint32_t nbytes) { return nbytes && (((long long)off + nbytes + 15) & ~15ll) > encoded_bytes; };
     auto start_of = [&](long long blk) { return v && blk < nblk ? (uint32_t)(thread_info[blk * 64 + v - 1] >> 3) : 0u; };
-    // by the pair's first thread: one arrival per phase, even for 0 bytes
+    // by the pair's first thread: one arrival per phase, even for 0 bytes (starve, tests of the bounded waits only: bytes are
+    // announced that are never copied)
     auto fetch = [&](uint32_t off, uint32_t nbytes, uint32_t lead) {
         const uint32_t bytes = nbytes && !beyond(off, nbytes) ? (lead + nbytes + 15u) & ~15u : 0u;
-        kvc_mbar_expect_tx(&sm.bar[pair], bytes);
-        if (bytes) kvc_bulk_g2s(slot, encoded + off - lead, bytes, &sm.bar[pair]);
+        kvc_mbar_expect_tx(&sm.bar[pair], starve ? 16u : bytes);
+        if (bytes && !starve) kvc_bulk_g2s(slot, encoded + off - lead, bytes, &sm.bar[pair]);
     };
     if (BULK && v == 0 && pair < pairs) { kvc_mbar_init(&sm.bar[pair], 1); kvc_mbar_fence_init(); sm.dead[pair] = 0; }
     // neighbouring pairs of the grid take neighbouring blocks
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
         if (BULK) {
             // a wait that runs out: the thread does not decode; a barrier whose phase its issuer did not see complete is
             // never armed again, and the pair stops
-            landed = kvc_mbar_wait(&sm.bar[pair], par);
+            landed = kvc_mbar_wait(&sm.bar[pair], par, wait_limit);
             par ^= 1u;
             if (!landed) { flags |= KVC_FLAG_WAIT_TIMEOUT; if (v == 0) sm.dead[pair] = 1; }
         }
@@ -181,11 +182,15 @@ __global__ void __launch_bounds__(64 * MAX_PAIRS, 1) decode_kernel(
         sync();                                             // the tile is free
     }
     // the last copy asked for is empty; after a wait that ran out, the one still open may be in flight
-    if (BULK && v == 0 && !kvc_mbar_wait(&sm.bar[pair], sm.dead[pair] ? par ^ 1u : par)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+    if (BULK && v == 0 && !kvc_mbar_wait(&sm.bar[pair], sm.dead[pair] ? par ^ 1u : par, wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
     if (flags) atomicOr(status, flags);
 }
 
 }  // namespace
+
+// Diagnostics for tests of the bounded waits (kvc_decode_debug): process-wide, read at every launch.
+static int g_wait_limit = 0, g_starve = 0;
+extern "C" void kvc_decode_debug(int wait_limit, int starve) { g_wait_limit = wait_limit; g_starve = starve; }
 
 // Both outputs' launch; codes or values is null.
 static int decode_launch(const char *who, const uint8_t *encoded, int64_t encoded_bytes, const void *block_info,
@@ -222,7 +227,8 @@ static int decode_launch(const char *who, const uint8_t *encoded, int64_t encode
     const long long ctas = (nblk + pairs - 1) / pairs;
     kernel<<<(unsigned)(ctas < sms ? ctas : sms), threads, smem, kvc_cu(stream)>>>(
         encoded, encoded_bytes, reinterpret_cast<const uint2 *>(block_info), thread_info, book, nblk, cols, is_k,
-        max_block, slot_bytes, pairs, codes, m, H, reinterpret_cast<__half *>(values), status);
+        max_block, slot_bytes, pairs, codes, m, H, reinterpret_cast<__half *>(values), status,
+        g_wait_limit > 0 ? g_wait_limit : KVC_WAIT_LIMIT, g_starve);
     KVC_LAUNCH_OK();
     return KVC_OK;
 }

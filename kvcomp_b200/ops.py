@@ -589,6 +589,11 @@ def encode_debug(wait_limit=0, starve=False):
     _lib.load().kvc_encode_debug(int(wait_limit), int(bool(starve)))
 
 
+def decode_debug(wait_limit=0, starve=False):
+    """Diagnostics of the decoder's bounded waits for a block's bytes (kvc_decode_debug); (0, False) restores the defaults."""
+    _lib.load().kvc_decode_debug(int(wait_limit), int(bool(starve)))
+
+
 def attn_debug(wait_limit=0, starve=False):
     """Diagnostics of the attention kernel's bounded staging waits (kvc_attn_debug); (0, False) restores
     the defaults."""

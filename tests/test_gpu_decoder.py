@@ -82,3 +82,39 @@ def test_streams_that_end_with_their_memory(ops, is_k, B, H, T, leads):
             st = ops.decode_values(ops.make_cache(cut, dbi, ti, book, mi, sc, spec, lead + size, bound), T, B, H, is_k, out)
             assert ops.read_status(st) == 0 and torch.equal(out.view(torch.int16), values.view(torch.int16))
     assert len(ends) == len(leads)
+
+
+@pytest.mark.parametrize("is_k", [True, False])
+@pytest.mark.parametrize("values", [True, False])
+@pytest.mark.parametrize("T", [128, 4096])                      # a block for a pair at most; several
+def test_a_staging_wait_that_runs_out(ops, is_k, values, T):
+    """The waits for a block's bytes are bounded.  With the diagnostic that announces bytes which are never copied they run
+    out after a few tries: the call returns, the status word says so, and the next ordinary call is correct."""
+    B, H = 2, 40
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, B, H, 128, device="cuda", generator=g).half()
+    hist = torch.zeros(256, dtype=torch.int64, device="cuda")
+    codes, mi, sc, spec, _ = ops.quantize(x, ops.MODE_CHANNEL if is_k else ops.MODE_TOKEN, 64, 0.05, False, min_dtype=torch.int16, hist=hist)
+    book = ops.build_codebook(hist)
+    bsz, tsz, _, n = ops.buffer_sizes(T, B * H * 128, is_k)
+    bi, ti = torch.empty(bsz, dtype=torch.uint8, device="cuda"), torch.empty(tsz, dtype=torch.uint8, device="cuda")
+    enc = torch.empty(n, dtype=torch.uint8, device="cuda")
+    total, st = ops.encode(codes, is_k, book.encode_table(), bi, ti, enc)
+    size, largest = total.tolist()
+    assert ops.read_status(st) == 0
+
+    def call():
+        if not values:
+            return ops.decode(enc[:size], bi, ti, book, T, B, H, is_k, max_block=largest)
+        out = torch.empty(T, B, H, 128, dtype=torch.float16, device="cuda")
+        return out, ops.decode_values(ops.make_cache(enc, bi, ti, book, mi, sc, spec, size, largest), T, B, H, is_k, out)
+    try:
+        ops.decode_debug(wait_limit=8, starve=True)
+        _, st = call()
+        torch.cuda.synchronize()
+        assert ops.read_status(st, raise_on_fatal=False) & 0x400
+    finally:
+        ops.decode_debug()
+    out, st = call()
+    want = ops.dequant(codes, mi, sc, spec) if values else codes
+    assert ops.read_status(st) == 0 and torch.equal(out.view(torch.uint8), want.view(torch.uint8))
