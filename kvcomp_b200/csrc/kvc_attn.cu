@@ -617,19 +617,30 @@ template <int G> int rows_fit(const AttnParams &p) {         // workers that an 
 int one_fit(const AttnParams &p);
 int rows_fit(const AttnParams &p, int heads) { return heads == 1 ? one_fit(p) : heads > 4 ? rows_fit<8>(p) : (heads > 2 ? rows_fit<4>(p) : rows_fit<2>(p)); }
 
+// Equal items for `most` takers per SM: in how many rounds they go, and the takers that this many rounds need: those of a
+// fuller SM would run slower and the last round leave more of them idle.  (One head, seven workers at first, device time: 320 columns
+// of 6144 tokens in 4 runs 254 us, now 229 (three CTAs of 256 threads, the kernel before the workers: 250); 192 of 4096 in 6 runs 127 and 107; 36 of
+// 4096, the library's plan, 36 and 27; 800 columns of 128 tokens, 4 heads, 39 and 31.)
+struct Spread { long long rounds, per_sm; };
+Spread spread(long long items, long long most, long long sms) {
+    const long long rounds = (items + most * sms - 1) / (most * sms);
+    return {rounds, (items + rounds * sms - 1) / (rounds * sms)};
+}
+
 // How many of an SM's workers share a column when every column's output is written directly (no workspace, or a single run
 // without a tail): without company a worker would take all of a column's `units` (steps and passes of the tail) in turn
 // while most of the device is idle.  A unit takes about 6 + a parts of time with `a` workers at work on the SM (2 heads: 9.2 us
 // alone, 14.4 us with five), a team's sums and its next column another 3.5: over 1 to 700 columns of 2 to 19 units the choice is
-// within 1 % of the best size on average, and nowhere behind a worker per column.  2 heads per column, no workspace, a worker per column against teams: 8 columns of 1024 tokens
-// 77.6 and 31.5 us, 64 of 8192 594 and 189 us, 256 of 256 (two teams of two on an SM) 26.1 and 19.6 us.
-int rows_team(long long cols, long long units, int workers, int sms) {
-    if (cols >= (long long)workers * sms) return 0;          // enough columns for all
+// within 1 % of the best size on average, and nowhere behind a worker per column.  2 heads per column, no workspace, a worker per column
+// against teams: 8 columns of 1024 tokens 77.6 and 31.5 us, 64 of 8192 594 and 189 us, 256 of 256 (two teams of two on an SM) 26.1 and
+// 19.6 us; more columns than workers, where a worker per column goes in two rounds, the second nearly empty: 1280 of 1024 tokens,
+// one head, 236 and 165 us.
+int rows_team(long long cols, long long units, int workers, int sms) {       // (0: each its own columns)
     int best = 0;
     long long least = 0;
     for (int size = 1; size <= workers && size <= units; size++) {
-        const long long teams = std::min<long long>(workers / size, (cols + sms - 1) / sms);     // of an SM
-        const long long cost = ((cols + teams * sms - 1) / (teams * sms)) * (2 * ((units + size - 1) / size) * (6 + teams * size) + (size > 1 ? 7 : 0));
+        const Spread s = spread(cols, workers / size, sms);
+        const long long teams = s.per_sm, cost = s.rounds * (2 * ((units + size - 1) / size) * (6 + teams * size) + (size > 1 ? 7 : 0));
         if (size == 1 || cost < least) { least = cost; best = size > 1 ? size : 0; }
     }
     return best;
@@ -1789,10 +1800,12 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
 #define KVC_AT(GG)                                                                                              \
     {                                                                                                           \
         int workers = rows_fit(p, GG);                                                                          \
-        p.team = p.partial ? 0 : rows_team(cols, p.n_tiles + (Tr + 127) / 128, workers, sms);                   \
-        if (p.team) { const long long n = (cols + sms - 1) / sms; workers = p.team * (int)std::min<long long>(n, workers / p.team); } \
-        /* fewer than fit an SM where the items then spread over more SMs */                                    \
-        else if (p.work < (long long)workers * sms) workers = (int)((p.work + sms - 1) / sms);                  \
+        /* (with a tail and columns for all workers a pass of the tail is no step: 1023 columns of 2048 tokens and 64 rows, 4 heads, */ \
+        /* a worker per column 464 us, teams as chosen for 18 steps 551) */                                     \
+        p.team = p.partial || (Tr > 0 && cols >= (long long)workers * sms) ? 0 : rows_team(cols, p.n_tiles + (Tr + 127) / 128, workers, sms); \
+        if (p.team) workers = p.team * (int)spread(cols, workers / p.team, sms).per_sm;                         \
+        /* (short runs at the end of the columns fill the last round up; a single round spreads over all SMs) */ \
+        else if (const Spread s = spread(p.work, workers, sms); p.long_runs == splits || s.rounds == 1) workers = (int)s.per_sm; \
         const size_t smem = attn_smem<GG>(p, workers);                                                          \
         static kvc_launch_slot slots[4];                                                                        \
         auto *kernel = p.team ? (bulk ? attn_kernel<GG, true, true>() : attn_kernel<GG, false, true>())         \
