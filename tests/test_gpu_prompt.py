@@ -1,5 +1,5 @@
 """Prompts quantised where their projections left them (kvc_quantize_heads) against the rotated and transposed rows through
-kvc_quantize, and the decoder's pairs of warps over every split of the blocks: the same bits."""
+kvc_quantize: the same bits; and the stores that quantise them."""
 import pytest
 import torch
 
@@ -98,6 +98,7 @@ def test_a_prompt_is_read_when_the_store_returns(ops, monkeypatch, is_k, heads_f
         torch.cuda._sleep(200_000_000)
         return dequant(*a, **kw)
     monkeypatch.setattr(ops, "dequant", late)
+    torch.empty_like(x).zero_()                                # (a kernel's first launch may wait for the device)
     torch.cuda.synchronize()
     with torch.cuda.stream(torch.cuda.Stream()):
         if heads_first:
