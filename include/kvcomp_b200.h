@@ -86,7 +86,7 @@ typedef struct {
     const void *book;             /* device, KVC_BOOK_BYTES, from kvc_build_codebook / kvc_book_from_tree */
     kvc_qmeta q;
     int32_t max_block_bytes;      /* upper bound of any block's byte count (kvc_encode reports it); 0 = unknown
-                                     (8191 is assumed).  A tight bound lets more CTAs share an SM. */
+                                     (8191 is assumed).  A tight bound lets more of them be at work on an SM. */
     int32_t reserved;
 } kvc_cache;
 
@@ -266,15 +266,14 @@ int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hkv, int64_t 
  * be NULL).  q: device fp16 [B,Hq,128]; out: device fp16
  * [B,Hq,128].  Scores never leave the SM; no fp16 K/V is written to memory.
  * Work is cut into items, one (sequence, KV head) column x one of `splits` equal runs of
- * 256-token tiles (with several query heads per KV head and room for partial results: where it pays, runs
- * of its own choice, at most twice as many, in the same workspace; without partial results: where it pays, a
- * column shared by several workers of a CTA); as many CTAs as the device holds at once take items until none
- * is left, and a second small kernel merges the `splits` partial results of every head and adds the
- * tail's tokens (it does the whole step when T = 0).  splits = 0
- * picks kvc_attn_splits(T, B, Hkv, 0).  workspace: kvc_attn_workspace(B, Hq, splits) bytes
+ * 256-token tiles (with room for partial results: where it pays, runs of its own choice, at most twice as
+ * many, in the same workspace; without partial results: where it pays, a column shared by several workers of
+ * a CTA); workers of 128 threads, several to an SM, take items until none is left, and a second small kernel
+ * merges the partial results of every head and adds the tail's tokens (it does the whole step when T = 0).
+ * splits = 0 picks kvc_attn_splits(T, B, Hkv, 0).  workspace: kvc_attn_workspace(B, Hq, splits) bytes
  * of device memory whose first 256 bytes the caller zeroes once before the first use (the
  * kernel leaves them zeroed); NULL is allowed when splits = 1 (a tail then costs more: the
- * first kernel reads it itself, a column's CTA at a time).  Launches that share a
+ * first kernel reads it itself, by the workers of a column).  Launches that share a
  * workspace must not overlap on the device.
  * The launch uses programmatic stream serialisation: it may read what k and v point to (streams, tables, books,
  * unit parameters) while the kernel directly ahead of it in the stream ends.  That kernel may write q, the tails and
@@ -302,7 +301,7 @@ int kvc_attn_decode_packed(const kvc_attn_args *args, kvc_stream_t stream);
 
 /* Diagnostics, no counterpart in the reference (its kernels have no device-side waits).  The attention
  * kernel waits for its staged blocks at most `wait_limit` tries (0 = the default of 2^22); a wait that
- * runs out raises KVC_FLAG_WAIT_TIMEOUT, the CTA stops taking work and the call returns.  starve != 0
+ * runs out raises KVC_FLAG_WAIT_TIMEOUT, the worker stops taking work and the call returns.  starve != 0
  * makes the kernel announce staging bytes that it never copies, so that a test can see a wait run out
  * with nothing in flight; outputs of such a call are undefined.  Process-wide, read at every launch. */
 void kvc_attn_debug(int wait_limit, int starve);

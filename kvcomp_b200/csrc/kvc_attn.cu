@@ -585,7 +585,8 @@ struct AttnParams {
 // tokens (two K blocks, the two V blocks of a column).  The tables take 32 KB
 // and a worker 35 to 45 KB: two CTAs of 256 threads with a copy each held four workers' worth of warps, and all eight
 // warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads, with workers 720; 448 and 404 us at
-// 32 x 16384 tokens, 4 x 2 heads, with workers 360).  Registers: 96 with two and four columns, where the compiler spills 60 to 70 bytes
+// 32 x 16384 tokens, 4 x 2 heads, with workers 360; all with the decode loop before the present one, with which the first takes
+// 648).  Registers: 96 with two and four columns, where the compiler spills 60 to 70 bytes
 // per thread (five workers leave no more), 128 without spills with eight.
 constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]
 static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "a workspace for n runs of 256-token tiles holds 2 n partial results");
