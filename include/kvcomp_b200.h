@@ -98,7 +98,7 @@ typedef struct {
 #define KVC_BOOK_OFF_LUT    (KVC_BOOK_OFF_TREE + 2048)    /* (1<<KVC_LUT_BITS) x u32 decode-table entries */
 #define KVC_BOOK_BYTES      (KVC_BOOK_OFF_LUT + 4 * (1 << KVC_LUT_BITS))
 
-typedef struct {             /* first 32 bytes of the blob */
+typedef struct {             /* first 36 bytes of the blob */
     int32_t n_symbols;       /* distinct symbols */
     int32_t min_sym, max_sym;
     int32_t max_len;         /* longest code in bits */
@@ -107,7 +107,10 @@ typedef struct {             /* first 32 bytes of the blob */
     int32_t lut_bits;
     int32_t escape;          /* 1: some decode-table entry holds no complete code (a code longer than the
                               * window, or bit patterns that belong to no code): decoders test for it */
+    uint32_t lone_windows;   /* KVC_LONE_KNOWN | decode-table entries with fewer than two codes: decoders choose their loop
+                              * by it (blobs from before this field hold anything here) */
 } kvc_book_header;
+#define KVC_LONE_KNOWN 0x4b560000u
 
 const char *kvc_last_error(void);
 int kvc_version(void);

@@ -86,73 +86,150 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 // ---- grouped queries (the attention kernel, G >= 2): decode first, multiply on the tensor cores -------
 // With several query heads per KV head the weight records of a position grow to 16 bytes and more, and 32
 // lanes at 32 different positions fetch 0.5 KB and more per lookup: the kernel becomes bound by shared-memory
-// wavefronts.  So a thread first decodes its vector into a private row of bytes in shared memory; then the
-// 32 rows of a warp are a 32 x 128 matrix of unsigned bytes, the weights of up to 8 heads a 128 x 8 matrix of
-// hi bytes and one of lo bytes, and m16n8k32 integer instructions multiply them.  The integer sums are the
-// same as in the one-pass form.  What bounds it is the issue rate: the chains of dependent lookups leave slots empty, and
-// shared memory (tables, slots, rows) limits an SM to 16 or 20 warps.  Against byte stores and four dp4a pairs per word:
-// 1777 -> 1000 shared-memory wavefronts per warp and 256 tokens.  One layer of 16 sequences x 32768 tokens, 8 x 4 heads,
-// rel 0.05 / 0.1: 981 us -> 822 us with the rows in two CTAs of 256 threads -> 735 us with attn_rows_kernel's workers, 720 with
-// the trees out of shared memory and sums in place of ORs.
-// Rows of 36 words: 128 symbols, the overrun of paired lookups, and a 16-byte alignment at which the fragment
-// loads (16 bytes of row 4r+i by lane 4r+q) touch every bank once per quarter warp.
-constexpr int ROW_WORDS = 36;
-static_assert(ROW_WORDS * 4 >= 128 + KVC_DECODE_OVERRUN + 3, "rows too short for paired lookups");
+// wavefronts.  So a warp decodes 32 symbols of each of its 32 vectors into rows of bytes in shared memory (KvcCursor: every lane
+// at the same position), and m16n8k32 integer instructions multiply the rows with the weights: two columns per head, the hi and
+// the lo bytes.  The integer sums are the same as in the one-pass form.  What bounds it: the shared-memory pipe (840 wavefronts per warp
+// and step of 128 tokens, 71 % busy; nine per round of two lookups) and, with 2450 instructions, issue (57 %) together.  One layer of
+// 16 sequences x 32768 tokens, 8 x 4 heads, rel 0.05 / 0.1: whole rows, each lane at its own position, up to three symbols per lookup (3440 instructions,
+// 1010 wavefronts) 650 us, now 536; 32 x 16384 tokens, 10 x 4, rel 0.02 / 0.15, 868 and 828; 8192 tokens of the first, 184 and 154.  Six workers of 80
+// registers are no faster than five of 96; tables of 8 to 12 bits repeated over the banks (32 KB each, one symbol per lookup) 660 us.
 constexpr int WROW = 136;                 // weight words per vector of the one-pass form: 128 positions + zeroed overrun
-__host__ __device__ constexpr int VEC_ROWS_WORDS(int G) { return 2 * G * 32; }     // weight words of one vector: [hi | lo][G][32 groups of 4 positions]
-// word of head g and position group w in the rows form: 16-byte chunks swizzled by the head, so that neither the
-// fragment loads (two heads x four chunks per quarter warp) nor the V phase's stores meet in a bank more than twice
-__device__ __forceinline__ uint32_t w_rows(uint32_t g, uint32_t w) { return g * 32u + (w ^ ((((g & 1u) << 2) | (g >> 1)) << 2)); }
 
-// {hi word, lo word} of 4 consecutive positions (byte i = position i)
-__device__ __forceinline__ uint2 pack4_dense(int q0, int q1, int q2, int q3) {
-    uint2 r;
-    r.x = ((uint32_t)(q0 >> 8) & 0xffu) | (((uint32_t)(q1 >> 8) & 0xffu) << 8) | (((uint32_t)(q2 >> 8) & 0xffu) << 16) | (((uint32_t)(q3 >> 8) & 0xffu) << 24);
-    r.y = ((uint32_t)q0 & 0xffu) | (((uint32_t)q1 & 0xffu) << 8) | (((uint32_t)q2 & 0xffu) << 16) | (((uint32_t)q3 & 0xffu) << 24);
-    return r;
+// Rows of 32 symbols, two units of 16 bytes each, swapped in every other four rows: a quarter warp's stores (eight rows, one unit) and a half
+// warp's loads (four rows, 8 bytes a lane) then meet every bank once.  32 symbols are one k step of the matrix instruction:
+// the rows of a warp take 1 KB instead of 4.5.
+constexpr int ROW_BYTES = 32;
+// A brief launch (a step per worker at most) is a matter of latency: its vectors are decoded whole, with up to three symbols per lookup and no
+// table to be made first, into rows of 128 symbols, the overrun of paired lookups and a 16-byte alignment that spreads over the banks.  (2 columns of
+// 8192 tokens, 4 heads: by pairs 18.2 us, whole 13.4; 12 columns of 2816, 6 heads: 24.8 and 23.2.)
+constexpr int WHOLE_ROW_BYTES = 144;
+static_assert(WHOLE_ROW_BYTES >= 128 + KVC_DECODE_OVERRUN + 3, "rows too short for paired lookups");
+// A vector's weights: two columns per head, the hi and the lo bytes of 4 positions to a word.  Column stride 40 words: the fragment
+// loads (four columns x 32 bytes per half warp) meet every bank once.
+constexpr int COL_WORDS = 40;
+__host__ __device__ constexpr int vec_words(int G) { return 2 * G * COL_WORDS; }
+// 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -32767 .. 127 * 256 + 127
+constexpr float FIX_DOWN = 32767.0f, FIX_UP = 32639.0f;
+constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+__device__ __forceinline__ float exp2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float log2_fast(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rcp_fast(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+
+// {hi word, lo word} of four values times inv, all of them within the range.  The product is rounded by adding 1.5 * 2^23, whose low bits
+// then hold it, and 128 more: byte 1 is the hi byte, byte 0 the lo byte with its sign bit turned.
+__device__ __forceinline__ uint2 pack_fix(float a, float b, float c, float d, float inv) {
+    const uint32_t t0 = __float_as_uint(fmaf(a, inv, 12583040.0f)), t1 = __float_as_uint(fmaf(b, inv, 12583040.0f));
+    const uint32_t t2 = __float_as_uint(fmaf(c, inv, 12583040.0f)), t3 = __float_as_uint(fmaf(d, inv, 12583040.0f));
+    const uint32_t x = __byte_perm(t0, t1, 0x5140), y = __byte_perm(t2, t3, 0x5140);          // {lo0, lo1, hi0, hi1}
+    return make_uint2(__byte_perm(x, y, 0x7632), __byte_perm(x, y, 0x5410) ^ 0x80808080u);
 }
 
-// c += A (16 x 32 unsigned bytes) * B (32 x 8 signed / unsigned bytes)
-__device__ __forceinline__ void mma_us(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+// c += A (16 x 32 unsigned bytes) * B (32 x 8 signed bytes)
+__device__ __forceinline__ void mma_us(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
 }
-__device__ __forceinline__ void mma_uu(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-// decode the thread's vector into its row (shared address, 16-byte aligned)
-__device__ __forceinline__ bool decode_row(uint32_t slot_s, uint32_t byte_pos, uint32_t lut_s, const void *book, bool esc, uint32_t row_s) {
-    const KvcTreeGlobal tree(book);
+// Which of its warp's 32 vectors a lane decodes.  Rows r, r + 8, r + 16 and r + 24 of a warp's matrix end up in the lanes 4 r .. 4 r + 3: with
+// this order they are the vectors 4 r .. 4 r + 3, four neighbouring tokens or channels.
+__device__ __forceinline__ int vec_of_lane(int lane) { return 4 * (lane & 7) + (lane >> 3); }
+
+// Decode a warp's 32 vectors, 32 symbols at a time, and multiply them with the weight columns at shared address w_s.  d[i][j]: vector
+// 4 * (lane >> 2) + i, head (lane & 3) % G + 4 * j.  A lane's two columns of the product are the hi and the lo sums of its head, so they
+// meet without an exchange; which word is which k index is free as long as A and B agree: a lane reads 8 consecutive bytes.
+// (A column of hi bytes per head in one matrix instruction and one of lo bytes in another, the rows whole and decoded with up to three
+// symbols per lookup at places of their own: twice the matrix instructions, twice the values per lane behind them with four heads.)
+template <int G> struct RowsSum {
+    static constexpr int HL = G == 8 ? 2 : 1;                  // heads per lane
+    int c[HL][2][4];
+    __device__ __forceinline__ RowsSum() {
+#pragma unroll
+        for (int j = 0; j < HL; j++)
+#pragma unroll
+            for (int t = 0; t < 2; t++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) c[j][t][i] = 0;
+    }
+    // 32 symbols: get: the lane's place in row lane >> 2; rows lie `stride` bytes apart; col: its place in its weight column
+    __device__ __forceinline__ void add(uint32_t get, uint32_t stride, uint32_t col) {
+        const uint2 a0 = kvc_lds64(get), a1 = kvc_lds64(get + 8 * stride), a2 = kvc_lds64(get + 16 * stride), a3 = kvc_lds64(get + 24 * stride);
+#pragma unroll
+        for (int j = 0; j < HL; j++) {
+            const uint2 bw = kvc_lds64(col + j * (8 * COL_WORDS * 4));
+            mma_us(c[j][0], a0.x, a1.x, a0.y, a1.y, bw);
+            mma_us(c[j][1], a2.x, a3.x, a2.y, a3.y, bw);
+        }
+    }
+    __device__ __forceinline__ void out(int (&d)[4][HL]) const {
+#pragma unroll
+        for (int j = 0; j < HL; j++) {                         // |256 hi + lo| <= 128 * 255 * 32767 < 2^31
+            d[0][j] = 256 * c[j][0][0] + c[j][0][1]; d[1][j] = 256 * c[j][0][2] + c[j][0][3];
+            d[2][j] = 256 * c[j][1][0] + c[j][1][1]; d[3][j] = 256 * c[j][1][2] + c[j][1][3];
+        }
+    }
+};
+// What a vector is decoded from: shared addresses of its slot, the table, the code lengths and the tree
+struct RowsFrom { uint32_t slot, at, lut, len, tree; };
+
+template <int G, int WAY, bool ESC>
+__device__ __forceinline__ bool rows_dot_way(const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL]) {
+    const uint32_t r = lane >> 2, q = lane & 3;
+    const uint32_t put = rows_s + lane * ROW_BYTES + (r & 1u) * 16;
+    const uint32_t get = rows_s + r * ROW_BYTES + (((q >> 1) ^ (r >> 2 & 1u)) * 16) + (q & 1u) * 8;
+    const uint32_t col = w_s + (r % (2 * G)) * (COL_WORDS * 4) + q * 8;
+    KvcCursor at(f.slot, f.at);
+    RowsSum<G> sum;
+    auto word = [&]() { return WAY == KVC_PAIRS ? at.pairs<ESC>(f.lut, f.tree) : at.singles<ESC>(f.lut, f.tree); };
+    if (WAY == KVC_PAIRS) word();
+#pragma unroll 1
+    for (uint32_t ch = 0; ch < 4; ch++) {
+        const uint32_t s0 = at.s, ptr0 = at.ptr, last0 = at.last, behind0 = at.behind;
+#pragma unroll ESC ? 1 : 2
+        for (int u = 0; u < 2; u++) {
+            const uint32_t w0 = word(), w1 = word(), w2 = word(), w3 = word();
+            sts128(u ? put ^ 16u : put, w0, w1, w2, w3);
+        }
+        if (WAY == KVC_PAIRS && __any_sync(0xffffffffu, at.behind >= 24u)) {
+            // a lane that fell more than a word behind: the 32 symbols again, one by one; the others that are behind catch up
+            const bool again = at.behind > 32u;
+            if (again) at.back(s0, ptr0, last0, behind0);
+            at.catch_up<ESC>(f.lut, f.len, f.tree);
+            if (again)
+#pragma unroll 1
+                for (uint32_t k = 0; k < 8; k++) {
+                    asm volatile("st.shared.u32 [%0], %1;" :: "r"((k < 4 ? put : put ^ 16u) + (k & 3u) * 4), "r"(at.last) : "memory");
+                    at.last = at.four<ESC>(f.lut, f.len, f.tree);
+                }
+        }
+        __syncwarp();
+        sum.add(get, ROW_BYTES, col + ch * 32);
+        __syncwarp();
+    }
+    sum.out(d);
+    return at.ok;
+}
+// a vector at a time, each lane at its own place, into whole rows
+template <int G, bool ESC>
+__device__ __forceinline__ bool rows_dot_whole(const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL]) {
+    const uint32_t r = lane >> 2, q = lane & 3;
     KvcRowWriter put;
-    return esc ? kvc_decode_vector<true, 0>(slot_s, byte_pos, lut_s, tree, row_s, put)
-               : kvc_decode_vector<false, 0>(slot_s, byte_pos, lut_s, tree, row_s, put);
+    const bool ok = kvc_decode_vector<ESC, 0>(f.slot, f.at, f.lut, KvcTreeShared{f.tree}, rows_s + lane * WHOLE_ROW_BYTES, put);
+    __syncwarp();
+    RowsSum<G> sum;
+#pragma unroll
+    for (uint32_t ch = 0; ch < 4; ch++) sum.add(rows_s + r * WHOLE_ROW_BYTES + ch * 32 + q * 8, WHOLE_ROW_BYTES, w_s + (r % (2 * G)) * (COL_WORDS * 4) + ch * 32 + q * 8);
+    __syncwarp();
+    sum.out(d);
+    return ok;
 }
-
-// The products of a warp's 32 rows (first one at shared address rows_s) with the weight words at shared address
-// w_s.  d[i][j]: row 4 * (lane >> 2) + i, head (2 * (lane & 3) + j) % G (fewer than 8 heads: the columns repeat).
-// Which row is which row of a fragment and which word is which k index are free as long as A and B agree: a lane
-// then reads 16 consecutive bytes of four neighbouring rows and ends up with four neighbouring rows' sums.
 template <int G>
-__device__ __forceinline__ void rows_dot(uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][2]) {
-    const uint32_t r = lane >> 2, q = lane & 3, g = r % G;
-    int h0[4] = {0, 0, 0, 0}, h1[4] = {0, 0, 0, 0}, l0[4] = {0, 0, 0, 0}, l1[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (uint32_t p = 0; p < 2; p++) {
-        const uint32_t aw = rows_s + (4 * r * ROW_WORDS + 16 * p + 4 * q) * 4, bw = w_s + w_rows(g, 16 * p + 4 * q) * 4;
-        const uint4 a0 = lds128(aw), a1 = lds128(aw + ROW_WORDS * 4), a2 = lds128(aw + ROW_WORDS * 8), a3 = lds128(aw + ROW_WORDS * 12);
-        const uint4 bh = lds128(bw), bl = lds128(bw + G * 32 * 4);
-        mma_us(h0, a0.x, a1.x, a0.y, a1.y, bh.x, bh.y); mma_us(h1, a2.x, a3.x, a2.y, a3.y, bh.x, bh.y);
-        mma_uu(l0, a0.x, a1.x, a0.y, a1.y, bl.x, bl.y); mma_uu(l1, a2.x, a3.x, a2.y, a3.y, bl.x, bl.y);
-        mma_us(h0, a0.z, a1.z, a0.w, a1.w, bh.z, bh.w); mma_us(h1, a2.z, a3.z, a2.w, a3.w, bh.z, bh.w);
-        mma_uu(l0, a0.z, a1.z, a0.w, a1.w, bl.z, bl.w); mma_uu(l1, a2.z, a3.z, a2.w, a3.w, bl.z, bl.w);
-    }
-#pragma unroll
-    for (int j = 0; j < 2; j++) {                              // |256 hi + lo| <= 128 * 255 * 32767 < 2^31
-        d[0][j] = 256 * h0[j] + l0[j]; d[1][j] = 256 * h0[2 + j] + l0[2 + j];
-        d[2][j] = 256 * h1[j] + l1[j]; d[3][j] = 256 * h1[2 + j] + l1[2 + j];
-    }
+__device__ __forceinline__ bool rows_dot(const KvcWay &way, const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL]) {
+    if (way.way == KVC_WHOLE) return way.esc ? rows_dot_whole<G, true>(f, rows_s, w_s, lane, d) : rows_dot_whole<G, false>(f, rows_s, w_s, lane, d);
+    if (!way.esc) return way.way == KVC_PAIRS ? rows_dot_way<G, KVC_PAIRS, false>(f, rows_s, w_s, lane, d) : rows_dot_way<G, KVC_SINGLES, false>(f, rows_s, w_s, lane, d);
+    return way.way == KVC_PAIRS ? rows_dot_way<G, KVC_PAIRS, true>(f, rows_s, w_s, lane, d) : rows_dot_way<G, KVC_SINGLES, true>(f, rows_s, w_s, lane, d);
 }
 
 // Where the hi / lo weight word of position c and head g sits in a vector's 2 * WROW * G words.  One or
@@ -256,6 +333,14 @@ __device__ __forceinline__ unsigned short vec_start_bits(const uint16_t *thread_
     return r;
 }
 
+__device__ __forceinline__ unsigned short vec_start_bits32(const uint16_t *thread_info, uint32_t blk, int v) {
+    return v ? thread_info[(size_t)blk * 64 + (uint32_t)(v - 1)] : (unsigned short)0;
+}
+// unit j of (sequence, head): what kvc_qmeta says, the channel aside
+__device__ __forceinline__ long long unit_of(const kvc_qmeta_dev &m, uint32_t j, int b, int h) {
+    return (long long)((unsigned long long)j * (unsigned long long)m.sj + (unsigned long long)(uint32_t)b * (unsigned long long)m.sb + (unsigned long long)(uint32_t)h * (unsigned long long)m.sh);
+}
+
 // ---- K weights --------------------------------------------------------------------------------------
 // Weight records of the 4 blocks of a 256-token tile: w[sub][c][hi|lo][g], step[sub][g], zp[sub][g].
 // Warp `wp` owns block sub = wp & 3 and the query heads g = (wp >> 2) * GH .. + GH - 1 (GH = G/2, or
@@ -330,33 +415,45 @@ __device__ __forceinline__ void k_weights_build(uint32_t *w, float *step, float 
     }
 }
 
-// The same in the rows form, for block `sub` and the heads part * G/2 .. + G/2 - 1: qh holds the query heads' fp16 bits
-// [G][128]; lane = 4 consecutive channels = one word.
+// The same in columns of bytes, for one block and the heads part * G/2 .. + G/2 - 1: w, step and zp are the block's, q the query heads [G][128],
+// times the scaling; lane = 4 consecutive channels = one word.
 template <int G>
-__device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *zp, const uint16_t *qh, float scaling,
-                                               const KUnit &u, bool channel_units, int min_bytes, int sub, int part, int lane) {
-    float sc[4];
+__device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *zp, const float *q, const KUnit &u, bool channel_units, int min_bytes,
+                                               int part, int lane) {
+    constexpr int GP = G >= 2 ? G / 2 : 1;
+    if (G == 1 && part) return;
+    float sc[4], mz[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++) sc[i] = kvc_scale_value(ku_scale(u, i));
+    for (int i = 0; i < 4; i++) { sc[i] = kvc_scale_value(ku_scale(u, i)); mz[i] = (float)ku_min(u, i, min_bytes) * sc[i]; }
+    float z[GP];
 #pragma unroll
-    for (int gi = 0; gi < G / 2; gi++) {
-        const int g = part * (G / 2) + gi;
-        const uint2 qb = *reinterpret_cast<const uint2 *>(qh + g * 128 + lane * 4);
-        const uint32_t q2[2] = {qb.x, qb.y};
-        float wv[4], z = 0.f;
+    for (int gi = 0; gi < GP; gi++) {
+        const int g = part * (GP) + gi;
+        const float4 x = *reinterpret_cast<const float4 *>(q + g * 128 + lane * 4);
+        const float w0 = x.x * sc[0], w1 = x.y * sc[1], w2 = x.z * sc[2], w3 = x.w * sc[3];
+        z[gi] = fmaf(mz[0], x.x, fmaf(mz[1], x.y, fmaf(mz[2], x.z, mz[3] * x.w)));
+        // The largest value of either sign (floats without a sign order as integers do).  The larger one takes the negative end of the range,
+        // which reaches 32767; the positive end reaches 32639.
+        const float up = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fmaxf(w0, w1), fmaxf(w2, w3)), 0.f)) & 0x7fffffffu));
+        const float down = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fminf(fminf(fminf(w0, w1), fminf(w2, w3)), 0.f)) & 0x7fffffffu));
+        const float big = fmaxf(up, down), st = fmaxf(big * (1.0f / FIX_DOWN), fminf(up, down) * (1.0f / FIX_UP));
+        const float inv = big > 1e-30f ? rcp_fast(st) : 0.f;
+        const uint2 r = pack_fix(w0, w1, w2, w3, up > down ? -inv : inv);
+        w[2 * g * COL_WORDS + lane] = r.x; w[(2 * g + 1) * COL_WORDS + lane] = r.y;
+        if (lane == 0) step[g] = up > down ? -st : st;
+    }
+    if (!channel_units) { if (lane < GP) zp[part * (GP) + lane] = 0.f; return; }
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float q = kvc_scale_value((unsigned short)(q2[i >> 1] >> (16 * (i & 1)))) * scaling;
-            wv[i] = q * sc[i];
-            z = fmaf((float)ku_min(u, i, min_bytes) * sc[i], q, z);
-        }
-        const float mx = kvc_warp_max(fmaxf(fmaxf(fabsf(wv[0]), fabsf(wv[1])), fmaxf(fabsf(wv[2]), fabsf(wv[3]))));
-        z = channel_units ? kvc_warp_sum(z) : 0.f;
-        const float st = fix_step(mx), inv = st > 0.f ? 1.0f / st : 0.f;
-        const uint2 r = pack4_dense(__float2int_rn(wv[0] * inv), __float2int_rn(wv[1] * inv), __float2int_rn(wv[2] * inv), __float2int_rn(wv[3] * inv));
-        uint32_t *vec = w + sub * VEC_ROWS_WORDS(G);
-        vec[w_rows(g, lane)] = r.x; vec[G * 32 + w_rows(g, lane)] = r.y;
-        if (lane == 0) { step[sub * G + g] = st; zp[sub * G + g] = z; }
+    for (int gi = 0; gi < GP; gi += 2) {                    // two heads' sums in one go: one to either half of the warp
+        float a = z[gi];
+        if (GP > 1) {
+            const float z1 = z[(gi + 1) % (GP)];
+            const float give = lane < 16 ? z1 : a;
+            a = (lane < 16 ? a : z1) + __shfl_xor_sync(0xffffffffu, give, 16);
+        } else a += __shfl_xor_sync(0xffffffffu, a, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if ((lane & 15) == 0 && (GP > 1 || lane == 0)) zp[part * (GP) + gi + (lane >> 4)] = a;
     }
 }
 
@@ -573,6 +670,8 @@ struct AttnParams {
     float *ws_part;               // [B*Hq][splits][ROWS_PART_FLOATS]
     int *sched;                   // {items handed out, workers finished}, or null: static shares
     int *status;
+    int workers;                  // per CTA
+    int brief;                    // a step per worker at most: vectors are decoded whole
     int team;                     // without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
     int wait_limit;               // tries of a staging wait before it gives up (KVC_FLAG_WAIT_TIMEOUT)
@@ -582,32 +681,30 @@ struct AttnParams {
 // ---- grouped queries: the same attention with workers of 128 threads --------------------------------
 // A CTA is one resident per SM, with one copy of the two decode tables and up to five (eight heads: four) workers.
 // A worker is four warps with slots, rows, weights and barriers of its own; it draws items and walks them in steps of 128
-// tokens (two K blocks, the two V blocks of a column).  The tables take 32 KB
-// and a worker 35 to 45 KB: two CTAs of 256 threads with a copy each held four workers' worth of warps, and all eight
-// warps of a CTA met at every barrier (822 and 735 us at 16 x 32768 tokens, 8 x 4 heads, with workers 720; 448 and 404 us at
-// 32 x 16384 tokens, 4 x 2 heads, with workers 360; all with the decode loop before the present one, with which the first takes
-// 648).  Registers: 96 with two and four columns, where the compiler spills 60 to 70 bytes
-// per thread (five workers leave no more), 128 without spills with eight.
+// tokens (two K blocks, the two V blocks of a column), with three barriers per step: K's weights are in, the largest score is known, V's
+// weights are in.  Threads beyond the workers that a launch needs help to load the tables.
 constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]
 static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "a workspace for n runs of 256-token tiles holds 2 n partial results");
-template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : (G == 1 ? 7 : 5); }
+template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : 5; }
+constexpr int ROWS_PLANNED = 5;              // workers per SM that the plan of a grouped launch counts
 
 template <int G>
 struct alignas(32) RowsWorker {
-    uint32_t w[2 * VEC_ROWS_WORDS(G)];       // K weight words of the step's two blocks; then V weight words; scratch of the tail
-    float red[4][4 * G];                     // per-warp max, sum, zero-point and weight-max partials
-    unsigned short q[G * 128];               // the query, fp16 bits
+    uint32_t w[3 * vec_words(G)];            // weight words: K of the step's two blocks, V; scratch of the tail and of a team's sums
+    float q[G * 128];                        // the query, times the scaling and log2 e
+    float vsc[128], vz[128], vlg[128];       // of the step's tokens: V's scale, scale * min_int, log2 of the scale
+    float red[G][4];                         // per-warp partials of a head
     float kstep[2 * G], zp[2 * G], qsum[G];
     uint64_t bar[2];                         // K and V staging barriers
     uint32_t leadK[4], leadV[4], nbK[4], nbV[4];   // of the two staged blocks (stage_bulk writes four entries)
     int okK[4], okV[4];
     int next_j, dead;
 };
-struct alignas(32) RowsTables { uint32_t lutK[KVC_LUT_SIZE], lutV[KVC_LUT_SIZE]; };   // the trees, for codes beyond the window, stay in global memory
+struct alignas(32) RowsTables { uint32_t lutK[KVC_LUT_SIZE], lutV[KVC_LUT_SIZE]; uint32_t tree[2][512]; uint8_t len[512]; };   // the trees are for codes beyond the window
 
 // shared memory of a CTA: tables, workers, slots (two of K and two of V each), rows; a corrupt stream's overrun ends in the rows
 template <int G> size_t rows_smem(const AttnParams &p, int workers) {
-    return sizeof(RowsTables) + workers * (sizeof(RowsWorker<G>) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes) + 128 * ROW_WORDS * 4);
+    return sizeof(RowsTables) + workers * (sizeof(RowsWorker<G>) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes) + 128 * (p.brief ? WHOLE_ROW_BYTES : ROW_BYTES));
 }
 
 template <int G> int rows_fit(const AttnParams &p) {         // workers that an SM holds
@@ -652,16 +749,19 @@ template <int G, bool BULK, bool TEAM>
 __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     RowsTables &tab = *reinterpret_cast<RowsTables *>(smem_raw);
-    const int workers = blockDim.x >> 7, wk = threadIdx.x >> 7;
-    const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
+    constexpr int HL = G == 8 ? 2 : 1;                     // heads per lane
+    constexpr int VW = vec_words(G);
+    const int workers = p.workers, wk = threadIdx.x >> 7;      // (threads beyond the workers help to load the tables)
+    const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, sub = warp >> 1;
+    // The lane decodes vector `vec` of the step, and holds the results of the vectors 4 r .. 4 r + 3 of its warp (tokens in the K phase,
+    // channels in the V phase) for the heads q4 % G and, with eight, q4 + 4.
+    const int vec = warp * 32 + vec_of_lane(lane), v = vec & 63;
+    const int r4 = lane & ~3, q4 = lane & 3, hd = q4 % G;
+    const bool own = q4 < G;                               // with two heads the other lanes hold copies
     uint8_t *const wbase = smem_raw + sizeof(RowsTables), *const sbase = wbase + workers * sizeof(RowsWorker<G>);
     RowsWorker<G> &sm = reinterpret_cast<RowsWorker<G> *>(wbase)[wk];
     uint8_t *const slotsK = sbase + wk * 2 * (p.slotK_bytes + p.slotV_bytes), *const slotsV = slotsK + 2 * p.slotK_bytes;
-    const uint32_t rows_s = kvc_smem_addr(sbase + workers * 2 * (p.slotK_bytes + p.slotV_bytes)) + wk * (128 * ROW_WORDS * 4);
-    const uint32_t warp_rows_s = rows_s + warp * (32 * ROW_WORDS * 4), row_s = rows_s + tid * (ROW_WORDS * 4);
-    // the lane's two heads and its four neighbouring rows (tokens in the K phase, channels in the V phase)
-    const int h2 = (2 * (lane & 3)) % G, r4 = lane & ~3;
-    const bool own = 2 * (lane & 3) < G;                   // with fewer than 8 heads the other lanes hold copies
+    const uint32_t rows_s = kvc_smem_addr(sbase + workers * 2 * (p.slotK_bytes + p.slotV_bytes)) + (wk * 4 + warp) * 32 * (p.brief ? WHOLE_ROW_BYTES : ROW_BYTES);
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
     // launched with programmatic stream serialisation: this kernel's own set-up -- the tables, the first blocks, the first step's metadata: cache
     // data that no kernel of a decode step writes -- runs before griddepcontrol.wait, possibly while the kernel ahead of it in the
@@ -699,43 +799,51 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
 
     Item it, nit;
     int j_n1 = draw ? P + me : (int)(p.work * me / P) + 1;
-    bool have = item_of(draw ? me : j_n1 - 1, it), have_next = have && item_of(j_n1, nit);
+    bool have = wk < workers && item_of(draw ? me : j_n1 - 1, it), have_next = have && item_of(j_n1, nit);
     int drawn = 0;                                         // thread 0: the counter's answer, used an item later
     const bool any = have && it.t_lo < it.t_hi;
 
     // the two blocks of a step, by the lanes 0 and 1 of the worker's first warp
     auto stage_K = [&](bool on, int col, int t) { stage_bulk(p.k, on && lane < 2, blkK_of(col, t, lane & 1), slotsK + (lane & 1) * p.slotK_bytes, sm.leadK, sm.okK, sm.nbK, &sm.bar[0], lane, p.starve != 0); };
     auto stage_V = [&](bool on, int col, int t) { stage_bulk(p.v, on && lane < 2, blkV_of(col, t, lane & 1), slotsV + (lane & 1) * p.slotV_bytes, sm.leadV, sm.okV, sm.nbV, &sm.bar[1], lane, p.starve != 0); };
-    if (BULK) {
+    if (BULK && wk < workers) {
         if (tid == 0) { kvc_mbar_init(&sm.bar[0], 1); kvc_mbar_init(&sm.bar[1], 1); kvc_mbar_fence_init(); sm.dead = 0; }
         sync();
         if (warp == 0 && any) { stage_K(true, it.col, it.t_lo); stage_V(true, it.col, it.t_lo); }
     }
-    kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
-    kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
-    const bool escK = book_has_long_codes(p.k.book), escV = book_has_long_codes(p.v.book);
+    const KvcWay wayK = kvc_book_way(p.k.book, p.brief != 0), wayV = kvc_book_way(p.v.book, p.brief != 0);
+    if (p.brief) {
+        kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
+        kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
+    } else kvc_load_ways(tab.lutK, tab.lutV, p.k.book, p.v.book, wayK.way == KVC_PAIRS, wayV.way == KVC_PAIRS, tab.len, threadIdx.x, blockDim.x);
+    if (wayK.esc) kvc_load_tree(tab.tree[0], p.k.book, threadIdx.x, blockDim.x);
+    if (wayV.esc) kvc_load_tree(tab.tree[1], p.v.book, threadIdx.x, blockDim.x);
+    const uint32_t lutK_s = kvc_smem_addr(tab.lutK), lutV_s = kvc_smem_addr(tab.lutV), len_s = kvc_smem_addr(tab.len), tree_s = kvc_smem_addr(tab.tree);
 
     struct StepMeta { unsigned short startK, startV, vsc, ksc; int vmi, kmi; KUnit ku; };   // as loaded: no arithmetic waits on them here
-    auto load_meta = [&](bool on, int col, int step, StepMeta &m) {
-        const long long t = (long long)step * 128 + tid;
-        const int b = col / Hkv, h = col % Hkv;
+    auto load_meta = [&](bool on, int b, int h, int col, int step, StepMeta &m) {
         m.startK = m.startV = 0; m.vsc = 0; m.vmi = m.kmi = 0; m.ksc = 0x3c00;
         m.ku.sc = make_uint2(0x3c003c00u, 0x3c003c00u); m.ku.mi = make_uint2(0u, 0u);          // 1.0, 0
         if (!on) return;
-        m.startK = vec_start_bits(p.k.thread_info, blkK_of(col, step, sub), v);
-        m.startV = vec_start_bits(p.v.thread_info, blkV_of(col, step, sub), v);
-        const long long u = kvc_tok_unit(t, vm.tok_div) * vm.sj + b * vm.sb + h * vm.sh;
+        // (token and block numbers fit 32 bits: the host's check, and the tables' size)
+        m.startK = vec_start_bits32(p.k.thread_info, (uint32_t)(step * 2 + sub) * (uint32_t)cols + (uint32_t)col, v);
+        m.startV = vec_start_bits32(p.v.thread_info, ((uint32_t)step * (uint32_t)cols + (uint32_t)col) * 2u + (uint32_t)sub, v);
+        const uint32_t t = (uint32_t)(step * 128 + vec);
+        const long long u = unit_of(vm, vm.tok_div == 1 ? t : t / (uint32_t)vm.tok_div, b, h);
         m.vsc = kvc_load_scale_bits(vm, u); m.vmi = kvc_load_min(vm, u);
-        if (km.sc == 0) k_token_unit(m.ksc, m.kmi, km, t, b, h);
-        else {                                             // of the block whose weights the warp builds (warp & 1), 4 channels per lane
-            const long long un = kvc_tok_unit((long long)step * 128 + (warp & 1) * 64, km.tok_div) * km.sj + b * km.sb + h * km.sh + lane * 4;
+        if (km.sc == 0) {
+            const long long uk = unit_of(km, km.tok_div == 1 ? t : t / (uint32_t)km.tok_div, b, h);
+            m.ksc = kvc_load_scale_bits(km, uk); m.kmi = kvc_load_min(km, uk);
+        } else {                                           // of the block whose weights the warp builds (warp & 1), 4 channels per lane
+            const uint32_t blk = (uint32_t)(step * 2 + (warp & 1));
+            const long long un = unit_of(km, km.tok_div == 64 ? blk : blk * 64u / (uint32_t)km.tok_div, b, h) + lane * 4;
             m.ku.sc = *reinterpret_cast<const uint2 *>(reinterpret_cast<const unsigned short *>(km.scale) + un);
             if (km.min_bytes == 1) m.ku.mi.x = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const int8_t *>(km.min_int) + un);
             else m.ku.mi = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int16_t *>(km.min_int) + un);
         }
     };
-    StepMeta cur, nxt;
-    load_meta(any, have ? it.col : 0, have ? it.t_lo : 0, cur);
+    StepMeta cur;
+    load_meta(any, have ? it.col / Hkv : 0, have ? it.col % Hkv : 0, have ? it.col : 0, have ? it.t_lo : 0, cur);
     unsigned short qn[G];                                  // the query of an item is fetched while the item before it runs
     auto q_fetch = [&](int col_) {
         const long long row0 = (long long)(col_ / Hkv) * Hq + (long long)(col_ % Hkv) * Gt + p.g0;
@@ -743,160 +851,151 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         for (int g = 0; g < G; g++) qn[g] = g < p.nh ? reinterpret_cast<const unsigned short *>(p.q)[(row0 + g) * 128 + tid] : (unsigned short)0;
     };
     __syncthreads();                                       // the tables are in; from here on the workers go their own ways
+    if (wk >= workers) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (have) q_fetch(it.col);
 
-    // over a warp's tokens: the lane's four, then the eight lanes with the same heads
+    const float qscale = p.scaling * LOG2E;                // scores in units of log 2
+    // over a warp's vectors: the lane's four, then the eight lanes with the same heads
     auto warp_max = [&](float x) { x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4)); x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8)); return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16)); };
     auto warp_sum = [&](float x) { x += __shfl_xor_sync(0xffffffffu, x, 4); x += __shfl_xor_sync(0xffffffffu, x, 8); return x + __shfl_xor_sync(0xffffffffu, x, 16); };
-    auto red_put = [&](int k, const float (&x)[2]) { if (lane < G / 2) *reinterpret_cast<float2 *>(&sm.red[k][warp * G + h2]) = make_float2(x[0], x[1]); };
-    auto red_get = [&](int k, int w4) { return *reinterpret_cast<const float2 *>(&sm.red[k][w4 * G + h2]); };
+    auto red_max = [&](int g) { const float4 x = *reinterpret_cast<const float4 *>(sm.red[g]); return fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)); };
+    auto red_sum = [&](int g) { const float4 x = *reinterpret_cast<const float4 *>(sm.red[g]); return (x.x + x.y) + (x.z + x.w); };
 
     uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
+    bool v_staged = any, v_landed = true;                  // V blocks of the step to come are on their way already; the last wait for them ended well
     while (have) {
     const int col = it.col, b = col / Hkv, h = col % Hkv;
     if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
 #pragma unroll
-    for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = qn[g];
+    for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = kvc_scale_value(qn[g]) * qscale;
     sync();
-    for (int g = warp; g < G; g += 4) {                    // sum of each query head's 128 (scaled) values
+    if (km.sc == 0) for (int g = warp; g < G; g += 4) {    // sum of each query head's 128 (scaled) values
         float a = 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; k++) a += kvc_scale_value(sm.q[g * 128 + k * 32 + lane]) * p.scaling;
+        for (int k = 0; k < 4; k++) a += sm.q[g * 128 + k * 32 + lane];
         a = kvc_warp_sum(a);
         if (lane == 0) sm.qsum[g] = a;
     }
-    float m_run[2], l_run[2], acc[4][2];
+    // acc: the lane's four channels.  l, z: the sums of the weights and of weight * scale * min_int over the lane's own tokens, added up
+    // over the lanes at the item's end.  All relative to 2^m.
+    float m_run[HL], l_run[HL], z_run[HL], acc[4][HL];
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        m_run[j] = -CUDART_INF_F; l_run[j] = 0.f;
+    for (int j = 0; j < HL; j++) {
+        m_run[j] = -CUDART_INF_F; l_run[j] = z_run[j] = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; i++) acc[i][j] = 0.f;
     }
 
     for (int step = it.t_lo; step < it.t_hi; step++) {
-        bool n_on = true; int n_col = col, n_step = step + 1;      // the worker's next step (it may open the next column)
-        if (n_step >= it.t_hi) {
-            n_on = have_next && nit.t_lo < nit.t_hi; n_col = n_on ? nit.col : col; n_step = n_on ? nit.t_lo : 0;
-            if (have_next) q_fetch(nit.col);
-        }
         if (!BULK) {
+            if (step != it.t_lo) sync();                   // every thread is done with the V slots
+            const int sb = tid >> 6, sv = tid & 63;
             uint32_t ld, nb;
-            bool ok = stage(p.k, blkK_of(col, step, sub), slotsK + sub * p.slotK_bytes, &ld, &nb, v);
-            if (v == 0) { sm.leadK[sub] = ld; sm.nbK[sub] = nb; sm.okK[sub] = ok; }
-            ok = stage(p.v, blkV_of(col, step, sub), slotsV + sub * p.slotV_bytes, &ld, &nb, v);
-            if (v == 0) { sm.leadV[sub] = ld; sm.nbV[sub] = nb; sm.okV[sub] = ok; }
+            bool ok = stage(p.k, blkK_of(col, step, sb), slotsK + sb * p.slotK_bytes, &ld, &nb, sv);
+            if (sv == 0) { sm.leadK[sb] = ld; sm.nbK[sb] = nb; sm.okK[sb] = ok; }
+            ok = stage(p.v, blkV_of(col, step, sb), slotsV + sb * p.slotV_bytes, &ld, &nb, sv);
+            if (sv == 0) { sm.leadV[sb] = ld; sm.nbV[sb] = nb; sm.okV[sb] = ok; }
         }
-        k_weights_rows<G>(sm.w, sm.kstep, sm.zp, sm.q, p.scaling, cur.ku, km.sc != 0, km.min_bytes, warp & 1, warp >> 1, lane);
+        k_weights_rows<G>(sm.w + (warp & 1) * VW, sm.kstep + (warp & 1) * G, sm.zp + (warp & 1) * G, sm.q, cur.ku, km.sc != 0, km.min_bytes, warp >> 1, lane);
+        {
+            const float sc = kvc_scale_value(cur.vsc);     // of the token `vec`; read by lanes of the same warp
+            sm.vsc[vec] = sc; sm.vz[vec] = sc * (float)cur.vmi; // (at least fp16's smallest; a negative scale's weights take the shorter end of the fixed-point range)
+            sm.vlg[vec] = log2_fast(fmaxf(fabsf(sc), 5.9604645e-8f)) + (sc < 0.f ? 0.006f : 0.f);
+        }
         bool k_landed = true;                              // (a wait that runs out: see attn_one_kernel)
         if (BULK) {
             k_landed = kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit);
             if (k_landed) par ^= 1u; else flags |= KVC_FLAG_WAIT_TIMEOUT;
         }
-        sync();
-        // ---- K: scores of this step's tokens
-        float s[4][2];
-        {
-            bool ok = k_landed && sm.okK[sub] && (uint32_t)(cur.startK >> 3) < sm.nbK[sub];      // a vector begins inside its block
-            if (ok) ok = decode_row(kvc_smem_addr(slotsK + sub * p.slotK_bytes), sm.leadK[sub] + (cur.startK >> 3), kvc_smem_addr(tab.lutK), p.k.book, escK, row_s);
-            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
-            __syncwarp();
-            int d[4][2];
-            rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w + sub * VEC_ROWS_WORDS(G)), lane, d);
-            const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the thread's own token
-            const float2 st = *reinterpret_cast<const float2 *>(&sm.kstep[sub * G + h2]), z = *reinterpret_cast<const float2 *>(&sm.zp[sub * G + h2]);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                s[i][0] = st.x * (float)d[i][0]; s[i][1] = st.y * (float)d[i][1];
-                if (km.sc != 0) { s[i][0] += z.x; s[i][1] += z.y; }
-                else {
-                    const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
-                    const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
-                    s[i][0] = sc * fmaf(mi, sm.qsum[h2], s[i][0]); s[i][1] = sc * fmaf(mi, sm.qsum[h2 + 1], s[i][1]);
-                }
-            }
-        }
-        // ---- online softmax over the step
-        float t1[2];
-#pragma unroll
-        for (int j = 0; j < 2; j++) t1[j] = warp_max(fmaxf(fmaxf(s[0][j], s[1][j]), fmaxf(s[2][j], s[3][j])));
-        red_put(0, t1);
-        sync();                                            // also: every thread is done with the K slots and weights
-        load_meta(n_on, n_col, n_step, nxt);               // in flight during the V phase, first touched in the next step
-        if (BULK && warp == 0) {                           // the next step's K blocks land during the V phase
-            if (__all_sync(0xffffffffu, k_landed)) stage_K(n_on, n_col, n_step);
+        sync();                                            // also: every thread is done with the V slots of the step before
+        if (BULK && warp == 0 && !v_staged) {              // this step's V blocks land during its K phase
+            if (__all_sync(0xffffffffu, v_landed)) stage_V(true, col, step);
             else if (lane == 0) sm.dead = 1;
         }
-        float alpha[2], vst[2];
+        // ---- K: scores of this step's tokens
+        float s[4][HL];
         {
-            const float2 x0 = red_get(0, 0), x1 = red_get(0, 1), x2 = red_get(0, 2), x3 = red_get(0, 3);
-            t1[0] = fmaxf(fmaxf(x0.x, x1.x), fmaxf(x2.x, x3.x)); t1[1] = fmaxf(fmaxf(x0.y, x1.y), fmaxf(x2.y, x3.y));
-        }
+            int d[4][HL];
+            const uint32_t start = cur.startK >> 3;
+            bool ok = k_landed && sm.okK[sub] && start < sm.nbK[sub];              // a vector begins inside its block
+            ok = rows_dot<G>(wayK, {kvc_smem_addr(slotsK + sub * p.slotK_bytes), ok ? sm.leadK[sub] + start : 1u, lutK_s, len_s, tree_s}, rows_s, kvc_smem_addr(sm.w + sub * VW), lane, d) && ok;
+            if (!ok) flags |= KVC_FLAG_BAD_STREAM;
+            const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the token `vec`
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const float m_new = fmaxf(m_run[j], t1[j]);
-            alpha[j] = __expf(m_run[j] - m_new);           // exp(-inf) = 0 on the first step
-            m_run[j] = m_new;
-        }
-        {
-            float ssum[2] = {0.f, 0.f}, zsum[2] = {0.f, 0.f}, wmax[2] = {0.f, 0.f};
-            const uint32_t unit = (uint32_t)cur.vsc | ((uint32_t)cur.vmi << 16);
+            for (int j = 0; j < HL; j++) {
+                const float st = sm.kstep[sub * G + hd + 4 * j], z = sm.zp[sub * G + hd + 4 * j];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t u = __shfl_sync(0xffffffffu, unit, r4 + i);
-                const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
+                for (int i = 0; i < 4; i++) s[i][j] = fmaf(st, (float)d[i][j], z);
+            }
+            if (km.sc == 0) {
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const float pr = __expf(s[i][j] - m_run[j]);
-                    s[i][j] = pr * sc;                     // from here on the token's V weight
-                    ssum[j] += pr; zsum[j] = fmaf(s[i][j], mi, zsum[j]); wmax[j] = fmaxf(wmax[j], fabsf(s[i][j]));
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t u = __shfl_sync(0xffffffffu, unit, (lane >> 2) + 8 * i);
+                    const float sc = kvc_scale_value((unsigned short)u), mi = (float)((int)u >> 16);
+#pragma unroll
+                    for (int j = 0; j < HL; j++) s[i][j] = sc * fmaf(mi, sm.qsum[hd + 4 * j], s[i][j]);
                 }
             }
-#pragma unroll
-            for (int j = 0; j < 2; j++) { ssum[j] = warp_sum(ssum[j]); zsum[j] = warp_sum(zsum[j]); wmax[j] = warp_max(wmax[j]); }
-            red_put(1, ssum); red_put(2, zsum); red_put(3, wmax);
         }
-        sync();
-        // the V weights' words: the lane's four tokens are one word of each of its heads (the K weights are spent)
+        // ---- online softmax over the step.  The reference of a step is the largest of weight * V scale over its tokens, i.e. of score + log2 of
+        // the scale: the V weights are then at most 1, and their fixed-point step is known without another exchange.
+        const float4 lg = *reinterpret_cast<const float4 *>(&sm.vlg[warp * 32 + r4]);
+#pragma unroll
+        for (int j = 0; j < HL; j++) {
+            const float x = warp_max(fmaxf(fmaxf(s[0][j] + lg.x, s[1][j] + lg.y), fmaxf(s[2][j] + lg.z, s[3][j] + lg.w)));
+            if (lane < 4 && own) sm.red[hd + 4 * j][warp] = x;
+        }
+        sync();                                            // also: every thread is done with the K slots and weights
+        const uint32_t startV = cur.startV >> 3;
         {
-            const float2 x0 = red_get(3, 0), x1 = red_get(3, 1), x2 = red_get(3, 2), x3 = red_get(3, 3);
-            t1[0] = fmaxf(fmaxf(x0.x, x1.x), fmaxf(x2.x, x3.x)); t1[1] = fmaxf(fmaxf(x0.y, x1.y), fmaxf(x2.y, x3.y));
+            bool n_on = true; int nb = b, nh = h, n_col = col, n_step = step + 1;      // the worker's next step (it may open the next column)
+            if (n_step >= it.t_hi) {
+                n_on = have_next && nit.t_lo < nit.t_hi;
+                if (n_on) { n_col = nit.col; n_step = nit.t_lo; nb = n_col / Hkv; nh = n_col % Hkv; }
+                if (have_next) q_fetch(nit.col);
+            }
+            // (its V units, on their way during the V phase, are first touched when it begins; this step's lie in shared memory)
+            load_meta(n_on, nb, nh, n_col, n_step, cur);
+            if (BULK && warp == 0) {                       // its K blocks land during the V phase
+                if (__all_sync(0xffffffffu, k_landed)) stage_K(n_on, n_col, n_step);
+                else if (lane == 0) sm.dead = 1;
+            }
         }
+        float alpha[HL], beta[HL];
+        {
+            const float4 sc = *reinterpret_cast<const float4 *>(&sm.vsc[warp * 32 + r4]), vz = *reinterpret_cast<const float4 *>(&sm.vz[warp * 32 + r4]);
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            vst[j] = fix_step(t1[j]);
-            const float inv = vst[j] > 0.f ? 1.0f / vst[j] : 0.f;
-            const uint2 w2 = pack4_dense(__float2int_rn(s[0][j] * inv), __float2int_rn(s[1][j] * inv), __float2int_rn(s[2][j] * inv), __float2int_rn(s[3][j] * inv));
-            const uint32_t at = w_rows(h2 + j, warp * 8 + (lane >> 2));
-            if (own) { sm.w[at] = w2.x; sm.w[G * 32 + at] = w2.y; }
+            for (int j = 0; j < HL; j++) {
+                const float u = red_max(hd + 4 * j), m_new = fmaxf(m_run[j], u);
+                alpha[j] = exp2_fast(m_run[j] - m_new); beta[j] = exp2_fast(u - m_new);       // exp(-inf) = 0 on the first step
+                m_run[j] = m_new;
+                const float p0 = exp2_fast(s[0][j] - u), p1 = exp2_fast(s[1][j] - u), p2 = exp2_fast(s[2][j] - u), p3 = exp2_fast(s[3][j] - u);
+                l_run[j] = fmaf(l_run[j], alpha[j], beta[j] * ((p0 + p1) + (p2 + p3)));
+                z_run[j] = fmaf(z_run[j], alpha[j], beta[j] * fmaf(p0, vz.x, fmaf(p1, vz.y, fmaf(p2, vz.z, p3 * vz.w))));
+                beta[j] *= -1.0f / FIX_DOWN;
+                // the lane's four tokens are one word of its head
+                const uint2 w2 = pack_fix(p0 * sc.x, p1 * sc.y, p2 * sc.z, p3 * sc.w, -FIX_DOWN);
+                uint32_t *at = sm.w + 2 * VW + 2 * (hd + 4 * j) * COL_WORDS + warp * 8 + (lane >> 2);
+                if (own) { at[0] = w2.x; at[COL_WORDS] = w2.y; }
+            }
         }
-        const bool v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
+        v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
         if (BULK && v_landed) par ^= 2u;
         if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        v_staged = false;
         sync();
         // ---- V: this step's contribution to the lane's four channels
         {
-            bool ok = v_landed && sm.okV[sub] && (uint32_t)(cur.startV >> 3) < sm.nbV[sub];
-            if (ok) ok = decode_row(kvc_smem_addr(slotsV + sub * p.slotV_bytes), sm.leadV[sub] + (cur.startV >> 3), kvc_smem_addr(tab.lutV), p.v.book, escV, row_s);
+            int d[4][HL];
+            bool ok = v_landed && sm.okV[sub] && startV < sm.nbV[sub];
+            ok = rows_dot<G>(wayV, {kvc_smem_addr(slotsV + sub * p.slotV_bytes), ok ? sm.leadV[sub] + startV : 1u, lutV_s, len_s + 256u, tree_s + 2048u}, rows_s, kvc_smem_addr(sm.w + 2 * VW), lane, d) && ok;
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
-            __syncwarp();
-            int d[4][2];
-            rows_dot<G>(warp_rows_s, kvc_smem_addr(sm.w), lane, d);
-            const float2 s0 = red_get(1, 0), s1 = red_get(1, 1), s2 = red_get(1, 2), s3 = red_get(1, 3);
-            l_run[0] = l_run[0] * alpha[0] + ((s0.x + s1.x) + (s2.x + s3.x)); l_run[1] = l_run[1] * alpha[1] + ((s0.y + s1.y) + (s2.y + s3.y));
-            const float2 z0 = red_get(2, 0), z1 = red_get(2, 1), z2 = red_get(2, 2), z3 = red_get(2, 3);
-            const float z[2] = {(z0.x + z1.x) + (z2.x + z3.x), (z0.y + z1.y) + (z2.y + z3.y)};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 2; j++) acc[i][j] = fmaf(acc[i][j], alpha[j], fmaf(vst[j], (float)d[i][j], z[j]));
+                for (int j = 0; j < HL; j++) acc[i][j] = fmaf(acc[i][j], alpha[j], beta[j] * (float)d[i][j]);
         }
-        sync();                                            // every thread is done with the V slots, weights and sums
-        if (BULK && warp == 0) {                           // the next step's V blocks land during its K phase
-            if (__all_sync(0xffffffffu, v_landed)) stage_V(n_on, n_col, n_step);
-            else if (lane == 0) sm.dead = 1;
-        }
-        cur = nxt;
     }
 
     // ---- uncompressed tail, only for callers without a workspace: otherwise the merge kernel adds it
@@ -917,33 +1016,29 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
 #pragma unroll
                     for (int k = 0; k < 8; k++)
 #pragma unroll
-                        for (int g = 0; g < G; g++) s[g] = fmaf(__half2float(kh[k]), kvc_scale_value(sm.q[g * 128 + c8 * 8 + k]) * p.scaling, s[g]);
+                        for (int g = 0; g < G; g++) s[g] = fmaf(__half2float(kh[k]), sm.q[g * 128 + c8 * 8 + k], s[g]);
                 }
             }
 #pragma unroll
-            for (int g = 0; g < G; g++) { const float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[0][warp * G + g] = mx; }
+            for (int g = 0; g < G; g++) { const float mx = kvc_warp_max(s[g]); if (lane == 0) sm.red[g][warp] = mx; }
             sync();
-            float alpha[2], dv[4][2];
-            {
-                const float2 x0 = red_get(0, 0), x1 = red_get(0, 1), x2 = red_get(0, 2), x3 = red_get(0, 3);
-                const float mt[2] = {fmaxf(fmaxf(x0.x, x1.x), fmaxf(x2.x, x3.x)), fmaxf(fmaxf(x0.y, x1.y), fmaxf(x2.y, x3.y))};
+            float alpha[HL], dv[4][HL];
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const float m_new = fmaxf(m_run[j], mt[j]);
-                    alpha[j] = __expf(m_run[j] - m_new);
-                    m_run[j] = m_new;
-                    if (tid < 4) sm.red[3][h2 + j] = m_new;
+            for (int j = 0; j < HL; j++) {
+                const float m_new = fmaxf(m_run[j], red_max(hd + 4 * j));
+                alpha[j] = exp2_fast(m_run[j] - m_new);
+                m_run[j] = m_new;
+                if (tid < 4) sm.zp[hd + 4 * j] = m_new;
 #pragma unroll
-                    for (int i = 0; i < 4; i++) dv[i][j] = 0.f;
-                }
+                for (int i = 0; i < 4; i++) dv[i][j] = 0.f;
             }
             sync();
 #pragma unroll
             for (int g = 0; g < G; g++) {
-                const float pr = act ? __expf(s[g] - sm.red[3][g]) : 0.f;
+                const float pr = act ? exp2_fast(s[g] - sm.zp[g]) : 0.f;
                 pt[tid * G + g] = pr;
                 const float ssum = kvc_warp_sum(pr);
-                if (lane == 0) sm.red[1][warp * G + g] = ssum;
+                if (lane == 0) sm.red[g][warp] = ssum;
             }
             sync();
             const int n_here = (int)min(128ll, p.Tr - r0);
@@ -952,38 +1047,54 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
 #pragma unroll
                 for (int c = 0; c < 4; c++)
 #pragma unroll
-                    for (int j = 0; j < 2; j++) dv[c][j] = fmaf(pt[i * G + h2 + j], __half2float(vr[c]), dv[c][j]);
+                    for (int j = 0; j < HL; j++) dv[c][j] = fmaf(pt[i * G + hd + 4 * j], __half2float(vr[c]), dv[c][j]);
             }
-            const float2 s0 = red_get(1, 0), s1 = red_get(1, 1), s2 = red_get(1, 2), s3 = red_get(1, 3);
-            l_run[0] = l_run[0] * alpha[0] + ((s0.x + s1.x) + (s2.x + s3.x)); l_run[1] = l_run[1] * alpha[1] + ((s0.y + s1.y) + (s2.y + s3.y));
 #pragma unroll
-            for (int j = 0; j < 2; j++)
+            for (int j = 0; j < HL; j++) {
+                z_run[j] *= alpha[j];
+                l_run[j] = fmaf(l_run[j], alpha[j], warp == 0 && r4 == 0 ? red_sum(hd + 4 * j) : 0.f);      // one of the lanes that are added up
 #pragma unroll
                 for (int c = 0; c < 4; c++) acc[c][j] = fmaf(acc[c][j], alpha[j], dv[c][j]);
+            }
         }
     }
     if (it.t_lo >= it.t_hi && have_next) q_fetch(nit.col);     // an item without steps fetched nothing yet
+    // the sums over the worker's tokens
+    sync();                                                // (the tail's scratch and the last maxima are read)
+#pragma unroll
+    for (int j = 0; j < HL; j++) {
+        const float l = warp_sum(l_run[j]), z = warp_sum(z_run[j]);
+        if (lane < 4 && own) { sm.red[hd + 4 * j][warp] = l; sm.w[(hd + 4 * j) * 4 + warp] = __float_as_uint(z); }
+    }
+    sync();
+#pragma unroll
+    for (int j = 0; j < HL; j++) {
+        l_run[j] = red_sum(hd + 4 * j);
+        const float4 z = *reinterpret_cast<const float4 *>(&sm.w[(hd + 4 * j) * 4]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[i][j] += (z.x + z.y) + (z.z + z.w);
+    }
     const long long head0 = (long long)b * Hq + (long long)h * Gt + p.g0;
     bool dead;
     if constexpr (TEAM) {                                  // each worker's share to its own shared memory, then a head per worker
         const int team = p.team, tm = wk / team, tk = wk % team;      // the worker's team and its place there
-        auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" :: "r"(rows_workers<2>() + 1 + tm), "r"(team * 128) : "memory"); };
-        sync();                                            // (the tail's scratch is read)
+        auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" :: "r"(rows_workers<G>() + 1 + tm), "r"(team * 128) : "memory"); };
+        sync();                                            // (the sums are read)
         float *mine = reinterpret_cast<float *>(sm.w);     // acc[G][128]
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
+        for (int j = 0; j < HL; j++) {
             if (!own) continue;
-            *reinterpret_cast<float4 *>(mine + (h2 + j) * 128 + warp * 32 + r4) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
-            if (warp == 0 && lane < 4) { sm.red[0][h2 + j] = m_run[j]; sm.red[1][h2 + j] = l_run[j]; }
+            *reinterpret_cast<float4 *>(mine + (hd + 4 * j) * 128 + warp * 32 + r4) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+            if (warp == 0 && lane < 4) { sm.red[hd + 4 * j][0] = m_run[j]; sm.red[hd + 4 * j][1] = l_run[j]; }
         }
         team_sync();
         const RowsWorker<G> *mates = &sm - tk;
         for (int g = tk; g < p.nh; g += team) {
             float M = -CUDART_INF_F, O = 0.f, L = 0.f;
-            for (int w = 0; w < team; w++) M = fmaxf(M, mates[w].red[0][g]);
+            for (int w = 0; w < team; w++) M = fmaxf(M, mates[w].red[g][0]);
             for (int w = 0; w < team; w++) {
-                const float m = mates[w].red[0][g], e = m == -CUDART_INF_F ? 0.f : __expf(m - M);     // a worker without tokens adds nothing
-                L = fmaf(mates[w].red[1][g], e, L);
+                const float m = mates[w].red[g][0], e = m == -CUDART_INF_F ? 0.f : exp2_fast(m - M);     // a worker without tokens adds nothing
+                L = fmaf(mates[w].red[g][1], e, L);
                 O = fmaf(reinterpret_cast<const float *>(mates[w].w)[g * 128 + tid], e, O);
             }
             p.out[(head0 + g) * 128 + tid] = __float2half_rn(O / L);
@@ -993,20 +1104,20 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         team_sync();
     } else {
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        if (!own || h2 + j >= p.nh) continue;
+    for (int j = 0; j < HL; j++) {
+        if (!own || hd + 4 * j >= p.nh) continue;
         if (!p.partial) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) p.out[(head0 + h2 + j) * 128 + warp * 32 + r4 + i] = __float2half_rn(acc[i][j] / l_run[j]);
+            for (int i = 0; i < 4; i++) p.out[(head0 + hd + 4 * j) * 128 + warp * 32 + r4 + i] = __float2half_rn(acc[i][j] / l_run[j]);
         } else {
-            float *dst = p.ws_part + ((head0 + h2 + j) * p.splits + it.part) * ROWS_PART_FLOATS;     // 8-byte aligned
+            float *dst = p.ws_part + ((head0 + hd + 4 * j) * p.splits + it.part) * ROWS_PART_FLOATS;     // 8-byte aligned
             *reinterpret_cast<float2 *>(dst + 2 + warp * 32 + r4) = make_float2(acc[0][j], acc[1][j]);
             *reinterpret_cast<float2 *>(dst + 4 + warp * 32 + r4) = make_float2(acc[2][j], acc[3][j]);
-            if (warp == 0 && lane < 4) { dst[0] = m_run[j]; dst[1] = l_run[j]; }
+            if (warp == 0 && lane < 4) { dst[0] = m_run[j] * LN2; dst[1] = l_run[j]; }        // the merge kernel counts in powers of e
         }
     }
     if (draw && tid == 0) sm.next_j = drawn;
-    sync();                                                // the tail's scratch is read before the next column's weights overwrite it
+    sync();                                                // the sums are read before the next column's weights overwrite them
     dead = BULK && sm.dead != 0;
     }
     if (dead) break;                                       // a staging wait ran out: the status word says so, the item's result is void
@@ -1014,10 +1125,10 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     it = nit; have = have_next; j_n1 = j_n2;
     have_next = have && item_of(j_n1, nit);
     }   // items of the worker
-    if (BULK && any) {                    // the copies issued after the last step are empty, but their phase must end;
+    if (BULK && any) {                    // the copy of K issued after the last step is empty, but its phase must end;
         // after a wait that ran out, these are the phases still open: nothing may be in flight at the return
         if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
-        if (!kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        if ((v_staged || !v_landed) && !kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
     }
     if (flags) atomicOr(p.status, flags);
     if (draw && tid == 0) {               // the last worker to finish leaves the scheduling counters zeroed for the next launch
@@ -1031,7 +1142,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
 // (decode_dot), so there are no rows, and an SM holds one copy of the tables and up to ONE_WORKERS workers: 28 warps of 72
 // registers where three CTAs of 256 threads with tables of their own, all eight warps at every barrier, were 24.  8 x 32 columns of
 // 4096 tokens, rel 0.05 / 0.1: 135 us, now 128.  (Eight workers of 64 registers, 52 bytes of spills: 145, with runs of other lengths 134.)
-constexpr int ONE_WORKERS = rows_workers<1>();
+constexpr int ONE_WORKERS = 7;
 
 struct alignas(32) OneWorker {
     uint32_t w[2 * 2 * WROW];                // K weight records of the step's two blocks; scratch of the tail
@@ -1747,7 +1858,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.out = reinterpret_cast<__half *>(out);
     p.scaling = scaling; p.splits = splits; p.tiles_per_split = tps; p.long_runs = long_runs; p.short_tiles = short_tiles;
     p.n_tiles = (int)n_tiles;
-    p.team = 0;
+    p.team = p.brief = 0;
     p.work = cols * splits;
     // with a workspace the CTAs draw their items from its counters (zero before the first launch, left zeroed)
     const bool have_ws = workspace && workspace_bytes >= ATTN_COUNTER_BYTES && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
@@ -1780,7 +1891,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             // (with grouped queries the plan counts five workers per SM also where the launch has fewer: the items are finer for it.  8 heads, four
             // workers: 16 x 8 columns of 16384 tokens 412 us, with a plan for four 423; 32 x 2 columns 217 and 224.  Three workers, as the
             // stream's largest block is unknown: 484 and 490 us, but 16 x 8 columns of 4096 tokens 144 and 137.)
-            if (asked <= 0) r = plan_runs(p.n_tiles, cols, heads == 1 ? most : (long long)rows_workers<4>() * sms);
+            if (asked <= 0) r = plan_runs(p.n_tiles, cols, heads == 1 ? most : (long long)ROWS_PLANNED * sms);
             // The caller's runs in halves where that is fewer steps one after the other: a worker takes a run's steps in turn, each
             // with 128 threads.  (32 columns, 2 heads each, 2048 tokens in 4
             // runs: 46.9 us, in halves 33.7; 64 columns in 8 runs: 36.0, in halves 42.2, as the halves no longer go in one round.)
@@ -1800,6 +1911,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
 #define KVC_AT(GG)                                                                                              \
     {                                                                                                           \
+        p.brief = 0;                                                                                            \
         int workers = rows_fit(p, GG);                                                                          \
         /* (with a tail and columns for all workers a pass of the tail is no step: 1023 columns of 2048 tokens and 64 rows, 4 heads, */ \
         /* a worker per column 464 us, teams as chosen for 18 steps 551) */                                     \
@@ -1807,16 +1919,20 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         if (p.team) workers = p.team * (int)spread(cols, workers / p.team, sms).per_sm;                         \
         /* (short runs at the end of the columns fill the last round up; a single round spreads over all SMs) */ \
         else if (const Spread s = spread(p.work, workers, sms); p.long_runs == splits || s.rounds == 1) workers = (int)s.per_sm; \
+        p.brief = GG > 1 && cols * (long long)p.n_tiles <= (long long)workers * sms;                              \
+        if (p.brief && attn_smem<GG>(p, workers) > MAX_CTA_SHARED) p.brief = 0;                                 \
         const size_t smem = attn_smem<GG>(p, workers);                                                          \
+        p.workers = workers;                                                                                    \
+        const int threads = 128 * (GG == 1 ? workers : rows_workers<GG>());                                     \
         static kvc_launch_slot slots[4];                                                                        \
         auto *kernel = p.team ? (bulk ? attn_kernel<GG, true, true>() : attn_kernel<GG, false, true>())         \
                               : (bulk ? attn_kernel<GG, true, false>() : attn_kernel<GG, false, false>());      \
         int occ = 0;                                                                                            \
-        if (int rc = kvc_prepare(slots[2 * (p.team != 0) + bulk], reinterpret_cast<const void *>(kernel), 128 * workers, smem, &occ)) return rc; \
+        if (int rc = kvc_prepare(slots[2 * (p.team != 0) + bulk], reinterpret_cast<const void *>(kernel), threads, smem, &occ)) return rc; \
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);             \
         long long ctas = p.team ? p.work : (p.work + workers - 1) / workers;                                    \
         if (ctas > sms) ctas = sms;                                                                             \
-        if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(128 * workers), smem, kvc_cu(stream), p)) return rc; \
+        if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(threads), smem, kvc_cu(stream), p)) return rc; \
     }
             if (p.nh > 4) KVC_AT(8) else if (p.nh > 2) KVC_AT(4) else if (p.nh > 1) KVC_AT(2) else KVC_AT(1)
 #undef KVC_AT

@@ -188,7 +188,7 @@ struct BookSmem {
     uint32_t enc_code[256], enc_len[256];
     uint32_t tree[512];          // wide tree: lo16 = child0 (or LEAF), hi16 = child1 (or symbol)
     long long count[256];        // the histogram, fetched by all threads at once
-    int n_nodes, n_symbols, min_sym, max_sym, max_len, flags;
+    int n_nodes, n_symbols, min_sym, max_sym, max_len, flags, lone;
 };
 
 // Exclusive prefix sum of x over the CTA's first 256 threads (the others pass 0); *total receives the sum.
@@ -311,7 +311,7 @@ __device__ uint32_t lut_entry(const uint32_t *tree, uint32_t w) {
     return (idx < 0 ? (uint32_t)KVC_TREE_NONE : (uint32_t)idx) << 8;
 }
 
-__device__ void write_book(const BookSmem &s, uint8_t *book, int tid, int nthr) {
+__device__ void write_book(BookSmem &s, uint8_t *book, int tid, int nthr) {
     uint32_t *enc = reinterpret_cast<uint32_t *>(book + KVC_BOOK_OFF_ENC);
     for (int i = tid; i < 256; i += nthr) { enc[2 * i] = s.enc_code[i]; enc[2 * i + 1] = s.enc_len[i]; }
     // reference-format tree: {u8 is_leaf, i8 a, i8 b}; indices and symbols narrowed to 8 bits as
@@ -333,17 +333,22 @@ __device__ void write_book(const BookSmem &s, uint8_t *book, int tid, int nthr) 
     uint32_t *wt = reinterpret_cast<uint32_t *>(book + KVC_BOOK_OFF_TREE);
     for (int i = tid; i < 512; i += nthr) wt[i] = s.tree[i];
     uint32_t *lut = reinterpret_cast<uint32_t *>(book + KVC_BOOK_OFF_LUT);
-    int no_code = 0;                                        // an entry whose window holds no complete code
+    int no_code = 0, lone = 0;                              // entries whose window holds no complete code, fewer than two of them
+    if (tid == 0) s.lone = 0;
     for (int w = tid; w < KVC_LUT_SIZE; w += nthr) {
         const uint32_t e = lut_entry(s.tree, (uint32_t)w);
         lut[w] = e;
         no_code |= (e & 0xffu) == 0;
+        lone += (e & 0x80u) == 0;
     }
     no_code = __syncthreads_or(no_code);
+    if (lone) atomicAdd(&s.lone, lone);
+    __syncthreads();
     if (tid == 0) {
         kvc_book_header *h = reinterpret_cast<kvc_book_header *>(book);
         h->n_symbols = s.n_symbols; h->min_sym = s.min_sym; h->max_sym = s.max_sym; h->max_len = s.max_len;
         h->n_nodes = s.n_nodes; h->flags = s.flags; h->lut_bits = KVC_LUT_BITS; h->escape = no_code ? 1 : 0;
+        h->lone_windows = KVC_LONE_KNOWN | (uint32_t)s.lone;
     }
 }
 

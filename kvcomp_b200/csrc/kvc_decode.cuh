@@ -239,3 +239,159 @@ struct KvcRowWriter {
         cur = left ? over : w;
     }
 };
+
+// ---- all lanes of a warp at the same position -----------------------------------------------------------
+// The loop above takes what a window holds, one to three symbols, and every lane is at a position of its own.  A consumer that
+// multiplies whole words of symbols on the tensor cores wants the opposite: every lane four symbols at a time.  With a fixed number of symbols per lookup
+// no position is kept and no end tested; words are put together by byte permutations and go to places known when the kernel is compiled.
+//   PAIRS    two symbols per lookup, four per round.  Where few windows hold one code only (two codes at the ends of a bell curve), a lane that meets
+//            one falls a symbol behind, up to four: words leave a round late, shifted by what the lane is behind, and every 32 symbols
+//            the lanes catch up if one is three or more behind; one that fell further behind takes its 32 symbols again, one by one.  (A branch for it in every round, taken in every tenth by some lane, cost a
+//            third of the attention kernel's time.)
+//   SINGLES  one symbol per lookup, for books with longer codes.
+// ESC (of PAIRS and SINGLES): some windows hold no complete code.
+//   WHOLE    the loop above
+enum { KVC_PAIRS = 0, KVC_SINGLES = 1, KVC_WHOLE = 2 };
+// Windows with one code or none, of 4096, up to which a book is decoded by pairs: beyond it catching up costs more than the lookups saved.
+// (Attention, 16 x 16384 tokens, 8 x 4 heads, pairs and singles: V at rel 0.05 (46 windows) 315 and 347 us, K at 0.03 (87) 374 and 347; with longer
+// codes than the window, whose singles are tested one by one, K per block at 0.02 (82) 383 and 404.)
+constexpr uint32_t KVC_PAIRS_LONE = 60, KVC_PAIRS_LONE_ESC = 100;
+
+struct KvcWay { int way; bool esc; };
+__device__ __forceinline__ KvcWay kvc_book_way(const void *book, bool whole) {
+    const kvc_book_header *h = reinterpret_cast<const kvc_book_header *>(book);
+    if (whole) return {KVC_WHOLE, h->escape != 0};
+    const bool pairs = (h->lone_windows & 0xffff0000u) == KVC_LONE_KNOWN ? (h->lone_windows & 0xffffu) <= (h->escape ? KVC_PAIRS_LONE_ESC : KVC_PAIRS_LONE) : h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS;
+    return {pairs ? KVC_PAIRS : KVC_SINGLES, h->escape != 0};
+}
+// An entry of these ways' tables: byte 0: 16 - bits of its codes, byte 1: 8 where a pair lacks its second symbol, bytes 2 and 3: the symbols.  No complete
+// code: 0 bits, bit 7 of byte 0, and the tree node in bytes 2 and 3.  e: the book's entry; len: bits per symbol.
+__device__ __forceinline__ uint32_t kvc_way_entry(uint32_t e, bool pairs, const uint8_t *len) {
+    const uint32_t n = (e >> 6) & 3u, bits = e & 63u;
+    if (n == 0) return 0x90u | (e << 8 & 0xffff0000u);
+    if (!pairs) return (16u - (n == 1 ? bits : len[e >> 8 & 0xffu])) | (e << 8 & 0xff0000u);
+    return (16u - bits + (n == 3 ? len[e >> 24] : 0u)) | (n == 1 ? 0x800u : 0u) | (e << 8 & 0xffff0000u);
+}
+// The tables of two books.  All threads of the CTA call; contains a barrier, between the loads (all of them on their way at once) and
+// the stores; the one behind the stores is the caller's.  len: the two books' bits per symbol, 512 bytes.
+__device__ __forceinline__ void kvc_load_ways(uint32_t *lut0, uint32_t *lut1, const void *book0, const void *book1, bool pairs0, bool pairs1, uint8_t *len, int tid, int nthr) {
+    auto at = [](const void *book, int off) { return reinterpret_cast<const uint8_t *>(book) + off; };
+    const uint4 *src0 = reinterpret_cast<const uint4 *>(at(book0, KVC_BOOK_OFF_LUT)), *src1 = reinterpret_cast<const uint4 *>(at(book1, KVC_BOOK_OFF_LUT));
+    constexpr int N = KVC_LUT_SIZE / 4, AHEAD = 2;
+    for (int i = tid; i < 512; i += nthr) len[i] = (uint8_t)__ldg(reinterpret_cast<const uint32_t *>(at(i < 256 ? book0 : book1, KVC_BOOK_OFF_ENC)) + 2 * (i & 255) + 1);
+    for (int i = tid; i < N; i += AHEAD * nthr) {
+        uint4 a[AHEAD], b[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) { const int k = min(i + j * nthr, N - 1); a[j] = __ldg(src0 + k); b[j] = __ldg(src1 + k); }
+        if (i == tid) __syncthreads();                     // (every thread has a first turn: nthr <= N)
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int k = i + j * nthr;
+            if (k >= N) break;
+            reinterpret_cast<uint4 *>(lut0)[k] = make_uint4(kvc_way_entry(a[j].x, pairs0, len), kvc_way_entry(a[j].y, pairs0, len), kvc_way_entry(a[j].z, pairs0, len), kvc_way_entry(a[j].w, pairs0, len));
+            reinterpret_cast<uint4 *>(lut1)[k] = make_uint4(kvc_way_entry(b[j].x, pairs1, len + 256), kvc_way_entry(b[j].y, pairs1, len + 256), kvc_way_entry(b[j].z, pairs1, len + 256), kvc_way_entry(b[j].w, pairs1, len + 256));
+        }
+    }
+}
+
+__device__ __forceinline__ void kvc_load_tree(uint32_t *tree, const void *book, int tid, int nthr) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_TREE);
+    for (int i = tid; i < 512 / 4; i += nthr) reinterpret_cast<uint4 *>(tree)[i] = src[i];
+}
+
+// A thread's place in its vector.  The stream's next bits as in kvc_decode_vector; f in the low five bits of s, over whatever the sums leave
+// above them: a funnel shift takes no more of it, and a refill is due when the 16s (32 in all) of a round did not carry out of them.
+// At most 132 codes of at most 12 bits, or walks of at most 52, are read: a corrupt stream's reads end 0.9 KB behind its vector.
+struct KvcCursor {
+    uint32_t hi, lo, nx, ptr, s;
+    uint32_t behind, last;                                 // PAIRS: 8 bits per symbol the lane is behind, and the word of the round before, its symbols on top
+    bool ok;
+    __device__ __forceinline__ KvcCursor(uint32_t slot_s, uint32_t byte_pos) {
+        const uint32_t before = slot_s + byte_pos - 1;
+        ptr = before & ~3u;
+        s = 26u - ((before & 3u) << 3);
+        hi = kvc_bswap(kvc_lds32(ptr)); lo = kvc_bswap(kvc_lds32(ptr + 4)); nx = kvc_lds32(ptr + 8);
+        ptr += 12;
+        behind = last = 0u;
+        ok = true;
+    }
+    __device__ __forceinline__ void step(uint32_t n) {
+        if (!((s ^ n) & 32u)) { hi = lo; lo = kvc_bswap(nx); nx = kvc_lds32(ptr); ptr += 4; }
+        s = n;
+    }
+    __device__ __forceinline__ uint32_t window() const { return __funnelshift_r(lo, hi, s); }
+    __device__ __forceinline__ uint32_t look(uint32_t lut_s, uint32_t t) const { return kvc_lds32(lut_s + (t & ((KVC_LUT_SIZE - 1) << 2))); }
+    // the symbol at the window, from the tree node its bits lead to, bit by bit
+    __device__ __forceinline__ uint32_t walk(uint32_t node, uint32_t tree_s) {
+        const KvcTreeShared tree{tree_s};
+        uint32_t sym = 0;
+        bool found = false;
+        step(s + 32u - KVC_LUT_BITS);
+        for (int guard = 0; guard < 40 && node < 512u; guard++) {
+            const uint32_t nd = tree(node);
+            if ((nd & 0xffffu) == KVC_TREE_LEAF) { sym = nd >> 16; found = true; break; }
+            const uint32_t bit = window() >> 29 & 1u;
+            step(s + 31u);
+            node = nd >> (16 * bit) & 0xffffu;
+        }
+        ok = ok && found;
+        return sym & 0xffu;
+    }
+    // two lookups and the step over them
+    template <bool ESC> __device__ __forceinline__ void two(uint32_t lut_s, uint32_t tree_s, uint32_t one, uint32_t &a, uint32_t &b) {
+        const uint32_t t = window();
+        a = look(lut_s, t >> 16);
+        b = look(lut_s, __funnelshift_r(t, 0u, a));
+        if (ESC && __builtin_expect((a | b) & 0x80u, 0)) {
+            // one of them is no code: its symbol by the tree, as an entry of one symbol and no bits
+            if (a & 0x80u) { a = 16u | one | walk(a >> 16, tree_s) << 16; b = look(lut_s, window() >> 16); }
+            else { step(s + 16u + (a & 31u)); a = (a & ~31u) | 16u; }
+            if (b & 0x80u) b = 16u | one | walk(b >> 16, tree_s) << 16;
+        }
+        step(s + a + b);
+    }
+    // PAIRS: the next round; returns the word of the round before (any word in the first one)
+    template <bool ESC> __device__ __forceinline__ uint32_t pairs(uint32_t lut_s, uint32_t tree_s) {
+        uint32_t a, b, sel = 0x7632u;
+        two<ESC>(lut_s, tree_s, 0x800u, a, b);
+        asm("dp2a.lo.u32.u32 %0, %1, %2, %0;" : "+r"(sel) : "r"(0x02260000u), "r"(a));         // + 0x1130 where a lacks a symbol: {a0, b0, b1, 0}
+        const uint32_t c = __byte_perm(a, b, sel);
+        const uint32_t out = __funnelshift_rc(last, c, behind);
+        // (the sums by byte products, as the shared-memory pipe and the integer ALU are the busiest)
+        const uint32_t now = (uint32_t)kvc_dp4a_uu(a, 0x100u, kvc_dp4a_uu(b, 0x100u, (int)behind));
+        last = c << (now - behind);
+        behind = now;
+        return out;
+    }
+    // one symbol, from either table; len_s: the book's bits per symbol
+    template <bool ESC> __device__ __forceinline__ uint32_t single(uint32_t lut_s, uint32_t len_s, uint32_t tree_s) {
+        const uint32_t x = look(lut_s, window() >> 16), sym = x >> 16 & 0xffu;
+        if (ESC && (x & 0x80u)) return walk(x >> 16, tree_s);
+        uint32_t n;
+        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(n) : "r"(len_s + sym));
+        step(s + 32u - n);
+        return sym;
+    }
+    // SINGLES: the next word
+    template <bool ESC> __device__ __forceinline__ uint32_t singles(uint32_t lut_s, uint32_t tree_s) {
+        uint32_t a, b, c, d;
+        two<ESC>(lut_s, tree_s, 0u, a, b);
+        two<ESC>(lut_s, tree_s, 0u, c, d);
+        return __byte_perm(__byte_perm(a, b, 0x0062), __byte_perm(c, d, 0x0062), 0x5410);
+    }
+    // PAIRS, between two rounds: lanes that are behind fetch what they lack
+    template <bool ESC> __device__ __forceinline__ void catch_up(uint32_t lut_s, uint32_t len_s, uint32_t tree_s) {
+        for (; behind; behind -= 8u) last = last >> 8 | single<ESC>(lut_s, len_s, tree_s) << 24;
+    }
+    // back to where the place was
+    __device__ __forceinline__ void back(uint32_t s0, uint32_t ptr0, uint32_t last0, uint32_t behind0) {
+        s = s0; ptr = ptr0; last = last0; behind = behind0;
+        hi = kvc_bswap(kvc_lds32(ptr - 12)); lo = kvc_bswap(kvc_lds32(ptr - 8)); nx = kvc_lds32(ptr - 4);
+    }
+    template <bool ESC> __device__ __forceinline__ uint32_t four(uint32_t lut_s, uint32_t len_s, uint32_t tree_s) {
+        uint32_t w = 0;
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) w |= single<ESC>(lut_s, len_s, tree_s) << (8 * k);
+        return w;
+    }
+};
