@@ -798,9 +798,13 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     auto blkV_of = [&](int col, int t, int l) { return (long long)t * (cols * 2) + (long long)col * 2 + l; };
 
     Item it, nit;
-    int j_n1 = draw ? P + me : (int)(p.work * me / P) + 1;
-    bool have = wk < workers && item_of(draw ? me : j_n1 - 1, it), have_next = have && item_of(j_n1, nit);
-    int drawn = 0;                                         // thread 0: the counter's answer, used an item later
+    // The first item is fixed by the worker's index; with a counter, the next one is drawn when an item begins and looked at in its last step, when
+    // that step's blocks are asked for.  (Drawn an item earlier, a worker held two when the counter ran out.)
+    int j_n1 = draw ? me : (int)(p.work * me / P);
+    bool have = wk < workers && item_of(j_n1, it), have_next = false;
+    if (!draw) have_next = have && item_of(++j_n1, nit);
+    const bool more = draw && p.work > P;                  // not all of the items are fixed
+    int drawn = 0;                                         // thread 0: the counter's answer
     const bool any = have && it.t_lo < it.t_hi;
 
     // the two blocks of a step, by the lanes 0 and 1 of the worker's first warp
@@ -866,7 +870,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     bool v_staged = any, v_landed = true;                  // V blocks of the step to come are on their way already; the last wait for them ended well
     while (have) {
     const int col = it.col, b = col / Hkv, h = col % Hkv;
-    if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
+    if (more && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
 #pragma unroll
     for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = kvc_scale_value(qn[g]) * qscale;
     sync();
@@ -946,11 +950,13 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             const float x = warp_max(fmaxf(fmaxf(s[0][j] + lg.x, s[1][j] + lg.y), fmaxf(s[2][j] + lg.z, s[3][j] + lg.w)));
             if (lane < 4 && own) sm.red[hd + 4 * j][warp] = x;
         }
+        if (more && tid == 0 && step + 1 >= it.t_hi) sm.next_j = drawn;
         sync();                                            // also: every thread is done with the K slots and weights
         const uint32_t startV = cur.startV >> 3;
         {
             bool n_on = true; int nb = b, nh = h, n_col = col, n_step = step + 1;      // the worker's next step (it may open the next column)
             if (n_step >= it.t_hi) {
+                if (more) have_next = item_of(P + sm.next_j, nit);
                 n_on = have_next && nit.t_lo < nit.t_hi;
                 if (n_on) { n_col = nit.col; n_step = nit.t_lo; nb = n_col / Hkv; nh = n_col % Hkv; }
                 if (have_next) q_fetch(nit.col);
@@ -1116,14 +1122,12 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             if (warp == 0 && lane < 4) { dst[0] = m_run[j] * LN2; dst[1] = l_run[j]; }        // the merge kernel counts in powers of e
         }
     }
-    if (draw && tid == 0) sm.next_j = drawn;
     sync();                                                // the sums are read before the next column's weights overwrite them
     dead = BULK && sm.dead != 0;
     }
     if (dead) break;                                       // a staging wait ran out: the status word says so, the item's result is void
-    const int j_n2 = draw ? 2 * P + sm.next_j : j_n1 + 1;
-    it = nit; have = have_next; j_n1 = j_n2;
-    have_next = have && item_of(j_n1, nit);
+    it = nit; have = have_next; have_next = false;
+    if (!draw) have_next = have && item_of(++j_n1, nit);
     }   // items of the worker
     if (BULK && any) {                    // the copy of K issued after the last step is empty, but its phase must end;
         // after a wait that ran out, these are the phases still open: nothing may be in flight at the return
