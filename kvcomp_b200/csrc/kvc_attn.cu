@@ -88,8 +88,8 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 // lanes at 32 different positions fetch 0.5 KB and more per lookup: the kernel becomes bound by shared-memory
 // wavefronts.  So a warp decodes 32 symbols of each of its 32 vectors into rows of bytes in shared memory (KvcCursor: every lane
 // at the same position), and m16n8k32 integer instructions multiply the rows with the weights: two columns per head, the hi and
-// the lo bytes.  The integer sums are the same as in the one-pass form.  What bounds it: the shared-memory pipe (840 wavefronts per warp
-// and step of 128 tokens, 71 % busy; nine per round of two lookups) and, with 2450 instructions, issue (57 %) together.  One layer of
+// the lo bytes.  The integer sums are the same as in the one-pass form.  What bounds it: the shared-memory pipe (846 wavefronts per warp
+// and step of 128 tokens, 76 % busy; nine per round of two lookups) and, with 2570 instructions, issue (59 %) together.  One layer of
 // 16 sequences x 32768 tokens, 8 x 4 heads, rel 0.05 / 0.1: whole rows, each lane at its own position, up to three symbols per lookup (3440 instructions,
 // 1010 wavefronts) 650 us, now 536; 32 x 16384 tokens, 10 x 4, rel 0.02 / 0.15, 868 and 828; 8192 tokens of the first, 184 and 154.  Six workers of 80
 // registers are no faster than five of 96; tables of 8 to 12 bits repeated over the banks (32 KB each, one symbol per lookup) 660 us.
