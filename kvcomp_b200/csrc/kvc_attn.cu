@@ -110,6 +110,10 @@ constexpr int COL_WORDS = 40;
 __host__ __device__ constexpr int vec_words(int G) { return 2 * G * COL_WORDS; }
 // 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -32767 .. 127 * 256 + 127
 constexpr float FIX_DOWN = 32767.0f, FIX_UP = 32639.0f;
+// V's weights: the largest one is 1 and takes 32880 (below the end, 32896, by what the approximate logarithm and power can be off together).
+// Their reference is a score plus a logarithm, rounded up: below FAR that lowers them by 2^-8 in log2 at most, and the fixed-point step stays finer
+// than 1/32767 of the largest.  Beyond FAR the reference is the largest score itself, and the largest weight is looked for.
+constexpr float FIX_V = 32880.0f, FAR = 65536.0f;
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 __device__ __forceinline__ float exp2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float log2_fast(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -905,7 +909,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         {
             const float sc = kvc_scale_value(cur.vsc);     // of the token `vec`; read by lanes of the same warp
             sm.vsc[vec] = sc; sm.vz[vec] = sc * (float)cur.vmi; // (at least fp16's smallest; a negative scale's weights take the shorter end of the fixed-point range)
-            sm.vlg[vec] = log2_fast(fmaxf(fabsf(sc), 5.9604645e-8f)) + (sc < 0.f ? 0.006f : 0.f);
+            sm.vlg[vec] = log2_fast(fmaxf(fabsf(sc), 5.9604645e-8f)) + (sc < 0.f ? 0.011f : 0.f);      // (32880 * 2^-0.011 < 32639)
         }
         bool k_landed = true;                              // (a wait that runs out: see attn_one_kernel)
         if (BULK) {
@@ -943,11 +947,12 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             }
         }
         // ---- online softmax over the step.  The reference of a step is the largest of weight * V scale over its tokens, i.e. of score + log2 of
-        // the scale: the V weights are then at most 1, and their fixed-point step is known without another exchange.
+        // the scale: the V weights are then at most 1, and their fixed-point step is known without another exchange.  (The sums are rounded up: rounded
+        // to nearest, half an ulp of a score of 1e5 took the largest weight beyond 16 bits.)
         const float4 lg = *reinterpret_cast<const float4 *>(&sm.vlg[warp * 32 + r4]);
 #pragma unroll
         for (int j = 0; j < HL; j++) {
-            const float x = warp_max(fmaxf(fmaxf(s[0][j] + lg.x, s[1][j] + lg.y), fmaxf(s[2][j] + lg.z, s[3][j] + lg.w)));
+            const float x = warp_max(fmaxf(fmaxf(__fadd_ru(s[0][j], lg.x), __fadd_ru(s[1][j], lg.y)), fmaxf(__fadd_ru(s[2][j], lg.z), __fadd_ru(s[3][j], lg.w))));
             if (lane < 4 && own) sm.red[hd + 4 * j][warp] = x;
         }
         if (more && tid == 0 && step + 1 >= it.t_hi) sm.next_j = drawn;
@@ -971,19 +976,63 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         float alpha[HL], beta[HL];
         {
             const float4 sc = *reinterpret_cast<const float4 *>(&sm.vsc[warp * 32 + r4]), vz = *reinterpret_cast<const float4 *>(&sm.vz[warp * 32 + r4]);
+            float u[HL];
+            bool far = false;
 #pragma unroll
-            for (int j = 0; j < HL; j++) {
-                const float u = red_max(hd + 4 * j), m_new = fmaxf(m_run[j], u);
-                alpha[j] = exp2_fast(m_run[j] - m_new); beta[j] = exp2_fast(u - m_new);       // exp(-inf) = 0 on the first step
-                m_run[j] = m_new;
-                const float p0 = exp2_fast(s[0][j] - u), p1 = exp2_fast(s[1][j] - u), p2 = exp2_fast(s[2][j] - u), p3 = exp2_fast(s[3][j] - u);
-                l_run[j] = fmaf(l_run[j], alpha[j], beta[j] * ((p0 + p1) + (p2 + p3)));
-                z_run[j] = fmaf(z_run[j], alpha[j], beta[j] * fmaf(p0, vz.x, fmaf(p1, vz.y, fmaf(p2, vz.z, p3 * vz.w))));
-                beta[j] *= -1.0f / FIX_DOWN;
-                // the lane's four tokens are one word of its head
-                const uint2 w2 = pack_fix(p0 * sc.x, p1 * sc.y, p2 * sc.z, p3 * sc.w, -FIX_DOWN);
+            for (int j = 0; j < HL; j++) { u[j] = red_max(hd + 4 * j); far = far || fabsf(u[j]) >= FAR; }
+            // the step's sums relative to 2^u, and its V weights: the lane's four tokens are one word of its head
+            auto put_weights = [&](int j, const float (&w)[4], float inv) {
+                const uint2 w2 = pack_fix(w[0], w[1], w[2], w[3], inv);
                 uint32_t *at = sm.w + 2 * VW + 2 * (hd + 4 * j) * COL_WORDS + warp * 8 + (lane >> 2);
                 if (own) { at[0] = w2.x; at[COL_WORDS] = w2.y; }
+            };
+            auto weigh = [&](int j, float (&w)[4]) {
+                const float m_new = fmaxf(m_run[j], u[j]);
+                alpha[j] = exp2_fast(m_run[j] - m_new); beta[j] = exp2_fast(u[j] - m_new);    // exp(-inf) = 0 on the first step
+                m_run[j] = m_new;
+                const float p0 = exp2_fast(s[0][j] - u[j]), p1 = exp2_fast(s[1][j] - u[j]), p2 = exp2_fast(s[2][j] - u[j]), p3 = exp2_fast(s[3][j] - u[j]);
+                l_run[j] = fmaf(l_run[j], alpha[j], beta[j] * ((p0 + p1) + (p2 + p3)));
+                z_run[j] = fmaf(z_run[j], alpha[j], beta[j] * fmaf(p0, vz.x, fmaf(p1, vz.y, fmaf(p2, vz.z, p3 * vz.w))));
+                w[0] = p0 * sc.x; w[1] = p1 * sc.y; w[2] = p2 * sc.z; w[3] = p3 * sc.w;
+            };
+            // (a warp holds all heads' maxima, so the worker's warps agree)
+            if (!__any_sync(0xffffffffu, far)) {
+#pragma unroll
+                for (int j = 0; j < HL; j++) {
+                    float w[4];
+                    weigh(j, w);
+                    beta[j] *= -1.0f / FIX_V;
+                    put_weights(j, w, -FIX_V);
+                }
+            } else {
+                float w[HL][4];
+                sync();                                    // the maxima are read
+#pragma unroll
+                for (int j = 0; j < HL; j++) {
+                    const float x = warp_max(fmaxf(fmaxf(s[0][j], s[1][j]), fmaxf(s[2][j], s[3][j])));
+                    if (lane < 4 && own) sm.red[hd + 4 * j][warp] = x;
+                }
+                sync();
+#pragma unroll
+                for (int j = 0; j < HL; j++) { u[j] = red_max(hd + 4 * j); weigh(j, w[j]); }
+                sync();
+#pragma unroll
+                for (int j = 0; j < HL; j++) {             // (a negative weight takes the shorter end of the range)
+                    float x = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) x = fmaxf(x, fmaxf(w[j][i], -w[j][i] * (FIX_V / FIX_UP)));
+                    x = warp_max(x);
+                    if (lane < 4 && own) sm.red[hd + 4 * j][warp] = x;
+                }
+                sync();
+#pragma unroll
+                for (int j = 0; j < HL; j++) {
+                    const float top = red_max(hd + 4 * j), inv = top > 0.f ? -FIX_V / top : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) w[j][i] = (float)__float2int_rn(w[j][i] * inv);       // (an infinite scale: no weight, and NaN through beta)
+                    beta[j] *= top * (-1.0f / FIX_V);
+                    put_weights(j, w[j], 1.0f);
+                }
             }
         }
         v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
