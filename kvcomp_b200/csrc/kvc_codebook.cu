@@ -426,9 +426,10 @@ __global__ void __launch_bounds__(BOOK_THREADS) book_from_tree_kernel(const uint
             if (rt[3 * nd]) {
                 int sym = rt[3 * nd + 1];
                 if (len > 32) s.flags |= KVC_FLAG_CODE_TOO_LONG;
+                nsym += s.enc_len[sym] == 0;                // (a symbol at two leaves is one symbol)
                 s.enc_code[sym] = (uint32_t)code; s.enc_len[sym] = (uint32_t)len;
                 if ((int)len > s.max_len) s.max_len = (int)len;
-                nsym++; if (sym < mn) mn = sym; if (sym > mx) mx = sym;
+                if (sym < mn) mn = sym; if (sym > mx) mx = sym;
             } else {
                 int c0 = rt[3 * nd + 1], c1 = rt[3 * nd + 2];
                 if (c1 != 0xff && sp < 510) { st_node[sp] = (short)c1; st_code[sp] = (long long)((((code << 1) | 1) & 0xffffffffffull) | ((len + 1) << 40)); sp++; }

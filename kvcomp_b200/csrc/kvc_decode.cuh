@@ -261,7 +261,11 @@ struct KvcWay { int way; bool esc; };
 __device__ __forceinline__ KvcWay kvc_book_way(const void *book, bool whole) {
     const kvc_book_header *h = reinterpret_cast<const kvc_book_header *>(book);
     if (whole) return {KVC_WHOLE, h->escape != 0};
-    const bool pairs = (h->lone_windows & 0xffff0000u) == KVC_LONE_KNOWN ? (h->lone_windows & 0xffffu) <= (h->escape ? KVC_PAIRS_LONE_ESC : KVC_PAIRS_LONE) : h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS;
+    // A code that lacks a branch (a lone symbol's, or a caller's tree) has more nodes than 2 n - 2: PAIRS looks up to four symbols beyond a vector's end,
+    // and what lies there may be no code.  SINGLES reads the 128 and no more.
+    const bool whole_code = h->escape == 0 || h->n_nodes == 2 * h->n_symbols - 2;
+    const bool pairs = whole_code && ((h->lone_windows & 0xffff0000u) == KVC_LONE_KNOWN ? (h->lone_windows & 0xffffu) <= (h->escape ? KVC_PAIRS_LONE_ESC : KVC_PAIRS_LONE)
+                                                                                        : h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS);
     return {pairs ? KVC_PAIRS : KVC_SINGLES, h->escape != 0};
 }
 // An entry of these ways' tables: byte 0: 16 - bits of its codes, byte 1: 8 where a pair lacks its second symbol, bytes 2 and 3: the symbols.  No complete
