@@ -111,11 +111,13 @@ __host__ __device__ constexpr int vec_words(int G) { return 2 * G * COL_WORDS; }
 // 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -32767 .. 127 * 256 + 127
 constexpr float FIX_DOWN = 32767.0f, FIX_UP = 32639.0f;
 // V's weights: the largest one is 1 and takes 32880 (below the end, 32896, by what the approximate logarithm and power can be off together).
-// Their reference is a score plus a logarithm, rounded up: below FAR that lowers them by 2^-8 in log2 at most, and the fixed-point step stays finer
-// than 1/32767 of the largest.  Beyond FAR the reference is the largest score itself, and the largest weight is looked for.
-constexpr float FIX_V = 32880.0f, FAR = 65536.0f;
+// Their reference is a score plus a logarithm, rounded up: below FAR that lowers them by a factor of exp(-2^-9) at most, and the fixed-point step stays
+// finer than 1/32767 of the largest.  Beyond FAR the reference is the largest score itself, and the largest weight is looked for.
+constexpr float FIX_V = 32880.0f, FAR = 32768.0f;
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
-__device__ __forceinline__ float exp2_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// (Scores stay in units of e, as the merge kernel and the dense rows behind the compressed part have them: a factor of log2 e in the query would round every
+// score, and at 1e4 two equal ones by two ways weigh 1e-3 apart.)
+__device__ __forceinline__ float exp_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * LOG2E)); return y; }
 __device__ __forceinline__ float log2_fast(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float rcp_fast(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
@@ -695,8 +697,8 @@ constexpr int ROWS_PLANNED = 5;              // workers per SM that the plan of 
 template <int G>
 struct alignas(32) RowsWorker {
     uint32_t w[3 * vec_words(G)];            // weight words: K of the step's two blocks, V; scratch of the tail and of a team's sums
-    float q[G * 128];                        // the query, times the scaling and log2 e
-    float vsc[128], vz[128], vlg[128];       // of the step's tokens: V's scale, scale * min_int, log2 of the scale
+    float q[G * 128];                        // the query, times the scaling
+    float vsc[128], vz[128], vlg[128];       // of the step's tokens: V's scale, scale * min_int, log of the scale
     float red[G][4];                         // per-warp partials of a head
     float kstep[2 * G], zp[2 * G], qsum[G];
     uint64_t bar[2];                         // K and V staging barriers
@@ -863,7 +865,6 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (have) q_fetch(it.col);
 
-    const float qscale = p.scaling * LOG2E;                // scores in units of log 2
     // over a warp's vectors: the lane's four, then the eight lanes with the same heads
     auto warp_max = [&](float x) { x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 4)); x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 8)); return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 16)); };
     auto warp_sum = [&](float x) { x += __shfl_xor_sync(0xffffffffu, x, 4); x += __shfl_xor_sync(0xffffffffu, x, 8); return x + __shfl_xor_sync(0xffffffffu, x, 16); };
@@ -876,7 +877,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     const int col = it.col, b = col / Hkv, h = col % Hkv;
     if (more && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
 #pragma unroll
-    for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = kvc_scale_value(qn[g]) * qscale;
+    for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = kvc_scale_value(qn[g]) * p.scaling;
     sync();
     if (km.sc == 0) for (int g = warp; g < G; g += 4) {    // sum of each query head's 128 (scaled) values
         float a = 0.f;
@@ -886,7 +887,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         if (lane == 0) sm.qsum[g] = a;
     }
     // acc: the lane's four channels.  l, z: the sums of the weights and of weight * scale * min_int over the lane's own tokens, added up
-    // over the lanes at the item's end.  All relative to 2^m.
+    // over the lanes at the item's end.  All relative to e^m.
     float m_run[HL], l_run[HL], z_run[HL], acc[4][HL];
 #pragma unroll
     for (int j = 0; j < HL; j++) {
@@ -909,7 +910,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         {
             const float sc = kvc_scale_value(cur.vsc);     // of the token `vec`; read by lanes of the same warp
             sm.vsc[vec] = sc; sm.vz[vec] = sc * (float)cur.vmi; // (at least fp16's smallest; a negative scale's weights take the shorter end of the fixed-point range)
-            sm.vlg[vec] = log2_fast(fmaxf(fabsf(sc), 5.9604645e-8f)) + (sc < 0.f ? 0.011f : 0.f);      // (32880 * 2^-0.011 < 32639)
+            sm.vlg[vec] = log2_fast(fmaxf(fabsf(sc), 5.9604645e-8f)) * LN2 + (sc < 0.f ? 0.0077f : 0.f);      // (32880 * exp(-0.0077) < 32639)
         }
         bool k_landed = true;                              // (a wait that runs out: see attn_one_kernel)
         if (BULK) {
@@ -946,7 +947,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
                 }
             }
         }
-        // ---- online softmax over the step.  The reference of a step is the largest of weight * V scale over its tokens, i.e. of score + log2 of
+        // ---- online softmax over the step.  The reference of a step is the largest of weight * V scale over its tokens, i.e. of score + log of
         // the scale: the V weights are then at most 1, and their fixed-point step is known without another exchange.  (The sums are rounded up: rounded
         // to nearest, half an ulp of a score of 1e5 took the largest weight beyond 16 bits.)
         const float4 lg = *reinterpret_cast<const float4 *>(&sm.vlg[warp * 32 + r4]);
@@ -980,7 +981,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             bool far = false;
 #pragma unroll
             for (int j = 0; j < HL; j++) { u[j] = red_max(hd + 4 * j); far = far || fabsf(u[j]) >= FAR; }
-            // the step's sums relative to 2^u, and its V weights: the lane's four tokens are one word of its head
+            // the step's sums relative to e^u, and its V weights: the lane's four tokens are one word of its head
             auto put_weights = [&](int j, const float (&w)[4], float inv) {
                 const uint2 w2 = pack_fix(w[0], w[1], w[2], w[3], inv);
                 uint32_t *at = sm.w + 2 * VW + 2 * (hd + 4 * j) * COL_WORDS + warp * 8 + (lane >> 2);
@@ -988,9 +989,9 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             };
             auto weigh = [&](int j, float (&w)[4]) {
                 const float m_new = fmaxf(m_run[j], u[j]);
-                alpha[j] = exp2_fast(m_run[j] - m_new); beta[j] = exp2_fast(u[j] - m_new);    // exp(-inf) = 0 on the first step
+                alpha[j] = exp_fast(m_run[j] - m_new); beta[j] = exp_fast(u[j] - m_new);    // exp(-inf) = 0 on the first step
                 m_run[j] = m_new;
-                const float p0 = exp2_fast(s[0][j] - u[j]), p1 = exp2_fast(s[1][j] - u[j]), p2 = exp2_fast(s[2][j] - u[j]), p3 = exp2_fast(s[3][j] - u[j]);
+                const float p0 = exp_fast(s[0][j] - u[j]), p1 = exp_fast(s[1][j] - u[j]), p2 = exp_fast(s[2][j] - u[j]), p3 = exp_fast(s[3][j] - u[j]);
                 l_run[j] = fmaf(l_run[j], alpha[j], beta[j] * ((p0 + p1) + (p2 + p3)));
                 z_run[j] = fmaf(z_run[j], alpha[j], beta[j] * fmaf(p0, vz.x, fmaf(p1, vz.y, fmaf(p2, vz.z, p3 * vz.w))));
                 w[0] = p0 * sc.x; w[1] = p1 * sc.y; w[2] = p2 * sc.z; w[3] = p3 * sc.w;
@@ -1081,7 +1082,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
 #pragma unroll
             for (int j = 0; j < HL; j++) {
                 const float m_new = fmaxf(m_run[j], red_max(hd + 4 * j));
-                alpha[j] = exp2_fast(m_run[j] - m_new);
+                alpha[j] = exp_fast(m_run[j] - m_new);
                 m_run[j] = m_new;
                 if (tid < 4) sm.zp[hd + 4 * j] = m_new;
 #pragma unroll
@@ -1090,7 +1091,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             sync();
 #pragma unroll
             for (int g = 0; g < G; g++) {
-                const float pr = act ? exp2_fast(s[g] - sm.zp[g]) : 0.f;
+                const float pr = act ? exp_fast(s[g] - sm.zp[g]) : 0.f;
                 pt[tid * G + g] = pr;
                 const float ssum = kvc_warp_sum(pr);
                 if (lane == 0) sm.red[g][warp] = ssum;
@@ -1148,7 +1149,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             float M = -CUDART_INF_F, O = 0.f, L = 0.f;
             for (int w = 0; w < team; w++) M = fmaxf(M, mates[w].red[g][0]);
             for (int w = 0; w < team; w++) {
-                const float m = mates[w].red[g][0], e = m == -CUDART_INF_F ? 0.f : exp2_fast(m - M);     // a worker without tokens adds nothing
+                const float m = mates[w].red[g][0], e = m == -CUDART_INF_F ? 0.f : exp_fast(m - M);     // a worker without tokens adds nothing
                 L = fmaf(mates[w].red[g][1], e, L);
                 O = fmaf(reinterpret_cast<const float *>(mates[w].w)[g * 128 + tid], e, O);
             }
@@ -1168,7 +1169,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             float *dst = p.ws_part + ((head0 + hd + 4 * j) * p.splits + it.part) * ROWS_PART_FLOATS;     // 8-byte aligned
             *reinterpret_cast<float2 *>(dst + 2 + warp * 32 + r4) = make_float2(acc[0][j], acc[1][j]);
             *reinterpret_cast<float2 *>(dst + 4 + warp * 32 + r4) = make_float2(acc[2][j], acc[3][j]);
-            if (warp == 0 && lane < 4) { dst[0] = m_run[j] * LN2; dst[1] = l_run[j]; }        // the merge kernel counts in powers of e
+            if (warp == 0 && lane < 4) { dst[0] = m_run[j]; dst[1] = l_run[j]; }
         }
     }
     sync();                                                // the sums are read before the next column's weights overwrite them

@@ -1,5 +1,6 @@
 """Grouped attention at scores far beyond those of trained models: fp16 queries and keys are finite up to scores of 1e11, where a rounding of the score
-is more than a weight's whole range.  A clear winner's weight stays 1 whatever the score and the sign of its V scale."""
+is more than a weight's whole range.  A clear winner's weight stays 1 whatever the score and the sign of its V scale, and rows behind the
+compressed part weigh what equal scores in it weigh."""
 import math
 
 import pytest
@@ -122,3 +123,28 @@ def test_what_is_not_finite_reaches_the_output(ops, G, long, where, value):
     assert not torch.isfinite(out[3]).any()
     rest = [b for b in range(B) if b != 3]
     assert torch.equal(out[rest], clean[rest])
+
+
+@pytest.mark.parametrize("long", [False, True])
+@pytest.mark.parametrize("G", [2, 4, 8])
+@pytest.mark.parametrize("q0", [10.0, 1000.0, 4097.0, 60000.0])
+@pytest.mark.parametrize("kw", [dict(), dict(splits=4), dict(splits=1, workspace=False)])
+def test_equal_scores_weigh_the_same(ops, G, long, q0, kw):
+    """One channel of the query is not zero, and there all keys are equal: every token has the same score, which 32 bits hold."""
+    g = torch.Generator(device="cuda").manual_seed(G)
+    T, B, H = _shape(long)
+    Tr = 200
+    codes = torch.randint(0, 8, (T, B, H, 128), device="cuda", generator=g).to(torch.uint8)
+    codes[..., 5] = 100
+    kc, ke, keep_k = _keys(ops, codes, torch.zeros(128, device="cuda", dtype=torch.int16), torch.ones(128, device="cuda").half())
+    vc, ve, keep_v = _values(ops, codes.shape, g, 1)
+    kt = torch.randn(Tr, B, H, 128, device="cuda", generator=g).half()
+    kt[..., 5] = 100.0
+    vt = (-5.0 * T / Tr * (0.5 + torch.rand(Tr, B, H, 128, device="cuda", generator=g))).half()      # (as heavy as the compressed part, the other way)
+    q = torch.zeros(B, H * G, 128, device="cuda").half()
+    q[..., 5] = q0
+    want = ((ve.sum(0) + vt.double().sum(0)) / (T + Tr)).repeat_interleave(G, 1)
+    out, st = ops.attn_decode(kc, vc, T, B, H, q, SCALING, kt, vt, **kw)
+    assert ops.read_status(st) == 0
+    # 1e-3 of the largest output, as for the attention everywhere (weights of 16 bits, fp16 outputs)
+    assert float((out.double() - want).abs().max() / want.abs().max()) <= 1e-3
