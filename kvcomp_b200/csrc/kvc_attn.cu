@@ -179,38 +179,34 @@ template <int G> struct RowsSum {
         }
     }
 };
-// What a vector is decoded from: shared addresses of its slot, the table, the code lengths and the tree
-struct RowsFrom { uint32_t slot, at, lut, len, tree; };
+// What a vector is decoded from: shared addresses of its slot, the table and the tree
+struct RowsFrom { uint32_t slot, at, lut, tree; };
 
+// lagged: in how many of the four parts a lane fell too far behind for PAIRS' rounds.
 template <int G, int WAY, bool ESC>
-__device__ __forceinline__ bool rows_dot_way(const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL]) {
+__device__ __forceinline__ bool rows_dot_way(const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL], uint32_t &lagged) {
     const uint32_t r = lane >> 2, q = lane & 3;
     const uint32_t put = rows_s + lane * ROW_BYTES + (r & 1u) * 16;
     const uint32_t get = rows_s + r * ROW_BYTES + (((q >> 1) ^ (r >> 2 & 1u)) * 16) + (q & 1u) * 8;
     const uint32_t col = w_s + (r % (2 * G)) * (COL_WORDS * 4) + q * 8;
     KvcCursor at(f.slot, f.at);
     RowsSum<G> sum;
-    auto word = [&]() { return WAY == KVC_PAIRS ? at.pairs<ESC>(f.lut, f.tree) : at.singles<ESC>(f.lut, f.tree); };
-    if (WAY == KVC_PAIRS) word();
+    auto word = [&](bool end) { return WAY == KVC_PAIRS ? at.pairs<ESC>(f.lut, f.tree, end) : at.singles<ESC>(f.lut, f.tree); };
+    if (WAY == KVC_PAIRS) word(false);
 #pragma unroll 1
     for (uint32_t ch = 0; ch < 4; ch++) {
         const uint32_t s0 = at.s, ptr0 = at.ptr, last0 = at.last, behind0 = at.behind;
 #pragma unroll ESC ? 1 : 2
-        for (int u = 0; u < 2; u++) {
-            const uint32_t w0 = word(), w1 = word(), w2 = word(), w3 = word();
+        for (uint32_t u = 0; u < 2; u++) {
+            const uint32_t w0 = word(false), w1 = word(false), w2 = word(false), w3 = word(ch + u == 4u);
             sts128(u ? put ^ 16u : put, w0, w1, w2, w3);
         }
         if (WAY == KVC_PAIRS && __any_sync(0xffffffffu, at.behind >= 24u)) {
-            // a lane that fell more than a word behind: the 32 symbols again, one by one; the others that are behind catch up
-            const bool again = at.behind > 32u;
-            if (again) at.back(s0, ptr0, last0, behind0);
-            at.catch_up<ESC>(f.lut, f.len, f.tree);
-            if (again)
-#pragma unroll 1
-                for (uint32_t k = 0; k < 8; k++) {
-                    asm volatile("st.shared.u32 [%0], %1;" :: "r"((k < 4 ? put : put ^ 16u) + (k & 3u) * 4), "r"(at.last) : "memory");
-                    at.last = at.four<ESC>(f.lut, f.len, f.tree);
-                }
+            // a lane that fell more than a word behind takes the 32 symbols again; it and the others that are behind catch up
+            lagged += __any_sync(0xffffffffu, at.behind > 32u);
+            if (at.behind > 32u)
+                at.again<ESC>(f.lut, f.tree, s0, ptr0, last0, behind0, ch == 3, [&](uint32_t k, uint32_t w) { asm volatile("st.shared.u32 [%0], %1;" :: "r"((k < 4 ? put : put ^ 16u) + (k & 3u) * 4), "r"(w) : "memory"); });
+            if (ch < 3) at.catch_up<ESC>(f.lut, f.tree);
         }
         __syncwarp();
         sum.add(get, ROW_BYTES, col + ch * 32);
@@ -234,10 +230,10 @@ __device__ __forceinline__ bool rows_dot_whole(const RowsFrom &f, uint32_t rows_
     return ok;
 }
 template <int G>
-__device__ __forceinline__ bool rows_dot(const KvcWay &way, const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL]) {
+__device__ __forceinline__ bool rows_dot(const KvcWay &way, const RowsFrom &f, uint32_t rows_s, uint32_t w_s, int lane, int (&d)[4][RowsSum<G>::HL], uint32_t &lagged) {
     if (way.way == KVC_WHOLE) return way.esc ? rows_dot_whole<G, true>(f, rows_s, w_s, lane, d) : rows_dot_whole<G, false>(f, rows_s, w_s, lane, d);
-    if (!way.esc) return way.way == KVC_PAIRS ? rows_dot_way<G, KVC_PAIRS, false>(f, rows_s, w_s, lane, d) : rows_dot_way<G, KVC_SINGLES, false>(f, rows_s, w_s, lane, d);
-    return way.way == KVC_PAIRS ? rows_dot_way<G, KVC_PAIRS, true>(f, rows_s, w_s, lane, d) : rows_dot_way<G, KVC_SINGLES, true>(f, rows_s, w_s, lane, d);
+    if (!way.esc) return way.way == KVC_PAIRS ? rows_dot_way<G, KVC_PAIRS, false>(f, rows_s, w_s, lane, d, lagged) : rows_dot_way<G, KVC_SINGLES, false>(f, rows_s, w_s, lane, d, lagged);
+    return way.way == KVC_PAIRS ? rows_dot_way<G, KVC_PAIRS, true>(f, rows_s, w_s, lane, d, lagged) : rows_dot_way<G, KVC_SINGLES, true>(f, rows_s, w_s, lane, d, lagged);
 }
 
 // Where the hi / lo weight word of position c and head g sits in a vector's 2 * WROW * G words.  One or
@@ -680,6 +676,7 @@ struct AttnParams {
     int *status;
     int workers;                  // per CTA
     int brief;                    // a step per worker at most: vectors are decoded whole
+    int spare;                    // there is room for a table of V's single symbols beside that of pairs
     int team;                     // without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
     int wait_limit;               // tries of a staging wait before it gives up (KVC_FLAG_WAIT_TIMEOUT)
@@ -694,6 +691,11 @@ struct AttnParams {
 constexpr int ROWS_PART_FLOATS = 130;        // a partial result: m, l, acc[128]
 static_assert(2 * ROWS_PART_FLOATS <= ATTN_PART_FLOATS, "a workspace for n runs of 256-token tiles holds 2 n partial results");
 template <int G> __host__ __device__ constexpr int rows_workers() { return G == 8 ? 4 : 5; }
+// Bytes of 128 symbols from which a vector has too many windows of one code for pairs: 5 bits a symbol.  (16 x 16384 tokens, 8 x 4 heads, one V channel of every head
+// six times the others, units of V per token at rel 0.05, and per token and head at 0.1: by pairs, with what fell behind again symbol by symbol, 517 and 523 us, at the
+// lane's own pace 439 and 456, from the spare table 343 and 380; from 88 bytes on 343 and 398, from 96 on 366 and 404.  A book that goes by pairs has 4.1 bits a symbol at most, 66
+// bytes a vector on average.)
+constexpr uint32_t LONG_VECTOR = 80;
 constexpr int ROWS_PLANNED = 5;              // workers per SM that the plan of a grouped launch counts
 
 template <int G>
@@ -712,7 +714,8 @@ struct alignas(32) RowsTables { uint32_t lutK[KVC_LUT_SIZE], lutV[KVC_LUT_SIZE];
 
 // shared memory of a CTA: tables, workers, slots (two of K and two of V each), rows; a corrupt stream's overrun ends in the rows
 template <int G> size_t rows_smem(const AttnParams &p, int workers) {
-    return sizeof(RowsTables) + workers * (sizeof(RowsWorker<G>) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes) + 128 * (p.brief ? WHOLE_ROW_BYTES : ROW_BYTES));
+    return sizeof(RowsTables) + workers * (sizeof(RowsWorker<G>) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes) + 128 * (p.brief ? WHOLE_ROW_BYTES : ROW_BYTES)) +
+           (p.spare ? 4 * KVC_LUT_SIZE : 0);
 }
 
 template <int G> int rows_fit(const AttnParams &p) {         // workers that an SM holds
@@ -770,6 +773,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     RowsWorker<G> &sm = reinterpret_cast<RowsWorker<G> *>(wbase)[wk];
     uint8_t *const slotsK = sbase + wk * 2 * (p.slotK_bytes + p.slotV_bytes), *const slotsV = slotsK + 2 * p.slotK_bytes;
     const uint32_t rows_s = kvc_smem_addr(sbase + workers * 2 * (p.slotK_bytes + p.slotV_bytes)) + (wk * 4 + warp) * 32 * (p.brief ? WHOLE_ROW_BYTES : ROW_BYTES);
+    uint32_t *const spare = reinterpret_cast<uint32_t *>(sbase + workers * (2 * (p.slotK_bytes + p.slotV_bytes) + 128 * ROW_BYTES));      // (never with brief)
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
     // launched with programmatic stream serialisation: this kernel's own set-up -- the tables, the first blocks, the first step's metadata: cache
     // data that no kernel of a decode step writes -- runs before griddepcontrol.wait, possibly while the kernel ahead of it in the
@@ -824,13 +828,14 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         if (warp == 0 && any) { stage_K(true, it.col, it.t_lo); stage_V(true, it.col, it.t_lo); }
     }
     const KvcWay wayK = kvc_book_way(p.k.book, p.brief != 0), wayV = kvc_book_way(p.v.book, p.brief != 0);
+    const bool spare_in = p.spare && wayV.way == KVC_PAIRS;
     if (p.brief) {
         kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
         kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
-    } else kvc_load_ways(tab.lutK, tab.lutV, p.k.book, p.v.book, wayK.way == KVC_PAIRS, wayV.way == KVC_PAIRS, tab.len, threadIdx.x, blockDim.x);
+    } else kvc_load_ways(tab.lutK, tab.lutV, spare_in ? spare : nullptr, p.k.book, p.v.book, wayK.way == KVC_PAIRS, wayV.way == KVC_PAIRS, tab.len, threadIdx.x, blockDim.x);
     if (wayK.esc) kvc_load_tree(tab.tree[0], p.k.book, threadIdx.x, blockDim.x);
     if (wayV.esc) kvc_load_tree(tab.tree[1], p.v.book, threadIdx.x, blockDim.x);
-    const uint32_t lutK_s = kvc_smem_addr(tab.lutK), lutV_s = kvc_smem_addr(tab.lutV), len_s = kvc_smem_addr(tab.len), tree_s = kvc_smem_addr(tab.tree);
+    const uint32_t lutK_s = kvc_smem_addr(tab.lutK), lutV_s = kvc_smem_addr(tab.lutV), tree_s = kvc_smem_addr(tab.tree), spare_s = kvc_smem_addr(spare);
 
     struct StepMeta { unsigned short startK, startV, vsc, ksc; int vmi, kmi; KUnit ku; };   // as loaded: no arithmetic waits on them here
     auto load_meta = [&](bool on, int b, int h, int col, int step, StepMeta &m) {
@@ -873,7 +878,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     auto red_max = [&](int g) { const float4 x = *reinterpret_cast<const float4 *>(sm.red[g]); return fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)); };
     auto red_sum = [&](int g) { const float4 x = *reinterpret_cast<const float4 *>(sm.red[g]); return (x.x + x.y) + (x.z + x.w); };
 
-    uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
+    uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next; bit 2: the item's V from the spare table
     bool v_staged = any, v_landed = true;                  // V blocks of the step to come are on their way already; the last wait for them ended well
     while (have) {
     const int col = it.col, b = col / Hkv, h = col % Hkv;
@@ -887,6 +892,13 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         for (int k = 0; k < 4; k++) a += sm.q[g * 128 + k * 32 + lane];
         a = kvc_warp_sum(a);
         if (lane == 0) sm.qsum[g] = a;
+    }
+    // A channel far beyond the others of its tokens has nothing but long codes, in every step of the column.  A warp with a vector of more than LONG_VECTOR
+    // bytes in the first step (up to where the next one begins; that of the warp's last is not known) takes the item's V one symbol per lookup, from
+    // the spare table.
+    if (spare_in) {
+        const uint32_t at = cur.startV >> 3, bytes = __shfl_sync(0xffffffffu, at, lane < 24 ? lane + 8 : (lane + 1) & 7) - at;
+        par = __any_sync(0xffffffffu, bytes > LONG_VECTOR && lane != 31) ? par | 4u : par & 3u;
     }
     // acc: the lane's four channels.  l, z: the sums of the weights and of weight * scale * min_int over the lane's own tokens, added up
     // over the lanes at the item's end.  All relative to e^m.
@@ -930,7 +942,8 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             int d[4][HL];
             const uint32_t start = cur.startK >> 3;
             bool ok = k_landed && sm.okK[sub] && start < sm.nbK[sub];              // a vector begins inside its block
-            ok = rows_dot<G>(wayK, {kvc_smem_addr(slotsK + sub * p.slotK_bytes), ok ? sm.leadK[sub] + start : 1u, lutK_s, len_s, tree_s}, rows_s, kvc_smem_addr(sm.w + sub * VW), lane, d) && ok;
+            uint32_t lagged = 0;
+            ok = rows_dot<G>(wayK, {kvc_smem_addr(slotsK + sub * p.slotK_bytes), ok ? sm.leadK[sub] + start : 1u, lutK_s, tree_s}, rows_s, kvc_smem_addr(sm.w + sub * VW), lane, d, lagged) && ok;
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
             const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the token `vec`
 #pragma unroll
@@ -1038,7 +1051,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
                 }
             }
         }
-        v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit);
+        v_landed = !BULK || kvc_mbar_wait(&sm.bar[1], par >> 1 & 1u, p.wait_limit);
         if (BULK && v_landed) par ^= 2u;
         if (!v_landed) flags |= KVC_FLAG_WAIT_TIMEOUT;
         v_staged = false;
@@ -1047,7 +1060,11 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         {
             int d[4][HL];
             bool ok = v_landed && sm.okV[sub] && startV < sm.nbV[sub];
-            ok = rows_dot<G>(wayV, {kvc_smem_addr(slotsV + sub * p.slotV_bytes), ok ? sm.leadV[sub] + startV : 1u, lutV_s, len_s + 256u, tree_s + 2048u}, rows_s, kvc_smem_addr(sm.w + 2 * VW), lane, d) && ok;
+            // (and so does a warp whose lanes lag in two parts of four, for the rest of the item)
+            uint32_t lagged = 0;
+            const bool lone = (par & 4u) != 0;
+            ok = rows_dot<G>(lone ? KvcWay{KVC_SINGLES, wayV.esc} : wayV, {kvc_smem_addr(slotsV + sub * p.slotV_bytes), ok ? sm.leadV[sub] + startV : 1u, lone ? spare_s : lutV_s, tree_s + 2048u}, rows_s, kvc_smem_addr(sm.w + 2 * VW), lane, d, lagged) && ok;
+            if (spare_in && lagged >= 2u) par |= 4u;
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
 #pragma unroll
             for (int i = 0; i < 4; i++)
@@ -1184,7 +1201,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     if (BULK && any) {                    // the copy of K issued after the last step is empty, but its phase must end;
         // after a wait that ran out, these are the phases still open: nothing may be in flight at the return
         if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
-        if ((v_staged || !v_landed) && !kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
+        if ((v_staged || !v_landed) && !kvc_mbar_wait(&sm.bar[1], par >> 1 & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
     }
     if (flags) atomicOr(p.status, flags);
     if (draw && tid == 0) {               // the last worker to finish leaves the scheduling counters zeroed for the next launch
@@ -1914,7 +1931,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     p.out = reinterpret_cast<__half *>(out);
     p.scaling = scaling; p.splits = splits; p.tiles_per_split = tps; p.long_runs = long_runs; p.short_tiles = short_tiles;
     p.n_tiles = (int)n_tiles;
-    p.team = p.brief = 0;
+    p.team = p.brief = p.spare = 0;
     p.work = cols * splits;
     // with a workspace the CTAs draw their items from its counters (zero before the first launch, left zeroed)
     const bool have_ws = workspace && workspace_bytes >= ATTN_COUNTER_BYTES && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
@@ -1967,7 +1984,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
 #define KVC_AT(GG)                                                                                              \
     {                                                                                                           \
-        p.brief = 0;                                                                                            \
+        p.brief = p.spare = 0;                                                                                  \
         int workers = rows_fit(p, GG);                                                                          \
         /* (with a tail and columns for all workers a pass of the tail is no step: 1023 columns of 2048 tokens and 64 rows, 4 heads, */ \
         /* a worker per column 464 us, teams as chosen for 18 steps 551) */                                     \
@@ -1977,6 +1994,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         else if (const Spread s = spread(p.work, workers, sms); p.long_runs == splits || s.rounds == 1) workers = (int)s.per_sm; \
         p.brief = GG > 1 && cols * (long long)p.n_tiles <= (long long)workers * sms;                              \
         if (p.brief && attn_smem<GG>(p, workers) > MAX_CTA_SHARED) p.brief = 0;                                 \
+        p.spare = GG > 1 && !p.brief && attn_smem<GG>(p, workers) + 4 * KVC_LUT_SIZE <= MAX_CTA_SHARED;         \
         const size_t smem = attn_smem<GG>(p, workers);                                                          \
         p.workers = workers;                                                                                    \
         const int threads = 128 * (GG == 1 ? workers : rows_workers<GG>());                                     \

@@ -246,26 +246,23 @@ struct KvcRowWriter {
 // no position is kept and no end tested; words are put together by byte permutations and go to places known when the kernel is compiled.
 //   PAIRS    two symbols per lookup, four per round.  Where few windows hold one code only (two codes at the ends of a bell curve), a lane that meets
 //            one falls a symbol behind, up to four: words leave a round late, shifted by what the lane is behind, and every 32 symbols
-//            the lanes catch up if one is three or more behind; one that fell further behind takes its 32 symbols again, one by one.  (A branch for it in every round, taken in every tenth by some lane, cost a
-//            third of the attention kernel's time.)
+//            the lanes catch up if one is three or more behind.  Where a lane fell further behind, the warp takes the 32 symbols again, waiting
+//            for the last lane at every word.  (A branch for it in every round, taken in every tenth by some lane, cost a third of the attention kernel's time.)
 //   SINGLES  one symbol per lookup, for books with longer codes.
 // ESC (of PAIRS and SINGLES): some windows hold no complete code.
 //   WHOLE    the loop above
 enum { KVC_PAIRS = 0, KVC_SINGLES = 1, KVC_WHOLE = 2 };
 // Windows with one code or none, of 4096, up to which a book is decoded by pairs: beyond it catching up costs more than the lookups saved.
-// (Attention, 16 x 16384 tokens, 8 x 4 heads, pairs and singles: V at rel 0.05 (46 windows) 315 and 347 us, K at 0.03 (87) 374 and 347; with longer
-// codes than the window, whose singles are tested one by one, K per block at 0.02 (82) 383 and 404.)
+// (Attention, 16 x 16384 tokens, 8 x 4 heads, pairs and singles: V at rel 0.05 (46 windows) 301 and 341 us, at 0.04 (68) 349 and 341; K, whose lanes have other
+// tokens in every step, bears some more: at 0.032 (64) 309 and 348, at 0.028 (96) 318 and 347, at 0.026 (130) 354 and 348; with longer codes than the window, whose
+// singles are tested one by one, K per block at 0.02 (82) 366 and 404.)
 constexpr uint32_t KVC_PAIRS_LONE = 60, KVC_PAIRS_LONE_ESC = 100;
 
 struct KvcWay { int way; bool esc; };
 __device__ __forceinline__ KvcWay kvc_book_way(const void *book, bool whole) {
     const kvc_book_header *h = reinterpret_cast<const kvc_book_header *>(book);
     if (whole) return {KVC_WHOLE, h->escape != 0};
-    // A code that lacks a branch (a lone symbol's, or a caller's tree) has more nodes than 2 n - 2: PAIRS looks up to four symbols beyond a vector's end,
-    // and what lies there may be no code.  SINGLES reads the 128 and no more.
-    const bool whole_code = h->escape == 0 || h->n_nodes == 2 * h->n_symbols - 2;
-    const bool pairs = whole_code && ((h->lone_windows & 0xffff0000u) == KVC_LONE_KNOWN ? (h->lone_windows & 0xffffu) <= (h->escape ? KVC_PAIRS_LONE_ESC : KVC_PAIRS_LONE)
-                                                                                        : h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS);
+    const bool pairs = (h->lone_windows & 0xffff0000u) == KVC_LONE_KNOWN ? (h->lone_windows & 0xffffu) <= (h->escape ? KVC_PAIRS_LONE_ESC : KVC_PAIRS_LONE) : h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS;
     return {pairs ? KVC_PAIRS : KVC_SINGLES, h->escape != 0};
 }
 // An entry of these ways' tables: byte 0: 16 - bits of its codes, byte 1: 8 where a pair lacks its second symbol, bytes 2 and 3: the symbols.  No complete
@@ -277,8 +274,9 @@ __device__ __forceinline__ uint32_t kvc_way_entry(uint32_t e, bool pairs, const 
     return (16u - bits + (n == 3 ? len[e >> 24] : 0u)) | (n == 1 ? 0x800u : 0u) | (e << 8 & 0xffff0000u);
 }
 // The tables of two books.  All threads of the CTA call; contains a barrier, between the loads (all of them on their way at once) and
-// the stores; the one behind the stores is the caller's.  len: the two books' bits per symbol, 512 bytes.
-__device__ __forceinline__ void kvc_load_ways(uint32_t *lut0, uint32_t *lut1, const void *book0, const void *book1, bool pairs0, bool pairs1, uint8_t *len, int tid, int nthr) {
+// the stores; the one behind the stores is the caller's.  len: the two books' bits per symbol, 512 bytes.  spare1: a table of single symbols of
+// the second book, or null.
+__device__ __forceinline__ void kvc_load_ways(uint32_t *lut0, uint32_t *lut1, uint32_t *spare1, const void *book0, const void *book1, bool pairs0, bool pairs1, uint8_t *len, int tid, int nthr) {
     auto at = [](const void *book, int off) { return reinterpret_cast<const uint8_t *>(book) + off; };
     const uint4 *src0 = reinterpret_cast<const uint4 *>(at(book0, KVC_BOOK_OFF_LUT)), *src1 = reinterpret_cast<const uint4 *>(at(book1, KVC_BOOK_OFF_LUT));
     constexpr int N = KVC_LUT_SIZE / 4, AHEAD = 2;
@@ -294,6 +292,7 @@ __device__ __forceinline__ void kvc_load_ways(uint32_t *lut0, uint32_t *lut1, co
             if (k >= N) break;
             reinterpret_cast<uint4 *>(lut0)[k] = make_uint4(kvc_way_entry(a[j].x, pairs0, len), kvc_way_entry(a[j].y, pairs0, len), kvc_way_entry(a[j].z, pairs0, len), kvc_way_entry(a[j].w, pairs0, len));
             reinterpret_cast<uint4 *>(lut1)[k] = make_uint4(kvc_way_entry(b[j].x, pairs1, len + 256), kvc_way_entry(b[j].y, pairs1, len + 256), kvc_way_entry(b[j].z, pairs1, len + 256), kvc_way_entry(b[j].w, pairs1, len + 256));
+            if (spare1) reinterpret_cast<uint4 *>(spare1)[k] = make_uint4(kvc_way_entry(b[j].x, false, len + 256), kvc_way_entry(b[j].y, false, len + 256), kvc_way_entry(b[j].z, false, len + 256), kvc_way_entry(b[j].w, false, len + 256));
         }
     }
 }
@@ -325,8 +324,8 @@ struct KvcCursor {
     }
     __device__ __forceinline__ uint32_t window() const { return __funnelshift_r(lo, hi, s); }
     __device__ __forceinline__ uint32_t look(uint32_t lut_s, uint32_t t) const { return kvc_lds32(lut_s + (t & ((KVC_LUT_SIZE - 1) << 2))); }
-    // the symbol at the window, from the tree node its bits lead to, bit by bit
-    __device__ __forceinline__ uint32_t walk(uint32_t node, uint32_t tree_s) {
+    // the symbol at the window, from the tree node its bits lead to, bit by bit; counts: it is one of the vector's
+    __device__ __forceinline__ uint32_t walk(uint32_t node, uint32_t tree_s, bool counts) {
         const KvcTreeShared tree{tree_s};
         uint32_t sym = 0;
         bool found = false;
@@ -338,64 +337,82 @@ struct KvcCursor {
             step(s + 31u);
             node = nd >> (16 * bit) & 0xffffu;
         }
-        ok = ok && found;
+        ok = ok && (found || !counts);
         return sym & 0xffu;
     }
-    // two lookups and the step over them
-    template <bool ESC> __device__ __forceinline__ void two(uint32_t lut_s, uint32_t tree_s, uint32_t one, uint32_t &a, uint32_t &b) {
+    // two lookups and the step over them; of their symbols the vector has the first `room` bits (8 per symbol) at least
+    template <bool ESC> __device__ __forceinline__ void two(uint32_t lut_s, uint32_t tree_s, uint32_t one, uint32_t room, uint32_t &a, uint32_t &b) {
         const uint32_t t = window();
         a = look(lut_s, t >> 16);
         b = look(lut_s, __funnelshift_r(t, 0u, a));
         if (ESC && __builtin_expect((a | b) & 0x80u, 0)) {
             // one of them is no code: its symbol by the tree, as an entry of one symbol and no bits
-            if (a & 0x80u) { a = 16u | one | walk(a >> 16, tree_s) << 16; b = look(lut_s, window() >> 16); }
+            if (a & 0x80u) { a = 16u | one | walk(a >> 16, tree_s, room > 0u) << 16; b = look(lut_s, window() >> 16); }
             else { step(s + 16u + (a & 31u)); a = (a & ~31u) | 16u; }
-            if (b & 0x80u) b = 16u | one | walk(b >> 16, tree_s) << 16;
+            if (b & 0x80u) b = 16u | one | walk(b >> 16, tree_s, room > 16u - (a >> 8 & 8u)) << 16;
         }
         step(s + a + b);
     }
-    // PAIRS: the next round; returns the word of the round before (any word in the first one)
-    template <bool ESC> __device__ __forceinline__ uint32_t pairs(uint32_t lut_s, uint32_t tree_s) {
+    // PAIRS: the next two, three or four symbols (any bits on top); now: missing, and 8 bits for each of the four that is not there
+    template <bool ESC> __device__ __forceinline__ uint32_t few(uint32_t lut_s, uint32_t tree_s, uint32_t room, uint32_t missing, uint32_t &now) {
         uint32_t a, b, sel = 0x7632u;
-        two<ESC>(lut_s, tree_s, 0x800u, a, b);
-        asm("dp2a.lo.u32.u32 %0, %1, %2, %0;" : "+r"(sel) : "r"(0x02260000u), "r"(a));         // + 0x1130 where a lacks a symbol: {a0, b0, b1, 0}
-        const uint32_t c = __byte_perm(a, b, sel);
-        const uint32_t out = __funnelshift_rc(last, c, behind);
+        two<ESC>(lut_s, tree_s, 0x800u, room, a, b);
+        asm("dp2a.lo.u32.u32 %0, %1, %2, %0;" : "+r"(sel) : "r"(0x02260000u), "r"(a));         // + 0x1130 where a lacks a symbol: {a0, b0, b1, anything}
         // (the sums by byte products, as the shared-memory pipe and the integer ALU are the busiest)
-        const uint32_t now = (uint32_t)kvc_dp4a_uu(a, 0x100u, kvc_dp4a_uu(b, 0x100u, (int)behind));
+        now = (uint32_t)kvc_dp4a_uu(a, 0x100u, kvc_dp4a_uu(b, 0x100u, (int)missing));
+        return __byte_perm(a, b, sel);
+    }
+    // PAIRS: the next round; returns the word of the round before (any word in the first one).  end: it is the vector's last; what the lane is not
+    // behind by lies beyond the vector, where there may be no code at all.
+    template <bool ESC> __device__ __forceinline__ uint32_t pairs(uint32_t lut_s, uint32_t tree_s, bool end) {
+        uint32_t now;
+        const uint32_t c = few<ESC>(lut_s, tree_s, end ? behind : ~0u, behind, now);
+        const uint32_t out = __funnelshift_rc(last, c, behind);
         last = c << (now - behind);
         behind = now;
         return out;
     }
-    // one symbol, from either table; len_s: the book's bits per symbol
-    template <bool ESC> __device__ __forceinline__ uint32_t single(uint32_t lut_s, uint32_t len_s, uint32_t tree_s) {
-        const uint32_t x = look(lut_s, window() >> 16), sym = x >> 16 & 0xffu;
-        if (ESC && (x & 0x80u)) return walk(x >> 16, tree_s);
-        uint32_t n;
-        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(n) : "r"(len_s + sym));
-        step(s + 32u - n);
-        return sym;
-    }
     // SINGLES: the next word
     template <bool ESC> __device__ __forceinline__ uint32_t singles(uint32_t lut_s, uint32_t tree_s) {
         uint32_t a, b, c, d;
-        two<ESC>(lut_s, tree_s, 0u, a, b);
-        two<ESC>(lut_s, tree_s, 0u, c, d);
+        two<ESC>(lut_s, tree_s, 0u, ~0u, a, b);
+        two<ESC>(lut_s, tree_s, 0u, ~0u, c, d);
         return __byte_perm(__byte_perm(a, b, 0x0062), __byte_perm(c, d, 0x0062), 0x5410);
     }
-    // PAIRS, between two rounds: lanes that are behind fetch what they lack
-    template <bool ESC> __device__ __forceinline__ void catch_up(uint32_t lut_s, uint32_t len_s, uint32_t tree_s) {
-        for (; behind; behind -= 8u) last = last >> 8 | single<ESC>(lut_s, len_s, tree_s) << 24;
+    // PAIRS: the next one or two symbols of a lane, n bits of them
+    template <bool ESC> __device__ __forceinline__ uint32_t take(uint32_t lut_s, uint32_t tree_s, uint32_t &n) {
+        const uint32_t a = look(lut_s, window() >> 16);
+        if (ESC && (a & 0x80u)) { n = 8u; return walk(a >> 16, tree_s, true); }
+        n = 16u - (a >> 8 & 8u);
+        step(s + 16u + (a & 31u));
+        return a >> 16;
     }
-    // back to where the place was
-    __device__ __forceinline__ void back(uint32_t s0, uint32_t ptr0, uint32_t last0, uint32_t behind0) {
-        s = s0; ptr = ptr0; last = last0; behind = behind0;
+    // PAIRS, between two rounds: lanes that are two or more behind fetch what they lack
+    template <bool ESC> __device__ __forceinline__ void catch_up(uint32_t lut_s, uint32_t tree_s) {
+        while (behind >= 16u) {
+            uint32_t n;
+            const uint32_t x = take<ESC>(lut_s, tree_s, n);
+            last = __funnelshift_r(last, x, n);
+            behind -= n;
+        }
+    }
+    // PAIRS, a lane that fell more than a word behind: back to a place 32 symbols ago, and on from there at the lane's own pace.  put(k, word): word k of 8
+    template <bool ESC, class Put> __device__ __forceinline__ void again(uint32_t lut_s, uint32_t tree_s, uint32_t s0, uint32_t ptr0, uint32_t last0, uint32_t behind0, bool end, const Put &put) {
+        s = s0; ptr = ptr0;
         hi = kvc_bswap(kvc_lds32(ptr - 12)); lo = kvc_bswap(kvc_lds32(ptr - 8)); nx = kvc_lds32(ptr - 4);
-    }
-    template <bool ESC> __device__ __forceinline__ uint32_t four(uint32_t lut_s, uint32_t len_s, uint32_t tree_s) {
-        uint32_t w = 0;
+        uint32_t have = 32u - behind0, acc = __funnelshift_rc(last0, 0u, behind0), over = 0u;       // bits that no word has yet
 #pragma unroll 1
-        for (int k = 0; k < 4; k++) w |= single<ESC>(lut_s, len_s, tree_s) << (8 * k);
-        return w;
+        for (uint32_t k = 0; k < 8; ) {
+            if (have < 32u) {
+                uint32_t n;
+                const uint32_t y = few<ESC>(lut_s, tree_s, end && k == 7u ? 32u - have : ~0u, 0u, n), x = y << n >> n;
+                acc |= x << have;
+                over = __funnelshift_lc(x, 0u, have);
+                have += 32u - n;
+            }
+            if (have >= 32u) { put(k, acc); acc = over; over = 0u; have -= 32u; k++; }
+        }
+        behind = 32u - have;                               // (8 to 32: a word takes 56 bits at most)
+        last = __funnelshift_lc(0u, acc, behind);
     }
 };
