@@ -710,7 +710,8 @@ struct alignas(32) RowsWorker {
     int okK[4], okV[4];
     int next_j, dead;
 };
-struct alignas(32) RowsTables { uint32_t lutK[KVC_LUT_SIZE], lutV[KVC_LUT_SIZE]; uint32_t tree[2][512]; uint8_t len[512]; };   // the trees are for codes beyond the window
+struct alignas(32) OneTables { uint32_t lutK[KVC_LUT_SIZE], lutV[KVC_LUT_SIZE]; };       // (the one-head kernel reads its trees from global memory)
+struct RowsTables : OneTables { uint32_t tree[2][512]; uint8_t len[512]; };              // the trees are for codes beyond the window
 
 // shared memory of a CTA: tables, workers, slots (two of K and two of V each), rows; a corrupt stream's overrun ends in the rows
 template <int G> size_t rows_smem(const AttnParams &p, int workers) {
@@ -1231,7 +1232,7 @@ struct alignas(32) OneWorker {
 };
 // tables, workers, slots (two of K and two of V each), bytes that a corrupt stream's overrun may read
 size_t one_smem(const AttnParams &p, int workers) {
-    return sizeof(RowsTables) + workers * (sizeof(OneWorker) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes)) + SLOT_PAD;
+    return sizeof(OneTables) + workers * (sizeof(OneWorker) + 2 * (size_t)(p.slotK_bytes + p.slotV_bytes)) + SLOT_PAD;
 }
 int one_fit(const AttnParams &p) {
     int workers = ONE_WORKERS;
@@ -1277,10 +1278,10 @@ __device__ __forceinline__ void sts8(uint32_t addr, uint32_t v) { asm volatile("
 template <bool BULK, bool TEAM>
 __global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    RowsTables &tab = *reinterpret_cast<RowsTables *>(smem_raw);
+    OneTables &tab = *reinterpret_cast<OneTables *>(smem_raw);
     const int workers = blockDim.x >> 7, wk = threadIdx.x >> 7;
     const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, sub = tid >> 6, v = tid & 63;
-    uint8_t *const wbase = smem_raw + sizeof(RowsTables), *const sbase = wbase + workers * sizeof(OneWorker);
+    uint8_t *const wbase = smem_raw + sizeof(OneTables), *const sbase = wbase + workers * sizeof(OneWorker);
     OneWorker &sm = reinterpret_cast<OneWorker *>(wbase)[wk];
     uint8_t *const slotsK = sbase + wk * 2 * (p.slotK_bytes + p.slotV_bytes), *const slotsV = slotsK + 2 * p.slotK_bytes;
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
