@@ -74,8 +74,14 @@ def _cache(ops, kind, shape, is_k, g):
 @pytest.mark.parametrize("G", [2, 4, 8])
 @pytest.mark.parametrize("kk,vk", [("pairs", "misses"), ("misses", "pairs"), ("singles", "misses"), ("pairs_long", "singles"), ("singles_long", "pairs_long"),
                                    ("misses", "singles_long")])
-@pytest.mark.parametrize("T,B,H", [(1536, 16, 4), (256, 2, 1)])       # steps for several rounds of workers; a step per worker
-def test_ways(ops, G, kk, vk, T, B, H):
+@pytest.mark.parametrize("T,B,H,rounds", [(1536, 16, 4, None), (6144, 16, 4, 4), (256, 2, 1, 0)])    # (rounds of steps that the device's workers take)
+def test_ways(ops, G, kk, vk, T, B, H, rounds):
+    workers = 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    steps = B * H * T // 128
+    if rounds == 0:
+        assert steps <= workers                            # vectors are decoded whole
+    elif rounds:
+        assert steps > rounds * workers                    # by pairs and singles; items of several steps
     g = torch.Generator(device="cuda").manual_seed(T + G)
     kc, ke, keep_k = _cache(ops, kk, (T, B, H, 128), True, g)
     vc, ve, keep_v = _cache(ops, vk, (T, B, H, 128), False, g)

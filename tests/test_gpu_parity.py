@@ -681,7 +681,7 @@ def _skewed_cache(ops, rng, is_k, T, B, H):
 @pytest.mark.parametrize("G", [1, 2, 4, 3, 5, 8, 9])
 def test_attn_decode_books_with_long_codes(ops, G):
     """Books whose header says `escape`: the fused kernels take the decoder that tests every table entry and
-    continues bit by bit from the tree in global memory -- with one query head per KV head and with
+    continues bit by bit from the tree -- with one query head per KV head and with
     several, in two, four and eight columns (3, 5: padded; 9: two launches) -- with and without a workspace."""
     rng = np.random.default_rng(5 + G)
     T, B, Hkv = 512, 2, 2
