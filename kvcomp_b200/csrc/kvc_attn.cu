@@ -179,8 +179,9 @@ template <int G> struct RowsSum {
         }
     }
 };
-// What a vector is decoded from: shared addresses of its slot, the table and the tree
-struct RowsFrom { uint32_t slot, at, lut, tree; };
+// What a vector is decoded from: shared addresses of its slot, the table (of single symbols: lone) and the tree.  (Both tables' addresses are the same for the
+// whole launch: one that is chosen from step to step costs an addition per lookup, 2 % of the kernel's time.)
+struct RowsFrom { uint32_t slot, at, lut, lone, tree; };
 
 // lagged: in how many of the four parts a lane fell too far behind for PAIRS' rounds.
 template <int G, int WAY, bool ESC>
@@ -191,7 +192,7 @@ __device__ __forceinline__ bool rows_dot_way(const RowsFrom &f, uint32_t rows_s,
     const uint32_t col = w_s + (r % (2 * G)) * (COL_WORDS * 4) + q * 8;
     KvcCursor at(f.slot, f.at);
     RowsSum<G> sum;
-    auto word = [&](bool end) { return WAY == KVC_PAIRS ? at.pairs<ESC>(f.lut, f.tree, end) : at.singles<ESC>(f.lut, f.tree); };
+    auto word = [&](bool end) { return WAY == KVC_PAIRS ? at.pairs<ESC>(f.lut, f.tree, end) : at.singles<ESC>(f.lone, f.tree); };
     if (WAY == KVC_PAIRS) word(false);
 #pragma unroll 1
     for (uint32_t ch = 0; ch < 4; ch++) {
@@ -836,7 +837,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     } else kvc_load_ways(tab.lutK, tab.lutV, spare_in ? spare : nullptr, p.k.book, p.v.book, wayK.way == KVC_PAIRS, wayV.way == KVC_PAIRS, tab.len, threadIdx.x, blockDim.x);
     if (wayK.esc) kvc_load_tree(tab.tree[0], p.k.book, threadIdx.x, blockDim.x);
     if (wayV.esc) kvc_load_tree(tab.tree[1], p.v.book, threadIdx.x, blockDim.x);
-    const uint32_t lutK_s = kvc_smem_addr(tab.lutK), lutV_s = kvc_smem_addr(tab.lutV), tree_s = kvc_smem_addr(tab.tree), spare_s = kvc_smem_addr(spare);
+    const uint32_t lutK_s = kvc_smem_addr(tab.lutK), lutV_s = kvc_smem_addr(tab.lutV), tree_s = kvc_smem_addr(tab.tree), loneV_s = spare_in ? kvc_smem_addr(spare) : lutV_s;
 
     struct StepMeta { unsigned short startK, startV, vsc, ksc; int vmi, kmi; KUnit ku; };   // as loaded: no arithmetic waits on them here
     auto load_meta = [&](bool on, int b, int h, int col, int step, StepMeta &m) {
@@ -944,7 +945,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             const uint32_t start = cur.startK >> 3;
             bool ok = k_landed && sm.okK[sub] && start < sm.nbK[sub];              // a vector begins inside its block
             uint32_t lagged = 0;
-            ok = rows_dot<G>(wayK, {kvc_smem_addr(slotsK + sub * p.slotK_bytes), ok ? sm.leadK[sub] + start : 1u, lutK_s, tree_s}, rows_s, kvc_smem_addr(sm.w + sub * VW), lane, d, lagged) && ok;
+            ok = rows_dot<G>(wayK, {kvc_smem_addr(slotsK + sub * p.slotK_bytes), ok ? sm.leadK[sub] + start : 1u, lutK_s, lutK_s, tree_s}, rows_s, kvc_smem_addr(sm.w + sub * VW), lane, d, lagged) && ok;
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
             const uint32_t unit = (uint32_t)cur.ksc | ((uint32_t)cur.kmi << 16);   // of the token `vec`
 #pragma unroll
@@ -1064,7 +1065,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
             // (and so does a warp whose lanes lag in two parts of four, for the rest of the item)
             uint32_t lagged = 0;
             const bool lone = (par & 4u) != 0;
-            ok = rows_dot<G>(lone ? KvcWay{KVC_SINGLES, wayV.esc} : wayV, {kvc_smem_addr(slotsV + sub * p.slotV_bytes), ok ? sm.leadV[sub] + startV : 1u, lone ? spare_s : lutV_s, tree_s + 2048u}, rows_s, kvc_smem_addr(sm.w + 2 * VW), lane, d, lagged) && ok;
+            ok = rows_dot<G>(lone ? KvcWay{KVC_SINGLES, wayV.esc} : wayV, {kvc_smem_addr(slotsV + sub * p.slotV_bytes), ok ? sm.leadV[sub] + startV : 1u, lutV_s, loneV_s, tree_s + 2048u}, rows_s, kvc_smem_addr(sm.w + 2 * VW), lane, d, lagged) && ok;
             if (spare_in && lagged >= 2u) par |= 4u;
             if (!ok) flags |= KVC_FLAG_BAD_STREAM;
 #pragma unroll
