@@ -99,9 +99,11 @@ constexpr int WROW = 136;                 // weight words per vector of the one-
 // warp's loads (four rows, 8 bytes a lane) then meet every bank once.  32 symbols are one k step of the matrix instruction:
 // the rows of a warp take 1 KB instead of 4.5.
 constexpr int ROW_BYTES = 32;
-// A brief launch (a step per worker at most) is a matter of latency: its vectors are decoded whole, with up to three symbols per lookup and no
-// table to be made first, into rows of 128 symbols, the overrun of paired lookups and a 16-byte alignment that spreads over the banks.  (2 columns of
-// 8192 tokens, 4 heads: by pairs 18.2 us, whole 13.4; 12 columns of 2816, 6 heads: 24.8 and 23.2.)
+// A brief launch (two steps per worker, one after the other, at most) is a matter of latency: its vectors are decoded whole, with up to three symbols per lookup and no
+// table to be made first, into rows of 128 symbols, the overrun of paired lookups and a 16-byte alignment that spreads over the banks.  (Device time by pairs or
+// singles, and whole: 2 columns of 8192 tokens, 4 heads, 16.5 and 13.3 us; 128 columns of 512, 22.0 and 20.8, of 768, two steps per worker, 31.2 and 29.4,
+// at rel 0.02 / 0.02 38.5 and 33.3; of 1536, three steps, 45.5 either way; without a workspace 32 columns of 2048, four steps, 48.0 and 49.1, 8 of 8192 147 and 157.)
+constexpr int BRIEF_STEPS = 2;
 constexpr int WHOLE_ROW_BYTES = 144;
 static_assert(WHOLE_ROW_BYTES >= 128 + KVC_DECODE_OVERRUN + 3, "rows too short for paired lookups");
 // A vector's weights: two columns per head, the hi and the lo bytes of 4 positions to a word.  Column stride 40 words: the fragment
@@ -676,7 +678,7 @@ struct AttnParams {
     int *sched;                   // {items handed out, workers finished}, or null: static shares
     int *status;
     int workers;                  // per CTA
-    int brief;                    // a step per worker at most: vectors are decoded whole
+    int brief;                    // BRIEF_STEPS steps per worker at most: vectors are decoded whole
     int spare;                    // there is room for a table of V's single symbols beside that of pairs
     int team;                     // without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
@@ -1994,7 +1996,10 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         if (p.team) workers = p.team * (int)spread(cols, workers / p.team, sms).per_sm;                         \
         /* (short runs at the end of the columns fill the last round up; a single round spreads over all SMs) */ \
         else if (const Spread s = spread(p.work, workers, sms); p.long_runs == splits || s.rounds == 1) workers = (int)s.per_sm; \
-        p.brief = GG > 1 && cols * (long long)p.n_tiles <= (long long)workers * sms;                              \
+        /* (steps that a worker takes one after the other) */                                                   \
+        const long long steps = p.team ? spread(cols, workers / p.team, sms).rounds * ((p.n_tiles + p.team - 1) / p.team) \
+                                       : spread(p.work, workers, sms).rounds * std::min(p.tiles_per_split, p.n_tiles);     \
+        p.brief = GG > 1 && steps <= BRIEF_STEPS;                                                               \
         if (p.brief && attn_smem<GG>(p, workers) > MAX_CTA_SHARED) p.brief = 0;                                 \
         p.spare = GG > 1 && !p.brief && attn_smem<GG>(p, workers) + 4 * KVC_LUT_SIZE <= MAX_CTA_SHARED;         \
         const size_t smem = attn_smem<GG>(p, workers);                                                          \
