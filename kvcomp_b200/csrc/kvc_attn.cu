@@ -110,10 +110,8 @@ static_assert(WHOLE_ROW_BYTES >= 128 + KVC_DECODE_OVERRUN + 3, "rows too short f
 // loads (four columns x 32 bytes per half warp) meet every bank once.
 constexpr int COL_WORDS = 40;
 __host__ __device__ constexpr int vec_words(int G) { return 2 * G * COL_WORDS; }
-// 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -128 * 257 .. 127 * 257.
-// K's weights: the largest one takes -32768, so its step is a power of two of it and the score of a single channel is exact.  Where the largest of the other
-// sign is within 0.4 % of it, that one takes 32639 and the step is up to 0.4 % coarser.
-constexpr float FIX_K = 32768.0f, FIX_UP = 32639.0f;
+// 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -32767 .. 127 * 256 + 127
+constexpr float FIX_DOWN = 32767.0f, FIX_UP = 32639.0f;
 // V's weights: the largest one is 1 and takes 32880 (below the end, 32896, by what the approximate logarithm and power can be off together).
 // Their reference is a score plus a logarithm, rounded up: below FAR that lowers them by a factor of exp(-2^-9) at most, and the fixed-point step stays
 // finer than 1/32767 of the largest.  Beyond FAR the reference is the largest score itself, and the largest weight is looked for.
@@ -175,7 +173,7 @@ template <int G> struct RowsSum {
     }
     __device__ __forceinline__ void out(int (&d)[4][HL]) const {
 #pragma unroll
-        for (int j = 0; j < HL; j++) {                         // |256 hi + lo| <= 128 * 255 * 32896 < 2^31
+        for (int j = 0; j < HL; j++) {                         // |256 hi + lo| <= 128 * 255 * 32767 < 2^31
             d[0][j] = 256 * c[j][0][0] + c[j][0][1]; d[1][j] = 256 * c[j][0][2] + c[j][0][3];
             d[2][j] = 256 * c[j][1][0] + c[j][1][1]; d[3][j] = 256 * c[j][1][2] + c[j][1][3];
         }
@@ -439,11 +437,11 @@ __device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *
         const float4 x = *reinterpret_cast<const float4 *>(q + g * 128 + lane * 4);
         const float w0 = x.x * sc[0], w1 = x.y * sc[1], w2 = x.z * sc[2], w3 = x.w * sc[3];
         z[gi] = fmaf(mz[0], x.x, fmaf(mz[1], x.y, fmaf(mz[2], x.z, mz[3] * x.w)));
-        // The largest value of either sign (floats without a sign order as integers do).  The larger one takes the negative side of the range,
-        // which reaches further.
+        // The largest value of either sign (floats without a sign order as integers do).  The larger one takes the negative end of the range,
+        // which reaches 32767; the positive end reaches 32639.
         const float up = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fmaxf(w0, w1), fmaxf(w2, w3)), 0.f)) & 0x7fffffffu));
         const float down = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fminf(fminf(fminf(w0, w1), fminf(w2, w3)), 0.f)) & 0x7fffffffu));
-        const float big = fmaxf(up, down), st = fmaxf(big * (1.0f / FIX_K), fminf(up, down) * (1.0f / FIX_UP));
+        const float big = fmaxf(up, down), st = fmaxf(big * (1.0f / FIX_DOWN), fminf(up, down) * (1.0f / FIX_UP));
         const float inv = big > 1e-30f ? rcp_fast(st) : 0.f;
         const uint2 r = pack_fix(w0, w1, w2, w3, up > down ? -inv : inv);
         w[2 * g * COL_WORDS + lane] = r.x; w[(2 * g + 1) * COL_WORDS + lane] = r.y;

@@ -127,7 +127,7 @@ def test_what_is_not_finite_reaches_the_output(ops, G, long, where, value):
 
 @pytest.mark.parametrize("long", [False, True])
 @pytest.mark.parametrize("G", [2, 4, 8])
-@pytest.mark.parametrize("q0", [10.0, 1000.0, 4097.0, 60000.0, -39999.0])
+@pytest.mark.parametrize("q0", [10.0, 1000.0, 4097.0, 60000.0])
 @pytest.mark.parametrize("kw", [dict(), dict(splits=4), dict(splits=1, workspace=False)])
 def test_equal_scores_weigh_the_same(ops, G, long, q0, kw):
     """One channel of the query is not zero, and there all keys are equal: every token has the same score, which 32 bits hold."""
