@@ -13,18 +13,18 @@
 //   V phase: thread = (128-token group, channel); its vector holds 128 tokens of that channel.
 //            out[ch] = sum_t code_t * ps[t] + zpv, with ps[t] = p[t]*scale[t] staged per group.
 // The attention kernels are launched with as many workers as the device holds at once.  Their work is cut into
-// items (one (b, kv head) column x one run of steps); a worker starts with two items fixed by
-// its index and draws the rest from a counter two items ahead, so that the workers an SM's schedulers
-// favour take more of them.  Staging copies, a step's metadata and the query vector of the next step or
+// items (one (b, kv head) column x one run of steps); a worker starts with items fixed by its index and draws the rest
+// from a counter, so that the workers an SM's schedulers favour take more of them: with one head per KV head two fixed and
+// two ahead, with several one fixed and one ahead.  Staging copies, a step's metadata and the query vector of the next step or
 // item are always fetched while the current one is decoded.  When a column has more than one item,
 // each leaves a partial result (max, sum, accumulators) and a second kernel merges them.
 // Both phases are "decode 128 symbols and dot them with a shared 128-vector", so they share one
-// decoder.  The shared vector is held in 16-bit block fixed point (one fp32 step per vector, value
-// = step * (256*hi + lo), hi signed and lo unsigned bytes): every table lookup yields up to three
-// symbols as bytes, and two dp4a instructions multiply them with the matching weight bytes -- integer arithmetic, exact, accumulated in int32.  The only rounding is that of the
-// weights (2^-16 of the largest weight of the vector); the zero-point terms and everything after
-// the dot product are fp32.  With several query heads per KV head they share every decode: in the unfused
-// kernels by weight records [position][G], up to four heads a launch, in the attention kernel see attn_rows_kernel.
+// decoder.  The shared vector is held in 16-bit block fixed point, one fp32 step per vector; the products with the symbols are integer arithmetic,
+// exact, accumulated in int32.  The only rounding is that of the weights (2^-16 of the largest weight of the vector); the zero-point terms and
+// everything after the dot product are fp32.  In the unfused kernels and with one head per KV head a weight is step * (256*hi + lo), hi a signed and
+// lo an unsigned byte: every table lookup yields up to three symbols as bytes, and two dp4a instructions multiply them with the matching weight
+// bytes.  With several query heads per KV head they share every decode: in the unfused kernels by weight records [position][G], up to four heads
+// a launch, in the attention kernel by matrix instructions with both bytes signed (attn_rows_kernel).
 #include <math_constants.h>
 #include <string.h>
 
@@ -88,11 +88,11 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 // lanes at 32 different positions fetch 0.5 KB and more per lookup: the kernel becomes bound by shared-memory
 // wavefronts.  So a warp decodes 32 symbols of each of its 32 vectors into rows of bytes in shared memory (KvcCursor: every lane
 // at the same position), and m16n8k32 integer instructions multiply the rows with the weights: two columns per head, the hi and
-// the lo bytes.  The integer sums are the same as in the one-pass form.  What bounds it: the shared-memory pipe (846 wavefronts per warp
-// and step of 128 tokens, 76 % busy; nine per round of two lookups) and, with 2570 instructions, issue (59 %) together.  One layer of
+// the lo bytes.  The integer sums are the same as in the one-pass form.  What bounds it: the shared-memory pipe (849 wavefronts per warp
+// and step of 128 tokens, 76 % busy; nine per round of two lookups) and, with 2610 instructions, issue (59 %) together.  One layer of
 // 16 sequences x 32768 tokens, 8 x 4 heads, rel 0.05 / 0.1: whole rows, each lane at its own position, up to three symbols per lookup (3440 instructions,
-// 1010 wavefronts) 650 us, now 536; 32 x 16384 tokens, 10 x 4, rel 0.02 / 0.15, 868 and 828; 8192 tokens of the first, 184 and 154.  Six workers of 80
-// registers are no faster than five of 96; tables of 8 to 12 bits repeated over the banks (32 KB each, one symbol per lookup) 660 us.
+// 1010 wavefronts) 650 us, now 536; 32 x 16384 tokens, 10 x 4, rel 0.02 / 0.15, 868 and 835; 4096 tokens of the first, 104 and 88.  (In an earlier state six workers
+// of 80 registers took 562 to 576 us where five of 96 took 577; tables of 8 to 12 bits repeated over the banks, 32 KB each, one symbol per lookup, 660.)
 constexpr int WROW = 136;                 // weight words per vector of the one-pass form: 128 positions + zeroed overrun
 
 // Rows of 32 symbols, two units of 16 bytes each, swapped in every other four rows: a quarter warp's stores (eight rows, one unit) and a half
@@ -110,7 +110,9 @@ static_assert(WHOLE_ROW_BYTES >= 128 + KVC_DECODE_OVERRUN + 3, "rows too short f
 // loads (four columns x 32 bytes per half warp) meet every bank once.
 constexpr int COL_WORDS = 40;
 __host__ __device__ constexpr int vec_words(int G) { return 2 * G * COL_WORDS; }
-// 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -32767 .. 127 * 256 + 127
+// 16-bit fixed point as two signed bytes (value = step * (256 * hi + lo)): -128 * 257 .. 127 * 257.
+// K's weights: the larger sign takes the negative side, to -32767.  Where the largest of the other sign is within 0.4 % of it, that one takes 32639, and the
+// step is up to 0.4 % coarser than in a symmetric range.
 constexpr float FIX_DOWN = 32767.0f, FIX_UP = 32639.0f;
 // V's weights: the largest one is 1 and takes 32880 (below the end, 32896, by what the approximate logarithm and power can be off together).
 // Their reference is a score plus a logarithm, rounded up: below FAR that lowers them by a factor of exp(-2^-9) at most, and the fixed-point step stays
@@ -173,7 +175,7 @@ template <int G> struct RowsSum {
     }
     __device__ __forceinline__ void out(int (&d)[4][HL]) const {
 #pragma unroll
-        for (int j = 0; j < HL; j++) {                         // |256 hi + lo| <= 128 * 255 * 32767 < 2^31
+        for (int j = 0; j < HL; j++) {                         // |256 hi + lo| <= 128 * 255 * 32896 < 2^31
             d[0][j] = 256 * c[j][0][0] + c[j][0][1]; d[1][j] = 256 * c[j][0][2] + c[j][0][3];
             d[2][j] = 256 * c[j][1][0] + c[j][1][1]; d[3][j] = 256 * c[j][1][2] + c[j][1][3];
         }
@@ -425,15 +427,14 @@ __device__ __forceinline__ void k_weights_build(uint32_t *w, float *step, float 
 template <int G>
 __device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *zp, const float *q, const KUnit &u, bool channel_units, int min_bytes,
                                                int part, int lane) {
-    constexpr int GP = G >= 2 ? G / 2 : 1;
-    if (G == 1 && part) return;
+    constexpr int GP = G / 2;
     float sc[4], mz[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) { sc[i] = kvc_scale_value(ku_scale(u, i)); mz[i] = (float)ku_min(u, i, min_bytes) * sc[i]; }
     float z[GP];
 #pragma unroll
     for (int gi = 0; gi < GP; gi++) {
-        const int g = part * (GP) + gi;
+        const int g = part * GP + gi;
         const float4 x = *reinterpret_cast<const float4 *>(q + g * 128 + lane * 4);
         const float w0 = x.x * sc[0], w1 = x.y * sc[1], w2 = x.z * sc[2], w3 = x.w * sc[3];
         z[gi] = fmaf(mz[0], x.x, fmaf(mz[1], x.y, fmaf(mz[2], x.z, mz[3] * x.w)));
@@ -447,18 +448,18 @@ __device__ __forceinline__ void k_weights_rows(uint32_t *w, float *step, float *
         w[2 * g * COL_WORDS + lane] = r.x; w[(2 * g + 1) * COL_WORDS + lane] = r.y;
         if (lane == 0) step[g] = up > down ? -st : st;
     }
-    if (!channel_units) { if (lane < GP) zp[part * (GP) + lane] = 0.f; return; }
+    if (!channel_units) { if (lane < GP) zp[part * GP + lane] = 0.f; return; }
 #pragma unroll
     for (int gi = 0; gi < GP; gi += 2) {                    // two heads' sums in one go: one to either half of the warp
         float a = z[gi];
         if (GP > 1) {
-            const float z1 = z[(gi + 1) % (GP)];
+            const float z1 = z[(gi + 1) % GP];
             const float give = lane < 16 ? z1 : a;
             a = (lane < 16 ? a : z1) + __shfl_xor_sync(0xffffffffu, give, 16);
         } else a += __shfl_xor_sync(0xffffffffu, a, 16);
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if ((lane & 15) == 0 && (GP > 1 || lane == 0)) zp[part * (GP) + gi + (lane >> 4)] = a;
+        if ((lane & 15) == 0 && (GP > 1 || lane == 0)) zp[part * GP + gi + (lane >> 4)] = a;
     }
 }
 
@@ -731,7 +732,7 @@ int rows_fit(const AttnParams &p, int heads) { return heads == 1 ? one_fit(p) : 
 // Equal items for `most` takers per SM: in how many rounds they go, and the takers that this many rounds need: those of a
 // fuller SM would run slower and the last round leave more of them idle.  (One head, seven workers at first, device time: 320 columns
 // of 6144 tokens in 4 runs 254 us, now 229 (three CTAs of 256 threads, the kernel before the workers: 250); 192 of 4096 in 6 runs 127 and 107; 36 of
-// 4096, the library's plan, 36 and 27; 800 columns of 128 tokens, 4 heads, 39 and 31.)
+// 4096, the library's plan, 36 and 27; 800 columns of 128 tokens, 4 heads, 34 and 28.)
 struct Spread { long long rounds, per_sm; };
 Spread spread(long long items, long long most, long long sms) {
     const long long rounds = (items + most * sms - 1) / (most * sms);
@@ -740,11 +741,11 @@ Spread spread(long long items, long long most, long long sms) {
 
 // How many of an SM's workers share a column when every column's output is written directly (no workspace, or a single run
 // without a tail): without company a worker would take all of a column's `units` (steps and passes of the tail) in turn
-// while most of the device is idle.  A unit takes about 6 + a parts of time with `a` workers at work on the SM (2 heads: 9.2 us
-// alone, 14.4 us with five), a team's sums and its next column another 3.5: over 1 to 700 columns of 2 to 19 units the choice is
-// within 1 % of the best size on average, and nowhere behind a worker per column.  2 heads per column, no workspace, a worker per column
-// against teams: 8 columns of 1024 tokens 77.6 and 31.5 us, 64 of 8192 594 and 189 us, 256 of 256 (two teams of two on an SM) 26.1 and
-// 19.6 us; more columns than workers, where a worker per column goes in two rounds, the second nearly empty: 1280 of 1024 tokens,
+// while most of the device is idle.  A unit takes about 6 + a parts of time with `a` workers at work on the SM (2 heads: 7.1 us
+// alone, 11.9 us with five), a team's sums and its next column another 3.5 (fitted to steps of 9.2 and 14.4 us: over 1 to 700 columns of 2 to 19 units the
+// choice was within 1 % of the best size on average, and nowhere behind a worker per column).  2 heads per column, no workspace, a worker per column
+// against teams: 8 columns of 1024 tokens 53.3 and 26.6 us, 64 of 8192 457 and 148 us, 256 of 256 (two teams of two on an SM) 22.1 and
+// 16.8 us; more columns than workers, where a worker per column goes in two rounds, the second nearly empty: 1280 of 1024 tokens,
 // one head, 236 and 165 us.
 int rows_team(long long cols, long long units, int workers, int sms) {       // (0: each its own columns)
     int best = 0;
@@ -1964,12 +1965,12 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         if (p.partial && ws_parts) {
             RunPlan r = {0, 0, 0, 0};
             // (with grouped queries the plan counts five workers per SM also where the launch has fewer: the items are finer for it.  8 heads, four
-            // workers: 16 x 8 columns of 16384 tokens 412 us, with a plan for four 423; 32 x 2 columns 217 and 224.  Three workers, as the
-            // stream's largest block is unknown: 484 and 490 us, but 16 x 8 columns of 4096 tokens 144 and 137.)
+            // workers: 16 x 8 columns of 16384 tokens 338 us, with a plan for four 345; 32 x 2 columns 191 and 195; 16 x 8 of 4096 115 either way.  Three
+            // workers, as the stream's largest block is unknown: 399 and 402 us.)
             if (asked <= 0) r = plan_runs(p.n_tiles, cols, heads == 1 ? most : (long long)ROWS_PLANNED * sms);
             // The caller's runs in halves where that is fewer steps one after the other: a worker takes a run's steps in turn, each
             // with 128 threads.  (32 columns, 2 heads each, 2048 tokens in 4
-            // runs: 46.9 us, in halves 33.7; 64 columns in 8 runs: 36.0, in halves 42.2, as the halves no longer go in one round.)
+            // runs: 37.0 us, in halves 22.1; 64 columns in 8 runs: 29.4, in halves 31.3, as the halves no longer go in one round.)
             else if ((2 * cols * splits + most - 1) / most < 2 * ((cols * splits + most - 1) / most)) {
                 r.tps = r.short_tiles = tps;
                 r.splits = r.long_runs = (p.n_tiles + tps - 1) / tps;
@@ -1981,7 +1982,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         p.work = cols * splits;
         for (long long g0 = 0; g0 < Gt; g0 += p.nh) {
             // Heads per launch: every launch decodes the whole cache, so up to 8 go together, in launches of equal shares.
-            // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 461 us in two launches of 4, 217 us in one.)
+            // (32 sequences x 16384 tokens, 2 x 8 heads, K rel 0.05: 321 us in two launches of 4, 181 us in one.)
             const long long launches = (Gt - g0 + 7) / 8;
             p.g0 = g0; p.nh = (int)((Gt - g0 + launches - 1) / launches);
 #define KVC_AT(GG)                                                                                              \
@@ -1989,7 +1990,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         p.brief = p.spare = 0;                                                                                  \
         int workers = rows_fit(p, GG);                                                                          \
         /* (with a tail and columns for all workers a pass of the tail is no step: 1023 columns of 2048 tokens and 64 rows, 4 heads, */ \
-        /* a worker per column 464 us, teams as chosen for 18 steps 551) */                                     \
+        /* a worker per column 440 us, teams as chosen for 18 steps 503) */                                     \
         p.team = p.partial || (Tr > 0 && cols >= (long long)workers * sms) ? 0 : rows_team(cols, p.n_tiles + (Tr + 127) / 128, workers, sms); \
         if (p.team) workers = p.team * (int)spread(cols, workers / p.team, sms).per_sm;                         \
         /* (short runs at the end of the columns fill the last round up; a single round spreads over all SMs) */ \
