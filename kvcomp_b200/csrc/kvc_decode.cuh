@@ -255,14 +255,19 @@ enum { KVC_PAIRS = 0, KVC_SINGLES = 1, KVC_WHOLE = 2 };
 // Windows with one code or none, of 4096, up to which a book is decoded by pairs: beyond it catching up costs more than the lookups saved.
 // (Attention, 16 x 16384 tokens, 8 x 4 heads, pairs and singles: V at rel 0.05 (46 windows) 301 and 341 us, at 0.04 (68) 349 and 341; K, whose lanes have other
 // tokens in every step, bears some more: at 0.032 (64) 309 and 348, at 0.028 (96) 318 and 347, at 0.026 (130) 354 and 348; with longer codes than the window, whose
-// singles are tested one by one, K per block at 0.02 (82) 366 and 404.)
+// singles are tested one by one, K per block at 0.02 (82 windows, 51 symbols) 362 and 390.)  Where codes go beyond the window, larger alphabets have more of them
+// in the same few channels, and every lane of a warp walks the tree there and falls behind: K per block at 0.018 (82, 57) 381 and 388, at 0.016 (82, 63) 408 and
+// 392, at 0.014 (82, 73) 446 and 400, there with 8 heads per KV head 522 and 476; whole rows took 392, 406, 435 and 477.
 constexpr uint32_t KVC_PAIRS_LONE = 60, KVC_PAIRS_LONE_ESC = 100;
+constexpr int KVC_PAIRS_SYMBOLS_ESC = 60;
 
 struct KvcWay { int way; bool esc; };
 __device__ __forceinline__ KvcWay kvc_book_way(const void *book, bool whole) {
     const kvc_book_header *h = reinterpret_cast<const kvc_book_header *>(book);
     if (whole) return {KVC_WHOLE, h->escape != 0};
-    const bool pairs = (h->lone_windows & 0xffff0000u) == KVC_LONE_KNOWN ? (h->lone_windows & 0xffffu) <= (h->escape ? KVC_PAIRS_LONE_ESC : KVC_PAIRS_LONE) : h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS;
+    const uint32_t lone = h->lone_windows & 0xffffu;
+    const bool pairs = (h->lone_windows & 0xffff0000u) != KVC_LONE_KNOWN ? h->escape == 0 && 2 * h->max_len <= KVC_LUT_BITS
+                       : h->escape == 0 ? lone <= KVC_PAIRS_LONE : lone <= KVC_PAIRS_LONE_ESC && h->n_symbols <= KVC_PAIRS_SYMBOLS_ESC;
     return {pairs ? KVC_PAIRS : KVC_SINGLES, h->escape != 0};
 }
 // An entry of these ways' tables: byte 0: 16 - bits of its codes, byte 1: 8 where a pair lacks its second symbol, bytes 2 and 3: the symbols.  No complete

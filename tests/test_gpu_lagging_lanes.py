@@ -118,3 +118,50 @@ def test_a_channel_of_long_codes_does_not_stop_the_others(ops):
             each.append(a.elapsed_time(b))
         times.append(sorted(each)[len(each) // 2])
     assert times[1] <= 1.55 * times[0], times
+
+
+def test_large_alphabets_with_long_codes_go_by_single_symbols(ops):
+    """Keys with a unit per block at a tight bound: the few channels far beyond the others hold the codes beyond the window, and every lane of a warp meets them
+    at once.  What the device takes against the same book that says it has few symbols, and goes by pairs (measured: 0.90)."""
+    from kvcomp_b200.synth import make_kv
+    T, B, H = _shape(8)
+    k, v, q = make_kv(T, B, H, 128, seed=1, device="cuda", Hq=H * 4)
+    k.clamp_(-24.0, 24.0)
+    q = (q.float() * math.sqrt(128)).half()
+    caches = []
+    for x, is_k, mode, rel in ((k, True, ops.MODE_BLOCK, 0.014), (v, False, ops.MODE_TOKEN, 0.1)):
+        hist = torch.zeros(256, dtype=torch.int64, device="cuda")
+        codes, mi, sc, spec, _ = ops.quantize(x, mode, 64, rel, False, min_dtype=torch.int16, hist=hist)
+        book = ops.build_codebook(hist)
+        bsz, tsz, _, n = ops.buffer_sizes(T, B * H * 128, is_k)
+        bi, ti = torch.empty(bsz, dtype=torch.uint8, device="cuda"), torch.empty(tsz // 2, dtype=torch.int16, device="cuda")
+        enc = torch.empty(n, dtype=torch.uint8, device="cuda")
+        total, st = ops.encode(codes, is_k, book.encode_table(), bi, ti, enc)
+        size, largest = total.tolist()
+        assert ops.read_status(st) & ~ops._lib.FLAG_VECTOR_LONG == 0
+        caches.append((enc, bi, ti, book, mi, sc, spec, size, largest))
+    enc, bi, ti, book, mi, sc, spec, size, largest = caches[0]
+    head = book.header()
+    assert head["escape"] == 1 and head["n_symbols"] > 60 and (book.host()[32:36].view(torch.int32).item() & 0xffff) < 120
+    few, many = type(book)(book.blob.clone()), type(book)(book.blob.clone())
+    few.blob[:4].view(torch.int32)[0] = 50
+    for b in (few, many):                                  # (some 80 to 105 windows of one code, from shape to shape)
+        b.blob[32:36].view(torch.int32)[0] = 0x4b560000 | 82
+    vc = ops.make_cache(*caches[1])
+    times, outs = [], []
+    for b in (few, many):
+        kc = ops.make_cache(enc, bi, ti, b, mi, sc, spec, size, largest)
+        each = []
+        for _ in range(12):
+            start, end = torch.cuda.Event(True), torch.cuda.Event(True)
+            start.record()
+            for _ in range(4):
+                out, st = ops.attn_decode(kc, vc, T, B, H, q, SCALING)
+            end.record()
+            end.synchronize()
+            each.append(start.elapsed_time(end))
+        assert ops.read_status(st) == 0
+        outs.append(out)
+        times.append(sorted(each)[len(each) // 2])
+    assert torch.equal(*outs)
+    assert times[1] <= 0.97 * times[0], times
