@@ -833,8 +833,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     const KvcWay wayK = kvc_book_way(p.k.book, p.brief != 0), wayV = kvc_book_way(p.v.book, p.brief != 0);
     const bool spare_in = p.spare && wayV.way == KVC_PAIRS;
     if (p.brief) {
-        kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
-        kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
+        kvc_load_luts(tab.lutK, tab.lutV, p.k.book, p.v.book, threadIdx.x, blockDim.x);
     } else kvc_load_ways(tab.lutK, tab.lutV, spare_in ? spare : nullptr, p.k.book, p.v.book, wayK.way == KVC_PAIRS, wayV.way == KVC_PAIRS, tab.len, threadIdx.x, blockDim.x);
     if (wayK.esc) kvc_load_tree(tab.tree[0], p.k.book, threadIdx.x, blockDim.x);
     if (wayV.esc) kvc_load_tree(tab.tree[1], p.v.book, threadIdx.x, blockDim.x);
@@ -1330,8 +1329,7 @@ __global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnPara
         sync();
         if (warp == 0 && any) { stage_K(true, it.col, it.t_lo); stage_V(true, it.col, it.t_lo); }
     }
-    kvc_load_lut(tab.lutK, p.k.book, threadIdx.x, blockDim.x);
-    kvc_load_lut(tab.lutV, p.v.book, threadIdx.x, blockDim.x);
+    kvc_load_luts(tab.lutK, tab.lutV, p.k.book, p.v.book, threadIdx.x, blockDim.x);
     const bool escK = book_has_long_codes(p.k.book), escV = book_has_long_codes(p.v.book);
     for (int i = tid; i < 2 * WROW; i += 128) sm.ps[i] = 0u;   // V records: the bytes that no token writes stay zero
 

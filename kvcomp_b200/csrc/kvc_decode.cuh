@@ -27,6 +27,25 @@ __device__ __forceinline__ void kvc_load_lut(uint32_t *lut, const void *book, in
         reinterpret_cast<uint4 *>(lut)[i] = make_uint4(form(e.x), form(e.y), form(e.z), form(e.w));
     }
 }
+// Two books' tables, up to four entries of 16 bytes of each on their way at once: a launch of few threads otherwise waits for one
+// after the other (two workers of 128 threads: eight trips to L2).  (Attention, a pass among others: 12 columns of 2816 tokens, 6 heads, 22.2 and 21.7 us; 256
+// columns of 4096, one head, 128.5 and 128.2.)
+__device__ __forceinline__ void kvc_load_luts(uint32_t *lut0, uint32_t *lut1, const void *book0, const void *book1, int tid, int nthr) {
+    const uint4 *src0 = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book0) + KVC_BOOK_OFF_LUT);
+    const uint4 *src1 = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book1) + KVC_BOOK_OFF_LUT);
+    constexpr int N = KVC_LUT_SIZE / 4, AHEAD = 4;
+    auto form = [](const uint4 &e) { return make_uint4(e.x + 16u - 2u * (e.x & 63u), e.y + 16u - 2u * (e.y & 63u), e.z + 16u - 2u * (e.z & 63u), e.w + 16u - 2u * (e.w & 63u)); };
+    for (int i = tid; i < N; i += AHEAD * nthr) {
+        uint4 a[AHEAD], b[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) if (i + j * nthr < N) { a[j] = __ldg(src0 + i + j * nthr); b[j] = __ldg(src1 + i + j * nthr); }
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) if (i + j * nthr < N) {
+            reinterpret_cast<uint4 *>(lut0)[i + j * nthr] = form(a[j]);
+            reinterpret_cast<uint4 *>(lut1)[i + j * nthr] = form(b[j]);
+        }
+    }
+}
 __device__ __forceinline__ void kvc_load_book(KvcBookSmem &b, const void *book, int tid, int nthr) {
     const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(book) + KVC_BOOK_OFF_TREE);
     for (int i = tid; i < 512 / 4; i += nthr) reinterpret_cast<uint4 *>(b.tree)[i] = src[i];
