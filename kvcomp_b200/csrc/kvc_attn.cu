@@ -778,11 +778,17 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     const uint32_t rows_s = kvc_smem_addr(sbase + workers * 2 * (p.slotK_bytes + p.slotV_bytes)) + (wk * 4 + warp) * 32 * (p.brief ? WHOLE_ROW_BYTES : ROW_BYTES);
     uint32_t *const spare = reinterpret_cast<uint32_t *>(sbase + workers * (2 * (p.slotK_bytes + p.slotV_bytes) + 128 * ROW_BYTES));      // (never with brief)
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
+    auto release = []() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); };
     // launched with programmatic stream serialisation: this kernel's own set-up -- the tables, the first blocks, the first step's metadata: cache
     // data that no kernel of a decode step writes -- runs before griddepcontrol.wait, possibly while the kernel ahead of it in the
     // stream (the merge of the layer before, which lets its dependents start early) still runs.  What that kernel or the one before it may
-    // write (the query, the scheduling counters, the workspace, the output, the status word) is touched after the wait.  (Letting this
-    // kernel's own dependents start early was measured: their waiting CTAs slow the launch by a tenth.)
+    // write (the query, the scheduling counters, the workspace, the output, the status word) is touched after the wait.  This kernel's own
+    // dependent, the merge kernel, is let go when a worker of every CTA has no further item, and never before the wait, as it reads the query and the tail's rows
+    // right away: it is set up, and has added up the tail, by the time that the last worker ends.  (It started 2.1 us after the last CTA's end and took 4 to 6 us for
+    // a tail.  Launch pair, device time, let go by the end of the CTAs and now: 12 columns of 2816 tokens and 165 rows, 6 heads, 22.3 and 17.1 us; 16 of 896 and 150, 4
+    // heads, 19.6 and 14.2; 32 of 1024, one head, no tail, 15.3 and 13.6; 256 of 4096 and 128 rows, one head, 128.8 and 123.2; 128 columns of 4096 and 128, 4 heads, 99.3 and
+    // 94.9; 16 of 16384, 49.1 and 45.9; 8 of 16384 30.9 and 31.1, of 32768 47.5 and 47.8.  Let go by a worker's end 126.2 where 123.2 stand, 18.7 where let go by its last item gives 17.1; at
+    // the kernel's top, whatever the items, 49.2 us where 47.8 stand.)
     const int B = (int)p.B, Hkv = (int)p.Hkv, Hq = (int)p.Hq;
     const int cols = B * Hkv, Gt = Hq / Hkv;
     const kvc_qmeta_dev &km = p.k.q, &vm = p.v.q;
@@ -884,6 +890,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
     bool v_staged = any, v_landed = true;                  // V blocks of the step to come are on their way already; the last wait for them ended well
     while (have) {
     const int col = it.col, b = col / Hkv, h = col % Hkv;
+    if (!more && !have_next) release();
     if (more && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
 #pragma unroll
     for (int g = 0; g < G; g++) sm.q[g * 128 + tid] = kvc_scale_value(qn[g]) * p.scaling;
@@ -979,7 +986,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         {
             bool n_on = true; int nb = b, nh = h, n_col = col, n_step = step + 1;      // the worker's next step (it may open the next column)
             if (n_step >= it.t_hi) {
-                if (more) have_next = item_of(P + sm.next_j, nit);
+                if (more) { have_next = item_of(P + sm.next_j, nit); if (!have_next) release(); }
                 n_on = have_next && nit.t_lo < nit.t_hi;
                 if (n_on) { n_col = nit.col; n_step = nit.t_lo; nb = n_col / Hkv; nh = n_col % Hkv; }
                 if (have_next) q_fetch(nit.col);
@@ -1205,6 +1212,7 @@ __global__ void __launch_bounds__(128 * rows_workers<G>(), 1) attn_rows_kernel(A
         if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
         if ((v_staged || !v_landed) && !kvc_mbar_wait(&sm.bar[1], par >> 1 & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
     }
+    release();
     if (flags) atomicOr(p.status, flags);
     if (draw && tid == 0) {               // the last worker to finish leaves the scheduling counters zeroed for the next launch
         __threadfence();
@@ -1286,6 +1294,7 @@ __global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnPara
     OneWorker &sm = reinterpret_cast<OneWorker *>(wbase)[wk];
     uint8_t *const slotsK = sbase + wk * 2 * (p.slotK_bytes + p.slotV_bytes), *const slotsV = slotsK + 2 * p.slotK_bytes;
     auto sync = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wk + 1) : "memory"); };     // the worker's threads
+    auto release = []() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); };
     // launched with programmatic stream serialisation, as the grouped kernel: set-up before griddepcontrol.wait reads cache data only
     const int B = (int)p.B, Hkv = (int)p.Hkv, cols = B * Hkv;
     const kvc_qmeta_dev &km = p.k.q, &vm = p.v.q;
@@ -1363,6 +1372,7 @@ __global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnPara
     uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
     while (have) {
     const int col = it.col, b = col / Hkv, h = col % Hkv;
+    if (!have_next) release();
     if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
     sm.q[tid] = qn;
     sync();
@@ -1552,6 +1562,7 @@ __global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnPara
         if (!kvc_mbar_wait(&sm.bar[0], par & 1u, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
         if (!kvc_mbar_wait(&sm.bar[1], par >> 1, p.wait_limit)) flags |= KVC_FLAG_WAIT_TIMEOUT;
     }
+    release();
     if (flags) atomicOr(p.status, flags);
     if (draw && tid == 0) {               // the last worker to finish leaves the scheduling counters zeroed for the next launch
         __threadfence();
@@ -2001,7 +2012,8 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         p.spare = GG > 1 && !p.brief && attn_smem<GG>(p, workers) + 4 * KVC_LUT_SIZE <= MAX_CTA_SHARED;         \
         const size_t smem = attn_smem<GG>(p, workers);                                                          \
         p.workers = workers;                                                                                    \
-        const int threads = 128 * (GG == 1 ? workers : rows_workers<GG>());                                     \
+        /* (threads that only help to load the tables would take the merge kernel's place beside a brief launch) */ \
+        const int threads = 128 * (GG == 1 || p.brief ? workers : rows_workers<GG>());                           \
         static kvc_launch_slot slots[4];                                                                        \
         auto *kernel = p.team ? (bulk ? attn_kernel<GG, true, true>() : attn_kernel<GG, false, true>())         \
                               : (bulk ? attn_kernel<GG, true, false>() : attn_kernel<GG, false, false>());      \
