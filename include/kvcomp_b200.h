@@ -220,6 +220,42 @@ int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_k,
                unsigned long long *total_bytes, void *workspace, int64_t workspace_bytes,
                int32_t *status, kvc_stream_t stream);
 
+/* A whole store of one tensor (models/cache/kvcomp_encode.py:60-207) in one call without a wait: the first T tokens are quantised
+ * (heads != 0: kvc_quantize_heads from x [B, H, x_tokens, 128], else kvc_quantize from rows [T, B, H, D]), with build != 0 the book is
+ * built from their codes, the first enc_T tokens of enc_codes are encoded (they may start before `codes`: codes that waited for their block),
+ * and scratch's first four words -- bytes of the stream, its largest block, the quantiser's and the encoder's status -- are copied to
+ * `report` (pinned host memory), which holds them once the stream has come that far.  rest_rows > 0 (heads only): the tokens behind the first T as rows
+ * (kvc_rope_store_rows); kept_rows > 0: the last of the T tokens dequantised (kvc_dequant).  The encoder's total starts at 0 with every call.
+ * T = 0: codes that the caller has are encoded, nothing else. */
+typedef struct {
+    const void *x, *cos_, *sin_;
+    int64_t cos_batch_stride, B, H, x_tokens, T, D, block;
+    uint8_t *codes;
+    void *min_int, *scale;
+    void *scratch;                /* kvc_store_scratch() bytes, 16-byte aligned */
+    int64_t scratch_bytes;
+    void *book;
+    const uint8_t *enc_codes;
+    int64_t enc_T, base_offset;
+    void *block_info;
+    uint16_t *thread_info;
+    uint8_t *encoded;
+    int64_t encoded_capacity;
+    void *rest;
+    int64_t rest_rows;
+    void *kept;
+    int64_t kept_rows;
+    int64_t *report;
+    const void *enc_table;        /* the encoder's table of n_entries, or null: the book's */
+    int32_t mode, batch_shared, heads, is_k, build, min_bytes;
+    float rel;
+    int32_t n_entries;
+} kvc_store_args;
+int64_t kvc_store_scratch(int mode, int batch_shared, int64_t T, int64_t B, int64_t H, int64_t block, int64_t enc_T, int is_k);
+int kvc_store_packed(const kvc_store_args *args, kvc_stream_t stream);
+/* Returns when the stream has finished what was launched on it so far. */
+int kvc_stream_wait(kvc_stream_t stream);
+
 /* Diagnostics, no counterpart in the reference.  The encoder's CTAs learn their block's byte offset from
  * the blocks before them and wait for each at most `wait_limit` polls (0 = the default of 2^21); a wait
  * that runs out raises KVC_FLAG_WAIT_TIMEOUT, the block and every later one write nothing, and the call

@@ -48,6 +48,7 @@ class Cache(C.Structure):
 CACHE_FIELDS = "7q2i4q2i"
 KV_STORE_ARGS = struct.Struct("<11q")
 ATTN_ARGS = struct.Struct("<" + 2 * CACHE_FIELDS + "12qfi")
+STORE_ARGS = struct.Struct("<29q6ifi")
 
 
 class KvcError(RuntimeError):
@@ -80,6 +81,9 @@ _SIGNATURES = {
     "kvc_build_codebook": (_i32, [_vp, _vp, _vp]),
     "kvc_book_from_tree": (_i32, [_vp, _i64, _vp, _vp]),
     "kvc_encode_workspace": (_i64, [_i64, _i64, _i32]),
+    "kvc_store_scratch": (_i64, [_i32, _i32, _i64, _i64, _i64, _i64, _i64, _i32]),
+    "kvc_store_packed": (_i32, [C.c_char_p, _vp]),
+    "kvc_stream_wait": (_i32, [_vp]),
     "kvc_encode_debug": (None, [_i32, _i32]),
     "kvc_encode": (_i32, [_vp, _i64, _i64, _i32, _vp, _i32, _u32, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _vp]),
     "kvc_decode": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _i64, _i32, _vp, _vp, _vp]),

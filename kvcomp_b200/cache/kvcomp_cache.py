@@ -52,6 +52,7 @@ class KVCompCache(_BASE):
         self.sins = [None] * layer_num
         self._ws = {}
         self._status = {}
+        self._last = None
 
     # ---- appending --------------------------------------------------------------------------------
     def _ctx(self, layer_idx, kv_heads):
@@ -68,7 +69,7 @@ class KVCompCache(_BASE):
         """Add new tokens (key/value_states: [B, Hkv, t, D]); keys get RoPE here unless pre-RoPE is on."""
         cfg = KVCompCacheConfigStatic.config
         cos, sin = cache_kwargs["cos"], cache_kwargs["sin"]
-        k_stored = False
+        k_stored, begun = False, None
         if cfg.enable_pre_rope:
             self.coss[layer_idx] = safe_cat(self.coss[layer_idx], cos, dim=1)
             self.sins[layer_idx] = safe_cat(self.sins[layer_idx], sin, dim=1)
@@ -94,7 +95,7 @@ class KVCompCache(_BASE):
                 ops.rope_store(key_states, cos, sin, out=place)
                 kc0.recent_commit(key_states.shape[2])
             else:
-                kc0.store_heads(key_states, cos, sin)           # rotated with torch's bits
+                begun = kc0.begin_heads(key_states, cos, sin)   # rotated with torch's bits
             k_stored = True
         else:
             key_states = apply_rotary_pos_emb_single(key_states, cos, sin)
@@ -105,8 +106,10 @@ class KVCompCache(_BASE):
         kc, vc = self._ctx(layer_idx, key_states.shape[1])
         if not k_stored:
             kc.store(key_states.permute(2, 0, 1, 3).contiguous().half())
+        if begun is not None and self._values_begun(kc, vc, begun, value_states):
+            return
         t = value_states.shape[2]
-        plain = value_states.is_cuda and value_states.dtype == torch.float16 and value_states.is_contiguous() and value_states.shape[3] % 16 == 0
+        plain = self._plain(value_states)
         place = vc.recent_place(t, value_states.device) if plain else None
         if place is not None:                                   # the transposition alone, straight into the window
             ops.rope_store(value_states, None, None, out=place)
@@ -115,6 +118,29 @@ class KVCompCache(_BASE):
             vc.store_heads(value_states)
         else:
             vc.store(value_states.permute(2, 0, 1, 3).contiguous().half())
+
+    @staticmethod
+    def _plain(x):
+        return x.is_cuda and x.dtype == torch.float16 and x.is_contiguous() and x.shape[3] % 16 == 0
+
+    @staticmethod
+    def _values_begun(kc, vc, begun, values):
+        """Finish the store of keys that has begun; True if the values' store went with it, behind one wait for both."""
+        both, v_begun = False, None
+        try:
+            if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and vc.recent_place(values.shape[2], values.device) is None:
+                v_begun = vc.begin_heads(values)
+                both = True
+        finally:
+            try:
+                kc._finish(begun)                               # (waits for both)
+            except BaseException:
+                if both:                                        # as if the values had not come yet
+                    vc._abandon(v_begun, values.shape[2])
+                raise
+        if both:
+            vc._finish(v_begun, waited=True)
+        return both
 
     def update(self, key_states, value_states, layer_idx, cache_kwargs=None):
         """The reference's Cache.update: append, then return the whole K and V as [B, Hkv, T, D]."""
@@ -190,6 +216,9 @@ class KVCompCache(_BASE):
     def _scratch(self, q, T, kv_heads):
         """Workspace and status word of a launch for q [B, Hq, ...] over T tokens of the streams."""
         B, Hq, device = q.shape[0], q.shape[1], q.device
+        last = self._last                                   # (T stays for 64 steps and more)
+        if last is not None and last[0] == (device, B, Hq, kv_heads, T):
+            return last[1], last[2]
         parts = ops.attn_splits(T, B, kv_heads)             # partial results per head of the balanced split
         ws = self._ws.get((device, B, Hq, parts))
         if ws is None:
@@ -197,6 +226,7 @@ class KVCompCache(_BASE):
         st = self._status.get(device)
         if st is None:
             st = self._status[device] = ops.new_status(device)
+        self._last = (device, B, Hq, kv_heads, T), ws, st
         return ws, st
 
     def _attend_step(self, q, kc, vc, scaling):

@@ -23,23 +23,52 @@ _MODE = {QuantMode.BlockQuant: ops.MODE_BLOCK, QuantMode.ChannelQuant: ops.MODE_
 
 
 class _Arena:
-    """A 1-D device buffer that grows geometrically; `n` elements are in use."""
+    """A 1-D device buffer that grows geometrically; `n` elements are in use.  Its memory is a tensor of its own or a part of one that several
+    arenas share (a context's first store makes one allocation for four of them)."""
 
     def __init__(self, dtype):
-        self.dtype, self.buf, self.n = dtype, None, 0
+        self.dtype, self.size, self.n = dtype, dtype.itemsize, 0
+        self._mem, self._off, self._cap, self._buf = None, 0, 0, None
 
-    def reserve(self, extra, device):
-        need = self.n + extra
-        if self.buf is None or self.buf.numel() < need:
-            cap = max(need, int((self.buf.numel() if self.buf is not None else 0) * 1.5), 1024)
-            new = torch.empty(cap, dtype=self.dtype, device=device)
-            if self.buf is not None and self.n:
+    @property
+    def buf(self):
+        if self._buf is None and self._mem is not None:
+            self._buf = self._mem[self._off:self._off + self._cap * self.size].view(self.dtype)
+        return self._buf
+
+    @buf.setter
+    def buf(self, t):
+        self._mem, self._off, self._cap, self._buf = t, 0, 0 if t is None else t.numel(), t
+
+    @property
+    def at(self):
+        """Address of the first element."""
+        return self._mem.data_ptr() + self._off
+
+    def need(self, extra):
+        """Elements to allocate for `extra` more."""
+        return max(self.n + extra, int(self._cap * 1.5), 1024)
+
+    def share(self, mem, off, cap):
+        """Lie in bytes off .. of `mem`, which nothing else uses."""
+        self._mem, self._off, self._cap, self._buf = mem, off, cap, None
+
+    def address(self, extra, device):
+        """Where the next `extra` elements go."""
+        if self._mem is None or self._cap < self.n + extra:
+            new = torch.empty(self.need(extra), dtype=self.dtype, device=device)
+            if self.n:
                 new[:self.n] = self.buf[:self.n]
             self.buf = new
-        return self.buf[self.n:need]
+        return self.at + self.n * self.size
+
+    def reserve(self, extra, device):
+        """The next `extra` elements."""
+        self.address(extra, device)
+        return self.buf[self.n:self.n + extra]
 
     def used(self):
-        return self.buf[:self.n] if self.buf is not None else None
+        return self.buf[:self.n] if self._mem is not None else None
 
 
 class _RecentRows:
@@ -296,11 +325,6 @@ class KVCompCtx:
             self.device = cache.device
         assert self.device == cache.device, "device mismatch"
 
-    def _units(self, T):
-        """Places for the unit parameters of T more tokens: (min_ints, scales, how many)."""
-        n = self.spec.units(T, self.batch_size, self.head_num, self.head_dim)
-        return self._mi.reserve(n, self.device), self._sc.reserve(n, self.device), n
-
     def _cut(self, live, t):
         """How many of the first tokens of (recent window + t new tokens) are compressed."""
         # utils/compute.py:59-72.  With recent_size = 0 and a ragged length the reference's slice clips to the length and
@@ -308,36 +332,37 @@ class KVCompCtx:
         return min(cut_len(live + t, self.cut_block, self.recent_size), live + t) // self.cut_block * self.cut_block
 
     def store_heads(self, x, cos=None, sin=None):
-        """store() of new tokens as a model's projections leave them, [B, H, t, D], rotated with cos / sin where they are
-        given.  A prompt into an empty window is quantised from where it lies."""
+        """store() of new tokens as a model's projections leave them, [B, H, t, D], rotated with cos / sin where they
+        are given.  A prompt into an empty window is quantised from where it lies."""
+        return self._finish(self.begin_heads(x, cos, sin))
+
+    def begin_heads(self, x, cos=None, sin=None):
+        """store_heads() up to its wait: what finish() takes."""
         B, H, t, D = x.shape
         live, mode = len(self._recent), _MODE[self.quant_mode]
         n = self._cut(live, t)
         if live or n == 0 or x.data_ptr() % 16 or not ops.quantize_heads_fits(mode, self.batch_shared, n, B, H, D, self.block_size) \
                 or (cos is not None and mode != ops.MODE_CHANNEL):
-            return self.store(ops.rope_store(x, cos, sin))
-        cos, sin, _ = ops._rotation(x, cos, sin)
+            return self._begin(ops.rope_store(x, cos, sin))
+        cos, sin, stride = ops._rotation(ops._cuda(x, torch.float16, "x"), cos, sin)
         if cos is not None and (cos.data_ptr() | sin.data_ptr()) % 16:
-            return self.store(ops.rope_store(x, cos, sin))
+            return self._begin(ops.rope_store(x, cos, sin))
         self._check(x.permute(2, 0, 1, 3))
         self.ctx_len += t
-
-        def quantize(report):
-            mi, sc, units = self._units(n)
-            return ops.quantize_heads(x, n, cos, sin, mode, self.block_size, self.quant_scale_rel, self.batch_shared, mi, sc,
-                                      report.hist, report.quant_status), units
-        return self._compress(quantize, n, 0, t - n, lambda place: ops.rope_store(x, cos, sin, out=place, first=n))
+        return self._launch(x, n, 0, t - n, t, None, cos, sin, stride)
 
     def store(self, cache):
         """Append tokens [t, B, H, D]; whole blocks beyond the recent window are quantised and encoded.
         Returns the uint8 codes of the newly compressed tokens as [n_blocks, block, B, H, D] (or None)."""
+        return self._finish(self._begin(cache))
+
+    def _begin(self, cache):
         self._check(cache)
         self.ctx_len += cache.shape[0]
         live, t = len(self._recent), cache.shape[0]
         n = self._cut(live, t)
-        room = self._room()
         if n == 0:
-            self._recent.append(cache, room)                  # the usual decode step: the new rows, nothing else moves
+            self._recent.append(cache, self._room())          # the usual decode step: the new rows, nothing else moves
             return None
         if live == 0:
             x, rest = cache[:n].contiguous(), cache[n:]       # a prefill: compressed from where it lies
@@ -345,41 +370,83 @@ class KVCompCtx:
             x, rest = self._recent.view()[:n].clone(), cache  # the window's front
         else:
             x, rest = torch.cat([self._recent.view(), cache[:n - live]], dim=0), cache[n - live:]
+        return self._launch(x, n, live, rest.shape[0], 0, lambda place: place.copy_(rest))
 
-        def quantize(report):
-            mi, sc, units = self._units(n)
-            return ops.quantize(x, _MODE[self.quant_mode], self.block_size, self.quant_scale_rel, self.batch_shared,
-                                min_dtype=self.min_dtype, hist=report.hist, min_int=mi, scale=sc, status=report.quant_status)[0], units
-        return self._compress(quantize, n, live, rest.shape[0], lambda place: place.copy_(rest))
-
-    def _compress(self, quantize, n, live, n_rest, put_rest):
-        """quantize(report) launches the quantiser for the first n tokens of (the `live` rows of the window + new tokens) and
-        returns their codes and how many units they have; put_rest(place) writes the n_rest last of the new tokens as rows."""
-        room, T = self._room(), n
-        # quantise, book and encode are launched one behind the other; one copy brings back what all of them report
-        # (a wait and a copy for each of them: a 333-token prompt 637 us, now 466)
-        report = ops.Report(self.device, with_hist=self.book is None)
-        codes, n_units = quantize(report)
-        if self.book is None:
-            self.book = ops.build_codebook(report.hist)
-        pend = codes if self._pending is None else torch.cat([self._pending, codes], dim=0)
-        n_enc = pend.shape[0] // self.enc_block * self.enc_block
-        part = pend[:n_enc].contiguous() if n_enc else None
+    def _launch(self, x, n, live, n_rest, x_tokens, put_rest, cos=None, sin=None, stride=0):
+        """Launch the compression of the first n tokens of (the `live` rows of the window + new tokens): x as rows, or (x_tokens > 0) as a
+        prompt's heads.  put_rest(place) writes the n_rest last of the new tokens as rows; the heads' own are written by the call."""
+        # quantise, book, encode and the rows are launched by one call; one copy brings back what the kernels report
+        # (a prompt of 333 tokens, K and V: a call, a wait and a copy for each kernel 637 us, one report per tensor 409;
+        # one call per tensor and one wait for both 261)
+        shape, T, dev = (self.batch_size, self.head_num, self.head_dim), n, self.device
+        B, H, D = shape
+        mode, build = _MODE[self.quant_mode], self.book is None
+        if build:
+            self.book = ops.new_book(dev)
+        old = 0 if self._pending is None else self._pending.shape[0]
+        pend = torch.empty((old + n,) + shape, dtype=torch.uint8, device=dev)
+        if old:
+            pend[:old] = self._pending
+        n_enc = (old + n) // self.enc_block * self.enc_block
+        part = pend if n_enc == old + n else pend[:n_enc]
         stream_room, cap = self._encode_room(part) if n_enc else (0, 0)
-        if n_enc:
-            self._encode_launch(part, stream_room, report)
+        blocks = n_enc * B * H * D // 8192
+        n_units = self.spec.units(n, B, H, D)
+        scratch = torch.empty(ops._lib.load().kvc_store_scratch(mode, self.batch_shared, n, B, H, self.block_size, n_enc, self.is_k), dtype=torch.uint8, device=dev)
         # Where the window starts over, the rest of the new tokens is written before the wait: a caller's tensors are then read
         # when the store returns, whichever stream they belong to.
-        over, k, n_old, buf = live == 0 or n > live, 0, 0, None
+        over, k, n_old, buf, at_kept, at_rest = live == 0 or n > live, 0, 0, None, 0, 0
         if over:
             if self.keep_dequantised:
                 k = min(n, max(self.KEEP_ROWS // self.cut_block, 1) * self.cut_block)    # a long prefill keeps its last rows only
                 n_old = self._recent.kept if k == n else 0
             if n_old + k + n_rest:
-                buf = torch.empty((n_old + k + n_rest + room,) + tuple(codes.shape[1:]), dtype=torch.float16, device=self.device)
-            if n_rest:
+                buf = torch.empty((n_old + k + n_rest + self._room(),) + shape, dtype=torch.float16, device=dev)
+                at_kept = buf.data_ptr() + n_old * (2 * B * H * D)
+                at_rest = at_kept + k * (2 * B * H * D)
+        if not x_tokens:
+            ops._cuda(x, torch.float16, "x")
+            if mode in (ops.MODE_BLOCK, ops.MODE_CHANNEL) and n % self.block_size:
+                raise KvcError("T=%d is not a multiple of block=%d" % (n, self.block_size))
+        if self._bi._mem is None and self._ti._mem is None and self._mi._mem is None and self._sc._mem is None:
+            parts, size = ((self._bi, blocks * 8), (self._ti, blocks * 64), (self._mi, n_units), (self._sc, n_units)), 0
+            for a, m in parts:
+                size += (a.need(m) * a.size + 255) // 256 * 256
+            mem, at = torch.empty(size, dtype=torch.uint8, device=dev), 0
+            for a, m in parts:
+                cap = a.need(m)
+                a.share(mem, at, cap)
+                at += (cap * a.size + 255) // 256 * 256
+        slot, report = ops.Reports.place()
+        try:
+            ops.store_at(dev, (x.data_ptr(), 0 if cos is None else cos.data_ptr(), 0 if sin is None else sin.data_ptr(), stride, B, H, x_tokens, n, D, self.block_size,
+                               pend.data_ptr() + old * (B * H * D), self._mi.address(n_units, dev), self._sc.address(n_units, dev), scratch.data_ptr(), scratch.numel(),
+                               self.book.blob.data_ptr(), pend.data_ptr(), n_enc, self._enc.n, self._bi.address(blocks * 8, dev), self._ti.address(blocks * 64, dev),
+                               self._enc.address(stream_room, dev), stream_room, at_rest, n_rest if x_tokens and over else 0, at_kept, k, report, 0),
+                         (mode, self.batch_shared, x_tokens > 0, self.is_k, build, self._mi.size), self.quant_scale_rel)
+            if over and n_rest and not x_tokens:
                 put_rest(buf[n_old + k:n_old + k + n_rest])
-        words = report.read()                                 # synchronises, as the reference does
+        except BaseException:                                 # nothing that is on its way may arrive in the place later
+            if build:
+                self.book = None
+            ops.wait(dev)
+            raise
+        return slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest, build, x, cos, sin, scratch
+
+    def _abandon(self, begun, t):
+        """A begun store of t tokens, waited for, is not to count."""
+        self.ctx_len -= t
+        if begun is not None and begun[15]:
+            self.book = None
+
+    def _finish(self, begun, waited=False):
+        """The rest of a begun store: waits for it (waited: the caller has), then it counts."""
+        if begun is None:
+            return None
+        slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest = begun[:15]
+        if not waited:
+            ops.wait(self.device)
+        words, room, n, codes = ops.Reports.read(slot), self._room(), T, pend[old:] if old else pend
         flags = ops.check_flags(words[2], what="quantize")
         if flags & ops._lib.FLAG_MIN_OVERFLOW:
             # int8 is the reference's CUDA path, which wraps silently (kvcomp_encode.py:97); its model path
@@ -390,10 +457,10 @@ class KVCompCtx:
             warnings.warn("a min_int wrapped in int8 as in the reference's CUDA path; set wide_min_ints to keep it")
         # the window: the compressed rows leave it, or stay as dequantised rows for a reader of the rows behind
         # the fused kernel's range (tail_from); the rest of the new tokens joins the recent rows
-        mi = self._mi.buf[self._mi.n:self._mi.n + n_units]
-        sc = self._sc.buf[self._sc.n:self._sc.n + n_units]
         if not over:
             if self.keep_dequantised:
+                mi = self._mi.buf[self._mi.n:self._mi.n + n_units]
+                sc = self._sc.buf[self._sc.n:self._sc.n + n_units]
                 ops.dequant(codes, mi, sc, self.spec, out=self._recent.view()[:n])     # in place of the rows themselves
                 self._recent.consume(n)
             else:
@@ -404,9 +471,6 @@ class KVCompCtx:
                 self._recent.commit(n_rest)
         else:
             self._recent.restart(n_old, k, n_rest, buf)
-            if k:                                             # dequantised where they stay
-                first = (n - k) // self.spec.tok_div * self.spec.sj                      # unit of the first kept token
-                ops.dequant(codes[n - k:], mi[first:], sc[first:], self.spec, out=buf[n_old:n_old + k])
         self._mi.n += n_units
         self._sc.n += n_units
         self.compressed_ctx_len += T
@@ -427,7 +491,7 @@ class KVCompCtx:
         # needs a fraction of that, so room is reserved from the density seen so far (8 bits per symbol at
         # first) with a quarter on top, and the store is repeated with the full reserve in the rare case
         # that the encoder reports the room as exceeded.
-        cap = ops.buffer_sizes(codes.shape[0], self.batch_size * self.head_num * self.head_dim, self.is_k)[3]
+        cap = codes.numel()
         seen = self.encoded_ctx_len * self.batch_size * self.head_num * self.head_dim
         return (cap if seen == 0 else min(cap, int(1.25 * self._enc.n / seen * codes.numel()) + 4096)), cap
 
@@ -448,10 +512,10 @@ class KVCompCtx:
         if words[3] & ops._lib.FLAG_SYMBOL_MISSING:
             return False
         ops.check_flags(words[3], what="entropy_encode")
-        bsz, tsz, _, _ = ops.buffer_sizes(codes.shape[0], self.batch_size * self.head_num * self.head_dim, self.is_k)
+        blocks = codes.numel() // 8192
         self._enc.n += words[0]
-        self._bi.n += bsz
-        self._ti.n += tsz // 2
+        self._bi.n += blocks * 8
+        self._ti.n += blocks * 64
         self.max_block_bytes = max(self.max_block_bytes, words[1])
         return True
 
@@ -567,17 +631,16 @@ class KVCompCtx:
                                                  self._sc.buf, self.spec, self._enc.n, self.max_block_bytes)
             self._cache_q = c.q
             return c
-        c.encoded, c.encoded_bytes, c.max_block_bytes = self._enc.buf.data_ptr(), self._enc.n, self.max_block_bytes
-        c.block_info, c.thread_info, c.book = self._bi.buf.data_ptr(), self._ti.buf.data_ptr(), self.book.blob.data_ptr()
-        self._cache_q.min_int, self._cache_q.scale = self._mi.buf.data_ptr(), self._sc.buf.data_ptr()
+        c.encoded, c.encoded_bytes, c.max_block_bytes = self._enc.at, self._enc.n, self.max_block_bytes
+        c.block_info, c.thread_info, c.book = self._bi.at, self._ti.at, self.book.blob.data_ptr()
+        self._cache_q.min_int, self._cache_q.scale = self._mi.at, self._sc.at
         return c
 
     def _fields(self):
         """cache()'s contents in the order of the structure, for a launch made right away."""
         assert self.encoded_ctx_len > 0 and self.book is not None, "nothing has been encoded yet"
-        s, e, mi = self.spec, self._enc, self._mi.buf
-        return (e.buf.data_ptr(), e.n, self._bi.buf.data_ptr(), self._ti.buf.data_ptr(), self.book.blob.data_ptr(), mi.data_ptr(),
-                self._sc.buf.data_ptr(), mi.element_size(), s.tok_div, s.sj, s.sb, s.sh, s.sc, self.max_block_bytes, 0)
+        s, e = self.spec, self._enc
+        return (e.at, e.n, self._bi.at, self._ti.at, self.book.blob.data_ptr(), self._mi.at, self._sc.at, self._mi.size, s.tok_div, s.sj, s.sb, s.sh, s.sc, self.max_block_bytes, 0)
 
     def mat_vec_mul(self, B):
         """K: scores [batch, heads, ctx] = q . K^T; V: [1, batch, heads, 128] = P . V over the compressed

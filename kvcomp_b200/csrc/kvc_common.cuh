@@ -41,6 +41,10 @@ void kvc_set_error(const char *fmt, ...);
 static inline cudaStream_t kvc_cu(kvc_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
 int kvc_sm_count();
+// kvc_encode into a workspace and a total that the caller has zeroed
+int kvc_encode_zeroed(const uint8_t *codes, int64_t T, int64_t cols, int is_k, const void *enc_table, int n_entries, uint32_t base_offset, void *block_info,
+                      uint16_t *thread_info, uint8_t *encoded, int64_t encoded_capacity, unsigned long long *total_bytes, void *workspace,
+                      int64_t workspace_bytes, int32_t *status, kvc_stream_t stream);
 
 constexpr int KVC_MAX_DEVICES = 64;
 // Number of the calling thread's current context, 0 .. KVC_MAX_CONTEXTS - 1, or -1: nothing is kept for it.  A kernel's

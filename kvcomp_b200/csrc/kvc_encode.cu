@@ -345,11 +345,8 @@ extern "C" int64_t kvc_encode_workspace(int64_t T, int64_t cols, int is_k) {
     return 16 + nblk * 8;                                  // the block counter, then a state word per block
 }
 
-extern "C" int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_k,
-                          const void *enc_table, int n_entries, uint32_t base_offset,
-                          void *block_info, uint16_t *thread_info, uint8_t *encoded, int64_t encoded_capacity,
-                          unsigned long long *total_bytes, void *workspace, int64_t workspace_bytes,
-                          int32_t *status, kvc_stream_t stream) {
+static int encode_check(const uint8_t *codes, int64_t T, int64_t cols, int is_k, const void *enc_table, int n_entries, void *block_info,
+                        uint16_t *thread_info, uint8_t *encoded, void *workspace, int64_t workspace_bytes, int32_t *status) {
     KVC_REQUIRE(codes && enc_table && block_info && thread_info && encoded && status, "kvc_encode: null pointer");
     KVC_REQUIRE(cols > 0 && T >= 0, "kvc_encode: bad shape");
     KVC_REQUIRE(n_entries >= 1 && n_entries <= 256, "kvc_encode: the encode table has 1..256 entries");
@@ -357,21 +354,39 @@ extern "C" int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_
                 is_k ? "K" : "V", is_k ? 64 : 128, (long long)T);
     KVC_REQUIRE((reinterpret_cast<uintptr_t>(codes) & 3) == 0 && (reinterpret_cast<uintptr_t>(block_info) & 7) == 0,
                 "kvc_encode: codes must be 4-byte and block_info 8-byte aligned");
-    cudaStream_t s = kvc_cu(stream);
     const long long nblk = is_k ? (T / 64) * cols : (T / 128) * cols * 2;
-    if (total_bytes) KVC_CUDA_OK(cudaMemsetAsync(total_bytes, 0, 8, s));
     if (nblk == 0) return KVC_OK;
     KVC_REQUIRE(nblk < (1ll << 31), "kvc_encode: too many blocks in one call");
     KVC_REQUIRE(workspace && workspace_bytes >= kvc_encode_workspace(T, cols, is_k),
                 "kvc_encode: workspace needs %lld bytes", (long long)kvc_encode_workspace(T, cols, is_k));
     KVC_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0, "kvc_encode: workspace must be 16-byte aligned");
-    const uint32_t *enc = reinterpret_cast<const uint32_t *>(enc_table);
-    KVC_CUDA_OK(cudaMemsetAsync(workspace, 0, 16 + nblk * 8, s));
-    encode_onepass_kernel<<<(unsigned)nblk, ENC_THREADS, 0, s>>>(
-        codes, cols, is_k, nblk, enc, n_entries, thread_info, reinterpret_cast<uint2 *>(block_info), base_offset, encoded,
+    return KVC_OK;
+}
+
+int kvc_encode_zeroed(const uint8_t *codes, int64_t T, int64_t cols, int is_k, const void *enc_table, int n_entries, uint32_t base_offset, void *block_info,
+                      uint16_t *thread_info, uint8_t *encoded, int64_t encoded_capacity, unsigned long long *total_bytes, void *workspace,
+                      int64_t workspace_bytes, int32_t *status, kvc_stream_t stream) {
+    if (int rc = encode_check(codes, T, cols, is_k, enc_table, n_entries, block_info, thread_info, encoded, workspace, workspace_bytes, status)) return rc;
+    const long long nblk = is_k ? (T / 64) * cols : (T / 128) * cols * 2;
+    if (nblk == 0) return KVC_OK;
+    encode_onepass_kernel<<<(unsigned)nblk, ENC_THREADS, 0, kvc_cu(stream)>>>(
+        codes, cols, is_k, nblk, reinterpret_cast<const uint32_t *>(enc_table), n_entries, thread_info, reinterpret_cast<uint2 *>(block_info), base_offset, encoded,
         encoded_capacity, reinterpret_cast<unsigned int *>(workspace),
         reinterpret_cast<unsigned long long *>(reinterpret_cast<uint8_t *>(workspace) + 16), total_bytes, status,
         g_enc_wait_limit ? g_enc_wait_limit : ENC_WAIT_LIMIT, g_enc_starve);
     KVC_LAUNCH_OK();
     return KVC_OK;
+}
+
+extern "C" int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_k,
+                          const void *enc_table, int n_entries, uint32_t base_offset,
+                          void *block_info, uint16_t *thread_info, uint8_t *encoded, int64_t encoded_capacity,
+                          unsigned long long *total_bytes, void *workspace, int64_t workspace_bytes,
+                          int32_t *status, kvc_stream_t stream) {
+    if (int rc = encode_check(codes, T, cols, is_k, enc_table, n_entries, block_info, thread_info, encoded, workspace, workspace_bytes, status)) return rc;
+    if (total_bytes) KVC_CUDA_OK(cudaMemsetAsync(total_bytes, 0, 8, kvc_cu(stream)));
+    const int64_t bytes = kvc_encode_workspace(T, cols, is_k);
+    if (bytes > 16) KVC_CUDA_OK(cudaMemsetAsync(workspace, 0, (size_t)bytes, kvc_cu(stream)));
+    return kvc_encode_zeroed(codes, T, cols, is_k, enc_table, n_entries, base_offset, block_info, thread_info, encoded, encoded_capacity, total_bytes, workspace,
+                             workspace_bytes, status, stream);
 }

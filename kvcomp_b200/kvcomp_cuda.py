@@ -85,13 +85,14 @@ def _encode(is_k, input, encode_code_book, block_infos, thread_infos, idx_offset
     cols = input.shape[2] * input.shape[3]
     bsz, tsz, _, _ = ops.buffer_sizes(tokens, cols * 128, is_k)
     codes = input.contiguous().view(tokens, input.shape[2], input.shape[3], 128)
-    report = ops.Report(codes.device)
-    ops.encode(codes, is_k, encode_code_book, block_infos, thread_infos, encoded_data,
-               base_offset=int(base_global_offset), total=report.total, status=report.enc_status)
-    n, _, _, flags = report.read()                 # synchronises, like the reference's cudaDeviceSynchronize
+    n, _, _, flags = ops.encode_now(codes, is_k, encode_code_book, block_infos, thread_infos, encoded_data,
+                                    int(base_global_offset))       # waits, like the reference's cudaDeviceSynchronize
     ops.check_flags(flags, what="entropy_encode")
     if idx_offset is not None and idx_offset.numel() >= 8:     # the reference's cursor: {blocks, bytes}
-        idx_offset.view(torch.int32)[:2] = torch.tensor([bsz // 8, n], dtype=torch.int32, device=idx_offset.device)
+        if idx_offset.numel() == 8 and idx_offset.element_size() == 1 and idx_offset.data_ptr() % 8 == 0 and n < 1 << 31:
+            idx_offset.view(torch.int64).fill_(n << 32 | bsz // 8)         # (no copy of a host tensor)
+        else:
+            idx_offset.view(torch.int32)[:2] = torch.tensor([bsz // 8, n], dtype=torch.int32, device=idx_offset.device)
     return encoded_data[:n], block_infos.view(torch.uint8)[:bsz], thread_infos.view(torch.uint8)[:tsz]
 
 

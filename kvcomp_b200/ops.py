@@ -4,6 +4,7 @@ PyTorch is only the carrier of device memory and streams here; every computation
 libkvcomp_b200.so.  Every function raises when the tensors are not CUDA tensors: there is no CPU path.
 """
 import ctypes as C
+import functools
 import threading
 from dataclasses import dataclass
 
@@ -82,23 +83,23 @@ def check_flags(v, raise_on_fatal=True, what="kvcomp_b200"):
 
 
 class TimedCall:
-    """What a call that returns only after the device has finished, with its time and its status, needs: two events, a status
-    word and its place in pinned memory.  One per thread and device, kept; the status word is zero between calls.
+    """What a call that returns only after the device has finished, with its time and its status, needs: two events and a status
+    word.  One per thread and device, kept; the status word is zero between calls.  It lies in pinned memory, where the kernels write it (only
+    to report something) and the host reads it: no copy of it stands between the last kernel and the host.
     `with TimedCall.on(device) as call:` begins; the launches and end() belong in the block, so that a call which an exception
     ends is waited for and its flags go with it.
-    (Events, a zeroed word and a pageable read-back made anew cost such a call some 20 us.)"""
-    __slots__ = ("start", "stop", "status", "host", "flags", "raw", "stream", "open")
+    (Events, a zeroed word and a pageable read-back made anew cost such a call some 20 us, a copy of the word 8.)"""
+    __slots__ = ("start", "stop", "status", "flags", "raw", "stream", "device", "open")
     _kept = threading.local()
 
     def __init__(self, device):
         self.start, self.stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        with torch.inference_mode(False):                  # normal tensors, whatever mode the thread's first call runs in:
-            self.status = new_status(device)               # they are written again in calls of either mode
-            self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
-        self.flags = self.host.numpy()
+        self.device = device
+        with torch.inference_mode(False):                  # a normal tensor, whatever mode the thread's first call runs in:
+            self.status = torch.zeros(1, dtype=torch.int32).pin_memory()       # it is written again in calls of either mode
+        self.flags = self.status.numpy()
         self.raw = self.stream = None
         self.open = False                                  # launches may be under way that write the status word
-        self._current().synchronize()                      # the word is zero, whichever stream uses it first
 
     @staticmethod
     def on(device):
@@ -111,9 +112,9 @@ class TimedCall:
     def _current(self):
         """The device's current stream; the object is made anew only when the stream is another one."""
         if _current_stream is None:
-            self.stream = torch.cuda.current_stream(self.status.device)
+            self.stream = torch.cuda.current_stream(self.device)
             return self.stream
-        raw = _current_stream(self.status.device.index)
+        raw = _current_stream(self.device.index)
         if raw != self.raw:
             self.raw, self.stream = raw, torch.cuda.Stream(stream_id=raw[0], device_index=raw[1], device_type=raw[2])
         return self.stream
@@ -130,20 +131,17 @@ class TimedCall:
 
     def _clear(self):
         """Zero the word behind everything the call has launched."""
-        with torch.cuda.stream(self.stream):
-            self.status.zero_()
         self.stream.synchronize()
+        self.flags[0] = 0
         self.open = False
 
     def end(self, what):
         """Waits; the time since the call began in ms.  Raises on a fatal status."""
         stream = self._current()
         self.stop.record(stream)
-        self.host.copy_(self.status, non_blocking=True)
         stream.synchronize()
         v = int(self.flags[0])
-        if v:
-            self._clear()
+        self.flags[0] = 0
         self.open = False
         check_flags(v, what=what)
         return self.start.elapsed_time(self.stop)
@@ -166,7 +164,39 @@ class Report:
         return self.words.tolist()
 
 
-@dataclass
+class Reports:
+    """Where the reports of a thread's stores arrive: two in pinned memory (a cache's K and V are on their way together), kept per thread.  A
+    store takes a place, launches, and reads its words behind a wait."""
+    _kept = threading.local()
+
+    def __init__(self):
+        with torch.inference_mode(False):
+            self.words = torch.zeros(2, 4, dtype=torch.int64).pin_memory()
+        self.view, self.next = self.words.numpy(), 0
+
+    @staticmethod
+    def place():
+        """(index, address) of a place that no store of this thread is using: the stores of one wait are two at most."""
+        r = getattr(Reports._kept, "r", None)
+        if r is None:
+            r = Reports._kept.r = Reports()
+        i = r.next
+        r.next = 1 - i
+        return i, r.words.data_ptr() + 32 * i
+
+    @staticmethod
+    def read(i):
+        """(bytes, largest block, quantiser flags, encoder flags) of a store that has been waited for."""
+        return Reports._kept.r.view[i].tolist()
+
+
+def wait(device):
+    """Wait for the device's current stream."""
+    with _on(device):
+        _lib.check(_lib.load().kvc_stream_wait(_stream()), "wait")
+
+
+@dataclass(frozen=True)
 class QSpec:
     """Unit layout of a (min_int, scale) pair: unit = (t // tok_div)*sj + b*sb + h*sh + c*sc."""
     mode: int
@@ -187,6 +217,7 @@ class QSpec:
                      self.sj, self.sb, self.sh, self.sc)
 
 
+@functools.lru_cache(maxsize=256)
 def qspec(mode, batch_shared, B, H, D, block):
     lib = _lib.load()
     q = QMeta()
@@ -415,6 +446,17 @@ class Book:
         return self.host()[BOOK_OFF_REFTREE: BOOK_OFF_REFTREE + 3 * n].clone()
 
 
+def new_book(device):
+    """A book that a store builds."""
+    return Book(torch.empty(BOOK_BYTES, dtype=torch.uint8, device=device))
+
+
+def store_at(device, words, ints, rel, n_entries=0):
+    """kvc_store: its arguments' words and ints in the structure's order.  The caller has checked the tensors."""
+    with _on(device):
+        _lib.check(_lib.load().kvc_store_packed(_lib.STORE_ARGS.pack(*words, *ints, rel, n_entries), _stream()), "store")
+
+
 def build_codebook(hist):
     lib = _lib.load()
     _cuda(hist, torch.int64, "hist")
@@ -439,15 +481,25 @@ def encode(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset
     of this call, [1] the largest block byte count (a running maximum when `total` is passed in again).
     enc_table: device uint8 tensor of {u32 code, u32 length} entries indexed by symbol."""
     lib = _lib.load()
+    T, cols = _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded)
+    dev = codes.device
+    status = new_status(dev) if status is None else status
+    total = torch.zeros(2, dtype=torch.int64, device=dev) if total is None else total
+    ws = torch.empty(max(lib.kvc_encode_workspace(T, cols, int(is_k)), 16), dtype=torch.uint8, device=dev)
+    with _on(dev):
+        _lib.check(lib.kvc_encode(_p(codes), T, cols, int(is_k), _p(enc_table), enc_table.numel() // 8,
+                                  int(base_offset), _p(block_info), _p(thread_info), _p(encoded),
+                                  encoded.numel(), _p(total), _p(ws), ws.numel(), _p(status), _stream()), "kvc_encode")
+    return total, status
+
+
+def _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded):
+    """Raise unless the encoder can take these; returns (T, sequences x heads)."""
     _cuda(codes, torch.uint8, "codes")
     T, B, H, D = codes.shape
     if D != 128:
         raise KvcError("head_dim must be 128")
     cols = B * H
-    dev = codes.device
-    status = new_status(dev) if status is None else status
-    total = torch.zeros(2, dtype=torch.int64, device=dev) if total is None else total
-    ws = torch.empty(max(lib.kvc_encode_workspace(T, cols, int(is_k)), 16), dtype=torch.uint8, device=dev)
     _cuda(enc_table, torch.uint8, "encode_code_book")
     for t, n in ((block_info, "block_infos"), (thread_info, "thread_infos"), (encoded, "encoded_data")):
         _cuda(t, None, n)
@@ -455,11 +507,22 @@ def encode(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset
     if block_info.numel() * block_info.element_size() < nblk * 8 or \
             thread_info.numel() * thread_info.element_size() < nblk * 128:
         raise KvcError("block_infos / thread_infos too small for %d blocks" % nblk)
-    with _on(dev):
-        _lib.check(lib.kvc_encode(_p(codes), T, cols, int(is_k), _p(enc_table), enc_table.numel() // 8,
-                                  int(base_offset), _p(block_info), _p(thread_info), _p(encoded),
-                                  encoded.numel(), _p(total), _p(ws), ws.numel(), _p(status), _stream()), "kvc_encode")
-    return total, status
+    return T, cols
+
+
+def encode_now(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset):
+    """encode() and a wait; returns (bytes, largest block, 0, status)."""
+    T, cols = _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded)
+    dev = codes.device
+    scratch = torch.empty(_lib.load().kvc_store_scratch(0, 1, 0, 1, cols, 64, T, int(is_k)), dtype=torch.uint8, device=dev)
+    slot, report = Reports.place()
+    try:
+        store_at(dev, (0, 0, 0, 0, 1, cols, 0, 0, 128, 64, 0, 0, 0, scratch.data_ptr(), scratch.numel(), 0, codes.data_ptr(), T, int(base_offset),
+                       block_info.data_ptr(), thread_info.data_ptr(), encoded.data_ptr(), encoded.numel(), 0, 0, 0, 0, report, enc_table.data_ptr()),
+                 (0, 1, 0, int(is_k), 0, 1), 0.0, enc_table.numel() // 8)
+    finally:
+        wait(dev)
+    return Reports.read(slot)
 
 
 def decode(encoded, block_info, thread_info, book, T, B, H, is_k, out=None, status=None, max_block=0):
