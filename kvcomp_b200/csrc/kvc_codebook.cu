@@ -171,14 +171,57 @@ __device__ short heap_pop(Heap &hp, long long *f_out) {
     return top_id;
 }
 
-// The heap is a serial chain by contract (its layout decides ties), everything around it is spread over the CTA:
-// with one thread walking the trees and symbols too, a book of 20 to 30 symbols took 76 us; now 19 to 26 us, of which
-// the heap takes most.
+// The heap is a serial chain by contract (its layout decides ties), everything around it is spread over the CTA.  Where all counts together fit 32 bits, its
+// words are split into frequencies and ids, two children come with one load, and what a pop has just moved is still in registers when the last word is sifted up.
+// (A book of 22 and of 12 symbols: 24.8 and 16.5 us with 64-bit words and the decode table bit by bit, now 18.7 and 12.0; with one thread for the trees as well, 76 us.  Each
+// operation by a warp -- the choices of all inner nodes by one ballot, a lane per node -- took 390 cycles a pop.)
 constexpr int BOOK_THREADS = 1024;
 
+struct Heap32 {
+    uint2 *w;                                               // {frequency, id} of element i at i + 1: an element's children lie in one aligned 128-bit word
+    int n;
+    __device__ __forceinline__ void sift_up(int hole, uint2 x) {
+        while (hole > 0) {
+            const int parent = (hole - 1) >> 1;
+            const uint2 p = w[parent + 1];
+            if (!(p.x > x.x)) break;
+            w[hole + 1] = p;
+            hole = parent;
+        }
+        w[hole + 1] = x;
+    }
+    __device__ __forceinline__ void push(uint32_t freq, uint32_t id) { n++; sift_up(n - 1, make_uint2(freq, id)); }
+    __device__ __forceinline__ uint2 pop() {
+        const uint2 top = w[1];
+        const int len = --n;
+        if (len == 0) return top;
+        const uint2 last = w[len + 1];
+        int hole = 0;
+        uint2 moved = make_uint2(0u, 0u);                   // what lies in the hole's parent by now
+        while (2 * hole + 2 < len) {
+            const uint4 c = *reinterpret_cast<const uint4 *>(w + 2 * hole + 2);
+            const bool right = !(c.z > c.x);
+            moved = right ? make_uint2(c.z, c.w) : make_uint2(c.x, c.y);
+            w[hole + 1] = moved;
+            hole = 2 * hole + 1 + (right ? 1 : 0);
+        }
+        if (2 * hole + 2 == len) {
+            moved = w[2 * hole + 2];
+            w[hole + 1] = moved;
+            hole = 2 * hole + 1;
+        }
+        if (hole > 0 && moved.x > last.x) {
+            w[hole + 1] = moved;
+            sift_up((hole - 1) >> 1, last);
+        } else w[hole + 1] = last;
+        return top;
+    }
+};
+
 struct BookSmem {
-    long long hf[512];
-    short hid[512];
+    alignas(16) long long hf[512];
+    alignas(16) short hid[512];
+    uint16_t first[KVC_LUT_SIZE];    // per window: the symbol that it begins with, and above it the bits of its code (0: no complete code)
     short parent[512];           // of a leaf (its symbol) or an inner node of the Huffman tree: node << 1 | bit
     uint8_t listed[256];         // the symbols that have a code, ascending
     uint32_t aligned[256];       // per listed symbol: its code, first bit on top
@@ -189,6 +232,7 @@ struct BookSmem {
     uint32_t tree[512];          // wide tree: lo16 = child0 (or LEAF), hi16 = child1 (or symbol)
     long long count[256];        // the histogram, fetched by all threads at once
     int n_nodes, n_symbols, min_sym, max_sym, max_len, flags, lone;
+    int n_listed, by_walk;       // listed symbols; the trees were built serially: they may lack codes
 };
 
 // Exclusive prefix sum of x over the CTA's first 256 threads (the others pass 0); *total receives the sum.
@@ -263,6 +307,7 @@ __device__ void build_trees(BookSmem &s, int tid) {
     }
     const int fresh = mine ? len - m : 0;
     const uint32_t base = 2u + book_scan(s, (uint32_t)fresh, tid, &total);
+    if (tid == 0) { s.n_listed = (int)n; s.by_walk = s.max_len > 32 || total + 2u > 512u; }
     if (s.max_len > 32 || total + 2u > 512u) {
         if (tid == 0) build_trees_serial(s);
         __syncthreads();
@@ -333,10 +378,29 @@ __device__ void write_book(BookSmem &s, uint8_t *book, int tid, int nthr) {
     uint32_t *wt = reinterpret_cast<uint32_t *>(book + KVC_BOOK_OFF_TREE);
     for (int i = tid; i < 512; i += nthr) wt[i] = s.tree[i];
     uint32_t *lut = reinterpret_cast<uint32_t *>(book + KVC_BOOK_OFF_LUT);
+    // The windows' first symbols, a warp per symbol: a code of up to KVC_LUT_BITS bits has a run of windows.  The others follow from the windows
+    // behind; only a window without a complete code walks the tree.
+    for (int i = tid; i < KVC_LUT_SIZE / 2; i += nthr) reinterpret_cast<uint32_t *>(s.first)[i] = 0u;
+    __syncthreads();
+    if (!s.by_walk) for (int i = tid >> 5; i < s.n_listed; i += nthr / 32) {
+        const uint32_t sym = s.listed[i], len = s.enc_len[sym];
+        if (len > KVC_LUT_BITS) continue;
+        const uint32_t at = s.aligned[i] >> (32 - KVC_LUT_BITS);
+        for (uint32_t k = tid & 31; k < 1u << (KVC_LUT_BITS - len); k += 32) s.first[at + k] = (uint16_t)(sym | len << 8);
+    }
+    __syncthreads();
     int no_code = 0, lone = 0;                              // entries whose window holds no complete code, fewer than two of them
     if (tid == 0) s.lone = 0;
     for (int w = tid; w < KVC_LUT_SIZE; w += nthr) {
-        const uint32_t e = lut_entry(s.tree, (uint32_t)w);
+        uint32_t e = 0, used = 0, nsym = 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const uint32_t f = s.first[((uint32_t)w << used) & (KVC_LUT_SIZE - 1)], len = f >> 8;
+            if (nsym < (uint32_t)k || len == 0 || used + len > KVC_LUT_BITS) continue;
+            e |= (f & 0xffu) << (8 * (k + 1));
+            used += len; nsym++;
+        }
+        e = nsym ? e | nsym << 6 | used : lut_entry(s.tree, (uint32_t)w);
         lut[w] = e;
         no_code |= (e & 0xffu) == 0;
         lone += (e & 0x80u) == 0;
@@ -363,13 +427,24 @@ __global__ void __launch_bounds__(BOOK_THREADS) build_codebook_kernel(const unsi
     uint32_t nsym;
     const uint32_t slot = book_scan(s, count > 0 ? 1u : 0u, tid, &nsym);
     if (count > 0) { s.listed[slot] = (uint8_t)tid; s.count[slot] = count; }
-    __syncthreads();
+    const int large = __syncthreads_or(count > 0 && (unsigned long long)count > 0xffffffffu / nsym);      // the sum may not fit 32 bits
     if (tid == 0) {
         s.n_symbols = (int)nsym; s.min_sym = nsym ? s.listed[0] : 0; s.max_sym = nsym ? s.listed[nsym - 1] : 0;
         if (nsym == 0) s.flags |= KVC_FLAG_NO_SYMBOLS;
+        short next = 256;
+        if (!large) {
+            Heap32 hp;
+            hp.w = reinterpret_cast<uint2 *>(s.hf); hp.n = 0;
+            for (uint32_t i = 0; i < nsym; i++) hp.push((uint32_t)s.count[i], s.listed[i]);
+            while (hp.n > 1) {
+                const uint2 a = hp.pop(), b = hp.pop();
+                s.parent[a.y] = (short)(next << 1); s.parent[b.y] = (short)(next << 1 | 1);
+                hp.push(a.x + b.x, (uint32_t)next);
+                next++;
+            }
+        } else {
         Heap hp; hp.w = reinterpret_cast<unsigned long long *>(s.hf); hp.n = 0;
         for (uint32_t i = 0; i < nsym; i++) heap_push(hp, s.count[i], (short)s.listed[i]);
-        short next = 256;
         while (hp.n > 1) {
             long long fa, fb;
             short a = heap_pop(hp, &fa);
@@ -377,6 +452,7 @@ __global__ void __launch_bounds__(BOOK_THREADS) build_codebook_kernel(const unsi
             s.parent[a] = (short)(next << 1); s.parent[b] = (short)(next << 1 | 1);
             heap_push(hp, fa + fb, next);
             next++;
+        }
         }
         s.total = next - 1;                                 // the root
     }
@@ -409,9 +485,47 @@ __global__ void __launch_bounds__(BOOK_THREADS) book_from_tree_kernel(const uint
     if (tid < 256) { s.enc_code[tid] = 0; s.enc_len[tid] = 0; }
     if (tid < 512) s.tree[tid] = KVC_TREE_NONE | (KVC_TREE_NONE << 16);
     if (tid < 3 * min(n_nodes, 256)) rt[tid] = tree[tid];
+    // A thread per node.  Where every node has one parent at most, the first two none, and no symbol two leaves, the leaves find their codes on the way up; any
+    // other tensor is walked from the top by one thread, the last leaf of a symbol counting.  (A tree of 43 nodes: 15.0 us with one thread and the table bit by bit, now 8.0.)
+    const bool live = tid < n_nodes && tid < 256;
+    int *const parents = reinterpret_cast<int *>(s.hf), *const leaves = parents + 256;      // by node and by symbol: how many
+    if (tid < 512) parents[tid] = 0;
+    if (tid < 256) s.parent[tid] = -1;
+    if (tid == 0) { s.flags = 0; s.max_len = 0; s.n_symbols = 0; s.min_sym = 256; s.max_sym = -1; }
     __syncthreads();
-    if (tid == 0) {
-        s.flags = 0; s.max_len = 0;
+    const int c0 = live ? rt[3 * tid + 1] : 0xff, c1 = live ? rt[3 * tid + 2] : 0xff;
+    const bool leaf = live && rt[3 * tid] != 0;
+    if (live && !leaf) {
+        if (c0 != 0xff && c0 < n_nodes) { atomicAdd(&parents[c0], 1); s.parent[c0] = (short)(tid << 1); }
+        if (c1 != 0xff && c1 < n_nodes) { atomicAdd(&parents[c1], 1); s.parent[c1] = (short)(tid << 1 | 1); }
+    }
+    __syncthreads();
+    int odd = live && parents[tid] > (tid < 2 ? 0 : 1);
+    uint32_t code = 0;
+    int len = 0;
+    if (leaf) {
+        int nd = tid;
+        for (; nd >= 2 && len < 256; len++) {
+            const int up = s.parent[nd];
+            if (up < 0) break;
+            if (len < 32) code |= (uint32_t)(up & 1) << len;
+            nd = up >> 1;
+        }
+        if (nd < 2) {                                       // (else: a leaf that no root leads to)
+            if (len < 32) code |= (uint32_t)nd << len;
+            len++;
+            odd |= atomicAdd(&leaves[c0], 1) > 0;
+        } else len = 0;
+    }
+    odd = __syncthreads_or(odd);
+    if (!odd && len) {
+        s.enc_code[c0] = code; s.enc_len[c0] = (uint32_t)len;
+        atomicAdd(&s.n_symbols, 1); atomicMax(&s.max_len, len); atomicMin(&s.min_sym, c0); atomicMax(&s.max_sym, c0);
+        if (len > 32) atomicOr(&s.flags, KVC_FLAG_CODE_TOO_LONG);
+    }
+    __syncthreads();
+    if (!odd && tid == 0 && s.n_symbols == 0) { s.min_sym = s.max_sym = 0; s.flags |= KVC_FLAG_NO_SYMBOLS; }
+    if (odd && tid == 0) {
         int nsym = 0, mn = 256, mx = -1;
         short *st_node = s.hid; long long *st_code = s.hf;
         int sp = 0;
