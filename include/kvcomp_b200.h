@@ -297,6 +297,9 @@ int kvc_fused_qk(const kvc_cache *k, int64_t T, int64_t B, int64_t Hkv, int64_t 
  * out: device fp16 [T/128, B, Hq, 128] (the reference's C; its caller sums over g). */
 int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hkv, int64_t Hq,
                  const void *P, void *out, int32_t *status, kvc_stream_t stream);
+/* The sum over kvc_fused_pv's groups (models/cache/kvcomp_encode.py:275): part device fp16 [groups, B, Hq, 128] -> out device fp16
+ * [B, Hq, 128], summed in fp32.  Both 8-byte aligned. */
+int kvc_pv_sum(const void *part, int64_t groups, int64_t B, int64_t Hq, void *out, kvc_stream_t stream);
 
 /* One decode step of eager_attention_forward (models/llama.py:211-234) straight from the
  * compressed caches: out[b,hq,:] = softmax(q K^T * scaling) V over T compressed tokens

@@ -91,6 +91,7 @@ _SIGNATURES = {
     "kvc_decode_values": (_i32, [C.POINTER(Cache), _i64, _i64, _i64, _i32, _vp, _vp, _vp]),
     "kvc_fused_qk": (_i32, [C.POINTER(Cache), _i64, _i64, _i64, _i64, _vp, _vp, _i32, _vp, _vp]),
     "kvc_fused_pv": (_i32, [C.POINTER(Cache), _i64, _i64, _i64, _i64, _vp, _vp, _vp, _vp]),
+    "kvc_pv_sum": (_i32, [_vp, _i64, _i64, _i64, _vp, _vp]),
     "kvc_attn_workspace": (_i64, [_i64, _i64, _i32]),
     "kvc_attn_splits": (_i32, [_i64, _i64, _i64, _i32]),
     "kvc_attn_decode": (_i32, [C.POINTER(Cache), C.POINTER(Cache), _i64, _i64, _i64, _i64, _vp, _f32, _vp, _vp,

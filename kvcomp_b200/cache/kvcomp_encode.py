@@ -663,7 +663,7 @@ class KVCompCtx:
                 C, _ = ops.fused_qk(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
             else:
                 part, _ = ops.fused_pv(self._argument(), self.compressed_ctx_len, self.batch_size, self.head_num, B, status=call.status)
-                C = part.sum(dim=0, keepdim=True, dtype=torch.float32).half()
+                C = ops.pv_sum(part)
             return C, call.end("mat_vec_mul")
 
     def save(self, path):

@@ -1839,6 +1839,43 @@ extern "C" int kvc_fused_pv(const kvc_cache *v, int64_t T, int64_t B, int64_t Hk
     return KVC_OK;
 }
 
+namespace {
+// The sum over a head's partial outputs: CTA = (sequence, query head); a warp takes every eighth row, 4 channels a lane, 8 rows on their way at
+// once.  Bound by the trips to L2.  (As a reduction and a conversion of torch's, 128 groups of 32 heads: 5.5 and 2.0 us and a launch more; now 3.0.)
+__global__ void __launch_bounds__(256) pv_sum_kernel(const __half *__restrict__ part, long long groups, long long rows, __half *__restrict__ out) {
+    __shared__ float4 sums[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const __half *src = part + (long long)blockIdx.x * 128 + lane * 4;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long g0 = warp; g0 < groups; g0 += 64) {
+        uint2 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) if (g0 + 8 * k < groups) x[k] = __ldg(reinterpret_cast<const uint2 *>(src + (g0 + 8 * k) * rows * 128));
+#pragma unroll
+        for (int k = 0; k < 8; k++) if (g0 + 8 * k < groups) {
+            const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&x[k].x)), hi = __half22float2(*reinterpret_cast<const __half2 *>(&x[k].y));
+            a.x += lo.x; a.y += lo.y; a.z += hi.x; a.w += hi.y;
+        }
+    }
+    sums[warp][lane] = a;
+    __syncthreads();
+    if (warp) return;
+#pragma unroll
+    for (int w = 1; w < 8; w++) { const float4 o = sums[w][lane]; a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w; }
+    __half2 r[2] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w)};
+    *reinterpret_cast<uint2 *>(out + (long long)blockIdx.x * 128 + lane * 4) = *reinterpret_cast<const uint2 *>(r);
+}
+}  // namespace
+
+extern "C" int kvc_pv_sum(const void *part, int64_t groups, int64_t B, int64_t Hq, void *out, kvc_stream_t stream) {
+    KVC_REQUIRE(part && out, "kvc_pv_sum: null pointer");
+    KVC_REQUIRE(groups > 0 && B > 0 && Hq > 0 && B * Hq < (1ll << 31), "kvc_pv_sum: bad shape");
+    KVC_REQUIRE(((reinterpret_cast<uintptr_t>(part) | reinterpret_cast<uintptr_t>(out)) & 7) == 0, "kvc_pv_sum: part and out must be 8-byte aligned");
+    pv_sum_kernel<<<(unsigned)(B * Hq), 256, 0, kvc_cu(stream)>>>(reinterpret_cast<const __half *>(part), groups, B * Hq, reinterpret_cast<__half *>(out));
+    KVC_LAUNCH_OK();
+    return KVC_OK;
+}
+
 // Diagnostics for tests of the bounded waits (kvc_attn_debug): process-wide, read at every launch.
 static int g_wait_limit = 0, g_starve = 0;
 extern "C" void kvc_attn_debug(int wait_limit, int starve) { g_wait_limit = wait_limit; g_starve = starve; }

@@ -591,6 +591,16 @@ def fused_pv(cache, T, B, Hkv, P, out=None, status=None):
     return out, status
 
 
+def pv_sum(part):
+    """The groups' partials of fused_pv summed: fp16 [n, B, Hq, 128] -> fp16 [1, B, Hq, 128]."""
+    _cuda(part, torch.float16, "part")
+    n, B, Hq, _ = part.shape
+    out = torch.empty((1, B, Hq, 128), dtype=torch.float16, device=part.device)
+    with _on(part.device):
+        _lib.check(_lib.load().kvc_pv_sum(_p(part), n, B, Hq, _p(out), _stream()), "kvc_pv_sum")
+    return out
+
+
 def attn_splits(T, B, Hkv):
     return int(_lib.load().kvc_attn_splits(T, B, Hkv, 0))
 
