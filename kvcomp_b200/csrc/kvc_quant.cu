@@ -62,19 +62,25 @@ __device__ __forceinline__ uint32_t quant_one(__half x, const UnitParam &p, int 
 }
 
 // quantise 8 halves held in a uint4 -> 8 code bytes in a uint2; optional smem histogram.
-// PS: 0 = the eight values share one unit (p[0]), 1 = value i belongs to unit p[i].
+// PS: 0 = the eight values share one unit (p[0]), 1 = value i belongs to unit p[i].  mi2: 512 + min_int (mid_of).
 //
-// Packed path, for units whose min_int lies in -255..255 (`small_min`; mi2 holds the min_ints as fp16 pairs):
+// Packed path, for units whose min_int lies in -255..255 (`small_min`; mi2 holds 512 + min_int as fp16 pairs):
 // after the fp32 product q0 = x * (1 / scale) everything is done on two values per instruction in fp16, which
 // is what the reference's tensors hold anyway.
 //  * fp16(q0) equals the reference's fp16(x / scale) except on exact ties between two fp16 subnormals, where
 //    both round to the integer 0 (checked over every pair of fp16 values).
-//  * (qh + 1536) - 1536 in fp16 is rint(qh) for |qh| <= 512; beyond that the result stays beyond 511 in
-//    magnitude or is no integer, and with |min_int| <= 255 such a value fails the range test below.
-//  * d = r - min_int, then d + 1024 has the bit pattern 0x6400 + d for the integers 0 <= d < 1024: the code is
-//    read from the mantissa, and one mask over all eight tells whether every code is in 0..255.
+//  * qh + 1536 in fp16 is rint(qh) + 1536, exactly, for |qh| <= 512, and 512 + min_int is exact, so their difference t is 1024 + code: the bit pattern
+//    0x6400 + code for codes 0 .. 1023, whose low byte is the code; one comparison over all eight tells whether every code is in 0 .. 255.  Beyond 512 the sum is
+//    2048 or more and t above 1280, below -512 the sum is below 1024 and t below 768: such values fail the comparison.
+//    (With rint(qh), the code and 1024 + code one after the other, 268 MB of keys 183.6 us and of values 114, now 177 and 104.6, a launch's 15 us included.)
 // Anything else (a value out of range, not finite, a unit with a large min_int) takes the fp32 path below it,
 // which follows the reference's arithmetic to the end.
+__device__ __forceinline__ float mid_of(float mi) { return 512.0f + mi; }
+// the bit patterns of 1024 + code of two values from their quotients; mid: 512 + min_int
+__device__ __forceinline__ uint32_t code_pair(float q0, float q1, const __half2 &mid) {
+    const __half2 t = __hsub2_rn(__hadd2_rn(__floats2half2_rn(q0, q1), __float2half2_rn(1536.0f)), mid);
+    return *reinterpret_cast<const uint32_t *>(&t);
+}
 template <int PS>
 __device__ __forceinline__ uint2 quant_eight(const uint4 &v, const UnitParam *p, bool small_min, const __half2 *mi2,
                                              int *flags, unsigned int *hist) {
@@ -82,21 +88,17 @@ __device__ __forceinline__ uint2 quant_eight(const uint4 &v, const UnitParam *p,
     uint2 o;
     if (small_min) {
         const __half2 *h2 = reinterpret_cast<const __half2 *>(&v);
-        const __half2 big = __float2half2_rn(1536.0f), nbig = __float2half2_rn(-1536.0f), k1024 = __float2half2_rn(1024.0f);
         uint32_t u[4], odd = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 xf = __half22float2(h2[k]);
-            const __half2 qh = __floats2half2_rn(__fmul_rn(xf.x, p[2 * k * PS].rcp), __fmul_rn(xf.y, p[(2 * k + 1) * PS].rcp));
-            const __half2 r = __hadd2(__hadd2(qh, big), nbig);
-            const __half2 t = __hadd2(__hsub2(r, mi2[k * PS]), k1024);
-            u[k] = *reinterpret_cast<const uint32_t *>(&t) - 0x64006400u;
-            odd |= u[k];
+            u[k] = code_pair(__fmul_rn(xf.x, p[2 * k * PS].rcp), __fmul_rn(xf.y, p[(2 * k + 1) * PS].rcp), mi2[k * PS]);
+            odd |= u[k] ^ 0x64006400u;
         }
         if ((odd & 0xff00ff00u) == 0) {
             if (hist) {
 #pragma unroll
-                for (int k = 0; k < 4; k++) { atomicAdd(&hist[u[k] & 0xffu], 1u); atomicAdd(&hist[u[k] >> 16], 1u); }
+                for (int k = 0; k < 4; k++) { atomicAdd(&hist[u[k] & 0xffu], 1u); atomicAdd(&hist[u[k] >> 16 & 0xffu], 1u); }
             }
             o.x = __byte_perm(u[0], u[1], 0x6420);
             o.y = __byte_perm(u[2], u[3], 0x6420);
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(128) quant_channel_kernel(
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         small = small && small_min_int(p[2 * k].mi) && small_min_int(p[2 * k + 1].mi);
-        mi2[k] = __floats2half2_rn(p[2 * k].mi, p[2 * k + 1].mi);
+        mi2[k] = __floats2half2_rn(mid_of(p[2 * k].mi), mid_of(p[2 * k + 1].mi));
     }
     for (int i = r; i < blk; i += 8) {
         uint4 v = *reinterpret_cast<const uint4 *>(x + base + i * row_stride);
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(256) quant_contig_kernel(
         UnitParam p = unit_param(mn, mx, rel, &sc, &flags);
         if (gl == 0) { scale[u] = sc; store_min(min_int, min_bytes, u, p.mi, &flags); }
         const bool small = small_min_int(p.mi);
-        const __half2 mi2 = __float2half2_rn(p.mi);
+        const __half2 mi2 = __float2half2_rn(mid_of(p.mi));
         for (long long k = gl; k < chunks; k += GROUP) {
             uint4 v = *reinterpret_cast<const uint4 *>(xu + k * 8);
             uint2 o = quant_eight<0>(v, &p, small, &mi2, &flags, ghist ? shist + warp * 256 : nullptr);
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__(WARPS == 1 ? 256 : WARPS * 32) quant_contig_re
         const UnitParam p = unit_param(mn, mx, rel, &sc, &flags);
         if (gt == 0) { scale[u] = sc; store_min(min_int, min_bytes, u, p.mi, &flags); }
         const bool small = small_min_int(p.mi);
-        const __half2 mi2 = __float2half2_rn(p.mi);
+        const __half2 mi2 = __float2half2_rn(mid_of(p.mi));
 #pragma unroll
         for (int i = 0; i < CH; i++) {
             const uint2 o = quant_eight<0>(v[i], &p, small, &mi2, &flags, ghist ? shist + warp * 256 : nullptr);
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(256) quant_block_apply_kernel(
     p.rcp = (p.sf == 0.0f || p.sf != p.sf) ? 0.0f : __frcp_rn(p.sf);
     int flags = 0;
     const bool small = small_min_int(p.mi);
-    const __half2 mi2 = __float2half2_rn(p.mi);
+    const __half2 mi2 = __float2half2_rn(mid_of(p.mi));
     for (long long k = tid; k < row_len / 8; k += 256) {
         uint4 v = *reinterpret_cast<const uint4 *>(x + row * row_len + k * 8);
         uint2 o = quant_eight<0>(v, &p, small, &mi2, &flags, ghist ? shist + (tid >> 5) * 256 : nullptr);
@@ -448,20 +450,22 @@ __device__ __forceinline__ void rope8(const uint4 &xa, const uint4 &xb, const ui
 // Bound by memory: 2 bytes read and 1 written per value, where a rotated and transposed copy of the tensor took 4 more before
 // the quantiser read it (K per channel: twice).
 
-// The CTA's histogram: codes below 32 are counted two at a time, n[first + 32 * second], others one by one behind these 1024
-// counters, n[1024 + code] (three instructions per code one by one, a good half of that for a pair; fewer lanes meet on a counter).
-struct PairBins { unsigned int n[1024 + 256]; };
+// The CTA's histogram: codes below 32 are counted two at a time, n[first + 39 * second], others one by one behind these
+// counters, n[PAIR_BINS + code] (three instructions per code one by one, a good half of that for a pair; fewer lanes meet on a counter).  39: the codes of a
+// unit are a bell curve, and with rows of 32 counters every pair of one first code lies in one bank (268 MB of keys 189 us, with 39 183.6; of values 116.3 and 114).
+constexpr int PAIR_ROW = 39, PAIR_BINS = 31 + 31 * PAIR_ROW + 1;
+struct PairBins { unsigned int n[PAIR_BINS + 256]; };
 __device__ __forceinline__ void bins_clear(PairBins &b, int tid, int nthr) {
-    for (int i = tid; i < 1024 + 256; i += nthr) b.n[i] = 0;
+    for (int i = tid; i < PAIR_BINS + 256; i += nthr) b.n[i] = 0;
     __syncthreads();
 }
-__device__ __forceinline__ void bins_add(PairBins &b, const uint32_t (&u)[4]) {     // two codes per word, 16 bits each
+__device__ __forceinline__ void bins_add(PairBins &b, const uint32_t (&u)[4]) {     // two codes per word, in the low bytes of its halves
     if (((u[0] | u[1] | u[2] | u[3]) & 0x00e000e0u) == 0) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) atomicAdd(reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(b.n) + __dp4a(u[k], 0x00800004u, 0u)), 1u);
+        for (int k = 0; k < 4; k++) atomicAdd(reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(b.n) + __dp4a(u[k], (uint32_t)(4 * PAIR_ROW << 16 | 4), 0u)), 1u);
     } else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) { atomicAdd(&b.n[1024 + (u[k] & 0xffu)], 1u); atomicAdd(&b.n[1024 + (u[k] >> 16)], 1u); }
+        for (int k = 0; k < 4; k++) { atomicAdd(&b.n[PAIR_BINS + (u[k] & 0xffu)], 1u); atomicAdd(&b.n[PAIR_BINS + (u[k] >> 16 & 0xffu)], 1u); }
     }
 }
 __device__ __forceinline__ void bins_flush(const PairBins &b, unsigned long long *gh, int tid) {      // by the first 256 threads
@@ -470,11 +474,11 @@ __device__ __forceinline__ void bins_flush(const PairBins &b, unsigned long long
     unsigned int c = 0;
     const int s = tid >> 3, part = tid & 7;                 // eight threads fold a symbol's row and column
 #pragma unroll
-    for (int k = 0; k < 4; k++) c += b.n[s + 32 * (part * 4 + k)] + b.n[32 * s + part * 4 + k];
+    for (int k = 0; k < 4; k++) c += b.n[s + PAIR_ROW * (part * 4 + k)] + b.n[PAIR_ROW * s + part * 4 + k];
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if (part == 0 && c) atomicAdd(&gh[s], (unsigned long long)c);
-    if (b.n[1024 + tid]) atomicAdd(&gh[tid], (unsigned long long)b.n[1024 + tid]);
+    if (b.n[PAIR_BINS + tid]) atomicAdd(&gh[tid], (unsigned long long)b.n[PAIR_BINS + tid]);
 }
 
 // the packed path of quant_eight with what it needs in registers; param(i): value i's unit, for anything else
@@ -482,16 +486,12 @@ template <class P>
 __device__ __forceinline__ uint2 quant_eight_at(const uint4 &v, const float (&rcp)[8], const __half2 (&mi2)[4], bool small_min, P param,
                                                 int *flags, PairBins *bins) {
     const __half2 *h2 = reinterpret_cast<const __half2 *>(&v);
-    const __half2 big = __float2half2_rn(1536.0f), nbig = __float2half2_rn(-1536.0f), k1024 = __float2half2_rn(1024.0f);
     uint32_t u[4], odd = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const float2 xf = __half22float2(h2[k]);
-        const __half2 qh = __floats2half2_rn(__fmul_rn(xf.x, rcp[2 * k]), __fmul_rn(xf.y, rcp[2 * k + 1]));
-        const __half2 r = __hadd2(__hadd2(qh, big), nbig);
-        const __half2 t = __hadd2(__hsub2(r, mi2[k]), k1024);
-        u[k] = *reinterpret_cast<const uint32_t *>(&t) - 0x64006400u;
-        odd |= u[k];
+        u[k] = code_pair(__fmul_rn(xf.x, rcp[2 * k]), __fmul_rn(xf.y, rcp[2 * k + 1]), mi2[k]);
+        odd |= u[k] ^ 0x64006400u;
     }
     if (!small_min || (odd & 0xff00ff00u) != 0) {
         const __half *h = reinterpret_cast<const __half *>(&v);
@@ -504,7 +504,7 @@ __device__ __forceinline__ uint2 quant_eight_at(const uint4 &v, const float (&rc
 
 // ChannelQuant.  CTA = THREADS / 8 * ROWS tokens (one block) of `heads` heads, one after the other; thread = 8 channels of either
 // half of ROWS rows, whose cos and sin it keeps; the next head's rows are fetched while this one's are at work.
-// (Issue bounds it, 29 instructions per value, with 128 registers two CTAs per SM: 1 GiB of keys 0.68 ms, values 0.43 ms by
+// (Issue bounds it, with 128 registers two CTAs per SM: 1 GiB of keys 0.62 ms, values 0.34 ms by
 // quant_heads_token_kernel; copies and the quantisers of rows took 1.17 and 0.79.  80 registers, three CTAs: 5 % slower.)
 template <int ROWS, int THREADS, bool ROPE>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_kernel(
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_ke
     constexpr int WARPS = THREADS / 32, RT = THREADS / 8;   // RT: rows side by side
     __shared__ __align__(16) __half smn[WARPS][128], smx[WARPS][128];
     __shared__ __align__(16) float psf[128], pmi[128], prcp[128];
-    __shared__ __align__(16) __half phm[128];               // min_int of the units of psmall
+    __shared__ __align__(16) __half phm[128];               // mid_of(min_int) of the units of psmall
     __shared__ unsigned int psmall[4];                      // a bit per channel: small_min_int
     __shared__ PairBins bins;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cg = tid & 7, r = tid >> 3;
@@ -537,6 +537,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_ke
         for (int k = 0; k < ROWS; k++) { na[k] = *reinterpret_cast<const uint4 *>(xr + k * (RT * 128)); nb[k] = *reinterpret_cast<const uint4 *>(xr + k * (RT * 128) + 64); }
     };
     fetch(h0);
+    uint8_t *const out0 = codes + ((tok0 * B + b) * H) * 128 + cg * 8;
+    const size_t out_row = (size_t)RT * B * H * 128;
     int flags = 0;
     for (uint32_t h = h0; h < h1; h++) {
         uint4 va[ROWS], vb[ROWS];
@@ -584,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_ke
             const long long u = ((j * B + b) * H + h) * 128 + tid;
             scale[u] = sc;
             store_min(min_int, min_bytes, u, q.mi, &flags);
-            psf[tid] = q.sf; pmi[tid] = q.mi; prcp[tid] = q.rcp; phm[tid] = __float2half_rn(q.mi);
+            psf[tid] = q.sf; pmi[tid] = q.mi; prcp[tid] = q.rcp; phm[tid] = __float2half_rn(mid_of(q.mi));
             const unsigned int small = __ballot_sync(0xffffffffu, small_min_int(q.mi));
             if (lane == 0) psmall[warp] = small;
         }
@@ -602,7 +604,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) quant_heads_channel_ke
 #pragma unroll
             for (int k = 0; k < ROWS; k++) {
                 const uint2 o = quant_eight_at(half ? vb[k] : va[k], rcp, mi2, small, param, &flags, ghist ? &bins : nullptr);
-                *reinterpret_cast<uint2 *>(codes + (((tok0 + RT * k) * B + b) * H + h) * 128 + c0) = o;
+                *reinterpret_cast<uint2 *>(out0 + k * out_row + (size_t)h * 128 + half * 64) = o;
             }
         }
     }
@@ -669,7 +671,7 @@ __global__ void __launch_bounds__(256) quant_heads_token_kernel(
                 p = unit_param(mn, mx, rel, &sc, &flags);
                 if (c0 == 0) { scale[u] = sc; store_min(min_int, min_bytes, u, p.mi, &flags); }
             }
-            const __half2 m2 = __float2half2_rn(p.mi);
+            const __half2 m2 = __float2half2_rn(mid_of(p.mi));
             const float rcp[8] = {p.rcp, p.rcp, p.rcp, p.rcp, p.rcp, p.rcp, p.rcp, p.rcp};
             const __half2 mi2[4] = {m2, m2, m2, m2};
             *reinterpret_cast<uint2 *>(codes + u * 128 + c0) = quant_eight_at(v[i], rcp, mi2, small_min_int(p.mi), [&](int) { return p; }, &flags, ghist ? &bins : nullptr);
