@@ -3,74 +3,95 @@
 // One launch, one 64-thread CTA per block of 64 vectors, a deterministic stream:
 //   sizes   the 64x128 code tile is staged in shared memory once; a thread per vector sums its code
 //           lengths, a two-warp scan gives thread_info and the block's byte count
-//   encode  the thread joins its codes to words (through a 64-bit register, or as below) and ORs these into a zeroed
-//           shared-memory image of the block (a vector shares its first and last word with its neighbours)
+//   encode  the thread joins its codes to words and stores these in a shared-memory image of the block (a vector shares its first and last word
+//           with its neighbours); larger alphabets and long codes go through a 64-bit register, ORed into a zeroed image
 //   offset  the block's place in the stream is the sum of the byte counts of all blocks before it: a chained
 //           scan over one state word per block, looked up after the encoding so that the wait is short
 //   copy    the image goes out as 128-bit stores, shifted to the destination's alignment on the way
 // Books whose symbols are all below 32 (error bounds of 0.05 and more) keep the code table in registers, look symbols
-// up with warp shuffles and fill words without a 64-bit register.  (The encoder alone, 256 columns of 4096 tokens, words through a
-// 64-bit register and now: K 125.6 and 124.0 us, V 131.0 and 129.2; 1024 columns 451 and 443, 468 and 458.  Runs differ by 0.2 us.)
+// up with warp shuffles and fill words without a 64-bit register.  What bounds it: the chain of a block's phases -- its number, its codes, sizes, words, offset, copy --
+// with 32 warps per SM that issue 55 % of the time (15 and 16 instructions per symbol).  256 columns of 4096 tokens, words ORed, a mask per code and lengths by byte products, V's
+// codes by 4-byte loads, and now: K 125 and 107 us, V 127 and 113.  (CTAs that stay and draw the next block while one's bytes go out: 196 where one block per CTA takes 135, a
+// block drawn early announces its size late; 18 or 20 CTAs per SM with fewer registers: 144.)
 #include "kvc_decode.cuh"
 
 namespace {
 
-constexpr int TILE_STRIDE = 132;                  // bytes per vector row in shared memory (padded)
+constexpr int TILE_STRIDE = 132;                  // bytes per vector row in shared memory (padded; K's rows written and read by 128-bit words, 144 bytes apart: 145 us where this takes 135)
 constexpr int OUT_CAP = 8192 + 32;                // block image: 8191 bytes max + alignment lead + slack
 
 constexpr int ENC_THREADS = 64;                   // one thread per vector of the block
 constexpr int ENC_WAIT_LIMIT = 1 << 21;           // polls of a block's state word (about 40 ns apart) before a CTA gives up
 
-// Stage the code tile of block `blk` as tile[vector][symbol].
+// The code tile of block `blk`, in shared memory tile[vector][symbol].
 // K: vector v = token 64j+v, symbols = its 128 channels (rows of 128 contiguous bytes).
 // V: vector v = channel column 64m+v, symbols = tokens 128g..128g+127 (transposed on the way in).
-__device__ __forceinline__ void stage_tile(uint8_t *tile, const uint8_t *__restrict__ codes, long long blk,
-                                           long long cols, int is_k, int tid) {
-    const long long row = cols * 128;
-    // K: 16-byte loads, all of a thread's 8 in flight at once (rows are 128 bytes at 16-byte aligned
-    // offsets of a 4-byte aligned base: the base decides whether the wide load is legal)
-    const bool wide = (reinterpret_cast<uintptr_t>(codes) & 15) == 0;
-    if (is_k) {
-        const long long j = blk / cols, col = blk % cols;
-        const uint8_t *src = codes + (j * 64) * row + col * 128;
-        if (wide) {
-            uint4 x[8];
+// (Block and column numbers fit 32 bits: a call has less than 2^31 blocks.)
+__device__ __forceinline__ const uint8_t *tile_source(const uint8_t *codes, uint32_t blk, uint32_t cols, int is_k, size_t row) {
+    const uint32_t per = is_k ? cols : cols * 2, j = blk / per, col = blk - j * per;
+    return is_k ? codes + (j * 64ull) * row + col * 128ull : codes + (j * 128ull) * row + col * 64ull;
+}
+// Codes that start on 16 bytes: a thread's eight 16-byte loads, all in flight at once, apart from the stores.
+struct TileLoads {
+    uint4 x[8];
+    __device__ __forceinline__ void fetch(const uint8_t *codes, uint32_t blk, uint32_t cols, int is_k, int tid) {
+        const size_t row = (size_t)cols * 128;
+        const uint8_t *p = tile_source(codes, blk, cols, is_k, row);
+        if (is_k) {                                             // 64 rows x 8 chunks
+            p += (tid >> 3) * row + (tid & 7) * 16;
 #pragma unroll
-            for (int k = 0; k < 8; k++) {                       // 64 rows x 8 chunks of 16 bytes
-                const int i = tid + k * ENC_THREADS, v = i >> 3, c = i & 7;
-                x[k] = *reinterpret_cast<const uint4 *>(src + v * row + c * 16);
-            }
+            for (int k = 0; k < 8; k++) x[k] = *reinterpret_cast<const uint4 *>(p + k * (8 * row));
+        } else {                                                // 4 rows of 4 chunks of 16 channels, twice
+            p += (size_t)((tid >> 2) * 4) * row + (tid & 3) * 16;
+#pragma unroll
+            for (int k = 0; k < 8; k++) x[k] = *reinterpret_cast<const uint4 *>(p + ((k >> 2) * 64 + (k & 3)) * row);
+        }
+    }
+    __device__ __forceinline__ void put(uint8_t *tile, int is_k, int tid) const {
+        if (is_k) {
 #pragma unroll
             for (int k = 0; k < 8; k++) {
-                const int i = tid + k * ENC_THREADS, v = i >> 3, c = i & 7;
-                uint32_t *d = reinterpret_cast<uint32_t *>(tile + v * TILE_STRIDE + c * 16);
+                uint32_t *d = reinterpret_cast<uint32_t *>(tile + ((tid >> 3) + k * 8) * TILE_STRIDE + (tid & 7) * 16);
                 d[0] = x[k].x; d[1] = x[k].y; d[2] = x[k].z; d[3] = x[k].w;
             }
         } else {
-#pragma unroll 8
-            for (int i = tid; i < 64 * 32; i += ENC_THREADS) {  // 64 rows x 32 words
-                int v = i >> 5, w = i & 31;
-                uint32_t x = *reinterpret_cast<const uint32_t *>(src + v * row + w * 4);
-                *reinterpret_cast<uint32_t *>(tile + v * TILE_STRIDE + w * 4) = x;
+            // a word per channel, its 4 tokens; the upper 32 channels' words lie 8 further on (before them where that is), so that no two lanes meet a bank
+            const int c = tid & 3;
+#pragma unroll
+            for (int k = 0; k < 8; k += 4) {
+                uint8_t *d = tile + c * 16 * TILE_STRIDE + ((((tid >> 2) + k * 4) ^ (c & 2) * 4)) * 4;
+                auto four = [&](uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+                    kvc_transpose4x4(x0, x1, x2, x3);
+                    *reinterpret_cast<uint32_t *>(d) = x0; *reinterpret_cast<uint32_t *>(d + TILE_STRIDE) = x1;
+                    *reinterpret_cast<uint32_t *>(d + 2 * TILE_STRIDE) = x2; *reinterpret_cast<uint32_t *>(d + 3 * TILE_STRIDE) = x3;
+                    d += 4 * TILE_STRIDE;
+                };
+                four(x[k].x, x[k + 1].x, x[k + 2].x, x[k + 3].x);
+                four(x[k].y, x[k + 1].y, x[k + 2].y, x[k + 3].y);
+                four(x[k].z, x[k + 1].z, x[k + 2].z, x[k + 3].z);
+                four(x[k].w, x[k + 1].w, x[k + 2].w, x[k + 3].w);
             }
         }
+    }
+};
+// Codes that start on 4 bytes.
+__device__ __forceinline__ void stage_words(uint8_t *tile, const uint8_t *codes, uint32_t blk, uint32_t cols, int is_k, int tid) {
+    const size_t row = (size_t)cols * 128;
+    const uint8_t *src = tile_source(codes, blk, cols, is_k, row);
+    if (is_k) {
+#pragma unroll 8
+        for (int i = tid; i < 64 * 32; i += ENC_THREADS)        // 64 rows x 32 words
+            *reinterpret_cast<uint32_t *>(tile + (i >> 5) * TILE_STRIDE + (i & 31) * 4) = *reinterpret_cast<const uint32_t *>(src + (i >> 5) * row + (i & 31) * 4);
     } else {
-        const long long g = blk / (cols * 2), m = blk % (cols * 2);
-        const uint8_t *src = codes + (g * 128) * row + m * 64;
-        {   // 4-byte loads: 16 lanes cover a token row's 64 bytes, and the transposed stores meet no bank twice
 #pragma unroll 2
-            for (int i = tid; i < 32 * 16; i += ENC_THREADS) {  // 32 groups of 4 token rows x 16 words of 4 channels
-                const int tg = i >> 4, w = i & 15;
-                uint32_t x0 = *reinterpret_cast<const uint32_t *>(src + (tg * 4 + 0) * row + w * 4);
-                uint32_t x1 = *reinterpret_cast<const uint32_t *>(src + (tg * 4 + 1) * row + w * 4);
-                uint32_t x2 = *reinterpret_cast<const uint32_t *>(src + (tg * 4 + 2) * row + w * 4);
-                uint32_t x3 = *reinterpret_cast<const uint32_t *>(src + (tg * 4 + 3) * row + w * 4);
-                kvc_transpose4x4(x0, x1, x2, x3);               // now one word per channel: its 4 tokens
-                *reinterpret_cast<uint32_t *>(tile + (w * 4 + 0) * TILE_STRIDE + tg * 4) = x0;
-                *reinterpret_cast<uint32_t *>(tile + (w * 4 + 1) * TILE_STRIDE + tg * 4) = x1;
-                *reinterpret_cast<uint32_t *>(tile + (w * 4 + 2) * TILE_STRIDE + tg * 4) = x2;
-                *reinterpret_cast<uint32_t *>(tile + (w * 4 + 3) * TILE_STRIDE + tg * 4) = x3;
-            }
+        for (int tg = tid >> 4; tg < 32; tg += ENC_THREADS / 16) {      // 32 groups of 4 token rows x 16 words of 4 channels
+            const uint8_t *p = src + (tg * 4) * row + (tid & 15) * 4;
+            uint32_t x0 = *reinterpret_cast<const uint32_t *>(p), x1 = *reinterpret_cast<const uint32_t *>(p + row);
+            uint32_t x2 = *reinterpret_cast<const uint32_t *>(p + 2 * row), x3 = *reinterpret_cast<const uint32_t *>(p + 3 * row);
+            kvc_transpose4x4(x0, x1, x2, x3);
+            uint8_t *d = tile + ((tid & 15) * 4) * TILE_STRIDE + (tg ^ (tid & 8)) * 4;
+            *reinterpret_cast<uint32_t *>(d) = x0; *reinterpret_cast<uint32_t *>(d + TILE_STRIDE) = x1;
+            *reinterpret_cast<uint32_t *>(d + 2 * TILE_STRIDE) = x2; *reinterpret_cast<uint32_t *>(d + 3 * TILE_STRIDE) = x3;
         }
     }
 }
@@ -120,31 +141,43 @@ __device__ __forceinline__ void encode_vector(const uint32_t (&row)[32], const u
 }
 
 // encode_vector<true> for a book whose symbols are all below 32: the table lives in the warp's registers, lane i
-// holding symbol i's code, first bit on top, with its length in the low byte, and a lookup is a shuffle (one pass of the
+// holding symbol i's code, first bit on top, with its length in the low six bits, and a lookup is a shuffle (one pass of the
 // shared-memory pipe, no bank conflicts) instead of a 64-bit shared load at a data-dependent address.  Every lane of the warp must
 // call this, with symbols below 32 only (the shuffle reads lane `symbol mod 32`).
-// `cur` holds the bits of the word at work, `have` how many (only the low five bits count; bit 5 changes when a word is full): a pair
-// of codes is at most 32 bits, so it fills one word at most.
-__device__ __forceinline__ void encode_vector_shfl(const uint32_t (&row)[32], uint32_t entry, uint32_t *out, uint32_t start) {
+// `cur` holds the bits of the word at work, `have` how many: only its low five bits count, bit 5 changes when a word is full, and whatever codes lie above the lengths that
+// are added to it stays above.  SIZE: bits of the longest code: of 13 or fewer a pair's 26 leave the lengths' six bits free, so that one mask clears both; of 8 or fewer
+// four codes make one piece.
+// Words are stored as they fill, the first with zeros in front (the vector has 32 bits or more); what does not fill a word is returned, with its place.
+// (Per pair of symbols, with a mask per code, lengths by byte products and an OR into a zeroed image: 18 instructions, now 13, four codes together 11.)
+struct Piece { uint32_t at, bits; };
+template <int SIZE>
+__device__ __forceinline__ Piece encode_vector_shfl(const uint32_t (&row)[32], uint32_t entry, uint32_t *out, uint32_t start) {
+    constexpr uint32_t CODE = 0xffffffc0u;
     uint32_t at = kvc_smem_addr(out) + (start & ~3u), have = (start & 3u) * 8, cur = 0;
-    auto put = [&](uint32_t e0, uint32_t e1) {
-        const uint32_t c = (e0 & 0xffffff00u) + __funnelshift_r(e1 & 0xffffff00u, 0u, e0);
-        cur += __funnelshift_r(c, 0u, have);
-        const uint32_t rest = __funnelshift_r(0u, c, have), next = (uint32_t)kvc_dp4a_uu(e1, 1u, kvc_dp4a_uu(e0, 1u, (int)have));
-        const uint32_t full = (next ^ have) & 32u;
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p red.shared.or.b32 [%1], %2;\n\t}" :: "r"(full), "r"(at), "r"(cur) : "memory");
-        at += full >> 3; cur = full ? rest : cur;
+    auto put = [&](uint32_t c, uint32_t next) {
+        const uint32_t w = cur + __funnelshift_r(c, 0u, have), rest = __funnelshift_r(0u, c, have);
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\txor.b32 t, %4, %5;\n\tand.b32 t, t, 32;\n\tsetp.ne.u32 p, t, 0;\n\t@p st.shared.u32 [%0], %2;\n\t@p add.u32 %0, %0, 4;\n\tselp.b32 %1, %3, %2, p;\n\t}"
+                     : "+r"(at), "=r"(cur) : "r"(w), "r"(rest), "r"(next), "r"(have) : "memory");
         have = next;
+    };
+    auto pair = [&](uint32_t e0, uint32_t e1) {
+        if (SIZE > 13) return (e0 & CODE) | __funnelshift_r(e1 & CODE, 0u, e0);
+        return (e0 | __funnelshift_r(e1, 0u, e0)) & CODE;
     };
 #pragma unroll
     for (int w = 0; w < 32; w++) {
         const uint32_t x = row[w];
         const uint32_t e0 = __shfl_sync(0xffffffffu, entry, x), e1 = __shfl_sync(0xffffffffu, entry, x >> 8);
         const uint32_t e2 = __shfl_sync(0xffffffffu, entry, x >> 16), e3 = __shfl_sync(0xffffffffu, entry, x >> 24);
-        put(e0, e1);
-        put(e2, e3);
+        if (SIZE <= 8) {
+            const uint32_t l = e0 + e1;
+            put(pair(e0, e1) | __funnelshift_r(pair(e2, e3), 0u, l), have + l + e2 + e3);
+        } else {
+            put(pair(e0, e1), have + e0 + e1);
+            put(pair(e2, e3), have + e2 + e3);
+        }
     }
-    if (have & 31u) asm volatile("red.shared.or.b32 [%0], %1;" :: "r"(at), "r"(cur) : "memory");
+    return {at, cur};
 }
 
 // ---- single pass ------------------------------------------------------------------------------
@@ -208,33 +241,48 @@ __global__ void __launch_bounds__(ENC_THREADS, 16) encode_onepass_kernel(
     __shared__ uint2 tab[256];                              // {code, length}
     __shared__ uint16_t lens[256];                          // length, or 1 << 14 for a symbol without a code
     __shared__ uint32_t wsum[2];
+    __shared__ int wkind[2];
     __shared__ unsigned int s_blk;
     __shared__ unsigned long long s_excl;
     __shared__ int s_dead;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) { s_blk = atomicAdd(ticket, 1u); s_dead = 0; }
-    int kind = 0;                                           // 1: a code longer than 16 bits, 2: a coded symbol >= 32
-    for (int i = tid; i < 256; i += ENC_THREADS) {
-        const uint2 e = i < n_entries ? make_uint2(enc[2 * i], enc[2 * i + 1]) : make_uint2(0u, 0u);
+    uint2 te[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) { const int i = tid + k * ENC_THREADS; te[k] = i < n_entries ? make_uint2(__ldg(enc + 2 * i), __ldg(enc + 2 * i + 1)) : make_uint2(0u, 0u); }
+    __syncthreads();
+    const uint32_t blk = s_blk;
+    TileLoads loads;
+    const bool wide = (reinterpret_cast<uintptr_t>(codes) & 15) == 0;
+    if (wide) loads.fetch(codes, blk, (uint32_t)cols, is_k, tid);
+    int kind = 0;                                           // 1: a code longer than 16 bits, 2: a coded symbol >= 32, 4, 8: a code longer than 13, 8 bits
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int i = tid + k * ENC_THREADS;
+        const uint2 e = te[k];
         tab[i] = e;
-        kind |= (e.y > 16u ? 1 : 0) | (e.y && i >= 32 ? 2 : 0);
+        kind |= (e.y > 16u ? 1 : 0) | (e.y && i >= 32 ? 2 : 0) | (e.y > 13u ? 4 : 0) | (e.y > 8u ? 8 : 0);
         const uint32_t l = min(e.y, 32u);
         lens[i] = (uint16_t)(l ? l : (1u << 14));
     }
-    kind = __syncthreads_or(kind);
+    kind = (int)__reduce_or_sync(0xffffffffu, (unsigned)kind);
+    if (lane == 0) wkind[warp] = kind;
+    __syncthreads();
+    kind = wkind[0] | wkind[1];                             // (__syncthreads_or would say whether any bit is set, not which)
     const bool long_codes = (kind & 1) != 0;
-    const bool small_book = kind == 0;                      // the table fits a warp's registers
-    const long long blk = s_blk;
+    const bool small_book = (kind & 3) == 0;                // the table fits a warp's registers
     // lane i: symbol i's code, first bit on top, and length for the encoding, and its length (or the marker) for the sizes
     const uint32_t my_entry = small_book && tab[lane].y ? (tab[lane].x << (32 - tab[lane].y)) | tab[lane].y : 0u, my_len = lens[lane];
-    stage_tile(tile, codes, blk, cols, is_k, tid);
+    if (wide) loads.put(tile, is_k, tid);
+    else stage_words(tile, codes, blk, (uint32_t)cols, is_k, tid);
     __syncthreads();
     int flags = 0;
     uint32_t bits = 0;
     const uint32_t *rowp = reinterpret_cast<const uint32_t *>(tile + tid * TILE_STRIDE);
+    const int turn = is_k ? 0 : warp * 8;                   // V's upper channels: words 8 .. 15 before 0 .. 7, 24 .. 31 before 16 .. 23
     uint32_t row[32];
 #pragma unroll
-    for (int w = 0; w < 32; w++) row[w] = rowp[w];
+    for (int w = 0; w < 32; w++) row[w] = (w & 8) ? rowp[w - turn] : rowp[w + turn];
     uint32_t seen = 0;
 #pragma unroll
     for (int w = 0; w < 32; w++) seen |= row[w];
@@ -248,9 +296,9 @@ __global__ void __launch_bounds__(ENC_THREADS, 16) encode_onepass_kernel(
                     __shfl_sync(0xffffffffu, my_len, x >> 16) + __shfl_sync(0xffffffffu, my_len, x >> 24);
         }
     } else {
-#pragma unroll 8
+#pragma unroll
         for (int w = 0; w < 32; w++) {
-            const uint32_t x = rowp[w];
+            const uint32_t x = row[w];
             bits += lens[x & 0xffu] + lens[(x >> 8) & 0xffu] + lens[(x >> 16) & 0xffu] + lens[x >> 24];
         }
     }
@@ -265,19 +313,30 @@ __global__ void __launch_bounds__(ENC_THREADS, 16) encode_onepass_kernel(
     if (warp == 1) start += wsum[0];
     const uint32_t nbytes = wsum[0] + wsum[1];
     // kernels.cu:462-465: (end byte << 3) + pad bits
-    thread_info[blk * 64 + tid] = (uint16_t)(((start + n) << 3) + (n * 8 - bits));
+    thread_info[(size_t)blk * 64 + tid] = (uint16_t)(((start + n) << 3) + (n * 8 - bits));
     const bool fits = nbytes <= 8191u;                       // else its u16 fields cannot describe the block
     // Later blocks may add this block's bytes to their offsets from here on; its own offset is looked up
     // after the encoding, when the blocks before it have long announced theirs.
     if (tid == 0 && !(starve && blk == 0)) st_state(state + blk, (blk > 0 ? ST_AGG : ST_PREFIX) | nbytes);   // the first block's offset is 0
     if (fits) {
-        // The image starts at byte 0 of the shared array, whatever the destination's alignment; it is zeroed
-        // past the words the copy-out may touch.
-        for (uint32_t i = tid; i * 16 < nbytes + 24; i += ENC_THREADS) reinterpret_cast<uint4 *>(out)[i] = make_uint4(0u, 0u, 0u, 0u);
-        __syncthreads();
-        if (by_shfl) encode_vector_shfl(row, my_entry, out, start);
-        else if (long_codes) encode_vector<false>(row, tab, out, start);
-        else encode_vector<true>(row, tab, out, start);
+        // The image starts at byte 0 of the shared array, whatever the destination's alignment.  Either all vectors store their words, or (a symbol that the
+        // table or the registers lack, a book of larger symbols) they OR them into zeroes.
+        const bool stored = __syncthreads_and(by_shfl && bits >= 32u);
+        if (!stored) {
+            for (uint32_t i = tid; i * 16 < nbytes + 24; i += ENC_THREADS) reinterpret_cast<uint4 *>(out)[i] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+            if (long_codes) encode_vector<false>(row, tab, out, start);
+            else encode_vector<true>(row, tab, out, start);
+        } else {
+            const Piece last = (kind & 4) ? encode_vector_shfl<16>(row, my_entry, out, start)
+                             : (kind & 8) ? encode_vector_shfl<13>(row, my_entry, out, start) : encode_vector_shfl<8>(row, my_entry, out, start);
+            // A vector that ends within a word shares it with the next one, which stores it with zeros in front: it is added behind the barrier.  One that ends with
+            // the word, its padding included, stores it, and so does the last.
+            const bool partial = (start * 8 + bits) & 31u, shared = ((start + n) & 3u) && tid != ENC_THREADS - 1;
+            if (partial && !shared) asm volatile("st.shared.u32 [%0], %1;" :: "r"(last.at), "r"(last.bits) : "memory");
+            __syncthreads();
+            if (partial && shared) asm volatile("red.shared.or.b32 [%0], %1;" :: "r"(last.at), "r"(last.bits) : "memory");
+        }
     }
     if (warp == 0) {
         unsigned long long excl = 0;
@@ -303,13 +362,12 @@ __global__ void __launch_bounds__(ENC_THREADS, 16) encode_onepass_kernel(
         }
     }
     if (flags) atomicOr(status, flags);
-    if (!fits || !room) return;                              // nothing of this block is written
     // Copy-out in 16-byte pieces of the destination.  Image words hold stream bytes most-significant first;
     // destination byte b (counted from the 16-byte boundary at or before the block's first byte) is image
     // byte b - lead, so a destination word is cut from two image words and swapped to memory order.
     uint8_t *dst = encoded + off;
     const uint32_t lead = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 15);
-    const uint32_t end = lead + nbytes;
+    const uint32_t end = fits && room ? lead + nbytes : 0u;     // (else nothing of this block is written)
     const uint32_t sh = ((4u - (lead & 3u)) & 3u) * 8u;
     uint8_t *g0 = dst - lead;                                   // 16-byte aligned
     for (uint32_t ch = tid; ch * 16 < end; ch += ENC_THREADS) {
