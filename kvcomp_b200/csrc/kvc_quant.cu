@@ -873,6 +873,41 @@ extern "C" int kvc_quantize(const void *x, int64_t T, int64_t B, int64_t H, int6
     return KVC_OK;
 }
 
+// The same for units side by side over the channels that cover TOKENS tokens or more: a thread's eight channels have the same units in all of them, so a
+// thread loads them once and has TOKENS loads of codes in flight.  (512 rows of 32 x 32 heads, 67 M values: 58 us where a thread takes the channels of one
+// token, now 31.)
+namespace {
+template <int TOKENS>
+__global__ void __launch_bounds__(256) dequant_channel_kernel(const uint8_t *__restrict__ codes, kvc_qmeta_dev m, uint32_t H, uint32_t per_head, uint32_t per_token,
+                                                              __half *__restrict__ out) {
+    const uint32_t c = blockIdx.x * 256 + threadIdx.x;      // eight channels of a token's row
+    if (c >= per_token) return;
+    const long long t0 = (long long)blockIdx.y * TOKENS;
+    const uint32_t c0 = (c % per_head) * 8, col = c / per_head, h = col % H, b = col / H;
+    uint2 cv[TOKENS];
+#pragma unroll
+    for (int k = 0; k < TOKENS; k++) cv[k] = *reinterpret_cast<const uint2 *>(codes + ((t0 + k) * per_token + c) * 8);
+    const long long u = kvc_tok_unit(t0, m.tok_div) * m.sj + b * m.sb + h * m.sh + c0;
+    const uint4 sv = *reinterpret_cast<const uint4 *>(m.scale + u);
+    const __half2 *s2 = reinterpret_cast<const __half2 *>(&sv);
+    const __half2 sc[4] = {s2[0], s2[1], s2[2], s2[3]};
+    float mi[8];
+    if (m.min_bytes == 1) {
+        const uint2 mv = *reinterpret_cast<const uint2 *>(reinterpret_cast<const int8_t *>(m.min_int) + u);
+        const int8_t *mb = reinterpret_cast<const int8_t *>(&mv);
+#pragma unroll
+        for (int k = 0; k < 8; k++) mi[k] = (float)mb[k] - 8388608.0f;
+    } else {
+        const uint4 mv = *reinterpret_cast<const uint4 *>(reinterpret_cast<const int16_t *>(m.min_int) + u);
+        const int16_t *mh = reinterpret_cast<const int16_t *>(&mv);
+#pragma unroll
+        for (int k = 0; k < 8; k++) mi[k] = (float)mh[k] - 8388608.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < TOKENS; k++) *reinterpret_cast<uint4 *>(out + ((t0 + k) * per_token + c) * 8) = kvc_dequant8(cv[k].x, cv[k].y, mi, sc);
+}
+}  // namespace
+
 extern "C" int kvc_dequant(const uint8_t *codes, const kvc_qmeta *q, int64_t T, int64_t B, int64_t H, int64_t D,
                            void *out, kvc_stream_t stream) {
     KVC_REQUIRE(codes && q && q->min_int && q->scale && out, "kvc_dequant: null pointer");
@@ -883,6 +918,15 @@ extern "C" int kvc_dequant(const uint8_t *codes, const kvc_qmeta *q, int64_t T, 
     const kvc_qmeta_dev m = kvc_to_dev(*q);
     const int wide_units = m.sc == 1 && m.sj % 8 == 0 && m.sb % 8 == 0 && m.sh % 8 == 0 &&
                            (reinterpret_cast<uintptr_t>(m.scale) & 15) == 0 && (reinterpret_cast<uintptr_t>(m.min_int) & (8 * m.min_bytes - 1)) == 0;
+    // (below 8 tokens for each of 512 threads per SM the single tokens fill the device better: 64 x 128 values 2.1 us)
+    constexpr int TOKENS = 4;
+    const long long per_token = B * H * (D / 8);
+    if (wide_units && m.tok_div % TOKENS == 0 && T % TOKENS == 0 && n > 8 * 512ll * kvc_sm_count() && T / TOKENS <= 65535 && per_token < (1ll << 31)) {
+        dequant_channel_kernel<TOKENS><<<dim3((unsigned)((per_token + 255) / 256), (unsigned)(T / TOKENS)), 256, 0, kvc_cu(stream)>>>(
+            codes, m, (uint32_t)H, (uint32_t)(D / 8), (uint32_t)per_token, reinterpret_cast<__half *>(out));
+        KVC_LAUNCH_OK();
+        return KVC_OK;
+    }
     const int groups = m.sc == 0 && n > 512ll * kvc_sm_count() ? 2 : 1;
     (groups == 2 ? dequant_kernel<2> : dequant_kernel<1>)<<<(unsigned)((n + 256 * groups - 1) / (256 * groups)), 256, 0, kvc_cu(stream)>>>(
         codes, m, rows, (uint32_t)B, (uint32_t)H, (uint32_t)D, wide_units, reinterpret_cast<__half *>(out));
