@@ -30,6 +30,12 @@ class _Arena:
         self.dtype, self.size, self.n = dtype, dtype.itemsize, 0
         self._mem, self._off, self._cap, self._buf = None, 0, 0, None
 
+    def __getstate__(self):                  # a copy makes the view of its own memory anew
+        state = self.__dict__.copy()
+        if state["_buf"] is not state["_mem"]:
+            state["_buf"] = None
+        return state
+
     @property
     def buf(self):
         if self._buf is None and self._mem is not None:

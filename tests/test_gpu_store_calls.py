@@ -65,6 +65,27 @@ def test_keys_that_are_refused_leave_the_values_as_they_were():
     assert _same(_state(vc), _state(cache.v_ctx[1]))
 
 
+@pytest.mark.parametrize("way", ["copy", "pickle"])
+def test_a_copy_goes_on_by_itself(way):
+    """The arenas of a first store share one allocation; a copy's and the original's do not."""
+    import copy
+    import pickle
+    from kvcomp_b200.cache.kvcomp_cache import KVCompCache
+    k, v, rot = _prompt(333, 3)
+    first = {n: x[:, :200].contiguous() for n, x in rot.items()}
+    rest = {n: x[:, 200:].contiguous() for n, x in rot.items()}
+    want, cache = KVCompCache(2, 3, 128, 1), KVCompCache(2, 3, 128, 1)
+    for c in (want, cache):
+        c.append(k[:, :, :200].contiguous(), v[:, :, :200].contiguous(), 0, first)
+    before = [_state(x) for x in (cache.k_ctx[0], cache.v_ctx[0])]
+    ctxs = [copy.deepcopy(x) if way == "copy" else pickle.loads(pickle.dumps(x)) for x in (cache.k_ctx[0], cache.v_ctx[0])]
+    want.append(k[:, :, 200:].contiguous(), v[:, :, 200:].contiguous(), 0, rest)
+    for c, x in zip(ctxs, (k, v)):
+        c.store(x[:, :, 200:].permute(2, 0, 1, 3).contiguous())
+    assert _same(_state(ctxs[0]), _state(want.k_ctx[0])) and _same(_state(ctxs[1]), _state(want.v_ctx[0]))
+    assert all(_same(a, _state(x)) for a, x in zip(before, (cache.k_ctx[0], cache.v_ctx[0])))
+
+
 def test_reports_of_two_threads():
     """Each thread's stores have places of their own."""
     import threading
