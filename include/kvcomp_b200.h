@@ -316,7 +316,8 @@ int kvc_pv_sum(const void *part, int64_t groups, int64_t B, int64_t Hq, void *ou
  * of device memory whose first 256 bytes the caller zeroes once before the first use (the
  * kernel leaves them zeroed); NULL is allowed when splits = 1 (a tail then costs more: the
  * first kernel reads it itself, by the workers of a column).  Launches that share a
- * workspace must not overlap on the device.
+ * workspace must not overlap on the device.  The second kernel runs beside the first where there is room, and reads q and the tails
+ * meanwhile (never before the kernels ahead of the first have ended).
  * The launch uses programmatic stream serialisation: it may read what k and v point to (streams, tables, books,
  * unit parameters) while the kernel directly ahead of it in the stream ends.  That kernel may write q, the tails and
  * anything else, but a kernel that writes the caches' memory needs an ordinary kernel, a copy or a host wait behind

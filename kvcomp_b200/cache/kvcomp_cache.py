@@ -95,7 +95,7 @@ class KVCompCache(_BASE):
                 ops.rope_store(key_states, cos, sin, out=place)
                 kc0.recent_commit(key_states.shape[2])
             else:
-                begun = kc0.begin_heads(key_states, cos, sin)   # rotated with torch's bits
+                begun = kc0.begin_heads(key_states, cos, sin, keep_codes=False)      # rotated with torch's bits
             k_stored = True
         else:
             key_states = apply_rotary_pos_emb_single(key_states, cos, sin)
@@ -129,7 +129,7 @@ class KVCompCache(_BASE):
         both, v_begun = False, None
         try:
             if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and vc.recent_place(values.shape[2], values.device) is None:
-                v_begun = vc.begin_heads(values)
+                v_begun = vc.begin_heads(values, keep_codes=False)
                 both = True
         finally:
             try:

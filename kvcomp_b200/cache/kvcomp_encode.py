@@ -342,8 +342,9 @@ class KVCompCtx:
         are given.  A prompt into an empty window is quantised from where it lies."""
         return self._finish(self.begin_heads(x, cos, sin))
 
-    def begin_heads(self, x, cos=None, sin=None):
-        """store_heads() up to its wait: what finish() takes."""
+    def begin_heads(self, x, cos=None, sin=None, keep_codes=True):
+        """store_heads() up to its wait: what finish() takes.  keep_codes = False: the caller has no use for the codes, and their memory
+        is the next launch's where nothing else needs them."""
         B, H, t, D = x.shape
         live, mode = len(self._recent), _MODE[self.quant_mode]
         n = self._cut(live, t)
@@ -355,7 +356,7 @@ class KVCompCtx:
             return self._begin(ops.rope_store(x, cos, sin))
         self._check(x.permute(2, 0, 1, 3))
         self.ctx_len += t
-        return self._launch(x, n, 0, t - n, t, None, cos, sin, stride)
+        return self._launch(x, n, 0, t - n, t, None, cos, sin, stride, keep_codes)
 
     def store(self, cache):
         """Append tokens [t, B, H, D]; whole blocks beyond the recent window are quantised and encoded.
@@ -378,7 +379,7 @@ class KVCompCtx:
             x, rest = torch.cat([self._recent.view(), cache[:n - live]], dim=0), cache[n - live:]
         return self._launch(x, n, live, rest.shape[0], 0, lambda place: place.copy_(rest))
 
-    def _launch(self, x, n, live, n_rest, x_tokens, put_rest, cos=None, sin=None, stride=0):
+    def _launch(self, x, n, live, n_rest, x_tokens, put_rest, cos=None, sin=None, stride=0, keep_codes=True):
         """Launch the compression of the first n tokens of (the `live` rows of the window + new tokens): x as rows, or (x_tokens > 0) as a
         prompt's heads.  put_rest(place) writes the n_rest last of the new tokens as rows; the heads' own are written by the call."""
         # quantise, book, encode and the rows are launched by one call; one copy brings back what the kernels report
@@ -437,7 +438,11 @@ class KVCompCtx:
                 self.book = None
             ops.wait(dev)
             raise
-        return slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest, build, x, cos, sin, scratch
+        # A book built from these very codes lacks none of them and the room is for the longest stream: with all of them in the stream and the kept rows
+        # written, nothing reads the codes again.  (Keys' and values' on their way together would else be held at the same time.)
+        if not keep_codes and build and over and n_enc == old + n:
+            pend = part = None
+        return slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest, build, blocks
 
     def _abandon(self, begun, t):
         """A begun store of t tokens, waited for, is not to count."""
@@ -449,10 +454,10 @@ class KVCompCtx:
         """The rest of a begun store: waits for it (waited: the caller has), then it counts."""
         if begun is None:
             return None
-        slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest = begun[:15]
+        slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest, _, blocks = begun
         if not waited:
             ops.wait(self.device)
-        words, room, n, codes = ops.Reports.read(slot), self._room(), T, pend[old:] if old else pend
+        words, room, n, codes = ops.Reports.read(slot), self._room(), T, pend[old:] if old and pend is not None else pend
         flags = ops.check_flags(words[2], what="quantize")
         if flags & ops._lib.FLAG_MIN_OVERFLOW:
             # int8 is the reference's CUDA path, which wraps silently (kvcomp_encode.py:97); its model path
@@ -481,15 +486,15 @@ class KVCompCtx:
         self._sc.n += n_units
         self.compressed_ctx_len += T
         if n_enc:
-            if not self._encode_finish(part, stream_room, cap, words):
+            if not self._encode_finish(part, blocks, stream_room, cap, words):
                 # A symbol the frozen book has no code for.  The reference drops such symbols silently
                 # (kernels.cu:197-205: a table entry of length 0 adds no bits), which corrupts the stream.
                 # Here the book is rebuilt over everything stored so far plus every reachable code, and the
                 # cache is re-encoded once; this cannot happen again for this context.
                 self._rebook(part)
             self.encoded_ctx_len += n_enc
-        self._pending = pend[n_enc:].contiguous() if pend.shape[0] > n_enc else None
-        return codes.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim)
+        self._pending = pend[n_enc:].contiguous() if pend is not None and pend.shape[0] > n_enc else None
+        return None if codes is None else codes.view(-1, self.block_size, self.batch_size, self.head_num, self.head_dim)
 
     def _encode_room(self, codes):
         """Bytes to reserve for the stream of `codes` [T, B, H, D]: (a first guess, the most it can take)."""
@@ -508,8 +513,8 @@ class KVCompCtx:
                    self._ti.reserve(tsz // 2, self.device), self._enc.reserve(room, self.device),
                    base_offset=self._enc.n, total=report.total, status=report.enc_status)
 
-    def _encode_finish(self, codes, room, cap, words):
-        """The launched stream joins the arenas.  False if the book lacks a symbol."""
+    def _encode_finish(self, codes, blocks, room, cap, words):
+        """The launched stream of `blocks` blocks joins the arenas.  False if the book lacks a symbol."""
         if words[3] & ops._lib.FLAG_STREAM_FULL and room != cap:
             self.stream_retries = getattr(self, "stream_retries", 0) + 1
             report = ops.Report(self.device)
@@ -518,7 +523,6 @@ class KVCompCtx:
         if words[3] & ops._lib.FLAG_SYMBOL_MISSING:
             return False
         ops.check_flags(words[3], what="entropy_encode")
-        blocks = codes.numel() // 8192
         self._enc.n += words[0]
         self._bi.n += blocks * 8
         self._ti.n += blocks * 64
@@ -530,7 +534,7 @@ class KVCompCtx:
         room, cap = self._encode_room(codes)
         report = ops.Report(self.device)
         self._encode_launch(codes, room, report)
-        return self._encode_finish(codes, room, cap, report.read())
+        return self._encode_finish(codes, codes.numel() // 8192, room, cap, report.read())
 
     def _rebook(self, new_codes):
         old = None
