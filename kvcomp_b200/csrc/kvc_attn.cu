@@ -1585,6 +1585,11 @@ __device__ __forceinline__ uint4 ld_nc_128_pinned(const void *p) {
     asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
+__device__ __forceinline__ uint32_t ld_nc_32_pinned(const void *p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ unsigned short ld_nc_16_pinned(const void *p) {
     unsigned short v;
     asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
@@ -1605,8 +1610,13 @@ __device__ __forceinline__ unsigned short ld_nc_16_pinned(const void *p) {
 // The loads of the partial results are issued in batches of 16 before any is used as well, by both halves of the CTA in turn:
 // (2 columns of 32768 tokens, 2 heads each, 256 partial results: 32.5 us for the step with batches of 8 by one half, now 24.5).
 constexpr int MERGE_THREADS = 256;
-__global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *__restrict__ ws_part, __half *__restrict__ out, int splits, TailArgs t) {
-    __shared__ float sm_red[8], sm_sum[8], sm_e[128], sm_o[128];
+// PAIRS: the tail's rows of V start on 4 bytes (else on 2: a load per channel).  REGS: with 96 registers a CTA finds room beside three workers of the grouped kernel or four
+// with one head, with 128 it stays off their SM: which is better as long as the SMs without attention CTAs, two a piece, hold them all, as company slows the workers.  (10 columns of 5504 tokens and 128
+// rows, 3 heads, 140 attention CTAs and 30 of this kernel: 23.3 and 17.1 us; 12 of 2816 and 165, 6 heads, 132 and 72: 16.9 and 16.3; 32 of 1792 and 208, one head, 112 and 32: 14.0 and 15.0.)
+template <bool PAIRS, int REGS>
+__global__ void __maxnreg__(REGS) attn_merge_kernel(const float *__restrict__ ws_part, __half *__restrict__ out, int splits, TailArgs t) {
+    __shared__ float sm_red[8], sm_sum[8];
+    __shared__ __align__(16) float sm_e[128], sm_o[512];
     __shared__ __align__(16) float sm_q[128];
     constexpr int PART = ROWS_PART_FLOATS;
     const float *src = ws_part + (size_t)blockIdx.x * splits * PART;
@@ -1616,15 +1626,17 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
     // resident before the attention kernel has finished; its partial results are complete and visible after the wait
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (splits == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-    float m_t = -CUDART_INF_F, l_t = 0.f, o_t = 0.f;      // the tail's running maximum and sum; output of channel tid & 127 over the thread's rows
+    float m_t = -CUDART_INF_F, l_t = 0.f, o_t = 0.f;      // the tail's running maximum and sum; its output of channel tid (of the first 128 threads)
     if (t.Tr > 0) {
-        // q.k: two threads per row, 64 channels each; P.V: thread = (half of the pass's rows, channel)
-        const int row = tid >> 1, part = tid & 1, ch = tid & 127, rg = tid >> 7;
+        // q.k: two threads per row, 64 channels each; P.V: thread = (quarter of the pass's rows, two channels).  (With a channel and half of
+        // the rows it took 128 registers.)
+        const int row = tid >> 1, part = tid & 1, ch = (tid & 63) * 2, rg = tid >> 6;
         const long long b = blockIdx.x / t.Hq, h = (blockIdx.x % t.Hq) / (t.Hq / t.Hkv);
         const long long rstride = (long long)t.B * t.Hkv * 128;                 // halves between two rows of a column
         const __half *kcol = t.ktail + (b * t.Hkv + h) * 128 + part * 64, *vcol = t.vtail + (b * t.Hkv + h) * 128 + ch;
-        // Every load of a pass -- the query (first pass), the thread's half row of K, its 64 rows of V -- is issued
+        // Every load of a pass -- the query (first pass), the thread's half row of K, its 32 rows of V -- is issued
         // before the first of them is used: one trip to memory per pass instead of one per step of the softmax.
+        float o0 = 0.f, o1 = 0.f;                                             // the thread's two channels over its rows
         const unsigned short qbits = tid < 128 ? ld_nc_16_pinned(t.q + (size_t)blockIdx.x * 128 + tid) : (unsigned short)0;
         for (long long r0 = 0; r0 < t.Tr; r0 += 128) {                        // 128 rows per pass
             const int n_here = (int)min(128ll, t.Tr - r0);
@@ -1633,10 +1645,18 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
             const __half *kr = kcol + (r0 + min(row, n_here - 1)) * rstride;  // rows beyond the pass: read again, not used
 #pragma unroll
             for (int j = 0; j < 8; j++) kv[j] = ld_nc_128_pinned(kr + j * 8);
-            unsigned short vv[64];
+            uint32_t vv[32];
             const __half *vr = vcol + r0 * rstride;
+            if (PAIRS) {
 #pragma unroll
-            for (int k = 0; k < 64; k++) vv[k] = ld_nc_16_pinned(vr + min(rg * 64 + k, n_here - 1) * rstride);   // rows beyond the pass: weight 0
+                for (int k = 0; k < 32; k++) vv[k] = ld_nc_32_pinned(vr + min(rg * 32 + k, n_here - 1) * rstride);   // rows beyond the pass: weight 0
+            } else {
+#pragma unroll
+                for (int k = 0; k < 32; k++) {
+                    const __half *x = vr + min(rg * 32 + k, n_here - 1) * rstride;
+                    vv[k] = (uint32_t)ld_nc_16_pinned(x) | (uint32_t)ld_nc_16_pinned(x + 1) << 16;
+                }
+            }
             if (r0 == 0 && tid < 128) sm_q[tid] = __half2float(__ushort_as_half(qbits)) * t.scaling;
             __syncthreads();                                                  // sm_q is written; the pass before is done with sm_e
             float sc = -CUDART_INF_F;
@@ -1673,20 +1693,20 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_merge_kernel(const float *
             for (int w = 0; w < 8; w++) lsum += sm_sum[w];
             l_t = l_t * alpha + lsum;
             m_t = m_new;
-            float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;                     // rows rg * 64 .. + 63 of the pass, four sums
+            float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;                     // rows rg * 32 .. + 31 of the pass, two sums per channel
 #pragma unroll
-            for (int k = 0; k < 64; k += 4) {
-                d0 = fmaf(sm_e[rg * 64 + k], __half2float(__ushort_as_half(vv[k])), d0);
-                d1 = fmaf(sm_e[rg * 64 + k + 1], __half2float(__ushort_as_half(vv[k + 1])), d1);
-                d2 = fmaf(sm_e[rg * 64 + k + 2], __half2float(__ushort_as_half(vv[k + 2])), d2);
-                d3 = fmaf(sm_e[rg * 64 + k + 3], __half2float(__ushort_as_half(vv[k + 3])), d3);
+            for (int k = 0; k < 32; k += 2) {
+                const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&vv[k])), y = __half22float2(*reinterpret_cast<const __half2 *>(&vv[k + 1]));
+                const float2 e = *reinterpret_cast<const float2 *>(&sm_e[rg * 32 + k]);
+                d0 = fmaf(e.x, x.x, d0); d1 = fmaf(e.x, x.y, d1);
+                d2 = fmaf(e.y, y.x, d2); d3 = fmaf(e.y, y.y, d3);
             }
-            o_t = fmaf(o_t, alpha, (d0 + d1) + (d2 + d3));
+            o0 = fmaf(o0, alpha, d0 + d2); o1 = fmaf(o1, alpha, d1 + d3);
         }
         __syncthreads();                                                      // sm_red and sm_e serve the merge below
-        if (tid >= 128) sm_o[tid - 128] = o_t;                                // the second half of the rows joins the first
+        *reinterpret_cast<float2 *>(&sm_o[rg * 128 + ch]) = make_float2(o0, o1);
         __syncthreads();
-        if (tid < 128) o_t += sm_o[tid];
+        if (tid < 128) o_t = (sm_o[tid] + sm_o[128 + tid]) + (sm_o[256 + tid] + sm_o[384 + tid]);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int BATCH = 16;                             // partial results whose channel a thread loads at once, the CTA's two halves in turn
@@ -2030,6 +2050,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
     const bool bulk = T > 0 && (reinterpret_cast<uintptr_t>(k->encoded) & 15) == 0 && (reinterpret_cast<uintptr_t>(v->encoded) & 15) == 0;
     const int sms = kvc_sm_count();
     const long long Gt = Hq / Hkv;
+    long long attn_ctas = 0;
     if (T > 0) {
         // The kernels count in steps of 128 tokens.  The workspace, sized for `splits` runs of 256-token tiles, holds twice as many
         // of their partial results: with many small workers the items are finer where it may be so.
@@ -2088,6 +2109,7 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         KVC_REQUIRE(occ >= 1, "kvc_attn_decode: %zu bytes of shared memory do not fit an SM", smem);             \
         long long ctas = p.team ? p.work : (p.work + workers - 1) / workers;                                    \
         if (ctas > sms) ctas = sms;                                                                             \
+        attn_ctas = ctas;                                                                                       \
         if (int rc = launch_overlapped(kernel, dim3((unsigned)ctas), dim3(threads), smem, kvc_cu(stream), p)) return rc; \
     }
             if (p.nh > 4) KVC_AT(8) else if (p.nh > 2) KVC_AT(4) else if (p.nh > 1) KVC_AT(2) else KVC_AT(1)
@@ -2100,7 +2122,9 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
             ta.q = p.q; ta.ktail = p.ktail; ta.vtail = p.vtail; ta.Tr = Tr;
             ta.B = (int)B; ta.Hkv = (int)Hkv; ta.Hq = (int)Hq; ta.scaling = scaling;
         }
-        if (int rc = launch_overlapped(attn_merge_kernel, dim3((unsigned)(B * Hq)), dim3(MERGE_THREADS), 0, kvc_cu(stream),
+        const bool pairs = (reinterpret_cast<uintptr_t>(ta.vtail) & 3) == 0, apart = B * Hq <= 2 * (sms - attn_ctas);
+        auto *merge = apart ? (pairs ? attn_merge_kernel<true, 128> : attn_merge_kernel<false, 128>) : (pairs ? attn_merge_kernel<true, 96> : attn_merge_kernel<false, 96>);
+        if (int rc = launch_overlapped(merge, dim3((unsigned)(B * Hq)), dim3(MERGE_THREADS), 0, kvc_cu(stream),
                                        (const float *)p.ws_part, p.out, T > 0 ? splits : 0, ta)) return rc;
     }
     KVC_LAUNCH_OK();

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 # launches of one round and of several, with one head and with groups; more heads than one launch takes; tails below and beyond a pass of 128 rows, and none
 @pytest.mark.parametrize("T,B,Hkv,G,Tr", [(1024, 1, 32, 1, 100), (4096, 3, 32, 1, 130), (896, 2, 8, 4, 128), (2816, 3, 4, 6, 165), (4096, 8, 8, 4, 40),
-                                          (640, 2, 3, 17, 129), (256, 1, 1, 2, 1), (16384, 1, 2, 8, 30), (1024, 2, 8, 2, 0)])
+                                          (640, 2, 3, 17, 129), (256, 1, 1, 2, 1), (16384, 1, 2, 8, 30), (1024, 2, 8, 2, 0),
+                                          (5504, 2, 5, 3, 128), (3200, 2, 10, 4, 150)])         # (the merge kernel beside three or more workers)
 def test_steps_without_a_wait(ops, T, B, Hkv, G, Tr):  # noqa: F811
     g = torch.Generator(device="cuda").manual_seed(T + G)
     kc, _, keep_k = _cache(ops, torch.randn(T, B, Hkv, 128, device="cuda", generator=g).half(), True, 0.05)
@@ -42,3 +43,20 @@ def test_steps_without_a_wait(ops, T, B, Hkv, G, Tr):  # noqa: F811
         assert torch.equal(run(False), want)
     assert ops.read_status(st) == 0
     assert torch.equal(want[0::2], want[1::2]) and not torch.equal(want[0], want[2])
+
+
+@pytest.mark.parametrize("T,B,Hkv,G,Tr", [(1024, 1, 32, 1, 100), (5504, 2, 5, 3, 129), (0, 3, 4, 2, 300)])
+def test_values_that_start_on_two_bytes(ops, T, B, Hkv, G, Tr):  # noqa: F811
+    """The tail's values by 4-byte and by 2-byte loads, in launches with room beside the attention kernel's CTAs and without: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(T + G)
+    kc = vc = None
+    if T:
+        kc, _, keep_k = _cache(ops, torch.randn(T, B, Hkv, 128, device="cuda", generator=g).half(), True, 0.05)
+        vc, _, keep_v = _cache(ops, torch.randn(T, B, Hkv, 128, device="cuda", generator=g).half(), False, 0.1)
+    q = torch.randn(B, Hkv * G, 128, device="cuda", generator=g).half()
+    kt, vt = (torch.randn(Tr, B, Hkv, 128, device="cuda", generator=g).half() for _ in range(2))
+    odd = torch.empty(vt.numel() + 1, dtype=torch.float16, device="cuda")[1:].view(vt.shape)
+    odd.copy_(vt)
+    assert odd.data_ptr() % 4 == 2
+    outs = [ops.attn_decode(kc, vc, T, B, Hkv, q, 0.1, kt, v)[0] for v in (vt, odd)]
+    assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all())
