@@ -1611,7 +1611,7 @@ __device__ __forceinline__ unsigned short ld_nc_16_pinned(const void *p) {
 // (2 columns of 32768 tokens, 2 heads each, 256 partial results: 32.5 us for the step with batches of 8 by one half, now 24.5).
 constexpr int MERGE_THREADS = 256;
 // PAIRS: the tail's rows of V start on 4 bytes (else on 2: a load per channel).  REGS: with 96 registers a CTA finds room beside three workers of the grouped kernel or four
-// with one head, with 128 it stays off their SM: which is better as long as the SMs without attention CTAs, two a piece, hold them all, as company slows the workers.  (10 columns of 5504 tokens and 128
+// with one head, with 128 it stays off their SM: which is better as long as the SMs without attention CTAs, two a piece, hold them all, as company slows the workers.  (10 columns of 5376 tokens and 152
 // rows, 3 heads, 140 attention CTAs and 30 of this kernel: 23.3 and 17.1 us; 12 of 2816 and 165, 6 heads, 132 and 72: 16.9 and 16.3; 32 of 1792 and 208, one head, 112 and 32: 14.0 and 15.0.)
 template <bool PAIRS, int REGS>
 __global__ void __maxnreg__(REGS) attn_merge_kernel(const float *__restrict__ ws_part, __half *__restrict__ out, int splits, TailArgs t) {
