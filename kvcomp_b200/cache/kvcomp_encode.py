@@ -355,8 +355,7 @@ class KVCompCtx:
         if cos is not None and (cos.data_ptr() | sin.data_ptr()) % 16:
             return self._begin(ops.rope_store(x, cos, sin))
         self._check(x.permute(2, 0, 1, 3))
-        self.ctx_len += t
-        return self._launch(x, n, 0, t - n, t, None, cos, sin, stride, keep_codes)
+        return self._launch(x, n, 0, t - n, t, t, None, cos, sin, stride, keep_codes)
 
     def store(self, cache):
         """Append tokens [t, B, H, D]; whole blocks beyond the recent window are quantised and encoded.
@@ -365,11 +364,11 @@ class KVCompCtx:
 
     def _begin(self, cache):
         self._check(cache)
-        self.ctx_len += cache.shape[0]
         live, t = len(self._recent), cache.shape[0]
         n = self._cut(live, t)
         if n == 0:
             self._recent.append(cache, self._room())          # the usual decode step: the new rows, nothing else moves
+            self.ctx_len += t
             return None
         if live == 0:
             x, rest = cache[:n].contiguous(), cache[n:]       # a prefill: compressed from where it lies
@@ -377,19 +376,19 @@ class KVCompCtx:
             x, rest = self._recent.view()[:n].clone(), cache  # the window's front
         else:
             x, rest = torch.cat([self._recent.view(), cache[:n - live]], dim=0), cache[n - live:]
-        return self._launch(x, n, live, rest.shape[0], 0, lambda place: place.copy_(rest))
+        return self._launch(x, n, live, rest.shape[0], t, 0, lambda place: place.copy_(rest))
 
-    def _launch(self, x, n, live, n_rest, x_tokens, put_rest, cos=None, sin=None, stride=0, keep_codes=True):
-        """Launch the compression of the first n tokens of (the `live` rows of the window + new tokens): x as rows, or (x_tokens > 0) as a
-        prompt's heads.  put_rest(place) writes the n_rest last of the new tokens as rows; the heads' own are written by the call."""
+    def _launch(self, x, n, live, n_rest, t, x_tokens, put_rest, cos=None, sin=None, stride=0, keep_codes=True):
+        """Launch the compression of the first n tokens of (the `live` rows of the window + t new tokens): x as rows, or (x_tokens > 0) as a
+        prompt's heads.  put_rest(place) writes the n_rest last of the new tokens as rows; the heads' own are written by the call.
+        The context has a book, and counts the tokens, once everything is launched: until then any step here may fail (an allocation)."""
         # quantise, book, encode and the rows are launched by one call; one copy brings back what the kernels report
         # (a prompt of 333 tokens, K and V: a call, a wait and a copy for each kernel 637 us, one report per tensor 409;
         # one call per tensor and one wait for both 261)
         shape, T, dev = (self.batch_size, self.head_num, self.head_dim), n, self.device
         B, H, D = shape
         mode, build = _MODE[self.quant_mode], self.book is None
-        if build:
-            self.book = ops.new_book(dev)
+        book = ops.new_book(dev) if build else self.book
         old = 0 if self._pending is None else self._pending.shape[0]
         pend = torch.empty((old + n,) + shape, dtype=torch.uint8, device=dev)
         if old:
@@ -428,16 +427,16 @@ class KVCompCtx:
         try:
             ops.store_at(dev, (x.data_ptr(), 0 if cos is None else cos.data_ptr(), 0 if sin is None else sin.data_ptr(), stride, B, H, x_tokens, n, D, self.block_size,
                                pend.data_ptr() + old * (B * H * D), self._mi.address(n_units, dev), self._sc.address(n_units, dev), scratch.data_ptr(), scratch.numel(),
-                               self.book.blob.data_ptr(), pend.data_ptr(), n_enc, self._enc.n, self._bi.address(blocks * 8, dev), self._ti.address(blocks * 64, dev),
+                               book.blob.data_ptr(), pend.data_ptr(), n_enc, self._enc.n, self._bi.address(blocks * 8, dev), self._ti.address(blocks * 64, dev),
                                self._enc.address(stream_room, dev), stream_room, at_rest, n_rest if x_tokens and over else 0, at_kept, k, report, 0),
                          (mode, self.batch_shared, x_tokens > 0, self.is_k, build, self._mi.size), self.quant_scale_rel)
             if over and n_rest and not x_tokens:
                 put_rest(buf[n_old + k:n_old + k + n_rest])
         except BaseException:                                 # nothing that is on its way may arrive in the place later
-            if build:
-                self.book = None
             ops.wait(dev)
             raise
+        self.book = book
+        self.ctx_len += t
         # A book built from these very codes lacks none of them and the room is for the longest stream: with all of them in the stream and the kept rows
         # written, nothing reads the codes again.  (Keys' and values' on their way together would else be held at the same time.)
         if not keep_codes and build and over and n_enc == old + n:

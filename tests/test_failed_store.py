@@ -1,0 +1,106 @@
+"""A store that cannot be begun, an allocation having failed, leaves the context as it was."""
+import pytest
+import torch
+
+from kvcomp_b200 import ops
+from kvcomp_b200.cache import kvcomp_encode
+from kvcomp_b200.cache.kvcomp_encode import KVCompCtx
+from kvcomp_b200.utils.compute import QuantMode
+from kvcomp_b200.utils.config import KVCompCacheConfig, KVCompCacheConfigStatic
+
+B, H, D = 2, 3, 128
+
+
+@pytest.fixture(autouse=True)
+def _config():
+    KVCompCacheConfigStatic.config = KVCompCacheConfig("synthetic", QuantMode("ChannelQuant"), QuantMode("TokenQuant"), 64, 64, 32, 32, 0.05, 0.1)
+    yield
+    KVCompCacheConfigStatic.config = None
+
+
+class _Failing:
+    """torch.empty whose call number `at` finds no memory."""
+
+    def __init__(self, at):
+        self.at, self.seen, self.real = at, 0, torch.empty
+
+    def __call__(self, *a, **kw):
+        self.seen += 1
+        if self.seen - 1 == self.at:
+            raise torch.cuda.OutOfMemoryError("no memory left")
+        return self.real(*a, **kw)
+
+
+def _untouched(ctx):
+    return ctx.book is None and (ctx.ctx_len, ctx.compressed_ctx_len, ctx.encoded_ctx_len, len(ctx._recent), ctx._enc.n, ctx._mi.n) == (0,) * 6
+
+
+def _each_failure(store):
+    """store(at) with the allocations failing one after the other; returns at how many places."""
+    at = 0
+    while store(at):
+        at += 1
+    assert at >= 5
+    return at
+
+
+@pytest.mark.parametrize("is_k", [True, False])
+def test_the_next_store_builds_the_book(monkeypatch, is_k):
+    """The calls that reach the device, on the CPU: the book's blob is given back, and the retry asks for a book."""
+    builds = []
+    monkeypatch.setattr(ops, "_cuda", lambda t, dtype, name: t)
+    monkeypatch.setattr(ops, "wait", lambda device: None)
+    monkeypatch.setattr(ops.Reports, "place", staticmethod(lambda: (0, 0)))
+    monkeypatch.setattr(ops, "store_at", lambda device, words, ints, rel, n_entries=0: builds.append(ints[4]))
+
+    def store(at):
+        ctx, x = KVCompCtx(is_k, B, H, D, 0.05, keep_dequantised=True), torch.zeros(200, B, H, D, dtype=torch.float16)
+        failing = _Failing(at)
+        with monkeypatch.context() as m:
+            m.setattr(kvcomp_encode.torch, "empty", failing)
+            try:
+                ctx._begin(x)
+            except torch.cuda.OutOfMemoryError:
+                pass
+        failed = failing.seen > at
+        if failed:
+            assert _untouched(ctx), "after allocation %d" % at
+            del builds[:]
+            ctx._begin(x)
+        assert builds == [True] and ctx.ctx_len == 200 and ctx.book is not None
+        del builds[:]
+        return failed
+    _each_failure(store)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [True, False])
+def test_a_retry_stores_what_a_first_call_would(monkeypatch, heads):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(B, H, 300, D, device="cuda", generator=g).half()
+    rows = x.permute(2, 0, 1, 3).contiguous()
+
+    def state(ctx):
+        return [ctx.ctx_len, ctx._enc.n, ctx.max_block_bytes] + \
+            [t.cpu() for t in (ctx.encoded_data, ctx.block_infos, ctx.thread_infos, ctx.quant_min_ints, ctx.quant_scales, ctx.buffer, ctx.get()[0])]
+
+    def call(ctx):
+        return ctx.store_heads(x) if heads else ctx.store(rows)
+    fresh = KVCompCtx(True, B, H, D, 0.05, batch_shared=False, keep_dequantised=True)
+    call(fresh)
+    want = state(fresh)
+
+    def store(at):
+        ctx, failing = KVCompCtx(True, B, H, D, 0.05, batch_shared=False, keep_dequantised=True), _Failing(at)
+        with monkeypatch.context() as m:
+            m.setattr(kvcomp_encode.torch, "empty", failing)
+            try:
+                call(ctx)
+            except torch.cuda.OutOfMemoryError:
+                pass
+        if failing.seen > at:
+            assert _untouched(ctx), "after allocation %d" % at
+            call(ctx)
+        assert all(torch.equal(a, b) if isinstance(a, torch.Tensor) else a == b for a, b in zip(state(ctx), want))
+        return failing.seen > at
+    _each_failure(store)
