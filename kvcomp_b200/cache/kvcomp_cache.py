@@ -128,7 +128,9 @@ class KVCompCache(_BASE):
         """Finish the store of keys that has begun; True if the values' store went with it, behind one wait for both."""
         both, v_begun = False, None
         try:
-            if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and vc.recent_place(values.shape[2], values.device) is None:
+            # (one wait is for one device)
+            if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and values.device == kc.device \
+                    and vc.recent_place(values.shape[2], values.device) is None:
                 v_begun = vc.begin_heads(values, keep_codes=False)
                 both = True
         finally:

@@ -1,9 +1,12 @@
-"""A store that cannot be begun, an allocation having failed, leaves the context as it was."""
+"""Stores that fail, in part or as a whole, and stores that wait together."""
+import types
+
 import pytest
 import torch
 
-from kvcomp_b200 import ops
+from kvcomp_b200 import _lib, ops
 from kvcomp_b200.cache import kvcomp_encode
+from kvcomp_b200.cache.kvcomp_cache import KVCompCache
 from kvcomp_b200.cache.kvcomp_encode import KVCompCtx
 from kvcomp_b200.utils.compute import QuantMode
 from kvcomp_b200.utils.config import KVCompCacheConfig, KVCompCacheConfigStatic
@@ -44,14 +47,23 @@ def _each_failure(store):
     return at
 
 
-@pytest.mark.parametrize("is_k", [True, False])
-def test_the_next_store_builds_the_book(monkeypatch, is_k):
-    """The calls that reach the device, on the CPU: the book's blob is given back, and the retry asks for a book."""
-    builds = []
+@pytest.fixture
+def on_cpu(monkeypatch):
+    """The calls that reach the device, on the CPU; returns what a test may set and look at."""
+    d = types.SimpleNamespace(waits=[], builds=[], flags=0)
     monkeypatch.setattr(ops, "_cuda", lambda t, dtype, name: t)
-    monkeypatch.setattr(ops, "wait", lambda device: None)
+    monkeypatch.setattr(ops, "wait", lambda device: d.waits.append(device))
     monkeypatch.setattr(ops.Reports, "place", staticmethod(lambda: (0, 0)))
-    monkeypatch.setattr(ops, "store_at", lambda device, words, ints, rel, n_entries=0: builds.append(ints[4]))
+    monkeypatch.setattr(ops.Reports, "read", staticmethod(lambda i: [1000, 500, d.flags, 0]))
+    monkeypatch.setattr(ops, "store_at", lambda device, words, ints, rel, n_entries=0: d.builds.append(ints[4]))
+    monkeypatch.setattr(ops, "rope_store", lambda x, cos, sin, out=None, first=0: x.permute(2, 0, 1, 3).contiguous())
+    monkeypatch.setattr(KVCompCache, "_plain", staticmethod(lambda x: True))
+    return d
+
+
+@pytest.mark.parametrize("is_k", [True, False])
+def test_the_next_store_builds_the_book(monkeypatch, on_cpu, is_k):
+    builds = on_cpu.builds
 
     def store(at):
         ctx, x = KVCompCtx(is_k, B, H, D, 0.05, keep_dequantised=True), torch.zeros(200, B, H, D, dtype=torch.float16)
@@ -71,6 +83,16 @@ def test_the_next_store_builds_the_book(monkeypatch, is_k):
         del builds[:]
         return failed
     _each_failure(store)
+
+
+def test_values_of_another_device_are_waited_for(on_cpu):
+    """One wait is for one device: elsewhere the values' store is a call of its own."""
+    x = torch.zeros(B, H, 200, D, dtype=torch.float16)
+    for values in (x.to("meta"), x):
+        kc, vc = KVCompCtx(True, B, H, D, 0.05, keep_dequantised=True), KVCompCtx(False, B, H, D, 0.1, keep_dequantised=True)
+        del on_cpu.waits[:]
+        both = KVCompCache._values_begun(kc, vc, kc.begin_heads(x, keep_codes=False), values)
+        assert both == (values is x) and (kc.ctx_len, vc.ctx_len) == (200, 200 if both else 0) and on_cpu.waits == [x.device]
 
 
 @pytest.mark.gpu
