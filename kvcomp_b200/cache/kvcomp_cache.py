@@ -126,23 +126,18 @@ class KVCompCache(_BASE):
     @staticmethod
     def _values_begun(kc, vc, begun, values):
         """Finish the store of keys that has begun; True if the values' store went with it, behind one wait for both."""
-        both, v_begun = False, None
+        v_begun = None
         try:
             # (one wait is for one device)
             if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and values.device == kc.device \
                     and vc.recent_place(values.shape[2], values.device) is None:
                 v_begun = vc.begin_heads(values, keep_codes=False)
-                both = True
         finally:
-            try:
-                kc._finish(begun)                               # (waits for both)
-            except BaseException:
-                if both:                                        # as if the values had not come yet
-                    vc._abandon(v_begun, values.shape[2])
-                raise
-        if both:
-            vc._finish(v_begun, waited=True)
-        return both
+            kc._finish(begun)                                   # waits for both; the values do not count where the keys are refused
+        if v_begun is None:
+            return False
+        vc._finish(v_begun, waited=True)
+        return True
 
     def update(self, key_states, value_states, layer_idx, cache_kwargs=None):
         """The reference's Cache.update: append, then return the whole K and V as [B, Hkv, T, D]."""

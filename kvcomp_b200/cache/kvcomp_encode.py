@@ -11,6 +11,8 @@ Tokens are quantised in whole blocks of the configured block size, exactly where
 block size is not a multiple of 128 (the reference's CUDA path forbids that, kvcomp_encode.py:52-54; its
 model path allows it), up to 127 quantised tokens wait as plain codes for their vector to fill.
 """
+from typing import NamedTuple
+
 import torch
 
 from .. import ops
@@ -160,6 +162,28 @@ class _RecentRows:
 
     def set(self, rows):
         self.buf, self.q, self.lo, self.hi = rows, 0, 0, (0 if rows is None else rows.shape[0])
+
+
+class _Begun(NamedTuple):
+    """A store that is on its way: what _finish needs of _launch."""
+    slot: int                # of ops.Reports
+    book: object             # the book that it encodes with, built by it where the context has none
+    pend: object             # codes: `old` rows that waited for their block, then the new ones; None: nobody needs them
+    old: int
+    part: object             # those of pend that are encoded, n_enc rows
+    n_enc: int
+    stream_room: int         # bytes for the stream, and the most that it can take
+    cap: int
+    n_units: int
+    n: int                   # tokens that are compressed
+    t: int                   # new tokens
+    over: bool               # the window starts over in buf: n_old kept rows, k more, n_rest recent ones
+    k: int
+    n_old: int
+    buf: object
+    n_rest: int
+    put_rest: object
+    blocks: int              # of the stream
 
 
 class KVCompCtx:
@@ -381,11 +405,11 @@ class KVCompCtx:
     def _launch(self, x, n, live, n_rest, t, x_tokens, put_rest, cos=None, sin=None, stride=0, keep_codes=True):
         """Launch the compression of the first n tokens of (the `live` rows of the window + t new tokens): x as rows, or (x_tokens > 0) as a
         prompt's heads.  put_rest(place) writes the n_rest last of the new tokens as rows; the heads' own are written by the call.
-        The context has a book, and counts the tokens, once everything is launched: until then any step here may fail (an allocation)."""
+        Nothing counts before _finish: any step here may fail (an allocation), and the device may refuse the tokens."""
         # quantise, book, encode and the rows are launched by one call; one copy brings back what the kernels report
         # (a prompt of 333 tokens, K and V: a call, a wait and a copy for each kernel 637 us, one report per tensor 409;
         # one call per tensor and one wait for both 261)
-        shape, T, dev = (self.batch_size, self.head_num, self.head_dim), n, self.device
+        shape, dev = (self.batch_size, self.head_num, self.head_dim), self.device
         B, H, D = shape
         mode, build = _MODE[self.quant_mode], self.book is None
         book = ops.new_book(dev) if build else self.book
@@ -435,28 +459,21 @@ class KVCompCtx:
         except BaseException:                                 # nothing that is on its way may arrive in the place later
             ops.wait(dev)
             raise
-        self.book = book
-        self.ctx_len += t
         # A book built from these very codes lacks none of them and the room is for the longest stream: with all of them in the stream and the kept rows
         # written, nothing reads the codes again.  (Keys' and values' on their way together would else be held at the same time.)
         if not keep_codes and build and over and n_enc == old + n:
             pend = part = None
-        return slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest, build, blocks
-
-    def _abandon(self, begun, t):
-        """A begun store of t tokens, waited for, is not to count."""
-        self.ctx_len -= t
-        if begun is not None and begun[15]:
-            self.book = None
+        return _Begun(slot, book, pend, old, part, n_enc, stream_room, cap, n_units, n, t, over, k, n_old, buf, n_rest, put_rest, blocks)
 
     def _finish(self, begun, waited=False):
-        """The rest of a begun store: waits for it (waited: the caller has), then it counts."""
+        """The rest of a begun store: waits for it (waited: the caller has), then it counts.  A store that the device refuses does not
+        count: the context is as it was, its book too."""
         if begun is None:
             return None
-        slot, pend, old, part, n_enc, stream_room, cap, n_units, T, over, k, n_old, buf, n_rest, put_rest, _, blocks = begun
+        slot, book, pend, old, part, n_enc, stream_room, cap, n_units, n, t, over, k, n_old, buf, n_rest, put_rest, blocks = begun
         if not waited:
             ops.wait(self.device)
-        words, room, n, codes = ops.Reports.read(slot), self._room(), T, pend[old:] if old and pend is not None else pend
+        words, room, codes = ops.Reports.read(slot), self._room(), pend[old:] if old and pend is not None else pend
         flags = ops.check_flags(words[2], what="quantize")
         if flags & ops._lib.FLAG_MIN_OVERFLOW:
             # int8 is the reference's CUDA path, which wraps silently (kvcomp_encode.py:97); its model path
@@ -465,6 +482,10 @@ class KVCompCtx:
                 raise KvcError("a min_int does not fit 16 bits: the data lies too far from zero for its range")
             import warnings
             warnings.warn("a min_int wrapped in int8 as in the reference's CUDA path; set wide_min_ints to keep it")
+        if n_enc and not words[3] & (ops._lib.FLAG_SYMBOL_MISSING | (ops._lib.FLAG_STREAM_FULL if stream_room != cap else 0)):
+            ops.check_flags(words[3], what="entropy_encode")  # (the two are seen to below)
+        self.book = book
+        self.ctx_len += t
         # the window: the compressed rows leave it, or stay as dequantised rows for a reader of the rows behind
         # the fused kernel's range (tail_from); the rest of the new tokens joins the recent rows
         if not over:
@@ -483,7 +504,7 @@ class KVCompCtx:
             self._recent.restart(n_old, k, n_rest, buf)
         self._mi.n += n_units
         self._sc.n += n_units
-        self.compressed_ctx_len += T
+        self.compressed_ctx_len += n
         if n_enc:
             if not self._encode_finish(part, blocks, stream_room, cap, words):
                 # A symbol the frozen book has no code for.  The reference drops such symbols silently

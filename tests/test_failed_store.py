@@ -50,11 +50,11 @@ def _each_failure(store):
 @pytest.fixture
 def on_cpu(monkeypatch):
     """The calls that reach the device, on the CPU; returns what a test may set and look at."""
-    d = types.SimpleNamespace(waits=[], builds=[], flags=0)
+    d = types.SimpleNamespace(waits=[], builds=[], flags=(0, 0))
     monkeypatch.setattr(ops, "_cuda", lambda t, dtype, name: t)
     monkeypatch.setattr(ops, "wait", lambda device: d.waits.append(device))
     monkeypatch.setattr(ops.Reports, "place", staticmethod(lambda: (0, 0)))
-    monkeypatch.setattr(ops.Reports, "read", staticmethod(lambda i: [1000, 500, d.flags, 0]))
+    monkeypatch.setattr(ops.Reports, "read", staticmethod(lambda i: [1000, 500, *d.flags]))
     monkeypatch.setattr(ops, "store_at", lambda device, words, ints, rel, n_entries=0: d.builds.append(ints[4]))
     monkeypatch.setattr(ops, "rope_store", lambda x, cos, sin, out=None, first=0: x.permute(2, 0, 1, 3).contiguous())
     monkeypatch.setattr(KVCompCache, "_plain", staticmethod(lambda x: True))
@@ -71,14 +71,14 @@ def test_the_next_store_builds_the_book(monkeypatch, on_cpu, is_k):
         with monkeypatch.context() as m:
             m.setattr(kvcomp_encode.torch, "empty", failing)
             try:
-                ctx._begin(x)
+                ctx.store(x)
             except torch.cuda.OutOfMemoryError:
                 pass
         failed = failing.seen > at
         if failed:
             assert _untouched(ctx), "after allocation %d" % at
             del builds[:]
-            ctx._begin(x)
+            ctx.store(x)
         assert builds == [True] and ctx.ctx_len == 200 and ctx.book is not None
         del builds[:]
         return failed
@@ -93,6 +93,25 @@ def test_values_of_another_device_are_waited_for(on_cpu):
         del on_cpu.waits[:]
         both = KVCompCache._values_begun(kc, vc, kc.begin_heads(x, keep_codes=False), values)
         assert both == (values is x) and (kc.ctx_len, vc.ctx_len) == (200, 200 if both else 0) and on_cpu.waits == [x.device]
+
+
+@pytest.mark.parametrize("flags", [(_lib.FLAG_CODE_OVERFLOW, 0), (_lib.FLAG_MIN_OVERFLOW, 0), (0, _lib.FLAG_BLOCK_LONG)])
+def test_refused_keys_do_not_count(on_cpu, flags):
+    """Neither they nor the values that were on their way with them; the next prompt's books are its own."""
+    x = torch.zeros(B, H, 200, D, dtype=torch.float16)
+    kc, vc = (KVCompCtx(is_k, B, H, D, 0.05, min_dtype=torch.int16, keep_dequantised=True) for is_k in (True, False))
+    on_cpu.flags = flags
+    with pytest.raises(_lib.KvcError):
+        KVCompCache._values_begun(kc, vc, kc.begin_heads(x, keep_codes=False), x)
+    assert _untouched(kc) and _untouched(vc) and on_cpu.builds == [True, True]
+    on_cpu.flags = (0, 0)
+    assert KVCompCache._values_begun(kc, vc, kc.begin_heads(x, keep_codes=False), x)
+    assert on_cpu.builds == [True] * 4 and (kc.ctx_len, vc.ctx_len) == (200, 200)
+    book = kc.book
+    on_cpu.flags = flags                                     # a later store: what is there stays
+    with pytest.raises(_lib.KvcError):
+        kc.store(x.permute(2, 0, 1, 3).contiguous())
+    assert kc.book is book and (kc.ctx_len, kc.compressed_ctx_len, kc.encoded_ctx_len) == (200, 192, 192) and on_cpu.builds[4:] == [False]
 
 
 @pytest.mark.gpu
@@ -126,3 +145,21 @@ def test_a_retry_stores_what_a_first_call_would(monkeypatch, heads):
         assert all(torch.equal(a, b) if isinstance(a, torch.Tensor) else a == b for a, b in zip(state(ctx), want))
         return failing.seen > at
     _each_failure(store)
+
+
+@pytest.mark.gpu
+def test_a_layer_whose_keys_were_refused_takes_the_next_prompt():
+    g = torch.Generator(device="cuda").manual_seed(6)
+    k, v = (torch.randn(B, H, 300, D, device="cuda", generator=g).half() for _ in range(2))
+    rot = {n: torch.full((1, 300, D), x, dtype=torch.float16, device="cuda") for n, x in (("cos", 1.0), ("sin", 0.0))}
+    bad = k.clone()
+    bad[1, 2, :, 5] = float("nan")
+    cache = KVCompCache(B, H, D, 2)
+    with pytest.raises(_lib.KvcError):
+        cache.append(bad, v, 0, rot)
+    for layer in range(2):
+        cache.append(k, v, layer, rot)
+    for a, b in zip((cache.k_ctx[0], cache.v_ctx[0]), (cache.k_ctx[1], cache.v_ctx[1])):
+        assert a.ctx_len == b.ctx_len == 300
+        for x, y in zip(*((c.encoded_data, c.block_infos, c.thread_infos, c.quant_min_ints, c.quant_scales, c.buffer, c.get()[0]) for c in (a, b))):
+            assert torch.equal(x, y)
