@@ -32,6 +32,8 @@ extern "C" int kvc_store_packed(const kvc_store_args *args, kvc_stream_t stream)
     KVC_REQUIRE((reinterpret_cast<uintptr_t>(a.scratch) & 15) == 0 && a.scratch_bytes >= kvc_store_scratch(a.mode, a.batch_shared, a.T, a.B, a.H, a.block, a.enc_T, a.is_k),
                 "kvc_store_packed: scratch must be 16-byte aligned and hold what kvc_store_scratch says");
     KVC_REQUIRE(a.kept_rows >= 0 && a.kept_rows <= a.T && a.rest_rows >= 0, "kvc_store_packed: bad row counts");
+    KVC_REQUIRE(a.enc_T <= 0 || (a.base_offset >= 0 && a.base_offset <= 0xffffffffll),
+                "kvc_store_packed: a block's offset has 32 bits, the stream begins at %lld", (long long)a.base_offset);
     uint8_t *const scratch = reinterpret_cast<uint8_t *>(a.scratch);
     unsigned long long *const total = reinterpret_cast<unsigned long long *>(scratch);
     int32_t *const quant_status = reinterpret_cast<int32_t *>(scratch + 16), *const enc_status = reinterpret_cast<int32_t *>(scratch + 24);

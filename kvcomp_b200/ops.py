@@ -481,7 +481,7 @@ def encode(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset
     of this call, [1] the largest block byte count (a running maximum when `total` is passed in again).
     enc_table: device uint8 tensor of {u32 code, u32 length} entries indexed by symbol."""
     lib = _lib.load()
-    T, cols = _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded)
+    T, cols = _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset)
     dev = codes.device
     status = new_status(dev) if status is None else status
     total = torch.zeros(2, dtype=torch.int64, device=dev) if total is None else total
@@ -493,7 +493,7 @@ def encode(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset
     return total, status
 
 
-def _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded):
+def _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset):
     """Raise unless the encoder can take these; returns (T, sequences x heads)."""
     _cuda(codes, torch.uint8, "codes")
     T, B, H, D = codes.shape
@@ -507,12 +507,14 @@ def _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded):
     if block_info.numel() * block_info.element_size() < nblk * 8 or \
             thread_info.numel() * thread_info.element_size() < nblk * 128:
         raise KvcError("block_infos / thread_infos too small for %d blocks" % nblk)
+    if not 0 <= int(base_offset) < 1 << 32:
+        raise KvcError("a block's offset has 32 bits, the stream begins at %d" % int(base_offset))
     return T, cols
 
 
 def encode_now(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset):
     """encode() and a wait; returns (bytes, largest block, 0, status)."""
-    T, cols = _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded)
+    T, cols = _encode_checks(codes, is_k, enc_table, block_info, thread_info, encoded, base_offset)
     dev = codes.device
     scratch = torch.empty(_lib.load().kvc_store_scratch(0, 1, 0, 1, cols, 64, T, int(is_k)), dtype=torch.uint8, device=dev)
     slot, report = Reports.place()
