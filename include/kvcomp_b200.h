@@ -225,7 +225,7 @@ int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_k,
  * built from their codes, the first enc_T tokens of enc_codes are encoded (they may start before `codes`: codes that waited for their block),
  * and scratch's first four words -- bytes of the stream, its largest block, the quantiser's and the encoder's status -- are copied to
  * `report` (pinned host memory), which holds them once the stream has come that far.  rest_rows > 0 (heads only): the tokens behind the first T as rows
- * (kvc_rope_store_rows); kept_rows > 0: the last of the T tokens dequantised (kvc_dequant).  The encoder's total starts at 0 with every call.
+ * (kvc_rope_store_rows), no more than x has; kept_rows > 0: the last of the T tokens, whole units of them, dequantised (kvc_dequant).  The encoder's total starts at 0 with every call.
  * T = 0: codes that the caller has are encoded, nothing else.  base_offset: below 2^32, as the recorded block offsets are. */
 typedef struct {
     const void *x, *cos_, *sin_;

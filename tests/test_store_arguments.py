@@ -27,6 +27,14 @@ def test_offsets_beyond_32_bits(offset):
     assert "32 bits" in _refusal(base_offset=offset)
 
 
+@pytest.mark.parametrize("change, words", [
+    (dict(rest_rows=73), "73 rows behind"), (dict(rest_rows=-1), "row counts"), (dict(heads=0), "72 rows behind"), (dict(rest=0), "72 rows behind"),
+    (dict(kept_rows=129), "row counts"), (dict(kept_rows=-64), "row counts"), (dict(kept_rows=32), "whole units"), (dict(kept=0), "whole units"),
+    (dict(T=0, build=0, kept_rows=0), "rows behind"), (dict(T=0, rest_rows=0, kept_rows=0), "nothing to build"), (dict(enc_T=-64), "bad shape")])
+def test_rows_that_the_call_cannot_write(change, words):
+    assert words in _refusal(**change)
+
+
 @pytest.mark.parametrize("offset", [1 << 32, -1])
 def test_the_encoders_refuse_them_too(monkeypatch, offset):
     monkeypatch.setattr(ops, "_cuda", lambda t, dtype, name: t)
