@@ -657,8 +657,10 @@ class KVCompCtx:
         assert self.encoded_ctx_len > 0 and self.book is not None, "nothing has been encoded yet"
         c = self._cache_arg
         if c is None:
-            c = self._cache_arg = ops.make_cache(self._enc.buf, self._bi.buf, self._ti.buf, self.book, self._mi.buf,
-                                                 self._sc.buf, self.spec, self._enc.n, self.max_block_bytes)
+            # (from addresses: as tensors, the parts of a shared allocation took 10 us of a cache's first get() or mat_vec_mul())
+            s = self.spec
+            c = self._cache_arg = ops.Cache(self._enc.at, self._enc.n, self._bi.at, self._ti.at, self.book.blob.data_ptr(),
+                                            ops.QMeta(self._mi.at, self._sc.at, self._mi.size, s.tok_div, s.sj, s.sb, s.sh, s.sc), self.max_block_bytes, 0)
             self._cache_q = c.q
             return c
         c.encoded, c.encoded_bytes, c.max_block_bytes = self._enc.at, self._enc.n, self.max_block_bytes
