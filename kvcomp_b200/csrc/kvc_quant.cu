@@ -874,8 +874,8 @@ extern "C" int kvc_quantize(const void *x, int64_t T, int64_t B, int64_t H, int6
 }
 
 // The same for units side by side over the channels that cover TOKENS tokens or more: a thread's eight channels have the same units in all of them, so a
-// thread loads them once and has TOKENS loads of codes in flight.  (512 rows of 32 x 32 heads, 67 M values: 58 us where a thread takes the channels of one
-// token, now 31.)
+// thread loads them once and has TOKENS loads of codes in flight.  (512 rows of 32 x 32 heads, 67 M values: 56 us where a thread takes the channels of one
+// token, now 33.)
 namespace {
 template <int TOKENS>
 __global__ void __launch_bounds__(256) dequant_channel_kernel(const uint8_t *__restrict__ codes, kvc_qmeta_dev m, uint32_t H, uint32_t per_head, uint32_t per_token,
@@ -918,10 +918,11 @@ extern "C" int kvc_dequant(const uint8_t *codes, const kvc_qmeta *q, int64_t T, 
     const kvc_qmeta_dev m = kvc_to_dev(*q);
     const int wide_units = m.sc == 1 && m.sj % 8 == 0 && m.sb % 8 == 0 && m.sh % 8 == 0 &&
                            (reinterpret_cast<uintptr_t>(m.scale) & 15) == 0 && (reinterpret_cast<uintptr_t>(m.min_int) & (8 * m.min_bytes - 1)) == 0;
-    // (below 8 tokens for each of 512 threads per SM the single tokens fill the device better: 64 x 128 values 2.1 us)
+    // (Four tokens and one per thread: 0.52 M values 2.04 and 2.04 us, 0.86 M 2.33 and 2.44, 1.05 M 2.34 and 2.75, 2.1 M 2.55 and 3.57, 8.4 M 5.0 and 8.7, 67 M 33 and
+    // 56; 0.12 M 2.23 and 2.14, 0.26 M 2.04 and 1.94: below 512 threads per SM the single tokens fill the device better.)
     constexpr int TOKENS = 4;
     const long long per_token = B * H * (D / 8);
-    if (wide_units && m.tok_div % TOKENS == 0 && T % TOKENS == 0 && n > 8 * 512ll * kvc_sm_count() && T / TOKENS <= 65535 && per_token < (1ll << 31)) {
+    if (wide_units && m.tok_div % TOKENS == 0 && T % TOKENS == 0 && n > 512ll * kvc_sm_count() && T / TOKENS <= 65535 && per_token < (1ll << 31)) {
         dequant_channel_kernel<TOKENS><<<dim3((unsigned)((per_token + 255) / 256), (unsigned)(T / TOKENS)), 256, 0, kvc_cu(stream)>>>(
             codes, m, (uint32_t)H, (uint32_t)(D / 8), (uint32_t)per_token, reinterpret_cast<__half *>(out));
         KVC_LAUNCH_OK();

@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T,B,H,block", [(64, 8, 74, 64), (64, 8, 75, 64), (320, 8, 20, 64), (256, 5, 31, 128), (130, 9, 33, 2), (63, 16, 40, 3), (128, 40, 8, 64)])
+@pytest.mark.parametrize("T,B,H,block", [(64, 1, 74, 64), (64, 1, 75, 64), (65, 3, 33, 5), (128, 2, 19, 2), (64, 8, 74, 64), (64, 8, 75, 64), (320, 8, 20, 64), (256, 5, 31, 128), (130, 9, 33, 2), (63, 16, 40, 3), (128, 40, 8, 64)])
 @pytest.mark.parametrize("dtype", [torch.int8, torch.int16])
 def test_values(T, B, H, block, dtype):
     if not torch.cuda.is_available():
