@@ -443,16 +443,16 @@ __global__ void __launch_bounds__(BOOK_THREADS) build_codebook_kernel(const unsi
                 next++;
             }
         } else {
-        Heap hp; hp.w = reinterpret_cast<unsigned long long *>(s.hf); hp.n = 0;
-        for (uint32_t i = 0; i < nsym; i++) heap_push(hp, s.count[i], (short)s.listed[i]);
-        while (hp.n > 1) {
-            long long fa, fb;
-            short a = heap_pop(hp, &fa);
-            short b = heap_pop(hp, &fb);
-            s.parent[a] = (short)(next << 1); s.parent[b] = (short)(next << 1 | 1);
-            heap_push(hp, fa + fb, next);
-            next++;
-        }
+            Heap hp;
+            hp.w = reinterpret_cast<unsigned long long *>(s.hf); hp.n = 0;
+            for (uint32_t i = 0; i < nsym; i++) heap_push(hp, s.count[i], (short)s.listed[i]);
+            while (hp.n > 1) {
+                long long fa, fb;
+                const short a = heap_pop(hp, &fa), b = heap_pop(hp, &fb);
+                s.parent[a] = (short)(next << 1); s.parent[b] = (short)(next << 1 | 1);
+                heap_push(hp, fa + fb, next);
+                next++;
+            }
         }
         s.total = next - 1;                                 // the root
     }

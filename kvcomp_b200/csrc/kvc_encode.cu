@@ -10,14 +10,15 @@
 //   copy    the image goes out as 128-bit stores, shifted to the destination's alignment on the way
 // Books whose symbols are all below 32 (error bounds of 0.05 and more) keep the code table in registers, look symbols
 // up with warp shuffles and fill words without a 64-bit register.  What bounds it: the chain of a block's phases -- its number, its codes, sizes, words, offset, copy --
-// with 32 warps per SM that issue 55 % of the time (15 and 16 instructions per symbol).  256 columns of 4096 tokens, words ORed, a mask per code and lengths by byte products, V's
-// codes by 4-byte loads, and now: K 125 and 107 us, V 127 and 113.  (CTAs that stay and draw the next block while one's bytes go out: 196 where one block per CTA takes 135, a
-// block drawn early announces its size late; 18 or 20 CTAs per SM with fewer registers: 144.)
+// with 32 warps per SM that issue 55 % of the time (15 and 16 instructions per symbol).  256 columns of 4096 tokens, the kernel by itself, words ORed, a mask per code and lengths by byte
+// products, V's codes by 4-byte loads, and now: K 121 and 102 us, V 125 and 111.  (With 18 CTAs per SM of 56 registers 108 and 122, with 20 of 48 112 and 126; 64 registers spill 8 bytes.
+// CTAs that stay and draw the next block while one's bytes go out: a whole call, 30 us around the kernel, took 196 us where one block per CTA then took 135: a block drawn early announces
+// its size late.)
 #include "kvc_decode.cuh"
 
 namespace {
 
-constexpr int TILE_STRIDE = 132;                  // bytes per vector row in shared memory (padded; K's rows written and read by 128-bit words, 144 bytes apart: 145 us where this takes 135)
+constexpr int TILE_STRIDE = 132;                  // bytes per vector row in shared memory (padded; rows written and read by 128-bit words, 144 bytes apart: K 111 us where this takes 102)
 constexpr int OUT_CAP = 8192 + 32;                // block image: 8191 bytes max + alignment lead + slack
 
 constexpr int ENC_THREADS = 64;                   // one thread per vector of the block

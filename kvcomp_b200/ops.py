@@ -148,19 +148,16 @@ class TimedCall:
 
 
 class Report:
-    """What a store's kernels report -- the encoder's byte count and largest block, the quantiser's and the encoder's
-    status words -- in one zeroed int64[4] (and the histogram behind it), so that one copy brings all of it to the host."""
-    __slots__ = ("words", "hist", "total", "quant_status", "enc_status")
+    """What an encoder launched by itself reports -- its byte count and largest block, its status word -- in one zeroed int64[4] laid out as
+    a store's (Reports), so that one copy brings all of it to the host."""
+    __slots__ = ("words", "total", "enc_status")
 
-    def __init__(self, device, with_hist=False):
-        buf = torch.zeros(260 if with_hist else 4, dtype=torch.int64, device=device)
-        self.words, self.hist = (buf[:4], buf[4:]) if with_hist else (buf, None)
-        self.total = buf[:2]
-        half = buf[2:4].view(torch.int32)
-        self.quant_status, self.enc_status = half[0:1], half[2:3]
+    def __init__(self, device):
+        self.words = torch.zeros(4, dtype=torch.int64, device=device)
+        self.total, self.enc_status = self.words[:2], self.words[3:].view(torch.int32)[:1]
 
     def read(self):
-        """(bytes, largest block, quantiser flags, encoder flags); synchronises."""
+        """(bytes, largest block, 0, encoder flags); synchronises."""
         return self.words.tolist()
 
 
@@ -345,7 +342,7 @@ def quantize_heads_fits(mode, batch_shared, T, B, H, D, block):
 def quantize_heads(x, T, cos, sin, mode, block, rel, batch_shared, min_int, scale, hist=None, status=None):
     """The first T tokens of a prompt x fp16 [B, H, t, 128] as its projections leave it, rotated with cos / sin where
     they are given: the codes u8 [T, B, H, 128], min_int and scale that quantize gives for rope_store's rows, without
-    the rows."""
+    the rows.  (For callers of their own: a context's store quantises, builds its book and encodes in one call, store_at.)"""
     lib = _lib.load()
     _cuda(x, torch.float16, "x")
     B, H, t, D = x.shape
