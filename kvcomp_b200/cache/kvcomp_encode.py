@@ -76,7 +76,8 @@ class _Arena:
         return self.buf[self.n:self.n + extra]
 
     def used(self):
-        return self.buf[:self.n] if self._mem is not None else None
+        """What is in use; None while nothing is, whether there is memory or not."""
+        return self.buf[:self.n] if self.n else None
 
 
 class _RecentRows:

@@ -114,6 +114,18 @@ def test_refused_keys_do_not_count(on_cpu, flags):
     assert kc.book is book and (kc.ctx_len, kc.compressed_ctx_len, kc.encoded_ctx_len) == (200, 192, 192) and on_cpu.builds[4:] == [False]
 
 
+def test_a_stream_that_holds_nothing_is_none(on_cpu):
+    """64 tokens of values wait for the other half of their Huffman block; refused keys have no unit parameters either."""
+    vc, kc = KVCompCtx(False, B, H, D, 0.1), KVCompCtx(True, B, H, D, 0.05)
+    vc.store(torch.zeros(64 + 32, B, H, D, dtype=torch.float16))
+    assert vc.compressed_ctx_len == 64 and vc.encoded_data is None and vc.block_infos is None and vc.thread_infos is None
+    assert vc.quant_min_ints.numel() == vc.quant_scales.numel() == 64
+    on_cpu.flags = (_lib.FLAG_CODE_OVERFLOW, 0)
+    with pytest.raises(_lib.KvcError):
+        kc.store(torch.zeros(128, B, H, D, dtype=torch.float16))
+    assert all(x is None for x in (kc.encoded_data, kc.block_infos, kc.thread_infos, kc.quant_min_ints, kc.quant_scales))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("heads", [True, False])
 def test_a_retry_stores_what_a_first_call_would(monkeypatch, heads):
