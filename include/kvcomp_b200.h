@@ -226,7 +226,7 @@ int kvc_encode(const uint8_t *codes, int64_t T, int64_t cols, int is_k,
  * and scratch's first four words -- bytes of the stream, its largest block, the quantiser's and the encoder's status -- are copied to
  * `report` (pinned host memory), which holds them once the stream has come that far.  rest_rows > 0 (heads only): the tokens behind the first T as rows
  * (kvc_rope_store_rows), no more than x has; kept_rows > 0: the last of the T tokens, whole units of them, dequantised (kvc_dequant).  The encoder's total starts at 0 with every call.
- * T = 0: codes that the caller has are encoded, nothing else.  base_offset: below 2^32, as the recorded block offsets are. */
+ * T = 0: codes that the caller has are encoded, nothing else; T = 0 and enc_T = 0 is refused.  base_offset: below 2^32, as the recorded block offsets are. */
 typedef struct {
     const void *x, *cos_, *sin_;
     int64_t cos_batch_stride, B, H, x_tokens, T, D, block;

@@ -32,6 +32,7 @@ extern "C" int kvc_store_packed(const kvc_store_args *args, kvc_stream_t stream)
     KVC_REQUIRE((reinterpret_cast<uintptr_t>(a.scratch) & 15) == 0 && a.scratch_bytes >= kvc_store_scratch(a.mode, a.batch_shared, a.T, a.B, a.H, a.block, a.enc_T, a.is_k),
                 "kvc_store_packed: scratch must be 16-byte aligned and hold what kvc_store_scratch says");
     KVC_REQUIRE(a.T > 0 || !a.build, "kvc_store_packed: nothing to build a book from");
+    KVC_REQUIRE(a.T > 0 || a.enc_T > 0, "kvc_store_packed: nothing to store");     // (kvc_encode has no codes to look at then and refuses the call)
     KVC_REQUIRE(a.kept_rows >= 0 && a.kept_rows <= a.T && a.rest_rows >= 0, "kvc_store_packed: bad row counts");
     KVC_REQUIRE(a.rest_rows == 0 || (a.heads && a.T > 0 && a.rest && a.rest_rows <= a.x_tokens - a.T),
                 "kvc_store_packed: %lld rows behind the first %lld of %lld tokens", (long long)a.rest_rows, (long long)a.T, (long long)a.x_tokens);

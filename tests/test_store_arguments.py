@@ -43,3 +43,8 @@ def test_the_encoders_refuse_them_too(monkeypatch, offset):
     for call in (ops.encode, ops.encode_now):
         with pytest.raises(_lib.KvcError, match="32 bits"):
             call(codes, True, buf, buf, buf, buf, base_offset=offset)
+
+
+def test_a_call_for_nothing():
+    """No token and no code: kvc_encode refused such a call, as a tensor without elements has no address."""
+    assert "nothing to store" in _refusal(T=0, enc_T=0, build=0, rest_rows=0, kept_rows=0)
