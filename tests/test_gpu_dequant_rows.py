@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T,B,H,block", [(64, 1, 74, 64), (64, 1, 75, 64), (65, 3, 33, 5), (128, 2, 19, 2), (64, 8, 74, 64), (64, 8, 75, 64), (320, 8, 20, 64), (256, 5, 31, 128), (130, 9, 33, 2), (63, 16, 40, 3), (128, 40, 8, 64)])
+@pytest.mark.parametrize("T,B,H,block", [(64, 8, 74, 64), (64, 8, 75, 64), (320, 8, 20, 64), (256, 5, 31, 128), (130, 9, 33, 2), (63, 16, 40, 3), (128, 40, 8, 64)])
 @pytest.mark.parametrize("dtype", [torch.int8, torch.int16])
 def test_values(T, B, H, block, dtype):
     if not torch.cuda.is_available():
@@ -22,3 +22,10 @@ def test_values(T, B, H, block, dtype):
     u = (T // block, 1, B, H, 128)
     want = ((codes.view(T // block, block, B, H, 128).int() + mi.view(u).int()).half() * sc.view(u)).view(codes.shape)      # the sum in whole numbers
     assert torch.equal(ops.dequant(codes, mi, sc, spec), want)
+
+
+# around 512 threads per SM, from where a thread takes several tokens
+@pytest.mark.parametrize("T,B,H,block", [(64, 1, 74, 64), (64, 1, 75, 64), (65, 3, 33, 5), (128, 2, 19, 2)])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.int16])
+def test_values_of_small_calls(T, B, H, block, dtype):
+    test_values(T, B, H, block, dtype)

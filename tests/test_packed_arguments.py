@@ -26,6 +26,13 @@ def test_packed_layouts_match_the_structures():
         assert got == list(range(first, first + 15))
 
 
+def test_packed_store_matches_the_structure():
+    """29 words, six numbers of 32 bits, a float and the number of entries."""
+    assert _lib.STORE_ARGS.size == 29 * 8 + 8 * 4
+    blob = _lib.STORE_ARGS.pack(*range(29), *range(6), 0.5, 0)
+    assert int.from_bytes(blob[28 * 8:29 * 8], "little") == 28 and int.from_bytes(blob[29 * 8 + 20:29 * 8 + 24], "little") == 5
+
+
 STORE_FIELDS = ("x cos_ sin_ cos_batch_stride B H x_tokens T D block codes min_int scale scratch scratch_bytes book enc_codes enc_T base_offset block_info "
                 "thread_info encoded encoded_capacity rest rest_rows kept kept_rows report enc_table mode batch_shared heads is_k build min_bytes rel n_entries").split()
 
@@ -45,7 +52,7 @@ def _header_fields(struct):
     return fields
 
 
-def test_packed_store_matches_the_structure():
+def test_packed_store_has_the_headers_fields():
     """The header's fields, in its order, with their sizes: 29 words, six numbers of 32 bits, a float and the number of the encode table's entries."""
     fields = _header_fields("kvc_store_args")
     assert [name for name, _ in fields] == STORE_FIELDS
