@@ -106,8 +106,10 @@ class KVCompCache(_BASE):
         kc, vc = self._ctx(layer_idx, key_states.shape[1])
         if not k_stored:
             kc.store(key_states.permute(2, 0, 1, 3).contiguous().half())
-        if begun is not None and self._values_begun(kc, vc, begun, value_states):
-            return
+        if begun is not None:
+            both, begun = self._values_begun(kc, vc, begun, value_states), None      # (no codes of the keys are held from here on)
+            if both:
+                return
         t = value_states.shape[2]
         plain = self._plain(value_states)
         place = vc.recent_place(t, value_states.device) if plain else None
@@ -123,13 +125,18 @@ class KVCompCache(_BASE):
     def _plain(x):
         return x.is_cuda and x.dtype == torch.float16 and x.is_contiguous() and x.shape[3] % 16 == 0
 
+    # Bytes that the keys' store may hold while the values' is launched.  A first prompt's holds nothing; a later one's codes and window came on top of
+    # all that the values' store takes (2048 tokens of 128 heads behind 2000 others: at its peak 329 MB, 239 one after the other).  One wait for both
+    # saves some 35 us whatever the size: 590 and 626 us with 67 MB of codes, 920 and 954 with 134, 1641 and 1669 with 268.
+    HELD = 64 << 20
+
     @staticmethod
     def _values_begun(kc, vc, begun, values):
         """Finish the store of keys that has begun; True if the values' store went with it, behind one wait for both."""
         v_begun = None
         try:
             # (one wait is for one device)
-            if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and values.device == kc.device \
+            if KVCompCache._plain(values) and values.data_ptr() % 16 == 0 and values.device == kc.device and kc.held(begun) <= KVCompCache.HELD \
                     and vc.recent_place(values.shape[2], values.device) is None:
                 v_begun = vc.begin_heads(values, keep_codes=False)
         finally:

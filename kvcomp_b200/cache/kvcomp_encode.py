@@ -183,7 +183,7 @@ class _Begun(NamedTuple):
     n_old: int
     buf: object
     n_rest: int
-    put_rest: object
+    put_rest: object         # None: the rest has been written
     blocks: int              # of the stream
 
 
@@ -464,7 +464,14 @@ class KVCompCtx:
         # written, nothing reads the codes again.  (Keys' and values' on their way together would else be held at the same time.)
         if not keep_codes and build and over and n_enc == old + n:
             pend = part = None
+        if over:
+            put_rest = None                                   # (it holds the new tokens' rows, all of them)
         return _Begun(slot, book, pend, old, part, n_enc, stream_room, cap, n_units, n, t, over, k, n_old, buf, n_rest, put_rest, blocks)
+
+    def held(self, begun):
+        """Bytes that a begun store keeps until _finish: its codes, and the window that another one takes the place of."""
+        window = self._recent.buf if begun.over else None
+        return (0 if begun.pend is None else begun.pend.numel()) + (0 if window is None else window.numel() * window.element_size())
 
     def _finish(self, begun, waited=False):
         """The rest of a begun store: waits for it (waited: the caller has), then it counts.  A store that the device refuses does not

@@ -1,4 +1,5 @@
 """Stores that fail, in part or as a whole, and stores that wait together."""
+import copy
 import types
 
 import pytest
@@ -95,6 +96,22 @@ def test_values_of_another_device_are_waited_for(on_cpu):
         assert both == (values is x) and (kc.ctx_len, vc.ctx_len) == (200, 200 if both else 0) and on_cpu.waits == [x.device]
 
 
+def test_values_wait_for_keys_that_hold_much(monkeypatch, on_cpu):
+    """A first prompt's store holds nothing for its end; a later one's codes and the window that is replaced count."""
+    x = torch.zeros(B, H, 200, D, dtype=torch.float16)
+    kc, vc = KVCompCtx(True, B, H, D, 0.05, keep_dequantised=True), KVCompCtx(False, B, H, D, 0.1, keep_dequantised=True)
+    monkeypatch.setattr(KVCompCache, "HELD", 0)
+    assert KVCompCache._values_begun(kc, vc, kc.begin_heads(x, keep_codes=False), x)
+    held = 192 * B * H * D + kc._recent.buf.numel() * 2
+    for limit, both in ((held - 1, False), (held, True)):
+        with monkeypatch.context() as m:
+            m.setattr(KVCompCache, "HELD", limit)
+            a, b = copy.deepcopy(kc), copy.deepcopy(vc)
+            begun = a.begin_heads(x, keep_codes=False)
+            assert begun.over and begun.n == 192 and begun.put_rest is None and a.held(begun) == held
+            assert KVCompCache._values_begun(a, b, begun, x) == both and (a.ctx_len, b.ctx_len) == (400, 400 if both else 200)
+
+
 @pytest.mark.parametrize("flags", [(_lib.FLAG_CODE_OVERFLOW, 0), (_lib.FLAG_MIN_OVERFLOW, 0), (0, _lib.FLAG_BLOCK_LONG)])
 def test_refused_keys_do_not_count(on_cpu, flags):
     """Neither they nor the values that were on their way with them; the next prompt's books are its own."""
@@ -175,3 +192,34 @@ def test_a_layer_whose_keys_were_refused_takes_the_next_prompt():
         assert a.ctx_len == b.ctx_len == 300
         for x, y in zip(*((c.encoded_data, c.block_infos, c.thread_infos, c.quant_min_ints, c.quant_scales, c.buffer, c.get()[0]) for c in (a, b))):
             assert torch.equal(x, y)
+
+
+@pytest.mark.gpu
+def test_a_long_prompt_behind_a_first_one_needs_little_more_memory_for_both():
+    """Than its keys and its values stored one after the other."""
+    heads, t = 128, 2048
+    g = torch.Generator(device="cuda").manual_seed(7)
+
+    def new(n):
+        return [torch.randn(1, heads, n, D, device="cuda", generator=g).half() for _ in range(2)], \
+            {name: torch.full((1, n, D), x, dtype=torch.float16, device="cuda") for name, x in (("cos", 1.0), ("sin", 0.0))}
+
+    def together(cache, kv, rot):
+        cache.append(kv[0], kv[1], 0, rot)
+
+    def apart(cache, kv, rot):
+        cache.k_ctx[0].store_heads(kv[0], rot["cos"], rot["sin"])
+        cache.v_ctx[0].store_heads(kv[1])
+    peaks = []
+    for call in (apart, together):
+        cache = KVCompCache(1, heads, D, 1)
+        cache.append(*new(2000)[0], 0, new(2000)[1])         # (leaves rows in the windows)
+        args = new(t)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        at = torch.cuda.memory_allocated()
+        call(cache, *args)
+        torch.cuda.synchronize()
+        peaks.append(torch.cuda.max_memory_allocated() - at)
+        del cache, args
+    assert peaks[1] <= peaks[0] + (64 << 20), peaks
