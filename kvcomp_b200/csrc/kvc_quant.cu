@@ -163,7 +163,10 @@ __device__ __forceinline__ void minmax8(const uint4 &v, float &mn, float &mx) {
 // CTA = one (j, b, h) tile of blk tokens x 128 channels; thread = 8 channels x every 8th token.
 // (Measured slower: several tiles per CTA with one flush of the bins; tiles of two or four heads; the tile's
 // rows held in registers between the two passes; four rows in flight per thread in either pass.)
-__global__ void __launch_bounds__(128) quant_channel_kernel(
+// Seven CTAs per SM: 71 registers.  (The tile's place by three 64-bit divisions took 72, and 74 since a code comes from one difference, which leaves room for six:
+// 256 columns of 4096 tokens, per head and channel, without and with a histogram 107.4 and 118.6 us, then 112.2 and 125.1, now 98.9 and 109.5; 16 columns of 4096
+// 8.5 and 9.5, 9.2 and 10.9, 7.7 and 9.0; one tile 3.6 and 4.1, 3.4 and 3.9, 3.2 and 3.7.)
+__global__ void __launch_bounds__(128, 7) quant_channel_kernel(
     const __half *__restrict__ x, long long B, long long H, int blk, float rel,
     uint8_t *__restrict__ codes, void *__restrict__ min_int, int min_bytes, __half *__restrict__ scale,
     unsigned long long *__restrict__ ghist, int *__restrict__ status) {
@@ -173,9 +176,8 @@ __global__ void __launch_bounds__(128) quant_channel_kernel(
     const long long row_stride = B * H * 128;
     if (ghist) { for (int i = tid; i < 256; i += 128) shist[i] = 0; }      // a barrier follows before the first count
     int flags = 0;
-    const long long tile = blockIdx.x;                 // (j * B + b) * H + h
-    const long long h = tile % H, b = (tile / H) % B, j = tile / (H * B);
-    const long long base = ((j * blk) * B + b) * H * 128 + h * 128 + cg * 8;
+    const uint32_t tile = blockIdx.x, cols = (uint32_t)(B * H), j = tile / cols;          // (j * B + b) * H + h, below 2^31
+    const long long base = ((long long)j * blk * cols + (tile - j * cols)) * 128 + cg * 8;
     __half2 mn2[4], mx2[4];                                 // extremes of the thread's 8 channels, two per register
 #pragma unroll
     for (int i = 0; i < 4; i++) { mn2[i] = __float2half2_rn(INFINITY); mx2[i] = __float2half2_rn(-INFINITY); }
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(128) quant_channel_kernel(
         for (int rr = 1; rr < 8; rr++) { a = fminf(a, smn[rr][tid]); z = fmaxf(z, smx[rr][tid]); }
         __half sc;
         const UnitParam q = unit_param(a, z, rel, &sc, &flags);
-        const long long u = tile * 128 + tid;
+        const long long u = tile * 128ll + tid;
         scale[u] = sc;
         store_min(min_int, min_bytes, u, q.mi, &flags);
         __syncthreads();                                   // every partial is read before the rows are reused
