@@ -681,6 +681,7 @@ struct AttnParams {
     int spare;                    // there is room for a table of V's single symbols beside that of pairs
     int team;                     // without partial results: this many workers of a CTA share a column's steps and add up in shared memory (0: each its own columns)
     int partial;                  // items leave partial results for the merge kernel (several runs per column, or a tail that the merge kernel adds)
+    int early;                    // one head: the merge kernel is let go when a worker of every CTA has no further item, else when one has ended
     int wait_limit;               // tries of a staging wait before it gives up (KVC_FLAG_WAIT_TIMEOUT)
     int starve;                   // tests of the bounded waits only: announce bytes that are never copied
 };
@@ -1372,7 +1373,7 @@ __global__ void __launch_bounds__(128 * ONE_WORKERS, 1) attn_one_kernel(AttnPara
     uint32_t par = 0;                                      // bit 0 / bit 1: parity of the staging phase the K / V barrier is waited for next
     while (have) {
     const int col = it.col, b = col / Hkv, h = col % Hkv;
-    if (!have_next) release();
+    if (!have_next && p.early) release();
     if (draw && tid == 0) drawn = atomicAdd(&p.sched[0], 1);
     sm.q[tid] = qn;
     sync();
@@ -2099,6 +2100,11 @@ extern "C" int kvc_attn_decode(const kvc_cache *k, const kvc_cache *v, int64_t T
         p.spare = GG > 1 && !p.brief && attn_smem<GG>(p, workers) + 4 * KVC_LUT_SIZE <= MAX_CTA_SHARED;         \
         const size_t smem = attn_smem<GG>(p, workers);                                                          \
         p.workers = workers;                                                                                    \
+        /* (one head) Without a tail the merge kernel has nothing to do beside the last items, and a CTA of more than four workers leaves it no room there: let go early it */ \
+        /* made long launches slower than one that is let go by a worker's end.  (Kernels by other ones, in a graph, let go early and now: 4 columns of 32768 tokens 27.2 and 25.8 us, of */ \
+        /* 65536 47.4 and 45.9, 16 of 20480 49.1 and 48.4, 8 of 65536 76.8 and 74.8; one behind the other 24.2 and 24.8, 45.3 and 42.6, 46.5 and 45.0, 74.4 and 71.4; 256 of */ \
+        /* 4096 120.6 and 120.8.  With up to four workers, let go early and late: 32 of 256 7.9 and 10.8, 16 of 4096 13.8 and 14.1.) */ \
+        p.early = Tr > 0 || workers <= 4;                                                                       \
         /* (threads that only help to load the tables would take the merge kernel's place beside a brief launch) */ \
         const int threads = 128 * (GG == 1 || p.brief ? workers : rows_workers<GG>());                           \
         static kvc_launch_slot slots[4];                                                                        \
