@@ -375,10 +375,10 @@ class KVCompCtx:
         n = self._cut(live, t)
         if live or n == 0 or x.data_ptr() % 16 or not ops.quantize_heads_fits(mode, self.batch_shared, n, B, H, D, self.block_size) \
                 or (cos is not None and mode != ops.MODE_CHANNEL):
-            return self._begin(ops.rope_store(x, cos, sin))
+            return self._begin(ops.rope_store(x, cos, sin), keep_codes)
         cos, sin, stride = ops._rotation(ops._cuda(x, torch.float16, "x"), cos, sin)
         if cos is not None and (cos.data_ptr() | sin.data_ptr()) % 16:
-            return self._begin(ops.rope_store(x, cos, sin))
+            return self._begin(ops.rope_store(x, cos, sin), keep_codes)
         self._check(x.permute(2, 0, 1, 3))
         return self._launch(x, n, 0, t - n, t, t, None, cos, sin, stride, keep_codes)
 
@@ -387,7 +387,7 @@ class KVCompCtx:
         Returns the uint8 codes of the newly compressed tokens as [n_blocks, block, B, H, D] (or None)."""
         return self._finish(self._begin(cache))
 
-    def _begin(self, cache):
+    def _begin(self, cache, keep_codes=True):
         self._check(cache)
         live, t = len(self._recent), cache.shape[0]
         n = self._cut(live, t)
@@ -401,7 +401,7 @@ class KVCompCtx:
             x, rest = self._recent.view()[:n].clone(), cache  # the window's front
         else:
             x, rest = torch.cat([self._recent.view(), cache[:n - live]], dim=0), cache[n - live:]
-        return self._launch(x, n, live, rest.shape[0], t, 0, lambda place: place.copy_(rest))
+        return self._launch(x, n, live, rest.shape[0], t, 0, lambda place: place.copy_(rest), keep_codes=keep_codes)
 
     def _launch(self, x, n, live, n_rest, t, x_tokens, put_rest, cos=None, sin=None, stride=0, keep_codes=True):
         """Launch the compression of the first n tokens of (the `live` rows of the window + t new tokens): x as rows, or (x_tokens > 0) as a

@@ -112,6 +112,17 @@ def test_values_wait_for_keys_that_hold_much(monkeypatch, on_cpu):
             assert KVCompCache._values_begun(a, b, begun, x) == both and (a.ctx_len, b.ctx_len) == (400, 400 if both else 200)
 
 
+def test_a_first_prompt_of_rows_holds_nothing(on_cpu):
+    """Keys whose units are not per channel are rotated into rows first."""
+    KVCompCacheConfigStatic.config.k_quant_mode = QuantMode("BlockQuant")
+    x, rot = torch.zeros(B, H, 200, D, dtype=torch.float16), torch.ones(1, 200, D, dtype=torch.float16)
+    kc = KVCompCtx(True, B, H, D, 0.05, keep_dequantised=True)
+    begun = kc.begin_heads(x, rot, rot, keep_codes=False)
+    assert begun.n == 192 and begun.n_rest == 8 and kc.held(begun) == 0 and begun.put_rest is None
+    assert kc._finish(begun) is None and kc.ctx_len == 200 and kc._pending is None
+    assert KVCompCtx(True, B, H, D, 0.05).store_heads(x, rot, rot).numel() == 192 * B * H * D
+
+
 @pytest.mark.parametrize("flags", [(_lib.FLAG_CODE_OVERFLOW, 0), (_lib.FLAG_MIN_OVERFLOW, 0), (0, _lib.FLAG_BLOCK_LONG)])
 def test_refused_keys_do_not_count(on_cpu, flags):
     """Neither they nor the values that were on their way with them; the next prompt's books are its own."""
