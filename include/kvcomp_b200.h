@@ -48,7 +48,7 @@ extern "C" {
 #define KVC_FLAG_ZERO_SCALE      0x001  /* quantiser: a unit is constant (reference: NaN codes) */
 #define KVC_FLAG_MIN_OVERFLOW    0x002  /* quantiser: min_int does not fit the requested width */
 #define KVC_FLAG_CODE_OVERFLOW   0x004  /* quantiser: a code is outside 0..255 */
-#define KVC_FLAG_SYMBOL_MISSING  0x008  /* encoder: symbol without a code was dropped */
+#define KVC_FLAG_SYMBOL_MISSING  0x008  /* encoder: symbol without a code, or with one of more than 32 bits, was dropped */
 #define KVC_FLAG_VECTOR_LONG     0x010  /* encoder: a vector exceeds the reference's scratch (K 128 B, V 256 B) */
 #define KVC_FLAG_BLOCK_LONG      0x020  /* encoder: a block exceeds 8191 B, its u16 fields are invalid */
 #define KVC_FLAG_STREAM_FULL     0x040  /* encoder: `encoded` capacity exceeded, output truncated */

@@ -260,11 +260,10 @@ __global__ void __launch_bounds__(ENC_THREADS, 16) encode_onepass_kernel(
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int i = tid + k * ENC_THREADS;
-        const uint2 e = te[k];
+        const uint2 e = te[k].y <= 32u ? te[k] : make_uint2(0u, 0u);     // (a code beyond the table's 32 bits is none: its symbol is reported as missing)
         tab[i] = e;
         kind |= (e.y > 16u ? 1 : 0) | (e.y && i >= 32 ? 2 : 0) | (e.y > 13u ? 4 : 0) | (e.y > 8u ? 8 : 0);
-        const uint32_t l = min(e.y, 32u);
-        lens[i] = (uint16_t)(l ? l : (1u << 14));
+        lens[i] = (uint16_t)(e.y ? e.y : (1u << 14));
     }
     kind = (int)__reduce_or_sync(0xffffffffu, (unsigned)kind);
     if (lane == 0) wkind[warp] = kind;

@@ -44,3 +44,29 @@ def test_longest_codes(is_k, longest, off):
         assert not ops.read_status(st, raise_on_fatal=False) & ~ops._lib.FLAG_VECTOR_LONG and int(total[0]) == odata.size
         assert np.array_equal(enc[:odata.size].cpu().numpy(), odata)
         assert np.array_equal(bi.cpu().numpy(), obi) and np.array_equal(ti.cpu().numpy().view(np.uint16), oti)
+
+
+@pytest.mark.parametrize("is_k", [True, False])
+@pytest.mark.parametrize("length", [32, 33, 36, 64, 1 << 31])
+def test_codes_beyond_the_table(is_k, length):
+    """A table entry has 32 bits for a code: a symbol whose code is longer has none, and is reported where it occurs."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from kvcomp_b200 import ops
+    T, B, H = 128, 1, 2
+    entries = np.zeros((256, 2), "<u4")
+    entries[:3] = [[0, 1], [2, 2], [0xc0000000, length]]
+    table = torch.from_numpy(entries.view(np.uint8).reshape(-1).copy()).cuda()
+    bsz, tsz, _, cap = ops.buffer_sizes(T, B * H * 128, is_k)
+    for used in (False, True):
+        codes = torch.zeros(T, B, H, 128, dtype=torch.uint8, device="cuda")
+        codes[5, 0, 1, 7] = 1
+        if used:
+            codes[T - 1, 0, H - 1, 127] = 2                   # the last vector's last symbol
+        bi, ti, enc = (torch.zeros(n, dtype=torch.uint8, device="cuda") for n in (bsz, tsz, cap))
+        total, st = ops.encode(codes, is_k, table, bi, ti, enc)
+        flags = ops.read_status(st, raise_on_fatal=False)
+        assert bool(flags & ops._lib.FLAG_SYMBOL_MISSING) == (used and length > 32)
+        # a bit a symbol, two for the one, and 31 more for a code of 32 bits
+        n = T * B * H * 16 + 1 + (4 if used and length == 32 else 0)
+        assert int(total[0]) == n
