@@ -60,3 +60,9 @@ def test_values_that_start_on_two_bytes(ops, T, B, Hkv, G, Tr):  # noqa: F811
     assert odd.data_ptr() % 4 == 2
     outs = [ops.attn_decode(kc, vc, T, B, Hkv, q, 0.1, kt, v)[0] for v in (vt, odd)]
     assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all())
+
+
+# one head and no tail: up to four workers in a CTA and more, in one round and in several
+@pytest.mark.parametrize("T,B,Hkv", [(256, 1, 32), (4096, 2, 8), (4096, 1, 32), (8448, 4, 4), (4096, 3, 40)])
+def test_steps_without_a_tail(ops, T, B, Hkv):  # noqa: F811
+    test_steps_without_a_wait(ops, T, B, Hkv, 1, 0)
